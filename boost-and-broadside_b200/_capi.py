@@ -154,6 +154,23 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
 lib = load_library()
 
 
+def _load_host_path():
+    """The CPython module with the host side of a call (csrc/host_path.cpp), linked against the
+    library loaded above."""
+    import importlib.util
+
+    path = os.path.join(_HERE, "_host_path.so")
+    if not os.path.exists(path):
+        raise RuntimeError(f"{path} is missing: build it with `python boost-and-broadside_b200/build.py`")
+    spec = importlib.util.spec_from_file_location("_host_path", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
+host = _load_host_path()
+
+
 class BnbError(RuntimeError):
     """A C-ABI call returned a non-zero status."""
 

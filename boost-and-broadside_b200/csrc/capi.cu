@@ -8,6 +8,7 @@
 #include "exact_kernels.h"
 #include "mlp_kernels.h"
 #include "grad_kernels.h"
+#include "host_calls.h"
 #include "launch_count.h"
 #include "validate.h"
 #include "tensor_kernels.h"
@@ -104,6 +105,79 @@ bool all_packed(const BnbSpatialWeights* s, int ns, const BnbTemporalWeights* t,
 }
 
 }  // namespace
+
+namespace bnb {
+namespace host {
+
+int trunk_call(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, int n_blocks, int n_spatial, int n_temporal,
+               int D, int H, const void* x_any, const uint8_t* alive, const BnbBullets* bullets, void* y_any, const float* hidden_in,
+               float* hidden_out, const uint8_t* done, const uint8_t* reset_env, const BnbBatch* batch, int T, int precision,
+               int engine, void* scratch, size_t scratch_bytes, void* stream, bool is_sequence, bool pack) {
+  const float* x = static_cast<const float*>(x_any);   // bfloat16 elements under BNB_BF16_IO
+  float* y = static_cast<float*>(y_any);
+  int st = check_dims(D, H);
+  if (st) return st;
+  if ((st = check_batch(batch))) return st;
+  if (n_blocks < 0 || n_spatial < 0 || n_temporal < 0 || T < 1) return BNB_ERR_BAD_ARGUMENT;
+  const bool io_bf16 = precision == BNB_BF16_IO;
+  if (io_bf16) precision = BNB_BF16;
+  if (precision != BNB_FP32 && precision != BNB_BF16) return BNB_ERR_BAD_ARGUMENT;
+  if (n_blocks * n_spatial > 0 && !spatial) return BNB_ERR_NULL_POINTER;
+  if (n_blocks * n_temporal > 0 && !temporal) return BNB_ERR_NULL_POINTER;
+  for (int i = 0; i < n_blocks * n_spatial; ++i)
+    if ((st = check_spatial(&spatial[i]))) return st;
+  for (int i = 0; i < n_blocks * n_temporal; ++i)
+    if ((st = check_temporal(&temporal[i], batch->total_tokens > batch->total_ships))) return st;
+  if ((st = check_bullets(bullets))) return st;
+  if (!any_reads_bullets(spatial, n_blocks * n_spatial, bullets)) bullets = nullptr;
+  size_t n_rows = (size_t)T * batch->total_tokens;
+  if (n_rows == 0) return BNB_OK;
+  if (!x || !y) return BNB_ERR_NULL_POINTER;
+  if (!aligned16(x) || !aligned16(y) || !aligned16(hidden_in) || !aligned16(hidden_out)) return BNB_ERR_MISALIGNED;
+  const bool has_state = n_blocks * n_temporal > 0 && batch->total_ships > 0;
+  if (has_state && !hidden_in) return BNB_ERR_NULL_POINTER;
+  if (has_state && !is_sequence && !hidden_out) return BNB_ERR_NULL_POINTER;
+  cudaStream_t cs = static_cast<cudaStream_t>(stream);
+
+  if (use_tensor(precision, engine, D, H, batch, bullets) &&
+      (engine == BNB_ENGINE_TENSOR || all_packed(spatial, n_blocks * n_spatial, temporal, n_blocks * n_temporal)))
+    return bnb::tensor::trunk(spatial, temporal, n_blocks, n_spatial, n_temporal, D, H, x, alive, bullets, y, hidden_in,
+                              hidden_out, done, reset_env, *batch, T, scratch, scratch_bytes, cs, io_bf16, pack);
+  if (engine == BNB_ENGINE_TENSOR || io_bf16 || (bullets && bullets->tokens_bf16)) return BNB_ERR_UNSUPPORTED_DIMS;
+
+  Scratch s{nullptr, nullptr, nullptr, 0};
+  if (n_blocks * n_spatial > 0 &&
+      (st = carve(scratch, scratch_bytes, n_rows, D, (long long)T * batch->n_envs, bullets ? bullets->per_env : 0, &s)))
+    return st;
+  const bool emu = precision == BNB_BF16;
+  const float* cur = x;
+  const size_t slot_stride = (size_t)batch->total_ships * 4 * D;
+  if (n_blocks * (n_spatial + n_temporal) == 0) {
+    if (y != x && cudaMemcpyAsync(y, x, n_rows * D * sizeof(float), cudaMemcpyDeviceToDevice, cs) != cudaSuccess)
+      return BNB_ERR_LAUNCH;
+    return BNB_OK;
+  }
+  for (int i = 0; i < n_blocks; ++i) {
+    for (int j = 0; j < n_spatial; ++j) {
+      st = bnb::exact::spatial_block(spatial[i * n_spatial + j], D, H, cur, alive, bullets, y, *batch, T, emu, s.qkv,
+                                     s.o, s.kvb, s.kvb_envs, cs);
+      if (st) return st;
+      cur = y;
+    }
+    for (int j = 0; j < n_temporal; ++j) {
+      int slot = i * n_temporal + j;
+      st = bnb::exact::temporal_block(temporal[slot], D, cur, y, hidden_in ? hidden_in + slot * slot_stride : nullptr,
+                                      hidden_out ? hidden_out + slot * slot_stride : nullptr, done, reset_env,
+                                      *batch, T, emu, cs);
+      if (st) return st;
+      cur = y;
+    }
+  }
+  return BNB_OK;
+}
+
+}  // namespace host
+}  // namespace bnb
 
 extern "C" {
 
@@ -209,80 +283,14 @@ int bnb_temporal_block_fwd(const BnbTemporalWeights* w, int d_model, const float
                                     precision == BNB_BF16, cs);
 }
 
-static int trunk_common(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, int n_blocks,
-                        int n_spatial, int n_temporal, int D, int H, const float* x, const uint8_t* alive,
-                        const BnbBullets* bullets, float* y, const float* hidden_in, float* hidden_out, const uint8_t* done,
-                        const uint8_t* reset_env, const BnbBatch* batch, int T, int precision, int engine,
-                        void* scratch, size_t scratch_bytes, void* stream, bool is_sequence) {
-  int st = check_dims(D, H);
-  if (st) return st;
-  if ((st = check_batch(batch))) return st;
-  if (n_blocks < 0 || n_spatial < 0 || n_temporal < 0 || T < 1) return BNB_ERR_BAD_ARGUMENT;
-  const bool io_bf16 = precision == BNB_BF16_IO;
-  if (io_bf16) precision = BNB_BF16;
-  if (precision != BNB_FP32 && precision != BNB_BF16) return BNB_ERR_BAD_ARGUMENT;
-  if (n_blocks * n_spatial > 0 && !spatial) return BNB_ERR_NULL_POINTER;
-  if (n_blocks * n_temporal > 0 && !temporal) return BNB_ERR_NULL_POINTER;
-  for (int i = 0; i < n_blocks * n_spatial; ++i)
-    if ((st = check_spatial(&spatial[i]))) return st;
-  for (int i = 0; i < n_blocks * n_temporal; ++i)
-    if ((st = check_temporal(&temporal[i], batch->total_tokens > batch->total_ships))) return st;
-  if ((st = check_bullets(bullets))) return st;
-  if (!any_reads_bullets(spatial, n_blocks * n_spatial, bullets)) bullets = nullptr;
-  size_t n_rows = (size_t)T * batch->total_tokens;
-  if (n_rows == 0) return BNB_OK;
-  if (!x || !y) return BNB_ERR_NULL_POINTER;
-  if (!aligned16(x) || !aligned16(y) || !aligned16(hidden_in) || !aligned16(hidden_out)) return BNB_ERR_MISALIGNED;
-  const bool has_state = n_blocks * n_temporal > 0 && batch->total_ships > 0;
-  if (has_state && !hidden_in) return BNB_ERR_NULL_POINTER;
-  if (has_state && !is_sequence && !hidden_out) return BNB_ERR_NULL_POINTER;
-  cudaStream_t cs = static_cast<cudaStream_t>(stream);
-
-  if (use_tensor(precision, engine, D, H, batch, bullets) &&
-      (engine == BNB_ENGINE_TENSOR || all_packed(spatial, n_blocks * n_spatial, temporal, n_blocks * n_temporal)))
-    return bnb::tensor::trunk(spatial, temporal, n_blocks, n_spatial, n_temporal, D, H, x, alive, bullets, y, hidden_in,
-                              hidden_out, done, reset_env, *batch, T, scratch, scratch_bytes, cs, io_bf16);
-  if (engine == BNB_ENGINE_TENSOR || io_bf16 || (bullets && bullets->tokens_bf16)) return BNB_ERR_UNSUPPORTED_DIMS;
-
-  Scratch s{nullptr, nullptr, nullptr, 0};
-  if (n_blocks * n_spatial > 0 &&
-      (st = carve(scratch, scratch_bytes, n_rows, D, (long long)T * batch->n_envs, bullets ? bullets->per_env : 0, &s)))
-    return st;
-  const bool emu = precision == BNB_BF16;
-  const float* cur = x;
-  const size_t slot_stride = (size_t)batch->total_ships * 4 * D;
-  if (n_blocks * (n_spatial + n_temporal) == 0) {
-    if (y != x && cudaMemcpyAsync(y, x, n_rows * D * sizeof(float), cudaMemcpyDeviceToDevice, cs) != cudaSuccess)
-      return BNB_ERR_LAUNCH;
-    return BNB_OK;
-  }
-  for (int i = 0; i < n_blocks; ++i) {
-    for (int j = 0; j < n_spatial; ++j) {
-      st = bnb::exact::spatial_block(spatial[i * n_spatial + j], D, H, cur, alive, bullets, y, *batch, T, emu, s.qkv,
-                                     s.o, s.kvb, s.kvb_envs, cs);
-      if (st) return st;
-      cur = y;
-    }
-    for (int j = 0; j < n_temporal; ++j) {
-      int slot = i * n_temporal + j;
-      st = bnb::exact::temporal_block(temporal[slot], D, cur, y, hidden_in ? hidden_in + slot * slot_stride : nullptr,
-                                      hidden_out ? hidden_out + slot * slot_stride : nullptr, done, reset_env,
-                                      *batch, T, emu, cs);
-      if (st) return st;
-      cur = y;
-    }
-  }
-  return BNB_OK;
-}
-
 int bnb_trunk_step(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, int n_blocks,
                    int n_spatial, int n_temporal, int d_model, int n_heads, const float* x,
                    const uint8_t* alive, const BnbBullets* bullets, float* y, const float* hidden_in,
                    float* hidden_out, const uint8_t* reset_env, const BnbBatch* batch, int precision, int engine,
                    void* scratch, size_t scratch_bytes, void* stream) {
-  return trunk_common(spatial, temporal, n_blocks, n_spatial, n_temporal, d_model, n_heads, x, alive, bullets, y,
-                      hidden_in, hidden_out, nullptr, reset_env, batch, 1, precision, engine, scratch, scratch_bytes, stream,
-                      false);
+  return bnb::host::trunk_call(spatial, temporal, n_blocks, n_spatial, n_temporal, d_model, n_heads, x, alive, bullets, y,
+                               hidden_in, hidden_out, nullptr, reset_env, batch, 1, precision, engine, scratch, scratch_bytes,
+                               stream, false, false);
 }
 
 int bnb_trunk_sequence(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, int n_blocks,
@@ -290,9 +298,9 @@ int bnb_trunk_sequence(const BnbSpatialWeights* spatial, const BnbTemporalWeight
                        const uint8_t* alive, const BnbBullets* bullets, float* y, const float* hidden_in,
                        float* hidden_out, const uint8_t* done, const BnbBatch* batch, int timesteps, int precision, int engine,
                        void* scratch, size_t scratch_bytes, void* stream) {
-  return trunk_common(spatial, temporal, n_blocks, n_spatial, n_temporal, d_model, n_heads, x, alive, bullets, y,
-                      hidden_in, hidden_out, done, nullptr, batch, timesteps, precision, engine, scratch, scratch_bytes, stream,
-                      true);
+  return bnb::host::trunk_call(spatial, temporal, n_blocks, n_spatial, n_temporal, d_model, n_heads, x, alive, bullets, y,
+                               hidden_in, hidden_out, done, nullptr, batch, timesteps, precision, engine, scratch, scratch_bytes,
+                               stream, true, false);
 }
 
 size_t bnb_trunk_bwd_scratch_bytes(int n_blocks, int n_spatial, int n_temporal, int d_model, const BnbBatch* batch,

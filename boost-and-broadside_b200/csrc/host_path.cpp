@@ -1,0 +1,343 @@
+// The host side of a call in native code: a CPython module (built as _host_path.so, linked against
+// libbnb_trunk.so) that gathers a trunk's parameters, fills the C structs, takes outputs from torch's
+// allocator and launches, without an interpreter in between.
+//
+// Why it exists: the same work as Python over ctypes took 230-250 us per trunk call (64 parameters
+// x several attribute look-ups and checks, then the operator dispatcher), against 140 us of kernels
+// at the small end.  Here it is a few microseconds beside the launches themselves.
+//
+// The Python side (yemong/_ops.py, yemong/_end_ops.py) keeps what is policy: which buffer is the
+// scratch of a stream, the warning about slow engine choices, the autograd formulas.
+#include <torch/extension.h>
+
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+
+#include <vector>
+
+#include "bnb_trunk.h"
+#include "host_calls.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = c10::optional<Tensor>;
+
+namespace {
+
+// ------------------------------------------------------------------ parameters of a trunk
+
+// Names interned once; a module's children and parameters are read from its own dictionaries, so a
+// replaced sub-module or parameter is seen at the next call.
+struct Names {
+  PyObject *modules, *parameters, *spatial, *temporal, *field_sub, *norm1, *qkv, *out_proj, *norm2, *ffn, *gate_proj, *up_proj,
+      *down_proj, *norm_bullet, *kv_bullet, *weight, *bias, *linear1, *conv, *rg_lru, *log_lambda, *linear_a, *linear_x, *linear2,
+      *linear_out, *gated_mlp;
+};
+const Names& names() {
+  static const Names* n = [] {
+    auto s = [](const char* t) { return PyUnicode_InternFromString(t); };
+    return new Names{s("_modules"), s("_parameters"), s("spatial"), s("temporal"), s("field_sub"), s("norm1"), s("qkv"), s("out_proj"),
+                     s("norm2"), s("ffn"), s("gate_proj"), s("up_proj"), s("down_proj"), s("norm_bullet"), s("kv_bullet"), s("weight"),
+                     s("bias"), s("linear1"), s("conv"), s("rg_lru"), s("log_lambda"), s("linear_a"), s("linear_x"), s("linear2"),
+                     s("linear_out"), s("gated_mlp")};
+  }();
+  return *n;
+}
+
+// Borrowed reference to module.<dict>[key], or nullptr without an exception set.
+PyObject* member(PyObject* module, PyObject* dict_name, PyObject* key) {
+  if (!module) return nullptr;
+  PyObject* d = PyObject_GetAttr(module, dict_name);
+  if (!d) { PyErr_Clear(); return nullptr; }
+  PyObject* v = PyDict_Check(d) ? PyDict_GetItemWithError(d, key) : nullptr;
+  Py_DECREF(d);   // the module keeps it
+  return v;
+}
+struct Gather {
+  std::vector<Tensor> out;
+  bool ok = true;
+  PyObject* child(PyObject* m, PyObject* key) { return member(m, names().modules, key); }
+  void param(PyObject* m, PyObject* key) {
+    PyObject* p = member(m, names().parameters, key);
+    if (!p || !THPVariable_Check(p)) { ok = false; return; }
+    out.push_back(THPVariable_Unpack(p));
+  }
+  void weight(PyObject* m, PyObject* name) { param(child(m, name), names().weight); }
+  void mlp(PyObject* m) {
+    const Names& n = names();
+    weight(m, n.gate_proj);
+    weight(m, n.up_proj);
+    weight(m, n.down_proj);
+  }
+  std::vector<PyObject*> items(PyObject* list) {   // children of a ModuleList, in order
+    std::vector<PyObject*> v;
+    if (!list) { ok = false; return v; }
+    PyObject* d = PyObject_GetAttr(list, names().modules);
+    if (!d) { PyErr_Clear(); ok = false; return v; }
+    PyObject *k, *m;
+    Py_ssize_t pos = 0;
+    if (PyDict_Check(d)) while (PyDict_Next(d, &pos, &k, &m)) v.push_back(m);
+    Py_DECREF(d);
+    return v;
+  }
+};
+
+// Parameters of `blocks` (YemongBlock modules) in the order of yemong/_weights.py, block-major, with
+// the field substitutes where the call has field tokens; None when a module does not hold its
+// parameters in the ordinary place (a parametrisation), and the caller gathers them by attribute.
+py::object trunk_params(const py::sequence& blocks, bool has_fields) {
+  const Names& n = names();
+  Gather g;
+  g.out.reserve(80);
+  for (const auto& b : blocks) {
+    PyObject* block = b.ptr();
+    for (PyObject* sp : g.items(g.child(block, n.spatial))) {
+      g.weight(sp, n.norm1);
+      g.weight(sp, n.qkv);
+      g.weight(sp, n.out_proj);
+      g.weight(sp, n.norm2);
+      g.mlp(g.child(sp, n.ffn));
+      if (g.child(sp, n.kv_bullet)) {
+        g.weight(sp, n.norm_bullet);
+        g.weight(sp, n.kv_bullet);
+      }
+    }
+    const auto subs = g.items(g.child(block, n.field_sub));
+    size_t j = 0;
+    for (PyObject* tp : g.items(g.child(block, n.temporal))) {
+      PyObject* lru = g.child(tp, n.rg_lru);
+      PyObject* conv = g.child(tp, n.conv);
+      g.weight(tp, n.norm1);
+      g.weight(tp, n.linear1);
+      g.param(conv, n.weight);
+      g.param(conv, n.bias);
+      g.param(lru, n.log_lambda);
+      PyObject* la = g.child(lru, n.linear_a);
+      PyObject* lx = g.child(lru, n.linear_x);
+      g.param(la, n.weight);
+      g.param(la, n.bias);
+      g.param(lx, n.weight);
+      g.param(lx, n.bias);
+      g.weight(tp, n.linear2);
+      g.weight(tp, n.linear_out);
+      g.weight(tp, n.norm2);
+      g.mlp(g.child(tp, n.gated_mlp));
+      if (has_fields) {
+        if (j >= subs.size()) { g.ok = false; break; }
+        g.param(subs[j], n.weight);
+      }
+      ++j;
+    }
+    if (!g.ok) return py::none();
+  }
+  return py::cast(g.out);
+}
+
+// ------------------------------------------------------------------ small helpers
+
+constexpr int kEngineSimt = BNB_ENGINE_SIMT;
+
+const void* ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
+
+Tensor f32c(const Tensor& t) {
+  const Tensor f = t.scalar_type() == at::kFloat ? t : t.to(at::kFloat);
+  return f.is_contiguous() ? f : f.contiguous();
+}
+Tensor contiguous(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+// One byte per element: a bool tensor as it is, anything else compared with zero.
+OptTensor bytes_of(const OptTensor& t) {
+  if (!t.has_value()) return c10::nullopt;
+  return t->scalar_type() == at::kBool ? contiguous(*t) : contiguous(t->ne(0));
+}
+const float* parameter(const Tensor& t, const c10::Device& dev, const char* what) {
+  if (t.device() != dev)
+    throw std::runtime_error(std::string(what) + " parameter is on " + t.device().str() + ", input on " + dev.str());
+  if (t.scalar_type() != at::kFloat || !t.is_contiguous())
+    throw std::runtime_error(std::string(what) + " parameter must be contiguous float32 (got " + c10::toString(t.scalar_type()) + ")");
+  return static_cast<const float*>(t.data_ptr());
+}
+void check(const char* fn, int status) {
+  if (status == BNB_OK) return;
+  const std::string text = std::string(fn) + ": " + bnb_status_string(status);
+  if (status == BNB_ERR_UNSUPPORTED_DIMS) throw py::value_error(text);
+  throw std::runtime_error(text + " (status " + std::to_string(status) + ")");
+}
+// A bounded wait of an earlier call on this device ran out (its kernels drained and its outputs were
+// garbage): say so once, at the next call, without synchronising.
+void raise_pending_status(const c10::Device& dev) {
+  const int st = bnb_last_status();
+  if (!st) return;
+  bnb_clear_status();
+  throw std::runtime_error("an earlier tensor-core call on " + dev.str() + " gave up a bounded wait: " + bnb_status_string(st) +
+                           " (status " + std::to_string(st) + "); its outputs, and any state carried from them, are invalid");
+}
+
+constexpr int N_SPATIAL = 7, N_TEMPORAL = 15;   // parameters of a sublayer, + bullets / field substitute
+
+// The integers of a call (yemong/_ops.py names the entries).
+struct Geometry {
+  int blocks, spatial, temporal, heads, bullet_cross, field_sub, envs, tokens_per_env, ships_per_env, max_tokens, total_tokens,
+      total_ships, tiles, timesteps, engine, precision;
+  explicit Geometry(const std::vector<int64_t>& g) {
+    if (g.size() != 16) throw std::runtime_error("geom must hold 16 integers");
+    int* f[] = {&blocks, &spatial, &temporal, &heads, &bullet_cross, &field_sub, &envs, &tokens_per_env, &ships_per_env, &max_tokens,
+                &total_tokens, &total_ships, &tiles, &timesteps, &engine, &precision};
+    for (int i = 0; i < 16; ++i) *f[i] = (int)g[i];
+  }
+  BnbBatch batch(const std::vector<Tensor>& offsets) const {
+    BnbBatch b{};
+    b.n_envs = envs;
+    b.tokens_per_env = offsets.empty() ? tokens_per_env : 0;
+    b.ships_per_env = offsets.empty() ? ships_per_env : 0;
+    b.max_tokens_per_env = max_tokens;
+    b.total_tokens = total_tokens;
+    b.total_ships = total_ships;
+    if (!offsets.empty()) {
+      b.tok_off = static_cast<const int32_t*>(offsets[0].data_ptr());
+      b.ship_off = static_cast<const int32_t*>(offsets[1].data_ptr());
+      if (offsets.size() > 2) b.tile_env_begin = static_cast<const int32_t*>(offsets[2].data_ptr());
+      if (offsets.size() > 3) b.tile_env_ids = static_cast<const int32_t*>(offsets[3].data_ptr());
+      b.n_tiles = tiles;
+    }
+    return b;
+  }
+};
+
+struct Weights {
+  std::vector<BnbSpatialWeights> spatial;
+  std::vector<BnbTemporalWeights> temporal;
+};
+Weights weight_structs(const Geometry& g, const std::vector<Tensor>& ts, const c10::Device& dev) {
+  Weights w;
+  w.spatial.resize((size_t)g.blocks * g.spatial);
+  w.temporal.resize((size_t)g.blocks * g.temporal);
+  size_t want = 0, pos = 0;
+  for (int j = 0; j < g.spatial; ++j) want += N_SPATIAL + (j < g.bullet_cross ? 2 : 0);
+  want += (size_t)g.temporal * (N_TEMPORAL + (g.field_sub ? 1 : 0));
+  want *= g.blocks;
+  if (want != ts.size())
+    throw std::runtime_error("expected " + std::to_string(want) + " parameter tensors for this trunk structure, got " + std::to_string(ts.size()));
+  for (int i = 0; i < g.blocks; ++i) {
+    for (int j = 0; j < g.spatial; ++j) {
+      BnbSpatialWeights& s = w.spatial[(size_t)i * g.spatial + j];
+      s = BnbSpatialWeights{};
+      const float** f[] = {&s.norm1_w, &s.qkv_w, &s.out_w, &s.norm2_w, &s.gate_w, &s.up_w, &s.down_w, &s.norm_bullet_w, &s.kv_bullet_w};
+      const int n = N_SPATIAL + (j < g.bullet_cross ? 2 : 0);
+      for (int k = 0; k < n; ++k) *f[k] = parameter(ts[pos++], dev, "spatial");
+    }
+    for (int j = 0; j < g.temporal; ++j) {
+      BnbTemporalWeights& s = w.temporal[(size_t)i * g.temporal + j];
+      s = BnbTemporalWeights{};
+      const float** f[] = {&s.norm1_w, &s.linear1_w, &s.conv_w, &s.conv_b, &s.log_lambda, &s.a_w, &s.a_b, &s.x_w, &s.x_b, &s.linear2_w,
+                           &s.out_w, &s.norm2_w, &s.gate_w, &s.up_w, &s.down_w, &s.field_sub_w};
+      const int n = N_TEMPORAL + (g.field_sub ? 1 : 0);
+      for (int k = 0; k < n; ++k) *f[k] = parameter(ts[pos++], dev, "temporal");
+    }
+  }
+  return w;
+}
+
+// The bullet tokens of a call in the form the C ABI takes; holds what it converted.
+struct Bullets {
+  Tensor tokens;
+  OptTensor active;
+  BnbBullets arg{};
+  bool present = false;
+  Bullets(const OptTensor& bullets, const OptTensor& mask, int64_t n_envs, int64_t d_model, bool keep_bf16) {
+    if (!bullets.has_value()) return;
+    const Tensor& b = *bullets;
+    if (b.dim() != 3 || b.size(0) != n_envs || b.size(2) != d_model || b.size(1) < 1) {
+      std::ostringstream s;
+      s << "bullets must have shape (" << n_envs << ", NB >= 1, " << d_model << "), got " << b.sizes();
+      throw std::runtime_error(s.str());
+    }
+    if (!b.is_cuda())
+      throw std::runtime_error("bullets is on " + b.device().str() + "; the trunk kernels run on CUDA only (sm_100a) and have no CPU path");
+    if (mask.has_value() && (mask->dim() != 2 || mask->size(0) != b.size(0) || mask->size(1) != b.size(1))) {
+      std::ostringstream s;
+      s << "bullet_mask must have shape (" << b.size(0) << ", " << b.size(1) << "), got " << mask->sizes();
+      throw std::runtime_error(s.str());
+    }
+    const bool is_bf16 = keep_bf16 && b.scalar_type() == at::kBFloat16;
+    tokens = is_bf16 ? contiguous(b) : f32c(b);
+    active = bytes_of(mask);
+    arg.tokens = static_cast<const float*>(tokens.data_ptr());
+    arg.active = static_cast<const uint8_t*>(ptr(active));
+    arg.per_env = (int)b.size(1);
+    arg.tokens_bf16 = is_bf16 ? 1 : 0;
+    present = true;
+  }
+  const BnbBullets* get() const { return present ? &arg : nullptr; }
+};
+
+size_t round256(size_t v) { return (v + 255) / 256 * 256; }
+
+// ------------------------------------------------------------------ the trunk
+
+// What bnb_b200::trunk_forward does (yemong/_ops.py).  scratch_for(device, bytes) returns the byte
+// buffer of the current stream.
+std::tuple<Tensor, Tensor> trunk_forward(const Tensor& x, const OptTensor& alive, const Tensor& hidden, const OptTensor& done,
+                                         const OptTensor& reset_env, const OptTensor& bullets, const OptTensor& bullet_mask,
+                                         const std::vector<Tensor>& weights, const std::vector<Tensor>& offsets,
+                                         const std::vector<int64_t>& geom, const py::object& scratch_for) {
+  const Geometry g(geom);
+  const c10::Device dev = x.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const int64_t D = x.size(-1);
+  const int T = g.timesteps > 1 ? g.timesteps : 1;
+  const BnbBatch batch = g.batch(offsets);
+  const bool bf16 = g.precision == BNB_BF16, tensor_engine = bf16 && g.engine != kEngineSimt;
+  const bool built = tensor_engine && g.max_tokens > 0 && bnb_supported((int)D, g.heads, g.max_tokens, BNB_BF16, BNB_ENGINE_TENSOR);
+  // bfloat16 tokens stay bfloat16 on the way in and out where the fused kernels serve the call;
+  // anything else is converted to float32 here
+  const bool io16 = built && x.scalar_type() == at::kBFloat16 && (offsets.empty() || offsets.size() > 2);
+  const bool images = tensor_engine && bnb_supported((int)D, g.heads, 1, BNB_BF16, BNB_ENGINE_TENSOR);
+
+  Weights w = weight_structs(g, weights, dev);
+  const Tensor hin = f32c(hidden);
+  const OptTensor alive_u8 = bytes_of(alive), done_u8 = bytes_of(done), reset_u8 = bytes_of(reset_env);
+  Tensor hout = at::empty_like(hin);
+  raise_pending_status(dev);
+  const auto stream = at::cuda::getCurrentCUDAStream(dev.index());
+
+  auto run = [&](bool tokens16, bool bullets16, Tensor* y, bool* used_bullets16) {
+    const Tensor xin = tokens16 ? contiguous(x) : f32c(x);
+    *y = at::empty_like(xin);
+    const Bullets b(g.bullet_cross > 0 ? bullets : c10::nullopt, bullet_mask, (int64_t)T * batch.n_envs, D, bullets16);
+    *used_bullets16 = b.present && b.arg.tokens_bf16;
+    const size_t need = round256(bnb_scratch_bytes((int)D, &batch, T, b.arg.per_env));
+    const size_t sp = round256(bnb_packed_spatial_bytes((int)D)), tp = round256(bnb_packed_temporal_bytes((int)D));
+    const size_t image_bytes = images ? sp * w.spatial.size() + tp * w.temporal.size() : 0;
+    const Tensor scratch = scratch_for(dev, need + image_bytes).cast<Tensor>();
+    uint8_t* base = static_cast<uint8_t*>(scratch.data_ptr());
+    // The weight images live behind the call's scratch and are rewritten from the parameters by every
+    // call, so they cannot go stale: not after an optimizer step, not after p.data.copy_() (which bumps
+    // no version counter; the reference's running-average policy is updated that way,
+    // train/rl/opponents.py:112), and not in a replayed CUDA graph.
+    uint8_t* image = base + need;
+    for (auto& s : w.spatial) { s.packed = images ? image : nullptr; image += sp; }
+    for (auto& s : w.temporal) { s.packed = images ? image : nullptr; image += tp; }
+    return bnb::host::trunk_call(w.spatial.data(), w.temporal.data(), g.blocks, g.spatial, g.temporal, (int)D, g.heads, xin.data_ptr(),
+                                 static_cast<const uint8_t*>(ptr(alive_u8)), b.get(), y->data_ptr(),
+                                 static_cast<const float*>(hin.data_ptr()), static_cast<float*>(hout.data_ptr()),
+                                 static_cast<const uint8_t*>(ptr(done_u8)), static_cast<const uint8_t*>(ptr(reset_u8)), &batch, T,
+                                 tokens16 ? BNB_BF16_IO : g.precision, g.engine, base, (size_t)scratch.numel(), stream.stream(),
+                                 g.timesteps != 0, images);
+  };
+  Tensor y;
+  bool used16 = false;
+  int st = run(io16, built, &y, &used16);
+  // a shape the tensor-core kernels do not serve (say, more bullet slots than their attention stages;
+  // nothing was launched): once more with float32 copies for the kernels that read float32
+  if (st == BNB_ERR_UNSUPPORTED_DIMS && (io16 || used16)) st = run(false, false, &y, &used16);
+  check(g.timesteps == 0 ? "bnb_trunk_step" : "bnb_trunk_sequence", st);
+  if (x.scalar_type() == at::kBFloat16 && y.scalar_type() != at::kBFloat16) y = y.to(at::kBFloat16);
+  return {y, hout};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_host_path, m) {
+  m.def("trunk_params", &trunk_params);
+  m.def("trunk_forward", &trunk_forward);
+}

@@ -915,7 +915,7 @@ __device__ __forceinline__ void issue_temporal(Issuer& m, bool has_fields) {
 __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_constant__ TrunkArgs args) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ int s_aborted[2];
+  __shared__ __align__(8) int s_aborted[4];   // [2..3]: address of the host's status word
   __shared__ int s_items;
   __shared__ SubLayer s_sub[MAX_SUBLAYERS];  // kernel parameters are slow to index dynamically
   __shared__ uint32_t s_sched[MAX_SCHED];
@@ -927,6 +927,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 8 * B_COUNT);
   if (tid == 0) {
     s_aborted[0] = (*args.status != 0) ? 1 : 0;
+    *reinterpret_cast<int**>(&s_aborted[2]) = args.host_status;
     s_aborted[1] = args.poll_limit > 0 ? args.poll_limit : DEFAULT_POLL_LIMIT;
     mbar_init(smem_u32(&bars[B_OP0]), EPI_WARPS);
     mbar_init(smem_u32(&bars[B_OP1]), EPI_WARPS);

@@ -84,6 +84,7 @@ struct TrunkArgs {
   const int* row_index;
   const int* n_rows_dev;
   int* status;
+  int* host_status;   // pinned host word that a wait which runs out writes its code to, or null
   // Test hooks of the bounded waits (0 / -1 in normal use): the poll limit of this launch, and the
   // ring operation of CTA 0 whose weight copy the fetching lane leaves out, so that the issuing
   // lane's wait for it runs out and the kernel has to drain and return with a status code.
@@ -116,9 +117,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 // Bounded wait: gives up after a number of polls, records `code` in the status word and lets the
-// caller go on.  `aborted` points at two shared ints: [0] is set once any wait of the CTA has run
+// caller go on.  `aborted` points at four shared ints: [0] is set once any wait of the CTA has run
 // out (later waits then give up after four polls, so the kernel drains quickly), [1] is the poll
-// limit of this launch.
+// limit of this launch, [2..3] hold the address of the host's status word (or null).
 constexpr int DEFAULT_POLL_LIMIT = 1 << 20;
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, int* status, volatile int* aborted, int code) {
   if (mbar_try_wait(bar, parity)) return;   // the common case costs one instruction
@@ -126,7 +127,9 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, int* st
   for (int i = 0; i < limit; ++i)
     if (mbar_try_wait(bar, parity)) return;
   *aborted = 1;
-  atomicCAS(status, 0, code);
+  if (atomicCAS(status, 0, code) == 0) {   // the first code of the call is the one reported
+    if (int* host = *reinterpret_cast<int* volatile*>(const_cast<int*>(&aborted[2]))) *static_cast<volatile int*>(host) = code;
+  }
 }
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"

@@ -139,11 +139,13 @@ __global__ void k_pack_temporal(BnbTemporalWeights w, uint8_t* out) {
 constexpr int MAX_PACK_JOBS = 8;
 struct PackJobs {
   int n_spatial, n_temporal;
+  int* status;   // zeroed by the launch (null: nobody asked)
   BnbSpatialWeights sw[MAX_PACK_JOBS];
   BnbTemporalWeights tw[MAX_PACK_JOBS];
 };
 __global__ void k_pack_trunk(const __grid_constant__ PackJobs jobs) {
   const int j = blockIdx.y;
+  if (jobs.status && j == 0 && blockIdx.x == 0 && threadIdx.x == 0) *jobs.status = 0;
   if (j < jobs.n_spatial) {
     const BnbSpatialWeights& w = jobs.sw[j];
     pack_image(w, N_SPATIAL_IMAGE, static_cast<uint8_t*>(const_cast<void*>(w.packed)),
@@ -921,7 +923,7 @@ template <int NQ, int MAXKB>
 __global__ void __launch_bounds__(128 * NQ, NQ == 4 ? 1 : 2) k_trunk_tiles(const __grid_constant__ TrunkArgs args) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ int s_aborted[2];
+  __shared__ __align__(8) int s_aborted[4];   // [2..3]: address of the host's status word
   __shared__ int s_items;
   __shared__ SubLayer s_sub[MAX_SUBLAYERS];  // kernel parameters are slow to index dynamically
   __shared__ uint16_t s_sched[MAX_SUBLAYERS * N_TEMPORAL_CHUNKS];  // (chunk << 6) | (sublayer << 2) | slot
@@ -947,6 +949,7 @@ __global__ void __launch_bounds__(128 * NQ, NQ == 4 ? 1 : 2) k_trunk_tiles(const
 
   if (tid == 0) {
     s_aborted[0] = (*args.status != 0) ? 1 : 0;
+    *reinterpret_cast<int**>(&s_aborted[2]) = args.host_status;
     s_aborted[1] = args.poll_limit > 0 ? args.poll_limit : DEFAULT_POLL_LIMIT;
     mbar_init(smem_u32(&bars[0]), 1);
     mbar_init(smem_u32(&bars[1]), 1);
@@ -1572,12 +1575,13 @@ int pack_temporal(const BnbTemporalWeights& w, int d_model, void* packed, cudaSt
 }
 
 int pack_trunk(const BnbSpatialWeights* spatial, int n_spatial, const BnbTemporalWeights* temporal, int n_temporal,
-               int d_model, int n_heads, cudaStream_t st) {
+               int d_model, int n_heads, cudaStream_t st, int* status) {
   if (d_model != D || n_heads != HEADS) return BNB_ERR_UNSUPPORTED_DIMS;
   // as many launches as it takes at MAX_PACK_JOBS sublayers of each kind per launch (one for the
   // trunks of the shipped profiles)
   for (int s0 = 0, t0 = 0; s0 < n_spatial || t0 < n_temporal;) {
     PackJobs jobs{};
+    jobs.status = status;
     for (; s0 < n_spatial && jobs.n_spatial < MAX_PACK_JOBS; ++s0) {
       if (!spatial[s0].packed) return BNB_ERR_NULL_POINTER;
       jobs.sw[jobs.n_spatial++] = spatial[s0];
@@ -1595,10 +1599,11 @@ int pack_trunk(const BnbSpatialWeights* spatial, int n_spatial, const BnbTempora
 
 // ------------------------------------------------------------------ status word on the host
 //
-// The bounded waits record a code in the status word at the head of the scratch buffer.  Every
-// call copies that word to a pinned host word of its device when its kernels are done
-// (asynchronously, on the call's stream); whoever asks later -- the next call, or
-// bnb_last_status -- finds a non-zero code there and keeps it until it is cleared.
+// The bounded waits record a code in the status word at the head of the scratch buffer, and the wait
+// that runs out writes the same code straight to a pinned, device-mapped host word of its device, so
+// that a call that goes well costs no copy (a 4-byte download per call took 3.4 us of the stream);
+// whoever asks later -- the next call, or bnb_last_status -- finds a non-zero code there and keeps it
+// until it is cleared.
 namespace {
 constexpr int kMaxDevices = 64;
 std::mutex g_status_mutex;
@@ -1613,22 +1618,22 @@ void latch_status(int dev) {
 }
 }  // namespace
 
-int report_status(const int* status, cudaStream_t st) {
+// Device address of the host word of the current device, allocating it on the first call (null
+// during a stream capture without it: that capture's launches then report to their scratch only).
+static int* host_status_word(cudaStream_t st) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return BNB_ERR_NO_DEVICE;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
   std::lock_guard<std::mutex> lock(g_status_mutex);
   if (!g_host_status[dev]) {
-    // the first call on a device allocates the word; it should not come during a stream capture
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return BNB_OK;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return nullptr;
     void* p = nullptr;
-    if (cudaHostAlloc(&p, 64, cudaHostAllocDefault) != cudaSuccess) { (void)cudaGetLastError(); return BNB_OK; }
+    if (cudaHostAlloc(&p, 64, cudaHostAllocMapped) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
     g_host_status[dev] = static_cast<int*>(p);
     *g_host_status[dev] = 0;
   }
   latch_status(dev);
-  if (cudaMemcpyAsync(g_host_status[dev], status, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return BNB_ERR_LAUNCH;
-  return BNB_OK;
+  return g_host_status[dev];   // one address space: the host address is the device's too
 }
 int last_status() {
   int dev = 0;
@@ -1669,6 +1674,7 @@ static int launch(TrunkArgs& a, const BnbBatch& b, cudaStream_t st) {
   a.has_fields = b.total_tokens > b.total_ships ? 1 : 0;
   a.poll_limit = g_debug_poll_limit;
   a.skip_op = g_debug_skip_op;
+  a.host_status = host_status_word(st);
   if (a.n_tiles == 0) return BNB_OK;
   {
     // the pipelined kernel runs every program of spatial (whole or split around the attention
@@ -1712,11 +1718,11 @@ static int launch(TrunkArgs& a, const BnbBatch& b, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
 }
 
-static int prepare_status(void* scratch, size_t scratch_bytes, cudaStream_t st, int** status) {
+static int prepare_status(void* scratch, size_t scratch_bytes, cudaStream_t st, bool clear, int** status) {
   if (!scratch) return BNB_ERR_NULL_POINTER;
   if (scratch_bytes < 65536) return BNB_ERR_SCRATCH_TOO_SMALL;
   *status = static_cast<int*>(scratch);
-  if (cudaMemsetAsync(scratch, 0, 256, st) != cudaSuccess) return BNB_ERR_LAUNCH;
+  if (clear && cudaMemsetAsync(scratch, 0, 256, st) != cudaSuccess) return BNB_ERR_LAUNCH;
   return BNB_OK;
 }
 
@@ -1921,8 +1927,8 @@ struct Plan {
   }
 };
 
-static int make_plan(Plan& p, void* scratch, size_t scratch_bytes, int T) {
-  int rc = prepare_status(scratch, scratch_bytes, p.st, &p.status);
+static int make_plan(Plan& p, void* scratch, size_t scratch_bytes, int T, bool clear_status = true) {
+  int rc = prepare_status(scratch, scratch_bytes, p.st, clear_status, &p.status);
   if (rc) return rc;
   p.split = !fits_tile(p.b);
   p.qkv = nullptr;
@@ -1962,8 +1968,7 @@ int spatial_block(const BnbSpatialWeights& w, int d_model, int n_heads, const fl
   int rc = make_plan(p, scratch, scratch_bytes, n_groups);
   if (rc) return rc;
   if ((rc = p.add_spatial(w, n_groups))) return rc;
-  if ((rc = p.flush())) return rc;
-  return report_status(p.status, st);
+  return p.flush();
 }
 
 int temporal_block(const BnbTemporalWeights& w, int d_model, const float* x, float* y, const float* hidden_in,
@@ -1974,14 +1979,13 @@ int temporal_block(const BnbTemporalWeights& w, int d_model, const float* x, flo
   int rc = make_plan(p, scratch, scratch_bytes, T);
   if (rc) return rc;
   if ((rc = p.add_temporal(w, hidden_in, hidden_out, T))) return rc;
-  if ((rc = p.flush())) return rc;
-  return report_status(p.status, st);
+  return p.flush();
 }
 
 int trunk(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, int n_blocks, int n_spatial,
           int n_temporal, int d_model, int n_heads, const float* x, const uint8_t* alive, const BnbBullets* bullets,
           float* y, const float* hidden_in, float* hidden_out, const uint8_t* done, const uint8_t* reset_env,
-          const BnbBatch& b, int T, void* scratch, size_t scratch_bytes, cudaStream_t st, bool io_bf16) {
+          const BnbBatch& b, int T, void* scratch, size_t scratch_bytes, cudaStream_t st, bool io_bf16, bool pack_images) {
   if (!supported_batch(d_model, n_heads, b)) return BNB_ERR_UNSUPPORTED_DIMS;
   // bfloat16 x / y: every tile-kernel launch of the call reads and writes bfloat16 rows, so the
   // residual stream is rounded where one launch hands over to the next (the reference, given
@@ -1992,8 +1996,10 @@ int trunk(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, 
   if (T > 1 && n_blocks * n_temporal > 0 && b.total_ships > 0 && !hidden_out) return BNB_ERR_NULL_POINTER;
   Plan p{b, st, nullptr, false, alive, done, reset_env, x, y, bullets};
   p.io_bf16 = io_bf16;
-  int rc = make_plan(p, scratch, scratch_bytes, T);
+  const bool pack = pack_images && n_blocks * (n_spatial + n_temporal) > 0;
+  int rc = make_plan(p, scratch, scratch_bytes, T, !pack);
   if (rc) return rc;
+  if (pack && (rc = pack_trunk(spatial, n_blocks * n_spatial, temporal, n_blocks * n_temporal, d_model, n_heads, st, p.status))) return rc;
   const size_t slot_stride = (size_t)b.total_ships * 4 * D;
   for (int i = 0; i < n_blocks; ++i) {
     for (int j = 0; j < n_spatial; ++j)
@@ -2009,7 +2015,7 @@ int trunk(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, 
     if (cudaMemcpyAsync(y, x, (size_t)T * b.total_tokens * D * (io_bf16 ? 2 : sizeof(float)), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
       return BNB_ERR_LAUNCH;
   }
-  return report_status(p.status, st);
+  return BNB_OK;
 }
 
 }  // namespace tensor

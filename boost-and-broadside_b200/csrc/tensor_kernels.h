@@ -26,11 +26,12 @@ size_t packed_temporal_bytes(int D);
 int pack_spatial(const BnbSpatialWeights& w, int D, int H, void* packed, cudaStream_t st);
 int pack_temporal(const BnbTemporalWeights& w, int D, void* packed, cudaStream_t st);
 // Every weight image of a trunk (each struct's `packed` names its destination) in one launch.
+// status: a word the (first) launch zeroes, or null.
 int pack_trunk(const BnbSpatialWeights* spatial, int n_spatial, const BnbTemporalWeights* temporal, int n_temporal,
-               int D, int H, cudaStream_t st);
+               int D, int H, cudaStream_t st, int* status = nullptr);
 
-// Status word of the bounded waits, as last copied to the host for the current device (sticky
-// until cleared); and the test hooks that make a wait run out.
+// Status code of the bounded waits, as a kernel left it in the pinned host word of the current device
+// (sticky until cleared); and the test hooks that make a wait run out.
 int last_status();
 void clear_status();
 void debug_wait_test(int skip_op, int poll_limit);
@@ -46,7 +47,7 @@ int temporal_block(const BnbTemporalWeights& w, int D, const float* x, float* y,
 int trunk(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, int n_blocks, int n_spatial,
           int n_temporal, int D, int H, const float* x, const uint8_t* alive, const BnbBullets* bullets, float* y,
           const float* hidden_in, float* hidden_out, const uint8_t* done, const uint8_t* reset_env, const BnbBatch& b, int T,
-          void* scratch, size_t scratch_bytes, cudaStream_t st, bool io_bf16 = false);
+          void* scratch, size_t scratch_bytes, cudaStream_t st, bool io_bf16 = false, bool pack_images = false);
 
 }  // namespace tensor
 }  // namespace bnb

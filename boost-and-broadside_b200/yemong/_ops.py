@@ -25,7 +25,7 @@ from torch import Tensor
 import os
 
 from .. import _capi
-from ._weights import N_SPATIAL, N_TEMPORAL, image_buffer, packed_image, spatial_struct_from, temporal_struct_from
+from ._weights import N_SPATIAL, N_TEMPORAL, packed_image, spatial_struct_from, temporal_struct_from
 
 # geom: the integers of a call, in this order
 (G_BLOCKS, G_SPATIAL, G_TEMPORAL, G_HEADS, G_BULLET_CROSS, G_FIELD_SUB, G_ENVS, G_TOKENS_PER_ENV, G_SHIPS_PER_ENV,
@@ -93,80 +93,18 @@ def trunk_forward(
     tile_env_ids)].  Returns (y like x: bfloat16 for bfloat16 tokens, else float32; new hidden like
     hidden, float32).
     """
-    dev = x.device
-    D = x.shape[-1]
-    n_blocks, n_spatial, n_temporal = geom[G_BLOCKS], geom[G_SPATIAL], geom[G_TEMPORAL]
-    n_heads, n_cross, field_sub = geom[G_HEADS], geom[G_BULLET_CROSS], geom[G_FIELD_SUB]
-    engine, precision = geom[G_ENGINE], geom[G_PRECISION]
-    T = max(1, geom[G_TIMESTEPS])
-    with torch.cuda.device(dev):
-        batch = _batch(geom, offsets)
-        # bfloat16 tokens (what the reference's encoder hands its trunk under CUDA autocast) stay
-        # bfloat16 on the way in and out where the fused kernel serves the call; the residual stream
-        # inside the call is float32 either way.  Anything else is converted to float32 here.
-        io16 = (x.dtype == torch.bfloat16 and precision == _capi.BNB_BF16 and engine != _capi.ENGINE_SIMT
-                and geom[G_MAX_TOKENS] > 0
-                and bool(_capi.lib.bnb_supported(D, n_heads, geom[G_MAX_TOKENS], _capi.BNB_BF16, _capi.ENGINE_TENSOR))
-                and (not offsets or len(offsets) > 2))
-        hin = _capi.f32c(hidden)
-        alive_u8 = _capi.u8(alive)
-        done_u8 = _capi.u8(done)
-        reset_u8 = _capi.u8(reset_env)
-        hout = torch.empty_like(hin)
-        sw = (_capi.SpatialWeights * max(1, n_blocks * n_spatial))()
-        tw = (_capi.TemporalWeights * max(1, n_blocks * n_temporal))()
-        pos = 0
-        for i in range(n_blocks):
-            for j in range(n_spatial):
-                n = N_SPATIAL + (2 if j < n_cross else 0)
-                ts = list(weights[pos : pos + n])
-                pos += n
-                sw[i * n_spatial + j] = spatial_struct_from(
-                    ts, dev, image_buffer("spatial", ts, n_heads, dev, precision, engine))
-            for j in range(n_temporal):
-                n = N_TEMPORAL + (1 if field_sub else 0)
-                ts = list(weights[pos : pos + n])
-                pos += n
-                tw[i * n_temporal + j] = temporal_struct_from(
-                    ts, dev, image_buffer("temporal", ts, 4, dev, precision, engine))
-        if pos != len(weights):
-            raise RuntimeError(f"expected {pos} parameter tensors for this trunk structure, got {len(weights)}")
-        bul16 = (precision == _capi.BNB_BF16 and engine != _capi.ENGINE_SIMT and geom[G_MAX_TOKENS] > 0
-                 and bool(_capi.lib.bnb_supported(D, n_heads, geom[G_MAX_TOKENS], _capi.BNB_BF16, _capi.ENGINE_TENSOR)))
-        stream = _capi.stream_handle(dev)
-        _raise_pending_status(dev)
-        ns_total, nt_total = n_blocks * n_spatial, n_blocks * n_temporal
-        if all(sw[i].packed for i in range(ns_total)) and all(tw[i].packed for i in range(nt_total)) and ns_total + nt_total > 0:
-            # the weight images of the whole trunk, rewritten from the live parameters on every call
-            _capi.check("bnb_pack_trunk", _capi.lib.bnb_pack_trunk(sw, ns_total, tw, nt_total, D, n_heads, stream))
+    return trunk_call(x, alive, hidden, done, reset_env, bullets, bullet_mask, weights, offsets, geom)
+
+
+def trunk_call(x, alive, hidden, done, reset_env, bullets, bullet_mask, weights, offsets, geom):
+    """The body of ``trunk_forward``, in native code (csrc/host_path.cpp); eager calls without gradients
+    come here directly, past the operator dispatcher."""
+    out = _capi.host.trunk_forward(x, alive, hidden, done, reset_env, bullets, bullet_mask, weights, offsets, geom, _capi.scratch_for)
+    if geom[G_PRECISION] == _capi.BNB_BF16:
         fn = "bnb_trunk_step" if geom[G_TIMESTEPS] == 0 else "bnb_trunk_sequence"
-
-        def run(tokens16: bool, bullets16: bool):
-            xin = (x if x.is_contiguous() else x.contiguous()) if tokens16 else _capi.f32c(x)
-            y = torch.empty_like(xin)
-            bul = _capi.BulletArgs(bullets if n_cross > 0 else None, bullet_mask, T * batch.n_envs, D, keep_bf16=bullets16)
-            scratch = _capi.scratch_for(dev, _capi.lib.bnb_scratch_bytes(D, batch, T, bul.per_env))
-            head = (sw, tw, n_blocks, n_spatial, n_temporal, D, n_heads, xin.data_ptr(), _capi.ptr(alive_u8), bul.arg,
-                    y.data_ptr(), _capi.ptr(hin), _capi.ptr(hout))
-            tail = (_capi.BNB_BF16_IO if tokens16 else precision, engine, scratch.data_ptr(), scratch.numel(), stream)
-            if geom[G_TIMESTEPS] == 0:
-                st = _capi.lib.bnb_trunk_step(*head, _capi.ptr(reset_u8), batch, *tail)
-            else:
-                st = _capi.lib.bnb_trunk_sequence(*head, _capi.ptr(done_u8), batch, T, *tail)
-            return st, y, bul.is_bf16
-
-        st, y, used_bul16 = run(io16, bul16)
-        if st == _capi.ERR_UNSUPPORTED_DIMS and (io16 or used_bul16):
-            # the call fell to the float32-reading kernels (a shape the tensor-core kernels do not serve,
-            # e.g. more bullet slots than their attention stages; nothing was launched): once more with
-            # float32 copies of the tokens and the bullet tokens
-            st, y, _ = run(False, False)
-    _capi.check(fn, st)
-    _capi.note_engine_choice(fn)
-    _debug_check(fn, dev, precision)
-    if x.dtype == torch.bfloat16 and y.dtype != torch.bfloat16:
-        y = y.to(torch.bfloat16)   # the same contract on the paths that compute from a float32 copy
-    return y, hout
+        _capi.note_engine_choice(fn)
+        _debug_check(fn, x.device, geom[G_PRECISION])
+    return out
 
 
 @trunk_forward.register_fake

@@ -205,31 +205,34 @@ def run_trunk(
     (T * n_envs, NB) feed the spatial sublayers that read them.  Returns (y, new_hidden).
 
     Everything below the parameter gathering happens inside the opaque operator
-    ``bnb_b200::trunk_forward``, so ``torch.compile`` records one node for the whole trunk.
+    ``bnb_b200::trunk_forward``, so ``torch.compile`` records one node for the whole trunk; an eager
+    call without gradients takes the operator's body directly.
     """
     n_blocks = len(blocks)
     n_spatial = len(blocks[0].spatial) if n_blocks else 0
     n_temporal = len(blocks[0].temporal) if n_blocks else 0
     n_cross = sum(1 for sp in blocks[0].spatial if sp.reads_bullets) if n_blocks else 0
     has_fields = batch_geom[4] > batch_geom[5]          # total_tokens > total_ships
-    weights: list[torch.Tensor] = []
-    for blk in blocks:
-        for sp in blk.spatial:
-            weights += spatial_tensors(sp)
-        for j, tp in enumerate(blk.temporal):
-            weights += temporal_tensors(tp, blk.field_sub[j] if has_fields else None)
+    tracing = torch.compiler.is_compiling() or type(x) is not torch.Tensor
+    weights = None if tracing else _capi.host.trunk_params(blocks, has_fields)
+    if weights is None:
+        weights = []
+        for blk in blocks:
+            for sp in blk.spatial:
+                weights += spatial_tensors(sp)
+            for j, tp in enumerate(blk.temporal):
+                weights += temporal_tensors(tp, blk.field_sub[j] if has_fields else None)
     geom = [n_blocks, n_spatial, n_temporal, n_heads, n_cross, 1 if has_fields else 0, *batch_geom,
             0 if timesteps is None else timesteps, engine, _capi.current_precision(x.device)]
-    if (torch.is_grad_enabled() and not offsets and reset_env is None
-            and (x.requires_grad or hidden.requires_grad or (bullets is not None and bullets.requires_grad)
-                 or any(w.requires_grad for w in weights))
-            and _keep(x, geom, bullets.shape[1] if n_cross and bullets is not None else 0)):
+    grad = torch.is_grad_enabled() and (x.requires_grad or hidden.requires_grad or (bullets is not None and bullets.requires_grad)
+                                        or any(w.requires_grad for w in weights))
+    bullets, bullet_mask = (bullets, bullet_mask) if n_cross else (None, None)
+    if grad and not offsets and reset_env is None and _keep(x, geom, 0 if bullets is None else bullets.shape[1]):
         # a call that will be differentiated: the forward that keeps its activations for the backward
-        y, nh, _ = _ops.trunk_forward_train(x, alive, hidden, done, bullets if n_cross else None,
-                                            bullet_mask if n_cross else None, weights, geom)
+        y, nh, _ = _ops.trunk_forward_train(x, alive, hidden, done, bullets, bullet_mask, weights, geom)
         return y, nh
-    return _ops.trunk_forward(x, alive, hidden, done, reset_env, bullets if n_cross else None,
-                              bullet_mask if n_cross else None, weights, offsets or [], geom)
+    run = _ops.trunk_forward if grad or tracing else _ops.trunk_call
+    return run(x, alive, hidden, done, reset_env, bullets, bullet_mask, weights, offsets or [], geom)
 
 
 class YemongBlock(nn.Module):

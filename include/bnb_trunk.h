@@ -56,11 +56,11 @@ typedef enum {
 /* The status word.  Every wait inside the tensor-core kernels is bounded.  A wait that runs out
  * writes one of the BNB_STATUS_WAIT_* codes into the first 4 bytes of the call's scratch buffer
  * (an int at byte offset 0; each call zeroes it first), the kernel drains and returns, and the
- * call's outputs are then unspecified.  The entry point has returned BNB_OK long before, so every
- * BNB_BF16 call also copies the word to a pinned host word of its device, asynchronously on its
- * stream; bnb_last_status() reports the first non-zero code seen there since the last
- * bnb_clear_status().  The first BNB_BF16 call on a device allocates the host word and should
- * come before any stream capture (a call that finds itself capturing without it skips the copy). */
+ * call's outputs are then unspecified.  The entry point has returned BNB_OK long before, so the wait
+ * that runs out also writes the code to a pinned host word of its device; bnb_last_status() reports
+ * the first non-zero code seen there since the last bnb_clear_status().  The first BNB_BF16 call on a
+ * device allocates the host word and should come before any stream capture (a launch captured
+ * without it reports to its scratch buffer only). */
 int bnb_last_status(void);
 void bnb_clear_status(void);
 
