@@ -17,6 +17,9 @@
 
 #include "bnb_trunk.h"
 #include "host_calls.h"
+#include "mlp_kernels.h"
+#include "policy_tail.h"
+#include "tensor_kernels.h"
 
 namespace py = pybind11;
 using at::Tensor;
@@ -335,9 +338,170 @@ std::tuple<Tensor, Tensor> trunk_forward(const Tensor& x, const OptTensor& alive
   return {y, hout};
 }
 
+// ------------------------------------------------------------------ the ends of the policy step
+
+int pad32(int64_t n) { return (int)((n + 31) / 32 * 32); }
+
+// The first Linear's input rows and one chain's parameters, where the tiled kernel serves the widths.
+bool chain_supported(int64_t in_dim, int64_t hidden, int64_t out_dim) {
+  return in_dim <= 128 && hidden <= 256 && out_dim <= 128 && bnb::mlp::supported(pad32(in_dim), (int)hidden, pad32(out_dim));
+}
+bnb::mlp::MlpChain chain_of(const std::vector<Tensor>& ps, const c10::Device& dev, const char* what, void* y, int out, int y_ld) {
+  bnb::mlp::MlpChain c{};
+  c.w1 = parameter(ps[0], dev, what);
+  c.b1 = parameter(ps[1], dev, what);
+  c.g1 = parameter(ps[2], dev, what);
+  c.w2 = parameter(ps[3], dev, what);
+  c.b2 = parameter(ps[4], dev, what);
+  c.g2 = ps.size() > 5 ? parameter(ps[5], dev, what) : nullptr;
+  if ((reinterpret_cast<uintptr_t>(c.w1) & 15) || (reinterpret_cast<uintptr_t>(c.w2) & 15))
+    throw std::runtime_error(std::string(what) + " parameter is not 16-byte aligned");
+  c.y = static_cast<__nv_bfloat16*>(y);
+  c.out_store = out;
+  c.y_ld = y_ld;
+  return c;
+}
+
+// bnb_b200::mlp_chain (yemong/_end_ops.py): params = w1, b1, g1, w2, b2[, g2].  active (rows,): only
+// those rows are computed, the others are left unwritten.
+Tensor mlp_chain(const Tensor& x, const std::vector<Tensor>& params, int precision, const OptTensor& active) {
+  const c10::Device dev = x.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const bool bf16 = precision == BNB_BF16, encoder = params.size() > 5;
+  const char* what = encoder ? "encoder" : "head";
+  const int64_t in_dim = params[0].size(1), hidden = params[0].size(0), out_dim = params[3].size(0);
+  const auto stream = at::cuda::getCurrentCUDAStream(dev.index()).stream();
+  Tensor y = at::empty({x.size(0), out_dim}, x.options().dtype(bf16 ? at::kBFloat16 : at::kFloat));
+  if (bf16 && chain_supported(in_dim, hidden, out_dim)) {
+    // a head fed bfloat16 tokens reads them as they are
+    const bool x16 = x.scalar_type() == at::kBFloat16 && in_dim % 32 == 0;
+    Tensor rows = x16 ? contiguous(x) : f32c(x);
+    if (x16 && (reinterpret_cast<uintptr_t>(rows.data_ptr()) & 15)) rows = rows.clone();
+    const OptTensor on = bytes_of(active);
+    bnb::mlp::MlpCall call{};
+    call.x = rows.data_ptr();
+    call.x_bf16 = x16 ? 1 : 0;
+    call.n_rows = (int)rows.size(0);
+    call.in_dim = call.w1_ld = (int)in_dim;
+    call.active = static_cast<const uint8_t*>(ptr(on));
+    call.chain[0] = chain_of(params, dev, what, y.data_ptr(), (int)out_dim, (int)out_dim);
+    check(encoder ? "bnb_encoder_mlp_fwd" : "bnb_head_mlp_fwd", bnb::mlp::run(call, 1, pad32(in_dim), (int)hidden, pad32(out_dim), stream));
+    return y;
+  }
+  // the CUDA-core kernels take weights padded with zeros to multiples of 32
+  const Tensor rows = f32c(x);
+  const int n = (int)rows.size(0);
+  const float *b1 = parameter(params[1], dev, what), *g1 = parameter(params[2], dev, what);
+  if (encoder) {
+    const int in_pad = pad32(in_dim);
+    const Tensor w1 = in_pad == in_dim ? params[0] : at::constant_pad_nd(params[0].detach(), {0, in_pad - in_dim});
+    check("bnb_encoder_mlp_fwd",
+          bnb_encoder_mlp_fwd(parameter(w1, dev, what), b1, g1, parameter(params[3], dev, what), parameter(params[4], dev, what),
+                              parameter(params[5], dev, what), (int)in_dim, in_pad, (int)hidden, (int)out_dim,
+                              static_cast<const float*>(rows.data_ptr()), y.data_ptr(), n, precision, stream));
+  } else {
+    const int out_pad = pad32(out_dim);
+    const Tensor w2 = at::constant_pad_nd(params[3].detach(), {0, 0, 0, out_pad - out_dim});
+    const Tensor b2 = at::constant_pad_nd(params[4].detach(), {0, out_pad - out_dim});
+    check("bnb_head_mlp_fwd",
+          bnb_head_mlp_fwd(parameter(params[0], dev, what), b1, g1, parameter(w2, dev, what), parameter(b2, dev, what), (int)in_dim,
+                           (int)hidden, (int)out_dim, out_pad, static_cast<const float*>(rows.data_ptr()), y.data_ptr(), n, precision,
+                           stream));
+  }
+  return y;
+}
+
+// Whether policy_tail below serves a step of these sizes.
+bool tail_supported(int64_t d_model, int64_t n_heads, int64_t ships, const std::vector<int64_t>& head_widths) {
+  if (d_model != 128 || n_heads != 4 || ships < 1 || ships > bnb::tail::MAX_SHIPS) return false;
+  for (int64_t w : head_widths) if (w < 1 || w > 32) return false;
+  return !head_widths.empty() && head_widths[0] == 12 && chain_supported(d_model, 2 * d_model, 32);
+}
+
+// Whether a bfloat16 trunk call with these environments reads the tokens of active bullet slots only
+// (the tensor-core kernels compact them; the exact kernels multiply masked values by zero).
+bool bullets_compacted(int64_t d_model, int64_t n_heads, int64_t tokens, int64_t slots) {
+  BnbBatch b{};
+  b.n_envs = 1;
+  b.tokens_per_env = b.max_tokens_per_env = b.total_tokens = (int)tokens;
+  return slots > 0 && bnb::tensor::supported_batch((int)d_model, (int)n_heads, b) && bnb::tensor::supported_bullets(b, (int)slots);
+}
+
+// bnb_b200::policy_tail (yemong/_end_ops.py): everything of the rollout step behind the trunk.  x
+// (B, N+M, 128) bfloat16, heads = five parameters each of the action, next-state and value head [and the
+// win head], pma = seeds, in_proj, out_proj, norm (empty: no team value), win_cols the value columns the
+// win head fills.
+std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const Tensor& alive_in, const Tensor& team_in,
+                                                       const Tensor& uniforms, const std::vector<Tensor>& heads,
+                                                       const std::vector<Tensor>& pma, const std::vector<int64_t>& win_cols, int64_t N) {
+  const c10::Device dev = x_in.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const auto stream = at::cuda::getCurrentCUDAStream(dev.index()).stream();
+  const Tensor x = contiguous(x_in);
+  const Tensor alive = *bytes_of(alive_in);
+  Tensor team = team_in;
+  if (team.scalar_type() != at::kLong && team.scalar_type() != at::kInt) team = team.to(at::kInt);
+  if (team.size(1) > 0 && team.stride(1) != 1) team = team.contiguous();
+  const int64_t B = x.size(0), NM = x.size(1), D = x.size(2);
+  bnb::tail::Ships s{};
+  s.x = static_cast<const __nv_bfloat16*>(x.data_ptr());
+  s.alive = static_cast<const uint8_t*>(alive.data_ptr());
+  s.team_id = team.data_ptr();
+  s.team_is_64 = team.scalar_type() == at::kLong ? 1 : 0;
+  s.team_ld = (int)team.stride(0);
+  s.n_envs = (int)B;
+  s.ships = (int)N;
+  s.tokens = (int)NM;
+
+  const auto bf = x.options();
+  const int64_t K = heads[13].size(0), P = heads[8].size(0), W = pma.empty() ? 0 : (int64_t)win_cols.size();
+  Tensor logits = at::empty({B, N, 12}, bf), pred = at::empty({B, N, P}, bf), value = at::empty({B, N, K}, bf);
+  Tensor action = at::empty({B, N, 3}, bf.dtype(at::kLong)), logprob = at::empty({B, N}, bf);
+
+  auto five = [&](int i) { return std::vector<Tensor>(heads.begin() + 5 * i, heads.begin() + 5 * i + 5); };
+  bnb::mlp::MlpCall call{};
+  call.x = x.data_ptr();
+  call.x_bf16 = 1;
+  call.n_rows = (int)(B * N);
+  call.in_dim = call.w1_ld = (int)D;
+  call.group_rows = (int)N;
+  call.group_stride = (int)NM;
+  call.chain[0] = chain_of(five(0), dev, "head", logits.data_ptr(), 12, 12);
+  call.chain[1] = chain_of(five(1), dev, "head", pred.data_ptr(), (int)P, (int)P);
+  call.chain[2] = chain_of(five(2), dev, "head", value.data_ptr(), (int)K, (int)K);
+  check("bnb_head_mlp_fwd", bnb::mlp::run(call, 3, (int)D, (int)(2 * D), 32, stream));
+
+  Tensor win, rows, fold;
+  std::vector<uint8_t> cols(win_cols.begin(), win_cols.end());
+  if (W > 0) {
+    rows = at::empty({B * 2, D}, bf);
+    win = at::empty({B * 2, W}, bf);
+    fold = at::empty({(int64_t)bnb::tail::scratch_bytes()}, bf.dtype(at::kByte));
+    check("bnb_team_pma_fwd", bnb::tail::team_rows(s, parameter(pma[0], dev, "TeamPMA"), parameter(pma[1], dev, "TeamPMA"),
+                                                   parameter(pma[2], dev, "TeamPMA"), parameter(pma[3], dev, "TeamPMA"), fold.data_ptr(),
+                                                   static_cast<__nv_bfloat16*>(rows.data_ptr()), stream));
+    bnb::mlp::MlpCall wc{};
+    wc.x = rows.data_ptr();
+    wc.x_bf16 = 1;
+    wc.n_rows = (int)(B * 2);
+    wc.in_dim = wc.w1_ld = (int)D;
+    wc.chain[0] = chain_of(five(3), dev, "head", win.data_ptr(), (int)W, (int)W);
+    check("bnb_head_mlp_fwd", bnb::mlp::run(wc, 1, (int)D, (int)(2 * D), 32, stream));
+  }
+  check("bnb_action_dist_fwd", bnb::tail::finish(s, static_cast<const __nv_bfloat16*>(logits.data_ptr()), static_cast<const float*>(uniforms.data_ptr()),
+                                                 static_cast<int64_t*>(action.data_ptr()), static_cast<__nv_bfloat16*>(logprob.data_ptr()),
+                                                 W > 0 ? static_cast<const __nv_bfloat16*>(win.data_ptr()) : nullptr, (int)W, cols.data(),
+                                                 static_cast<__nv_bfloat16*>(value.data_ptr()), (int)K, stream));
+  return {action, logprob, value, pred};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_host_path, m) {
   m.def("trunk_params", &trunk_params);
+  m.def("mlp_chain", &mlp_chain);
+  m.def("policy_tail", &policy_tail);
+  m.def("tail_supported", &tail_supported);
+  m.def("bullets_compacted", &bullets_compacted);
   m.def("trunk_forward", &trunk_forward);
 }

@@ -40,6 +40,7 @@ constexpr int SLICE = 16;      // rows per warp slice (one mma.sync row block)
 // Warps per CTA: 16 where the output accumulators take 64 registers (out_dim 128), 28 where they
 // take 16 (out_dim 32: the heads, whose 65 536 rows are then one 16-row slice per warp of the grid).
 __host__ __device__ constexpr int max_warps(int out_dim) { return out_dim <= 32 ? 28 : 16; }
+constexpr int WINDOW = 128;    // slots a warp compacts at a time when only some rows are wanted (MlpCall::active)
 constexpr int PAD = 8;         // bf16 elements of padding per staged row: ldmatrix stays conflict-free
 constexpr size_t SMEM_MAX = 227 * 1024;
 
@@ -57,7 +58,7 @@ __host__ __device__ inline Layout layout(int in_pad, int hidden, int out_dim) {
   l.w2 = off; off += (size_t)out_dim * l.ldw * 2;
   l.vec = off; off += (size_t)(2 * hidden + 2 * out_dim) * 4;   // b1, g1, b2, g2
   l.slices = off;
-  l.per_warp = (size_t)SLICE * l.ldx * 2;                        // a warp's staged input rows
+  l.per_warp = (size_t)SLICE * l.ldx * 2 + 2 * WINDOW;           // a warp's staged input rows, its list of live slots
   const size_t room = SMEM_MAX > off ? SMEM_MAX - off : 0;
   int w = (int)(room / l.per_warp);
   w = w > max_warps(out_dim) ? max_warps(out_dim) : w & ~1;
@@ -93,12 +94,16 @@ __device__ __forceinline__ void linear1_chunk(float (&acc)[8][4], uint32_t sX, u
 // NCH: 64-column chunks of the hidden layer (hidden = 64 NCH).  Both are compile-time so that every
 // loop over fragments unrolls without guards; so is IN16, the 16-wide k steps of the first product
 // (in_pad = 16 IN16).
+// blockIdx.y: the chain of the call (the heads of a policy share one launch and one input).
 template <int NP2, int NCH, int IN16>
-__global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1)
-k_mlp_bf16(const float* __restrict__ x, int x_bf16, __nv_bfloat16* __restrict__ y, int n_rows, int in_dim, int in_pad, int hidden,
-           int out_dim, int out_store, const float* __restrict__ w1, const float* __restrict__ b1,
-           const float* __restrict__ g1, const float* __restrict__ w2, const float* __restrict__ b2,
-           const float* __restrict__ g2) {
+__global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const __grid_constant__ MlpCall call) {
+  constexpr int in_pad = 16 * IN16, hidden = 64 * NCH, out_dim = 16 * NP2;
+  const MlpChain& chain = call.chain[blockIdx.y];
+  const float* __restrict__ x = static_cast<const float*>(call.x);
+  const int x_bf16 = call.x_bf16, n_rows = call.n_rows, in_dim = call.in_dim, out_store = chain.out_store;
+  const float* __restrict__ w1 = chain.w1;
+  const float* __restrict__ w2 = chain.w2;
+  const float* __restrict__ g2 = chain.g2;
   extern __shared__ __align__(16) uint8_t sm[];
   const Layout L = layout(in_pad, hidden, out_dim);
   __nv_bfloat16* W1 = reinterpret_cast<__nv_bfloat16*>(sm + L.w1);
@@ -112,10 +117,25 @@ k_mlp_bf16(const float* __restrict__ x, int x_bf16, __nv_bfloat16* __restrict__ 
   const int n_threads = blockDim.x;
   const int g = lane >> 2, t = lane & 3;
 
-  // the weights, once per CTA: float32 in global memory (rows of whole 16-byte pieces on 16-byte
-  // boundaries), bfloat16 operands here; four loads in flight per thread
-  {
-    constexpr int Q1 = 4 * IN16, Q2 = 16 * NCH;   // 16-byte pieces per row of w1 (in_pad wide) and w2 (hidden wide)
+  // the weights, once per CTA: float32 in global memory, bfloat16 operands here; four loads in flight
+  // per thread.  w1 has rows of whole 16-byte pieces on 16-byte boundaries, or odd ones read element by
+  // element (columns past the raw width are zero); w2 rows past out_store are zero.
+  constexpr int Q1 = 4 * IN16, Q2 = 16 * NCH;   // 16-byte pieces per row of w1 (in_pad wide) and w2 (hidden wide)
+  if (call.w1_ld != in_pad) {
+    for (int i0 = tid; i0 < hidden * in_pad; i0 += 8 * n_threads) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int idx = i0 + j * n_threads, r = idx / in_pad, c = idx - r * in_pad;
+        v[j] = idx < hidden * in_pad && c < in_dim ? w1[r * call.w1_ld + c] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int idx = i0 + j * n_threads, r = idx / in_pad, c = idx - r * in_pad;
+        if (idx < hidden * in_pad) W1[r * ldx + c] = __float2bfloat16_rn(v[j]);
+      }
+    }
+  } else {
     const float4* s1 = reinterpret_cast<const float4*>(w1);
     for (int i0 = tid; i0 < hidden * Q1; i0 += 4 * n_threads) {
       float4 v[4];
@@ -133,13 +153,16 @@ k_mlp_bf16(const float* __restrict__ x, int x_bf16, __nv_bfloat16* __restrict__ 
         }
       }
     }
+  }
+  {
     const float4* s2 = reinterpret_cast<const float4*>(w2);
     for (int i0 = tid; i0 < out_dim * Q2; i0 += 4 * n_threads) {
       float4 v[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int idx = i0 + j * n_threads;
-        if (idx < out_dim * Q2) v[j] = s2[idx];
+        v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (idx < out_store * Q2) v[j] = s2[idx];
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -152,12 +175,12 @@ k_mlp_bf16(const float* __restrict__ x, int x_bf16, __nv_bfloat16* __restrict__ 
     }
   }
   for (int i = tid; i < hidden; i += n_threads) {
-    b1s[i] = round_bf16(b1[i]);
-    g1s[i] = g1[i];
+    b1s[i] = round_bf16(chain.b1[i]);
+    g1s[i] = chain.g1[i];
   }
   for (int i = tid; i < out_dim; i += n_threads) {
-    b2s[i] = round_bf16(b2[i]);
-    g2s[i] = g2 ? g2[i] : 1.0f;
+    b2s[i] = i < out_store ? round_bf16(chain.b2[i]) : 0.f;
+    g2s[i] = g2 && i < out_store ? g2[i] : 1.0f;
   }
   __syncthreads();   // the only CTA-wide barrier: from here on every warp works alone
 
@@ -167,75 +190,111 @@ k_mlp_bf16(const float* __restrict__ x, int x_bf16, __nv_bfloat16* __restrict__ 
   // lane % 8 + 8 (lane / 16), k half by (lane / 8) % 2
   const int a_off = (lane & 15) * ldx + (lane >> 4) * 8;
   const int b_row = (lane & 7) + (lane >> 4) * 8, b_k = ((lane >> 3) & 1) * 8;
-  const int n_slices = (n_rows + SLICE - 1) / SLICE;
   const int warps = n_threads >> 5;
   constexpr bool two_pass = NCH > 1;
-  // input rows as 16-byte pieces when rows are whole pieces on 16-byte boundaries, else element by
-  // element; idx / d for idx < 2048 and d <= 128 as a multiplication (exact: the error stays below 1 / 512)
+  // input rows as 16-byte pieces when rows are whole pieces on 16-byte boundaries, as pairs when the
+  // width is even (8-byte boundaries), else element by element
   const bool vec_in = in_dim == in_pad && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  const int q_per_row = in_pad >> 2;
-  const int recip = ((1 << 20) + (vec_in ? q_per_row : in_pad) - 1) / (vec_in ? q_per_row : in_pad);
+  const bool pair_in = (in_dim & 1) == 0 && (reinterpret_cast<uintptr_t>(x) & 7) == 0;
+  uint16_t* live = reinterpret_cast<uint16_t*>(sm + L.slices + (size_t)warp * L.per_warp + (size_t)SLICE * ldx * 2);
 
-  for (int slice = blockIdx.x * warps + warp; slice < n_slices; slice += gridDim.x * warps) {
-    const int row0 = slice * SLICE;
-    const int n_valid = min(SLICE, n_rows - row0);
-    // ---- this slice's input rows: one contiguous span of global memory.  Eight loads (four 16-byte
-    // ones) are issued before the first is used: a warp keeps that many requests in flight.
+  // A warp's unit of work: a slice of 16 rows, or with a mask the wanted rows among WINDOW slots
+  // (compacted here, so that the work goes with the rows wanted, not with the slots).
+  const int unit_rows = call.active ? WINDOW : SLICE;
+  const int n_units = (n_rows + unit_rows - 1) / unit_rows;
+  for (int unit = blockIdx.x * warps + warp; unit < n_units; unit += gridDim.x * warps) {
+    const int base = unit * unit_rows;
+    int n_live = min(SLICE, n_rows - base);
+    if (call.active) {
+      n_live = 0;
+#pragma unroll
+      for (int j = 0; j < WINDOW; j += 32) {
+        const int slot = base + j + lane;
+        const bool on = slot < n_rows && call.active[slot];
+        const uint32_t m = __ballot_sync(0xffffffffu, on);
+        if (on) live[n_live + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(j + lane);
+        n_live += __popc(m);
+      }
+      __syncwarp();
+    }
+   for (int s0 = 0; s0 < n_live; s0 += SLICE) {
+    const int n_valid = min(SLICE, n_live - s0);
+    // row of the output this lane's slice row (lane % 16) goes to, and the input row it comes from
+    int my_row = base + min(lane & (SLICE - 1), n_valid - 1);
+    if (call.active) my_row = base + live[s0 + min(lane & (SLICE - 1), n_valid - 1)];
+    const int my_src = call.group_rows ? my_row / call.group_rows * call.group_stride + my_row % call.group_rows : my_row;
+    // ---- this slice's input rows.  Eight loads (four 16-byte ones) are issued before the first is
+    // used: a warp keeps that many requests in flight.
     if (x_bf16) {   // rows already hold bfloat16 (in_dim == in_pad, a multiple of 16): 16-byte pieces, copied as they are
-      const int p_per_row = in_pad >> 3, pieces = n_valid * p_per_row;
-      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(x) + (size_t)row0 * in_dim);
+      constexpr int p_per_row = in_pad >> 3;
+      const uint4* src = static_cast<const uint4*>(call.x);
+#pragma unroll
       for (int i0 = 0; i0 < (in_pad >> 4); i0 += 4) {   // SLICE * p_per_row / 32 iterations in all
         uint4 v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int idx = lane + 32 * (i0 + j);
+          const int idx = lane + 32 * (i0 + j), r = idx / p_per_row, q = idx % p_per_row;
+          const int from = __shfl_sync(0xffffffffu, my_src, r & (SLICE - 1));
           v[j] = make_uint4(0u, 0u, 0u, 0u);
-          if (idx < pieces) v[j] = src[idx];
+          if (r < n_valid) v[j] = src[(size_t)from * p_per_row + q];
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int idx = lane + 32 * (i0 + j);
-          if (idx < SLICE * p_per_row) {
-            const int r = idx / p_per_row, q = idx - r * p_per_row;
-            *reinterpret_cast<uint4*>(X + r * ldx + q * 8) = v[j];
-          }
+          const int idx = lane + 32 * (i0 + j), r = idx / p_per_row, q = idx % p_per_row;
+          if (r < SLICE) *reinterpret_cast<uint4*>(X + r * ldx + q * 8) = v[j];
         }
       }
     } else if (vec_in) {
-      const int quads = n_valid * q_per_row;
-      const float4* src = reinterpret_cast<const float4*>(x + (size_t)row0 * in_dim);
-      for (int i0 = 0; i0 < (in_pad >> 3); i0 += 4) {   // SLICE * q_per_row / 32 iterations in all, a multiple of 4 or just 2
+      constexpr int q_per_row = in_pad >> 2;
+      const float4* src = reinterpret_cast<const float4*>(x);
+#pragma unroll 1
+      for (int i0 = 0; i0 < (in_pad >> 3); i0 += 4) {   // SLICE * q_per_row / 32 iterations in all, a multiple of 4
         float4 v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int idx = lane + 32 * (i0 + j);
+          const int idx = lane + 32 * (i0 + j), r = idx / q_per_row, q = idx % q_per_row;
+          const int from = __shfl_sync(0xffffffffu, my_src, r & (SLICE - 1));
           v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (idx < quads) v[j] = src[idx];
+          if (r < n_valid) v[j] = src[(size_t)from * q_per_row + q];
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int idx = lane + 32 * (i0 + j);
-          if (idx < SLICE * q_per_row) {
-            const int r = (idx * recip) >> 20, q = idx - r * q_per_row;
-            *reinterpret_cast<uint2*>(X + r * ldx + q * 4) = make_uint2(pack_bf16(v[j].x, v[j].y), pack_bf16(v[j].z, v[j].w));
-          }
+          const int idx = lane + 32 * (i0 + j), r = idx / q_per_row, q = idx % q_per_row;
+          if (r < SLICE) *reinterpret_cast<uint2*>(X + r * ldx + q * 4) = make_uint2(pack_bf16(v[j].x, v[j].y), pack_bf16(v[j].z, v[j].w));
+        }
+      }
+    } else if (pair_in) {
+      constexpr int h_per_row = in_pad >> 1;   // pairs
+#pragma unroll 1
+      for (int i0 = 0; i0 < (in_pad >> 2); i0 += 8) {   // SLICE * h_per_row / 32 iterations in all, a multiple of 8
+        float2 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int idx = lane + 32 * (i0 + j), r = idx / h_per_row, c = idx % h_per_row * 2;
+          const int from = __shfl_sync(0xffffffffu, my_src, r & (SLICE - 1));
+          v[j] = make_float2(0.f, 0.f);
+          if (r < n_valid && c < in_dim) v[j] = *reinterpret_cast<const float2*>(x + (size_t)from * in_dim + c);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int idx = lane + 32 * (i0 + j), r = idx / h_per_row, c = idx % h_per_row * 2;
+          *reinterpret_cast<uint32_t*>(X + r * ldx + c) = pack_bf16(v[j].x, v[j].y);
         }
       }
     } else {
-      const float* src = x + (size_t)row0 * in_dim;
+#pragma unroll 1
       for (int i0 = 0; i0 < (in_pad >> 1); i0 += 8) {   // SLICE * in_pad / 32 iterations in all, a multiple of 8
         float v[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const int idx = lane + 32 * (i0 + j);
-          const int r = (idx * recip) >> 20, c = idx - r * in_pad;
+          const int idx = lane + 32 * (i0 + j), r = idx / in_pad, c = idx % in_pad;
+          const int from = __shfl_sync(0xffffffffu, my_src, r & (SLICE - 1));
           v[j] = 0.f;
-          if (r < n_valid && c < in_dim) v[j] = src[r * in_dim + c];
+          if (r < n_valid && c < in_dim) v[j] = x[(size_t)from * in_dim + c];
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const int idx = lane + 32 * (i0 + j);
-          const int r = (idx * recip) >> 20, c = idx - r * in_pad;
+          const int idx = lane + 32 * (i0 + j), r = idx / in_pad, c = idx % in_pad;
           X[r * ldx + c] = __float2bfloat16_rn(v[j]);
         }
       }
@@ -338,35 +397,35 @@ k_mlp_bf16(const float* __restrict__ x, int x_bf16, __nv_bfloat16* __restrict__ 
       o0 = rsqrtf(ss0 / (float)out_dim + kRmsEps);
       o1 = rsqrtf(ss1 / (float)out_dim + kRmsEps);
     }
-    __nv_bfloat16* y0 = y + (size_t)(row0 + g) * out_store;
-    __nv_bfloat16* y1 = y + (size_t)(row0 + g + 8) * out_store;
-    const bool pair_store = (out_store & 1) == 0;   // columns 2t, 2t+1 of a row share an aligned 4-byte word
+    const int row_a = __shfl_sync(0xffffffffu, my_row, g), row_b = __shfl_sync(0xffffffffu, my_row, g + 8);
+    __nv_bfloat16* y0 = chain.y + (size_t)row_a * chain.y_ld;
+    __nv_bfloat16* y1 = chain.y + (size_t)row_b * chain.y_ld;
+    const bool pair_store = ((out_store | chain.y_ld) & 1) == 0;   // columns 2t, 2t+1 of a row share an aligned 4-byte word
 #pragma unroll
     for (int nt = 0; nt < 2 * NP2; ++nt) {
-      {
-        const int c = nt * 8 + 2 * t;
-        if (c < out_store) {
-          const float2 s = *reinterpret_cast<const float2*>(g2s + c);
-          const uint32_t v0 = pack_bf16(acc2[nt][0] * o0 * s.x, acc2[nt][1] * o0 * s.y);
-          const uint32_t v1 = pack_bf16(acc2[nt][2] * o1 * s.x, acc2[nt][3] * o1 * s.y);
-          if (pair_store) {
-            if (g < n_valid) *reinterpret_cast<uint32_t*>(y0 + c) = v0;
-            if (g + 8 < n_valid) *reinterpret_cast<uint32_t*>(y1 + c) = v1;
-          } else {
-            const __nv_bfloat162 p0 = *reinterpret_cast<const __nv_bfloat162*>(&v0), p1 = *reinterpret_cast<const __nv_bfloat162*>(&v1);
-            if (g < n_valid) {
-              y0[c] = p0.x;
-              if (c + 1 < out_store) y0[c + 1] = p0.y;
-            }
-            if (g + 8 < n_valid) {
-              y1[c] = p1.x;
-              if (c + 1 < out_store) y1[c + 1] = p1.y;
-            }
+      const int c = nt * 8 + 2 * t;
+      if (c < out_store) {
+        const float2 s = *reinterpret_cast<const float2*>(g2s + c);
+        const uint32_t v0 = pack_bf16(acc2[nt][0] * o0 * s.x, acc2[nt][1] * o0 * s.y);
+        const uint32_t v1 = pack_bf16(acc2[nt][2] * o1 * s.x, acc2[nt][3] * o1 * s.y);
+        if (pair_store) {
+          if (g < n_valid) *reinterpret_cast<uint32_t*>(y0 + c) = v0;
+          if (g + 8 < n_valid) *reinterpret_cast<uint32_t*>(y1 + c) = v1;
+        } else {
+          const __nv_bfloat162 p0 = *reinterpret_cast<const __nv_bfloat162*>(&v0), p1 = *reinterpret_cast<const __nv_bfloat162*>(&v1);
+          if (g < n_valid) {
+            y0[c] = p0.x;
+            if (c + 1 < out_store) y0[c + 1] = p0.y;
+          }
+          if (g + 8 < n_valid) {
+            y1[c] = p1.x;
+            if (c + 1 < out_store) y1[c + 1] = p1.y;
           }
         }
       }
     }
     __syncwarp();   // every lane is done with the staged input rows before the next slice overwrites them
+   }
   }
 }
 
@@ -379,16 +438,14 @@ bool supported(int in_pad, int hidden, int out_dim) {
   return layout(in_pad, hidden, out_dim).warps >= 4;
 }
 
-int encoder_mlp_bf16(const float* w1, const float* b1, const float* g1, const float* w2, const float* b2, const float* g2,
-                     int in_dim, int in_pad, int hidden, int out_dim, int out_store, const void* x, bool x_bf16, void* y,
-                     int n_rows, cudaStream_t st) {
-  if (!supported(in_pad, hidden, out_dim)) return BNB_ERR_UNSUPPORTED_DIMS;
-  if (x_bf16 && (in_dim != in_pad || (reinterpret_cast<uintptr_t>(x) & 15))) return BNB_ERR_UNSUPPORTED_DIMS;
-  if (n_rows <= 0) return BNB_OK;
-  if (reinterpret_cast<uintptr_t>(y) & 3) return BNB_ERR_MISALIGNED;
+int run(const MlpCall& call, int n_chains, int in_pad, int hidden, int out_dim, cudaStream_t st) {
+  if (!supported(in_pad, hidden, out_dim) || n_chains < 1 || n_chains > MAX_CHAINS) return BNB_ERR_UNSUPPORTED_DIMS;
+  if (call.x_bf16 && (call.in_dim != in_pad || (reinterpret_cast<uintptr_t>(call.x) & 15))) return BNB_ERR_UNSUPPORTED_DIMS;
+  if (call.n_rows <= 0) return BNB_OK;
+  for (int i = 0; i < n_chains; ++i)
+    if (reinterpret_cast<uintptr_t>(call.chain[i].y) & 3) return BNB_ERR_MISALIGNED;
   const Layout L = layout(in_pad, hidden, out_dim);
-  using Kernel = void (*)(const float*, int, __nv_bfloat16*, int, int, int, int, int, int, const float*, const float*, const float*,
-                          const float*, const float*, const float*);
+  using Kernel = void (*)(MlpCall);
 #define BNB_MLP_ROW(NP2, NCH) {k_mlp_bf16<NP2, NCH, 2>, k_mlp_bf16<NP2, NCH, 4>, k_mlp_bf16<NP2, NCH, 6>, k_mlp_bf16<NP2, NCH, 8>}
   static const Kernel table[2][3][4] = {{BNB_MLP_ROW(2, 1), BNB_MLP_ROW(2, 2), BNB_MLP_ROW(2, 4)},
                                         {BNB_MLP_ROW(8, 1), BNB_MLP_ROW(8, 2), BNB_MLP_ROW(8, 4)}};
@@ -398,13 +455,27 @@ int encoder_mlp_bf16(const float* w1, const float* b1, const float* g1, const fl
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return BNB_ERR_NO_DEVICE;
-  const int n_slices = (n_rows + SLICE - 1) / SLICE;
-  const int want = (n_slices + L.warps - 1) / L.warps;
-  const int grid = want < sms ? want : sms;
+  const int unit = call.active ? WINDOW : SLICE;
+  const int n_units = (call.n_rows + unit - 1) / unit;
+  const int want = (n_units + L.warps - 1) / L.warps;
+  // a CTA fills an SM and stages its weights once: the chains of a call share the SMs out
+  const int per_chain = (sms + n_chains - 1) / n_chains;
   count_launch();
-  kernel<<<grid, 32 * L.warps, L.total, st>>>(static_cast<const float*>(x), x_bf16 ? 1 : 0, static_cast<__nv_bfloat16*>(y), n_rows, in_dim, in_pad, hidden, out_dim, out_store,
-                                              w1, b1, g1, w2, b2, g2);
+  kernel<<<dim3(want < per_chain ? want : per_chain, n_chains), 32 * L.warps, L.total, st>>>(call);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+}
+
+int encoder_mlp_bf16(const float* w1, const float* b1, const float* g1, const float* w2, const float* b2, const float* g2,
+                     int in_dim, int in_pad, int hidden, int out_dim, int out_store, const void* x, bool x_bf16, void* y,
+                     int n_rows, cudaStream_t st) {
+  MlpCall call{};
+  call.x = x;
+  call.x_bf16 = x_bf16 ? 1 : 0;
+  call.n_rows = n_rows;
+  call.in_dim = in_dim;
+  call.w1_ld = in_pad;
+  call.chain[0] = MlpChain{w1, b1, g1, w2, b2, g2, static_cast<__nv_bfloat16*>(y), out_store, out_store};
+  return run(call, 1, in_pad, hidden, out_dim, st);
 }
 
 }  // namespace mlp

@@ -10,7 +10,7 @@ All of them are forward-only.
 
 from __future__ import annotations
 
-from typing import Optional, Tuple
+from typing import List, Optional, Tuple
 
 import torch
 from torch import Tensor
@@ -30,48 +30,46 @@ def _check_params(dev: torch.device, what: str, *ps: Optional[Tensor]) -> None:
 
 @torch.library.custom_op("bnb_b200::mlp_chain", mutates_args=(), device_types="cuda")
 def mlp_chain(x: Tensor, w1: Tensor, b1: Tensor, g1: Tensor, w2: Tensor, b2: Tensor, g2: Optional[Tensor],
-              precision: int) -> Tensor:
+              precision: int, active: Optional[Tensor] = None) -> Tensor:
     """Linear(w1, b1) -> RMSNorm(g1) -> GELU -> Linear(w2, b2) [-> RMSNorm(g2)] over the rows of
-    x (rows, in): ``bnb_encoder_mlp_fwd`` with g2 (the encoders), ``bnb_head_mlp_fwd`` without (the
-    heads).  Returns (rows, out), bfloat16 under the bfloat16 contract, else float32.  The weights
-    are zero-padded to the kernels' multiples of 32 here, from the live parameters, on every call."""
-    dev = x.device
-    in_dim, hidden, out_dim = w1.shape[1], w1.shape[0], w2.shape[0]
-    with torch.cuda.device(dev):
-        # a head fed bfloat16 tokens under the bfloat16 contract reads them as they are
-        x16 = g2 is None and precision == _capi.BNB_BF16 and x.dtype == torch.bfloat16 and in_dim % 32 == 0
-        flat = (x if x.is_contiguous() else x.contiguous()) if x16 else _capi.f32c(x)
-        rows = flat.shape[0]
-        y = torch.empty(rows, out_dim, device=dev, dtype=_out_dtype(precision))
-        if g2 is not None:
-            in_pad = (in_dim + 31) // 32 * 32
-            w1p = w1.detach()
-            if in_pad != in_dim:
-                w1p = torch.nn.functional.pad(w1p, (0, in_pad - in_dim))
-            w1p = w1p.contiguous()
-            _check_params(dev, "encoder", w1p, b1, g1, w2, b2, g2)
-            st = _capi.lib.bnb_encoder_mlp_fwd(w1p.data_ptr(), b1.data_ptr(), g1.data_ptr(), w2.data_ptr(), b2.data_ptr(),
-                                               g2.data_ptr(), in_dim, in_pad, hidden, out_dim, flat.data_ptr(), y.data_ptr(),
-                                               rows, precision, _capi.stream_handle(dev))
-            _capi.check("bnb_encoder_mlp_fwd", st)
-        else:
-            out_pad = (out_dim + 31) // 32 * 32
-            w2p = torch.nn.functional.pad(w2.detach(), (0, 0, 0, out_pad - out_dim)).contiguous()
-            b2p = torch.nn.functional.pad(b2.detach(), (0, out_pad - out_dim)).contiguous()
-            _check_params(dev, "head", w1, b1, g1, w2p, b2p)
-            args = (w1.data_ptr(), b1.data_ptr(), g1.data_ptr(), w2p.data_ptr(), b2p.data_ptr(), in_dim, hidden, out_dim, out_pad)
-            st = _capi.lib.bnb_head_mlp_fwd(*args, flat.data_ptr(), y.data_ptr(), rows, _capi.BNB_BF16_IO if x16 else precision,
-                                            _capi.stream_handle(dev))
-            if st == _capi.ERR_UNSUPPORTED_DIMS and x16:   # widths the tiled kernel does not serve: the float32-reading kernel
-                flat = _capi.f32c(x)
-                st = _capi.lib.bnb_head_mlp_fwd(*args, flat.data_ptr(), y.data_ptr(), rows, precision, _capi.stream_handle(dev))
-            _capi.check("bnb_head_mlp_fwd", st)
-    return y
+    x (rows, in): with g2 the encoders, without it the heads.  Returns (rows, out), bfloat16 under the
+    bfloat16 contract, else float32.  ``active`` (rows,) bool: the caller uses only these rows of the
+    result; where the tiled kernel serves the call the others are not computed and hold anything."""
+    return mlp_call(x, w1, b1, g1, w2, b2, g2, precision, active)
+
+
+def mlp_call(x, w1, b1, g1, w2, b2, g2, precision, active=None):
+    """The body of ``mlp_chain``, in native code (csrc/host_path.cpp)."""
+    return _capi.host.mlp_chain(x, [w1, b1, g1, w2, b2] if g2 is None else [w1, b1, g1, w2, b2, g2], precision, active)
 
 
 @mlp_chain.register_fake
-def _(x, w1, b1, g1, w2, b2, g2, precision):
+def _(x, w1, b1, g1, w2, b2, g2, precision, active=None):
     return x.new_empty((x.shape[0], w2.shape[0]), dtype=_out_dtype(precision))
+
+
+def direct(t: Tensor) -> bool:
+    """Whether an operator's body may be called as it is: an ordinary eager tensor, no tracer."""
+    return type(t) is Tensor and not torch.compiler.is_compiling()
+
+
+@torch.library.custom_op("bnb_b200::policy_tail", mutates_args=(), device_types="cuda")
+def policy_tail(x: Tensor, alive: Tensor, team_id: Tensor, uniforms: Tensor, heads: List[Tensor], pma: List[Tensor],
+                win_cols: List[int], n_ships: int) -> Tuple[Tensor, Tensor, Tensor, Tensor]:
+    """Everything of the rollout step behind the trunk under the bfloat16 contract, in six launches: the
+    heads, TeamPMA, the win head on one row per team, the action draw.  x (B, N+M, 128) bfloat16 trunk
+    output, alive and team_id (B, N+M), uniforms (B * N, 3) float32; ``heads`` five parameters each of the
+    action, next-state and value head and, with ``pma`` = [seeds, in_proj, out_proj, norm], the win head,
+    whose outputs go to the columns ``win_cols`` of the value.  Returns (action (B, N, 3) int64, logprob
+    (B, N), value (B, N, K), pred_next (B, N, P)), bfloat16 but for the action."""
+    return _capi.host.policy_tail(x, alive, team_id, uniforms, heads, pma, win_cols, n_ships)
+
+
+@policy_tail.register_fake
+def _(x, alive, team_id, uniforms, heads, pma, win_cols, n_ships):
+    B = x.shape[0]
+    return (x.new_empty((B, n_ships, 3), dtype=torch.int64), x.new_empty((B, n_ships)),
+            x.new_empty((B, n_ships, heads[13].shape[0])), x.new_empty((B, n_ships, heads[8].shape[0])))
 
 
 @torch.library.custom_op("bnb_b200::team_pma", mutates_args=(), device_types="cuda")

@@ -20,7 +20,8 @@ from .. import _capi
 from . import _end_ops
 
 
-def _encoder_chain(raw: torch.Tensor, lin1: nn.Linear, norm1: nn.RMSNorm, lin2: nn.Linear, norm2: nn.RMSNorm) -> torch.Tensor:
+def _encoder_chain(raw: torch.Tensor, lin1: nn.Linear, norm1: nn.RMSNorm, lin2: nn.Linear, norm2: nn.RMSNorm,
+                   active: torch.Tensor | None = None) -> torch.Tensor:
     """norm2(lin2(gelu(norm1(lin1(raw))))) over the last dim of ``raw`` through the C ABI
     (one opaque operator, ``bnb_b200::mlp_chain``)."""
     _capi.require_cuda(raw, "the raw feature vector")
@@ -28,8 +29,9 @@ def _encoder_chain(raw: torch.Tensor, lin1: nn.Linear, norm1: nn.RMSNorm, lin2: 
     if raw.shape[-1] != in_dim:
         raise RuntimeError(f"expected raw features of width {in_dim}, got {tuple(raw.shape)}")
     precision = _capi.current_precision(raw.device)
-    y = _end_ops.mlp_chain(raw.reshape(-1, in_dim), lin1.weight, lin1.bias, norm1.weight, lin2.weight, lin2.bias, norm2.weight,
-                           precision)
+    run = _end_ops.mlp_call if _end_ops.direct(raw) else _end_ops.mlp_chain
+    y = run(raw.reshape(-1, in_dim), lin1.weight, lin1.bias, norm1.weight, lin2.weight, lin2.bias, norm2.weight, precision,
+            None if active is None else active.reshape(-1))
     return y.reshape(*raw.shape[:-1], out_dim)
 
 
@@ -53,10 +55,11 @@ class BulletEncoder(nn.Module):
             nn.RMSNorm(model_config.d_model),
         )
 
-    def encode_raw(self, raw: torch.Tensor) -> torch.Tensor:
-        """``net`` on raw feature vectors (..., total_input_dimension) -> (..., d_model)."""
+    def encode_raw(self, raw: torch.Tensor, active: torch.Tensor | None = None) -> torch.Tensor:
+        """``net`` on raw feature vectors (..., total_input_dimension) -> (..., d_model).  ``active``
+        (...) bool: only these vectors' tokens are wanted; the others may hold anything."""
         _no_grad(raw)
-        return _encoder_chain(raw, self.net[0], self.net[1], self.net[3], self.net[4])
+        return _encoder_chain(raw, self.net[0], self.net[1], self.net[3], self.net[4], active)
 
     def forward(self, obs) -> torch.Tensor:
         """obs carrying bullet channels -> (..., N*K, d_model)."""

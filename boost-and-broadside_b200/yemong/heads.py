@@ -30,6 +30,11 @@ class HeadMLP(nn.Sequential):
             nn.Linear(2 * d_model, out_dim),
         )
 
+    def parameter_list(self) -> list[torch.Tensor]:
+        """w1, b1, g1, w2, b2."""
+        lin1, norm, lin2 = self[0], self[1], self[3]
+        return [lin1.weight, lin1.bias, norm.weight, lin2.weight, lin2.bias]
+
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """x (..., d_model) -> (..., out_dim)."""
         if torch.is_grad_enabled() and x.requires_grad:
@@ -39,8 +44,9 @@ class HeadMLP(nn.Sequential):
         in_dim, out_dim = lin1.in_features, lin2.out_features
         if x.shape[-1] != in_dim:
             raise RuntimeError(f"expected tokens of width {in_dim}, got {tuple(x.shape)}")
-        y = _end_ops.mlp_chain(x.reshape(-1, in_dim), lin1.weight, lin1.bias, norm.weight, lin2.weight, lin2.bias, None,
-                               _capi.current_precision(x.device))
+        run = _end_ops.mlp_call if _end_ops.direct(x) else _end_ops.mlp_chain
+        y = run(x.reshape(-1, in_dim), lin1.weight, lin1.bias, norm.weight, lin2.weight, lin2.bias, None,
+                _capi.current_precision(x.device))
         return y.reshape(*x.shape[:-1], out_dim)
 
 

@@ -19,12 +19,25 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from .. import _capi
+from . import _end_ops
 from .encoder import BulletEncoder, ShipEncoder
 from .griffin import YemongBlock
 from .heads import HeadMLP, NextStateHead, TeamPMA, evaluate_action, sample_action
 from .trunk import YemongTrunk
 
 TOTAL_ACTION_LOGITS = 12  # constants.py:43
+
+
+# Queries of the library about sizes: constants of a trace.
+@torch.compiler.assume_constant_result
+def _bullets_compacted(d_model: int, n_heads: int, n_tokens: int, n_slots: int) -> bool:
+    return _capi.host.bullets_compacted(d_model, n_heads, n_tokens, n_slots)
+
+
+@torch.compiler.assume_constant_result
+def _tail_supported(d_model: int, n_heads: int, n_ships: int, *head_widths: int) -> bool:
+    return _capi.host.tail_supported(d_model, n_heads, n_ships, list(head_widths))
 
 
 class YemongPolicy(YemongTrunk):
@@ -56,11 +69,30 @@ class YemongPolicy(YemongTrunk):
     def num_recurrent_tokens(self) -> int:
         return self._num_ships
 
-    def _encode_bullets(self, obs):
-        if self.bullet_encoder is None or obs.bullets is None:
+    def _encode_bullets(self, obs, n_tokens: int):
+        """Bullet tokens and their mask.  The trunk's tensor-core kernels read the tokens of active slots
+        only, so where they serve the call (environments of ``n_tokens``) the others are not encoded."""
+        enc = self.bullet_encoder
+        if enc is None or obs.bullets is None:
             return None, None
         active = next(v for k, v in obs.bullets.items() if getattr(k, "name", str(k)).upper().endswith("ACTIVE"))
-        return self.bullet_encoder(obs), active
+        raw = enc.coordinator.get_input_vector(obs)
+        compacts = (_capi.current_precision(raw.device) == _capi.BNB_BF16 and tuple(active.shape) == tuple(raw.shape[:-1])
+                    and _bullets_compacted(self.d_model, self.n_heads, n_tokens, raw.shape[-2]))
+        return enc.encode_raw(raw, active if compacts else None), active
+
+    def _tail_lists(self):
+        """Parameters of the heads and of TeamPMA as ``_end_ops.policy_tail`` takes them, or None where
+        its kernels do not serve this policy (or the call is not under the bfloat16 contract)."""
+        heads = [self.action_head, self.next_state_head.net, self.value_head_local]
+        pma: list[torch.Tensor] = []
+        if self._team_pma_k:
+            heads.append(self.value_head_win)
+            pma = [self.team_pma.seeds, self.team_pma.attn.in_proj_weight, self.team_pma.attn.out_proj.weight, self.team_pma.norm.weight]
+        lists = [h.parameter_list() for h in heads]
+        if not _tail_supported(self.d_model, self.n_heads, self._num_ships, *[ps[3].shape[0] for ps in lists]):
+            return None
+        return [p for ps in lists for p in ps], pma
 
     @torch.no_grad()
     def get_action_and_value(self, obs, hidden: torch.Tensor, generator: torch.Generator | None = None):
@@ -68,9 +100,15 @@ class YemongPolicy(YemongTrunk):
         value (B, N, K), pred_next (B, N, pred_dim), new_hidden)."""
         alive = obs["alive"]
         x = self.encoder(obs)
-        bullets, bullet_mask = self._encode_bullets(obs)
+        bullets, bullet_mask = self._encode_bullets(obs, x.shape[1])
         x, new_hidden = self.step(x, alive, hidden, bullets=bullets, bullet_mask=bullet_mask)
         N = self._num_ships
+        lists = self._tail_lists() if x.dtype == torch.bfloat16 else None
+        if lists is not None:
+            uniforms = torch.rand(x.shape[0] * N, 3, device=x.device, generator=generator)
+            run = _capi.host.policy_tail if _end_ops.direct(x) else _end_ops.policy_tail
+            action, logprob, value, pred_next = run(x, alive, obs["team_id"], uniforms, *lists, list(self._team_pma_k), N)
+            return action, logprob, value, pred_next, new_hidden
         x_ships = x[:, :N, :].contiguous()
         logits = self.action_head(x_ships)
         pred_next = self.next_state_head(x_ships)
@@ -97,7 +135,7 @@ class YemongPolicy(YemongTrunk):
         x = self.encoder(flat)
         NM, D = x.shape[1], x.shape[2]
         x = x.reshape(T, B, NM, D)
-        bullets, bullet_mask = self._encode_bullets(flat)
+        bullets, bullet_mask = self._encode_bullets(flat, NM)
         z = x if return_encoder_output else None
         x, _ = self.sequence(x, alive_mask, initial_hidden, done_mask, bullets=bullets, bullet_mask=bullet_mask)
         x_ships = x[:, :, :N, :].contiguous()

@@ -1,0 +1,98 @@
+"""The native end of a rollout step (``bnb_b200::policy_tail``: heads, team pooling, win head, action
+draw) and the encoder that skips idle bullet slots, against the same policy assembled from its modules
+(which the fixtures of the reference pin) and a plain float32 pooling.
+"""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+class _Obs(dict):
+    bullets = None
+
+
+class _Coordinator:
+    total_prediction_dimension = 10
+
+    def __init__(self, width, read):
+        self.total_input_dimension = width
+        self.get_input_vector = read
+
+
+def _policy(N, seed=0, ks=(0, 1)):
+    import boost_and_broadside_b200 as bnb
+    from boost_and_broadside_b200 import workloads
+
+    torch.manual_seed(seed)
+    p = bnb.YemongPolicy(workloads.rl_config(), _Coordinator(66, lambda o: o["raw"]), 11, N, ks,
+                         bullet_coordinator=_Coordinator(26, lambda o: o.bullets["raw"])).to(DEV).eval()
+    with torch.no_grad():
+        if ks:
+            p.team_pma.seeds.normal_(0.0, 0.5)
+    return p
+
+
+def _obs(B, N, M, NB, seed, int_type=torch.int64):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    alive = torch.rand(B, N + M, device=DEV, generator=gen) < 0.7
+    obs = _Obs(alive=alive, raw=torch.randn(B, N + M, 66, device=DEV, generator=gen),
+               team_id=torch.randint(0, 2, (B, N + M), device=DEV, generator=gen).to(int_type))
+    obs["alive"][0, :N] = False            # a team (here both) without a ship alive
+    if NB:
+        mask = torch.rand(B, NB, device=DEV, generator=gen) < 0.3
+        mask[B // 2] = False
+        obs.bullets = {"raw": torch.randn(B, NB, 26, device=DEV, generator=gen), "ACTIVE": mask}
+    hidden = torch.randn(2, B * N, 512, device=DEV, generator=gen) * 0.5
+    return obs, hidden
+
+
+def _modules_step(p, obs, hidden, generator):
+    """The same step through the modules one by one, every bullet slot encoded."""
+    from boost_and_broadside_b200 import sample_action
+
+    N = p._num_ships
+    bullets = mask = None
+    if obs.bullets is not None:
+        bullets, mask = p.bullet_encoder(obs), obs.bullets["ACTIVE"]
+    x, nh = p.step(p.encoder(obs), obs["alive"], hidden, bullets=bullets, bullet_mask=mask)
+    xs = x[:, :N].contiguous()
+    logits, pred, value = p.action_head(xs), p.next_state_head(xs), p.value_head_local(xs)
+    if p._team_pma_k:
+        win = p.value_head_win(p.team_pma(xs, obs["team_id"][:, :N], obs["alive"][:, :N]))
+        for i, k in enumerate(p._team_pma_k):
+            value[:, :, k] = win[:, :, i]
+    action, logprob = sample_action(logits, generator)
+    return action, logprob, value, pred, nh
+
+
+@pytest.mark.parametrize("B,N,M,NB,ks", [(1, 1, 0, 0, (0, 1)), (17, 8, 4, 80, (0, 1)), (150, 3, 1, 7, (4,)), (5, 152, 0, 0, (2, 0, 10)),
+                                         (40, 8, 4, 129, ()), (2500, 2, 0, 1, (0, 1))])
+def test_native_tail_matches_the_modules(B, N, M, NB, ks):
+    p = _policy(N, seed=B, ks=ks)
+    obs, hidden = _obs(B, N, M, NB, seed=B + N, int_type=torch.int64 if B % 2 else torch.int32)
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        got = p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
+        ref = _modules_step(p, obs, hidden, torch.Generator(device=DEV).manual_seed(3))
+    for name, g, r in zip(("action", "logprob", "value", "pred_next", "hidden"), got, ref):
+        assert g.shape == r.shape and g.dtype == r.dtype, name
+        if name != "value":   # the same kernels' arithmetic: the same bits
+            assert torch.equal(g, r), name
+    err = (got[2].float() - ref[2].float()).abs().max() / ref[2].float().abs().max()
+    assert float(err) <= 1e-2   # the pooled rows are projected after pooling, not before
+
+
+def test_native_tail_under_torch_compile_is_one_graph_and_matches_eager():
+    p = _policy(8, seed=5)
+    obs, hidden = _obs(16, 8, 4, 24, seed=6)
+    compiled = torch.compile(p.get_action_and_value, mode="reduce-overhead", fullgraph=True)
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        _, _, v0, p0, h0 = p.get_action_and_value(obs, hidden)
+        for _ in range(3):
+            _, _, v, pn, h = compiled(obs, hidden)
+            v, pn, h = v.clone(), pn.clone(), h.clone()
+    assert torch.equal(v, v0) and torch.equal(pn, p0) and torch.equal(h, h0)
