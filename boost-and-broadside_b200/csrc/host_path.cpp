@@ -338,6 +338,43 @@ std::tuple<Tensor, Tensor> trunk_forward(const Tensor& x, const OptTensor& alive
   return {y, hout};
 }
 
+// ------------------------------------------------------------------ ragged batches
+
+// RaggedBatch.build (yemong/trunk.py): the batch integers of a call, the device arrays [tok_off,
+// ship_off(, tile_env_begin, tile_env_ids)] and the share of tile rows in use.  Everything is laid out in
+// one pinned buffer and uploaded with one asynchronous copy: from pageable memory the copies waited for
+// the kernels of the previous step, and the planning then ran with the device idle.
+std::tuple<std::vector<int64_t>, std::vector<Tensor>, double> ragged_build(const Tensor& n_tokens, const Tensor& n_ships, const c10::Device& dev) {
+  const Tensor nt = n_tokens.to(at::kCPU, at::kLong).contiguous(), ns = n_ships.to(at::kCPU, at::kLong).contiguous();
+  if (nt.dim() != 1 || nt.sizes() != ns.sizes()) throw std::runtime_error("n_tokens and n_ships must be 1-D tensors of equal length");
+  const int64_t B = nt.numel();
+  const int64_t *t = nt.data_ptr<int64_t>(), *s = ns.data_ptr<int64_t>();
+  const c10::cuda::OptionalCUDAGuard guard(dev.is_cuda() ? c10::optional<c10::Device>(dev) : c10::nullopt);
+  const int64_t stride = (B + 1 + 3) / 4 * 4;   // 16-byte pieces
+  Tensor host = at::empty({4 * stride}, at::TensorOptions().dtype(at::kInt).pinned_memory(dev.is_cuda()));
+  int32_t* tok = host.data_ptr<int32_t>();
+  int32_t *ship = tok + stride, *tiles = tok + 2 * stride, *ids = tok + 3 * stride;
+  int64_t most = 0, least = INT64_MAX;
+  tok[0] = ship[0] = 0;
+  for (int64_t e = 0; e < B; ++e) {
+    if (s[e] > t[e] || s[e] < 0) throw std::runtime_error("each environment needs 0 <= n_ships <= n_tokens");
+    most = std::max(most, t[e]);
+    least = std::min(least, t[e]);
+    tok[e + 1] = tok[e] + (int32_t)t[e];
+    ship[e + 1] = ship[e] + (int32_t)s[e];
+  }
+  int n_tiles = 0;
+  const bool planned = B > 0 && most <= 128 && least >= 1;   // the tensor-core engine's ragged tiles
+  if (planned) check("bnb_plan_tiles", bnb_plan_tiles(tok, (int)B, tiles, ids, (int)B + 1, &n_tiles));
+  const Tensor device = host.slice(0, 0, planned ? 4 * stride : 2 * stride).to(at::TensorOptions().device(dev), /*non_blocking=*/true);
+  std::vector<Tensor> offsets{device.slice(0, 0, B + 1), device.slice(0, stride, stride + B + 1)};
+  if (planned) {
+    offsets.push_back(device.slice(0, 2 * stride, 2 * stride + n_tiles + 1));
+    offsets.push_back(device.slice(0, 3 * stride, 3 * stride + B));
+  }
+  return {{B, 0, 0, most, tok[B], ship[B], n_tiles}, offsets, n_tiles ? tok[B] / (128.0 * n_tiles) : 0.0};
+}
+
 // ------------------------------------------------------------------ the ends of the policy step
 
 int pad32(int64_t n) { return (int)((n + 31) / 32 * 32); }
@@ -499,6 +536,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const
 
 PYBIND11_MODULE(_host_path, m) {
   m.def("trunk_params", &trunk_params);
+  m.def("ragged_build", &ragged_build);
   m.def("mlp_chain", &mlp_chain);
   m.def("policy_tail", &policy_tail);
   m.def("tail_supported", &tail_supported);

@@ -1488,44 +1488,60 @@ int plan_tiles(const int32_t* tok_off, int n_envs, int32_t* tile_env_begin, int3
   // Best-fit decreasing: environments sorted by size (counting sort, sizes 1..128), each put into
   // the open tile with the least room that still takes it.  Tiles are then listed as ranges of
   // tile_env_ids.  Near-full tiles matter: a tile costs about the same whatever its fill.
+  // Flat arrays throughout (16 384 environments: about 0.1 ms; with a vector per tile and per room
+  // it was 0.7 ms of a step's host time): open tiles of one room form a stack linked through
+  // next_open, a 129-bit mask says which rooms have any, the environments of a tile a chain.
   if (capacity < n_envs + 1) return BNB_ERR_SCRATCH_TOO_SMALL;
-  std::vector<int> order;
-  order.reserve(n_envs);
-  {
-    std::vector<std::vector<int>> by_size(TILE + 1);
-    for (int e = 0; e < n_envs; ++e) {
-      const int n = tok_off[e + 1] - tok_off[e];
-      if (n <= 0 || n > TILE) return BNB_ERR_TOO_MANY_TOKENS;
-      by_size[n].push_back(e);
-    }
-    for (int n = TILE; n >= 1; --n) order.insert(order.end(), by_size[n].begin(), by_size[n].end());
-  }
-  std::vector<std::vector<int>> tiles;                   // environments of each tile
-  std::vector<std::vector<int>> open_by_room(TILE + 1);  // tiles with exactly r free rows
-  for (int e : order) {
+  int begin[TILE + 2] = {};
+  for (int e = 0; e < n_envs; ++e) {
     const int n = tok_off[e + 1] - tok_off[e];
+    if (n <= 0 || n > TILE) return BNB_ERR_TOO_MANY_TOKENS;
+    ++begin[TILE - n + 1];   // largest first
+  }
+  for (int i = 1; i <= TILE; ++i) begin[i] += begin[i - 1];
+  std::vector<int> store((size_t)n_envs * 6);
+  int* order = store.data();
+  int* next_env = order + n_envs;      // next environment of the same tile
+  int* first_env = next_env + n_envs;  // per tile
+  int* last_env = first_env + n_envs;
+  int* next_open = last_env + n_envs;
+  for (int e = 0; e < n_envs; ++e) order[begin[TILE - (tok_off[e + 1] - tok_off[e])]++] = e;
+  int open[TILE + 1];
+  for (int& o : open) o = -1;
+  uint64_t mask[3] = {0, 0, 0};
+  int tiles = 0;
+  for (int i = 0; i < n_envs; ++i) {
+    const int e = order[i], n = tok_off[e + 1] - tok_off[e];
     int room = -1;
-    for (int r = n; r <= TILE; ++r)
-      if (!open_by_room[r].empty()) { room = r; break; }
+    for (int w = n >> 6; w < 3; ++w) {
+      const uint64_t m = w == n >> 6 ? mask[w] >> (n & 63) << (n & 63) : mask[w];
+      if (m) { room = w * 64 + __builtin_ctzll(m); break; }
+    }
     int t;
     if (room < 0) {
-      t = (int)tiles.size();
-      tiles.emplace_back();
+      t = tiles++;
       room = TILE;
+      first_env[t] = e;
     } else {
-      t = open_by_room[room].back();
-      open_by_room[room].pop_back();
+      t = open[room];
+      open[room] = next_open[t];
+      if (open[room] < 0) mask[room >> 6] &= ~(1ull << (room & 63));
+      next_env[last_env[t]] = e;
     }
-    tiles[t].push_back(e);
-    open_by_room[room - n].push_back(t);
+    last_env[t] = e;
+    next_env[e] = -1;
+    const int left = room - n;
+    next_open[t] = open[left];
+    open[left] = t;
+    mask[left >> 6] |= 1ull << (left & 63);
   }
   int k = 0;
-  for (size_t t = 0; t < tiles.size(); ++t) {
+  for (int t = 0; t < tiles; ++t) {
     tile_env_begin[t] = k;
-    for (int e : tiles[t]) tile_env_ids[k++] = e;
+    for (int e = first_env[t]; e >= 0; e = next_env[e]) tile_env_ids[k++] = e;
   }
-  tile_env_begin[tiles.size()] = k;
-  *n_tiles = (int)tiles.size();
+  tile_env_begin[tiles] = k;
+  *n_tiles = tiles;
   return BNB_OK;
 }
 

@@ -37,33 +37,7 @@ class RaggedBatch:
 
     def build(self, device: torch.device) -> tuple[list[int], list[torch.Tensor]]:
         """Batch integers (the ``_ops`` geometry entries) and the device prefix sums / tile plan."""
-        nt = self.n_tokens.to("cpu", torch.int64)
-        ns = self.n_ships.to("cpu", torch.int64)
-        if nt.shape != ns.shape or nt.dim() != 1:
-            raise RuntimeError("n_tokens and n_ships must be 1-D tensors of equal length")
-        if bool((ns > nt).any()) or bool((ns < 0).any()):
-            raise RuntimeError("each environment needs 0 <= n_ships <= n_tokens")
-        B = nt.numel()
-        tok_off = torch.zeros(B + 1, dtype=torch.int32)
-        ship_off = torch.zeros(B + 1, dtype=torch.int32)
-        tok_off[1:] = nt.cumsum(0)
-        ship_off[1:] = ns.cumsum(0)
-        tok_d = tok_off.to(device)
-        ship_d = ship_off.to(device)
-        # tile plan for the tensor-core engine (environments of at most 128 tokens only)
-        tiles_d, ids_d, n_tiles = None, None, 0
-        if B and int(nt.max()) <= 128 and int(nt.min()) >= 1:
-            plan = torch.zeros(B + 1, dtype=torch.int32)
-            ids = torch.zeros(B, dtype=torch.int32)
-            n = _capi.C.c_int(0)
-            st = _capi.lib.bnb_plan_tiles(tok_off.data_ptr(), B, plan.data_ptr(), ids.data_ptr(), B + 1, _capi.C.byref(n))
-            _capi.check("bnb_plan_tiles", st)
-            n_tiles = n.value
-            tiles_d = plan[: n_tiles + 1].to(device)
-            ids_d = ids.to(device)
-        geom = [B, 0, 0, int(nt.max()) if B else 0, int(tok_off[-1]), int(ship_off[-1]), n_tiles]
-        self.tile_fill = float(tok_off[-1]) / (128.0 * n_tiles) if n_tiles else 0.0
-        offsets = [tok_d, ship_d] + ([tiles_d, ids_d] if tiles_d is not None else [])
+        geom, offsets, self.tile_fill = _capi.host.ragged_build(self.n_tokens, self.n_ships, torch.device(device))
         return geom, offsets
 
 
