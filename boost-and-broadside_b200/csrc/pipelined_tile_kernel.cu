@@ -5,12 +5,12 @@
 //   16 epilogue warps   four threads per tile row (thread (row, part): TMEM lane = row, a quarter
 //                       of whatever columns are being read).  RMSNorm, q|k|v staging, attention
 //                       (mma.sync), gelu(gate) * up, causal conv, RG-LRU gates and state update.
-//   1 issuing warp      one lane issues every tcgen05.mma.  It waits for "operand ready" (the
+//   1 issuing warp      issues every tcgen05.mma.  It waits for "operand ready" (the
 //                       epilogue warps arrive on an mbarrier after fence.proxy.async) and for
 //                       "chunk landed" (the bulk copy's complete_tx), and signals "accumulator
 //                       ready" / "slot free" with tcgen05.commit.
-//   1 fetching warp     one lane streams the pre-tiled weight image through a ring of nine
-//                       16 KB slots with cp.async.bulk, following a static schedule.
+//   1 fetching warp     streams the pre-tiled weight image through a ring of nine 16 KB
+//                       slots with cp.async.bulk, following a static schedule.
 //
 //   TMEM  [0,128)    residual stream, fp32, lane = tile row (out_proj, linear_out and down_proj
 //                    accumulate straight into it)
@@ -61,14 +61,16 @@ constexpr int OFF_BAR = OFF_BIAS + 576;
 constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
 
 // mbarrier indices
-// OP: operand ready (epilogue warps -> issuing lane).  KVREL: the key/value area may take weights
-// again (epilogue warps -> fetching lane).  FULL[s]: the weights of slot s have landed.  DONE[s]:
-// the MMAs that read slot s are complete (tcgen05.commit) -- the fetching lane takes it as "slot
-// free" and, inside the GatedMLP pipeline, the epilogue warps as "accumulator ready" / "product
-// buffer read": one commit per ring operation serves both.  ACC: every MMA of a round outside the
-// GatedMLP pipeline is complete (one more commit per round).  DRAIN: every MMA of the CTA is
-// complete (once, at the end).
-enum : int { B_OP0 = 0, B_OP1, B_KVREL, B_ACC, B_DRAIN, B_FULL0, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
+// OP0: operand ready (epilogue warps -> issuing warp).  FFN[a]: the GatedMLP product in accumulator a is
+// written (the eight warps that own the chunk -> issuing warp); the next chunk of that accumulator is
+// issued after the wait, so a phase is never overtaken.  KVREL: the key/value area
+// may take weights again (epilogue warps -> fetching warp).  FULL[s]: the weights of slot s have landed.
+// DONE[s]: the MMAs that read slot s are complete (tcgen05.commit) -- the fetching warp takes it as
+// "slot free" and the epilogue warps as "accumulator ready" for gate|up of one chunk, whose slot is not
+// used again before they have seen it.  QKV[h]: q|k|v of head h is complete (a barrier per head: a slot
+// serves two heads, and a phase waited for too late would look like the one after next).  ACC: every MMA of a round is complete (one more commit per round).  DRAIN: every MMA of the
+// CTA is complete (once, at the end).
+enum : int { B_OP0 = 0, B_FFN0, B_FFN1, B_FFN2, B_KVREL, B_ACC, B_DRAIN, B_QKV0, B_FULL0 = B_QKV0 + HEADS, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
 static_assert(B_COUNT * 8 + 8 <= 256, "barrier area");
 
 constexpr uint32_t COL_RESID = 0;
@@ -117,11 +119,14 @@ __device__ __forceinline__ void trace(Trace& t, int id) {
 #define TRACE(t, id)
 #endif
 
-// Schedule entry of one ring operation: slot (3 bits) | sublayer (3) | first chunk (6) | second
-// chunk (6; 63 = none: a single) | wait for the key/value area first (1).
+// One ring operation as the fetching warp needs it: source of the first chunk (64 bits), byte distance
+// from it to the second chunk (0: a single), and slot (bits 0-2) | wait for the key/value area first (8).
+// Resolved once at kernel start, so that a fetch is a dozen instructions.
 constexpr uint32_t NO_CHUNK = 63;
-__device__ __forceinline__ uint32_t sched_entry(int slot, int si, int ch0, int ch1, bool kvwait) {
-  return (uint32_t)slot | ((uint32_t)si << 3) | ((uint32_t)ch0 << 6) | ((uint32_t)ch1 << 12) | (kvwait ? 1u << 18 : 0u);
+__device__ __forceinline__ uint4 sched_entry(int slot, const uint8_t* image, int ch0, uint32_t ch1, bool kvwait) {
+  const unsigned long long src = reinterpret_cast<unsigned long long>(image + (size_t)ch0 * CHUNK_BYTES);
+  return make_uint4((uint32_t)src, (uint32_t)(src >> 32), ch1 == NO_CHUNK ? 0u : (ch1 - (uint32_t)ch0) * CHUNK_BYTES,
+                    (uint32_t)slot | (kvwait ? 8u : 0u));
 }
 constexpr int MAX_SCHED = MAX_SUBLAYERS * 22;
 
@@ -129,56 +134,57 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// Ring operations of a sublayer in the order the issuing lane consumes them.  GatedMLP with
-// image base b: gate|up of chunk c are chunks b + 3c, b + 3c + 1 (a pair), its down projection is
-// b + 3c + 2 (a single); the three-deep pipeline consumes GU0 GU1 GU2 D0 GU3 D1 GU4 D2 ... GU7 D5 D6 D7.
+// Ring operations of a sublayer in the order the issuing warp consumes them.  All three roles walk the
+// same order with the same slot rotation.  GatedMLP with image base b: gate|up of chunk c are chunks
+// b + 3c, b + 3c + 1 (a pair), its down projection is b + 3c + 2 (a single); the three-deep pipeline
+// consumes GU0 GU1 GU2 D0 GU3 D1 GU4 D2 ... GU7 D5 D6 D7.
 struct SlotRotation {
-  int pair, single;
-  __device__ __forceinline__ int next_pair() { const int r = pair; pair = pair == 2 ? 0 : pair + 1; return r; }
-  __device__ __forceinline__ int next_single() { const int r = single; single = single == 5 ? 3 : single + 1; return r; }
+  uint32_t pair, single;
+  __device__ __forceinline__ uint32_t next_pair() { const uint32_t r = pair; pair = pair == 2 ? 0 : pair + 1; return r; }
+  __device__ __forceinline__ uint32_t next_single() { const uint32_t r = single; single = single == 5 ? 3 : single + 1; return r; }
 };
-__device__ __forceinline__ int ffn_ops(uint32_t* out, int n, int si, int base, SlotRotation& rot, int first_flagged) {
+// q|k|v of the four heads: the one slot inside the key/value area first, because keys and values are
+// staged there as soon as a head is ready; then the dedicated slots.
+__device__ __forceinline__ uint32_t qkv_slot(uint32_t h) { return h == 0 ? 2u : h == 2 ? 0u : 1u; }
+// After them out_proj goes to pair slot 0, the first gate|up to pair slot 1 and the first down projection
+// to single slot 3 (all dedicated: fetched while the attention runs); the second gate|up is the first
+// operation that goes to the key/value area and waits for it.
+__device__ __forceinline__ void after_qkv(SlotRotation& rot) { rot.pair = 0; rot.single = 3; }
+
+__device__ __forceinline__ int ffn_ops(uint4* out, int n, const uint8_t* image, int base, SlotRotation& rot, int first_flagged) {
   // first_flagged: index (in GU order) of the first gate|up pair that must wait for the key/value area, or -1
-  for (int c = 0; c < 3; ++c) out[n++] = sched_entry(rot.next_pair(), si, base + 3 * c, base + 3 * c + 1, c == first_flagged);
+  for (int c = 0; c < 3; ++c) out[n++] = sched_entry(rot.next_pair(), image, base + 3 * c, base + 3 * c + 1, c == first_flagged);
   for (int c = 0; c < 8; ++c) {
-    out[n++] = sched_entry(rot.next_single(), si, base + 3 * c + 2, NO_CHUNK, false);
-    if (c + 3 < 8) out[n++] = sched_entry(rot.next_pair(), si, base + 3 * (c + 3), base + 3 * (c + 3) + 1, false);
+    out[n++] = sched_entry(rot.next_single(), image, base + 3 * c + 2, NO_CHUNK, false);
+    if (c + 3 < 8) out[n++] = sched_entry(rot.next_pair(), image, base + 3 * (c + 3), base + 3 * (c + 3) + 1, false);
   }
   return n;
 }
-__device__ __forceinline__ int build_schedule(const SubLayer* subs, int n_sub, bool has_fields, uint32_t* out) {
+__device__ __forceinline__ int build_schedule(const SubLayer* subs, int n_sub, bool has_fields, uint4* out) {
   int n = 0;
   SlotRotation rot{0, 3};
   for (int si = 0; si < n_sub; ++si) {
-    if (subs[si].type == SUB_SPATIAL) {
+    const uint8_t* image = subs[si].packed;
+    if (subs[si].type == SUB_SPATIAL || subs[si].type == SUB_SPATIAL_PRE) {
       for (int h = 0; h < HEADS; ++h) {
         const int ch = 5 * (h >> 1) + 2 * (h & 1);
-        out[n++] = sched_entry(rot.next_pair(), si, ch, ch + 1, false);
+        out[n++] = sched_entry(qkv_slot(h), image, ch, ch + 1, false);
       }
-      // fetched while the attention runs: the dedicated slots only.  out_proj -> pair slot 0, the
-      // first gate|up -> pair slot 1 and the first down projection -> single slot 3; the second
-      // gate|up is the first operation that goes to the key/value area and waits for it.
-      out[n++] = sched_entry(0, si, 4, 9, false);
-      rot.pair = 1;
-      rot.single = 3;
-      n = ffn_ops(out, n, si, 10, rot, 1);
-    } else if (subs[si].type == SUB_SPATIAL_PRE) {
-      // q|k|v only: the attention runs in a kernel of its own between this launch and the next
-      for (int h = 0; h < HEADS; ++h) {
-        const int ch = 5 * (h >> 1) + 2 * (h & 1);
-        out[n++] = sched_entry(rot.next_pair(), si, ch, ch + 1, false);
-      }
+      after_qkv(rot);
+      if (subs[si].type == SUB_SPATIAL_PRE) continue;   // the attention runs in a kernel of its own between this launch and the next
+      out[n++] = sched_entry(rot.next_pair(), image, 4, 9, false);
+      n = ffn_ops(out, n, image, 10, rot, 1);
     } else if (subs[si].type == SUB_SPATIAL_POST) {
       // out_proj on the attention output read back from global memory, then the GatedMLP; nothing
       // of this sublayer uses the key/value area, so no operation waits for it
-      out[n++] = sched_entry(rot.next_pair(), si, 4, 9, false);
-      n = ffn_ops(out, n, si, 10, rot, -1);
+      out[n++] = sched_entry(rot.next_pair(), image, 4, 9, false);
+      n = ffn_ops(out, n, image, 10, rot, -1);
     } else {
       for (int i = 0; i < 6; ++i) {
         if (!has_fields && i == 4) continue;
-        out[n++] = sched_entry(rot.next_pair(), si, 2 * i, 2 * i + 1, false);
+        out[n++] = sched_entry(rot.next_pair(), image, 2 * i, 2 * i + 1, false);
       }
-      n = ffn_ops(out, n, si, 12, rot, -1);
+      n = ffn_ops(out, n, image, 12, rot, -1);
     }
   }
   return n;
@@ -209,9 +215,8 @@ struct Epi {
   uint32_t sbase;       // shared address of smem
   uint32_t bars;        // shared address of the barrier array
   uint32_t lane_addr;   // tensor-memory address of this thread's lane, column 0
-  uint32_t par;         // phase bits of the DONE barriers, one per ring slot
-  const uint32_t* sched;
-  int sched_len, cur;   // cursor into the schedule: the next ring operation this thread waits for
+  uint32_t par;         // phase bits of the pair slots' DONE barriers (0..2), of ACC (8) and of QKV (9)
+  SlotRotation rot;     // pair slot of the next ring operation
   int row, part;
   int* status;
   volatile int* aborted;
@@ -227,39 +232,32 @@ __device__ __forceinline__ void post(Epi& e, int bar) {
   if ((threadIdx.x & 31) == 0) mbar_arrive(e.bars + 8 * bar);
   TRACE(e.tr, 210 + bar);
 }
-// The epilogue threads walk the schedule of ring operations with a cursor of their own and keep
-// one phase bit per DONE barrier.
+// The epilogue threads keep one phase bit per pair slot and flip it for every pair operation of the
+// schedule, in order, whether they wait for it or not.
 //
-// wait_round: a round outside the GatedMLP pipeline (n operations, then a commit on ACC).  The
-// threads wait on ACC and flip the phase bits of the n operations, which are complete by then.
-__device__ __forceinline__ void wait_round(Epi& e, int n) {
+// wait_acc: every MMA issued so far is complete (a commit on ACC ends every round).
+__device__ __forceinline__ void wait_acc(Epi& e) {
   T_BEGIN();
   mbar_wait(e.bars + 8 * B_ACC, (e.par >> 8) & 1u, e.status, e.aborted, ST_TIMEOUT_ACC);
   e.par ^= 1u << 8;
-  for (int i = 0; i < n; ++i) {
-    const uint32_t slot = e.sched[e.cur] & 7u;
-    e.cur = e.cur + 1 == e.sched_len ? 0 : e.cur + 1;
-    e.par ^= 1u << slot;
-  }
   tc_fence_after();
   T_END(e.tacc, e.wait_slot);
-  TRACE(e.tr, 110 + n);
+  TRACE(e.tr, 110);
 }
-// wait_ops: inside the GatedMLP pipeline the threads wait for each operation on its own DONE
-// barrier, in schedule order.  A slot is not reused before the threads have seen its previous
-// operation complete: the reuse distance is three operations of a kind, and the issuing lane
-// issues gate|up of chunk c + 3 and the down projection of chunk c only after the post of chunk c.
-__device__ __forceinline__ void wait_ops(Epi& e, int n) {
+// wait_round: a round of n pair operations in rotation order, then a commit on ACC.
+__device__ __forceinline__ void wait_round(Epi& e, int n) {
+  wait_acc(e);
+  for (int i = 0; i < n; ++i) e.par ^= 1u << e.rot.next_pair();
+}
+// wait_op: gate|up of one chunk.  A thread that skips operations of a slot must not find the slot a phase
+// behind or two ahead: it waits only when an operation issued after the skipped one is known to be
+// complete (MMAs complete in order), and the slot's next one is issued only after its post.
+__device__ __forceinline__ void wait_op(Epi& e, uint32_t slot) {
   T_BEGIN();
-  for (int i = 0; i < n; ++i) {
-    const uint32_t slot = e.sched[e.cur] & 7u;
-    e.cur = e.cur + 1 == e.sched_len ? 0 : e.cur + 1;
-    mbar_wait(e.bars + 8 * (B_DONE0 + slot), (e.par >> slot) & 1u, e.status, e.aborted, ST_TIMEOUT_ACC);
-    e.par ^= 1u << slot;
-  }
+  mbar_wait(e.bars + 8 * (B_DONE0 + slot), (e.par >> slot) & 1u, e.status, e.aborted, ST_TIMEOUT_ACC);
   tc_fence_after();
   T_END(e.tacc, e.wait_slot);
-  TRACE(e.tr, 100 + n);
+  TRACE(e.tr, 100);
 }
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
 
@@ -301,65 +299,63 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* s) {
 }
 
 // GatedMLP on the A operand (already normed and posted on OP0): residual += down(gelu(gate) * up).
-// Chunk c: gate = acc[c % 3][0,64), up = acc[c % 3][64,128); this thread: hidden columns
-// [16 part, 16 part + 16) of the chunk.
+// Chunk c: gate = acc[c % 3][0,64), up = acc[c % 3][64,128).  Two groups of eight warps take turns
+// (parts 0, 1 the even chunks, parts 2, 3 the odd ones), so that one group's waits and tensor-memory
+// latencies hide behind the other's arithmetic; a thread owns 32 of the 64 hidden columns of its row,
+// columns [32 (part & 1), +32), in two passes of 16.
+//
+// The gated product stays in tensor memory as the A operand of the down projection: 16 k at a time
+// (8 columns of packed bf16 pairs) over the first half of 16 gate columns the thread has just read;
+// K step s of the MMA reads exactly the columns at 16 s.
 __device__ __forceinline__ void ffn(Epi& e) {
+  const int group = e.part >> 1, half = e.part & 1;
+  T_WAITSLOT(e, TE_FFN_ACC_WAIT);
 #pragma unroll 1
   for (int c = 0; c < 8; ++c) {
-    const int ai = c % 3, pi = c & 1;
-    T_WAITSLOT(e, TE_FFN_ACC_WAIT);
-    wait_ops(e, 1);   // gate|up of chunk c
-    T_BEGIN();
-    uint32_t gv[16], uv[16];
-    const uint32_t acc = e.lane_addr + COL_ACC0 + ai * 128 + e.part * 16;
-    tmem_ld16_nowait(acc, gv);
-    tmem_ld16_nowait(acc + 64, uv);
-    tmem_wait_ld();
-    uint4 o[2];
+    const uint32_t slot = e.rot.next_pair();
+    if ((c & 1) == group) {
+      wait_op(e, slot);   // gate|up of chunk c; the slot's previous operation, c - 3, came before c - 2
+      T_BEGIN();
+      const uint32_t acc = e.lane_addr + COL_ACC0 + (c % 3) * 128 + half * 32;
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      uint32_t w[4];
+      for (int p = 0; p < 2; ++p) {
+        uint32_t gv[16], uv[16];
+        tmem_ld16_nowait(acc + 16 * p, gv);
+        tmem_ld16_nowait(acc + 64 + 16 * p, uv);
+        tmem_wait_ld();
+        uint32_t w8[8];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        w[j] = gelu_mul_bf16x2(__uint_as_float(gv[q * 8 + 2 * j]), __uint_as_float(gv[q * 8 + 2 * j + 1]),
-                               __uint_as_float(uv[q * 8 + 2 * j]), __uint_as_float(uv[q * 8 + 2 * j + 1]));
-      o[q] = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int j = 0; j < 8; ++j)
+          w8[j] = gelu_mul_bf16x2(__uint_as_float(gv[2 * j]), __uint_as_float(gv[2 * j + 1]), __uint_as_float(uv[2 * j]), __uint_as_float(uv[2 * j + 1]));
+        tmem_st8_nowait(acc + 16 * p, w8);
+      }
+      tmem_wait_st();
+      T_END(e.tacc, TE_FFN_MATH);
+      post(e, B_FFN0 + c % 3);
     }
-    T_END(e.tacc, TE_FFN_MATH);
-    // the down projection of chunk c - 2 is next in the schedule: its wait keeps the cursor in step
-    T_WAITSLOT(e, TE_FFN_PF_WAIT);
-    if (c >= 2) wait_ops(e, 1);
-    // The gated product stays in tensor memory as the A operand of the down projection: this
-    // thread's 16 k (8 columns of packed bf16 pairs) over the first half of its own 16 gate
-    // columns, which it has just read; K step `part` of the MMA reads exactly those columns.
-    {
-      const uint32_t w8[8] = {o[0].x, o[0].y, o[0].z, o[0].w, o[1].x, o[1].y, o[1].z, o[1].w};
-      tmem_st8(e.lane_addr + COL_ACC0 + ai * 128 + e.part * 16, w8);
-    }
-    post(e, B_OP0 + pi);
+    e.par ^= 1u << slot;
   }
-  // residual complete: the down projections of chunks 6 and 7
-  wait_ops(e, 2);
   T_WAITSLOT(e, TE_ACC_WAIT);
+  wait_acc(e);   // residual complete: every down projection
 }
 
-// Attention of every head and environment of the tile from the staged q (A area), k and v (KV
+// Attention of every head and environment of the tile from the staged q (P area), k and v (KV
 // area), all in the swizzled operand layout (128 rows x 64 bf16 atoms; head h sits in atom h / 2,
-// columns 32 (h % 2) ..).  Warp w serves head w % 4 and every fourth block of 16 query rows;
-// keys are walked in blocks of 16 with a running maximum.  Output: bf16 into the P area as the
-// A operand of out_proj.
+// columns 32 (h % 2) ..).  The four warps of part h serve head h, which they have staged themselves,
+// and take turns at the blocks of 16 query rows; keys are walked in blocks of 16 with a running
+// maximum.  Output: bf16 into the P area as the A operand of out_proj, each block over its own q.
 __device__ __forceinline__ void attention(Epi& e, int n_items) {
   TRACE(e.tr, 310);
   const uint8_t* meta = e.smem + OFF_META;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int h = warp & 3;
+  const int h = e.part;
   const uint32_t atom = (uint32_t)(h >> 1) * CHUNK_BYTES;
   const int c8h = (h & 1) * 4;
-  const uint32_t sQ = e.sbase + OFF_A + atom, sK = e.sbase + OFF_KV + atom, sV = sK + 2 * CHUNK_BYTES;
+  const uint32_t sQ = e.sbase + OFF_P + atom, sK = e.sbase + OFF_KV + atom, sV = sK + 2 * CHUNK_BYTES;
   const float* key_bias = reinterpret_cast<const float*>(e.smem + OFF_BIAS);
   const float c2 = 0.17677669529663687f * 1.4426950408889634f;  // log2(e) / sqrt(32): scores in the log2 domain
-  for (int it = warp >> 2; it < n_items; it += EPI_WARPS / 4) {
+  for (int it = warp & 3; it < n_items; it += EPI_WARPS / 4) {
     const int r0 = meta[384 + it];
     const int e0 = meta[r0], n = meta[128 + r0] + 1;   // first tile row and size of the environment
     const int last = e0 + n - 1;
@@ -460,38 +456,44 @@ __device__ __forceinline__ void attention(Epi& e, int n_items) {
   }
 }
 
+// q|k|v of head `part` in columns [128 + 96 part, +96): the threads of part h go on while the later heads
+// are multiplied.
+__device__ __forceinline__ void wait_qkv(Epi& e) {
+  T_BEGIN();
+  mbar_wait(e.bars + 8 * (B_QKV0 + e.part), (e.par >> 9) & 1u, e.status, e.aborted, ST_TIMEOUT_ACC);
+  tc_fence_after();
+  e.par ^= 1u << 9;
+#pragma unroll
+  for (uint32_t h = 0; h < HEADS; ++h) e.par ^= 1u << qkv_slot(h);
+  after_qkv(e.rot);
+  T_END(e.tacc, e.wait_slot);
+  TRACE(e.tr, 114);
+}
+
 __device__ __forceinline__ void run_spatial(Epi& e, int n_items, bool row_valid) {
   norm_to_A(e);
   post(e, B_OP0);
-  wait_round(e, HEADS);   // q|k|v of head h in columns [128 + 96 h, +96)
+  wait_qkv(e);
   {
     T_BEGIN();
-    // this thread stages head `part` of its row: q into the A area (the normed operand has been
-    // consumed), k and v into the KV area, all in the swizzled atom layout
+    // this thread stages head `part` of its row: q into the P area (the normed operand is still being
+    // read for the later heads), k and v into the KV area (whose ring slot served head 0), all in the
+    // swizzled atom layout.  Rows outside every environment are zero rows from the input on.
     const int h = e.part;
     const uint32_t atom = (uint32_t)(h >> 1) * CHUNK_BYTES;
     const int c8h = (h & 1) * 4;
-    const uint32_t dst[3] = {OFF_A + atom, OFF_KV + atom, OFF_KV + 2 * CHUNK_BYTES + atom};
+    const uint32_t dst[3] = {OFF_P + atom, OFF_KV + atom, OFF_KV + 2 * CHUNK_BYTES + atom};
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
       uint32_t v[32];
       tmem_ld32(e.lane_addr + COL_ACC0 + h * 96 + p * 32, v);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(e.smem + dst[p] + swz(e.row, c8h + q)) = pack8(&v[q * 8]);
-    }
-    if (!row_valid) {
-      // rows outside every environment contribute a zero operand row to out_proj
-#pragma unroll
-      for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(e.smem + OFF_P + atom + swz(e.row, c8h + q)) = make_uint4(0u, 0u, 0u, 0u);
+      for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(e.smem + dst[p] + swz(e.row, c8h + q)) = row_valid ? pack8(&v[q * 8]) : make_uint4(0u, 0u, 0u, 0u);
     }
     T_END(e.tacc, TE_STAGE);
   }
   tc_fence_before();
-  {
-    T_BEGIN();
-    epi_sync();
-    T_END(e.tacc, TE_SYNC);
-  }
+  asm volatile("bar.sync %0, 128;" ::"r"(7 + e.part) : "memory");   // the four warps of this head
   {
     T_BEGIN();
     attention(e, n_items);
@@ -513,7 +515,7 @@ __device__ __forceinline__ void run_spatial(Epi& e, int n_items, bool row_valid)
 __device__ __forceinline__ void run_spatial_pre(Epi& e, const SubLayer& s, size_t grow, bool row_valid) {
   norm_to_A(e);
   post(e, B_OP0);
-  wait_round(e, HEADS);   // q|k|v of head h in columns [128 + 96 h, +96)
+  wait_qkv(e);
   const int h = e.part;
   __nv_bfloat16* dst = s.qkv_out + grow * (3 * D) + h * DH;
 #pragma unroll
@@ -765,7 +767,14 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
   ffn(e);
 }
 
-// ------------------------------------------------------------------ issuing side (one lane)
+// ------------------------------------------------------------------ issuing side (one warp)
+//
+// The whole warp runs this code with the same values in every lane, and one elected lane issues: the
+// operands of the MMAs then stay in uniform registers and an MMA costs three instructions.  Run by a
+// single lane, each MMA had to move its descriptors over first, and under the instruction-cache pressure
+// of the sixteen epilogue warps eight MMAs took 790 cycles of issue (1000 for the four of a down
+// projection) against the 520 (260) they need in the tensor pipe, which made the issue the slowest stage
+// of the GatedMLP.  For the same reason everything here is inlined.
 
 struct Issuer {
 #ifdef BNB_TRACE
@@ -775,139 +784,143 @@ struct Issuer {
   long long tacc[T_COUNT];
 #endif
   uint32_t sbase, bars, tmem;
-  uint32_t full_par;   // per-slot phase bits of the full barriers
-  uint32_t op_par;     // phase bits of OP0, OP1
-  const uint32_t* sched;
-  int sched_len, idx;
-  uint32_t next_slot;  // ring slot of the next chunk of the schedule
+  uint32_t elected;    // 1 in the lane that issues
+  uint32_t full_par;   // per-slot phase bits of the FULL barriers
+  uint32_t op_par;     // phase bits of OP0 and FFN0..2
+  SlotRotation rot;
   int* status;
   volatile int* aborted;
 };
 
-__device__ __forceinline__ void wait_operand(Issuer& m, int i) {
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p;
+}
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+__device__ __forceinline__ void wait_operand(Issuer& m, int bar) {
   T_BEGIN();
-  mbar_wait(m.bars + 8 * (B_OP0 + i), (m.op_par >> i) & 1u, m.status, m.aborted, ST_TIMEOUT_OPERAND);
-  m.op_par ^= 1u << i;
+  mbar_wait(m.bars + 8 * bar, (m.op_par >> bar) & 1u, m.status, m.aborted, ST_TIMEOUT_OPERAND);
+  m.op_par ^= 1u << bar;
   tc_fence_after();
   T_END(m.tacc, TM_OP_WAIT);
-  TRACE(m.tr, 400 + i);
+  TRACE(m.tr, 400 + bar);
 }
-// tcgen05.mma with both shared-memory descriptors built from 32-bit halves inside the asm block
-// (K-major, 128-byte swizzle, 8-row groups 1024 B apart: the high word is a constant), which keeps
-// the issuing lane's register count low.
+// tcgen05.mma with the shared-memory descriptors built from 32-bit halves inside the asm block
+// (K-major, 128-byte swizzle, 8-row groups 1024 B apart: the high word is a constant); A in shared
+// memory, or (TMEM_A) in tensor memory: lane = row, a 32-bit column = two consecutive k as bfloat16.
 __device__ __forceinline__ uint32_t desc_lo(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); }
-__device__ __forceinline__ void tc_mma_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-      "mov.b64 da, {%1, %5};\n\t"
-      "mov.b64 db, {%2, %5};\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0x40004040u) : "memory");
+template <bool TMEM_A>
+__device__ __forceinline__ void mma_one(uint32_t elected, uint32_t d_tmem, uint32_t a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (TMEM_A)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
+        "mov.b64 db, {%2, %5};\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0x40004040u), "r"(elected) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %5};\n\t"
+        "mov.b64 db, {%2, %5};\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0x40004040u), "r"(elected) : "memory");
 }
-
-// The next ring operation of the schedule: wait for its weights, issue its MMAs
-// (D[128 x n] (+)= A[128 x 64] * W[n x 64]^T per K atom: a pair reads K atom 0 of the operand at
-// a_off0 and K atom 1 at a_off1), and commit on the slot's DONE barrier.
-__device__ __forceinline__ void issue_op(Issuer& m, bool pair, uint32_t a_off0, uint32_t a_off1, uint32_t n, uint32_t d_col,
-                                         uint32_t accumulate) {
-  const uint32_t slot = m.next_slot;
-  m.idx = m.idx + 1 == m.sched_len ? 0 : m.idx + 1;
-  m.next_slot = m.sched[m.idx] & 7u;   // not needed before the next call: the load's latency is hidden
+__device__ __forceinline__ void commit_one(const Issuer& m, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(m.bars + 8 * bar), "r"(m.elected) : "memory");
+}
+// Waits for the weights of a slot; returns the low descriptor word of its first chunk.
+__device__ __forceinline__ uint32_t wait_weights(Issuer& m, uint32_t slot) {
   T_MARK(tw);
   mbar_wait(m.bars + 8 * (B_FULL0 + slot), (m.full_par >> slot) & 1u, m.status, m.aborted, ST_TIMEOUT_FULL);
   m.full_par ^= 1u << slot;
   T_SINCE(m.tacc, TM_FULL_WAIT, tw);
   TRACE(m.tr, 410);
-  const uint32_t b_lo = desc_lo(m.sbase + slot_offset(slot));
+  return uniform(desc_lo(m.sbase + slot_offset(slot)));
+}
+// A pair operation: D[128 x n] (+)= A[128 x 128] * W[n x 128]^T, K atom 0 of the operand at a_off0 and K
+// atom 1 at a_off1; commits on the slot's DONE barrier.  (A step of 16 K columns = 32 bytes = 2 in
+// descriptor units; a K atom = 16 KB = 1024 units.)
+__device__ __forceinline__ void issue_pair(Issuer& m, uint32_t slot, uint32_t a_off0, uint32_t a_off1, uint32_t n, uint32_t d_col,
+                                           uint32_t accumulate) {
+  const uint32_t b_lo = wait_weights(m, slot);
+  T_MARK(tw);
   const uint32_t idesc = instr_desc(n);
-  // a step of 16 K columns = 32 bytes = 2 in descriptor units; a K atom = 16 KB = 1024 units
-  const uint32_t a0 = desc_lo(m.sbase + a_off0);
+  const uint32_t a0 = desc_lo(m.sbase + a_off0), a1 = desc_lo(m.sbase + a_off1);
 #pragma unroll
-  for (uint32_t k = 0; k < 4; ++k) tc_mma_lo(m.tmem + d_col, a0 + 2 * k, b_lo + 2 * k, idesc, (accumulate | k) ? 1u : 0u);
-  if (pair) {
-    const uint32_t a1 = desc_lo(m.sbase + a_off1);
+  for (uint32_t k = 0; k < 4; ++k) mma_one<false>(m.elected, m.tmem + d_col, a0 + 2 * k, b_lo + 2 * k, idesc, (accumulate | k) ? 1u : 0u);
 #pragma unroll
-    for (uint32_t k = 0; k < 4; ++k) tc_mma_lo(m.tmem + d_col, a1 + 2 * k, b_lo + 1024 + 2 * k, idesc, 1u);
-  }
-  tc_commit(m.bars + 8 * (B_DONE0 + slot));
+  for (uint32_t k = 0; k < 4; ++k) mma_one<false>(m.elected, m.tmem + d_col, a1 + 2 * k, b_lo + 1024 + 2 * k, idesc, 1u);
+  commit_one(m, B_DONE0 + slot);
   T_SINCE(m.tacc, TM_ISSUE, tw);
   TRACE(m.tr, 420);
 }
-// The same with the A operand in tensor memory: K step k reads the 8 columns at a_col + 16 k
-// (lane = row, a 32-bit column = two consecutive k as bfloat16).
-__device__ __forceinline__ void tc_mma_tmem_a(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-      "mov.b64 db, {%2, %5};\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0x40004040u) : "memory");
+__device__ __forceinline__ void issue_from_A(Issuer& m, uint32_t slot, uint32_t n, uint32_t d_col) {
+  issue_pair(m, slot, OFF_A, OFF_A + CHUNK_BYTES, n, d_col, 0);
 }
-__device__ __forceinline__ void issue_down_tmem(Issuer& m, uint32_t a_col) {
-  const uint32_t slot = m.next_slot;
-  m.idx = m.idx + 1 == m.sched_len ? 0 : m.idx + 1;
-  m.next_slot = m.sched[m.idx] & 7u;
-  mbar_wait(m.bars + 8 * (B_FULL0 + slot), (m.full_par >> slot) & 1u, m.status, m.aborted, ST_TIMEOUT_FULL);
-  m.full_par ^= 1u << slot;
-  const uint32_t b_lo = desc_lo(m.sbase + slot_offset(slot));
+// The down projection of a chunk: its A operand in tensor memory, K step k in the 8 columns at a_col + 16 k.
+__device__ __forceinline__ void issue_down(Issuer& m, uint32_t a_col) {
+  const uint32_t slot = m.rot.next_single();
+  const uint32_t b_lo = wait_weights(m, slot);
+  T_MARK(tw);
   const uint32_t idesc = instr_desc(128);
 #pragma unroll
-  for (uint32_t k = 0; k < 4; ++k) tc_mma_tmem_a(m.tmem + COL_RESID, m.tmem + a_col + 16 * k, b_lo + 2 * k, idesc, 1u);
-  tc_commit(m.bars + 8 * (B_DONE0 + slot));
+  for (uint32_t k = 0; k < 4; ++k) mma_one<true>(m.elected, m.tmem + COL_RESID, m.tmem + a_col + 16 * k, b_lo + 2 * k, idesc, 1u);
+  commit_one(m, B_DONE0 + slot);
+  T_SINCE(m.tacc, TM_ISSUE, tw);
+  TRACE(m.tr, 430);
 }
-__device__ __forceinline__ void issue_pair(Issuer& m, uint32_t a_off, uint32_t n, uint32_t d_col) {
-  issue_op(m, true, a_off, a_off + CHUNK_BYTES, n, d_col, 0);
-}
-__device__ __forceinline__ void commit_round(const Issuer& m) { tc_commit(m.bars + 8 * B_ACC); }
+__device__ __forceinline__ void commit_round(const Issuer& m) { commit_one(m, B_ACC); }
 
 __device__ __forceinline__ void issue_ffn(Issuer& m) {
-  wait_operand(m, 0);
+  wait_operand(m, B_OP0);
 #pragma unroll 1
-  for (int c = 0; c < 3; ++c) issue_pair(m, OFF_A, 128, COL_ACC0 + 128 * c);
+  for (uint32_t c = 0; c < 3; ++c) issue_from_A(m, m.rot.next_pair(), 128, COL_ACC0 + 128 * c);
+  uint32_t a = 0;
 #pragma unroll 1
-  for (int c = 0; c < 8; ++c) {
-    wait_operand(m, c & 1);   // product of chunk c written, accumulator c % 3 read
-    issue_down_tmem(m, COL_ACC0 + 128 * (c % 3));
-    if (c + 3 < 8) issue_pair(m, OFF_A, 128, COL_ACC0 + 128 * (c % 3));
+  for (uint32_t c = 0; c < 8; ++c) {
+    wait_operand(m, B_FFN0 + a);   // product of chunk c written, accumulator a = c % 3 read
+    issue_down(m, COL_ACC0 + 128 * a);
+    if (c + 3 < 8) issue_from_A(m, m.rot.next_pair(), 128, COL_ACC0 + 128 * a);
+    a = a == 2 ? 0 : a + 1;
   }
+  commit_round(m);
 }
-__device__ __forceinline__ void issue_spatial(Issuer& m) {
-  wait_operand(m, 0);
+__device__ __forceinline__ void issue_qkv(Issuer& m) {
+  wait_operand(m, B_OP0);
 #pragma unroll 1
-  for (int h = 0; h < HEADS; ++h) issue_pair(m, OFF_A, 96, COL_ACC0 + 96 * h);
-  commit_round(m);
-  wait_operand(m, 0);   // attention output: K atom 0 = heads 0, 1; K atom 1 = heads 2, 3
-  issue_op(m, true, OFF_P, OFF_P + CHUNK_BYTES, 128, COL_RESID, 1);
-  commit_round(m);
-  issue_ffn(m);
+  for (uint32_t h = 0; h < HEADS; ++h) {
+    issue_from_A(m, qkv_slot(h), 96, COL_ACC0 + 96 * h);
+    commit_one(m, B_QKV0 + h);
+  }
+  after_qkv(m.rot);
 }
-__device__ __forceinline__ void issue_spatial_pre(Issuer& m) {
-  wait_operand(m, 0);
-#pragma unroll 1
-  for (int h = 0; h < HEADS; ++h) issue_pair(m, OFF_A, 96, COL_ACC0 + 96 * h);
+__device__ __forceinline__ void issue_out_proj(Issuer& m, uint32_t a_off) {
+  wait_operand(m, B_OP0);   // attention output: K atom 0 = heads 0, 1; K atom 1 = heads 2, 3
+  issue_pair(m, m.rot.next_pair(), a_off, a_off + CHUNK_BYTES, 128, COL_RESID, 1);
   commit_round(m);
-}
-__device__ __forceinline__ void issue_spatial_post(Issuer& m) {
-  wait_operand(m, 0);   // attention output in A: K atom 0 = heads 0, 1; K atom 1 = heads 2, 3
-  issue_op(m, true, OFF_A, OFF_A + CHUNK_BYTES, 128, COL_RESID, 1);
-  commit_round(m);
-  issue_ffn(m);
 }
 __device__ __forceinline__ void issue_temporal(Issuer& m, bool has_fields) {
-  wait_operand(m, 0);
-  issue_pair(m, OFF_A, 128, COL_ACC0);   // linear2
-  issue_pair(m, OFF_A, 128, COL_ACC1);   // linear1
+  wait_operand(m, B_OP0);
+  issue_from_A(m, m.rot.next_pair(), 128, COL_ACC0);   // linear2
+  issue_from_A(m, m.rot.next_pair(), 128, COL_ACC1);   // linear1
   commit_round(m);
-  wait_operand(m, 0);
-  issue_pair(m, OFF_A, 128, COL_ACC0);   // gates of hidden columns [0,64)
-  issue_pair(m, OFF_A, 128, COL_ACC1);   // gates of hidden columns [64,128)
-  if (has_fields) issue_pair(m, OFF_A, 128, COL_ACC2);   // field_sub
+  wait_operand(m, B_OP0);
+  issue_from_A(m, m.rot.next_pair(), 128, COL_ACC0);   // gates of hidden columns [0,64)
+  issue_from_A(m, m.rot.next_pair(), 128, COL_ACC1);   // gates of hidden columns [64,128)
+  if (has_fields) issue_from_A(m, m.rot.next_pair(), 128, COL_ACC2);   // field_sub
   commit_round(m);
-  wait_operand(m, 0);
-  issue_op(m, true, OFF_P, OFF_A + CHUNK_BYTES, 128, COL_RESID, 1);   // linear_out: K atom 0 from P0, K atom 1 in place in A
+  wait_operand(m, B_OP0);
+  issue_pair(m, m.rot.next_pair(), OFF_P, OFF_A + CHUNK_BYTES, 128, COL_RESID, 1);   // linear_out: K atom 0 from P0, K atom 1 in place in A
   commit_round(m);
-  issue_ffn(m);
 }
 
 // ------------------------------------------------------------------ the kernel
@@ -918,7 +931,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
   __shared__ __align__(8) int s_aborted[4];   // [2..3]: address of the host's status word
   __shared__ int s_items;
   __shared__ SubLayer s_sub[MAX_SUBLAYERS];  // kernel parameters are slow to index dynamically
-  __shared__ uint32_t s_sched[MAX_SCHED];
+  __shared__ uint4 s_sched[MAX_SCHED];
   __shared__ int s_sched_len;
   const int tid = threadIdx.x, warp = tid >> 5;
   if (tid < args.n_sub) s_sub[tid] = args.sub[tid];
@@ -930,7 +943,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     *reinterpret_cast<int**>(&s_aborted[2]) = args.host_status;
     s_aborted[1] = args.poll_limit > 0 ? args.poll_limit : DEFAULT_POLL_LIMIT;
     mbar_init(smem_u32(&bars[B_OP0]), EPI_WARPS);
-    mbar_init(smem_u32(&bars[B_OP1]), EPI_WARPS);
+    for (int i = B_FFN0; i <= B_FFN2; ++i) mbar_init(smem_u32(&bars[i]), EPI_WARPS / 2);
     mbar_init(smem_u32(&bars[B_KVREL]), EPI_WARPS);
     for (int i = B_ACC; i < B_COUNT; ++i) mbar_init(smem_u32(&bars[i]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -948,11 +961,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
 
   if (warp == LOAD_WARP) {
     // ---------------------------------------------------------------- weight stream
-    if ((tid & 31) == 0) {
+    // The whole warp runs the same code and one elected lane copies, as on the issuing side.
+    {
       const uint32_t sbase = smem_u32(smem), bar0 = smem_u32(bars);
+      const bool elected = elect_one() != 0;
       uint32_t free_par = (1u << N_SLOTS) - 1u;   // a fresh barrier passes a wait on parity 1: every slot starts free
       uint32_t kv_par = 0;
       const int len = s_sched_len;
+      const int skip_op = blockIdx.x == 0 ? args.skip_op : -1;
 #ifdef BNB_TIMING
       long long tacc[T_COUNT];
       for (int i = 0; i < T_COUNT; ++i) tacc[i] = 0;
@@ -961,13 +977,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
 #ifdef BNB_TRACE
       Trace ltr;
       trace_init(ltr, args.status, 2);
+      if ((tid & 31) != 0) ltr.n = 1500;
 #endif
+      int op = 0;
       for (int pass = 0; pass < passes; ++pass)
-        for (int i = 0; i < len; ++i) {
-          const uint32_t en = s_sched[i];
-          const uint32_t slot = en & 7u;
+        for (int i = 0; i < len; ++i, ++op) {
+          const uint4 en = s_sched[i];
+          const uint32_t slot = uniform(en.w & 7u);
           T_MARK(tw);
-          if (en & (1u << 18)) {
+          if (en.w & 8u) {
             mbar_wait(bar0 + 8 * B_KVREL, kv_par, args.status, s_aborted, ST_TIMEOUT_FREE);
             kv_par ^= 1u;
           }
@@ -977,71 +995,68 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
           // Once a wait of this CTA has run out nothing is in step any more: stop fetching.  Arming a
           // FULL barrier again before its previous copy has landed would arrive on it twice in one
           // phase, which is undefined; the other roles' waits give up at once and the kernel drains.
-          if (*static_cast<volatile int*>(s_aborted)) { pass = passes; break; }
+          if (__any_sync(0xffffffffu, *static_cast<volatile int*>(s_aborted))) { pass = passes; break; }
           T_SINCE(tacc, TL_FREE_WAIT, tw);
           TRACE(ltr, 500 + slot);
           const uint32_t full = bar0 + 8 * (B_FULL0 + slot);
-          const uint8_t* image = s_sub[(en >> 3) & 7u].packed;
-          const uint32_t ch0 = (en >> 6) & 63u, ch1 = (en >> 12) & 63u;
           const uint32_t dst = sbase + slot_offset(slot);
-          if (blockIdx.x == 0 && pass * len + i == args.skip_op) {
-            // test hook: this operation's weights never arrive
-          } else if (ch1 == NO_CHUNK) {
-            mbar_expect_tx(full, CHUNK_BYTES);
-            bulk_g2s(dst, image + (size_t)ch0 * CHUNK_BYTES, CHUNK_BYTES, full);
-          } else if (ch1 == ch0 + 1) {
-            mbar_expect_tx(full, 2 * CHUNK_BYTES);
-            bulk_g2s(dst, image + (size_t)ch0 * CHUNK_BYTES, 2 * CHUNK_BYTES, full);
-          } else {
-            mbar_expect_tx(full, 2 * CHUNK_BYTES);
-            bulk_g2s(dst, image + (size_t)ch0 * CHUNK_BYTES, CHUNK_BYTES, full);
-            bulk_g2s(dst + CHUNK_BYTES, image + (size_t)ch1 * CHUNK_BYTES, CHUNK_BYTES, full);
+          if (elected && op != skip_op) {   // skip_op: test hook, this operation's weights never arrive
+            const uint8_t* src = reinterpret_cast<const uint8_t*>(((unsigned long long)en.y << 32) | en.x);
+            mbar_expect_tx(full, en.z ? 2 * CHUNK_BYTES : CHUNK_BYTES);
+            bulk_g2s(dst, src, CHUNK_BYTES, full);
+            if (en.z) bulk_g2s(dst + CHUNK_BYTES, src + en.z, CHUNK_BYTES, full);
           }
+          __syncwarp();
         }
 #ifdef BNB_TIMING
       tacc[TL_TOTAL] = clock64() - t_start;
-      T_STORE(args, tacc, TL_FREE_WAIT, T_COUNT);
+      if ((tid & 31) == 0) T_STORE(args, tacc, TL_FREE_WAIT, T_COUNT);
 #endif
     }
   } else if (warp == MMA_WARP) {
     // ---------------------------------------------------------------- tensor-core issue
-    if ((tid & 31) == 0) {
+    {
       Issuer m;
       m.sbase = smem_u32(smem);
       m.bars = smem_u32(bars);
-      m.tmem = tmem_base;
+      m.tmem = uniform(tmem_base);
+      m.elected = elect_one();
       m.full_par = 0;
       m.op_par = 0;
-      m.sched = s_sched;
-      m.sched_len = s_sched_len;
-      m.idx = 0;
-      m.next_slot = s_sched[0] & 7u;
+      m.rot = SlotRotation{0, 3};
       m.status = args.status;
       m.aborted = s_aborted;
 #ifdef BNB_TRACE
       trace_init(m.tr, args.status, 1);
+      if ((tid & 31) != 0) m.tr.n = 1500;
 #endif
 #ifdef BNB_TIMING
       for (int i = 0; i < T_COUNT; ++i) m.tacc[i] = 0;
 #endif
       T_MARK(t_start);
-      for (int pass = 0; pass < passes; ++pass)
+      for (int pass = 0; pass < passes; ++pass) {
+        m.rot = SlotRotation{0, 3};   // every pass walks the schedule from its start
         for (int si = 0; si < args.n_sub; ++si) {
-          const int type = s_sub[si].type;
-          if (type == SUB_SPATIAL) issue_spatial(m);
-          else if (type == SUB_SPATIAL_PRE) issue_spatial_pre(m);
-          else if (type == SUB_SPATIAL_POST) issue_spatial_post(m);
-          else issue_temporal(m, args.has_fields != 0);
+          const int type = (int)uniform((uint32_t)s_sub[si].type);
+          if (type == SUB_TEMPORAL) {
+            issue_temporal(m, args.has_fields != 0);
+          } else {
+            if (type != SUB_SPATIAL_POST) issue_qkv(m);
+            if (type == SUB_SPATIAL_PRE) continue;
+            issue_out_proj(m, type == SUB_SPATIAL_POST ? OFF_A : OFF_P);
+          }
+          issue_ffn(m);
         }
+      }
       // Nothing issued here may outlive the CTA: its tensor memory is freed and its barriers go
       // away at the end.  In a normal run the epilogue warps' last waits already imply this; after
       // a wait has run out nobody has waited for anything, so wait here, with the full limit.
-      tc_commit(m.bars + 8 * B_DRAIN);
+      commit_one(m, B_DRAIN);
       for (int i = 0; i < DEFAULT_POLL_LIMIT && !mbar_try_wait(m.bars + 8 * B_DRAIN, 0); ++i) {
       }
 #ifdef BNB_TIMING
       m.tacc[TM_TOTAL] = clock64() - t_start;
-      T_STORE(args, m.tacc, TM_FULL_WAIT, TL_FREE_WAIT);
+      if ((tid & 31) == 0) T_STORE(args, m.tacc, TM_FULL_WAIT, TL_FREE_WAIT);
 #endif
     }
   } else {
@@ -1054,9 +1069,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     e.part = tid >> 7;
     e.lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
     e.par = 0;
-    e.sched = s_sched;
-    e.sched_len = s_sched_len;
-    e.cur = 0;
+    e.rot = SlotRotation{0, 3};
     e.status = args.status;
     e.aborted = s_aborted;
     e.ss_part = reinterpret_cast<float*>(smem + OFF_SS);
@@ -1187,6 +1200,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
         epi_sync();
         T_SINCE(e.tacc, TE_IO, t_io);
         const int n_items = s_items;
+        e.rot = SlotRotation{0, 3};
         for (int si = 0; si < args.n_sub; ++si) {
           const SubLayer& s = s_sub[si];
           // Ask L2 for the recurrent state of the temporal sublayer that follows this one: the
