@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "launch_count.h"
+#include "train_attention.h"
 
 namespace bnb {
 namespace grad {
@@ -1580,6 +1581,12 @@ void attn_fwd_t(const Ctx& c, const float* qkv, const uint8_t* alive, float* o, 
 void attn_fwd(const Ctx& c, const float* qkv, const uint8_t* alive, float* o, int G, int NM, const float* kvb,
               const uint8_t* bactive, int nb) {
   if (!G) return;
+  if (train_attn::supported(c.D, c.H, NM, nb)) {
+    train_attn::Call a{};
+    a.qkv = qkv; a.alive = alive; a.kvb = kvb; a.bactive = bactive; a.G = G; a.n = NM; a.nb = nb; a.o = o;
+    train_attn::forward(a, c.st);
+    return;
+  }
   if (c.D / c.H == 32 && NM <= 32 && !kvb) {
     const int n_pairs = G * c.H;
     const int lpp = NM <= 8 ? 8 : NM <= 16 ? 16 : 32;
@@ -1661,16 +1668,24 @@ int spatial_bwd(const Ctx& c, const BnbSpatialWeights& w, const BnbSpatialGrads&
 
   mm(c, TN, dx1, D, o, D, dw.out_w, D, D, D, M);
   mm(c, NN, dx1, D, w.out_w, D, d_o, D, M, D, D);
-  const int dh = D / c.H;
-  const float scale = 1.0f / sqrtf((float)dh);
-  AttnBwdArgs self{qkv, 3 * D, qkv + D, 3 * D, D, alive, d_o, D, dqkv, 3 * D, 0, dqkv + D, 3 * D, D, NM, NM, dh, scale, 0};
-  int rc = attn_bwd(c, self, G);
-  if (rc) return rc;
+  int rc;
+  if (train_attn::supported(D, c.H, NM, nb)) {
+    train_attn::Call a{};
+    a.qkv = qkv; a.alive = alive; a.kvb = reads ? b.kvb : nullptr; a.bactive = reads ? bul->active : nullptr;
+    a.G = G; a.n = NM; a.nb = nb; a.d_o = d_o; a.dqkv = dqkv; a.dkvb = b.dkvb;
+    if ((rc = train_attn::backward(a, c.st))) return rc;
+  } else {
+    const int dh = D / c.H;
+    const float scale = 1.0f / sqrtf((float)dh);
+    AttnBwdArgs self{qkv, 3 * D, qkv + D, 3 * D, D, alive, d_o, D, dqkv, 3 * D, 0, dqkv + D, 3 * D, D, NM, NM, dh, scale, 0};
+    if ((rc = attn_bwd(c, self, G))) return rc;
+    if (reads) {
+      AttnBwdArgs cross{qkv, 3 * D, b.kvb, 2 * D, D, bul->active, d_o, D, dqkv, 3 * D, 1, b.dkvb, 2 * D, D, NM, nb, dh, scale,
+                        bul->active ? 1 : 0};
+      if ((rc = attn_bwd(c, cross, G))) return rc;
+    }
+  }
   if (reads) {
-    AttnBwdArgs cross{qkv, 3 * D, b.kvb, 2 * D, D, bul->active, d_o, D, dqkv, 3 * D, 1, b.dkvb, 2 * D, D, NM, nb, dh, scale,
-                      bul->active ? 1 : 0};
-    rc = attn_bwd(c, cross, G);
-    if (rc) return rc;
     mmh(c, TN, H_B, b.dkvb, 2 * D, b.bul_n, D, dw.kv_bullet_w, D, 2 * D, D, (int)RB);
     mm(c, NN, b.dkvb, 2 * D, w.kv_bullet_w, D, b.bul_dn, D, (int)RB, D, 2 * D);
     // the bullet tokens feed every sublayer that reads them: their gradient accumulates

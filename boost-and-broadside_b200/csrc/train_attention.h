@@ -1,0 +1,29 @@
+// Attention of the training path for small environments (train_attention.cu): forward and gradient of
+// the self-attention and the bullet branch, float32.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+#include <stdint.h>
+
+namespace bnb {
+namespace train_attn {
+
+struct Call {
+  const float* qkv;         // (G * n, 3 * 128) q | k | v, four heads of 32 side by side in each
+  const uint8_t* alive;     // (G * n) or null
+  const float* kvb;         // (G * nb, 2 * 128) bullet keys | values, or null
+  const uint8_t* bactive;   // (G * nb) or null: every slot is a key
+  int G, n, nb;
+  float* o;                 // forward: (G * n, 128)
+  const float* d_o;         // gradient: (G * n, 128) in; (G * n, 384) and (G * nb, 256) out
+  float* dqkv;
+  float* dkvb;
+};
+
+// d_model 128, 4 heads, up to 32 tokens per environment.
+bool supported(int d_model, int n_heads, int n, int nb);
+int forward(const Call& c, cudaStream_t st);
+int backward(const Call& c, cudaStream_t st);
+
+}  // namespace train_attn
+}  // namespace bnb
