@@ -28,6 +28,7 @@
 #include "common.cuh"
 #include "launch_count.h"
 #include "train_attention.h"
+#include "train_mlp.h"
 
 namespace bnb {
 namespace grad {
@@ -1412,15 +1413,29 @@ struct Bufs {
   float* w4[3];        // rows x 4D
   float* inv[2];       // rows
   float *bul_n, *bul_inv, *kvb, *dkvb, *bul_dn;
+  // bf16 mode at d_model 128, where the gated MLPs run fused (train_mlp.cu)
+  int* status;
+  uint8_t *images;     // weight images of every sublayer's MLP
+  uint8_t *n_image, *dy_image;
 };
 
-// half_mlp: the three 4D-wide buffers hold bfloat16 (bf16 mode), so they take half the bytes.
-void plan(Arena& ar, Bufs& b, int S, size_t R, int D, size_t RB, bool half_mlp) {
+// Whether the gated MLPs of a call run on the fused kernels, which keep nothing 4 d_model wide.
+bool fused_mlp(int D, bool bf16) { return bf16 && D == 128; }
+
+// bf16: the 4D-wide buffers, where they exist at all (see fused_mlp), hold bfloat16.
+void plan(Arena& ar, Bufs& b, int S, int n_images, size_t R, int D, size_t RB, bool bf16) {
   b.bound = ar.take((size_t)(S > 1 ? S - 1 : 0) * R * D);
   for (auto& p : b.ping) p = ar.take(R * D);
   for (auto& p : b.d) p = ar.take(R * D);
   for (auto& p : b.w3) p = ar.take(R * 3 * D);
-  for (auto& p : b.w4) p = ar.take(R * 4 * D / (half_mlp ? 2 : 1));
+  if (fused_mlp(D, bf16)) {
+    b.status = reinterpret_cast<int*>(ar.take(64));
+    b.images = reinterpret_cast<uint8_t*>(ar.take((size_t)n_images * train_mlp::image_bytes() / 4));
+    b.n_image = reinterpret_cast<uint8_t*>(ar.take(train_mlp::rows_image_bytes(R) / 4));
+    b.dy_image = reinterpret_cast<uint8_t*>(ar.take(train_mlp::rows_image_bytes(R) / 4));
+  } else {
+    for (auto& p : b.w4) p = ar.take(R * 4 * D / (bf16 ? 2 : 1));
+  }
   for (auto& p : b.inv) p = ar.take(R);
   b.bul_n = ar.take(RB * D);
   b.bul_inv = ar.take(RB);
@@ -1439,17 +1454,19 @@ void bind_forward(Arena& ar, Bufs& b, PathKind kind, size_t rows, int D, size_t 
   // MLP) are bfloat16 in bf16 mode: half the floats
   const size_t normed = half_mlp ? (rows * D + 1) / 2 : rows * D;
   const int n_slot = kind == P_SPATIAL ? 0 : 1;
+  const bool fused = fused_mlp(D, half_mlp);   // then the MLP keeps nothing: its gradient starts from its input
   for (int i = 0; i < nd; ++i) b.d[i] = ar.take(i == n_slot ? normed : rows * D);
-  b.d[15] = ar.take(normed);
+  if (!fused) b.d[15] = ar.take(normed);
   b.inv[0] = ar.take(rows);
-  b.inv[1] = ar.take(rows);
+  if (!fused) b.inv[1] = ar.take(rows);
   if (kind == P_SPATIAL) {
     b.w3[0] = ar.take(rows * 3 * D);
     b.bul_n = ar.take(RB * D);
     b.bul_inv = ar.take(RB);
     b.kvb = ar.take(RB * 2 * D);
   }
-  for (auto& p : b.w4) p = ar.take(rows * 4 * D / (half_mlp ? 2 : 1));
+  if (!fused)
+    for (auto& p : b.w4) p = ar.take(rows * 4 * D / (half_mlp ? 2 : 1));
 }
 
 inline int blocks_for(size_t n, int per_block, int cap = 148 * 8) {
@@ -1462,6 +1479,7 @@ struct Ctx {
   int D, H;
   bool bf16;   // products round their operands to bfloat16 (the forward ran under autocast)
   cudaStream_t st;
+  const uint8_t* mlp_image;   // weight image of the current sublayer's MLP (fused_mlp)
   Bufs b;
 };
 
@@ -1519,6 +1537,10 @@ void colsum(const Ctx& c, const float* a, float* out, size_t rows, int N) {
 // writes y when y is given.
 void mlp_fwd(const Ctx& c, const float* x1, float* y, size_t rows, const float* g2, const float* Wg, const float* Wu,
              const float* Wd) {
+  if (fused_mlp(c.D, c.bf16)) {   // nothing to leave behind
+    if (y) train_mlp::forward(x1, g2, c.mlp_image, y, rows, c.b.status, c.st);
+    return;
+  }
   const int D = c.D, F = 4 * c.D, M = (int)rows;
   float *n2 = c.b.d[15], *gb = c.b.w4[0], *ub = c.b.w4[1], *hb = c.b.w4[2];
   rmsnorm_fwd(c, x1, g2, n2, c.b.inv[1], rows);
@@ -1542,6 +1564,10 @@ void mlp_fwd(const Ctx& c, const float* x1, float* y, size_t rows, const float* 
 // After mlp_fwd: given d y, accumulates the weight gradients and writes d x1.  Uses d[16].
 void mlp_bwd(const Ctx& c, const float* x1, const float* dy, float* dx1, size_t rows, const float* g2, const float* Wg,
              const float* Wu, const float* Wd, float* dg2, float* dWg, float* dWu, float* dWd) {
+  if (fused_mlp(c.D, c.bf16)) {
+    train_mlp::backward(x1, g2, c.mlp_image, dy, dx1, dg2, dWg, dWu, dWd, c.b.n_image, c.b.dy_image, rows, c.b.status, c.st);
+    return;
+  }
   const int D = c.D, F = 4 * c.D, M = (int)rows;
   float *n2 = c.b.d[15], *dn2 = c.b.d[16], *gb = c.b.w4[0], *ub = c.b.w4[1], *hb = c.b.w4[2];
   if (c.bf16) {
@@ -1918,7 +1944,7 @@ size_t scratch_bytes(int n_blocks, int n_spatial, int n_temporal, int D, const B
   Bufs b;
   const int S = n_blocks * (n_spatial + n_temporal);
   const size_t G = (size_t)T * bt.n_envs;
-  plan(ar, b, S, G * bt.tokens_per_env, D, G * (bullets_per_env > 0 ? bullets_per_env : 0), bf16);
+  plan(ar, b, S, S, G * bt.tokens_per_env, D, G * (bullets_per_env > 0 ? bullets_per_env : 0), bf16);
   return ar.off + 256;
 }
 
@@ -1940,7 +1966,7 @@ int open_buffers(Ctx& c, Kept* kept, const Walk& wk, int n_blocks, int n_spatial
                  size_t scratch_bytes, void* kept_ptr, size_t kept_size) {
   uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + 255) & ~(uintptr_t)255;
   Arena ar{reinterpret_cast<char*>(base)};
-  plan(ar, c.b, kept_ptr ? 0 : wk.S, wk.R, wk.D, wk.RB, c.bf16);
+  plan(ar, c.b, kept_ptr ? 0 : wk.S, wk.S, wk.R, wk.D, wk.RB, c.bf16);
   if (ar.off + (base - reinterpret_cast<uintptr_t>(scratch)) > scratch_bytes) return BNB_ERR_SCRATCH_TOO_SMALL;
   if (kept_ptr) {
     uintptr_t kb = (reinterpret_cast<uintptr_t>(kept_ptr) + 255) & ~(uintptr_t)255;
@@ -1950,6 +1976,27 @@ int open_buffers(Ctx& c, Kept* kept, const Walk& wk, int n_blocks, int n_spatial
   }
   return BNB_OK;
 }
+
+// Weight images of the call's MLPs, in sublayer order, and a clean status word.
+int prepare_mlps(Ctx& c, const Walk& wk, const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, int n_blocks, int n_spatial,
+                 int n_temporal) {
+  if (!fused_mlp(c.D, c.bf16)) return BNB_OK;
+  train_mlp::Weights w[256];
+  int s = 0;
+  for (int blk = 0; blk < n_blocks; ++blk) {
+    for (int j = 0; j < n_spatial; ++j, ++s) {
+      const BnbSpatialWeights& sw = spatial[blk * n_spatial + j];
+      w[s] = {sw.gate_w, sw.up_w, sw.down_w};
+    }
+    for (int j = 0; j < n_temporal; ++j, ++s) {
+      const BnbTemporalWeights& tw = temporal[blk * n_temporal + j];
+      w[s] = {tw.gate_w, tw.up_w, tw.down_w};
+    }
+  }
+  if (cudaMemsetAsync(c.b.status, 0, sizeof(int), c.st) != cudaSuccess) return BNB_ERR_LAUNCH;
+  return train_mlp::pack(w, wk.S, c.b.images, c.st);
+}
+const uint8_t* mlp_image(const Ctx& c, int s) { return fused_mlp(c.D, c.bf16) ? c.b.images + (size_t)s * train_mlp::image_bytes() : nullptr; }
 
 }  // namespace
 
@@ -1962,7 +2009,7 @@ int trunk_sequence_fwd_train(const TrunkFwdTrainArgs& a) {
   if (rc) return rc;
   if (wk.R == 0) return BNB_OK;
   const int D = wk.D;
-  Ctx c;
+  Ctx c{};
   c.D = D; c.H = a.H; c.bf16 = a.bf16_products; c.st = a.stream;
   static thread_local Kept kept;
   if ((rc = open_buffers(c, &kept, wk, a.n_blocks, a.n_spatial, a.n_temporal, a.scratch, a.scratch_bytes, a.kept, a.kept_bytes)))
@@ -1971,10 +2018,12 @@ int trunk_sequence_fwd_train(const TrunkFwdTrainArgs& a) {
     cudaMemcpyAsync(a.y, a.x, wk.R * D * sizeof(float), cudaMemcpyDeviceToDevice, a.stream);
     return BNB_OK;
   }
+  if ((rc = prepare_mlps(c, wk, a.spatial, a.temporal, a.n_blocks, a.n_spatial, a.n_temporal))) return rc;
   const float* cur = a.x;
   int s = 0;
   for (int blk = 0; blk < a.n_blocks; ++blk) {
     for (int j = 0; j < a.n_spatial; ++j, ++s) {
+      c.mlp_image = mlp_image(c, s);
       float* out = s + 1 == wk.S ? a.y : kept.bound + (size_t)s * wk.R * D;
       Ctx cs = c;
       cs.b = kept.first[s];
@@ -1982,6 +2031,7 @@ int trunk_sequence_fwd_train(const TrunkFwdTrainArgs& a) {
       cur = out;
     }
     for (int j = 0; j < a.n_temporal; ++j, ++s) {
+      c.mlp_image = mlp_image(c, s);
       float* out = s + 1 == wk.S ? a.y : kept.bound + (size_t)s * wk.R * D;
       const int slot = blk * a.n_temporal + j;
       const size_t hoff = (size_t)slot * wk.Rr * 4 * D;
@@ -2005,7 +2055,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
   const int D = wk.D, S = wk.S, G = wk.G, NM = wk.NM;
   const size_t R = wk.R, Rr = wk.Rr;
   cudaStream_t st = a.stream;
-  Ctx c;
+  Ctx c{};
   c.D = D; c.H = a.H; c.bf16 = a.bf16_products; c.st = st;
   static thread_local Kept kept;
   const bool have_fwd = a.kept != nullptr;
@@ -2017,6 +2067,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
     return BNB_OK;
   }
 
+  if ((rc = prepare_mlps(c, wk, a.spatial, a.temporal, a.n_blocks, a.n_spatial, a.n_temporal))) return rc;
   // the input of every sublayer: kept by the training forward, or from a first pass here
   const float* inputs[256];
   if (have_fwd) {
@@ -2028,6 +2079,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
       for (int j = 0; j < a.n_spatial; ++j, ++s) {
         inputs[s] = cur;
         if (s + 1 == S) break;
+        c.mlp_image = mlp_image(c, s);
         float* out = c.b.bound + (size_t)s * R * D;
         spatial_fwd(c, a.spatial[blk * a.n_spatial + j], cur, a.alive, a.bullets, out, G, NM);
         cur = out;
@@ -2035,6 +2087,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
       for (int j = 0; j < a.n_temporal; ++j, ++s) {
         inputs[s] = cur;
         if (s + 1 == S) break;
+        c.mlp_image = mlp_image(c, s);
         float* out = c.b.bound + (size_t)s * R * D;
         const int slot = blk * a.n_temporal + j;
         rc = temporal_fwd(c, c, a.temporal[slot], cur, a.hidden_in + (size_t)slot * Rr * 4 * D, a.done, out, nullptr, wk.tgm);
@@ -2054,6 +2107,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
       float* dout = s == 0 ? a.dx : c.b.ping[s & 1];
       const int slot = blk * a.n_temporal + j;
       const size_t hoff = (size_t)slot * Rr * 4 * D;
+      c.mlp_image = mlp_image(c, s);
       Ctx cs = c, cf = c;
       if (have_fwd) {
         cs.b = kept.first[s];
@@ -2069,6 +2123,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
       const int s = blk * (a.n_spatial + a.n_temporal) + j;
       float* dout = s == 0 ? a.dx : c.b.ping[s & 1];
       const int k = blk * a.n_spatial + j;
+      c.mlp_image = mlp_image(c, s);
       Ctx cs = c;
       if (have_fwd) cs.b = kept.first[s];
       rc = spatial_bwd(cs, a.spatial[k], a.d_spatial[k], inputs[s], a.alive, a.bullets, a.d_bullets, dcur, dout, G, NM,

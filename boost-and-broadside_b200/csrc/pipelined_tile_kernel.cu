@@ -130,10 +130,6 @@ __device__ __forceinline__ uint4 sched_entry(int slot, const uint8_t* image, int
 }
 constexpr int MAX_SCHED = MAX_SUBLAYERS * 22;
 
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
 // Ring operations of a sublayer in the order the issuing warp consumes them.  All three roles walk the
 // same order with the same slot rotation.  GatedMLP with image base b: gate|up of chunk c are chunks
 // b + 3c, b + 3c + 1 (a pair), its down projection is b + 3c + 2 (a single); the three-deep pipeline
@@ -792,13 +788,6 @@ struct Issuer {
   volatile int* aborted;
 };
 
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
-  return p;
-}
-__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
-
 __device__ __forceinline__ void wait_operand(Issuer& m, int bar) {
   T_BEGIN();
   mbar_wait(m.bars + 8 * bar, (m.op_par >> bar) & 1u, m.status, m.aborted, ST_TIMEOUT_OPERAND);
@@ -807,36 +796,7 @@ __device__ __forceinline__ void wait_operand(Issuer& m, int bar) {
   T_END(m.tacc, TM_OP_WAIT);
   TRACE(m.tr, 400 + bar);
 }
-// tcgen05.mma with the shared-memory descriptors built from 32-bit halves inside the asm block
-// (K-major, 128-byte swizzle, 8-row groups 1024 B apart: the high word is a constant); A in shared
-// memory, or (TMEM_A) in tensor memory: lane = row, a 32-bit column = two consecutive k as bfloat16.
-__device__ __forceinline__ uint32_t desc_lo(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); }
-template <bool TMEM_A>
-__device__ __forceinline__ void mma_one(uint32_t elected, uint32_t d_tmem, uint32_t a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
-  if constexpr (TMEM_A)
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
-        "mov.b64 db, {%2, %5};\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0x40004040u), "r"(elected) : "memory");
-  else
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-        "mov.b64 da, {%1, %5};\n\t"
-        "mov.b64 db, {%2, %5};\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0x40004040u), "r"(elected) : "memory");
-}
-__device__ __forceinline__ void commit_one(const Issuer& m, uint32_t bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      ::"r"(m.bars + 8 * bar), "r"(m.elected) : "memory");
-}
+__device__ __forceinline__ void commit_one(const Issuer& m, uint32_t bar) { tc_commit_if(m.elected, m.bars + 8 * bar); }
 // Waits for the weights of a slot; returns the low descriptor word of its first chunk.
 __device__ __forceinline__ uint32_t wait_weights(Issuer& m, uint32_t slot) {
   T_MARK(tw);

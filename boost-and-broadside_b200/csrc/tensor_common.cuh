@@ -312,6 +312,51 @@ __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v 
 // 128-row x 64-column bf16 atom with the 128-byte swizzle.
 __device__ __forceinline__ uint32_t swz(int r, int c8) { return (uint32_t)(r * 128 + ((c8 ^ (r & 7)) << 4)); }
 
+// ------------------------------------------------------------------ issuing from a whole warp
+//
+// A warp that issues tensor-core work runs with the same values in every lane and lets one elected lane
+// execute the instruction: its operands then stay in uniform registers.
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p;
+}
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+// tcgen05.mma with the shared-memory descriptors built from 32-bit halves inside the asm block
+// (K-major, 128-byte swizzle, 8-row groups 1024 B apart: the high word is a constant); A in shared
+// memory, or (TMEM_A) in tensor memory: lane = row, a 32-bit column = two consecutive k as bfloat16.
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); }
+template <bool TMEM_A>
+__device__ __forceinline__ void mma_one(uint32_t elected, uint32_t d_tmem, uint32_t a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (TMEM_A)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
+        "mov.b64 db, {%2, %5};\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0x40004040u), "r"(elected) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %5};\n\t"
+        "mov.b64 db, {%2, %5};\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(0x40004040u), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(uint32_t elected, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(bar), "r"(elected) : "memory");
+}
+
 // The fused one-CTA-per-SM kernel (pipelined_tile_kernel.cu): programs of whole-environment tiles
 // made of SUB_SPATIAL and SUB_TEMPORAL sublayers only.
 int launch_pipelined(const TrunkArgs& a, cudaStream_t st);

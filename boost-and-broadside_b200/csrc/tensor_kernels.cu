@@ -1636,7 +1636,7 @@ void latch_status(int dev) {
 
 // Device address of the host word of the current device, allocating it on the first call (null
 // during a stream capture without it: that capture's launches then report to their scratch only).
-static int* host_status_word(cudaStream_t st) {
+int* host_status_word(cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
   std::lock_guard<std::mutex> lock(g_status_mutex);

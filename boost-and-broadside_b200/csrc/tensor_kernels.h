@@ -34,6 +34,7 @@ int pack_trunk(const BnbSpatialWeights* spatial, int n_spatial, const BnbTempora
 // (sticky until cleared); and the test hooks that make a wait run out.
 int last_status();
 void clear_status();
+int* host_status_word(cudaStream_t st);   // device address of that word, or null (see tensor_kernels.cu)
 void debug_wait_test(int skip_op, int poll_limit);
 
 int spatial_block(const BnbSpatialWeights& w, int D, int H, const float* x, const uint8_t* alive,
