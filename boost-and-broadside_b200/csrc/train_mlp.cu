@@ -1,6 +1,6 @@
 // The GatedMLP of the training path: y = x + down(gelu(gate n) * up n) with n = rmsnorm(x) * gain, and its
-// gradient, under the bfloat16 contract (every product's operands bfloat16, float32 accumulation; gate, up,
-// gelu, their product and the gradients of gate and up rounded to bfloat16), d_model 128, hidden 512.
+// gradient, under the bfloat16 contract (every product's operands bfloat16, float32 accumulation; what lies
+// between two products is float32 and rounded once, where it becomes an operand), d_model 128, hidden 512.
 // models/yemong/attention.py:21-37 under autocast; norms and residual stream float32.
 //
 // Nothing 4 d_model wide leaves the chip.  As separate products, gate, up, their product and its
@@ -125,22 +125,30 @@ __device__ __forceinline__ float rcp_fast(float v) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
   return r;
 }
-// Phi(x) and exp(-x^2 / 2): erf by formula 7.1.26 of Abramowitz and Stegun (absolute error 1.5e-7), whose
-// exponential is the density's too.
-__device__ __forceinline__ float normal_cdf(float x, float& e) {
-  const float t = rcp_fast(fmaf(fabsf(x), 0.3275911f * 0.70710678f, 1.0f));
-  e = ex2_fast(x * x * -0.72134752f);    // log2(e) / 2
-  float p = fmaf(t, 1.061405429f, -1.453152027f);
-  p = fmaf(t, p, 1.421413741f);
-  p = fmaf(t, p, -0.284496736f);
-  p = fmaf(t, p, 0.254829592f);
-  const float half = 0.5f * p * t * e;
-  return x >= 0.f ? 1.0f - half : half;
+// Two floats in one 64-bit register pair: one instruction for two multiply-adds.
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float lo, float hi) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ F2 f2(float both) { return f2(both, both); }
+__device__ __forceinline__ float2 split(F2 a) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v)); return r; }
+__device__ __forceinline__ F2 mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+// Phi(x) and exp(-x^2 / 2) for two x: erf by formula 7.1.26 of Abramowitz and Stegun (absolute error 1.5e-7),
+// whose exponential is the density's too.
+__device__ __forceinline__ F2 normal_cdf(F2 x, F2& e) {
+  const float2 xs = split(x);
+  const float2 d = split(fma(f2(fabsf(xs.x), fabsf(xs.y)), f2(0.3275911f * 0.70710678f), f2(1.0f)));
+  const F2 t = f2(rcp_fast(d.x), rcp_fast(d.y));
+  const float2 q = split(mul(mul(x, x), f2(-0.72134752f)));   // log2(e) / 2
+  e = f2(ex2_fast(q.x), ex2_fast(q.y));
+  F2 p = fma(t, f2(0.5f * 1.061405429f), f2(0.5f * -1.453152027f));
+  p = fma(t, p, f2(0.5f * 1.421413741f));
+  p = fma(t, p, f2(0.5f * -0.284496736f));
+  p = fma(t, p, f2(0.5f * 0.254829592f));
+  const float2 half = split(mul(mul(p, t), e));               // (1 - erf(|x| / sqrt 2)) / 2
+  return f2(xs.x >= 0.f ? 1.0f - half.x : half.x, xs.y >= 0.f ? 1.0f - half.y : half.y);
 }
-__device__ __forceinline__ float2 round2(float a, float b) {
-  const uint32_t w = pack_bf16(a, b);
-  return make_float2(bf16_lo(w), bf16_hi(w));
-}
+__device__ __forceinline__ uint32_t pack_f2(F2 a) { const float2 v = split(a); return pack_bf16(v.x, v.y); }
+__device__ __forceinline__ F2 acc_pair(const uint32_t* v) { return f2(__uint_as_float(v[0]), __uint_as_float(v[1])); }
 // The epilogue warps' arrival on an operand barrier.
 __device__ __forceinline__ void post(const Sync& s, int bar) {
   fence_proxy_async();
@@ -149,33 +157,73 @@ __device__ __forceinline__ void post(const Sync& s, int bar) {
   if ((threadIdx.x & 31) == 0) mbar_arrive(s.bars + 8 * bar);
 }
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
-// Sum over the four threads of a row (the four warps of 32 rows meet at a barrier of their own).
-__device__ __forceinline__ float row_sum(float v, float* part_sums, int row, int part) {
-  part_sums[part * TILE + row] = v;
-  asm volatile("bar.sync %0, 128;" ::"r"(3 + ((threadIdx.x >> 5) & 3)) : "memory");
-  const float s = (part_sums[row] + part_sums[TILE + row]) + (part_sums[2 * TILE + row] + part_sums[3 * TILE + row]);
-  asm volatile("bar.sync %0, 128;" ::"r"(3 + ((threadIdx.x >> 5) & 3)) : "memory");   // before the next use
-  return s;
+// Rows move between global memory and the warps in a layout of their own: warp w owns rows 32 (w % 4) .. and
+// columns 32 (w / 4) .., and in its i-th request (i < 8) lane l takes the sixteen bytes at row 4 i + l / 8,
+// columns 4 (l % 8).. : a request touches four lines.  (With a thread per tile row, as tensor memory has it, each
+// request touched 32 lines, and the loads and stores alone took 25 000 of a tile's 67 000 cycles.)
+struct RowMap {
+  int lane, row0, col;     // first tile row and this lane's first column
+  __device__ __forceinline__ int row(int i) const { return row0 + 4 * i + (lane >> 3); }
+};
+__device__ __forceinline__ RowMap row_map() {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  return {lane, 32 * (warp & 3), 32 * (warp >> 2) + 4 * (lane & 7)};
 }
-// 32 consecutive floats of a row; invalid rows read zeros
-__device__ __forceinline__ void load_row(float (&v)[32], const float* src, bool valid) {
+__device__ __forceinline__ void rows_in(float4 (&v)[8], const float* src, const RowMap& m, int first, int rows) {
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid) f = *reinterpret_cast<const float4*>(src + 4 * q);
-    v[4 * q] = f.x; v[4 * q + 1] = f.y; v[4 * q + 2] = f.z; v[4 * q + 3] = f.w;
+  for (int i = 0; i < 8; ++i) {
+    const int r = first + m.row(i);
+    v[i] = r < rows ? *reinterpret_cast<const float4*>(src + (size_t)r * D + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
-// n = bf16(x inv gain) of this thread's 32 columns into an operand tile
-__device__ __forceinline__ void store_normed(uint8_t* tile, const float (&x)[32], float inv, const float* gain, int row, int part) {
+// Per-row sums of one value per request: over the eight lanes of a row here, over the four column parts
+// through shared memory.  Returns the totals of this lane's rows; two barriers of the four warps of these rows.
+__device__ __forceinline__ void row_sums(float (&v)[8], float* part_sums, const RowMap& m) {
+  const int part = threadIdx.x >> 7, bar = 3 + ((threadIdx.x >> 5) & 3);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const float4 ga = *reinterpret_cast<const float4*>(gain + part * 32 + q * 8), gb = *reinterpret_cast<const float4*>(gain + part * 32 + q * 8 + 4);
-    const float* s = &x[q * 8];
-    const int col = part * 32 + q * 8;
-    *reinterpret_cast<uint4*>(tile + (col >> 6) * CHUNK_BYTES + swz(row, (col & 63) >> 3)) =
-        make_uint4(pack_bf16(s[0] * inv * ga.x, s[1] * inv * ga.y), pack_bf16(s[2] * inv * ga.z, s[3] * inv * ga.w),
-                   pack_bf16(s[4] * inv * gb.x, s[5] * inv * gb.y), pack_bf16(s[6] * inv * gb.z, s[7] * inv * gb.w));
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+  if ((m.lane & 7) == 0)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) part_sums[part * TILE + m.row(i)] = v[i];
+  asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float* p = part_sums + m.row(i);
+    v[i] = (p[0] + p[TILE]) + (p[2 * TILE] + p[3 * TILE]);
+  }
+  asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");   // before the next use
+}
+// four values as bfloat16 into an operand tile
+__device__ __forceinline__ void put4(uint8_t* tile, int row, int col, float a, float b, float c, float d) {
+  *reinterpret_cast<uint2*>(tile + (col >> 6) * CHUNK_BYTES + swz(row, (col & 63) >> 3) + ((col >> 2) & 1) * 8) = make_uint2(pack_bf16(a, b), pack_bf16(c, d));
+}
+// n = bf16(x inv gain) into an operand tile; inv[i] of this lane's rows on the way
+__device__ __forceinline__ void norm_rows(uint8_t* tile, const float4 (&x)[8], float (&inv)[8], const float4& gain, float* part_sums, const RowMap& m) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) inv[i] = fmaf(x[i].x, x[i].x, fmaf(x[i].y, x[i].y, fmaf(x[i].z, x[i].z, x[i].w * x[i].w)));
+  row_sums(inv, part_sums, m);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    inv[i] = rsqrtf(inv[i] * (1.0f / D) + kRmsEps);
+    put4(tile, m.row(i), m.col, x[i].x * inv[i] * gain.x, x[i].y * inv[i] * gain.y, x[i].z * inv[i] * gain.z, x[i].w * inv[i] * gain.w);
+  }
+}
+// 32 accumulator columns from the thread-per-row layout of tensor memory to the row layout, through 4 KB of
+// shared memory of the warp's own.
+__device__ __forceinline__ void transpose_rows(float4 (&v)[8], uint32_t taddr, uint8_t* stage, const RowMap& m) {
+  uint32_t t[32];
+  tmem_ld32(taddr, t);
+  const int r = m.lane;
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    *reinterpret_cast<uint4*>(stage + r * 128 + ((q ^ (r & 7)) << 4)) = make_uint4(t[4 * q], t[4 * q + 1], t[4 * q + 2], t[4 * q + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int rr = 4 * i + (m.lane >> 3);
+    v[i] = *reinterpret_cast<const float4*>(stage + rr * 128 + (((m.lane & 7) ^ (rr & 7)) << 4));
   }
 }
 
@@ -242,19 +290,20 @@ __device__ __forceinline__ void product128(uint32_t el, uint32_t d, uint32_t a, 
 
 // ------------------------------------------------------------------ forward
 
-// Shared memory: n (32 KB), three gate|up slots (32 KB), three down slots (16 KB), row sums, gain, frame.
-constexpr uint32_t FW_PAIR = 32768, FW_SINGLE = FW_PAIR + 3 * 32768, FW_SUMS = FW_SINGLE + 3 * 16384, FW_GAIN = FW_SUMS + 2048,
-                   FW_FRAME = FW_GAIN + 512, FW_BYTES = FW_FRAME + FRAME_BYTES;
+// Shared memory: n (32 KB), three gate|up slots (32 KB), three down slots (16 KB), row sums, frame.
+constexpr uint32_t FW_PAIR = 32768, FW_SINGLE = FW_PAIR + 3 * 32768, FW_SUMS = FW_SINGLE + 3 * 16384, FW_FRAME = FW_SUMS + 2048,
+                   FW_BYTES = FW_FRAME + FRAME_BYTES;
 enum : int { FB_OP = 0, FB_FFN0, FB_ACC = FB_FFN0 + 3, FB_DRAIN, FB_FULL0, FB_DONE0 = FB_FULL0 + 6, FB_COUNT = FB_DONE0 + 6 };
 
 __device__ __forceinline__ uint32_t fw_slot(uint32_t i) { return i < 3 ? FW_PAIR + i * 32768 : FW_SINGLE + (i - 3) * 16384; }
 
-// Tensor memory: residual [0, 128), three gate|up accumulators.
+// Tensor memory: down projection [0, 128), three gate|up accumulators.  The output transpose stages in the
+// operand area, free once a tile's products are complete (the ring behind it may be refilling): 4 KB per warp,
+// eight warps at a time.
 __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ Args a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int counts[FB_COUNT] = {EPI_WARPS, EPI_WARPS / 2, EPI_WARPS / 2, EPI_WARPS / 2, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
   const int tid = threadIdx.x, warp = tid >> 5;
-  if (tid < D) reinterpret_cast<float*>(smem + FW_GAIN)[tid] = a.gain[tid];
   const Frame f = open_frame(smem + FW_FRAME, a, counts);
   const Sync s{smem_u32(f.bars), a.status, f.aborted};
   const uint32_t tmem = *f.tmem_slot;
@@ -305,7 +354,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
         full ^= 1u << single;
         const uint32_t b = uniform(desc_lo(base + FW_SINGLE + (single - 3) * 16384));
 #pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) mma_one<true>(el, tm, tm + 128 + 128 * acc + 16 * k, b + 2 * k, idesc, 1u);
+        for (uint32_t k = 0; k < 4; ++k) mma_one<true>(el, tm, tm + 128 + 128 * acc + 16 * k, b + 2 * k, idesc, (c | k) ? 1u : 0u);
         tc_commit_if(el, s.bars + 8 * (FB_DONE0 + single));
         single = single == 5 ? 3 : single + 1;
         if (c + 3 < 8) gate_up(acc);
@@ -317,20 +366,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
     for (int i = 0; i < DEFAULT_POLL_LIMIT && !mbar_try_wait(s.bars + 8 * FB_DRAIN, 0); ++i) {
     }
   } else {
-    const int row = tid & (TILE - 1), part = tid >> 7, group = part >> 1, half = part & 1;
+    const int part = tid >> 7, group = part >> 1, half = part & 1;
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     uint32_t pair = 0, par = 0, acc_par = 0;
+    const RowMap m = row_map();
+    const float4 gain = *reinterpret_cast<const float4*>(a.gain + m.col);
     for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
-      const int r = tile * TILE + row;
-      const bool valid = r < a.rows;
+      epi_sync();   // every warp is done with the operand area of the previous tile
       {
-        float x[32], ss = 0.f;
-        load_row(x, a.x1 + (size_t)r * D + part * 32, valid);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) ss = fmaf(x[i], x[i], ss);
-        tmem_st32(lane_addr + part * 32, reinterpret_cast<uint32_t(&)[32]>(x));
-        ss = row_sum(ss, reinterpret_cast<float*>(smem + FW_SUMS), row, part);
-        store_normed(smem, x, rsqrtf(ss * (1.0f / D) + kRmsEps), reinterpret_cast<const float*>(smem + FW_GAIN), row, part);
+        float4 x[8];
+        float inv[8];
+        rows_in(x, a.x1, m, tile * TILE, a.rows);
+        norm_rows(smem, x, inv, gain, reinterpret_cast<float*>(smem + FW_SUMS), m);
       }
       post(s, FB_OP);
 #pragma unroll 1
@@ -347,11 +394,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
             tmem_wait_ld();
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-              const float2 gv = round2(__uint_as_float(g[2 * j]), __uint_as_float(g[2 * j + 1]));
-              const float2 uv = round2(__uint_as_float(u[2 * j]), __uint_as_float(u[2 * j + 1]));
-              float e;
-              const float2 h = round2(gv.x * normal_cdf(gv.x, e), gv.y * normal_cdf(gv.y, e));
-              w[j] = pack_bf16(h.x * uv.x, h.y * uv.y);
+              const F2 x = acc_pair(&g[2 * j]);
+              F2 e;
+              w[j] = pack_f2(mul(mul(x, normal_cdf(x, e)), acc_pair(&u[2 * j])));
             }
             tmem_st8_nowait(acc + 16 * p, w);
           }
@@ -364,12 +409,19 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
       s.wait(FB_ACC, acc_par, TIMEOUT_ACC);
       acc_par ^= 1u;
       tc_fence_after();
-      uint32_t v[32];
-      tmem_ld32(lane_addr + part * 32, v);
-      if (valid)
+      // y = x + down, row layout; the first eight warps stage in the operand area, then the others
+      float4 x[8], d[8];
+      rows_in(x, a.x1, m, tile * TILE, a.rows);
+      if (group == 0) transpose_rows(d, lane_addr + part * 32, smem + (warp & 7) * 4096, m);
+      epi_sync();
+      if (group == 1) transpose_rows(d, lane_addr + part * 32, smem + (warp & 7) * 4096, m);
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          *reinterpret_cast<uint4*>(a.out + (size_t)r * D + part * 32 + 4 * q) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      for (int i = 0; i < 8; ++i) {
+        const int r = tile * TILE + m.row(i);
+        if (r < a.rows)
+          *reinterpret_cast<float4*>(a.out + (size_t)r * D + m.col) = make_float4(x[i].x + d[i].x, x[i].y + d[i].y, x[i].z + d[i].z, x[i].w + d[i].w);
+      }
+      tc_fence_before();
     }
   }
   close_frame(f, tmem);
@@ -378,9 +430,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
 // ------------------------------------------------------------------ gradient of the input
 
 // Shared memory: n and dy (32 KB each), two slots of gate|up and transposed down (48 KB), two of transposed
-// gate and up (32 KB), row sums, gain, frame.
-constexpr uint32_t DX_DY = 32768, DX_W1 = 65536, DX_W2 = DX_W1 + 2 * 49152, DX_SUMS = DX_W2 + 2 * 32768, DX_GAIN = DX_SUMS + 2048,
-                   DX_FRAME = DX_GAIN + 512, DX_BYTES = DX_FRAME + FRAME_BYTES;
+// gate and up (32 KB), row sums, frame.
+constexpr uint32_t DX_DY = 32768, DX_W1 = 65536, DX_W2 = DX_W1 + 2 * 49152, DX_SUMS = DX_W2 + 2 * 32768, DX_FRAME = DX_SUMS + 2048,
+                   DX_BYTES = DX_FRAME + FRAME_BYTES;
 enum : int { XB_OP = 0, XB_FF0, XB_ACC = XB_FF0 + 2, XB_DRAIN, XB_FULL1, XB_DONE1 = XB_FULL1 + 2, XB_FULL2 = XB_DONE1 + 2, XB_DONE2 = XB_FULL2 + 2, XB_COUNT = XB_DONE2 + 2 };
 // Tensor memory: dn [0, 128), two accumulator sets of gate|up (128 columns) and d h (64).
 __device__ __forceinline__ uint32_t dx_acc(uint32_t i) { return 128 + 192 * i; }
@@ -389,8 +441,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
   extern __shared__ __align__(1024) uint8_t smem[];
   const int counts[XB_COUNT] = {EPI_WARPS, EPI_WARPS / 2, EPI_WARPS / 2, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
   const int tid = threadIdx.x, warp = tid >> 5;
-  float* gain = reinterpret_cast<float*>(smem + DX_GAIN);
-  if (tid < D) gain[tid] = a.gain[tid];
   const Frame f = open_frame(smem + DX_FRAME, a, counts);
   const Sync s{smem_u32(f.bars), a.status, f.aborted};
   const uint32_t tmem = *f.tmem_slot;
@@ -458,36 +508,26 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
     for (int i = 0; i < DEFAULT_POLL_LIMIT && !mbar_try_wait(s.bars + 8 * XB_DRAIN, 0); ++i) {
     }
   } else {
-    const int row = tid & (TILE - 1), part = tid >> 7, group = part >> 1, half = part & 1, lane = tid & 31;
+    const int part = tid >> 7, group = part >> 1, half = part & 1;
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     float* sums = reinterpret_cast<float*>(smem + DX_SUMS);
     uint32_t par = 0, acc_par = 0;
-    float gsum[4] = {0.f, 0.f, 0.f, 0.f};   // gain gradient of columns 32 part + 8 q + (lane & 7), rows 4-interleaved
+    const RowMap m = row_map();
+    const float4 gain = *reinterpret_cast<const float4*>(a.gain + m.col);
+    float4 gsum = make_float4(0.f, 0.f, 0.f, 0.f);   // gain gradient of this lane's columns
     for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
-      const int r = tile * TILE + row;
-      const bool valid = r < a.rows;
-      const float* xr = a.x1 + (size_t)r * D + part * 32;
-      const float* dr = a.dy + (size_t)r * D + part * 32;
-      float inv;
-      // the operand tiles of the previous round are on their way to global memory: wait until they are read
+      float inv[8];
+      // the operand area: its tiles on their way to global memory are read, the transposes of the previous
+      // round done
       if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
       epi_sync();
       {
-        float x[32], ss = 0.f;
-        load_row(x, xr, valid);
+        float4 x[8];
+        rows_in(x, a.x1, m, tile * TILE, a.rows);
+        norm_rows(smem, x, inv, gain, sums, m);
+        rows_in(x, a.dy, m, tile * TILE, a.rows);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) ss = fmaf(x[i], x[i], ss);
-        ss = row_sum(ss, sums, row, part);
-        inv = rsqrtf(ss * (1.0f / D) + kRmsEps);
-        store_normed(smem, x, inv, gain, row, part);
-        load_row(x, dr, valid);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int col = part * 32 + q * 8;
-          *reinterpret_cast<uint4*>(smem + DX_DY + (col >> 6) * CHUNK_BYTES + swz(row, (col & 63) >> 3)) =
-              make_uint4(pack_bf16(x[8 * q], x[8 * q + 1]), pack_bf16(x[8 * q + 2], x[8 * q + 3]), pack_bf16(x[8 * q + 4], x[8 * q + 5]),
-                         pack_bf16(x[8 * q + 6], x[8 * q + 7]));
-        }
+        for (int i = 0; i < 8; ++i) put4(smem + DX_DY, m.row(i), m.col, x[i].x, x[i].y, x[i].z, x[i].w);
       }
       post(s, XB_OP);
       epi_sync();
@@ -512,14 +552,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
           tmem_wait_ld();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float2 gv = round2(__uint_as_float(g[2 * j]), __uint_as_float(g[2 * j + 1]));
-            const float2 uv = round2(__uint_as_float(u[2 * j]), __uint_as_float(u[2 * j + 1]));
-            const float2 hv = round2(__uint_as_float(h[2 * j]), __uint_as_float(h[2 * j + 1]));
-            float e0, e1;
-            const float c0 = normal_cdf(gv.x, e0), c1 = normal_cdf(gv.y, e1);
-            // gelu' = Phi + g phi
-            wg[j] = pack_bf16(hv.x * uv.x * fmaf(gv.x * 0.39894228f, e0, c0), hv.y * uv.y * fmaf(gv.y * 0.39894228f, e1, c1));
-            wu[j] = pack_bf16(hv.x * (gv.x * c0), hv.y * (gv.y * c1));
+            const F2 x = acc_pair(&g[2 * j]), dh = acc_pair(&h[2 * j]);
+            F2 e;
+            const F2 cdf = normal_cdf(x, e);
+            // gelu' = Phi + x phi
+            wg[j] = pack_f2(mul(mul(dh, acc_pair(&u[2 * j])), fma(mul(x, f2(0.39894228f)), e, cdf)));
+            wu[j] = pack_f2(mul(dh, mul(x, cdf)));
           }
           tmem_st8_nowait(acc + 16 * p, wg);
           tmem_st8_nowait(acc + 64 + 16 * p, wu);
@@ -530,68 +568,40 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
       s.wait(XB_ACC, acc_par, TIMEOUT_ACC);
       acc_par ^= 1u;
       tc_fence_after();
-      // the norm: dx = dy + inv gain dn - x inv^3 mean(x gain dn);  d gain += sum over rows of dn x inv
-      float dot = 0.f;
-#pragma unroll 1
-      for (int q = 0; q < 4; ++q) {
-        uint32_t v[8];
-        tmem_ld8_nowait(lane_addr + part * 32 + 8 * q, v);
-        float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
-        if (valid) {
-          x0 = *reinterpret_cast<const float4*>(xr + 8 * q);
-          x1 = *reinterpret_cast<const float4*>(xr + 8 * q + 4);
-        }
-        const float4 g0 = *reinterpret_cast<const float4*>(gain + part * 32 + 8 * q), g1 = *reinterpret_cast<const float4*>(gain + part * 32 + 8 * q + 4);
-        tmem_wait_ld();
-        const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+      // the norm: dx = dy + inv gain dn - x inv^3 mean(x gain dn);  d gain += sum over rows of dn x inv.  The operand
+      // area (64 KB, 4 KB per warp) stages the transpose once its copies to global memory have read it.
+      if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      epi_sync();
+      float4 x[8], dn[8];
+      rows_in(x, a.x1, m, tile * TILE, a.rows);
+      transpose_rows(dn, lane_addr + part * 32, smem + warp * 4096, m);
+      tc_fence_before();
+      float coef[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) dot = fmaf(x[j] * g[j], __uint_as_float(v[j]), dot);
-      }
-      dot = row_sum(dot, sums, row, part);
-      const float coef = dot * inv * inv * inv * (1.0f / D);
+      for (int i = 0; i < 8; ++i)
+        coef[i] = fmaf(x[i].x * gain.x, dn[i].x, fmaf(x[i].y * gain.y, dn[i].y, fmaf(x[i].z * gain.z, dn[i].z, x[i].w * gain.w * dn[i].w)));
+      row_sums(coef, sums, m);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t v[8];
-        tmem_ld8_nowait(lane_addr + part * 32 + 8 * q, v);
-        float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0, d0 = x0, d1 = x0;
-        if (valid) {
-          x0 = *reinterpret_cast<const float4*>(xr + 8 * q);
-          x1 = *reinterpret_cast<const float4*>(xr + 8 * q + 4);
-          d0 = *reinterpret_cast<const float4*>(dr + 8 * q);
-          d1 = *reinterpret_cast<const float4*>(dr + 8 * q + 4);
-        }
-        const float4 g0 = *reinterpret_cast<const float4*>(gain + part * 32 + 8 * q), g1 = *reinterpret_cast<const float4*>(gain + part * 32 + 8 * q + 4);
-        tmem_wait_ld();
-        const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w},
-                    d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-        float o[8], w[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float dn = __uint_as_float(v[j]);
-          o[j] = d[j] + inv * g[j] * dn - x[j] * coef;
-          w[j] = dn * x[j] * inv;
-        }
-        if (valid) {
-          *reinterpret_cast<float4*>(a.out + (size_t)r * D + part * 32 + 8 * q) = make_float4(o[0], o[1], o[2], o[3]);
-          *reinterpret_cast<float4*>(a.out + (size_t)r * D + part * 32 + 8 * q + 4) = make_float4(o[4], o[5], o[6], o[7]);
-        }
-        // eight column sums over the warp's 32 rows, halving the columns a lane keeps: lane ends with column lane & 7
-        const bool b4 = lane & 4, b2 = lane & 2, b1 = lane & 1;
-        float p4[4], p2[2];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) p4[j] = (b4 ? w[4 + j] : w[j]) + __shfl_xor_sync(0xffffffffu, b4 ? w[j] : w[4 + j], 4);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) p2[j] = (b2 ? p4[2 + j] : p4[j]) + __shfl_xor_sync(0xffffffffu, b2 ? p4[j] : p4[2 + j], 2);
-        float p1 = (b1 ? p2[1] : p2[0]) + __shfl_xor_sync(0xffffffffu, b1 ? p2[0] : p2[1], 1);
-        gsum[q] += p1;
+      for (int i = 0; i < 8; ++i) {
+        const int r = tile * TILE + m.row(i);
+        if (r >= a.rows) continue;
+        const float iv = inv[i], k = coef[i] * iv * iv * iv * (1.0f / D);
+        const float4 d = *reinterpret_cast<const float4*>(a.dy + (size_t)r * D + m.col);
+        *reinterpret_cast<float4*>(a.out + (size_t)r * D + m.col) =
+            make_float4(d.x + iv * gain.x * dn[i].x - x[i].x * k, d.y + iv * gain.y * dn[i].y - x[i].y * k,
+                        d.z + iv * gain.z * dn[i].z - x[i].z * k, d.w + iv * gain.w * dn[i].w - x[i].w * k);
+        gsum.x = fmaf(dn[i].x * x[i].x, iv, gsum.x); gsum.y = fmaf(dn[i].y * x[i].y, iv, gsum.y);
+        gsum.z = fmaf(dn[i].z * x[i].z, iv, gsum.z); gsum.w = fmaf(dn[i].w * x[i].w, iv, gsum.w);
       }
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      gsum[q] += __shfl_xor_sync(0xffffffffu, gsum[q], 8);
-      gsum[q] += __shfl_xor_sync(0xffffffffu, gsum[q], 16);
-      if (lane < 8 && my_tiles > 0) atomicAdd(a.d_gain + part * 32 + 8 * q + lane, gsum[q]);
+    for (int o = 8; o < 32; o <<= 1) {
+      gsum.x += __shfl_xor_sync(0xffffffffu, gsum.x, o);
+      gsum.y += __shfl_xor_sync(0xffffffffu, gsum.y, o);
+      gsum.z += __shfl_xor_sync(0xffffffffu, gsum.z, o);
+      gsum.w += __shfl_xor_sync(0xffffffffu, gsum.w, o);
     }
+    if (m.lane < 8 && my_tiles > 0) atomicAdd(reinterpret_cast<float4*>(a.d_gain + m.col), gsum);
     if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   close_frame(f, tmem);
@@ -695,16 +705,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dw(const __grid_constant__ A
       uint32_t wg[8], wu[8], wh[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float2 gv = round2(__uint_as_float(g[2 * j]), __uint_as_float(g[2 * j + 1]));
-        const float2 uv = round2(__uint_as_float(u[2 * j]), __uint_as_float(u[2 * j + 1]));
-        const float2 hv = round2(__uint_as_float(h[2 * j]), __uint_as_float(h[2 * j + 1]));
-        float e0, e1;
-        const float c0 = normal_cdf(gv.x, e0), c1 = normal_cdf(gv.y, e1);
-        const float y0 = gv.x * c0, y1 = gv.y * c1;
-        const float2 yr = round2(y0, y1);
-        wg[j] = pack_bf16(hv.x * uv.x * fmaf(gv.x * 0.39894228f, e0, c0), hv.y * uv.y * fmaf(gv.y * 0.39894228f, e1, c1));
-        wu[j] = pack_bf16(hv.x * y0, hv.y * y1);
-        wh[j] = pack_bf16(yr.x * uv.x, yr.y * uv.y);
+        const F2 x = acc_pair(&g[2 * j]), up = acc_pair(&u[2 * j]), dh = acc_pair(&h[2 * j]);
+        F2 e;
+        const F2 cdf = normal_cdf(x, e), y = mul(x, cdf);
+        wg[j] = pack_f2(mul(mul(dh, up), fma(mul(x, f2(0.39894228f)), e, cdf)));
+        wu[j] = pack_f2(mul(dh, y));
+        wh[j] = pack_f2(mul(y, up));
       }
       if (i > 0) {   // the previous tile's operands have been read
         s.wait(WB_DONE0 + ((i - 1) & 1), done >> ((i - 1) & 1), TIMEOUT_ACC);
