@@ -11,8 +11,15 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <cstdlib>
+#include <cstring>
+#include <memory>
 #include <vector>
 
 #include "bnb_trunk.h"
@@ -338,6 +345,203 @@ std::tuple<Tensor, Tensor> trunk_forward(const Tensor& x, const OptTensor& alive
   return {y, hout};
 }
 
+// ------------------------------------------------------------------ the trunk under autograd
+
+int grad_precision(const Geometry& g) { return g.precision == BNB_BF16 ? BNB_BF16 : BNB_FP32; }
+
+// Whether a differentiated call keeps its activations (faster) or lets the backward recompute them:
+// BNB_GRAD_MODE=keep | recompute decides; otherwise keep when the kept buffer plus the backward's scratch
+// fit in 70 % of the memory that is free or cached.  What torch's allocator holds unused is looked at
+// first: the driver's own answer takes 0.1 ms.
+bool keep_activations(const c10::Device& dev, const Geometry& g, int64_t D, int64_t n_bullets) {
+  const char* env = std::getenv("BNB_GRAD_MODE");
+  const std::string mode = env ? env : "";
+  if (mode == "recompute") return false;
+  const c10::cuda::CUDAGuard guard(dev);
+  const BnbBatch b = g.batch({});
+  const int T = g.timesteps > 1 ? g.timesteps : 1;
+  size_t need = bnb_trunk_kept_bytes(g.blocks, g.spatial, g.temporal, (int)D, g.heads, &b, T, (int)n_bullets, grad_precision(g));
+  if (need == 0) return false;
+  if (mode == "keep") return true;
+  need += bnb_trunk_bwd_scratch_bytes(g.blocks, g.spatial, g.temporal, (int)D, &b, T, (int)n_bullets, grad_precision(g));
+  const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats(dev.index());
+  const double cached = (double)(stats.reserved_bytes[0].current - stats.allocated_bytes[0].current);
+  if ((double)need <= 0.7 * cached) return true;
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return false;
+  return (double)need <= 0.7 * ((double)free_bytes + cached);
+}
+
+template <class S>
+void fill_grads(S& out, const float* flat, const std::vector<Tensor>& ts, size_t& pos, int n, size_t& off) {
+  float** f = reinterpret_cast<float**>(&out);   // the struct is a row of float*
+  for (int k = 0; k < n; ++k) {
+    f[k] = const_cast<float*>(flat) + off;
+    off += ((size_t)ts[pos++].numel() + 3) / 4 * 4;   // 16-byte granules
+  }
+}
+
+struct BackwardResult { Tensor dx, dh, dbul, flat; };
+// bnb_b200::trunk_backward (yemong/_ops.py).
+BackwardResult run_backward(const Tensor& dy, const OptTensor& dhidden, const OptTensor& kept, const Tensor& x, const OptTensor& alive,
+                            const Tensor& hidden, const OptTensor& done, const OptTensor& bullets, const OptTensor& mask,
+                            const std::vector<Tensor>& weights, const std::vector<int64_t>& geom) {
+  const Geometry g(geom);
+  const c10::Device dev = x.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const int D = (int)x.size(-1), T = g.timesteps > 1 ? g.timesteps : 1;
+  const BnbBatch batch = g.batch({});
+  const Tensor xin = f32c(x), hin = f32c(hidden), dyin = f32c(dy);
+  OptTensor dho;
+  if (dhidden.has_value() && dhidden->defined()) dho = f32c(*dhidden);
+  const OptTensor alive_u8 = bytes_of(alive), done_u8 = bytes_of(done);
+  const Weights w = weight_structs(g, weights, dev);
+  size_t total = 0;
+  for (const Tensor& t : weights) total += ((size_t)t.numel() + 3) / 4 * 4;
+  BackwardResult r;
+  // one zeroed buffer for every parameter gradient: the kernels accumulate into it
+  r.flat = at::zeros({(int64_t)total}, xin.options());
+  std::vector<BnbSpatialGrads> sg(w.spatial.size());
+  std::vector<BnbTemporalGrads> tg(w.temporal.size());
+  size_t pos = 0, off = 0;
+  const float* flat = static_cast<const float*>(r.flat.data_ptr());
+  for (int i = 0; i < g.blocks; ++i) {
+    for (int j = 0; j < g.spatial; ++j) {
+      BnbSpatialGrads& s = sg[(size_t)i * g.spatial + j];
+      s = BnbSpatialGrads{};
+      fill_grads(s, flat, weights, pos, N_SPATIAL + (j < g.bullet_cross ? 2 : 0), off);
+    }
+    for (int j = 0; j < g.temporal; ++j) {
+      BnbTemporalGrads& t = tg[(size_t)i * g.temporal + j];
+      t = BnbTemporalGrads{};
+      fill_grads(t, flat, weights, pos, N_TEMPORAL + (g.field_sub ? 1 : 0), off);
+    }
+  }
+  const Bullets b(g.bullet_cross > 0 ? bullets : c10::nullopt, mask, (int64_t)T * batch.n_envs, D, false);
+  r.dx = at::empty_like(xin);
+  r.dh = at::zeros_like(hin);
+  r.dbul = b.present ? at::empty_like(b.tokens) : at::empty({0}, xin.options());   // zeroed by the library
+  const size_t bytes = bnb_trunk_bwd_scratch_bytes(g.blocks, g.spatial, g.temporal, D, &batch, T, b.arg.per_env, grad_precision(g));
+  const Tensor scratch = at::empty({(int64_t)std::max<size_t>(bytes, 256)}, xin.options().dtype(at::kByte));   // released after the call's stream work
+  check("bnb_trunk_sequence_bwd",
+        bnb_trunk_sequence_bwd(w.spatial.data(), w.temporal.data(), sg.data(), tg.data(), g.blocks, g.spatial, g.temporal, D, g.heads,
+                               static_cast<const float*>(xin.data_ptr()), static_cast<const uint8_t*>(ptr(alive_u8)), b.get(),
+                               static_cast<const float*>(hin.data_ptr()), static_cast<const uint8_t*>(ptr(done_u8)), &batch, T, grad_precision(g),
+                               static_cast<const float*>(dyin.data_ptr()), static_cast<const float*>(ptr(dho)), static_cast<float*>(r.dx.data_ptr()),
+                               static_cast<float*>(r.dh.data_ptr()), b.present ? static_cast<float*>(r.dbul.data_ptr()) : nullptr,
+                               kept.has_value() ? kept->data_ptr() : nullptr, kept.has_value() ? (size_t)kept->numel() : 0, scratch.data_ptr(),
+                               (size_t)scratch.numel(), at::cuda::getCurrentCUDAStream(dev.index()).stream()));
+  return r;
+}
+std::vector<Tensor> trunk_backward(const Tensor& dy, const OptTensor& dhidden, const OptTensor& kept, const Tensor& x, const OptTensor& alive,
+                                   const Tensor& hidden, const OptTensor& done, const OptTensor& bullets, const OptTensor& mask,
+                                   const std::vector<Tensor>& weights, const std::vector<int64_t>& geom) {
+  const BackwardResult r = run_backward(dy, dhidden, kept, x, alive, hidden, done, bullets, mask, weights, geom);
+  return {r.dx, r.dh, r.dbul, r.flat};
+}
+
+// bnb_b200::trunk_forward_train (yemong/_ops.py): (y, new hidden, kept activations).
+std::tuple<Tensor, Tensor, Tensor> trunk_forward_train(const Tensor& x, const OptTensor& alive, const Tensor& hidden, const OptTensor& done,
+                                                       const OptTensor& bullets, const OptTensor& mask, const std::vector<Tensor>& weights,
+                                                       const std::vector<int64_t>& geom) {
+  const Geometry g(geom);
+  const c10::Device dev = x.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const int D = (int)x.size(-1), T = g.timesteps > 1 ? g.timesteps : 1;
+  const BnbBatch batch = g.batch({});
+  const Tensor xin = f32c(x), hin = f32c(hidden);
+  const OptTensor alive_u8 = bytes_of(alive), done_u8 = bytes_of(done);
+  const Weights w = weight_structs(g, weights, dev);
+  raise_pending_status(dev);
+  const Bullets b(g.bullet_cross > 0 ? bullets : c10::nullopt, mask, (int64_t)T * batch.n_envs, D, false);
+  Tensor y = at::empty_like(xin), hout = at::empty_like(hin);
+  const auto bytes = xin.options().dtype(at::kByte);
+  Tensor kept = at::empty({(int64_t)std::max<size_t>(256, bnb_trunk_kept_bytes(g.blocks, g.spatial, g.temporal, D, g.heads, &batch, T, b.arg.per_env, grad_precision(g)))}, bytes);
+  const size_t need = bnb_trunk_bwd_scratch_bytes(g.blocks, g.spatial, g.temporal, D, &batch, T, b.arg.per_env, grad_precision(g));
+  const Tensor scratch = at::empty({(int64_t)std::max<size_t>(need, 256)}, bytes);
+  check("bnb_trunk_sequence_fwd_train",
+        bnb_trunk_sequence_fwd_train(w.spatial.data(), w.temporal.data(), g.blocks, g.spatial, g.temporal, D, g.heads,
+                                     static_cast<const float*>(xin.data_ptr()), static_cast<const uint8_t*>(ptr(alive_u8)), b.get(),
+                                     static_cast<float*>(y.data_ptr()), static_cast<const float*>(hin.data_ptr()), static_cast<float*>(hout.data_ptr()),
+                                     static_cast<const uint8_t*>(ptr(done_u8)), &batch, T, grad_precision(g), kept.data_ptr(), (size_t)kept.numel(),
+                                     scratch.data_ptr(), (size_t)scratch.numel(), at::cuda::getCurrentCUDAStream(dev.index()).stream()));
+  if (x.scalar_type() == at::kBFloat16) y = y.to(at::kBFloat16);
+  return {y, hout, kept};
+}
+
+// The autograd node of an eager differentiated call: what the operators' formulas do, without Python in
+// the backward pass.
+struct TrunkNode : public torch::autograd::Node {
+  torch::autograd::SavedVariable x, alive, hidden, done, bullets, mask;
+  std::vector<torch::autograd::SavedVariable> weights;
+  Tensor kept;
+  std::vector<int64_t> geom;
+  bool consumed = false;
+
+  static OptTensor opt(const Tensor& t) { return t.defined() ? OptTensor(t) : c10::nullopt; }
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    if (consumed)
+      throw std::runtime_error("the kept activations of this trunk call were consumed by an earlier backward; for a second backward "
+                               "through the same graph set BNB_GRAD_MODE=recompute");
+    consumed = true;
+    const at::NoGradGuard no_grad;
+    const Tensor xv = x.unpack(), hv = hidden.unpack(), bv = bullets.unpack();
+    std::vector<Tensor> ws;
+    ws.reserve(weights.size());
+    for (auto& w : weights) ws.push_back(w.unpack());
+    const Tensor dy = grads[0].defined() ? grads[0] : at::zeros_like(xv, xv.options().dtype(at::kFloat));
+    const BackwardResult r = run_backward(dy, opt(grads[1]), kept, xv, opt(alive.unpack()), hv, opt(done.unpack()), opt(bv), opt(mask.unpack()), ws, geom);
+    kept.reset();
+    torch::autograd::variable_list out;
+    out.reserve(3 + ws.size());
+    out.push_back(task_should_compute_output(0) ? r.dx.reshape(xv.sizes()).to(xv.scalar_type()) : Tensor());
+    out.push_back(task_should_compute_output(1) ? r.dh.reshape(hv.sizes()).to(hv.scalar_type()) : Tensor());
+    out.push_back(bv.defined() && r.dbul.numel() && task_should_compute_output(2) ? r.dbul.reshape(bv.sizes()).to(bv.scalar_type()) : Tensor());
+    int64_t off = 0;
+    for (size_t i = 0; i < ws.size(); ++i) {
+      const int64_t n = ws[i].numel();
+      out.push_back(task_should_compute_output(3 + i) ? r.flat.narrow(0, off, n).view(ws[i].sizes()) : Tensor());
+      off += (n + 3) / 4 * 4;
+    }
+    return out;
+  }
+  void release_variables() override {
+    for (auto* v : {&x, &alive, &hidden, &done, &bullets, &mask}) v->reset_data();
+    weights.clear();
+    kept.reset();
+  }
+};
+
+// A differentiated call with its activations kept: (y, new hidden) with the node above behind them.
+std::tuple<Tensor, Tensor> trunk_train(const Tensor& x, const OptTensor& alive, const Tensor& hidden, const OptTensor& done,
+                                       const OptTensor& bullets, const OptTensor& mask, const std::vector<Tensor>& weights,
+                                       const std::vector<int64_t>& geom) {
+  auto node = std::make_shared<TrunkNode>();
+  torch::autograd::variable_list inputs{x, hidden, bullets.has_value() ? *bullets : Tensor()};
+  inputs.insert(inputs.end(), weights.begin(), weights.end());
+  node->set_next_edges(torch::autograd::collect_next_edges(inputs));
+  Tensor y, hout;
+  {
+    const at::NoGradGuard no_grad;
+    std::tie(y, hout, node->kept) = trunk_forward_train(x, alive, hidden, done, bullets, mask, weights, geom);
+  }
+  using torch::autograd::SavedVariable;
+  auto save = [](const OptTensor& t) { return SavedVariable(t.has_value() ? *t : Tensor(), false); };
+  node->x = SavedVariable(x, false);
+  node->hidden = SavedVariable(hidden, false);
+  node->alive = save(alive);
+  node->done = save(done);
+  node->bullets = save(bullets);
+  node->mask = save(mask);
+  node->weights.reserve(weights.size());
+  for (const Tensor& w : weights) node->weights.emplace_back(w, false);
+  node->geom = geom;
+  torch::autograd::create_gradient_edge(y, node);
+  torch::autograd::create_gradient_edge(hout, node);
+  return {y, hout};
+}
+
 // ------------------------------------------------------------------ ragged batches
 
 // RaggedBatch.build (yemong/trunk.py): the batch integers of a call, the device arrays [tok_off,
@@ -536,6 +740,12 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const
 
 PYBIND11_MODULE(_host_path, m) {
   m.def("trunk_params", &trunk_params);
+  m.def("keep_activations", [](const c10::Device& dev, const std::vector<int64_t>& geom, int64_t d_model, int64_t n_bullets) {
+    return keep_activations(dev, Geometry(geom), d_model, n_bullets);
+  });
+  m.def("trunk_backward", &trunk_backward);
+  m.def("trunk_forward_train", &trunk_forward_train);
+  m.def("trunk_train", &trunk_train);
   m.def("ragged_build", &ragged_build);
   m.def("mlp_chain", &mlp_chain);
   m.def("policy_tail", &policy_tail);

@@ -25,7 +25,7 @@ from torch import Tensor
 import os
 
 from .. import _capi
-from ._weights import N_SPATIAL, N_TEMPORAL, packed_image, spatial_struct_from, temporal_struct_from
+from ._weights import N_SPATIAL, packed_image, spatial_struct_from
 
 # geom: the integers of a call, in this order
 (G_BLOCKS, G_SPATIAL, G_TEMPORAL, G_HEADS, G_BULLET_CROSS, G_FIELD_SUB, G_ENVS, G_TOKENS_PER_ENV, G_SHIPS_PER_ENV,
@@ -125,23 +125,6 @@ def _kept_size(geom: List[int], d_model: int, bullets_per_env: int) -> int:
     return max(256, int(need))
 
 
-def _sublayer_lists(weights: List[Tensor], n_blocks: int, n_spatial: int, n_temporal: int, n_cross: int, field_sub: int):
-    """``weights`` cut into the per-sublayer lists, block-major, spatial before temporal."""
-    spatial, temporal, pos = [], [], 0
-    for _ in range(n_blocks):
-        for j in range(n_spatial):
-            n = N_SPATIAL + (2 if j < n_cross else 0)
-            spatial.append(list(weights[pos : pos + n]))
-            pos += n
-        for _j in range(n_temporal):
-            n = N_TEMPORAL + (1 if field_sub else 0)
-            temporal.append(list(weights[pos : pos + n]))
-            pos += n
-    if pos != len(weights):
-        raise RuntimeError(f"expected {pos} parameter tensors for this trunk structure, got {len(weights)}")
-    return spatial, temporal
-
-
 @torch.library.custom_op("bnb_b200::trunk_backward", mutates_args=(), device_types="cuda")
 def trunk_backward(
     dy: Tensor,
@@ -163,48 +146,7 @@ def trunk_backward(
     (``_split_grads`` cuts it into one view per tensor of ``weights``)].
     ``kept``: the activations ``trunk_forward_train`` kept for this call (the backward consumes
     them), or None: every sublayer's intermediates are recomputed."""
-    dev = x.device
-    D = x.shape[-1]
-    n_blocks, n_spatial, n_temporal = geom[G_BLOCKS], geom[G_SPATIAL], geom[G_TEMPORAL]
-    n_heads, n_cross, field_sub = geom[G_HEADS], geom[G_BULLET_CROSS], geom[G_FIELD_SUB]
-    T = max(1, geom[G_TIMESTEPS])
-    with torch.cuda.device(dev):
-        batch = _batch(geom, [])
-        xin, hin, dyin = _capi.f32c(x), _capi.f32c(hidden), _capi.f32c(dy)
-        dho = None if dhidden_out is None else _capi.f32c(dhidden_out)
-        alive_u8, done_u8 = _capi.u8(alive), _capi.u8(done)
-        spatial, temporal = _sublayer_lists(weights, n_blocks, n_spatial, n_temporal, n_cross, field_sub)
-        # one zeroed buffer for every parameter gradient (the kernels accumulate into it), cut into
-        # views at 16-byte boundaries
-        flat_grads = torch.zeros(sum(_grad_sizes(weights)), dtype=torch.float32, device=dev)
-        grads = _split_grads(flat_grads, weights)
-        g_spatial, g_temporal = _sublayer_lists(grads, n_blocks, n_spatial, n_temporal, n_cross, field_sub)
-        sw = (_capi.SpatialWeights * max(1, len(spatial)))()
-        tw = (_capi.TemporalWeights * max(1, len(temporal)))()
-        sg = (_capi.SpatialGrads * max(1, len(spatial)))()
-        tg = (_capi.TemporalGrads * max(1, len(temporal)))()
-        for i, (ts, gs) in enumerate(zip(spatial, g_spatial)):
-            sw[i] = spatial_struct_from(ts, dev)
-            sg[i] = _capi.SpatialGrads(*[g.data_ptr() for g in gs], *([None] * (N_SPATIAL + 2 - len(gs))))
-        for i, (ts, gs) in enumerate(zip(temporal, g_temporal)):
-            tw[i] = temporal_struct_from(ts, dev)
-            tg[i] = _capi.TemporalGrads(*[g.data_ptr() for g in gs], *([None] * (N_TEMPORAL + 1 - len(gs))))
-        bul = _capi.BulletArgs(bullets if n_cross > 0 else None, bullet_mask, T * batch.n_envs, D)
-        dx = torch.empty_like(xin)
-        dh = torch.zeros_like(hin)
-        dbul = torch.zeros_like(bul.tokens) if bul.struct is not None else xin.new_empty(0)
-        nbytes = _capi.lib.bnb_trunk_bwd_scratch_bytes(n_blocks, n_spatial, n_temporal, D, batch, T, bul.per_env,
-                                                       _grad_precision(geom))
-        scratch = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=dev)   # released after the call's stream work
-        st = _capi.lib.bnb_trunk_sequence_bwd(
-            sw, tw, sg, tg, n_blocks, n_spatial, n_temporal, D, n_heads, xin.data_ptr(), _capi.ptr(alive_u8), bul.arg,
-            _capi.ptr(hin), _capi.ptr(done_u8), batch, T, _grad_precision(geom),
-            dyin.data_ptr(), _capi.ptr(dho), dx.data_ptr(),
-            _capi.ptr(dh), _capi.ptr(dbul) if bul.struct is not None else None, _capi.ptr(kept),
-            0 if kept is None else kept.numel(), scratch.data_ptr(), scratch.numel(), _capi.stream_handle(dev),
-        )
-    _capi.check("bnb_trunk_sequence_bwd", st)
-    return [dx, dh, dbul, flat_grads]
+    return _capi.host.trunk_backward(dy, dhidden_out, kept, x, alive, hidden, done, bullets, bullet_mask, weights, geom)
 
 
 @trunk_backward.register_fake
@@ -272,39 +214,7 @@ def trunk_forward_train(
     every sublayer's intermediates, as autograd does for the reference without grad_checkpoint;
     the backward then skips its recomputation.  Returns (y, new hidden, kept activations); y is
     float32, or bfloat16 for bfloat16 tokens."""
-    dev = x.device
-    D = x.shape[-1]
-    n_blocks, n_spatial, n_temporal = geom[G_BLOCKS], geom[G_SPATIAL], geom[G_TEMPORAL]
-    n_heads, n_cross, field_sub = geom[G_HEADS], geom[G_BULLET_CROSS], geom[G_FIELD_SUB]
-    T = max(1, geom[G_TIMESTEPS])
-    with torch.cuda.device(dev):
-        batch = _batch(geom, [])
-        xin, hin = _capi.f32c(x), _capi.f32c(hidden)
-        alive_u8, done_u8 = _capi.u8(alive), _capi.u8(done)
-        spatial, temporal = _sublayer_lists(weights, n_blocks, n_spatial, n_temporal, n_cross, field_sub)
-        sw = (_capi.SpatialWeights * max(1, len(spatial)))()
-        tw = (_capi.TemporalWeights * max(1, len(temporal)))()
-        for i, ts in enumerate(spatial):
-            sw[i] = spatial_struct_from(ts, dev)
-        for i, ts in enumerate(temporal):
-            tw[i] = temporal_struct_from(ts, dev)
-        bul = _capi.BulletArgs(bullets if n_cross > 0 else None, bullet_mask, T * batch.n_envs, D)
-        y = torch.empty_like(xin)
-        hout = torch.empty_like(hin)
-        kept = torch.empty(_kept_size(geom, D, bul.per_env), dtype=torch.uint8, device=dev)
-        nbytes = _capi.lib.bnb_trunk_bwd_scratch_bytes(n_blocks, n_spatial, n_temporal, D, batch, T, bul.per_env,
-                                                       _grad_precision(geom))
-        scratch = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=dev)
-        st = _capi.lib.bnb_trunk_sequence_fwd_train(
-            sw, tw, n_blocks, n_spatial, n_temporal, D, n_heads, xin.data_ptr(), _capi.ptr(alive_u8), bul.arg, y.data_ptr(),
-            _capi.ptr(hin), _capi.ptr(hout), _capi.ptr(done_u8), batch, T,
-            _grad_precision(geom), kept.data_ptr(), kept.numel(),
-            scratch.data_ptr(), scratch.numel(), _capi.stream_handle(dev),
-        )
-    _capi.check("bnb_trunk_sequence_fwd_train", st)
-    if x.dtype == torch.bfloat16:
-        y = y.to(torch.bfloat16)
-    return y, hout, kept
+    return _capi.host.trunk_forward_train(x, alive, hidden, done, bullets, bullet_mask, weights, geom)
 
 
 @trunk_forward_train.register_fake
@@ -339,29 +249,6 @@ def _train_backward_formula(ctx, dy, dhidden_out, _dkept):
 
 
 trunk_forward_train.register_autograd(_train_backward_formula, setup_context=_train_setup_context)
-
-
-def keep_activations(dev: torch.device, geom: List[int], d_model: int, n_bullets: int) -> bool:
-    """Whether a differentiated call keeps its activations (faster) or lets the backward recompute
-    them (about a sixth of the memory): BNB_GRAD_MODE=keep | recompute decides; otherwise keep when
-    the kept buffer plus the backward's scratch fit in 70 % of the memory that is free or cached."""
-    mode = os.environ.get("BNB_GRAD_MODE", "")
-    if mode == "recompute":
-        return False
-    with torch.cuda.device(dev):
-        batch = _batch(geom, [])
-        T = max(1, geom[G_TIMESTEPS])
-        need = _capi.lib.bnb_trunk_kept_bytes(geom[G_BLOCKS], geom[G_SPATIAL], geom[G_TEMPORAL], d_model, geom[G_HEADS], batch, T,
-                                              n_bullets, _grad_precision(geom))
-        if need == 0:
-            return False
-        if mode == "keep":
-            return True
-        need += _capi.lib.bnb_trunk_bwd_scratch_bytes(geom[G_BLOCKS], geom[G_SPATIAL], geom[G_TEMPORAL], d_model, batch, T, n_bullets,
-                                                      _grad_precision(geom))
-        free, _ = torch.cuda.mem_get_info(dev)
-        cached = torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
-    return need <= 0.7 * (free + cached)
 
 
 @torch.library.custom_op("bnb_b200::spatial_forward", mutates_args=(), device_types="cuda")

@@ -175,10 +175,10 @@ class GriffinTemporalBlock(nn.Module):
 def _keep(x: torch.Tensor, geom: list[int], n_bullets: int) -> bool:
     """Keep activations for the backward, or recompute them?  While a compiler traces the call the
     answer comes from BNB_GRAD_MODE alone (the memory query is a library call a tracer cannot see
-    through); otherwise ``_ops.keep_activations`` also looks at the free memory."""
+    through); otherwise the native side also looks at the free memory."""
     if torch.compiler.is_compiling():
         return os.environ.get("BNB_GRAD_MODE", "") != "recompute" and 0 < geom[_ops.G_MAX_TOKENS]
-    return _ops.keep_activations(x.device, geom, x.shape[-1], n_bullets)
+    return _capi.host.keep_activations(x.device, geom, x.shape[-1], n_bullets)
 
 
 def run_trunk(
@@ -229,6 +229,8 @@ def run_trunk(
     bullets, bullet_mask = (bullets, bullet_mask) if n_cross else (None, None)
     if grad and not offsets and reset_env is None and _keep(x, geom, 0 if bullets is None else bullets.shape[1]):
         # a call that will be differentiated: the forward that keeps its activations for the backward
+        if not tracing:
+            return _capi.host.trunk_train(x, alive, hidden, done, bullets, bullet_mask, weights, geom)
         y, nh, _ = _ops.trunk_forward_train(x, alive, hidden, done, bullets, bullet_mask, weights, geom)
         return y, nh
     run = _ops.trunk_forward if grad or tracing else _ops.trunk_call
