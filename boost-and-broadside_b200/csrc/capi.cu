@@ -10,6 +10,7 @@
 #include "grad_kernels.h"
 #include "host_calls.h"
 #include "launch_count.h"
+#include "split_kernels.h"
 #include "validate.h"
 #include "tensor_kernels.h"
 
@@ -149,14 +150,24 @@ int trunk_call(const BnbSpatialWeights* spatial, const BnbTemporalWeights* tempo
   if (n_blocks * n_spatial > 0 &&
       (st = carve(scratch, scratch_bytes, n_rows, D, (long long)T * batch->n_envs, bullets ? bullets->per_env : 0, &s)))
     return st;
-  const bool emu = precision == BNB_BF16;
-  const float* cur = x;
-  const size_t slot_stride = (size_t)batch->total_ships * 4 * D;
   if (n_blocks * (n_spatial + n_temporal) == 0) {
     if (y != x && cudaMemcpyAsync(y, x, n_rows * D * sizeof(float), cudaMemcpyDeviceToDevice, cs) != cudaSuccess)
       return BNB_ERR_LAUNCH;
     return BNB_OK;
   }
+  // With weight images to work on, a float32 step goes to the tensor-core tiles whatever its size: one tile
+  // takes them a tenth of what it takes the exact kernels.  Sequences stay with those, whose recurrence walks
+  // the timesteps inside a kernel.
+  if (pack && precision == BNB_FP32 && T == 1 && y != x && bnb::split::supported(D, H)) {
+    const size_t used = simt_scratch_bytes(n_rows, D, batch->n_envs, bullets ? bullets->per_env : 0);
+    if (!s.qkv && (st = carve(scratch, scratch_bytes, n_rows, D, batch->n_envs, bullets ? bullets->per_env : 0, &s))) return st;
+    const bnb::split::Scratch area{reinterpret_cast<int*>(static_cast<char*>(scratch) + used), s.qkv, s.o, s.kvb, s.kvb_envs};
+    return bnb::split::step(spatial, temporal, n_blocks, n_spatial, n_temporal, x, alive, bullets, y, hidden_in, hidden_out, reset_env,
+                            *batch, area, cs);
+  }
+  const bool emu = precision == BNB_BF16;
+  const float* cur = x;
+  const size_t slot_stride = (size_t)batch->total_ships * 4 * D;
   for (int i = 0; i < n_blocks; ++i) {
     for (int j = 0; j < n_spatial; ++j) {
       st = bnb::exact::spatial_block(spatial[i * n_spatial + j], D, H, cur, alive, bullets, y, *batch, T, emu, s.qkv,

@@ -26,6 +26,7 @@
 #include "host_calls.h"
 #include "mlp_kernels.h"
 #include "policy_tail.h"
+#include "split_kernels.h"
 #include "tensor_kernels.h"
 
 namespace py = pybind11;
@@ -301,7 +302,9 @@ std::tuple<Tensor, Tensor> trunk_forward(const Tensor& x, const OptTensor& alive
   // bfloat16 tokens stay bfloat16 on the way in and out where the fused kernels serve the call;
   // anything else is converted to float32 here
   const bool io16 = built && x.scalar_type() == at::kBFloat16 && (offsets.empty() || offsets.size() > 2);
-  const bool images = tensor_engine && bnb_supported((int)D, g.heads, 1, BNB_BF16, BNB_ENGINE_TENSOR);
+  // a float32 step runs from weight images too, unless the caller named the exact engine
+  const bool split = !bf16 && g.engine != kEngineSimt && g.timesteps == 0 && bnb::split::supported((int)D, g.heads);
+  const bool images = split || (tensor_engine && bnb_supported((int)D, g.heads, 1, BNB_BF16, BNB_ENGINE_TENSOR));
 
   Weights w = weight_structs(g, weights, dev);
   const Tensor hin = f32c(hidden);
@@ -316,7 +319,8 @@ std::tuple<Tensor, Tensor> trunk_forward(const Tensor& x, const OptTensor& alive
     const Bullets b(g.bullet_cross > 0 ? bullets : c10::nullopt, bullet_mask, (int64_t)T * batch.n_envs, D, bullets16);
     *used_bullets16 = b.present && b.arg.tokens_bf16;
     const size_t need = round256(bnb_scratch_bytes((int)D, &batch, T, b.arg.per_env));
-    const size_t sp = round256(bnb_packed_spatial_bytes((int)D)), tp = round256(bnb_packed_temporal_bytes((int)D));
+    const size_t sp = round256(split ? bnb::split::spatial_image_bytes() : bnb_packed_spatial_bytes((int)D));
+    const size_t tp = round256(split ? bnb::split::temporal_image_bytes() : bnb_packed_temporal_bytes((int)D));
     const size_t image_bytes = images ? sp * w.spatial.size() + tp * w.temporal.size() : 0;
     const Tensor scratch = scratch_for(dev, need + image_bytes).cast<Tensor>();
     uint8_t* base = static_cast<uint8_t*>(scratch.data_ptr());

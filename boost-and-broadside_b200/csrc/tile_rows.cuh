@@ -1,0 +1,85 @@
+// Row tiles of 128 x 128 on one CTA: the roles, waits and data movement that the kernels with sixteen epilogue
+// warps, one issuing and one fetching warp share (train_mlp.cu, split_kernels.cu).
+#pragma once
+
+#include "tensor_common.cuh"
+
+namespace bnb {
+namespace tensor {
+
+constexpr int EPI_WARPS = 16, EPI_THREADS = 512, MMA_WARP = 16, LOAD_WARP = 17, THREADS = 576;
+enum : int { TIMEOUT_FULL = 101, TIMEOUT_FREE = 102, TIMEOUT_ACC = 103, TIMEOUT_OPERAND = 104 };
+
+// What every role needs for its waits.
+struct Sync {
+  uint32_t bars;           // shared address of the barrier array
+  int* status;
+  volatile int* aborted;
+  __device__ __forceinline__ void wait(int bar, uint32_t parity, int code) const { mbar_wait(bars + 8 * bar, parity & 1u, status, aborted, code); }
+};
+
+// The epilogue warps' arrival on an operand barrier.
+__device__ __forceinline__ void post(const Sync& s, int bar) {
+  fence_proxy_async();
+  tc_fence_before();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(s.bars + 8 * bar);
+}
+__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
+// Rows move between global memory and the warps in a layout of their own: warp w owns rows 32 (w % 4) .. and
+// columns 32 (w / 4) .., and in its i-th request (i < 8) lane l takes the sixteen bytes at row 4 i + l / 8,
+// columns 4 (l % 8).. : a request touches four lines.  (With a thread per tile row, as tensor memory has it, each
+// request touched 32 lines, and the loads and stores alone took 25 000 of a tile's 67 000 cycles.)
+struct RowMap {
+  int lane, row0, col;     // first tile row and this lane's first column
+  __device__ __forceinline__ int row(int i) const { return row0 + 4 * i + (lane >> 3); }
+};
+__device__ __forceinline__ RowMap row_map() {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  return {lane, 32 * (warp & 3), 32 * (warp >> 2) + 4 * (lane & 7)};
+}
+__device__ __forceinline__ void rows_in(float4 (&v)[8], const float* src, const RowMap& m, int first, int rows) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = first + m.row(i);
+    v[i] = r < rows ? *reinterpret_cast<const float4*>(src + (size_t)r * D + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+// Per-row sums of one value per request: over the eight lanes of a row here, over the four column parts
+// through shared memory.  Returns the totals of this lane's rows; two barriers of the four warps of these rows.
+__device__ __forceinline__ void row_sums(float (&v)[8], float* part_sums, const RowMap& m) {
+  const int part = threadIdx.x >> 7, bar = 3 + ((threadIdx.x >> 5) & 3);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+  if ((m.lane & 7) == 0)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) part_sums[part * TILE + m.row(i)] = v[i];
+  asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float* p = part_sums + m.row(i);
+    v[i] = (p[0] + p[TILE]) + (p[2 * TILE] + p[3 * TILE]);
+  }
+  asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");   // before the next use
+}
+// 32 accumulator columns from the thread-per-row layout of tensor memory to the row layout, through 4 KB of
+// shared memory of the warp's own.
+__device__ __forceinline__ void transpose_rows(float4 (&v)[8], uint32_t taddr, uint8_t* stage, const RowMap& m) {
+  uint32_t t[32];
+  tmem_ld32(taddr, t);
+  const int r = m.lane;
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    *reinterpret_cast<uint4*>(stage + r * 128 + ((q ^ (r & 7)) << 4)) = make_uint4(t[4 * q], t[4 * q + 1], t[4 * q + 2], t[4 * q + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int rr = 4 * i + (m.lane >> 3);
+    v[i] = *reinterpret_cast<const float4*>(stage + rr * 128 + (((m.lane & 7) ^ (rr & 7)) << 4));
+  }
+}
+
+}  // namespace tensor
+}  // namespace bnb

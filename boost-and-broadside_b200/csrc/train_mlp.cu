@@ -25,8 +25,8 @@
 #include "train_mlp.h"
 
 #include "launch_count.h"
-#include "tensor_common.cuh"
 #include "tensor_kernels.h"
+#include "tile_rows.cuh"
 
 namespace bnb {
 namespace train_mlp {
@@ -40,9 +40,6 @@ constexpr int F = 512, NCHUNK = 8;                 // hidden width, chunks of 64
 // gate and up transposed (128 rows x 64 k each), down (128 rows x 64 k)
 constexpr uint32_t IMG_GU = 0, IMG_DH = 32768, IMG_DN = 49152, IMG_D = 81920, IMG_CHUNK = 98304;
 constexpr uint32_t IMAGE = NCHUNK * IMG_CHUNK;
-
-constexpr int EPI_WARPS = 16, EPI_THREADS = 512, MMA_WARP = 16, LOAD_WARP = 17, THREADS = 576;
-enum : int { TIMEOUT_FULL = 101, TIMEOUT_FREE = 102, TIMEOUT_ACC = 103, TIMEOUT_OPERAND = 104 };
 
 // ------------------------------------------------------------------ weight images
 
@@ -108,14 +105,6 @@ struct Args {
   int* host_status;
 };
 
-// What every role needs for its waits.
-struct Sync {
-  uint32_t bars;           // shared address of the barrier array
-  int* status;
-  volatile int* aborted;
-  __device__ __forceinline__ void wait(int bar, uint32_t parity, int code) const { mbar_wait(bars + 8 * bar, parity & 1u, status, aborted, code); }
-};
-
 // The descriptor of an MN-major operand (two 64-wide atoms CHUNK_BYTES apart): see mma_one for the rest.
 __device__ __forceinline__ uint32_t desc_mn(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | ((CHUNK_BYTES >> 4) << 16); }
 constexpr uint32_t BOTH_MN = (1u << 15) | (1u << 16);
@@ -149,52 +138,6 @@ __device__ __forceinline__ F2 normal_cdf(F2 x, F2& e) {
 }
 __device__ __forceinline__ uint32_t pack_f2(F2 a) { const float2 v = split(a); return pack_bf16(v.x, v.y); }
 __device__ __forceinline__ F2 acc_pair(const uint32_t* v) { return f2(__uint_as_float(v[0]), __uint_as_float(v[1])); }
-// The epilogue warps' arrival on an operand barrier.
-__device__ __forceinline__ void post(const Sync& s, int bar) {
-  fence_proxy_async();
-  tc_fence_before();
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) mbar_arrive(s.bars + 8 * bar);
-}
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
-// Rows move between global memory and the warps in a layout of their own: warp w owns rows 32 (w % 4) .. and
-// columns 32 (w / 4) .., and in its i-th request (i < 8) lane l takes the sixteen bytes at row 4 i + l / 8,
-// columns 4 (l % 8).. : a request touches four lines.  (With a thread per tile row, as tensor memory has it, each
-// request touched 32 lines, and the loads and stores alone took 25 000 of a tile's 67 000 cycles.)
-struct RowMap {
-  int lane, row0, col;     // first tile row and this lane's first column
-  __device__ __forceinline__ int row(int i) const { return row0 + 4 * i + (lane >> 3); }
-};
-__device__ __forceinline__ RowMap row_map() {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  return {lane, 32 * (warp & 3), 32 * (warp >> 2) + 4 * (lane & 7)};
-}
-__device__ __forceinline__ void rows_in(float4 (&v)[8], const float* src, const RowMap& m, int first, int rows) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = first + m.row(i);
-    v[i] = r < rows ? *reinterpret_cast<const float4*>(src + (size_t)r * D + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-}
-// Per-row sums of one value per request: over the eight lanes of a row here, over the four column parts
-// through shared memory.  Returns the totals of this lane's rows; two barriers of the four warps of these rows.
-__device__ __forceinline__ void row_sums(float (&v)[8], float* part_sums, const RowMap& m) {
-  const int part = threadIdx.x >> 7, bar = 3 + ((threadIdx.x >> 5) & 3);
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
-  if ((m.lane & 7) == 0)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) part_sums[part * TILE + m.row(i)] = v[i];
-  asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float* p = part_sums + m.row(i);
-    v[i] = (p[0] + p[TILE]) + (p[2 * TILE] + p[3 * TILE]);
-  }
-  asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");   // before the next use
-}
 // four values as bfloat16 into an operand tile
 __device__ __forceinline__ void put4(uint8_t* tile, int row, int col, float a, float b, float c, float d) {
   *reinterpret_cast<uint2*>(tile + (col >> 6) * CHUNK_BYTES + swz(row, (col & 63) >> 3) + ((col >> 2) & 1) * 8) = make_uint2(pack_bf16(a, b), pack_bf16(c, d));
@@ -210,23 +153,6 @@ __device__ __forceinline__ void norm_rows(uint8_t* tile, const float4 (&x)[8], f
     put4(tile, m.row(i), m.col, x[i].x * inv[i] * gain.x, x[i].y * inv[i] * gain.y, x[i].z * inv[i] * gain.z, x[i].w * inv[i] * gain.w);
   }
 }
-// 32 accumulator columns from the thread-per-row layout of tensor memory to the row layout, through 4 KB of
-// shared memory of the warp's own.
-__device__ __forceinline__ void transpose_rows(float4 (&v)[8], uint32_t taddr, uint8_t* stage, const RowMap& m) {
-  uint32_t t[32];
-  tmem_ld32(taddr, t);
-  const int r = m.lane;
-#pragma unroll
-  for (int q = 0; q < 8; ++q)
-    *reinterpret_cast<uint4*>(stage + r * 128 + ((q ^ (r & 7)) << 4)) = make_uint4(t[4 * q], t[4 * q + 1], t[4 * q + 2], t[4 * q + 3]);
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int rr = 4 * i + (m.lane >> 3);
-    v[i] = *reinterpret_cast<const float4*>(stage + rr * 128 + (((m.lane & 7) ^ (rr & 7)) << 4));
-  }
-}
-
 // Kernel frame: barriers (counts given), tensor memory, status.  smem is the dynamic array itself, on a
 // 1024-byte boundary because nothing static stands in front of it.
 struct Frame {
