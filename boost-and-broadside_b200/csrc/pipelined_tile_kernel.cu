@@ -68,9 +68,10 @@ constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
 // DONE[s]: the MMAs that read slot s are complete (tcgen05.commit) -- the fetching warp takes it as
 // "slot free" and the epilogue warps as "accumulator ready" for gate|up of one chunk, whose slot is not
 // used again before they have seen it.  QKV[h]: q|k|v of head h is complete (a barrier per head: a slot
-// serves two heads, and a phase waited for too late would look like the one after next).  ACC: every MMA of a round is complete (one more commit per round).  DRAIN: every MMA of the
+// serves two heads, and a phase waited for too late would look like the one after next).  ACC: every MMA of a round is complete (one more commit per round).
+// EARLY: the first product of a temporal sublayer's two larger rounds is.  DRAIN: every MMA of the
 // CTA is complete (once, at the end).
-enum : int { B_OP0 = 0, B_FFN0, B_FFN1, B_FFN2, B_KVREL, B_ACC, B_DRAIN, B_QKV0, B_FULL0 = B_QKV0 + HEADS, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
+enum : int { B_OP0 = 0, B_FFN0, B_FFN1, B_FFN2, B_KVREL, B_ACC, B_EARLY, B_DRAIN, B_QKV0, B_FULL0 = B_QKV0 + HEADS, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
 static_assert(B_COUNT * 8 + 8 <= 256, "barrier area");
 
 constexpr uint32_t COL_RESID = 0;
@@ -214,6 +215,7 @@ struct Epi {
   uint32_t par;         // phase bits of the pair slots' DONE barriers (0..2), of ACC (8) and of QKV (9)
   SlotRotation rot;     // pair slot of the next ring operation
   int row, part;
+  bool wide;            // 32-byte accesses: every row pointer is aligned for them
   int* status;
   volatile int* aborted;
   float* ss_part;
@@ -240,6 +242,15 @@ __device__ __forceinline__ void wait_acc(Epi& e) {
   T_END(e.tacc, e.wait_slot);
   TRACE(e.tr, 110);
 }
+// wait_early: the first product of a temporal round, read while the others are multiplied (1 % of a step).
+// Every thread waits for each of its phases before it posts what the next one is issued after.
+__device__ __forceinline__ void wait_early(Epi& e) {
+  T_BEGIN();
+  mbar_wait(e.bars + 8 * B_EARLY, (e.par >> 10) & 1u, e.status, e.aborted, ST_TIMEOUT_ACC);
+  e.par ^= 1u << 10;
+  tc_fence_after();
+  T_END(e.tacc, e.wait_slot);
+}
 // wait_round: a round of n pair operations in rotation order, then a commit on ACC.
 __device__ __forceinline__ void wait_round(Epi& e, int n) {
   wait_acc(e);
@@ -256,6 +267,29 @@ __device__ __forceinline__ void wait_op(Epi& e, uint32_t slot) {
   TRACE(e.tr, 100);
 }
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
+
+// Eight floats of one row per thread.  Threads own rows here, so every request of a warp touches 32 lines
+// whatever its width: 32-byte accesses (where the pointers allow them) make it half as many requests as
+// 16-byte ones.  In a sequence of 32 steps, whose state is read and written at every step, that is 4 % of
+// the time (7442 -> 7153 us at 4096 x 8 tokens).
+__device__ __forceinline__ void load8(float (&v)[8], const float* p, bool wide) {
+  if (wide) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p) : "memory");
+  } else {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  }
+}
+__device__ __forceinline__ void store8(float* p, const float (&v)[8], bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.f32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
+                 ::"f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "l"(p) : "memory");
+  } else {
+    reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+  }
+}
 
 // residual (TMEM) -> x * rsqrt(mean x^2 + eps) -> bf16 A operand (the RMSNorm gain is in the weights)
 __device__ __forceinline__ void norm_to_A(Epi& e) {
@@ -556,7 +590,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
   const bool is_ship = rs.hrow >= 0;
   norm_to_A(e);
   post(e, B_OP0);
-  wait_round(e, 2);   // acc0 = linear2 n, acc1 = linear1 n
+  wait_early(e);      // acc0 = linear2 n
   T_MARK(tt);
   // b2 = bf16(gelu(linear2 n)) for this thread's columns, parked as packed bf16 pairs
   uint32_t b2p[2][8];
@@ -568,6 +602,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
 #pragma unroll
     for (int j = 0; j < 8; ++j) b2p[rnd][j] = pack_bf16(gelu_fast(__uint_as_float(v[2 * j])), gelu_fast(__uint_as_float(v[2 * j + 1])));
   }
+  wait_round(e, 2);   // acc1 = linear1 n
   // b1 = bf16(linear1 n) into the A operand; ships: causal conv with the stored taps -> u
   {
     uint32_t v[32];
@@ -652,28 +687,31 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
   post(e, B_OP0);   // A = u (ship rows) / b1 (field rows)
   T_SINCE(e.tacc, TE_TEMPORAL, tt);
   // previous state of this thread's columns of the first half, requested before the gates arrive
-  float4 hprev[4];
+  float hprev[2][8];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    hprev[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (is_ship && !rs.zero_in) hprev[q] = *reinterpret_cast<const float4*>(hin + e.part * 16 + q * 4);
+  for (int q = 0; q < 2; ++q) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) hprev[q][i] = 0.f;
+    if (is_ship && !rs.zero_in) load8(hprev[q], hin + e.part * 16 + q * 8, e.wide);
   }
-  wait_round(e, has_fields ? 3 : 2);   // acc0 / acc1 = [W_a u | W_x u] of hidden columns [0,64) / [64,128); acc2 = field_sub b1
+  wait_early(e);   // acc0 / acc1 = [W_a u | W_x u] of hidden columns [0,64) / [64,128)
   T_MARK(tu);
   // gates and state update
 #pragma unroll
   for (int rnd = 0; rnd < 2; ++rnd) {
+    if (rnd == 1) wait_round(e, has_fields ? 3 : 2);   // the rest; acc2 = field_sub b1
     uint32_t rv[16], iv[16];
     const uint32_t acc = e.lane_addr + COL_ACC0 + rnd * 128 + e.part * 16;
     tmem_ld16_nowait(acc, rv);        // executed by every lane of the warp
     tmem_ld16_nowait(acc + 64, iv);
     tmem_wait_ld();
-    float4 hnext[4];
+    float hnext[2][8];
     if (rnd == 0) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        hnext[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (is_ship && !rs.zero_in) hnext[q] = *reinterpret_cast<const float4*>(hin + 64 + e.part * 16 + q * 4);
+      for (int q = 0; q < 2; ++q) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) hnext[q][i] = 0.f;
+        if (is_ship && !rs.zero_in) load8(hnext[q], hin + 64 + e.part * 16 + q * 8, e.wide);
       }
     }
     if (is_ship) {
@@ -685,18 +723,17 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
         const uint4 ub = *reinterpret_cast<const uint4*>(ua);
         const uint32_t uw[4] = {ub.x, ub.y, ub.z, ub.w};
         uint32_t ob[4];
+        float hn[8];
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           const int cc = col + hf * 4;
-          const float4 hv = hprev[q * 2 + hf];
           const float4 ab = __ldg(reinterpret_cast<const float4*>(s.a_b + cc));
           const float4 xb = __ldg(reinterpret_cast<const float4*>(s.x_b + cc));
           const float4 dl = __ldg(reinterpret_cast<const float4*>(s.decay_log2 + cc));
           const float abv[4] = {ab.x, ab.y, ab.z, ab.w}, xbv[4] = {xb.x, xb.y, xb.z, xb.w}, dlv[4] = {dl.x, dl.y, dl.z, dl.w};
-          float hn[4] = {hv.x, hv.y, hv.z, hv.w};
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const int k = q * 8 + hf * 4 + i;
+            const int k = q * 8 + hf * 4 + i, j = hf * 4 + i;
             const float rg = round_bf16(sigmoid_fast(__uint_as_float(rv[k]) + abv[i]));
             const float ig = round_bf16(sigmoid_fast(__uint_as_float(iv[k]) + xbv[i]));
             // sigmoid(Lambda)^(8 r) = 2^(r * 8 log2 sigmoid(Lambda)); the table is part of the weight image
@@ -706,13 +743,13 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
             const float uu = (i & 1) ? bf16_hi(uword) : bf16_lo(uword);
             const float bb = gate * (ig * uu);
             if (boundary) a = 0.f;
-            hn[i] = fmaf(a, hn[i], bb);
+            hn[j] = fmaf(a, hprev[q][j], bb);
           }
-          *reinterpret_cast<float4*>(hout + cc) = make_float4(hn[0], hn[1], hn[2], hn[3]);
           const int bi = q * 4 + hf * 2;
-          ob[hf * 2] = pack_bf16(hn[0] * bf16_lo(b2p[rnd][bi]), hn[1] * bf16_hi(b2p[rnd][bi]));
-          ob[hf * 2 + 1] = pack_bf16(hn[2] * bf16_lo(b2p[rnd][bi + 1]), hn[3] * bf16_hi(b2p[rnd][bi + 1]));
+          ob[hf * 2] = pack_bf16(hn[hf * 4] * bf16_lo(b2p[rnd][bi]), hn[hf * 4 + 1] * bf16_hi(b2p[rnd][bi]));
+          ob[hf * 2 + 1] = pack_bf16(hn[hf * 4 + 2] * bf16_lo(b2p[rnd][bi + 1]), hn[hf * 4 + 3] * bf16_hi(b2p[rnd][bi + 1]));
         }
+        store8(hout + col, hn, e.wide);
         // branch operand of linear_out: K atom 0 lives in P0, K atom 1 in place in A
         uint8_t* dst = rnd == 0 ? e.smem + OFF_P + swz(e.row, e.part * 2 + q) : ua;
         *reinterpret_cast<uint4*>(dst) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
@@ -720,7 +757,9 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
     }
     if (rnd == 0) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) hprev[q] = hnext[q];
+      for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) hprev[q][i] = hnext[q][i];
     }
   }
   if (has_fields) {
@@ -871,10 +910,12 @@ __device__ __forceinline__ void issue_out_proj(Issuer& m, uint32_t a_off) {
 __device__ __forceinline__ void issue_temporal(Issuer& m, bool has_fields) {
   wait_operand(m, B_OP0);
   issue_from_A(m, m.rot.next_pair(), 128, COL_ACC0);   // linear2
+  commit_one(m, B_EARLY);
   issue_from_A(m, m.rot.next_pair(), 128, COL_ACC1);   // linear1
   commit_round(m);
   wait_operand(m, B_OP0);
   issue_from_A(m, m.rot.next_pair(), 128, COL_ACC0);   // gates of hidden columns [0,64)
+  commit_one(m, B_EARLY);
   issue_from_A(m, m.rot.next_pair(), 128, COL_ACC1);   // gates of hidden columns [64,128)
   if (has_fields) issue_from_A(m, m.rot.next_pair(), 128, COL_ACC2);   // field_sub
   commit_round(m);
@@ -1027,6 +1068,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     e.bars = smem_u32(bars);
     e.row = tid & (TILE - 1);
     e.part = tid >> 7;
+    e.wide = args.wide != 0;
     e.lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
     e.par = 0;
     e.rot = SlotRotation{0, 3};
@@ -1127,25 +1169,24 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
         {
           uint32_t v[32];
           if (args.io_bf16) {
-            const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(args.x) + trow * D + e.part * 32);
+            const float* src = reinterpret_cast<const float*>(reinterpret_cast<const __nv_bfloat16*>(args.x) + trow * D + e.part * 32);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint4 w = make_uint4(0u, 0u, 0u, 0u);
-              if (valid) w = src[q];
-              const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+            for (int q = 0; q < 2; ++q) {
+              float w[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+              if (valid) load8(w, src + 8 * q, e.wide);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                v[q * 8 + 2 * j] = ws[j] << 16;              // a bfloat16 is the upper half of its float
-                v[q * 8 + 2 * j + 1] = ws[j] & 0xFFFF0000u;
+              for (int j = 0; j < 8; ++j) {
+                v[q * 16 + 2 * j] = __float_as_uint(w[j]) << 16;              // a bfloat16 is the upper half of its float
+                v[q * 16 + 2 * j + 1] = __float_as_uint(w[j]) & 0xFFFF0000u;
               }
             }
           } else {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (valid) f = *reinterpret_cast<const float4*>(args.x + trow * D + e.part * 32 + q * 4);
-              v[q * 4 + 0] = __float_as_uint(f.x); v[q * 4 + 1] = __float_as_uint(f.y);
-              v[q * 4 + 2] = __float_as_uint(f.z); v[q * 4 + 3] = __float_as_uint(f.w);
+            for (int q = 0; q < 4; ++q) {
+              float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+              if (valid) load8(f, args.x + trow * D + e.part * 32 + q * 8, e.wide);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) v[q * 8 + j] = __float_as_uint(f[j]);
             }
           }
           tmem_st32(e.lane_addr + COL_RESID + e.part * 32, v);
@@ -1181,14 +1222,22 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
           uint32_t v[32];
           tmem_ld32(e.lane_addr + COL_RESID + e.part * 32, v);
           if (valid && args.io_bf16) {
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(args.y) + trow * D + e.part * 32);
+            float* dst = reinterpret_cast<float*>(reinterpret_cast<__nv_bfloat16*>(args.y) + trow * D + e.part * 32);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) dst[q] = pack8(&v[q * 8]);
+            for (int q = 0; q < 2; ++q) {
+              float w[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) w[j] = __uint_as_float(pack_bf16(__uint_as_float(v[q * 16 + 2 * j]), __uint_as_float(v[q * 16 + 2 * j + 1])));
+              store8(dst + 8 * q, w, e.wide);
+            }
           } else if (valid) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-              *reinterpret_cast<float4*>(args.y + trow * D + e.part * 32 + q * 4) =
-                  make_float4(__uint_as_float(v[q * 4]), __uint_as_float(v[q * 4 + 1]), __uint_as_float(v[q * 4 + 2]), __uint_as_float(v[q * 4 + 3]));
+            for (int q = 0; q < 4; ++q) {
+              float f[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[q * 8 + j]);
+              store8(args.y + trow * D + e.part * 32 + q * 8, f, e.wide);
+            }
           }
         }
         T_SINCE(e.tacc, TE_IO, t_io);

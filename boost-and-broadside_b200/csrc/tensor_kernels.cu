@@ -1698,6 +1698,9 @@ static int launch(TrunkArgs& a, const BnbBatch& b, cudaStream_t st) {
   a.poll_limit = g_debug_poll_limit;
   a.skip_op = g_debug_skip_op;
   a.host_status = host_status_word(st);
+  uintptr_t places = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.y);
+  for (int i = 0; i < a.n_sub; ++i) places |= reinterpret_cast<uintptr_t>(a.sub[i].hid_in) | reinterpret_cast<uintptr_t>(a.sub[i].hid_out);
+  a.wide = places % 32 == 0;
   if (a.n_tiles == 0) return BNB_OK;
   {
     // the pipelined kernel runs every program of spatial (whole or split around the attention
