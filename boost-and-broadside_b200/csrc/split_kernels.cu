@@ -19,8 +19,10 @@
 //               cluster, whose partial sums meet in distributed shared memory.
 //
 // One step of 96 environments of 37 tokens took 1457 us with a CTA per 32 rows walking all layers on mma.sync
-// (111 CTAs, each streaming every weight through registers).  What bounds these kernels is the chain inside a
-// CTA (rows in, products, exchange, rows out), a few us each; launches overlap by programmatic dependence.
+// (111 CTAs, each streaming every weight through registers), and takes 258 here.  What bounds these kernels is
+// the chain inside a CTA: k_post's 24 us are rows in 2, output projection 2, norm 1.5, gate|up 4.5, GELU and down
+// projection 3, exchange 4 and the start; the tensor cores work for a third of that.  Launches overlap by
+// programmatic dependence (289 us without), clusters of two instead of four take 295.
 #include "split_kernels.h"
 
 #include "common.cuh"
@@ -73,12 +75,12 @@ __host__ __device__ constexpr size_t image_bytes(int rows, int k) { return (size
 struct Image { const uint8_t* at; int rows; };
 // Places of a sublayer's images.
 enum : int { IM_QKV = 0, IM_OUT, IM_GATE, IM_UP, IM_DOWN, IM_KVB };
-enum : int { IM_LIN1 = 0, IM_LIN2, IM_A, IM_X, IM_OUT_T, IM_GATE_T, IM_UP_T, IM_DOWN_T, IM_FIELD };
+enum : int { IM_LIN1 = 0, IM_LIN2, IM_A, IM_X, IM_OUT_T, IM_GATE_T, IM_UP_T, IM_DOWN_T, IM_FIELD, IM_DECAY };
 __host__ __device__ constexpr size_t spatial_at(int i) {
   return image_bytes(128, 128) * (i == IM_QKV ? 0 : i == IM_OUT ? 3 : 4 + 4 * (i - IM_GATE));
 }
 __host__ __device__ constexpr size_t temporal_at(int i) {
-  return image_bytes(128, 128) * (i <= IM_GATE_T ? i : i <= IM_DOWN_T ? 5 + 4 * (i - IM_GATE_T) : 17);
+  return image_bytes(128, 128) * (i <= IM_GATE_T ? i : i <= IM_DOWN_T ? 5 + 4 * (i - IM_GATE_T) : 17 + i - IM_FIELD);
 }
 
 constexpr int MAX_PACK = 96;
@@ -92,9 +94,18 @@ struct PackJobs {
 // times that: bound by the launch.
 __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackJobs jobs) {
   if (jobs.status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *jobs.status = 0;
-  const int rows = jobs.rows[blockIdx.y], k = jobs.k[blockIdx.y], per_row = k / 8;
+  const int rows = jobs.rows[blockIdx.y], k = jobs.k[blockIdx.y], per_row = k / 8;   // k = 0: a vector
   const float* src = jobs.src[blockIdx.y];
   uint8_t* dst = jobs.dst[blockIdx.y];
+  if (k == 0) {   // Lambda: the logarithm of its sigmoid as high and low part
+    float* out = reinterpret_cast<float*>(dst);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
+      const double v = log((double)sigmoidf_(src[i]));
+      out[i] = (float)v;
+      out[rows + i] = (float)(v - (double)(float)v);
+    }
+    return;
+  }
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += gridDim.x * blockDim.x) {
     const int r = i / per_row, g = i - r * per_row;
     const float4 a = *reinterpret_cast<const float4*>(src + (size_t)r * k + 8 * g), b = *reinterpret_cast<const float4*>(src + (size_t)r * k + 8 * g + 4);
@@ -133,7 +144,7 @@ __device__ __forceinline__ Frame open_frame(uint8_t* smem, const Waits& w) {
     aborted[1] = DEFAULT_POLL_LIMIT;
     *reinterpret_cast<int**>(&aborted[2]) = w.host_status;
     for (int i = 0; i < B_COUNT; ++i)
-      mbar_init(bars + 8 * i, i == B_OP0 || i == B_OP1 ? EPI_WARPS : i >= B_H0 ? EPI_WARPS / 2 : 1);
+      mbar_init(bars + 8 * i, i == B_OP0 || i == B_OP1 || i >= B_H0 ? EPI_WARPS : 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x < 32) {
@@ -200,36 +211,80 @@ __device__ __forceinline__ bool fetch_product(const Frame& f, Ring& ring, uint32
 __device__ __forceinline__ void product(const Frame& f, Ring& ring, uint32_t base, uint32_t el, uint32_t d, uint32_t idesc) {
   const uint32_t a_lo = uniform(desc_lo(base));
 #pragma unroll 1
-  for (uint32_t i = 0; i < 6; ++i) {
-    const uint32_t atom = i >= 3 ? 1 : 0, weak = i - 3 * atom;   // weight piece 2 - weak meets operand pieces weak .. 0
-    f.s.wait(B_FULL + ring.slot, ring.parity >> ring.slot, TIMEOUT_FULL);
-    const uint32_t b = uniform(desc_lo(base + ring.at()));
-#pragma unroll 1
-    for (uint32_t j = 0; j <= weak; ++j) {
-      const uint32_t a = uniform(a_lo + (PIECE >> 4) * (weak - j) + (ATOM >> 4) * atom);
+  for (uint32_t atom = 0; atom < 2; ++atom) {
+    const uint32_t a_at = uniform(a_lo + (ATOM >> 4) * atom);
 #pragma unroll
-      for (uint32_t k = 0; k < 4; ++k) mma_one<false>(el, d, a + 2 * k, b + 2 * k, idesc, (i | j | k) ? 1u : 0u);
+    for (uint32_t weak = 0; weak < 3; ++weak) {   // weight piece 2 - weak meets operand pieces weak .. 0
+      f.s.wait(B_FULL + ring.slot, ring.parity >> ring.slot, TIMEOUT_FULL);
+      const uint32_t b = uniform(desc_lo(base + ring.at()));
+#pragma unroll
+      for (uint32_t j = 0; j <= weak; ++j)
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+          mma_one<false>(el, d, a_at + (PIECE >> 4) * (weak - j) + 2 * k, b + 2 * k, idesc, (atom | weak | j | k) ? 1u : 0u);
+      tc_commit_if(el, f.s.bars + 8 * (B_FREE + ring.slot));
+      ring.next();
     }
-    tc_commit_if(el, f.s.bars + 8 * (B_FREE + ring.slot));
-    ring.next();
   }
 }
 
-// Rows of the operand: n = x inv gain, as pieces.
-__device__ __forceinline__ void norm_pieces(uint8_t* tile, const float4 (&x)[8], const float4& gain, float* part_sums, const RowMap& m) {
-  float ss[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) ss[i] = fmaf(x[i].x, x[i].x, fmaf(x[i].y, x[i].y, fmaf(x[i].z, x[i].z, x[i].w * x[i].w)));
-  row_sums(ss, part_sums, m);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float inv = rsqrtf(ss[i] / (float)D + kRmsEps);
-    put_pieces(tile, m.row(i), m.col, make_float4(x[i].x * inv * gain.x, x[i].y * inv * gain.y, x[i].z * inv * gain.z, x[i].w * inv * gain.w));
-  }
-}
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void store4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
 __device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+// How rows come in: warp w takes rows 32 (w % 4) .. and columns 32 (w / 4) .., in its i-th request (i < 4) lane l
+// eight columns of row 8 i + l / 4.  A request touches eight lines, and a piece of eight columns is sixteen
+// bytes of the operand tile, stored without bank conflicts.
+struct Rows8 {
+  int row0, col;
+  __device__ __forceinline__ int row(int i) const { return row0 + 8 * i + ((threadIdx.x & 31) >> 2); }
+};
+__device__ __forceinline__ Rows8 rows8() { return {32 * ((int)(threadIdx.x >> 5) & 3), 32 * (int)(threadIdx.x >> 7) + 8 * (int)(threadIdx.x & 3)}; }
+__device__ __forceinline__ void rows_in8(float4 (&v)[8], const float* src, const Rows8& m, int first, int rows) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = first + m.row(i);
+    const float* p = src + (size_t)r * D + m.col;
+    v[2 * i] = r < rows ? load4(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[2 * i + 1] = r < rows ? load4(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+// Eight columns of a row into the operand tile.
+__device__ __forceinline__ void put_pieces8(uint8_t* tile, int row, int col, const float4& a, const float4& b) {
+  uint32_t h[4], m[4], l[4];
+  split3(a.x, a.y, h[0], m[0], l[0]);
+  split3(a.z, a.w, h[1], m[1], l[1]);
+  split3(b.x, b.y, h[2], m[2], l[2]);
+  split3(b.z, b.w, h[3], m[3], l[3]);
+  uint8_t* at = tile + (col >> 6) * ATOM + swz(row, (col & 63) >> 3);
+  *reinterpret_cast<uint4*>(at) = make_uint4(h[0], h[1], h[2], h[3]);
+  *reinterpret_cast<uint4*>(at + PIECE) = make_uint4(m[0], m[1], m[2], m[3]);
+  *reinterpret_cast<uint4*>(at + 2 * PIECE) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+__device__ __forceinline__ float4 norm4(const float4& x, float inv, const float4& g) {
+  return make_float4(x.x * inv * g.x, x.y * inv * g.y, x.z * inv * g.z, x.w * inv * g.w);
+}
+__device__ __forceinline__ float square4(const float4& x) { return fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w))); }
+// Rows of the operand: n = x inv gain, as pieces.  The four lanes of a row, then the four warps of these rows,
+// add up their squares.
+__device__ __forceinline__ void norm_pieces(uint8_t* tile, const float4 (&x)[8], const float* gain, float* part_sums, const Rows8& m) {
+  float ss[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    ss[i] = square4(x[2 * i]) + square4(x[2 * i + 1]);
+    ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 1);
+    ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 2);
+    if ((threadIdx.x & 3) == 0) part_sums[(threadIdx.x >> 7) * TILE + m.row(i)] = ss[i];
+  }
+  asm volatile("bar.sync %0, 128;" ::"r"(3 + ((threadIdx.x >> 5) & 3)) : "memory");
+  const float4 g0 = load4(gain + m.col), g1 = load4(gain + m.col + 4);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float* p = part_sums + m.row(i);
+    const float inv = rsqrtf(((p[0] + p[TILE]) + (p[2 * TILE] + p[3 * TILE])) / (float)D + kRmsEps);
+    put_pieces8(tile, m.row(i), m.col, norm4(x[2 * i], inv, g0), norm4(x[2 * i + 1], inv, g1));
+  }
+}
 
 // ------------------------------------------------------------------ norm -> product -> rows
 
@@ -266,8 +321,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_project(const __grid_constant__ 
   } else {
     const RowMap m = row_map();
     float4 x[8];
-    rows_in(x, a.x, m, first, a.rows);
-    norm_pieces(smem, x, load4(a.gain + m.col), reinterpret_cast<float*>(smem + S_SUMS), m);
+    rows_in8(x, a.x, rows8(), first, a.rows);
+    norm_pieces(smem, x, a.gain, reinterpret_cast<float*>(smem + S_SUMS), rows8());
     post(f.s, B_OP0);
     f.s.wait(B_ACC0, 0, TIMEOUT_ACC);
     tc_fence_after();
@@ -286,58 +341,68 @@ __global__ void __launch_bounds__(THREADS, 1) k_project(const __grid_constant__ 
 
 // ------------------------------------------------------------------ attention
 
-// Running softmax of one query over keys staged sixteen at a time.
+// Running softmax of one query of one head, channels in pairs.
 struct Soft {
-  float m, l, acc[DH];
+  float m, l;
+  F2 acc[DH / 2];
   __device__ __forceinline__ void clear() {
     m = -INFINITY;
     l = 0.f;
 #pragma unroll
-    for (int d = 0; d < DH; ++d) acc[d] = 0.f;
+    for (int d = 0; d < DH / 2; ++d) acc[d] = f2(0.f);
   }
 };
-constexpr int KEYS = 16;
-// kv: staged rows [k (128) | v (128)] at this head's columns; live: bit per key, a key that is not live scores
-// kMaskedScore, as attention.py:101-112 has it.
-__device__ __forceinline__ void absorb(Soft& t, const float (&q)[DH], const float* kv, int n, uint32_t live, float scale) {
-  float s[KEYS], mx = t.m;
+constexpr int KEYS = 16;                        // of a staged chunk, for each of the two warps of a group of queries
+constexpr int KV_HEAD = DH + 4, KV_V = 4 * KV_HEAD, KV_ROW = 2 * KV_V;   // staged key: four heads of k, of v, 4 floats of padding each
+// kv: staged rows at this lane's head; live: bit per key, a key that is not live scores kMaskedScore, as
+// attention.py:101-112 has it.  Four keys a turn, in a loop: the code runs a few times only, and unrolled over all
+// keys its fetch took longer than its arithmetic.
+__device__ __forceinline__ void absorb(Soft& t, const F2 (&q)[DH / 2], const float* kv, int n, uint32_t live, float scale) {
+#pragma unroll 1
+  for (int j0 = 0; j0 < n; j0 += 4, kv += 4 * KV_ROW, live >>= 4) {
+    float s[4], mx = t.m;
 #pragma unroll
-  for (int j = 0; j < KEYS; ++j) {
-    s[j] = -INFINITY;
-    if (j < n) {
-      float a = 0.f, b = 0.f;
+    for (int j = 0; j < 4; ++j) {   // rows past the n-th hold older keys: read, not used
+      F2 a = f2(0.f), b = f2(0.f);
 #pragma unroll
-      for (int d = 0; d < DH; d += 8) {
-        const float4 u = load4(kv + j * 256 + d), v = load4(kv + j * 256 + d + 4);
-        a = fmaf(q[d], u.x, a); a = fmaf(q[d + 1], u.y, a); a = fmaf(q[d + 2], u.z, a); a = fmaf(q[d + 3], u.w, a);
-        b = fmaf(q[d + 4], v.x, b); b = fmaf(q[d + 5], v.y, b); b = fmaf(q[d + 6], v.z, b); b = fmaf(q[d + 7], v.w, b);
+      for (int d = 0; d < DH; d += 4) {
+        const float4 u = load4(kv + j * KV_ROW + d);
+        a = fma(q[d / 2], f2(u.x, u.y), a);
+        b = fma(q[d / 2 + 1], f2(u.z, u.w), b);
       }
-      s[j] = (live >> j) & 1u ? (a + b) * scale : kMaskedScore;
+      const float2 p = halves(a), r = halves(b);
+      s[j] = j0 + j < n ? ((live >> j) & 1u ? ((p.x + p.y) + (r.x + r.y)) * scale : kMaskedScore) : -INFINITY;
+      mx = fmaxf(mx, s[j]);
     }
-    mx = fmaxf(mx, s[j]);
-  }
-  const float corr = expf(t.m - mx);   // exp(-inf) = 0 at the first keys
-  t.m = mx;
-  t.l *= corr;
+    const float corr = expf(t.m - mx);   // exp(-inf) = 0 at the first keys
+    t.m = mx;
+    t.l *= corr;
+    const F2 c2 = f2(corr);
 #pragma unroll
-  for (int d = 0; d < DH; ++d) t.acc[d] *= corr;
+    for (int d = 0; d < DH / 2; ++d) t.acc[d] = mul(t.acc[d], c2);
 #pragma unroll
-  for (int j = 0; j < KEYS; ++j)
-    if (j < n) {
+    for (int j = 0; j < 4; ++j) {
+      if (j0 + j >= n) break;
       const float p = expf(s[j] - mx);
+      const F2 p2 = f2(p);
       t.l += p;
 #pragma unroll
       for (int d = 0; d < DH; d += 4) {
-        const float4 v = load4(kv + j * 256 + 128 + d);
-        t.acc[d] = fmaf(p, v.x, t.acc[d]); t.acc[d + 1] = fmaf(p, v.y, t.acc[d + 1]);
-        t.acc[d + 2] = fmaf(p, v.z, t.acc[d + 2]); t.acc[d + 3] = fmaf(p, v.w, t.acc[d + 3]);
+        const float4 v = load4(kv + j * KV_ROW + KV_V + d);
+        t.acc[d / 2] = fma(p2, f2(v.x, v.y), t.acc[d / 2]);
+        t.acc[d / 2 + 1] = fma(p2, f2(v.z, v.w), t.acc[d / 2 + 1]);
       }
     }
+  }
 }
 
-// One environment and 32 of its queries per CTA: warp = head, lane = query, so that every lane reads the same key
-// (a broadcast).  Keys and values pass through shared memory once per CTA in whole rows; of the bullets only the
-// active slots do, since the others' weight is exactly zero (and the sum is, if none is active).
+// One environment and 128 of its (head, query) pairs per CTA, a lane per pair, head by head: the lanes of a warp
+// read the same key of one head, or of the two that meet in it (broadcasts on different banks).  Two warps share
+// 32 pairs, each takes half of a chunk of 32 keys; the halves meet at the end.  Bound by instructions, which is
+// why lanes hold pairs (37 queries fill 5 warps, a warp per head and 32 queries would be 8) and channels go two at
+// a time.  Keys and values pass through shared memory once per CTA in whole rows, the next chunk's on their way
+// while one is worked on; of the bullets only the active slots do, since the others' weight is exactly zero (and
+// the sum is, if none is active).
 struct AttendArgs {
   const float* qkv;
   const uint8_t* alive;
@@ -348,41 +413,81 @@ struct AttendArgs {
   const uint8_t* active;    // (environments, nb), or null: all
   int nb;
 };
-__global__ void __launch_bounds__(128) k_attend(const __grid_constant__ AttendArgs a) {
-  __shared__ __align__(16) float kv[KEYS * 256];
-  __shared__ int slots[128], counts[4];
+constexpr int KV_BUF = (2 * KEYS + 4) * KV_ROW, ATT_SMEM = 2 * KV_BUF * 4;   // a turn of four may reach past a chunk's last key
+constexpr int ATT_THREADS = 256, ATT_PAIRS = ATT_THREADS / 2, SLOTS = ATT_THREADS;
+template <bool BULLETS>
+__global__ void __launch_bounds__(ATT_THREADS, 2) k_attend(const __grid_constant__ AttendArgs a) {
+  extern __shared__ __align__(16) float kv[];   // two chunks
+  __shared__ int slots[SLOTS], counts[ATT_THREADS / 32];
   wait_for_previous();
   let_next_start();
   const int e = a.env0 + blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tok0 = a.map.env_tok_begin(e), n = a.map.env_tok_count(e), q0 = blockIdx.y * 32;
-  if (q0 >= n) return;
-  const int row = tok0 + min(q0 + lane, n - 1), h = warp * DH;
+  const int tok0 = a.map.env_tok_begin(e), n = a.map.env_tok_count(e), first = blockIdx.y * ATT_PAIRS + 32 * (warp & 3);
+  if ((int)blockIdx.y * ATT_PAIRS >= HEADS * n) return;
+  const bool working = first < HEADS * n;        // the same in the whole warp
+  const int pair = min(first + lane, HEADS * n - 1), head = pair / n, row = tok0 + pair - head * n, half = warp >> 2;
   const float scale = rsqrtf((float)DH);
-  float q[DH];
+  F2 q[DH / 2];
 #pragma unroll
   for (int d = 0; d < DH; d += 4) {
-    const float4 v = load4(a.qkv + (size_t)row * 384 + h + d);
-    q[d] = v.x; q[d + 1] = v.y; q[d + 2] = v.z; q[d + 3] = v.w;
+    const float4 v = load4(a.qkv + (size_t)row * 384 + head * DH + d);
+    q[d / 2] = f2(v.x, v.y);
+    q[d / 2 + 1] = f2(v.z, v.w);
   }
   Soft t;
-  t.clear();
-  for (int k0 = 0; k0 < n; k0 += KEYS) {
-    const int nk = min(KEYS, n - k0);
-    __syncthreads();
-    for (int i = tid; i < nk * 64; i += 128) store4(kv + i * 4, load4(a.qkv + (size_t)(tok0 + k0 + (i >> 6)) * 384 + 128 + (i & 63) * 4));
-    const bool up = lane < nk && (!a.alive || a.alive[tok0 + k0 + lane]);
-    const uint32_t live = __ballot_sync(0xffffffffu, up);
-    __syncthreads();
-    absorb(t, q, kv + h, nk, live, scale);
-  }
-  float out[DH];
-  const float inv = 1.0f / t.l;
+  // count keys in chunks: row_of(k) is key k's [k | v] row, up(k) whether it is live
+  auto walk = [&](int count, auto row_of, auto up) {
+    auto request = [&](int k0) {
+      const uint32_t dst = smem_u32(kv + ((k0 / (2 * KEYS)) & 1) * KV_BUF + ((tid >> 5) & 1) * KV_V + ((tid >> 3) & 3) * KV_HEAD + (tid & 7) * 4);
 #pragma unroll
-  for (int d = 0; d < DH; ++d) out[d] = t.acc[d] * inv;
-  if (a.kvb) {
+      for (int j = 0; j < 8; ++j) {
+        const int k = (tid >> 6) + 4 * j;
+        if (k0 + k < count) cp_async16(dst + k * KV_ROW * 4, row_of(k0 + k) + (tid & 63) * 4);
+      }
+    };
+    __syncthreads();
+    request(0);
+    for (int k0 = 0; k0 < count; k0 += 2 * KEYS) {
+      const int nk = min(2 * KEYS, count - k0);
+      const bool lit = lane < nk && up(k0 + lane);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      const uint32_t live = __ballot_sync(0xffffffffu, lit);
+      __syncthreads();   // this chunk is there for everyone, everyone is done with the one before
+      if (k0 + 2 * KEYS < count) request(k0 + 2 * KEYS);
+      const int mine = half ? nk / 2 : nk - nk / 2, begin = half ? nk - nk / 2 : 0;
+      if (working) absorb(t, q, kv + ((k0 / (2 * KEYS)) & 1) * KV_BUF + begin * KV_ROW + head * KV_HEAD, mine, live >> begin, scale);
+    }
+  };
+  // the two halves: the upper one's through shared memory into the lower one's result
+  auto merge = [&](F2 (&out)[DH / 2], bool add) {
+    float* share = kv + (warp & 3) * 32 * (DH + 2) + lane;
+    __syncthreads();
+    if (half) {
+      share[0] = t.m;
+      share[32] = t.l;
+#pragma unroll
+      for (int d = 0; d < DH / 2; ++d) {
+        const float2 v = halves(t.acc[d]);
+        share[(2 + 2 * d) * 32] = v.x;
+        share[(3 + 2 * d) * 32] = v.y;
+      }
+    }
+    __syncthreads();
+    if (half || !working || (add && !(t.l + share[32] > 0.f))) return;
+    const float m = fmaxf(t.m, share[0]), ea = expf(t.m - m), eb = expf(share[0] - m), inv = 1.0f / (t.l * ea + share[32] * eb);
+    const F2 ca = f2(ea * inv), cb = f2(eb * inv);
+#pragma unroll
+    for (int d = 0; d < DH / 2; ++d)
+      out[d] = fma(t.acc[d], ca, fma(f2(share[(2 + 2 * d) * 32], share[(3 + 2 * d) * 32]), cb, add ? out[d] : f2(0.f)));
+  };
+  F2 out[DH / 2];
+  t.clear();
+  walk(n, [&](int k) { return a.qkv + (size_t)(tok0 + k) * 384 + 128; }, [&](int k) { return !a.alive || a.alive[tok0 + k]; });
+  merge(out, false);
+  if constexpr (BULLETS) {
     t.clear();
     const float* rows = a.kvb + (size_t)blockIdx.x * a.nb * 256;
-    for (int s0 = 0; s0 < a.nb; s0 += 128) {
+    for (int s0 = 0; s0 < a.nb; s0 += SLOTS) {
       const int slot = s0 + tid;
       const bool on = slot < a.nb && (!a.active || a.active[(size_t)e * a.nb + slot]);
       const uint32_t ballot = __ballot_sync(0xffffffffu, on);
@@ -391,28 +496,22 @@ __global__ void __launch_bounds__(128) k_attend(const __grid_constant__ AttendAr
       __syncthreads();
       int at = __popc(ballot & ((1u << lane) - 1)), total = 0;
 #pragma unroll
-      for (int w = 0; w < 4; ++w) {
+      for (int w = 0; w < ATT_THREADS / 32; ++w) {
         if (w < warp) at += counts[w];
         total += counts[w];
       }
       if (on) slots[at] = slot;
-      for (int k0 = 0; k0 < total; k0 += KEYS) {
-        const int nk = min(KEYS, total - k0);
-        __syncthreads();
-        for (int i = tid; i < nk * 64; i += 128) store4(kv + i * 4, load4(rows + (size_t)slots[k0 + (i >> 6)] * 256 + (i & 63) * 4));
-        __syncthreads();
-        absorb(t, q, kv + h, nk, 0xFFFFu, scale);
-      }
+      __syncthreads();
+      walk(total, [&](int k) { return rows + (size_t)slots[k] * 256; }, [](int) { return true; });
     }
-    if (t.l > 0.f) {
-      const float invb = 1.0f / t.l;
-#pragma unroll
-      for (int d = 0; d < DH; ++d) out[d] += t.acc[d] * invb;
-    }
+    merge(out, true);
   }
-  if (q0 + lane < n)
+  if (!half && first + lane < HEADS * n)
 #pragma unroll
-    for (int d = 0; d < DH; d += 4) store4(a.o + (size_t)row * D + h + d, make_float4(out[d], out[d + 1], out[d + 2], out[d + 3]));
+    for (int d = 0; d < DH; d += 4) {
+      const float2 u = halves(out[d / 2]), v = halves(out[d / 2 + 1]);
+      store4(a.o + (size_t)row * D + head * DH + d, make_float4(u.x, u.y, v.x, v.y));
+    }
 }
 
 // ------------------------------------------------------------------ temporal sublayer, first half
@@ -428,12 +527,16 @@ struct FrontArgs {
   int cols, splits;         // columns of a CTA, CTAs per row tile
   BnbTemporalWeights w;
   Image lin1, lin2, gate_a, gate_x, field;
+  const float* decay;       // log sigmoid(Lambda): high parts, low parts
   Waits waits;
 };
 
-__device__ __forceinline__ float rglru(float ga, float gx, float ba, float bx, float lam, float u, float h) {
-  const float rg = sigmoidf_(ga + ba), ig = sigmoidf_(gx + bx);
-  const float a = powf(sigmoidf_(lam), kRglruC * rg);
+// sigmoid(Lambda)^(8 r) from the logarithm of the sigmoid in two parts, so that the product with 8 r keeps the
+// precision a powf has (which took half of the kernel's last phase).
+__device__ __forceinline__ float rglru(float ga, float gx, float ba, float bx, float log_hi, float log_lo, float u, float h) {
+  const float c = kRglruC * sigmoidf_(ga + ba), ig = sigmoidf_(gx + bx);
+  const float e = c * log_hi, rest = fmaf(c, log_lo, fmaf(c, log_hi, -e)), ea = expf(e);
+  const float a = fmaf(ea, rest, ea);
   return a * h + sqrtf(fmaxf((1.0f - a) * (1.0f + a), kGateFloor)) * (ig * u);
 }
 
@@ -449,6 +552,34 @@ __global__ void __launch_bounds__(THREADS, 1) k_front(const __grid_constant__ Fr
   const int tile = blockIdx.x / a.splits, c0 = (blockIdx.x % a.splits) * a.cols;
   const bool ships = tile < a.ship_tiles;
   const uint32_t slot_bytes = (a.cols == 128 ? 256 : 128 + a.cols) * 128;
+  // What comes from the caller is there before the wait: the rows' places, their incoming state.
+  const int item0 = (ships ? tile : tile - a.ship_tiles) * TILE, n_items = ships ? a.map.total_ships : a.map.total_fields();
+  int* token = reinterpret_cast<int*>(smem + S_ROWS);    // token row of each tile row, -1 past the end
+  int* fresh = token + TILE;                             // its incoming state counts as zero
+  const RowMap m = row_map();
+  // Stored conv taps of four of this lane's rows at a time, all loads before the stores of
+  // the new taps (behind them they would wait for each other)
+  float4 taps[12];
+  auto load_taps = [&](int i0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = m.row(i0 + i);
+      const float* h = a.hidden_in + (size_t)(item0 + r) * 4 * D + m.col;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) taps[3 * i + k] = fresh[r] ? make_float4(0.f, 0.f, 0.f, 0.f) : load4(h + (k + 1) * D);
+    }
+  };
+  if (warp < EPI_WARPS) {
+    if (tid < TILE) {
+      const int it = item0 + tid;
+      int row = -1, e = 0;
+      if (it < n_items) row = ships ? a.map.ship_token_row(it, &e) : a.map.field_token_row(it);
+      token[tid] = row;
+      fresh[tid] = row < 0 || (ships && a.reset_env && a.reset_env[e]);
+    }
+    epi_sync();
+    if (ships) load_taps(0);
+  }
   if (warp != LOAD_WARP || !a.waits.weights_early) {
     wait_for_previous();
     let_next_start();
@@ -474,61 +605,73 @@ __global__ void __launch_bounds__(THREADS, 1) k_front(const __grid_constant__ Fr
     tc_commit_if(el, f.s.bars + 8 * B_ACC1);
     f.s.wait(B_ACC1, 0, TIMEOUT_ACC);
   } else {
-    const RowMap m = row_map();
     const uint32_t lane_addr = f.tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const int part = warp >> 2, item0 = (ships ? tile : tile - a.ship_tiles) * TILE;
-    const int n_items = ships ? a.map.total_ships : a.map.total_fields();
-    int* token = reinterpret_cast<int*>(smem + S_ROWS);    // token row of each tile row, -1 past the end
-    int* fresh = token + TILE;                             // its incoming state counts as zero
-    if (tid < TILE) {
-      const int it = item0 + tid;
-      int row = -1, e = 0;
-      if (it < n_items) row = ships ? a.map.ship_token_row(it, &e) : a.map.field_token_row(it);
-      token[tid] = row;
-      fresh[tid] = row < 0 || (ships && a.reset_env && a.reset_env[e]);
-    }
-    epi_sync();
+    const int part = warp >> 2;
     float4 v[8];
+    {
+      const Rows8 in = rows8();
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = token[m.row(i)];
-      v[i] = row >= 0 ? load4(a.x + (size_t)row * D + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < 4; ++i) {
+        const int row = token[in.row(i)];
+        const float* p = a.x + (size_t)row * D + in.col;
+        v[2 * i] = row >= 0 ? load4(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[2 * i + 1] = row >= 0 ? load4(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      norm_pieces(smem, v, a.w.norm1_w, reinterpret_cast<float*>(smem + S_SUMS), in);
     }
-    norm_pieces(smem, v, load4(a.w.norm1_w + m.col), reinterpret_cast<float*>(smem + S_SUMS), m);
     post(f.s, B_OP0);
     f.s.wait(B_ACC0, 0, TIMEOUT_ACC);
     tc_fence_after();
     // linear1: through shared memory (the operand is done with) into the row layout
-    transpose_rows(v, lane_addr + part * 32, smem + warp * 4096, m);
+    uint8_t* own_stage = smem + warp * 4096;
+    stage_rows(lane_addr + part * 32, own_stage, m.lane);
+    __syncwarp();
     if (ships) {
-      float4 cw[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) cw[j] = load4(a.w.conv_w + (m.col + j) * BNB_CONV_KERNEL);
-      const float4 cb = load4(a.w.conv_b + m.col);
       const bool own = (unsigned)(m.col - c0) < (unsigned)a.cols;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int r = m.row(i);
-        float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0, t2 = t0;
-        if (!fresh[r]) {
-          const float* h = a.hidden_in + (size_t)(item0 + r) * 4 * D + m.col;
-          t0 = load4(h + D); t1 = load4(h + 2 * D); t2 = load4(h + 3 * D);
+      for (int i0 = 0; i0 < 8; i0 += 4) {
+        if (i0) load_taps(i0);
+        float4 cw[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) cw[j] = load4(a.w.conv_w + (m.col + j) * BNB_CONV_KERNEL);
+        const float4 cb = load4(a.w.conv_b + m.col);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = m.row(i0 + i);
+          const float4 t0 = taps[3 * i], t1 = taps[3 * i + 1], t2 = taps[3 * i + 2], b1 = staged_row(own_stage, i0 + i, m.lane);
+          if (own && token[r] >= 0) {
+            float* h = a.hidden_out + (size_t)(item0 + r) * 4 * D + m.col;
+            store4(h + D, t1); store4(h + 2 * D, t2); store4(h + 3 * D, b1);
+          }
+          auto conv = [](float p0, float p1, float p2, float p3, const float4& w, float b) {
+            return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(p0, w.x), __fmul_rn(p1, w.y)), __fmul_rn(p2, w.z)), __fmul_rn(p3, w.w)), b);
+          };
+          v[i0 + i] = make_float4(conv(t0.x, t1.x, t2.x, b1.x, cw[0], cb.x), conv(t0.y, t1.y, t2.y, b1.y, cw[1], cb.y),
+                                  conv(t0.z, t1.z, t2.z, b1.z, cw[2], cb.z), conv(t0.w, t1.w, t2.w, b1.w, cw[3], cb.w));
         }
-        if (own && token[r] >= 0) {
-          float* h = a.hidden_out + (size_t)(item0 + r) * 4 * D + m.col;
-          store4(h + D, t1); store4(h + 2 * D, t2); store4(h + 3 * D, v[i]);
-        }
-        auto conv = [](float p0, float p1, float p2, float p3, const float4& w, float b) {
-          return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(p0, w.x), __fmul_rn(p1, w.y)), __fmul_rn(p2, w.z)), __fmul_rn(p3, w.w)), b);
-        };
-        v[i] = make_float4(conv(t0.x, t1.x, t2.x, v[i].x, cw[0], cb.x), conv(t0.y, t1.y, t2.y, v[i].y, cw[1], cb.y),
-                           conv(t0.z, t1.z, t2.z, v[i].z, cw[2], cb.z), conv(t0.w, t1.w, t2.w, v[i].w, cw[3], cb.w));
       }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = staged_row(own_stage, i, m.lane);
     }
     epi_sync();   // every warp has read its part of the stage
 #pragma unroll
     for (int i = 0; i < 8; ++i) put_pieces(smem, m.row(i), m.col, v[i]);
     post(f.s, B_OP1);
+    // per group of 32 own columns: this thread's four columns of biases and decay, two rows of state
+    float4 ba, bx, lh, ll, state[2];
+    const int q = tid & 7;
+    auto load_group = [&](int g) {
+      const int col = c0 + g + 4 * q;
+      ba = load4(a.w.a_b + col); bx = load4(a.w.x_b + col);
+      lh = load4(a.decay + col); ll = load4(a.decay + D + col);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int r = (tid + 512 * k) >> 3;
+        state[k] = fresh[r] ? make_float4(0.f, 0.f, 0.f, 0.f) : load4(a.hidden_in + (size_t)(item0 + r) * 4 * D + col);
+      }
+    };
+    if (ships) load_group(0);
     f.s.wait(B_ACC1, 0, TIMEOUT_ACC);
     tc_fence_after();
     // 32 own columns at a time: the accumulators through the ring's memory (every slot has been read) to 1024
@@ -544,21 +687,21 @@ __global__ void __launch_bounds__(THREADS, 1) k_front(const __grid_constant__ Fr
         for (int q = 0; q < 8; ++q)
           *reinterpret_cast<uint4*>(at + ((q ^ (m.lane & 7)) << 4)) = make_uint4(t[4 * q], t[4 * q + 1], t[4 * q + 2], t[4 * q + 3]);
       }
+      if (g > 0 && ships) load_group(g);
       epi_sync();
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const int r = (tid + 512 * k) >> 3, q = tid & 7, col = c0 + g + 4 * q;
+        const int r = (tid + 512 * k) >> 3, col = c0 + g + 4 * q;
         if (token[r] < 0) continue;
         const uint8_t* at = stage + (r >> 5) * 4096 + (r & 31) * 128 + ((q ^ (r & 7)) << 4);
         const float4 p = *reinterpret_cast<const float4*>(at), l2 = *reinterpret_cast<const float4*>(at + 2 * 16384);
         float4 out = make_float4(gelu_erf(l2.x), gelu_erf(l2.y), gelu_erf(l2.z), gelu_erf(l2.w));
         if (ships) {
           const float4 gx = *reinterpret_cast<const float4*>(at + 16384), u = get_pieces(smem, r, col);
-          const float4 ba = load4(a.w.a_b + col), bx = load4(a.w.x_b + col), lam = load4(a.w.log_lambda + col);
           const size_t at_h = (size_t)(item0 + r) * 4 * D + col;
-          float4 h = fresh[r] ? make_float4(0.f, 0.f, 0.f, 0.f) : load4(a.hidden_in + at_h);
-          h = make_float4(rglru(p.x, gx.x, ba.x, bx.x, lam.x, u.x, h.x), rglru(p.y, gx.y, ba.y, bx.y, lam.y, u.y, h.y),
-                          rglru(p.z, gx.z, ba.z, bx.z, lam.z, u.z, h.z), rglru(p.w, gx.w, ba.w, bx.w, lam.w, u.w, h.w));
+          float4 h = state[k];
+          h = make_float4(rglru(p.x, gx.x, ba.x, bx.x, lh.x, ll.x, u.x, h.x), rglru(p.y, gx.y, ba.y, bx.y, lh.y, ll.y, u.y, h.y),
+                          rglru(p.z, gx.z, ba.z, bx.z, lh.z, ll.z, u.z, h.z), rglru(p.w, gx.w, ba.w, bx.w, lh.w, ll.w, u.w, h.w));
           store4(a.hidden_out + at_h, h);
           out = make_float4(out.x * h.x, out.y * h.y, out.z * h.z, out.w * h.w);
         } else {
@@ -592,13 +735,12 @@ __device__ __forceinline__ float4 peer_load4(uint32_t addr, uint32_t rank) {
   asm volatile(
       "{\n\t.reg .b32 p;\n\tmapa.shared::cluster.u32 p, %4, %5;\n\t"
       "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [p];\n\t}"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank));   // between two cluster barriers
   return v;
 }
 
 // A hidden chunk is 64 gate and 64 up columns in one accumulator of 128.  Its gated product goes back into the
-// columns it came from, as the operand of the down projection: thread pieces of 16 hidden columns at
-// half * 32 + 16 p, packed to eight words, the high piece there, the middle one 8 further, the low one in the up
+// columns it came from, as the operand of the down projection: a thread's 16 hidden columns of a row, packed to eight words, the high piece there, the middle one 8 further, the low one in the up
 // half.  Tensor memory: down 0, output projection 128, two chunks at 256 and 384.
 __device__ __forceinline__ uint32_t hidden_piece(uint32_t p) { return p == 2 ? 64 : 8 * p; }
 
@@ -670,40 +812,59 @@ __global__ void __launch_bounds__(THREADS, 1) k_post(const __grid_constant__ Pos
   } else {
     const RowMap m = row_map();
     const uint32_t lane_addr = f.tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const int part = warp >> 2, half = part & 1;
-    float4 v[8], x[8];
-    rows_in(v, a.o, m, first, a.rows);
-    rows_in(x, a.x, m, first, a.rows);
+    const int part = warp >> 2;
+    {
+      const Rows8 in = rows8();
+      float4 v[8];
+      rows_in8(v, a.o, in, first, a.rows);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) put_pieces(smem, m.row(i), m.col, v[i]);
+      for (int i = 0; i < 4; ++i) put_pieces8(smem, in.row(i), in.col, v[2 * i], v[2 * i + 1]);
+    }
     post(f.s, B_OP0);
-    f.s.wait(B_ACC0, 0, TIMEOUT_ACC);
-    tc_fence_after();
-    transpose_rows(v, lane_addr + 128 + part * 32, smem + warp * 4096, m);
+    {
+      // residual and norm with a thread per row and 32 columns, as the accumulator comes: x in that layout
+      // touches 32 lines a request, but while the product runs
+      const int r = tid & (TILE - 1), row = first + r;
+      float4 x[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = add4(x[i], v[i]);
-    epi_sync();   // every warp has read its part of the stage
-    norm_pieces(smem, x, load4(a.gain + m.col), reinterpret_cast<float*>(smem + S_SUMS), m);
+      for (int q = 0; q < 8; ++q) x[q] = row < a.rows ? load4(a.x + (size_t)row * D + part * 32 + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+      f.s.wait(B_ACC0, 0, TIMEOUT_ACC);
+      tc_fence_after();
+      uint32_t t[32];
+      tmem_ld32(lane_addr + 128 + part * 32, t);
+      float ss = 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        x[q] = add4(x[q], make_float4(__uint_as_float(t[4 * q]), __uint_as_float(t[4 * q + 1]), __uint_as_float(t[4 * q + 2]), __uint_as_float(t[4 * q + 3])));
+        ss += square4(x[q]);
+      }
+      float* sums = reinterpret_cast<float*>(smem + S_SUMS) + r;
+      sums[part * TILE] = ss;
+      asm volatile("bar.sync %0, 128;" ::"r"(3 + (warp & 3)) : "memory");
+      const float inv = rsqrtf(((sums[0] + sums[TILE]) + (sums[2 * TILE] + sums[3 * TILE])) / (float)D + kRmsEps);
+#pragma unroll
+      for (int q = 0; q < 8; q += 2) {
+        const float* g = a.gain + part * 32 + 4 * q;
+        put_pieces8(smem, r, part * 32 + 4 * q, norm4(x[q], inv, load4(g)), norm4(x[q + 1], inv, load4(g + 4)));
+      }
+    }
     post(f.s, B_OP1);
 #pragma unroll 1
-    for (int i = part >> 1; i < chunks; i += 2) {   // two groups of eight warps take turns
+    for (int i = 0; i < chunks; ++i) {
       f.s.wait(B_GU0 + i, 0, TIMEOUT_ACC);
       tc_fence_after();
-      const uint32_t acc = lane_addr + 256 + 128 * (i & 1) + 32 * half;
-#pragma unroll 1
-      for (int p = 0; p < 2; ++p) {
-        uint32_t g[16], u[16], hh[8], hm[8], hl[8];
-        tmem_ld16_nowait(acc + 16 * p, g);
-        tmem_ld16_nowait(acc + 64 + 16 * p, u);
-        tmem_wait_ld();
+      const uint32_t acc = lane_addr + 256 + 128 * (i & 1) + 16 * part;
+      uint32_t g[16], u[16], hh[8], hm[8], hl[8];
+      tmem_ld16_nowait(acc, g);
+      tmem_ld16_nowait(acc + 64, u);
+      tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          split3(gelu_erf(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]),
-                 gelu_erf(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]), hh[j], hm[j], hl[j]);
-        tmem_st8_nowait(acc + 16 * p, hh);
-        tmem_st8_nowait(acc + 16 * p + 8, hm);
-        tmem_st8_nowait(acc + 16 * p + 64, hl);
-      }
+      for (int j = 0; j < 8; ++j)
+        split3(gelu_erf(__uint_as_float(g[2 * j])) * __uint_as_float(u[2 * j]),
+               gelu_erf(__uint_as_float(g[2 * j + 1])) * __uint_as_float(u[2 * j + 1]), hh[j], hm[j], hl[j]);
+      tmem_st8_nowait(acc, hh);
+      tmem_st8_nowait(acc + 8, hm);
+      tmem_st8_nowait(acc + 64, hl);
       tmem_wait_st();
       post(f.s, B_H0 + i);
     }
@@ -729,19 +890,21 @@ __global__ void __launch_bounds__(THREADS, 1) k_post(const __grid_constant__ Pos
   if (warp < EPI_WARPS) {
     // this CTA's rows: the ranks' parts in order, then the residual
     const int rows = TILE / a.cluster;
+#pragma unroll 1
     for (int i = tid; i < rows * 32; i += EPI_THREADS) {
       const int r = rank * rows + (i >> 5), c = i & 31, row = first + r;
       if (row >= a.rows) continue;
       const uint32_t at = base + ((r >> 5) + 4 * (c >> 3)) * 4096 + (r & 31) * 128 + (((c & 7) ^ (r & 7)) << 4);
-      const float4 x = load4(a.x + (size_t)row * D + 4 * c);
+      const float4 res = load4(a.x + (size_t)row * D + 4 * c);
       float4 sum;
       if (a.cluster == 1) {
         sum = *reinterpret_cast<const float4*>(smem + (at - base));
       } else {
         sum = peer_load4(at, 0);
+#pragma unroll 1
         for (int k = 1; k < a.cluster; ++k) sum = add4(sum, peer_load4(at, k));
       }
-      store4(a.y + (size_t)row * D + 4 * c, add4(x, sum));
+      store4(a.y + (size_t)row * D + 4 * c, add4(res, sum));
     }
   }
   if (a.cluster > 1) cluster_sync();   // nobody leaves while its memory is read
@@ -755,7 +918,9 @@ bool configure() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
   if (!done[dev])
-    done[dev] = cudaFuncSetAttribute(k_project, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) == cudaSuccess &&
+    done[dev] = cudaFuncSetAttribute(k_attend<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) == cudaSuccess &&
+                cudaFuncSetAttribute(k_attend<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) == cudaSuccess &&
+                cudaFuncSetAttribute(k_project, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) == cudaSuccess &&
                 cudaFuncSetAttribute(k_front, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) == cudaSuccess &&
                 cudaFuncSetAttribute(k_post, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) == cudaSuccess;
   return done[dev];
@@ -831,6 +996,7 @@ int pack(const BnbSpatialWeights* s, int ns, const BnbTemporalWeights* t, int nt
     add(w.up_w, w.packed, temporal_at(IM_UP_T), F, D);
     add(w.down_w, w.packed, temporal_at(IM_DOWN_T), D, F);
     if (fields) add(w.field_sub_w, w.packed, temporal_at(IM_FIELD), D, D);
+    add(w.log_lambda, w.packed, temporal_at(IM_DECAY), D, 0);
   }
   flush();
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
@@ -854,7 +1020,7 @@ int post_half(Call& c, const float* o, const float* x, float* y, const float* ga
 }  // namespace
 
 size_t spatial_image_bytes() { return spatial_at(IM_KVB) + image_bytes(256, 128); }
-size_t temporal_image_bytes() { return temporal_at(IM_FIELD) + image_bytes(128, 128); }
+size_t temporal_image_bytes() { return temporal_at(IM_DECAY) + 2 * D * sizeof(float); }
 
 int step(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, int n_blocks, int n_spatial, int n_temporal,
          const float* x, const uint8_t* alive, const BnbBullets* bullets, float* y, const float* hidden_in, float* hidden_out,
@@ -882,7 +1048,7 @@ int step(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, i
           rc = project(c, static_cast<const float*>(bullets->tokens) + (size_t)e0 * a.nb * D, w.norm_bullet_w,
                        image(im, spatial_at(IM_KVB), 256), scratch.kvb, (long long)ne * a.nb);
         }
-        if (!rc) rc = c.launch(k_attend, a, dim3((unsigned)ne, (unsigned)((b.max_tokens_per_env + 31) / 32)), 128, 0, 1);
+        if (!rc) rc = c.launch(cross ? k_attend<true> : k_attend<false>, a, dim3((unsigned)ne, (unsigned)((HEADS * b.max_tokens_per_env + ATT_PAIRS - 1) / ATT_PAIRS)), ATT_THREADS, ATT_SMEM, 1);
       }
       if (!rc)
         rc = post_half(c, scratch.o, cur, y, w.norm2_w, image(im, spatial_at(IM_OUT), D), image(im, spatial_at(IM_GATE), F),
@@ -899,7 +1065,8 @@ int step(const BnbSpatialWeights* spatial, const BnbTemporalWeights* temporal, i
       if (!rc) {
         const FrontArgs a{cur, scratch.o, hidden_in + at, hidden_out + at, reset_env, map, ship_tiles, 128 / splits, splits, w,
                           image(im, temporal_at(IM_LIN1), D), image(im, temporal_at(IM_LIN2), D), image(im, temporal_at(IM_A), D),
-                          image(im, temporal_at(IM_X), D), image(im, temporal_at(IM_FIELD), D), c.waits()};
+                          image(im, temporal_at(IM_X), D), image(im, temporal_at(IM_FIELD), D),
+                          reinterpret_cast<const float*>(static_cast<const uint8_t*>(im) + temporal_at(IM_DECAY)), c.waits()};
         rc = c.launch(k_front, a, dim3((unsigned)(tiles * splits)), THREADS, SMEM, 1);
       }
       if (!rc)

@@ -10,6 +10,14 @@ namespace tensor {
 constexpr int EPI_WARPS = 16, EPI_THREADS = 512, MMA_WARP = 16, LOAD_WARP = 17, THREADS = 576;
 enum : int { TIMEOUT_FULL = 101, TIMEOUT_FREE = 102, TIMEOUT_ACC = 103, TIMEOUT_OPERAND = 104 };
 
+// Two floats in one 64-bit register pair: one instruction for two multiply-adds.
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float lo, float hi) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ F2 f2(float both) { return f2(both, both); }
+__device__ __forceinline__ float2 halves(F2 a) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v)); return r; }
+__device__ __forceinline__ F2 mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+
 // What every role needs for its waits.
 struct Sync {
   uint32_t bars;           // shared address of the barrier array
@@ -65,20 +73,23 @@ __device__ __forceinline__ void row_sums(float (&v)[8], float* part_sums, const 
   asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");   // before the next use
 }
 // 32 accumulator columns from the thread-per-row layout of tensor memory to the row layout, through 4 KB of
-// shared memory of the warp's own.
-__device__ __forceinline__ void transpose_rows(float4 (&v)[8], uint32_t taddr, uint8_t* stage, const RowMap& m) {
+// shared memory of the warp's own: in with stage_rows, out with staged_row (i-th request) behind a __syncwarp.
+__device__ __forceinline__ void stage_rows(uint32_t taddr, uint8_t* stage, int lane) {
   uint32_t t[32];
   tmem_ld32(taddr, t);
-  const int r = m.lane;
 #pragma unroll
   for (int q = 0; q < 8; ++q)
-    *reinterpret_cast<uint4*>(stage + r * 128 + ((q ^ (r & 7)) << 4)) = make_uint4(t[4 * q], t[4 * q + 1], t[4 * q + 2], t[4 * q + 3]);
+    *reinterpret_cast<uint4*>(stage + lane * 128 + ((q ^ (lane & 7)) << 4)) = make_uint4(t[4 * q], t[4 * q + 1], t[4 * q + 2], t[4 * q + 3]);
+}
+__device__ __forceinline__ float4 staged_row(const uint8_t* stage, int i, int lane) {
+  const int r = 4 * i + (lane >> 3);
+  return *reinterpret_cast<const float4*>(stage + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+}
+__device__ __forceinline__ void transpose_rows(float4 (&v)[8], uint32_t taddr, uint8_t* stage, const RowMap& m) {
+  stage_rows(taddr, stage, m.lane);
   __syncwarp();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int rr = 4 * i + (m.lane >> 3);
-    v[i] = *reinterpret_cast<const float4*>(stage + rr * 128 + (((m.lane & 7) ^ (rr & 7)) << 4));
-  }
+  for (int i = 0; i < 8; ++i) v[i] = staged_row(stage, i, m.lane);
 }
 
 }  // namespace tensor

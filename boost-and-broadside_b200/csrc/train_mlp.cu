@@ -114,29 +114,22 @@ __device__ __forceinline__ float rcp_fast(float v) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
   return r;
 }
-// Two floats in one 64-bit register pair: one instruction for two multiply-adds.
-struct F2 { unsigned long long v; };
-__device__ __forceinline__ F2 f2(float lo, float hi) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi)); return r; }
-__device__ __forceinline__ F2 f2(float both) { return f2(both, both); }
-__device__ __forceinline__ float2 split(F2 a) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v)); return r; }
-__device__ __forceinline__ F2 mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
 // Phi(x) and exp(-x^2 / 2) for two x: erf by formula 7.1.26 of Abramowitz and Stegun (absolute error 1.5e-7),
 // whose exponential is the density's too.
 __device__ __forceinline__ F2 normal_cdf(F2 x, F2& e) {
-  const float2 xs = split(x);
-  const float2 d = split(fma(f2(fabsf(xs.x), fabsf(xs.y)), f2(0.3275911f * 0.70710678f), f2(1.0f)));
+  const float2 xs = halves(x);
+  const float2 d = halves(fma(f2(fabsf(xs.x), fabsf(xs.y)), f2(0.3275911f * 0.70710678f), f2(1.0f)));
   const F2 t = f2(rcp_fast(d.x), rcp_fast(d.y));
-  const float2 q = split(mul(mul(x, x), f2(-0.72134752f)));   // log2(e) / 2
+  const float2 q = halves(mul(mul(x, x), f2(-0.72134752f)));   // log2(e) / 2
   e = f2(ex2_fast(q.x), ex2_fast(q.y));
   F2 p = fma(t, f2(0.5f * 1.061405429f), f2(0.5f * -1.453152027f));
   p = fma(t, p, f2(0.5f * 1.421413741f));
   p = fma(t, p, f2(0.5f * -0.284496736f));
   p = fma(t, p, f2(0.5f * 0.254829592f));
-  const float2 half = split(mul(mul(p, t), e));               // (1 - erf(|x| / sqrt 2)) / 2
+  const float2 half = halves(mul(mul(p, t), e));               // (1 - erf(|x| / sqrt 2)) / 2
   return f2(xs.x >= 0.f ? 1.0f - half.x : half.x, xs.y >= 0.f ? 1.0f - half.y : half.y);
 }
-__device__ __forceinline__ uint32_t pack_f2(F2 a) { const float2 v = split(a); return pack_bf16(v.x, v.y); }
+__device__ __forceinline__ uint32_t pack_f2(F2 a) { const float2 v = halves(a); return pack_bf16(v.x, v.y); }
 __device__ __forceinline__ F2 acc_pair(const uint32_t* v) { return f2(__uint_as_float(v[0]), __uint_as_float(v[1])); }
 // four values as bfloat16 into an operand tile
 __device__ __forceinline__ void put4(uint8_t* tile, int row, int col, float a, float b, float c, float d) {
