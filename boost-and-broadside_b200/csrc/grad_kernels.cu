@@ -25,9 +25,14 @@
 // an environment whose keys are all dead it is the reference's value too (lse rounds to the bias).
 #include "grad_kernels.h"
 
+#include <algorithm>
+#include <initializer_list>
+#include <vector>
+
 #include "common.cuh"
 #include "launch_count.h"
 #include "train_attention.h"
+#include "train_linear.h"
 #include "train_mlp.h"
 
 namespace bnb {
@@ -1416,11 +1421,16 @@ struct Bufs {
   // bf16 mode at d_model 128, where the gated MLPs run fused (train_mlp.cu)
   int* status;
   uint8_t *images;     // weight images of every sublayer's MLP
+  uint8_t *linears;    // and of its Linears, MAX_LINEARS blocks a sublayer
   uint8_t *n_image, *dy_image;
 };
 
 // Whether the gated MLPs of a call run on the fused kernels, which keep nothing 4 d_model wide.
 bool fused_mlp(int D, bool bf16) { return bf16 && D == 128; }
+
+// Weight blocks of a sublayer's Linears in its image area: q, k, v, out, keys and values of the bullets; or linear1,
+// linear2, a, x, out, field_sub.
+enum : int { L_QKV = 0, L_OUT = 3, L_KVB = 4, L_LIN1 = 0, L_LIN2 = 1, L_GATES = 2, L_OUT_T = 4, L_FIELD = 5, MAX_LINEARS = 6 };
 
 // bf16: the 4D-wide buffers, where they exist at all (see fused_mlp), hold bfloat16.
 void plan(Arena& ar, Bufs& b, int S, int n_images, size_t R, int D, size_t RB, bool bf16) {
@@ -1431,6 +1441,7 @@ void plan(Arena& ar, Bufs& b, int S, int n_images, size_t R, int D, size_t RB, b
   if (fused_mlp(D, bf16)) {
     b.status = reinterpret_cast<int*>(ar.take(64));
     b.images = reinterpret_cast<uint8_t*>(ar.take((size_t)n_images * train_mlp::image_bytes() / 4));
+    b.linears = reinterpret_cast<uint8_t*>(ar.take((size_t)n_images * MAX_LINEARS * train_linear::BLOCK_IMAGE / 4));
     b.n_image = reinterpret_cast<uint8_t*>(ar.take(train_mlp::rows_image_bytes(R) / 4));
     b.dy_image = reinterpret_cast<uint8_t*>(ar.take(train_mlp::rows_image_bytes(R) / 4));
   } else {
@@ -1480,6 +1491,7 @@ struct Ctx {
   bool bf16;   // products round their operands to bfloat16 (the forward ran under autocast)
   cudaStream_t st;
   const uint8_t* mlp_image;   // weight image of the current sublayer's MLP (fused_mlp)
+  const uint8_t* linears;     // and of its Linears, or null: products one by one
   Bufs b;
 };
 
@@ -1652,6 +1664,50 @@ int attn_bwd(const Ctx& c, const AttnBwdArgs& a, int G) {
   return BNB_OK;
 }
 
+const uint8_t* block_image(const Ctx& c, int i) { return c.linears + (size_t)i * train_linear::BLOCK_IMAGE; }
+// n = rmsnorm(x), inv its roots, and the Linears whose weight blocks start at `first`, from their images.
+void norm_linear(const Ctx& c, const float* x, const float* gain, float* n, float* inv, int first, std::initializer_list<float*> out, int ld,
+                 size_t rows) {
+  train_linear::Forward f;
+  f.x = x; f.gain = gain; f.n_out = n; f.inv = inv; f.image = block_image(c, first); f.ld_out = ld; f.rows = rows;
+  f.blocks = (int)out.size();
+  std::copy(out.begin(), out.end(), f.out);
+  train_linear::forward(f, c.b.status, c.st);
+}
+// y = x W^T (+ bias) (+ residual) for a square W.
+void linear(const Ctx& c, const float* x, int first, const float* W, float* y, size_t rows, const float* bias = nullptr,
+            const float* residual = nullptr) {
+  if (!c.linears) {
+    mm(c, NT, x, c.D, W, c.D, y, c.D, (int)rows, c.D, c.D, bias, residual, c.D);
+    return;
+  }
+  train_linear::Forward f;
+  f.x = x; f.image = block_image(c, first); f.out[0] = y; f.bias[0] = bias; f.residual = residual; f.rows = rows;
+  train_linear::forward(f, c.b.status, c.st);
+}
+// Its gradients: d W += dy^T x, dx = dy W.
+void linear_bwd(const Ctx& c, const float* dy, const float* x, int first, const float* W, float* dW, float* dx, size_t rows) {
+  const int D = c.D, M = (int)rows;
+  if (!c.linears) {
+    mm(c, TN, dy, D, x, D, dW, D, D, D, M);
+    mm(c, NN, dy, D, W, D, dx, D, M, D, D);
+    return;
+  }
+  train_linear::Backward b;
+  b.dy[0] = dy; b.n = x; b.image = block_image(c, first); b.d_weight[0] = dW; b.dx = dx; b.rows = rows;
+  train_linear::backward(b, c.b.status, c.st);
+}
+// The gradients behind norm_linear: weights, the norm's gain, and dx = dres + what comes through the norm.
+void norm_linear_bwd(const Ctx& c, std::initializer_list<const float*> dy, int ld, const float* n, int first, std::initializer_list<float*> dW,
+                     const float* x, const float* gain, const float* inv, const float* dres, float* dx, float* d_gain, size_t rows) {
+  train_linear::Backward b;
+  b.ld_dy = ld; b.n = n; b.image = block_image(c, first); b.blocks = (int)dy.size();
+  std::copy(dy.begin(), dy.end(), b.dy);
+  std::copy(dW.begin(), dW.end(), b.d_weight);
+  b.x = x; b.gain = gain; b.inv = inv; b.dres = dres; b.dx = dx; b.d_gain = d_gain; b.rows = rows;
+  train_linear::backward(b, c.b.status, c.st);
+}
+
 // Spatial sublayer, forward part.  Leaves n1 in d[0] (roots in inv[0]), q|k|v in w3[0], the attention
 // output in d[1], x1 in d[2], the bullet norm / keys and values in bul_n / bul_inv / kvb, and what
 // mlp_fwd leaves; writes y when y is given.
@@ -1665,14 +1721,19 @@ void spatial_fwd(const Ctx& c, const BnbSpatialWeights& w, const float* x, const
   const bool reads = bul && w.kv_bullet_w;
   const int nb = reads ? bul->per_env : 0;
   const size_t RB = (size_t)G * nb;
-  rmsnorm_fwd(c, x, w.norm1_w, n1, b.inv[0], R);
-  mmh(c, NT, H_A, n1, D, w.qkv_w, D, qkv, 3 * D, M, 3 * D, D);
-  if (reads) {
-    rmsnorm_fwd(c, bul->tokens, w.norm_bullet_w, b.bul_n, b.bul_inv, RB);
-    mmh(c, NT, H_A, b.bul_n, D, w.kv_bullet_w, D, b.kvb, 2 * D, (int)RB, 2 * D, D);
+  if (c.linears) {
+    norm_linear(c, x, w.norm1_w, n1, b.inv[0], L_QKV, {qkv, qkv + D, qkv + 2 * D}, 3 * D, R);
+    if (reads) norm_linear(c, bul->tokens, w.norm_bullet_w, b.bul_n, b.bul_inv, L_KVB, {b.kvb, b.kvb + D}, 2 * D, RB);
+  } else {
+    rmsnorm_fwd(c, x, w.norm1_w, n1, b.inv[0], R);
+    mmh(c, NT, H_A, n1, D, w.qkv_w, D, qkv, 3 * D, M, 3 * D, D);
+    if (reads) {
+      rmsnorm_fwd(c, bul->tokens, w.norm_bullet_w, b.bul_n, b.bul_inv, RB);
+      mmh(c, NT, H_A, b.bul_n, D, w.kv_bullet_w, D, b.kvb, 2 * D, (int)RB, 2 * D, D);
+    }
   }
   attn_fwd(c, qkv, alive, o, G, NM, reads ? b.kvb : nullptr, reads ? bul->active : nullptr, nb);
-  mm(c, NT, o, D, w.out_w, D, x1, D, M, D, D, nullptr, x, D);            // x1 = x + o Wout^T
+  linear(c, o, L_OUT, w.out_w, x1, R, nullptr, x);            // x1 = x + o Wout^T
   mlp_fwd(c, x1, y, R, w.norm2_w, w.gate_w, w.up_w, w.down_w);
 }
 
@@ -1692,8 +1753,7 @@ int spatial_bwd(const Ctx& c, const BnbSpatialWeights& w, const BnbSpatialGrads&
   if (!have_fwd) spatial_fwd(c, w, x, alive, bul, nullptr, G, NM);
   mlp_bwd(c, x1, dy, dx1, R, w.norm2_w, w.gate_w, w.up_w, w.down_w, dw.norm2_w, dw.gate_w, dw.up_w, dw.down_w);
 
-  mm(c, TN, dx1, D, o, D, dw.out_w, D, D, D, M);
-  mm(c, NN, dx1, D, w.out_w, D, d_o, D, M, D, D);
+  linear_bwd(c, dx1, o, L_OUT, w.out_w, dw.out_w, d_o, R);
   int rc;
   if (train_attn::supported(D, c.H, NM, nb)) {
     train_attn::Call a{};
@@ -1710,6 +1770,16 @@ int spatial_bwd(const Ctx& c, const BnbSpatialWeights& w, const BnbSpatialGrads&
                         bul->active ? 1 : 0};
       if ((rc = attn_bwd(c, cross, G))) return rc;
     }
+  }
+  const size_t square = (size_t)D * D;
+  if (c.linears) {
+    // the bullet tokens feed every sublayer that reads them: their gradient accumulates
+    if (reads)
+      norm_linear_bwd(c, {b.dkvb, b.dkvb + D}, 2 * D, b.bul_n, L_KVB, {dw.kv_bullet_w, dw.kv_bullet_w + square}, bul->tokens, w.norm_bullet_w,
+                      b.bul_inv, d_bullets, d_bullets ? d_bullets : b.bul_dn, dw.norm_bullet_w, RB);
+    norm_linear_bwd(c, {dqkv, dqkv + D, dqkv + 2 * D}, 3 * D, n1, L_QKV, {dw.qkv_w, dw.qkv_w + square, dw.qkv_w + 2 * square}, x, w.norm1_w,
+                    b.inv[0], dx1, dx, dw.norm1_w, R);
+    return BNB_OK;
   }
   if (reads) {
     mmh(c, TN, H_B, b.dkvb, 2 * D, b.bul_n, D, dw.kv_bullet_w, D, 2 * D, D, (int)RB);
@@ -1755,27 +1825,39 @@ void ships_fwd(const Ctx& c, const BnbTemporalWeights& w, const float* x, const 
   const size_t Rs = tg.Rs();
   const int M = (int)Rs, Rr = tg.B * tg.n_rec;
   ShipGeom gm{tg.T, Rr, D, tg.n_rec, tg.B, done};
-  float *xs = b.d[0], *n = b.d[1], *b1 = b.d[2], *u = b.d[3], *za = b.d[4], *zx = b.d[5], *hs = b.d[6], *b2p = b.d[7],
-        *m = b.d[8], *x1 = b.d[9];
+  float *n = b.d[1], *b1 = b.d[2], *u = b.d[3], *za = b.d[4], *zx = b.d[5], *hs = b.d[6], *b2p = b.d[7], *m = b.d[8], *x1 = b.d[9];
   const int sblocks = (int)(((size_t)Rr * D + 255) / 256);
-  gather(c, x, xs, Rs, tg.n_rec, tg.NM, 0);
-  rmsnorm_fwd(c, xs, w.norm1_w, n, b.inv[0], Rs);
-  mmh(c, NT, H_A, n, D, w.linear1_w, D, b1, D, M, D, D);
+  const bool all = tg.Rf() == 0;   // every row is a ship's: nothing to pick out
+  if (!all) gather(c, x, b.d[0], Rs, tg.n_rec, tg.NM, 0);
+  const float* xs = all ? x : b.d[0];
+  if (c.linears) {
+    norm_linear(c, xs, w.norm1_w, n, b.inv[0], L_LIN1, {b1, b2p}, D, Rs);
+  } else {
+    rmsnorm_fwd(c, xs, w.norm1_w, n, b.inv[0], Rs);
+    mmh(c, NT, H_A, n, D, w.linear1_w, D, b1, D, M, D, D);
+    mmh(c, NT, H_A, n, D, w.linear2_w, D, b2p, D, M, D, D);
+  }
   count_launch();
   k_conv_fwd<<<sblocks, 256, 0, c.st>>>(b1, hid, w.conv_w, w.conv_b, u, gm);
-  mm(c, NT, u, D, w.a_w, D, za, D, M, D, D, w.a_b);
-  mm(c, NT, u, D, w.x_w, D, zx, D, M, D, D, w.x_b);
+  if (c.linears) {
+    train_linear::Forward f;
+    f.x = u; f.image = block_image(c, L_GATES); f.blocks = 2; f.rows = Rs;
+    f.out[0] = za; f.out[1] = zx; f.bias[0] = w.a_b; f.bias[1] = w.x_b;
+    train_linear::forward(f, c.b.status, c.st);
+  } else {
+    mm(c, NT, u, D, w.a_w, D, za, D, M, D, D, w.a_b);
+    mm(c, NT, u, D, w.x_w, D, zx, D, M, D, D, w.x_b);
+  }
   count_launch();
   k_scan_fwd<<<sblocks, 256, 0, c.st>>>(za, zx, u, hid, w.log_lambda, hs, gm);
   if (hid_out) {
     count_launch();
     k_final_state<<<sblocks, 256, 0, c.st>>>(hs, b1, hid, hid_out, gm);
   }
-  mmh(c, NT, H_A, n, D, w.linear2_w, D, b2p, D, M, D, D);
   gelu_mul_fwd(c, b2p, hs, m, Rs * D);                                  // m = h * gelu(linear2 n)
-  mm(c, NT, m, D, w.out_w, D, x1, D, M, D, D, nullptr, xs, D);
-  mlp_fwd(c, x1, y ? b.d[14] : nullptr, Rs, w.norm2_w, w.gate_w, w.up_w, w.down_w);
-  if (y) scatter(c, b.d[14], y, Rs, tg.n_rec, tg.NM, 0);
+  linear(c, m, L_OUT_T, w.out_w, x1, Rs, nullptr, xs);
+  mlp_fwd(c, x1, y ? (all ? y : b.d[14]) : nullptr, Rs, w.norm2_w, w.gate_w, w.up_w, w.down_w);
+  if (y && !all) scatter(c, b.d[14], y, Rs, tg.n_rec, tg.NM, 0);
 }
 
 // Non-recurrent path over the field rows (griffin.py:288-317).  Buffers: xf d[0], n d[1], linear1 out
@@ -1787,12 +1869,16 @@ void fields_fwd(const Ctx& c, const BnbTemporalWeights& w, const float* x, float
   const int M = (int)Rf, nf = tg.NM - tg.n_rec;
   float *xf = b.d[0], *n = b.d[1], *c1 = b.d[2], *b1 = b.d[3], *b2p = b.d[4], *m = b.d[5], *x1 = b.d[6];
   gather(c, x, xf, Rf, nf, tg.NM, tg.n_rec);
-  rmsnorm_fwd(c, xf, w.norm1_w, n, b.inv[0], Rf);
-  mmh(c, NT, H_A, n, D, w.linear1_w, D, c1, D, M, D, D);
-  mm(c, NT, c1, D, w.field_sub_w, D, b1, D, M, D, D);
-  mmh(c, NT, H_A, n, D, w.linear2_w, D, b2p, D, M, D, D);
+  if (c.linears) {
+    norm_linear(c, xf, w.norm1_w, n, b.inv[0], L_LIN1, {c1, b2p}, D, Rf);
+  } else {
+    rmsnorm_fwd(c, xf, w.norm1_w, n, b.inv[0], Rf);
+    mmh(c, NT, H_A, n, D, w.linear1_w, D, c1, D, M, D, D);
+    mmh(c, NT, H_A, n, D, w.linear2_w, D, b2p, D, M, D, D);
+  }
+  linear(c, c1, L_FIELD, w.field_sub_w, b1, Rf);
   gelu_mul_fwd(c, b2p, b1, m, Rf * D);
-  mm(c, NT, m, D, w.out_w, D, x1, D, M, D, D, nullptr, xf, D);
+  linear(c, m, L_OUT_T, w.out_w, x1, Rf, nullptr, xf);
   mlp_fwd(c, x1, y ? b.d[14] : nullptr, Rf, w.norm2_w, w.gate_w, w.up_w, w.down_w);
   if (y) scatter(c, b.d[14], y, Rf, nf, tg.NM, tg.n_rec);
 }
@@ -1819,34 +1905,50 @@ int temporal_bwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
     const Bufs& b = c.b;
     const int M = (int)Rs, Rr = tg.B * tg.n_rec;
     ShipGeom gm{tg.T, Rr, D, tg.n_rec, tg.B, done};
-    float *xs = b.d[0], *n = b.d[1], *b1 = b.d[2], *u = b.d[3], *za = b.d[4], *zx = b.d[5], *hs = b.d[6], *b2p = b.d[7],
-          *m = b.d[8], *x1 = b.d[9], *dys = b.d[10], *dx1 = b.d[11], *dm = b.d[12], *dn = b.d[13], *dxs = b.d[14];
+    float *n = b.d[1], *b1 = b.d[2], *u = b.d[3], *za = b.d[4], *zx = b.d[5], *hs = b.d[6], *b2p = b.d[7],
+          *m = b.d[8], *x1 = b.d[9], *dx1 = b.d[11], *dm = b.d[12], *dn = b.d[13];
     const int sblocks = (int)(((size_t)Rr * D + 255) / 256);
+    const bool all = Rf == 0;
+    const float *xs = all ? x : b.d[0], *dys = all ? dy : b.d[10];
+    float* dxs = all ? dx : b.d[14];
     if (!have_fwd) ships_fwd(c, w, x, hid, done, nullptr, nullptr, tg);
-    gather(c, dy, dys, Rs, tg.n_rec, tg.NM, 0);
+    if (!all) gather(c, dy, b.d[10], Rs, tg.n_rec, tg.NM, 0);
     mlp_bwd(c, x1, dys, dx1, Rs, w.norm2_w, w.gate_w, w.up_w, w.down_w, dw.norm2_w, dw.gate_w, dw.up_w, dw.down_w);
 
-    mm(c, TN, dx1, D, m, D, dw.out_w, D, D, D, M);
-    mm(c, NN, dx1, D, w.out_w, D, dm, D, M, D, D);
+    linear_bwd(c, dx1, m, L_OUT_T, w.out_w, dw.out_w, dm, Rs);
     gelu_mul_bwd(c, b2p, hs, dm, b2p, dm, Rs * D);                      // b2p <- d linear2 out, dm <- d h
-    mmh(c, TN, H_B, b2p, D, n, D, dw.linear2_w, D, D, D, M);
-    mm(c, NN, b2p, D, w.linear2_w, D, dn, D, M, D, D);
+    if (!c.linears) {
+      mmh(c, TN, H_B, b2p, D, n, D, dw.linear2_w, D, D, D, M);
+      mm(c, NN, b2p, D, w.linear2_w, D, dn, D, M, D, D);
+    }
     count_launch();
     k_scan_bwd<<<sblocks, 256, 0, c.st>>>(za, zx, u, hs, dm, hid, d_hid_out, d_hid_in, w.log_lambda, dw.log_lambda, gm);
     // za, zx hold d za, d zx; dm the direct part of d u
-    mm(c, TN, za, D, u, D, dw.a_w, D, D, D, M);
-    mm(c, TN, zx, D, u, D, dw.x_w, D, D, D, M);
-    colsum(c, za, dw.a_b, Rs, D);
-    colsum(c, zx, dw.x_b, Rs, D);
-    mm(c, NN, za, D, w.a_w, D, dm, D, M, D, D, nullptr, nullptr, 0, 1);
-    mm(c, NN, zx, D, w.x_w, D, dm, D, M, D, D, nullptr, nullptr, 0, 1);
+    if (c.linears) {
+      train_linear::Backward g;
+      g.dy[0] = za; g.dy[1] = zx; g.n = u; g.image = block_image(c, L_GATES); g.blocks = 2; g.rows = Rs;
+      g.d_weight[0] = dw.a_w; g.d_weight[1] = dw.x_w; g.d_bias[0] = dw.a_b; g.d_bias[1] = dw.x_b;
+      g.dx = dm; g.accumulate = true;
+      train_linear::backward(g, c.b.status, c.st);
+    } else {
+      mm(c, TN, za, D, u, D, dw.a_w, D, D, D, M);
+      mm(c, TN, zx, D, u, D, dw.x_w, D, D, D, M);
+      colsum(c, za, dw.a_b, Rs, D);
+      colsum(c, zx, dw.x_b, Rs, D);
+      mm(c, NN, za, D, w.a_w, D, dm, D, M, D, D, nullptr, nullptr, 0, 1);
+      mm(c, NN, zx, D, w.x_w, D, dm, D, M, D, D, nullptr, nullptr, 0, 1);
+    }
     float* db1 = za;   // free now
     count_launch();
     k_conv_bwd<<<sblocks, 256, 0, c.st>>>(dm, b1, hid, d_hid_out, d_hid_in, w.conv_w, db1, dw.conv_w, dw.conv_b, gm);
-    mmh(c, TN, H_B, db1, D, n, D, dw.linear1_w, D, D, D, M);
-    mm(c, NN, db1, D, w.linear1_w, D, dn, D, M, D, D, nullptr, nullptr, 0, 1);
-    rmsnorm_bwd(c, xs, w.norm1_w, b.inv[0], dn, dx1, dxs, dw.norm1_w, Rs);
-    scatter(c, dxs, dx, Rs, tg.n_rec, tg.NM, 0);
+    if (c.linears) {
+      norm_linear_bwd(c, {db1, b2p}, D, n, L_LIN1, {dw.linear1_w, dw.linear2_w}, xs, w.norm1_w, b.inv[0], dx1, dxs, dw.norm1_w, Rs);
+    } else {
+      mmh(c, TN, H_B, db1, D, n, D, dw.linear1_w, D, D, D, M);
+      mm(c, NN, db1, D, w.linear1_w, D, dn, D, M, D, D, nullptr, nullptr, 0, 1);
+      rmsnorm_bwd(c, xs, w.norm1_w, b.inv[0], dn, dx1, dxs, dw.norm1_w, Rs);
+    }
+    if (!all) scatter(c, dxs, dx, Rs, tg.n_rec, tg.NM, 0);
   }
   if (Rf) {
     const Ctx& c = cf;
@@ -1859,16 +1961,18 @@ int temporal_bwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
     gather(c, dy, dyf, Rf, nf, tg.NM, tg.n_rec);
     mlp_bwd(c, x1, dyf, dx1, Rf, w.norm2_w, w.gate_w, w.up_w, w.down_w, dw.norm2_w, dw.gate_w, dw.up_w, dw.down_w);
 
-    mm(c, TN, dx1, D, m, D, dw.out_w, D, D, D, M);
-    mm(c, NN, dx1, D, w.out_w, D, dm, D, M, D, D);
+    linear_bwd(c, dx1, m, L_OUT_T, w.out_w, dw.out_w, dm, Rf);
     gelu_mul_bwd(c, b2p, b1, dm, b2p, dm, Rf * D);                      // b2p <- d linear2 out, dm <- d b1
-    mm(c, TN, dm, D, c1, D, dw.field_sub_w, D, D, D, M);
-    mm(c, NN, dm, D, w.field_sub_w, D, dc1, D, M, D, D);
-    mmh(c, TN, H_B, dc1, D, n, D, dw.linear1_w, D, D, D, M);
-    mm(c, NN, dc1, D, w.linear1_w, D, dn, D, M, D, D);
-    mmh(c, TN, H_B, b2p, D, n, D, dw.linear2_w, D, D, D, M);
-    mm(c, NN, b2p, D, w.linear2_w, D, dn, D, M, D, D, nullptr, nullptr, 0, 1);
-    rmsnorm_bwd(c, xf, w.norm1_w, b.inv[0], dn, dx1, dxf, dw.norm1_w, Rf);
+    linear_bwd(c, dm, c1, L_FIELD, w.field_sub_w, dw.field_sub_w, dc1, Rf);
+    if (c.linears) {
+      norm_linear_bwd(c, {dc1, b2p}, D, n, L_LIN1, {dw.linear1_w, dw.linear2_w}, xf, w.norm1_w, b.inv[0], dx1, dxf, dw.norm1_w, Rf);
+    } else {
+      mmh(c, TN, H_B, dc1, D, n, D, dw.linear1_w, D, D, D, M);
+      mm(c, NN, dc1, D, w.linear1_w, D, dn, D, M, D, D);
+      mmh(c, TN, H_B, b2p, D, n, D, dw.linear2_w, D, D, D, M);
+      mm(c, NN, b2p, D, w.linear2_w, D, dn, D, M, D, D, nullptr, nullptr, 0, 1);
+      rmsnorm_bwd(c, xf, w.norm1_w, b.inv[0], dn, dx1, dxf, dw.norm1_w, Rf);
+    }
     scatter(c, dxf, dx, Rf, nf, tg.NM, tg.n_rec);
   }
   return BNB_OK;
@@ -1994,9 +2098,31 @@ int prepare_mlps(Ctx& c, const Walk& wk, const BnbSpatialWeights* spatial, const
     }
   }
   if (cudaMemsetAsync(c.b.status, 0, sizeof(int), c.st) != cudaSuccess) return BNB_ERR_LAUNCH;
-  return train_mlp::pack(w, wk.S, c.b.images, c.st);
+  std::vector<const float*> blocks((size_t)wk.S * MAX_LINEARS);
+  const size_t step = (size_t)wk.D * wk.D;
+  s = 0;
+  for (int blk = 0; blk < n_blocks; ++blk) {
+    for (int j = 0; j < n_spatial; ++j, ++s) {
+      const BnbSpatialWeights& sw = spatial[blk * n_spatial + j];
+      const float* kv = sw.kv_bullet_w ? sw.kv_bullet_w : sw.qkv_w;   // absent: never read
+      const float* of[MAX_LINEARS] = {sw.qkv_w, sw.qkv_w + step, sw.qkv_w + 2 * step, sw.out_w, kv, kv + step};
+      std::copy(of, of + MAX_LINEARS, &blocks[(size_t)s * MAX_LINEARS]);
+    }
+    for (int j = 0; j < n_temporal; ++j, ++s) {
+      const BnbTemporalWeights& tw = temporal[blk * n_temporal + j];
+      const float* of[MAX_LINEARS] = {tw.linear1_w, tw.linear2_w, tw.a_w, tw.x_w, tw.out_w, tw.field_sub_w ? tw.field_sub_w : tw.out_w};
+      std::copy(of, of + MAX_LINEARS, &blocks[(size_t)s * MAX_LINEARS]);
+    }
+  }
+  const int rc = train_linear::pack(blocks.data(), (int)blocks.size(), c.b.linears, c.st);
+  return rc ? rc : train_mlp::pack(w, wk.S, c.b.images, c.st);
 }
-const uint8_t* mlp_image(const Ctx& c, int s) { return fused_mlp(c.D, c.bf16) ? c.b.images + (size_t)s * train_mlp::image_bytes() : nullptr; }
+// The images of sublayer s, for the calls that follow.
+void use_images(Ctx& c, int s) {
+  const bool fused = fused_mlp(c.D, c.bf16);
+  c.mlp_image = fused ? c.b.images + (size_t)s * train_mlp::image_bytes() : nullptr;
+  c.linears = fused ? c.b.linears + (size_t)s * MAX_LINEARS * train_linear::BLOCK_IMAGE : nullptr;
+}
 
 }  // namespace
 
@@ -2023,7 +2149,7 @@ int trunk_sequence_fwd_train(const TrunkFwdTrainArgs& a) {
   int s = 0;
   for (int blk = 0; blk < a.n_blocks; ++blk) {
     for (int j = 0; j < a.n_spatial; ++j, ++s) {
-      c.mlp_image = mlp_image(c, s);
+      use_images(c, s);
       float* out = s + 1 == wk.S ? a.y : kept.bound + (size_t)s * wk.R * D;
       Ctx cs = c;
       cs.b = kept.first[s];
@@ -2031,7 +2157,7 @@ int trunk_sequence_fwd_train(const TrunkFwdTrainArgs& a) {
       cur = out;
     }
     for (int j = 0; j < a.n_temporal; ++j, ++s) {
-      c.mlp_image = mlp_image(c, s);
+      use_images(c, s);
       float* out = s + 1 == wk.S ? a.y : kept.bound + (size_t)s * wk.R * D;
       const int slot = blk * a.n_temporal + j;
       const size_t hoff = (size_t)slot * wk.Rr * 4 * D;
@@ -2079,7 +2205,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
       for (int j = 0; j < a.n_spatial; ++j, ++s) {
         inputs[s] = cur;
         if (s + 1 == S) break;
-        c.mlp_image = mlp_image(c, s);
+        use_images(c, s);
         float* out = c.b.bound + (size_t)s * R * D;
         spatial_fwd(c, a.spatial[blk * a.n_spatial + j], cur, a.alive, a.bullets, out, G, NM);
         cur = out;
@@ -2087,7 +2213,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
       for (int j = 0; j < a.n_temporal; ++j, ++s) {
         inputs[s] = cur;
         if (s + 1 == S) break;
-        c.mlp_image = mlp_image(c, s);
+        use_images(c, s);
         float* out = c.b.bound + (size_t)s * R * D;
         const int slot = blk * a.n_temporal + j;
         rc = temporal_fwd(c, c, a.temporal[slot], cur, a.hidden_in + (size_t)slot * Rr * 4 * D, a.done, out, nullptr, wk.tgm);
@@ -2107,7 +2233,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
       float* dout = s == 0 ? a.dx : c.b.ping[s & 1];
       const int slot = blk * a.n_temporal + j;
       const size_t hoff = (size_t)slot * Rr * 4 * D;
-      c.mlp_image = mlp_image(c, s);
+      use_images(c, s);
       Ctx cs = c, cf = c;
       if (have_fwd) {
         cs.b = kept.first[s];
@@ -2123,7 +2249,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
       const int s = blk * (a.n_spatial + a.n_temporal) + j;
       float* dout = s == 0 ? a.dx : c.b.ping[s & 1];
       const int k = blk * a.n_spatial + j;
-      c.mlp_image = mlp_image(c, s);
+      use_images(c, s);
       Ctx cs = c;
       if (have_fwd) cs.b = kept.first[s];
       rc = spatial_bwd(cs, a.spatial[k], a.d_spatial[k], inputs[s], a.alive, a.bullets, a.d_bullets, dcur, dout, G, NM,

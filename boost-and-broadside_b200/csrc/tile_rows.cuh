@@ -91,6 +91,64 @@ __device__ __forceinline__ void transpose_rows(float4 (&v)[8], uint32_t taddr, u
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = staged_row(stage, i, m.lane);
 }
+// four values as bfloat16 into an operand tile
+__device__ __forceinline__ void put4(uint8_t* tile, int row, int col, float a, float b, float c, float d) {
+  *reinterpret_cast<uint2*>(tile + (col >> 6) * CHUNK_BYTES + swz(row, (col & 63) >> 3) + ((col >> 2) & 1) * 8) = make_uint2(pack_bf16(a, b), pack_bf16(c, d));
+}
+// The descriptor of an MN-major operand (two 64-wide atoms CHUNK_BYTES apart): see mma_one for the rest.
+__device__ __forceinline__ uint32_t desc_mn(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | ((CHUNK_BYTES >> 4) << 16); }
+constexpr uint32_t BOTH_MN = (1u << 15) | (1u << 16);
+
+// MMAs over a 128-deep operand pair of K-major tiles: A at a, B at b (low descriptor words), B's second K
+// atom b_atom units further.
+__device__ __forceinline__ void product128(uint32_t el, uint32_t d, uint32_t a, uint32_t b, uint32_t b_atom, uint32_t idesc) {
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k) mma_one<false>(el, d, a + 2 * k, b + 2 * k, idesc, k ? 1u : 0u);
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k) mma_one<false>(el, d, a + 1024 + 2 * k, b + b_atom + 2 * k, idesc, 1u);
+}
+
+
+// Kernel frame: barriers (counts given), tensor memory, status.  smem is the dynamic array itself, on a
+// 1024-byte boundary because nothing static stands in front of it.
+struct Frame {
+  uint64_t* bars;
+  uint32_t* tmem_slot;
+  int* aborted;            // four ints, see mbar_wait
+};
+template <int N>
+__device__ __forceinline__ Frame open_frame(uint8_t* at, int* status, int* host_status, const int (&counts)[N]) {
+  static_assert(N <= 28, "barrier area");
+  Frame f{reinterpret_cast<uint64_t*>(at), reinterpret_cast<uint32_t*>(at + 8 * 28), reinterpret_cast<int*>(at + 8 * 29)};
+  if (threadIdx.x == 0) {
+    f.aborted[0] = *status != 0 ? 1 : 0;
+    f.aborted[1] = DEFAULT_POLL_LIMIT;
+    *reinterpret_cast<int**>(&f.aborted[2]) = host_status;
+#pragma unroll
+    for (int i = 0; i < N; ++i) mbar_init(smem_u32(&f.bars[i]), counts[i]);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 32) {
+    __syncwarp();
+    tmem_alloc(smem_u32(f.tmem_slot), 512);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  return f;
+}
+constexpr int FRAME_BYTES = 256;
+__device__ __forceinline__ void close_frame(const Frame& f, uint32_t tmem) {
+  tc_fence_before();
+  __syncthreads();
+  if (f.aborted[0] && threadIdx.x >= 32 * LOAD_WARP)   // copies may still be on their way here
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    __syncwarp();
+    tmem_dealloc(tmem, 512);
+  }
+}
 
 }  // namespace tensor
 }  // namespace bnb

@@ -105,10 +105,6 @@ struct Args {
   int* host_status;
 };
 
-// The descriptor of an MN-major operand (two 64-wide atoms CHUNK_BYTES apart): see mma_one for the rest.
-__device__ __forceinline__ uint32_t desc_mn(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | ((CHUNK_BYTES >> 4) << 16); }
-constexpr uint32_t BOTH_MN = (1u << 15) | (1u << 16);
-
 __device__ __forceinline__ float rcp_fast(float v) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
@@ -131,10 +127,6 @@ __device__ __forceinline__ F2 normal_cdf(F2 x, F2& e) {
 }
 __device__ __forceinline__ uint32_t pack_f2(F2 a) { const float2 v = halves(a); return pack_bf16(v.x, v.y); }
 __device__ __forceinline__ F2 acc_pair(const uint32_t* v) { return f2(__uint_as_float(v[0]), __uint_as_float(v[1])); }
-// four values as bfloat16 into an operand tile
-__device__ __forceinline__ void put4(uint8_t* tile, int row, int col, float a, float b, float c, float d) {
-  *reinterpret_cast<uint2*>(tile + (col >> 6) * CHUNK_BYTES + swz(row, (col & 63) >> 3) + ((col >> 2) & 1) * 8) = make_uint2(pack_bf16(a, b), pack_bf16(c, d));
-}
 // n = bf16(x inv gain) into an operand tile; inv[i] of this lane's rows on the way
 __device__ __forceinline__ void norm_rows(uint8_t* tile, const float4 (&x)[8], float (&inv)[8], const float4& gain, float* part_sums, const RowMap& m) {
 #pragma unroll
@@ -144,46 +136,6 @@ __device__ __forceinline__ void norm_rows(uint8_t* tile, const float4 (&x)[8], f
   for (int i = 0; i < 8; ++i) {
     inv[i] = rsqrtf(inv[i] * (1.0f / D) + kRmsEps);
     put4(tile, m.row(i), m.col, x[i].x * inv[i] * gain.x, x[i].y * inv[i] * gain.y, x[i].z * inv[i] * gain.z, x[i].w * inv[i] * gain.w);
-  }
-}
-// Kernel frame: barriers (counts given), tensor memory, status.  smem is the dynamic array itself, on a
-// 1024-byte boundary because nothing static stands in front of it.
-struct Frame {
-  uint64_t* bars;
-  uint32_t* tmem_slot;
-  int* aborted;            // four ints, see mbar_wait
-};
-template <int N>
-__device__ __forceinline__ Frame open_frame(uint8_t* at, const Args& a, const int (&counts)[N]) {
-  static_assert(N <= 28, "barrier area");
-  Frame f{reinterpret_cast<uint64_t*>(at), reinterpret_cast<uint32_t*>(at + 8 * 28), reinterpret_cast<int*>(at + 8 * 29)};
-  if (threadIdx.x == 0) {
-    f.aborted[0] = *a.status != 0 ? 1 : 0;
-    f.aborted[1] = DEFAULT_POLL_LIMIT;
-    *reinterpret_cast<int**>(&f.aborted[2]) = a.host_status;
-#pragma unroll
-    for (int i = 0; i < N; ++i) mbar_init(smem_u32(&f.bars[i]), counts[i]);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (threadIdx.x < 32) {
-    __syncwarp();
-    tmem_alloc(smem_u32(f.tmem_slot), 512);
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  return f;
-}
-constexpr int FRAME_BYTES = 256;
-__device__ __forceinline__ void close_frame(const Frame& f, uint32_t tmem) {
-  tc_fence_before();
-  __syncthreads();
-  if (f.aborted[0] && threadIdx.x >= 32 * LOAD_WARP)   // copies may still be on their way here
-    for (int i = 0; i < 64; ++i) __nanosleep(1000);
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    __syncwarp();
-    tmem_dealloc(tmem, 512);
   }
 }
 // One fetch by the fetching warp: wait for the slot, copy, signal.  Stops after a wait has run out.
@@ -198,15 +150,6 @@ __device__ __forceinline__ bool fetch(const Sync& s, int full, int done, uint32_
   __syncwarp();
   return true;
 }
-// MMAs over a 128-deep operand pair of K-major tiles: A at a, B at b (low descriptor words), B's second K
-// atom b_atom units further.
-__device__ __forceinline__ void product128(uint32_t el, uint32_t d, uint32_t a, uint32_t b, uint32_t b_atom, uint32_t idesc) {
-#pragma unroll
-  for (uint32_t k = 0; k < 4; ++k) mma_one<false>(el, d, a + 2 * k, b + 2 * k, idesc, k ? 1u : 0u);
-#pragma unroll
-  for (uint32_t k = 0; k < 4; ++k) mma_one<false>(el, d, a + 1024 + 2 * k, b + b_atom + 2 * k, idesc, 1u);
-}
-
 // ------------------------------------------------------------------ forward
 
 // Shared memory: n (32 KB), three gate|up slots (32 KB), three down slots (16 KB), row sums, frame.
@@ -223,7 +166,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
   extern __shared__ __align__(1024) uint8_t smem[];
   const int counts[FB_COUNT] = {EPI_WARPS, EPI_WARPS / 2, EPI_WARPS / 2, EPI_WARPS / 2, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
   const int tid = threadIdx.x, warp = tid >> 5;
-  const Frame f = open_frame(smem + FW_FRAME, a, counts);
+  const Frame f = open_frame(smem + FW_FRAME, a.status, a.host_status, counts);
   const Sync s{smem_u32(f.bars), a.status, f.aborted};
   const uint32_t tmem = *f.tmem_slot;
   const int my_tiles = (int)blockIdx.x < a.tiles ? (a.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
@@ -360,7 +303,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
   extern __shared__ __align__(1024) uint8_t smem[];
   const int counts[XB_COUNT] = {EPI_WARPS, EPI_WARPS / 2, EPI_WARPS / 2, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
   const int tid = threadIdx.x, warp = tid >> 5;
-  const Frame f = open_frame(smem + DX_FRAME, a, counts);
+  const Frame f = open_frame(smem + DX_FRAME, a.status, a.host_status, counts);
   const Sync s{smem_u32(f.bars), a.status, f.aborted};
   const uint32_t tmem = *f.tmem_slot;
   const int my_tiles = (int)blockIdx.x < a.tiles ? (a.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
@@ -540,7 +483,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dw(const __grid_constant__ A
   extern __shared__ __align__(1024) uint8_t smem[];
   const int counts[WB_COUNT] = {1, 1, EPI_WARPS, EPI_WARPS, 1, 1, 1, 1, 1};
   const int tid = threadIdx.x, warp = tid >> 5;
-  const Frame f = open_frame(smem + DW_FRAME, a, counts);
+  const Frame f = open_frame(smem + DW_FRAME, a.status, a.host_status, counts);
   const Sync s{smem_u32(f.bars), a.status, f.aborted};
   const uint32_t tmem = *f.tmem_slot;
   // CTAs of eight neighbouring indices share their row tiles (one chunk each): a tile comes from HBM once
