@@ -151,6 +151,14 @@ constexpr int kEngineSimt = BNB_ENGINE_SIMT;
 const void* ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 
 Tensor f32c(const Tensor& t) {
+  if (t.scalar_type() == at::kBFloat16 && t.is_cuda() && t.is_contiguous() && t.numel() % 8 == 0 &&
+      reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0) {
+    const c10::cuda::CUDAGuard guard(t.device());
+    const Tensor f = at::empty(t.sizes(), t.options().dtype(at::kFloat));
+    if (bnb::host::widen(t.data_ptr(), static_cast<float*>(f.data_ptr()), (size_t)t.numel(), at::cuda::getCurrentCUDAStream(t.device().index()).stream()) != BNB_OK)
+      throw std::runtime_error("the bfloat16 conversion could not be launched");
+    return f;
+  }
   const Tensor f = t.scalar_type() == at::kFloat ? t : t.to(at::kFloat);
   return f.is_contiguous() ? f : f.contiguous();
 }
