@@ -554,7 +554,12 @@ __device__ __forceinline__ void run_spatial_pre(Epi& e, const SubLayer& s, size_
     tmem_ld32(e.lane_addr + COL_ACC0 + h * 96 + p * 32, v);
     if (row_valid) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(dst + p * D + q * 8) = pack8(&v[q * 8]);
+      for (int q = 0; q < 2; ++q) {
+        float w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = __uint_as_float(pack_bf16(__uint_as_float(v[q * 16 + 2 * j]), __uint_as_float(v[q * 16 + 2 * j + 1])));
+        store8(reinterpret_cast<float*>(dst + p * D + q * 16), w, e.wide);
+      }
     }
   }
   tc_fence_before();
@@ -562,13 +567,16 @@ __device__ __forceinline__ void run_spatial_pre(Epi& e, const SubLayer& s, size_
 // Second part: the attention output (bf16, (rows, 128)) becomes the A operand of out_proj, which
 // accumulates into the residual; then norm2 and the GatedMLP.
 __device__ __forceinline__ void run_spatial_post(Epi& e, const SubLayer& s, size_t grow, bool row_valid) {
-  const uint4* src = reinterpret_cast<const uint4*>(s.o_in + grow * D + e.part * 32);
+  const float* src = reinterpret_cast<const float*>(s.o_in + grow * D + e.part * 32);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int col = e.part * 32 + q * 8;
-    uint4 o = make_uint4(0u, 0u, 0u, 0u);
-    if (row_valid) o = src[q];
-    *reinterpret_cast<uint4*>(e.smem + OFF_A + (col >> 6) * CHUNK_BYTES + swz(e.row, (col & 63) >> 3)) = o;
+  for (int q = 0; q < 2; ++q) {
+    float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (row_valid) load8(o, src + 8 * q, e.wide);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int col = e.part * 32 + q * 16 + j * 8;
+      *reinterpret_cast<float4*>(e.smem + OFF_A + (col >> 6) * CHUNK_BYTES + swz(e.row, (col & 63) >> 3)) = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+    }
   }
   post(e, B_OP0);
   wait_round(e, 1);   // out_proj accumulated into the residual

@@ -21,30 +21,12 @@ constexpr int N_SPATIAL_CHUNKS = 34;       // chunks of a spatial sublayer prope
 constexpr int N_BULLET_CHUNKS = 4;         // kv_bullet: keys (2 K atoms), values (2 K atoms); zero when absent
 constexpr int N_SPATIAL_IMAGE = N_SPATIAL_CHUNKS + N_BULLET_CHUNKS;
 constexpr int N_TEMPORAL_CHUNKS = 36;
-constexpr int STAGE_STRIDE = 208;        // bytes per staged q|k|v row (96 bf16 + pad)
 constexpr int MAX_SUBLAYERS = 8;
-
-// shared memory map (offsets from a 1024-aligned base)
-constexpr int OFF_A = 0;                 // 32 KB
-constexpr int OFF_P = 32768;             // 16 KB
-constexpr int OFF_RING = 49152;          // 2 x 16 KB
-constexpr int OFF_STAGE = 81920;         // 128 x 208 = 26624
-constexpr int OFF_META = 108544;         // env_first[128], env_n[128], alive[128], items[128]
-constexpr int OFF_BAR = 109056;          // full[2], empty[2], acc, tmem base
-constexpr int OFF_SS = 109120;           // partial sums of squares, up to 4 x 128 floats
-constexpr int OFF_ROWINFO = 111168;      // hidden row of each tile row (int, -1 = no state), then flags
-constexpr int SMEM_BYTES = 111168 + 512 + 128 + 1024;
-
-constexpr uint32_t TMEM_COLS = 256;
-constexpr uint32_t COL_RESID = 0;
-constexpr uint32_t COL_ACC = 128;
 
 // SUB_SPATIAL_PRE / _POST split a spatial sublayer around a separate attention kernel
 // (environments larger than one tile): PRE = norm1 + QKV to global scratch, POST = attention
 // output from scratch + out_proj + norm2 + GatedMLP.
-// SUB_BULLET_KV runs over bullet rows instead of token rows: norm_bullet + kv_bullet, keys and
-// values written as bf16 to global scratch for the attention kernel; it leaves no residual.
-enum : int { SUB_SPATIAL = 0, SUB_TEMPORAL = 1, SUB_SPATIAL_PRE = 2, SUB_SPATIAL_POST = 3, SUB_BULLET_KV = 4 };
+enum : int { SUB_SPATIAL = 0, SUB_TEMPORAL = 1, SUB_SPATIAL_PRE = 2, SUB_SPATIAL_POST = 3 };
 enum : int { ST_TIMEOUT_FULL = 101, ST_TIMEOUT_EMPTY = 102, ST_TIMEOUT_ACC = 103 };
 
 struct SubLayer {
@@ -59,7 +41,6 @@ struct SubLayer {
   float* hid_out;
   __nv_bfloat16* qkv_out;        // PRE: (rows, 384) q|k|v, head-major inside each third
   const __nv_bfloat16* o_in;     // POST: (rows, 128) attention output
-  __nv_bfloat16* kvb_out;        // BULLET_KV: (rows, 256) k | v of the bullet rows
 };
 
 struct TrunkArgs {
@@ -79,10 +60,6 @@ struct TrunkArgs {
   int flat_rows;      // 1: tiles are plain 128-row slices of the token rows (no attention inside)
   const int* tile_env_begin;  // ragged batches: range of each tile in tile_env_ids (+ end), else null
   const int* tile_env_ids;    // ragged batches: environments in tile order
-  // Bullet key/value program only: tile row r reads input row row_index[r], and only the first
-  // *n_rows_dev rows exist (the active bullets, compacted on the device); null = all rows, in order.
-  const int* row_index;
-  const int* n_rows_dev;
   int* status;
   int* host_status;   // pinned host word that a wait which runs out writes its code to, or null
   // Test hooks of the bounded waits (0 / -1 in normal use): the poll limit of this launch, and the
@@ -90,7 +67,7 @@ struct TrunkArgs {
   // lane's wait for it runs out and the kernel has to drain and return with a status code.
   int poll_limit;
   int skip_op;
-  int wide;      // x, y and every hidden state are 32-byte aligned
+  int wide;      // x, y, every hidden state and the split path's buffers are 32-byte aligned
   int io_bf16;   // x and y hold bfloat16 (BNB_BF16_IO) instead of float32
   SubLayer sub[MAX_SUBLAYERS];
 };
@@ -143,33 +120,12 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Named barriers of the epilogue threads (ids 1 and 2; id 0 is __syncthreads).
-template <int NQ>
-__device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(128 * NQ) : "memory"); }
-template <int NQ>
-__device__ __forceinline__ void wake_barrier() { asm volatile("bar.sync 2, %0;" ::"n"(128 * NQ) : "memory"); }
-
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// D[tmem] (+)= A[smem] * B[smem]^T, bf16 operands, fp32 accumulate, M = 128.
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// Shared-memory operand descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 // Instruction descriptor: fp32 accumulator, bf16 A and B, both K-major, M = 128, N = n.
 __device__ __forceinline__ uint32_t instr_desc(uint32_t n) {
