@@ -19,7 +19,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libbnb_trunk.so")
 HOST_MODULE = os.path.join(HERE, "_host_path.so")
-SOURCES = ["capi.cu", "exact_kernels.cu", "tensor_kernels.cu", "bullet_kv.cu", "pipelined_tile_kernel.cu", "static_scratch.cu", "grad_kernels.cu", "mlp_kernels.cu", "policy_tail.cu", "train_attention.cu", "train_mlp.cu", "train_linear.cu", "split_kernels.cu"]
+SOURCES = ["capi.cu", "exact_kernels.cu", "tensor_kernels.cu", "bullet_kv.cu", "pipelined_tile_kernel.cu", "static_scratch.cu", "grad_kernels.cu", "mlp_kernels.cu", "head_tiles.cu", "policy_tail.cu", "train_attention.cu", "train_mlp.cu", "train_linear.cu", "split_kernels.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC",

@@ -22,6 +22,7 @@
 #include "mlp_kernels.h"
 
 #include "common.cuh"
+#include "head_tiles.h"
 #include "launch_count.h"
 #include "tensor_common.cuh"
 
@@ -444,6 +445,7 @@ int run(const MlpCall& call, int n_chains, int in_pad, int hidden, int out_dim, 
   if (call.n_rows <= 0) return BNB_OK;
   for (int i = 0; i < n_chains; ++i)
     if (reinterpret_cast<uintptr_t>(call.chain[i].y) & 3) return BNB_ERR_MISALIGNED;
+  if (head_tiles_serve(call, n_chains, in_pad, hidden, out_dim)) return head_tiles(call, n_chains, out_dim, st);
   const Layout L = layout(in_pad, hidden, out_dim);
   using Kernel = void (*)(MlpCall);
 #define BNB_MLP_ROW(NP2, NCH) {k_mlp_bf16<NP2, NCH, 2>, k_mlp_bf16<NP2, NCH, 4>, k_mlp_bf16<NP2, NCH, 6>, k_mlp_bf16<NP2, NCH, 8>}
