@@ -53,6 +53,13 @@ __device__ __forceinline__ void rows_in(float4 (&v)[8], const float* src, const 
     v[i] = r < rows ? *reinterpret_cast<const float4*>(src + (size_t)r * D + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
+// Asks L2 for the rows of a tile, `bytes` each, one behind the other (a multiple of 16): their loads, a tile later, then
+// find them there.  One thread.
+__device__ __forceinline__ void prefetch_rows(const void* src, int tile, int rows, uint32_t bytes) {
+  const int first = tile * TILE, n = rows - first < TILE ? rows - first : TILE;
+  if (n <= 0) return;
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(static_cast<const uint8_t*>(src) + (size_t)first * bytes), "r"((uint32_t)n * bytes) : "memory");
+}
 // Per-row sums of one value per request: over the eight lanes of a row here, over the four column parts
 // through shared memory.  Returns the totals of this lane's rows; two barriers of the four warps of these rows.
 __device__ __forceinline__ void row_sums(float (&v)[8], float* part_sums, const RowMap& m) {

@@ -176,7 +176,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
     const bool elected = elect_one() != 0;
     uint32_t pair = 0, single = 3, par = 0x3F;   // a fresh barrier passes a wait on parity 1
     bool go = true;
-    for (int t = 0; t < my_tiles && go; ++t)
+    for (int t = 0; t < my_tiles && go; ++t) {
+      if (elected) prefetch_rows(a.x1, blockIdx.x + (t + 1) * gridDim.x, a.rows, D * 4);
 #pragma unroll 1
       for (int i = 0; i < 16 && go; ++i) {
         // GU0 GU1 GU2 D0 GU3 D1 ... GU7 D5 D6 D7
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
                    down ? 16384 : 32768, elected);
         par ^= 1u << slot;
       }
+    }
   } else if (warp == MMA_WARP) {
     const uint32_t base = smem_u32(smem), el = elect_one(), tm = uniform(tmem);
     const uint32_t n_lo = desc_lo(base), idesc = instr_desc(128);
@@ -314,7 +316,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
     uint32_t par1 = 3, par2 = 3;
     bool go = true;
     // W1(0) W1(1) then W2(c), W1(c + 2)
-    for (int t = 0; t < my_tiles && go; ++t)
+    for (int t = 0; t < my_tiles && go; ++t) {
+      if (elected) {
+        prefetch_rows(a.x1, blockIdx.x + (t + 1) * gridDim.x, a.rows, D * 4);
+        prefetch_rows(a.dy, blockIdx.x + (t + 1) * gridDim.x, a.rows, D * 4);
+      }
 #pragma unroll 1
       for (int i = 0; i < 16 && go; ++i) {
         const bool second = i >= 2 && (!(i & 1) || i > 13);
@@ -329,6 +335,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
           par1 ^= 1u << slot;
         }
       }
+    }
   } else if (warp == MMA_WARP) {
     const uint32_t base = smem_u32(smem), el = elect_one(), tm = uniform(tmem);
     const uint32_t n_lo = desc_lo(base), dy_lo = desc_lo(base + DX_DY), id128 = instr_desc(128), id64 = instr_desc(64);
