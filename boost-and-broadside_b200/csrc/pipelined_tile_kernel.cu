@@ -934,6 +934,9 @@ __device__ __forceinline__ void issue_temporal(Issuer& m, bool has_fields) {
 
 // ------------------------------------------------------------------ the kernel
 
+// WHOLE: programs of whole sublayers on tiles of whole environments, most calls by far; the code they do not need cost
+// them registers and instruction fetches.
+template <bool WHOLE>
 __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_constant__ TrunkArgs args) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1050,9 +1053,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
           if (type == SUB_TEMPORAL) {
             issue_temporal(m, args.has_fields != 0);
           } else {
-            if (type != SUB_SPATIAL_POST) issue_qkv(m);
-            if (type == SUB_SPATIAL_PRE) continue;
-            issue_out_proj(m, type == SUB_SPATIAL_POST ? OFF_A : OFF_P);
+            if (WHOLE || type != SUB_SPATIAL_POST) issue_qkv(m);
+            if (!WHOLE && type == SUB_SPATIAL_PRE) continue;
+            issue_out_proj(m, !WHOLE && type == SUB_SPATIAL_POST ? OFF_A : OFF_P);
           }
           issue_ffn(m);
         }
@@ -1105,7 +1108,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       int env, tok, env_first, env_n, env_ships;
       size_t grow = 0;
       int hrow_if_ship;
-      if (args.flat_rows) {
+      if (!WHOLE && args.flat_rows) {
         // plain 128-row slices of the token rows (programs without attention inside: the
         // environments are larger than a tile); the environment of a row is looked up
         const int r = eb * TILE + row;
@@ -1220,6 +1223,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
             for (int l = 0; l < 4; ++l) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + l * 128));
           }
           if (s.type == SUB_SPATIAL) run_spatial(e, n_items, valid);
+          else if (WHOLE) run_temporal(e, s, rs, is_field, boundary, args.has_fields != 0, t == 0 ? s.hid_in : s.hid_out);
           else if (s.type == SUB_SPATIAL_PRE) run_spatial_pre(e, s, trow, valid);
           else if (s.type == SUB_SPATIAL_POST) run_spatial_post(e, s, trow, valid);
           else run_temporal(e, s, rs, is_field, boundary, args.has_fields != 0, t == 0 ? s.hid_in : s.hid_out);
@@ -1277,13 +1281,17 @@ int launch_pipelined(const TrunkArgs& a, cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BNB_ERR_NO_DEVICE;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(pipe::k_trunk_pipelined, cudaFuncAttributeMaxDynamicSharedMemorySize, pipe::SMEM_BYTES) != cudaSuccess)
+    if (cudaFuncSetAttribute(pipe::k_trunk_pipelined<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pipe::SMEM_BYTES) != cudaSuccess ||
+        cudaFuncSetAttribute(pipe::k_trunk_pipelined<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, pipe::SMEM_BYTES) != cudaSuccess)
       return BNB_ERR_LAUNCH;
     configured[dev] = true;
   }
   const int grid = a.n_tiles < 148 ? a.n_tiles : 148;
   count_launch();
-  pipe::k_trunk_pipelined<<<grid, pipe::THREADS, pipe::SMEM_BYTES, st>>>(a);
+  bool whole = !a.flat_rows;
+  for (int i = 0; i < a.n_sub; ++i) whole = whole && (a.sub[i].type == SUB_SPATIAL || a.sub[i].type == SUB_TEMPORAL);
+  if (whole) pipe::k_trunk_pipelined<true><<<grid, pipe::THREADS, pipe::SMEM_BYTES, st>>>(a);
+  else pipe::k_trunk_pipelined<false><<<grid, pipe::THREADS, pipe::SMEM_BYTES, st>>>(a);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
 }
 
