@@ -234,7 +234,7 @@ __device__ __forceinline__ float4 add4(const float4& a, const float4& b) { retur
 
 // How rows come in: warp w takes rows 32 (w % 4) .. and columns 32 (w / 4) .., in its i-th request (i < 4) lane l
 // eight columns of row 8 i + l / 4.  A request touches eight lines, and a piece of eight columns is sixteen
-// bytes of the operand tile, stored without bank conflicts.
+// bytes of the operand tile, stored with two lanes to a bank at most.
 struct Rows8 {
   int row0, col;
   __device__ __forceinline__ int row(int i) const { return row0 + 8 * i + ((threadIdx.x & 31) >> 2); }

@@ -393,8 +393,8 @@ int bnb_trunk_sequence_bwd(const BnbSpatialWeights* spatial, const BnbTemporalWe
                            void* stream);
 
 /* Bytes of activations bnb_trunk_sequence_fwd_train keeps for the backward (for two blocks of two
- * spatial and one temporal sublayer at d_model 128: about 65 KB per token row with BNB_FP32, 47 KB
- * with BNB_BF16, where the 4 d_model-wide buffers of the gated MLPs hold bfloat16); 0 for a geometry
+ * spatial and one temporal sublayer at d_model 128: about 65 KB per token row with BNB_FP32, 23 KB
+ * with BNB_BF16, where nothing 4 d_model wide is kept); 0 for a geometry
  * the backward does not cover.  Sizes depend on the precision: query with the call's. */
 size_t bnb_trunk_kept_bytes(int n_blocks, int n_spatial, int n_temporal, int d_model, int n_heads,
                             const BnbBatch* batch, int timesteps, int bullets_per_env, int precision);
