@@ -1,5 +1,5 @@
 """Bullet keys and values at the edges of their row tiles: active rows 0, 1, around one tile, above one tile per SM,
-every row without a mask, both token types, against the exact kernels."""
+every row without a mask, both token types, environments around the single-CTA compaction, against the exact kernels."""
 
 import pytest
 import torch
@@ -11,7 +11,7 @@ DEV = "cuda"
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("B,NB,active", [(3, 5, 0), (3, 5, 1), (2, 64, 127), (2, 64, 128), (3, 43, 129), (1, 1, None), (300, 80, 19000), (3, 43, None)])
+@pytest.mark.parametrize("B,NB,active", [(3, 5, 0), (3, 5, 1), (2, 64, 127), (2, 64, 128), (3, 43, 129), (1, 1, None), (300, 80, 19000), (3, 43, None), (255, 3, 300), (256, 33, 3000), (257, 2, 200)])
 def test_bullet_rows(B, NB, active, dtype):
     from boost_and_broadside_b200 import _capi
 
