@@ -1528,7 +1528,18 @@ struct Ctx {
   const uint8_t* mlp_image;   // weight image of the current sublayer's MLP (fused_mlp)
   const uint8_t* linears;     // and of its Linears, or null: products one by one
   Bufs b;
+  // The first status of the call that is not BNB_OK.  The row-tile kernels test their own launches, which takes the
+  // error out of cudaGetLastError: what they return is the only trace of it.
+  int* failed;
+  void note(int rc) const {
+    if (rc && !*failed) *failed = rc;
+  }
 };
+// The status of everything launched so far under this context; takes a pending launch error with it.
+int status_of(const Ctx& c) {
+  c.note(cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH);
+  return *c.failed;
+}
 
 void mm(const Ctx& c, GemmMode mode, const float* A, int lda, const float* B, int ldb, float* C, int ldc, int M, int N, int K,
         const float* bias = nullptr, const float* R = nullptr, int ldr = 0, int beta = 0) {
@@ -1585,7 +1596,7 @@ void colsum(const Ctx& c, const float* a, float* out, size_t rows, int N) {
 void mlp_fwd(const Ctx& c, const float* x1, float* y, size_t rows, const float* g2, const float* Wg, const float* Wu,
              const float* Wd) {
   if (fused_mlp(c.D, c.bf16)) {   // nothing to leave behind
-    if (y) train_mlp::forward(x1, g2, c.mlp_image, y, rows, c.b.status, c.st);
+    if (y) c.note(train_mlp::forward(x1, g2, c.mlp_image, y, rows, c.b.status, c.st));
     return;
   }
   const int D = c.D, F = 4 * c.D, M = (int)rows;
@@ -1612,7 +1623,7 @@ void mlp_fwd(const Ctx& c, const float* x1, float* y, size_t rows, const float* 
 void mlp_bwd(const Ctx& c, const float* x1, const float* dy, float* dx1, size_t rows, const float* g2, const float* Wg,
              const float* Wu, const float* Wd, float* dg2, float* dWg, float* dWu, float* dWd) {
   if (fused_mlp(c.D, c.bf16)) {
-    train_mlp::backward(x1, g2, c.mlp_image, dy, dx1, dg2, dWg, dWu, dWd, c.b.n_image, c.b.dy_image, rows, c.b.status, c.st);
+    c.note(train_mlp::backward(x1, g2, c.mlp_image, dy, dx1, dg2, dWg, dWu, dWd, c.b.n_image, c.b.dy_image, rows, c.b.status, c.st));
     return;
   }
   const int D = c.D, F = 4 * c.D, M = (int)rows;
@@ -1657,7 +1668,7 @@ void attn_fwd(const Ctx& c, const float* qkv, const uint8_t* alive, float* o, in
   if (train_attn::supported(c.D, c.H, NM, nb)) {
     train_attn::Call a{};
     a.qkv = qkv; a.alive = alive; a.kvb = kvb; a.bactive = bactive; a.G = G; a.n = NM; a.nb = nb; a.o = o;
-    train_attn::forward(a, c.st);
+    c.note(train_attn::forward(a, c.st));
     return;
   }
   if (c.D / c.H == 32 && NM <= 32 && !kvb) {
@@ -1707,7 +1718,7 @@ void norm_linear(const Ctx& c, const float* x, const float* gain, float* n, floa
   f.x = x; f.gain = gain; f.n_out = n; f.inv = inv; f.image = block_image(c, first); f.ld_out = ld; f.rows = rows;
   f.blocks = (int)out.size();
   std::copy(out.begin(), out.end(), f.out);
-  train_linear::forward(f, c.b.status, c.st);
+  c.note(train_linear::forward(f, c.b.status, c.st));
 }
 // y = x W^T (+ bias) (+ residual) for a square W.
 void linear(const Ctx& c, const float* x, int first, const float* W, float* y, size_t rows, const float* bias = nullptr,
@@ -1718,7 +1729,7 @@ void linear(const Ctx& c, const float* x, int first, const float* W, float* y, s
   }
   train_linear::Forward f;
   f.x = x; f.image = block_image(c, first); f.out[0] = y; f.bias[0] = bias; f.residual = residual; f.rows = rows;
-  train_linear::forward(f, c.b.status, c.st);
+  c.note(train_linear::forward(f, c.b.status, c.st));
 }
 // Its gradients: d W += dy^T x, dx = dy W.
 void linear_bwd(const Ctx& c, const float* dy, const float* x, int first, const float* W, float* dW, float* dx, size_t rows) {
@@ -1730,7 +1741,7 @@ void linear_bwd(const Ctx& c, const float* dy, const float* x, int first, const 
   }
   train_linear::Backward b;
   b.dy[0] = dy; b.n = x; b.image = block_image(c, first); b.d_weight[0] = dW; b.dx = dx; b.rows = rows;
-  train_linear::backward(b, c.b.status, c.st);
+  c.note(train_linear::backward(b, c.b.status, c.st));
 }
 // The gradients behind norm_linear: weights, the norm's gain, and dx = dres + what comes through the norm.
 void norm_linear_bwd(const Ctx& c, std::initializer_list<const float*> dy, int ld, const float* n, int first, std::initializer_list<float*> dW,
@@ -1740,13 +1751,13 @@ void norm_linear_bwd(const Ctx& c, std::initializer_list<const float*> dy, int l
   std::copy(dy.begin(), dy.end(), b.dy);
   std::copy(dW.begin(), dW.end(), b.d_weight);
   b.x = x; b.gain = gain; b.inv = inv; b.dres = dres; b.dx = dx; b.d_gain = d_gain; b.rows = rows;
-  train_linear::backward(b, c.b.status, c.st);
+  c.note(train_linear::backward(b, c.b.status, c.st));
 }
 
 // Spatial sublayer, forward part.  Leaves n1 in d[0] (roots in inv[0]), q|k|v in w3[0], the attention
 // output in d[1], x1 in d[2], the bullet norm / keys and values in bul_n / bul_inv / kvb, and what
 // mlp_fwd leaves; writes y when y is given.
-void spatial_fwd(const Ctx& c, const BnbSpatialWeights& w, const float* x, const uint8_t* alive, const BnbBullets* bul,
+int spatial_fwd(const Ctx& c, const BnbSpatialWeights& w, const float* x, const uint8_t* alive, const BnbBullets* bul,
                  float* y, int G, int NM) {
   const int D = c.D;
   const size_t R = (size_t)G * NM;
@@ -1770,6 +1781,7 @@ void spatial_fwd(const Ctx& c, const BnbSpatialWeights& w, const float* x, const
   attn_fwd(c, qkv, alive, o, G, NM, reads ? b.kvb : nullptr, reads ? bul->active : nullptr, nb);
   linear(c, o, L_OUT, w.out_w, x1, R, nullptr, x);            // x1 = x + o Wout^T
   mlp_fwd(c, x1, y, R, w.norm2_w, w.gate_w, w.up_w, w.down_w);
+  return status_of(c);
 }
 
 int spatial_bwd(const Ctx& c, const BnbSpatialWeights& w, const BnbSpatialGrads& dw, const float* x, const uint8_t* alive,
@@ -1785,7 +1797,10 @@ int spatial_bwd(const Ctx& c, const BnbSpatialWeights& w, const BnbSpatialGrads&
   const size_t RB = (size_t)G * nb;
   if (reads && (!dw.kv_bullet_w || !dw.norm_bullet_w)) return BNB_ERR_NULL_POINTER;
 
-  if (!have_fwd) spatial_fwd(c, w, x, alive, bul, nullptr, G, NM);
+  if (!have_fwd) {
+    const int st = spatial_fwd(c, w, x, alive, bul, nullptr, G, NM);
+    if (st) return st;
+  }
   mlp_bwd(c, x1, dy, dx1, R, w.norm2_w, w.gate_w, w.up_w, w.down_w, dw.norm2_w, dw.gate_w, dw.up_w, dw.down_w);
 
   linear_bwd(c, dx1, o, L_OUT, w.out_w, dw.out_w, d_o, R);
@@ -1814,7 +1829,7 @@ int spatial_bwd(const Ctx& c, const BnbSpatialWeights& w, const BnbSpatialGrads&
                       b.bul_inv, d_bullets, d_bullets ? d_bullets : b.bul_dn, dw.norm_bullet_w, RB);
     norm_linear_bwd(c, {dqkv, dqkv + D, dqkv + 2 * D}, 3 * D, n1, L_QKV, {dw.qkv_w, dw.qkv_w + square, dw.qkv_w + 2 * square}, x, w.norm1_w,
                     b.inv[0], dx1, dx, dw.norm1_w, R);
-    return BNB_OK;
+    return status_of(c);
   }
   if (reads) {
     mmh(c, TN, H_B, b.dkvb, 2 * D, b.bul_n, D, dw.kv_bullet_w, D, 2 * D, D, (int)RB);
@@ -1826,7 +1841,7 @@ int spatial_bwd(const Ctx& c, const BnbSpatialWeights& w, const BnbSpatialGrads&
   mmh(c, TN, H_B, dqkv, 3 * D, n1, D, dw.qkv_w, D, 3 * D, D, M);
   mm(c, NN, dqkv, 3 * D, w.qkv_w, D, dn1, D, M, D, 3 * D);
   rmsnorm_bwd(c, x, w.norm1_w, b.inv[0], dn1, dx1, dx, dw.norm1_w, R);
-  return BNB_OK;
+  return status_of(c);
 }
 
 void gather(const Ctx& c, const float* full, float* compact, size_t rows, int per_grp, int NM, int n0) {
@@ -1878,7 +1893,7 @@ void ships_fwd(const Ctx& c, const BnbTemporalWeights& w, const float* x, const 
     train_linear::Forward f;
     f.x = u; f.image = block_image(c, L_GATES); f.blocks = 2; f.rows = Rs;
     f.out[0] = za; f.out[1] = zx; f.bias[0] = w.a_b; f.bias[1] = w.x_b;
-    train_linear::forward(f, c.b.status, c.st);
+    c.note(train_linear::forward(f, c.b.status, c.st));
   } else {
     mm(c, NT, u, D, w.a_w, D, za, D, M, D, D, w.a_b);
     mm(c, NT, u, D, w.x_w, D, zx, D, M, D, D, w.x_b);
@@ -1924,7 +1939,7 @@ int temporal_fwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
     if (!w.field_sub_w) return BNB_ERR_NULL_POINTER;
     fields_fwd(cf, w, x, y, tg);
   }
-  return BNB_OK;
+  return status_of(cs);
 }
 
 // One temporal sublayer: the recurrent path over the ship rows, the non-recurrent one over the
@@ -1958,7 +1973,7 @@ int temporal_bwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
       g.dy[0] = za; g.dy[1] = zx; g.n = u; g.image = block_image(c, L_GATES); g.blocks = 2; g.rows = Rs;
       g.d_weight[0] = dw.a_w; g.d_weight[1] = dw.x_w; g.d_bias[0] = dw.a_b; g.d_bias[1] = dw.x_b;
       g.dx = dm; g.accumulate = true;
-      train_linear::backward(g, c.b.status, c.st);
+      c.note(train_linear::backward(g, c.b.status, c.st));
     } else {
       mm(c, TN, za, D, u, D, dw.a_w, D, D, D, M);
       mm(c, TN, zx, D, u, D, dw.x_w, D, D, D, M);
@@ -2006,7 +2021,7 @@ int temporal_bwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
     }
     scatter(c, dxf, dx, Rf, nf, tg.NM, tg.n_rec);
   }
-  return BNB_OK;
+  return status_of(cs);
 }
 
 bool dims_ok(int D, int H) {
@@ -2155,25 +2170,21 @@ void use_images(Ctx& c, int s) {
   c.linears = fused ? c.b.linears + (size_t)s * MAX_LINEARS * train_linear::BLOCK_IMAGE : nullptr;
 }
 
-}  // namespace
-
-// The forward of a call that will be differentiated: the same sublayer forward parts the backward
-// recomputes from, run once with every path's intermediates written to `kept`, plus the trunk's
-// output and final state.
-int trunk_sequence_fwd_train(const TrunkFwdTrainArgs& a) {
+int run_fwd_train(const TrunkFwdTrainArgs& a) {
   Walk wk;
   int rc = make_walk(wk, a.n_blocks, a.n_spatial, a.n_temporal, a.D, a.H, *a.batch, a.T, a.bullets);
   if (rc) return rc;
   if (wk.R == 0) return BNB_OK;
   const int D = wk.D;
+  int failed = BNB_OK;
   Ctx c{};
-  c.D = D; c.H = a.H; c.bf16 = a.bf16_products; c.st = a.stream;
+  c.D = D; c.H = a.H; c.bf16 = a.bf16_products; c.st = a.stream; c.failed = &failed;
   static thread_local Kept kept;
   if ((rc = open_buffers(c, &kept, wk, a.n_blocks, a.n_spatial, a.n_temporal, a.scratch, a.scratch_bytes, a.kept, a.kept_bytes)))
     return rc;
   if (wk.S == 0) {
     cudaMemcpyAsync(a.y, a.x, wk.R * D * sizeof(float), cudaMemcpyDeviceToDevice, a.stream);
-    return BNB_OK;
+    return status_of(c);
   }
   if ((rc = prepare_mlps(c, wk, a.spatial, a.temporal, a.n_blocks, a.n_spatial, a.n_temporal))) return rc;
   const float* cur = a.x;
@@ -2184,7 +2195,7 @@ int trunk_sequence_fwd_train(const TrunkFwdTrainArgs& a) {
       float* out = s + 1 == wk.S ? a.y : kept.bound + (size_t)s * wk.R * D;
       Ctx cs = c;
       cs.b = kept.first[s];
-      spatial_fwd(cs, a.spatial[blk * a.n_spatial + j], cur, a.alive, a.bullets, out, wk.G, wk.NM);
+      if ((rc = spatial_fwd(cs, a.spatial[blk * a.n_spatial + j], cur, a.alive, a.bullets, out, wk.G, wk.NM))) return rc;
       cur = out;
     }
     for (int j = 0; j < a.n_temporal; ++j, ++s) {
@@ -2201,10 +2212,10 @@ int trunk_sequence_fwd_train(const TrunkFwdTrainArgs& a) {
       cur = out;
     }
   }
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+  return status_of(c);
 }
 
-int trunk_sequence_bwd(const TrunkBwdArgs& a) {
+int run_bwd(const TrunkBwdArgs& a) {
   Walk wk;
   int rc = make_walk(wk, a.n_blocks, a.n_spatial, a.n_temporal, a.D, a.H, *a.batch, a.T, a.bullets);
   if (rc) return rc;
@@ -2212,8 +2223,9 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
   const int D = wk.D, S = wk.S, G = wk.G, NM = wk.NM;
   const size_t R = wk.R, Rr = wk.Rr;
   cudaStream_t st = a.stream;
+  int failed = BNB_OK;
   Ctx c{};
-  c.D = D; c.H = a.H; c.bf16 = a.bf16_products; c.st = st;
+  c.D = D; c.H = a.H; c.bf16 = a.bf16_products; c.st = st; c.failed = &failed;
   static thread_local Kept kept;
   const bool have_fwd = a.kept != nullptr;
   if ((rc = open_buffers(c, &kept, wk, a.n_blocks, a.n_spatial, a.n_temporal, a.scratch, a.scratch_bytes, a.kept, a.kept_bytes)))
@@ -2221,7 +2233,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
 
   if (S == 0) {
     cudaMemcpyAsync(a.dx, a.dy, R * D * sizeof(float), cudaMemcpyDeviceToDevice, st);
-    return BNB_OK;
+    return status_of(c);
   }
 
   if ((rc = prepare_mlps(c, wk, a.spatial, a.temporal, a.n_blocks, a.n_spatial, a.n_temporal))) return rc;
@@ -2238,7 +2250,7 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
         if (s + 1 == S) break;
         use_images(c, s);
         float* out = c.b.bound + (size_t)s * R * D;
-        spatial_fwd(c, a.spatial[blk * a.n_spatial + j], cur, a.alive, a.bullets, out, G, NM);
+        if ((rc = spatial_fwd(c, a.spatial[blk * a.n_spatial + j], cur, a.alive, a.bullets, out, G, NM))) return rc;
         cur = out;
       }
       for (int j = 0; j < a.n_temporal; ++j, ++s) {
@@ -2289,8 +2301,22 @@ int trunk_sequence_bwd(const TrunkBwdArgs& a) {
       dcur = dout;
     }
   }
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+  return status_of(c);
 }
+
+// A call that gave up takes its error with it: the next one starts clean.
+int settle(int rc) {
+  if (rc) (void)cudaGetLastError();
+  return rc;
+}
+
+}  // namespace
+
+// The forward of a call that will be differentiated: the same sublayer forward parts the backward
+// recomputes from, run once with every path's intermediates written to `kept`, plus the trunk's
+// output and final state.
+int trunk_sequence_fwd_train(const TrunkFwdTrainArgs& a) { return settle(run_fwd_train(a)); }
+int trunk_sequence_bwd(const TrunkBwdArgs& a) { return settle(run_bwd(a)); }
 
 }  // namespace grad
 

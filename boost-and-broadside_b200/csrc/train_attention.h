@@ -22,8 +22,8 @@ struct Call {
 
 // d_model 128, 4 heads, up to 32 tokens per environment.
 bool supported(int d_model, int n_heads, int n, int nb);
-int forward(const Call& c, cudaStream_t st);
-int backward(const Call& c, cudaStream_t st);
+[[nodiscard]] int forward(const Call& c, cudaStream_t st);
+[[nodiscard]] int backward(const Call& c, cudaStream_t st);
 
 }  // namespace train_attn
 }  // namespace bnb

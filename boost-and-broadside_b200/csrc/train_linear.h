@@ -12,7 +12,7 @@ constexpr int MAX_BLOCKS = 3;             // 128-row blocks of weights in one ca
 constexpr size_t BLOCK_IMAGE = 32768;     // bfloat16 image of one block
 
 // Images of n (128, 128) weight blocks (row-major, 512 bytes a row), one after the other at `image`.
-int pack(const float* const* blocks, int n, uint8_t* image, cudaStream_t st);
+[[nodiscard]] int pack(const float* const* blocks, int n, uint8_t* image, cudaStream_t st);
 
 // out[b] = n W_b^T (+ bias[b]) (+ residual, one block only) for the blocks at `image`.  With a gain, n = bf16 of
 // x's RMSNorm, written to n_out, the reciprocal roots to inv; without, n = bf16(x).
@@ -29,7 +29,7 @@ struct Forward {
   const float* residual = nullptr;
   size_t rows = 0;
 };
-int forward(const Forward& f, int* status, cudaStream_t st);
+[[nodiscard]] int forward(const Forward& f, int* status, cudaStream_t st);
 
 // Given dy[b]: dn = sum_b dy_b W_b; d_weight[b] (128, 128) += dy_b^T n; without a gain d_bias[b] += column sums of dy_b.
 // Without a gain (one or two blocks, n float32): dx = dn (+ dx before, if accumulate).
@@ -52,7 +52,7 @@ struct Backward {
   float* d_gain = nullptr;
   size_t rows = 0;
 };
-int backward(const Backward& b, int* status, cudaStream_t st);
+[[nodiscard]] int backward(const Backward& b, int* status, cudaStream_t st);
 
 }  // namespace train_linear
 }  // namespace bnb
