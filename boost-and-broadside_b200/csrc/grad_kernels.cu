@@ -492,9 +492,13 @@ inline bool gemm_is_full(const GemmArgs& g) {
 // TN: C (M, N) += A (K, M)^T . B (K, N)      dW += dy^T x   (split over K, atomics)
 template <bool A_KC, bool B_KC, bool BF16>
 void launch_gemm_t(const GemmArgs& g, dim3 grid, cudaStream_t st) {
-  static const bool opted =
-      cudaFuncSetAttribute(k_gemm<A_KC, B_KC, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM) == cudaSuccess;
-  (void)opted;
+  // an opt-in holds for one device; where it fails, so does the launch
+  static bool opted[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !opted[dev]) {
+    const bool ok = cudaFuncSetAttribute(k_gemm<A_KC, B_KC, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM) == cudaSuccess;
+    if (dev >= 0 && dev < 64) opted[dev] = ok;
+  }
   k_gemm<A_KC, B_KC, BF16><<<grid, GT, GEMM_SMEM, st>>>(g);
 }
 
