@@ -404,6 +404,13 @@ BackwardResult run_backward(const Tensor& dy, const OptTensor& dhidden, const Op
   const int D = (int)x.size(-1), T = g.timesteps > 1 ? g.timesteps : 1;
   const BnbBatch batch = g.batch({});
   const Tensor xin = f32c(x), hin = f32c(hidden), dyin = f32c(dy);
+  OptTensor arena;   // may have been somewhere else since the forward wrote it
+  if (kept.has_value()) {
+    if (kept->device() != dev || kept->scalar_type() != at::kByte || kept->dim() != 1)
+      throw std::runtime_error("the kept activations came back as another tensor: saved-tensor hooks have to return device, type and shape as they were");
+    arena = contiguous(*kept);
+    if (reinterpret_cast<uintptr_t>(arena->data_ptr()) % 256) arena = arena->clone();   // its layout counts from a 256-byte boundary
+  }
   OptTensor dho;
   if (dhidden.has_value() && dhidden->defined()) dho = f32c(*dhidden);
   const OptTensor alive_u8 = bytes_of(alive), done_u8 = bytes_of(done);
@@ -441,7 +448,7 @@ BackwardResult run_backward(const Tensor& dy, const OptTensor& dhidden, const Op
                                static_cast<const float*>(hin.data_ptr()), static_cast<const uint8_t*>(ptr(done_u8)), &batch, T, grad_precision(g),
                                static_cast<const float*>(dyin.data_ptr()), static_cast<const float*>(ptr(dho)), static_cast<float*>(r.dx.data_ptr()),
                                static_cast<float*>(r.dh.data_ptr()), b.present ? static_cast<float*>(r.dbul.data_ptr()) : nullptr,
-                               kept.has_value() ? kept->data_ptr() : nullptr, kept.has_value() ? (size_t)kept->numel() : 0, scratch.data_ptr(),
+                               arena.has_value() ? arena->data_ptr() : nullptr, arena.has_value() ? (size_t)arena->numel() : 0, scratch.data_ptr(),
                                (size_t)scratch.numel(), at::cuda::getCurrentCUDAStream(dev.index()).stream()));
   return r;
 }
@@ -484,9 +491,10 @@ std::tuple<Tensor, Tensor, Tensor> trunk_forward_train(const Tensor& x, const Op
 // The autograd node of an eager differentiated call: what the operators' formulas do, without Python in
 // the backward pass.
 struct TrunkNode : public torch::autograd::Node {
-  torch::autograd::SavedVariable x, alive, hidden, done, bullets, mask;
+  // saved as autograd saves them, the kept activations among them: saved-tensor hooks (torch.utils.checkpoint,
+  // save_on_cpu) move or recompute what they are given, and nothing else here holds on to it
+  torch::autograd::SavedVariable x, alive, hidden, done, bullets, mask, kept;
   std::vector<torch::autograd::SavedVariable> weights;
-  Tensor kept;
   std::vector<int64_t> geom;
   bool consumed = false;
 
@@ -498,13 +506,14 @@ struct TrunkNode : public torch::autograd::Node {
                                "through the same graph set BNB_GRAD_MODE=recompute");
     consumed = true;
     const at::NoGradGuard no_grad;
-    const Tensor xv = x.unpack(), hv = hidden.unpack(), bv = bullets.unpack();
+    const Tensor xv = x.unpack(), av = alive.unpack(), hv = hidden.unpack(), ov = done.unpack(), bv = bullets.unpack(), mv = mask.unpack();
+    const Tensor kv = kept.unpack();
+    kept.reset_data();
     std::vector<Tensor> ws;
     ws.reserve(weights.size());
     for (auto& w : weights) ws.push_back(w.unpack());
     const Tensor dy = grads[0].defined() ? grads[0] : at::zeros_like(xv, xv.options().dtype(at::kFloat));
-    const BackwardResult r = run_backward(dy, opt(grads[1]), kept, xv, opt(alive.unpack()), hv, opt(done.unpack()), opt(bv), opt(mask.unpack()), ws, geom);
-    kept.reset();
+    const BackwardResult r = run_backward(dy, opt(grads[1]), kv, xv, opt(av), hv, opt(ov), opt(bv), opt(mv), ws, geom);
     torch::autograd::variable_list out;
     out.reserve(3 + ws.size());
     out.push_back(task_should_compute_output(0) ? r.dx.reshape(xv.sizes()).to(xv.scalar_type()) : Tensor());
@@ -519,9 +528,8 @@ struct TrunkNode : public torch::autograd::Node {
     return out;
   }
   void release_variables() override {
-    for (auto* v : {&x, &alive, &hidden, &done, &bullets, &mask}) v->reset_data();
+    for (auto* v : {&x, &alive, &hidden, &done, &bullets, &mask, &kept}) v->reset_data();
     weights.clear();
-    kept.reset();
   }
 };
 
@@ -533,19 +541,20 @@ std::tuple<Tensor, Tensor> trunk_train(const Tensor& x, const OptTensor& alive, 
   torch::autograd::variable_list inputs{x, hidden, bullets.has_value() ? *bullets : Tensor()};
   inputs.insert(inputs.end(), weights.begin(), weights.end());
   node->set_next_edges(torch::autograd::collect_next_edges(inputs));
-  Tensor y, hout;
+  Tensor y, hout, kept;
   {
     const at::NoGradGuard no_grad;
-    std::tie(y, hout, node->kept) = trunk_forward_train(x, alive, hidden, done, bullets, mask, weights, geom);
+    std::tie(y, hout, kept) = trunk_forward_train(x, alive, hidden, done, bullets, mask, weights, geom);
   }
   using torch::autograd::SavedVariable;
   auto save = [](const OptTensor& t) { return SavedVariable(t.has_value() ? *t : Tensor(), false); };
   node->x = SavedVariable(x, false);
-  node->hidden = SavedVariable(hidden, false);
   node->alive = save(alive);
+  node->hidden = SavedVariable(hidden, false);
   node->done = save(done);
   node->bullets = save(bullets);
   node->mask = save(mask);
+  node->kept = SavedVariable(kept, false);
   node->weights.reserve(weights.size());
   for (const Tensor& w : weights) node->weights.emplace_back(w, false);
   node->geom = geom;
@@ -757,7 +766,7 @@ PYBIND11_MODULE(_host_path, m) {
   });
   m.def("trunk_backward", &trunk_backward);
   m.def("trunk_forward_train", &trunk_forward_train);
-  m.def("trunk_train", &trunk_train);
+  m.def("trunk_train", torch::wrap_pybind_function(trunk_train));   // saved-tensor hooks may raise
   m.def("ragged_build", &ragged_build);
   m.def("mlp_chain", &mlp_chain);
   m.def("policy_tail", &policy_tail);
