@@ -488,6 +488,14 @@ std::tuple<Tensor, Tensor, Tensor> trunk_forward_train(const Tensor& x, const Op
   return {y, hout, kept};
 }
 
+// Behind the gradients of a backward pass that is itself recorded (create_graph=True): the trunk has no second-order
+// gradient, and whoever asks for one is told so, as by an operator without an autograd formula.
+struct NoSecondOrder : public torch::autograd::Node {
+  torch::autograd::variable_list apply(torch::autograd::variable_list&&) override {
+    throw std::runtime_error("the gradients of the CUDA trunk cannot be differentiated again (a second-order gradient through it was asked for)");
+  }
+};
+
 // The autograd node of an eager differentiated call: what the operators' formulas do, without Python in
 // the backward pass.
 struct TrunkNode : public torch::autograd::Node {
@@ -505,6 +513,7 @@ struct TrunkNode : public torch::autograd::Node {
       throw std::runtime_error("the kept activations of this trunk call were consumed by an earlier backward; for a second backward "
                                "through the same graph set BNB_GRAD_MODE=recompute");
     consumed = true;
+    const bool recorded = at::GradMode::is_enabled();
     const at::NoGradGuard no_grad;
     const Tensor xv = x.unpack(), av = alive.unpack(), hv = hidden.unpack(), ov = done.unpack(), bv = bullets.unpack(), mv = mask.unpack();
     const Tensor kv = kept.unpack();
@@ -524,6 +533,17 @@ struct TrunkNode : public torch::autograd::Node {
       const int64_t n = ws[i].numel();
       out.push_back(task_should_compute_output(3 + i) ? r.flat.narrow(0, off, n).view(ws[i].sizes()) : Tensor());
       off += (n + 3) / 4 * 4;
+    }
+    if (recorded) {
+      torch::autograd::variable_list from{xv, hv, bv, grads[0], grads[1]};
+      from.insert(from.end(), ws.begin(), ws.end());
+      auto again = std::make_shared<NoSecondOrder>();
+      again->set_next_edges(torch::autograd::collect_next_edges(from));
+      for (Tensor& t : out)
+        if (t.defined()) {
+          t = t.detach();   // a tensor of its own, not a view of the flat buffer
+          torch::autograd::create_gradient_edge(t, again);
+        }
     }
     return out;
   }
