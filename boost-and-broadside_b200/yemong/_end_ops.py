@@ -48,11 +48,6 @@ def _(x, w1, b1, g1, w2, b2, g2, precision, active=None):
     return x.new_empty((x.shape[0], w2.shape[0]), dtype=_out_dtype(precision))
 
 
-def direct(t: Tensor) -> bool:
-    """Whether an operator's body may be called as it is: an ordinary eager tensor, no tracer."""
-    return type(t) is Tensor and not torch.compiler.is_compiling()
-
-
 @torch.library.custom_op("bnb_b200::policy_tail", mutates_args=(), device_types="cuda")
 def policy_tail(x: Tensor, alive: Tensor, team_id: Tensor, uniforms: Tensor, heads: List[Tensor], pma: List[Tensor],
                 win_cols: List[int], n_ships: int) -> Tuple[Tensor, Tensor, Tensor, Tensor]:

@@ -19,10 +19,11 @@ from __future__ import annotations
 
 from typing import List, Optional, Tuple
 
+import os
+
 import torch
 from torch import Tensor
-
-import os
+from torch.autograd import forward_ad
 
 from .. import _capi
 from ._weights import N_SPATIAL, packed_image, spatial_struct_from
@@ -52,6 +53,18 @@ def _raise_pending_status(dev: torch.device) -> None:
             raise RuntimeError(
                 f"an earlier tensor-core call on {dev} gave up a bounded wait: {_capi.lib.bnb_status_string(st).decode()} "
                 f"(status {st}); its outputs, and any state carried from them, are invalid")
+
+
+_dispatch_modes, _function_transform, _jit_trace = (torch._C._len_torch_dispatch_stack, torch._C._functorch.peek_interpreter_stack,
+                                                    torch._C._get_tracing_state)
+
+
+def direct(t: Tensor) -> bool:
+    """Whether an operator's body may be called as it is: an ordinary eager tensor, and nobody at work who has
+    to see the operator: a compiler, TorchScript's tracer, a dispatch mode (make_fx, flop counting), a
+    function transform (vmap) or forward-mode differentiation, whose tangents the body would drop."""
+    return (not torch.compiler.is_compiling() and type(t) is Tensor and not _dispatch_modes() and _function_transform() is None
+            and _jit_trace() is None and forward_ad._current_level < 0)
 
 
 def uniform_geom(n_envs: int, tokens: int, ships: int) -> List[int]:

@@ -17,7 +17,7 @@ import torch
 import torch.nn as nn
 
 from .. import _capi
-from . import _end_ops
+from . import _end_ops, _ops
 
 
 def _encoder_chain(raw: torch.Tensor, lin1: nn.Linear, norm1: nn.RMSNorm, lin2: nn.Linear, norm2: nn.RMSNorm,
@@ -29,7 +29,7 @@ def _encoder_chain(raw: torch.Tensor, lin1: nn.Linear, norm1: nn.RMSNorm, lin2: 
     if raw.shape[-1] != in_dim:
         raise RuntimeError(f"expected raw features of width {in_dim}, got {tuple(raw.shape)}")
     precision = _capi.current_precision(raw.device)
-    run = _end_ops.mlp_call if _end_ops.direct(raw) else _end_ops.mlp_chain
+    run = _end_ops.mlp_call if _ops.direct(raw) else _end_ops.mlp_chain
     y = run(raw.reshape(-1, in_dim), lin1.weight, lin1.bias, norm1.weight, lin2.weight, lin2.bias, norm2.weight, precision,
             None if active is None else active.reshape(-1))
     return y.reshape(*raw.shape[:-1], out_dim)

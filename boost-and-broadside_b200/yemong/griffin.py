@@ -213,8 +213,8 @@ def run_trunk(
     n_temporal = len(blocks[0].temporal) if n_blocks else 0
     n_cross = sum(1 for sp in blocks[0].spatial if sp.reads_bullets) if n_blocks else 0
     has_fields = batch_geom[4] > batch_geom[5]          # total_tokens > total_ships
-    tracing = torch.compiler.is_compiling() or type(x) is not torch.Tensor
-    weights = None if tracing else _capi.host.trunk_params(blocks, has_fields)
+    direct = _ops.direct(x)
+    weights = _capi.host.trunk_params(blocks, has_fields) if direct else None
     if weights is None:
         weights = []
         for blk in blocks:
@@ -229,11 +229,11 @@ def run_trunk(
     bullets, bullet_mask = (bullets, bullet_mask) if n_cross else (None, None)
     if grad and not offsets and reset_env is None and _keep(x, geom, 0 if bullets is None else bullets.shape[1]):
         # a call that will be differentiated: the forward that keeps its activations for the backward
-        if not tracing:
+        if direct:
             return _capi.host.trunk_train(x, alive, hidden, done, bullets, bullet_mask, weights, geom)
         y, nh, _ = _ops.trunk_forward_train(x, alive, hidden, done, bullets, bullet_mask, weights, geom)
         return y, nh
-    run = _ops.trunk_forward if grad or tracing else _ops.trunk_call
+    run = _ops.trunk_call if direct and not grad else _ops.trunk_forward
     return run(x, alive, hidden, done, reset_env, bullets, bullet_mask, weights, offsets or [], geom)
 
 

@@ -16,7 +16,7 @@ import torch
 import torch.nn as nn
 
 from .. import _capi
-from . import _end_ops
+from . import _end_ops, _ops
 
 
 class HeadMLP(nn.Sequential):
@@ -44,7 +44,7 @@ class HeadMLP(nn.Sequential):
         in_dim, out_dim = lin1.in_features, lin2.out_features
         if x.shape[-1] != in_dim:
             raise RuntimeError(f"expected tokens of width {in_dim}, got {tuple(x.shape)}")
-        run = _end_ops.mlp_call if _end_ops.direct(x) else _end_ops.mlp_chain
+        run = _end_ops.mlp_call if _ops.direct(x) else _end_ops.mlp_chain
         y = run(x.reshape(-1, in_dim), lin1.weight, lin1.bias, norm.weight, lin2.weight, lin2.bias, None,
                 _capi.current_precision(x.device))
         return y.reshape(*x.shape[:-1], out_dim)

@@ -20,7 +20,7 @@ import torch
 import torch.nn as nn
 
 from .. import _capi
-from . import _end_ops
+from . import _end_ops, _ops
 from .encoder import BulletEncoder, ShipEncoder
 from .griffin import YemongBlock
 from .heads import HeadMLP, NextStateHead, TeamPMA, evaluate_action, sample_action
@@ -106,7 +106,7 @@ class YemongPolicy(YemongTrunk):
         lists = self._tail_lists() if x.dtype == torch.bfloat16 else None
         if lists is not None:
             uniforms = torch.rand(x.shape[0] * N, 3, device=x.device, generator=generator)
-            run = _capi.host.policy_tail if _end_ops.direct(x) else _end_ops.policy_tail
+            run = _capi.host.policy_tail if _ops.direct(x) else _end_ops.policy_tail
             action, logprob, value, pred_next = run(x, alive, obs["team_id"], uniforms, *lists, list(self._team_pma_k), N)
             return action, logprob, value, pred_next, new_hidden
         x_ships = x[:, :N, :].contiguous()
