@@ -709,6 +709,21 @@ bool bullets_compacted(int64_t d_model, int64_t n_heads, int64_t tokens, int64_t
   return slots > 0 && bnb::tensor::supported_batch((int)d_model, (int)n_heads, b) && bnb::tensor::supported_bullets(b, (int)slots);
 }
 
+// The value columns that the win head's outputs go to, as indexing a tensor takes them: from the end when negative,
+// refused outside, and each an output that the win head has.
+std::vector<uint8_t> value_columns(const std::vector<int64_t>& win_cols, int64_t value_width, int64_t win_width) {
+  auto refuse = [](int64_t i, int64_t size) {
+    throw py::index_error("index " + std::to_string(i) + " is out of bounds for a last dimension of size " + std::to_string(size));
+  };
+  std::vector<uint8_t> cols;
+  for (int64_t k : win_cols) {
+    if (k < -value_width || k >= value_width) refuse(k, value_width);
+    if ((int64_t)cols.size() >= win_width) refuse((int64_t)cols.size(), win_width);
+    cols.push_back((uint8_t)(k < 0 ? k + value_width : k));
+  }
+  return cols;
+}
+
 // bnb_b200::policy_tail (yemong/_end_ops.py): everything of the rollout step behind the trunk.  x
 // (B, N+M, 128) bfloat16, heads = five parameters each of the action, next-state and value head [and the
 // win head], pma = seeds, in_proj, out_proj, norm (empty: no team value), win_cols the value columns the
@@ -716,6 +731,8 @@ bool bullets_compacted(int64_t d_model, int64_t n_heads, int64_t tokens, int64_t
 std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const Tensor& alive_in, const Tensor& team_in,
                                                        const Tensor& uniforms, const std::vector<Tensor>& heads,
                                                        const std::vector<Tensor>& pma, const std::vector<int64_t>& win_cols, int64_t N) {
+  const int64_t K = heads.at(13).size(0), P = heads[8].size(0), W = pma.empty() ? 0 : (int64_t)win_cols.size();
+  const std::vector<uint8_t> cols = W > 0 ? value_columns(win_cols, K, heads.at(18).size(0)) : std::vector<uint8_t>();
   const c10::Device dev = x_in.device();
   const c10::cuda::CUDAGuard guard(dev);
   const auto stream = at::cuda::getCurrentCUDAStream(dev.index()).stream();
@@ -736,7 +753,6 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const
   s.tokens = (int)NM;
 
   const auto bf = x.options();
-  const int64_t K = heads[13].size(0), P = heads[8].size(0), W = pma.empty() ? 0 : (int64_t)win_cols.size();
   Tensor logits = at::empty({B, N, 12}, bf), pred = at::empty({B, N, P}, bf), value = at::empty({B, N, K}, bf);
   Tensor action = at::empty({B, N, 3}, bf.dtype(at::kLong)), logprob = at::empty({B, N}, bf);
 
@@ -754,7 +770,6 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const
   check("bnb_head_mlp_fwd", bnb::mlp::run(call, 3, (int)D, (int)(2 * D), 32, stream));
 
   Tensor win, rows, fold;
-  std::vector<uint8_t> cols(win_cols.begin(), win_cols.end());
   if (W > 0) {
     rows = at::empty({B * 2, D}, bf);
     win = at::empty({B * 2, W}, bf);

@@ -96,3 +96,15 @@ def test_native_tail_under_torch_compile_is_one_graph_and_matches_eager():
             _, _, v, pn, h = compiled(obs, hidden)
             v, pn, h = v.clone(), pn.clone(), h.clone()
     assert torch.equal(v, v0) and torch.equal(pn, p0) and torch.equal(h, h0)
+
+
+def test_value_columns_count_from_the_end_as_indexing_does():
+    p = _policy(4, seed=2, ks=(-1, -11, 3))
+    obs, hidden = _obs(9, 4, 1, 0, seed=8)
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        got = p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
+        ref = _modules_step(p, obs, hidden, torch.Generator(device=DEV).manual_seed(3))
+        assert float((got[2].float() - ref[2].float()).abs().max()) <= 1e-2 * float(ref[2].float().abs().max())
+        p._team_pma_k = (11,)
+        with pytest.raises(IndexError):
+            p.get_action_and_value(obs, hidden)

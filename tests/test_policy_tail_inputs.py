@@ -1,0 +1,41 @@
+"""What the native end of the policy step refuses before anything is launched: on CPU tensors, whose device
+is the last thing it looks at."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+B, N, M, D = 3, 5, 2, 128
+
+
+def _head(out):
+    return [torch.zeros(2 * D, D), torch.zeros(2 * D), torch.ones(2 * D), torch.zeros(out, 2 * D), torch.zeros(out)]
+
+
+def _call(**change):
+    from boost_and_broadside_b200 import _capi
+
+    a = dict(x=torch.zeros(B, N + M, D, dtype=torch.bfloat16), alive=torch.ones(B, N + M, dtype=torch.bool),
+             team_id=torch.zeros(B, N + M, dtype=torch.int64), uniforms=torch.zeros(B * N, 3),
+             heads=[*_head(12), *_head(10), *_head(11), *_head(2)],
+             pma=[torch.zeros(2, D), torch.zeros(3 * D, D), torch.zeros(D, D), torch.ones(D)], win_cols=[0, 1], n_ships=N)
+    a.update(change)
+    return _capi.host.policy_tail(a["x"], a["alive"], a["team_id"], a["uniforms"], a["heads"], a["pma"], a["win_cols"], a["n_ships"])
+
+
+@pytest.mark.parametrize("cols", [[11], [0, 11], [-12], [256], [1 << 40]])
+def test_value_columns_outside_the_value_raise(cols):
+    with pytest.raises(IndexError, match="out of bounds"):
+        _call(win_cols=cols)
+
+
+def test_more_value_columns_than_the_win_head_has_raise():
+    with pytest.raises(IndexError, match="out of bounds"):
+        _call(win_cols=[0, 1, 2])
+
+
+def test_inputs_in_order_reach_the_device_check():
+    for cols in ([0, 1], [-1], [10, -11]):
+        with pytest.raises(RuntimeError, match="(?i)cuda"):
+            _call(win_cols=cols)
