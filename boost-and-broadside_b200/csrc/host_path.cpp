@@ -648,6 +648,8 @@ bnb::mlp::MlpChain chain_of(const std::vector<Tensor>& ps, const c10::Device& de
 // those rows are computed, the others are left unwritten.
 Tensor mlp_chain(const Tensor& x, const std::vector<Tensor>& params, int precision, const OptTensor& active) {
   const c10::Device dev = x.device();
+  if (active.has_value() && (active->numel() != x.size(0) || active->device() != dev))
+    throw std::runtime_error("active must hold one element per row, on the rows' device");
   const c10::cuda::CUDAGuard guard(dev);
   const bool bf16 = precision == BNB_BF16, encoder = params.size() > 5;
   const char* what = encoder ? "encoder" : "head";
@@ -724,30 +726,85 @@ std::vector<uint8_t> value_columns(const std::vector<int64_t>& win_cols, int64_t
   return cols;
 }
 
+void expect_shape(const Tensor& t, c10::IntArrayRef want, const char* what) {
+  if (t.defined() && t.sizes() == want) return;
+  std::ostringstream s;
+  s << what << " must have shape " << want << ", got ";
+  if (t.defined()) s << t.sizes();
+  else s << "nothing";
+  throw std::runtime_error(s.str());
+}
+// What the kernels of policy_tail take on trust: the sizes of everything they read.
+void check_tail(const Tensor& x, const Tensor& alive, const Tensor& team, const Tensor& uniforms, const std::vector<Tensor>& heads,
+                const std::vector<Tensor>& pma, int64_t N) {
+  if (x.dim() != 3 || x.size(2) != 128 || x.scalar_type() != at::kBFloat16) throw std::runtime_error("expected bfloat16 tokens of shape (B, N+M, 128)");
+  const int64_t B = x.size(0), NM = x.size(1), D = x.size(2);
+  if (N < 1 || N > NM || N > bnb::tail::MAX_SHIPS)
+    throw std::runtime_error(std::to_string(N) + " ships of " + std::to_string(NM) + " tokens are not served by the native end of the policy step");
+  expect_shape(uniforms, {B * N, 3}, "uniforms");
+  if (uniforms.scalar_type() != at::kFloat || !uniforms.is_contiguous()) throw std::runtime_error("uniforms must be contiguous float32");
+  if (heads.size() != (pma.empty() ? 15u : 20u) || (!pma.empty() && pma.size() != 4)) throw std::runtime_error("expected five parameters per head and four of TeamPMA");
+  for (size_t h = 0; h < heads.size(); h += 5) {
+    const int64_t out = heads[h + 3].dim() == 2 ? heads[h + 3].size(0) : 0;
+    if (out < 1 || out > 32 || (h == 0 && out != 12)) throw std::runtime_error("a head of this width is not served by the native end of the policy step");
+    expect_shape(heads[h], {2 * D, D}, "a head's first weight");
+    expect_shape(heads[h + 1], {2 * D}, "a head's first bias");
+    expect_shape(heads[h + 2], {2 * D}, "a head's norm");
+    expect_shape(heads[h + 3], {out, 2 * D}, "a head's second weight");
+    expect_shape(heads[h + 4], {out}, "a head's second bias");
+  }
+  if (!pma.empty()) {
+    expect_shape(pma[0], {2, D}, "TeamPMA's seeds");
+    expect_shape(pma[1], {3 * D, D}, "TeamPMA's in_proj");
+    expect_shape(pma[2], {D, D}, "TeamPMA's out_proj");
+    expect_shape(pma[3], {D}, "TeamPMA's norm");
+    expect_shape(alive, {B, NM}, "alive");
+    if (!team.defined() || team.dim() != 2 || team.size(0) != B || team.size(1) < N) {
+      std::ostringstream s;
+      s << "team_id must have shape (" << B << ", " << N << ") or more columns";
+      throw std::runtime_error(s.str());
+    }
+  }
+}
+void check_tail_devices(const Tensor& x, std::initializer_list<const Tensor*> others) {
+  if (!x.is_cuda()) throw std::runtime_error("x is on " + x.device().str() + "; the policy's kernels run on CUDA only (sm_100a)");
+  for (const Tensor* t : others)
+    if (t->defined() && t->device() != x.device())
+      throw std::runtime_error("an input of the policy step is on " + t->device().str() + ", the tokens on " + x.device().str());
+}
+
 // bnb_b200::policy_tail (yemong/_end_ops.py): everything of the rollout step behind the trunk.  x
-// (B, N+M, 128) bfloat16, heads = five parameters each of the action, next-state and value head [and the
+// (B, N+M, 128) bfloat16, alive (B, N+M) and team_id (B, N or more columns) only read with pma, heads = five parameters each of the action, next-state and value head [and the
 // win head], pma = seeds, in_proj, out_proj, norm (empty: no team value), win_cols the value columns the
 // win head fills.
-std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const Tensor& alive_in, const Tensor& team_in,
+std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const OptTensor& alive_in, const OptTensor& team_in,
                                                        const Tensor& uniforms, const std::vector<Tensor>& heads,
                                                        const std::vector<Tensor>& pma, const std::vector<int64_t>& win_cols, int64_t N) {
-  const int64_t K = heads.at(13).size(0), P = heads[8].size(0), W = pma.empty() ? 0 : (int64_t)win_cols.size();
-  const std::vector<uint8_t> cols = W > 0 ? value_columns(win_cols, K, heads.at(18).size(0)) : std::vector<uint8_t>();
+  Tensor team = team_in.has_value() ? *team_in : Tensor();
+  Tensor flags = alive_in.has_value() ? *alive_in : Tensor();
+  check_tail(x_in, flags, team, uniforms, heads, pma, N);
+  const int64_t K = heads[13].size(0), P = heads[8].size(0), W = pma.empty() ? 0 : (int64_t)win_cols.size();
+  const std::vector<uint8_t> cols = W > 0 ? value_columns(win_cols, K, heads[18].size(0)) : std::vector<uint8_t>();
+  if (W == 0) team = flags = Tensor();   // only read with a win head
+  check_tail_devices(x_in, {&uniforms, &flags, &team});
   const c10::Device dev = x_in.device();
   const c10::cuda::CUDAGuard guard(dev);
   const auto stream = at::cuda::getCurrentCUDAStream(dev.index()).stream();
   const Tensor x = contiguous(x_in);
-  const Tensor alive = *bytes_of(alive_in);
-  Tensor team = team_in;
-  if (team.scalar_type() != at::kLong && team.scalar_type() != at::kInt) team = team.to(at::kInt);
-  if (team.size(1) > 0 && team.stride(1) != 1) team = team.contiguous();
+  const OptTensor alive = W > 0 ? bytes_of(flags) : OptTensor();
+  if (team.defined()) {
+    if (team.scalar_type() != at::kLong && team.scalar_type() != at::kInt) team = team.to(at::kInt);
+    if (team.stride(1) != 1 || team.stride(0) > INT32_MAX) team = team.contiguous();
+  }
   const int64_t B = x.size(0), NM = x.size(1), D = x.size(2);
   bnb::tail::Ships s{};
   s.x = static_cast<const __nv_bfloat16*>(x.data_ptr());
-  s.alive = static_cast<const uint8_t*>(alive.data_ptr());
-  s.team_id = team.data_ptr();
-  s.team_is_64 = team.scalar_type() == at::kLong ? 1 : 0;
-  s.team_ld = (int)team.stride(0);
+  s.alive = static_cast<const uint8_t*>(ptr(alive));
+  if (team.defined()) {
+    s.team_id = team.data_ptr();
+    s.team_is_64 = team.scalar_type() == at::kLong ? 1 : 0;
+    s.team_ld = (int)team.stride(0);
+  }
   s.n_envs = (int)B;
   s.ships = (int)N;
   s.tokens = (int)NM;

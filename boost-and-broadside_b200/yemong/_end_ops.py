@@ -49,14 +49,15 @@ def _(x, w1, b1, g1, w2, b2, g2, precision, active=None):
 
 
 @torch.library.custom_op("bnb_b200::policy_tail", mutates_args=(), device_types="cuda")
-def policy_tail(x: Tensor, alive: Tensor, team_id: Tensor, uniforms: Tensor, heads: List[Tensor], pma: List[Tensor],
-                win_cols: List[int], n_ships: int) -> Tuple[Tensor, Tensor, Tensor, Tensor]:
+def policy_tail(x: Tensor, alive: Optional[Tensor], team_id: Optional[Tensor], uniforms: Tensor, heads: List[Tensor],
+                pma: List[Tensor], win_cols: List[int], n_ships: int) -> Tuple[Tensor, Tensor, Tensor, Tensor]:
     """Everything of the rollout step behind the trunk under the bfloat16 contract, in six launches: the
     heads, TeamPMA, the win head on one row per team, the action draw.  x (B, N+M, 128) bfloat16 trunk
-    output, alive and team_id (B, N+M), uniforms (B * N, 3) float32; ``heads`` five parameters each of the
-    action, next-state and value head and, with ``pma`` = [seeds, in_proj, out_proj, norm], the win head,
-    whose outputs go to the columns ``win_cols`` of the value.  Returns (action (B, N, 3) int64, logprob
-    (B, N), value (B, N, K), pred_next (B, N, P)), bfloat16 but for the action."""
+    output, uniforms (B * N, 3) float32; ``heads`` five parameters each of the action, next-state and
+    value head and, with ``pma`` = [seeds, in_proj, out_proj, norm], the win head, whose outputs go to the
+    columns ``win_cols`` of the value; alive (B, N+M) and team_id (B, N or more columns) are only read
+    then.  Returns (action (B, N, 3) int64, logprob (B, N), value (B, N, K), pred_next (B, N, P)),
+    bfloat16 but for the action."""
     return _capi.host.policy_tail(x, alive, team_id, uniforms, heads, pma, win_cols, n_ships)
 
 

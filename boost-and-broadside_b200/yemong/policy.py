@@ -107,7 +107,8 @@ class YemongPolicy(YemongTrunk):
         if lists is not None:
             uniforms = torch.rand(x.shape[0] * N, 3, device=x.device, generator=generator)
             run = _capi.host.policy_tail if _ops.direct(x) else _end_ops.policy_tail
-            action, logprob, value, pred_next = run(x, alive, obs["team_id"], uniforms, *lists, list(self._team_pma_k), N)
+            teams = (alive, obs["team_id"]) if self._team_pma_k else (None, None)
+            action, logprob, value, pred_next = run(x, *teams, uniforms, *lists, list(self._team_pma_k), N)
             return action, logprob, value, pred_next, new_hidden
         x_ships = x[:, :N, :].contiguous()
         logits = self.action_head(x_ships)

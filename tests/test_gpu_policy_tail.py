@@ -108,3 +108,30 @@ def test_value_columns_count_from_the_end_as_indexing_does():
         p._team_pma_k = (11,)
         with pytest.raises(IndexError):
             p.get_action_and_value(obs, hidden)
+
+
+def test_without_a_team_value_neither_teams_nor_alive_flags_are_needed():
+    p = _policy(4, seed=2, ks=())
+    obs, hidden = _obs(9, 4, 1, 0, seed=8)
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        full = p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
+        del obs["team_id"]
+        bare = p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
+        assert all(torch.equal(a, b) for a, b in zip(full, bare))
+        obs["alive"] = None
+        p.get_action_and_value(obs, hidden)
+
+
+def test_a_short_team_id_raises():
+    p = _policy(4, seed=2)
+    obs, hidden = _obs(9, 4, 1, 0, seed=8)
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        whole = p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
+        team = obs["team_id"]
+        obs["team_id"] = team[:, :4]   # the ships' columns are enough, at any stride
+        ships = p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
+        assert all(torch.equal(a, b) for a, b in zip(whole, ships))
+        for short in (team[:, :3], team[:8]):
+            obs["team_id"] = short
+            with pytest.raises(RuntimeError, match="team_id"):
+                p.get_action_and_value(obs, hidden)
