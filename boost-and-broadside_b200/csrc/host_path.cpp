@@ -696,10 +696,11 @@ Tensor mlp_chain(const Tensor& x, const std::vector<Tensor>& params, int precisi
 }
 
 // Whether policy_tail below serves a step of these sizes.
-bool tail_supported(int64_t d_model, int64_t n_heads, int64_t ships, const std::vector<int64_t>& head_widths) {
+bool tail_supported(int64_t d_model, int64_t n_heads, int64_t ships, const std::vector<int64_t>& heads) {
   if (d_model != 128 || n_heads != 4 || ships < 1 || ships > bnb::tail::MAX_SHIPS) return false;
-  for (int64_t w : head_widths) if (w < 1 || w > 32) return false;
-  return !head_widths.empty() && head_widths[0] == 12 && chain_supported(d_model, 2 * d_model, 32);
+  for (size_t i = 0; i + 2 < heads.size(); i += 3)   // input, hidden and output width
+    if (heads[i] != d_model || heads[i + 1] != 2 * d_model || heads[i + 2] < 1 || heads[i + 2] > 32) return false;
+  return heads.size() >= 3 && heads[2] == 12 && chain_supported(d_model, 2 * d_model, 32);
 }
 
 // Whether a bfloat16 trunk call with these environments reads the tokens of active bullet slots only

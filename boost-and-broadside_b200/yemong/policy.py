@@ -40,6 +40,12 @@ def _tail_supported(d_model: int, n_heads: int, n_ships: int, *head_widths: int)
     return _capi.host.tail_supported(d_model, n_heads, n_ships, list(head_widths))
 
 
+def _plain(module: nn.Module, cls: type) -> bool:
+    """Whether calling ``module`` is what ``cls.forward`` does: no subclass's forward, no hooks."""
+    return (type(module) is cls and not module._forward_hooks and not module._forward_pre_hooks
+            and not torch.nn.modules.module._has_any_global_hook())
+
+
 class YemongPolicy(YemongTrunk):
     """Encoder -> n x YemongBlock -> heads (policy.py:135-214), rollout path."""
 
@@ -76,6 +82,8 @@ class YemongPolicy(YemongTrunk):
         if enc is None or obs.bullets is None:
             return None, None
         active = next(v for k, v in obs.bullets.items() if getattr(k, "name", str(k)).upper().endswith("ACTIVE"))
+        if not _plain(enc, BulletEncoder):
+            return enc(obs), active
         raw = enc.coordinator.get_input_vector(obs)
         compacts = (_capi.current_precision(raw.device) == _capi.BNB_BF16 and tuple(active.shape) == tuple(raw.shape[:-1])
                     and _bullets_compacted(self.d_model, self.n_heads, n_tokens, raw.shape[-2]))
@@ -83,14 +91,21 @@ class YemongPolicy(YemongTrunk):
 
     def _tail_lists(self):
         """Parameters of the heads and of TeamPMA as ``_end_ops.policy_tail`` takes them, or None where
-        its kernels do not serve this policy (or the call is not under the bfloat16 contract)."""
+        its kernels do not serve this policy (modules of other widths, replaced ones, ones with hooks)."""
+        if not _plain(self.next_state_head, NextStateHead):
+            return None
         heads = [self.action_head, self.next_state_head.net, self.value_head_local]
         pma: list[torch.Tensor] = []
         if self._team_pma_k:
             heads.append(self.value_head_win)
+            if not _plain(self.team_pma, TeamPMA) or self.team_pma.n_heads != self.n_heads or self.team_pma.d_model != self.d_model:
+                return None
             pma = [self.team_pma.seeds, self.team_pma.attn.in_proj_weight, self.team_pma.attn.out_proj.weight, self.team_pma.norm.weight]
+        if not all(_plain(h, HeadMLP) for h in heads):
+            return None
         lists = [h.parameter_list() for h in heads]
-        if not _tail_supported(self.d_model, self.n_heads, self._num_ships, *[ps[3].shape[0] for ps in lists]):
+        if not _tail_supported(self.d_model, self.n_heads, self._num_ships,
+                               *[w for ps in lists for w in (ps[0].shape[1], ps[0].shape[0], ps[3].shape[0])]):
             return None
         return [p for ps in lists for p in ps], pma
 
@@ -103,7 +118,7 @@ class YemongPolicy(YemongTrunk):
         bullets, bullet_mask = self._encode_bullets(obs, x.shape[1])
         x, new_hidden = self.step(x, alive, hidden, bullets=bullets, bullet_mask=bullet_mask)
         N = self._num_ships
-        lists = self._tail_lists() if x.dtype == torch.bfloat16 else None
+        lists = self._tail_lists() if x.dtype == torch.bfloat16 and x.shape[1] >= N else None
         if lists is not None:
             uniforms = torch.rand(x.shape[0] * N, 3, device=x.device, generator=generator)
             run = _capi.host.policy_tail if _ops.direct(x) else _end_ops.policy_tail

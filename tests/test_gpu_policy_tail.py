@@ -135,3 +135,27 @@ def test_a_short_team_id_raises():
             obs["team_id"] = short
             with pytest.raises(RuntimeError, match="team_id"):
                 p.get_action_and_value(obs, hidden)
+
+
+def test_replaced_heads_and_hooks_are_called():
+    import boost_and_broadside_b200 as bnb
+
+    p = _policy(4, seed=2)
+    obs, hidden = _obs(9, 4, 1, 6, seed=8)
+    seen = []
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        for module in (p.action_head, p.team_pma, p.next_state_head, p.bullet_encoder):
+            handle = module.register_forward_hook(lambda m, a, out: seen.append(m))
+            got = p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
+            handle.remove()
+            assert seen[-1] is module
+
+        class Doubled(bnb.HeadMLP):
+            def forward(self, x):
+                return 2 * super().forward(x)
+
+        doubled = Doubled(128, 10).to(DEV)
+        doubled.load_state_dict(p.next_state_head.net.state_dict())
+        p.next_state_head.net = doubled
+        twice = p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
+        assert torch.equal(twice[3], 2 * got[3])

@@ -67,3 +67,13 @@ def test_rows_wanted_of_an_encoder_are_as_many_as_its_rows():
 
     with pytest.raises(RuntimeError, match="one element per row"):
         _capi.host.mlp_chain(torch.zeros(8, D), [*_head(12)], _capi.BNB_BF16, torch.ones(7, dtype=torch.bool))
+
+
+def test_only_policies_of_the_built_sizes_take_the_native_end():
+    from boost_and_broadside_b200 import _capi
+
+    head = lambda out, hidden=256, width=128: [width, hidden, out]
+    ok = _capi.host.tail_supported
+    assert ok(128, 4, 8, [*head(12), *head(10), *head(11), *head(2)])
+    for other in ([*head(12, 128), *head(10)], [*head(12), *head(10, 512)], [*head(12), *head(10), *head(11, 256, 64)], [*head(11), *head(10)], []):
+        assert not ok(128, 4, 8, other)
