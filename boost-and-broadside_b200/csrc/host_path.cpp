@@ -628,15 +628,27 @@ int pad32(int64_t n) { return (int)((n + 31) / 32 * 32); }
 bool chain_supported(int64_t in_dim, int64_t hidden, int64_t out_dim) {
   return in_dim <= 128 && hidden <= 256 && out_dim <= 128 && bnb::mlp::supported(pad32(in_dim), (int)hidden, pad32(out_dim));
 }
-bnb::mlp::MlpChain chain_of(const std::vector<Tensor>& ps, const c10::Device& dev, const char* what, void* y, int out, int y_ld) {
+bool on16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+// A parameter that its kernel reads in pieces of 16 bytes and that may start anywhere: a view into a flat buffer that
+// does not is copied, and the copy lives in `held` until the call is queued.
+const float* aligned_parameter(const Tensor& t, const c10::Device& dev, const char* what, std::vector<Tensor>& held) {
+  const float* p = parameter(t, dev, what);
+  if (on16(p)) return p;
+  held.push_back(t.detach().clone());
+  return static_cast<const float*>(held.back().data_ptr());
+}
+// Kernels read first weights of whole 32-column pieces, and an encoder's second one, in 16-byte pieces and refuse them
+// elsewhere; first weights of other widths are read element by element, a head's second weight may start anywhere.
+bnb::mlp::MlpChain chain_of(const std::vector<Tensor>& ps, const c10::Device& dev, const char* what, void* y, int out, int y_ld,
+                            std::vector<Tensor>& held) {
   bnb::mlp::MlpChain c{};
   c.w1 = parameter(ps[0], dev, what);
   c.b1 = parameter(ps[1], dev, what);
   c.g1 = parameter(ps[2], dev, what);
-  c.w2 = parameter(ps[3], dev, what);
+  c.w2 = ps.size() > 5 ? parameter(ps[3], dev, what) : aligned_parameter(ps[3], dev, what, held);
   c.b2 = parameter(ps[4], dev, what);
   c.g2 = ps.size() > 5 ? parameter(ps[5], dev, what) : nullptr;
-  if ((reinterpret_cast<uintptr_t>(c.w1) & 15) || (reinterpret_cast<uintptr_t>(c.w2) & 15))
+  if ((ps[0].size(1) % 32 == 0 && !on16(c.w1)) || !on16(c.w2))
     throw std::runtime_error(std::string(what) + " parameter is not 16-byte aligned");
   c.y = static_cast<__nv_bfloat16*>(y);
   c.out_store = out;
@@ -668,7 +680,8 @@ Tensor mlp_chain(const Tensor& x, const std::vector<Tensor>& params, int precisi
     call.n_rows = (int)rows.size(0);
     call.in_dim = call.w1_ld = (int)in_dim;
     call.active = static_cast<const uint8_t*>(ptr(on));
-    call.chain[0] = chain_of(params, dev, what, y.data_ptr(), (int)out_dim, (int)out_dim);
+    std::vector<Tensor> held;
+    call.chain[0] = chain_of(params, dev, what, y.data_ptr(), (int)out_dim, (int)out_dim, held);
     check(encoder ? "bnb_encoder_mlp_fwd" : "bnb_head_mlp_fwd", bnb::mlp::run(call, 1, pad32(in_dim), (int)hidden, pad32(out_dim), stream));
     return y;
   }
@@ -814,6 +827,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const
   Tensor logits = at::empty({B, N, 12}, bf), pred = at::empty({B, N, P}, bf), value = at::empty({B, N, K}, bf);
   Tensor action = at::empty({B, N, 3}, bf.dtype(at::kLong)), logprob = at::empty({B, N}, bf);
 
+  std::vector<Tensor> held;
   auto five = [&](int i) { return std::vector<Tensor>(heads.begin() + 5 * i, heads.begin() + 5 * i + 5); };
   bnb::mlp::MlpCall call{};
   call.x = x.data_ptr();
@@ -822,9 +836,9 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const
   call.in_dim = call.w1_ld = (int)D;
   call.group_rows = (int)N;
   call.group_stride = (int)NM;
-  call.chain[0] = chain_of(five(0), dev, "head", logits.data_ptr(), 12, 12);
-  call.chain[1] = chain_of(five(1), dev, "head", pred.data_ptr(), (int)P, (int)P);
-  call.chain[2] = chain_of(five(2), dev, "head", value.data_ptr(), (int)K, (int)K);
+  call.chain[0] = chain_of(five(0), dev, "head", logits.data_ptr(), 12, 12, held);
+  call.chain[1] = chain_of(five(1), dev, "head", pred.data_ptr(), (int)P, (int)P, held);
+  call.chain[2] = chain_of(five(2), dev, "head", value.data_ptr(), (int)K, (int)K, held);
   check("bnb_head_mlp_fwd", bnb::mlp::run(call, 3, (int)D, (int)(2 * D), 32, stream));
 
   Tensor win, rows, fold;
@@ -832,15 +846,17 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const
     rows = at::empty({B * 2, D}, bf);
     win = at::empty({B * 2, W}, bf);
     fold = at::empty({(int64_t)bnb::tail::scratch_bytes()}, bf.dtype(at::kByte));
-    check("bnb_team_pma_fwd", bnb::tail::team_rows(s, parameter(pma[0], dev, "TeamPMA"), parameter(pma[1], dev, "TeamPMA"),
-                                                   parameter(pma[2], dev, "TeamPMA"), parameter(pma[3], dev, "TeamPMA"), fold.data_ptr(),
+    const float *in_proj = parameter(pma[1], dev, "TeamPMA"), *out_proj = parameter(pma[2], dev, "TeamPMA");
+    if (!on16(in_proj) || !on16(out_proj)) check("bnb_team_pma_fwd", BNB_ERR_MISALIGNED);
+    check("bnb_team_pma_fwd", bnb::tail::team_rows(s, aligned_parameter(pma[0], dev, "TeamPMA", held), in_proj, out_proj,
+                                                   aligned_parameter(pma[3], dev, "TeamPMA", held), fold.data_ptr(),
                                                    static_cast<__nv_bfloat16*>(rows.data_ptr()), stream));
     bnb::mlp::MlpCall wc{};
     wc.x = rows.data_ptr();
     wc.x_bf16 = 1;
     wc.n_rows = (int)(B * 2);
     wc.in_dim = wc.w1_ld = (int)D;
-    wc.chain[0] = chain_of(five(3), dev, "head", win.data_ptr(), (int)W, (int)W);
+    wc.chain[0] = chain_of(five(3), dev, "head", win.data_ptr(), (int)W, (int)W, held);
     check("bnb_head_mlp_fwd", bnb::mlp::run(wc, 1, (int)D, (int)(2 * D), 32, stream));
   }
   check("bnb_action_dist_fwd", bnb::tail::finish(s, static_cast<const __nv_bfloat16*>(logits.data_ptr()), static_cast<const float*>(uniforms.data_ptr()),

@@ -159,3 +159,40 @@ def test_replaced_heads_and_hooks_are_called():
         p.next_state_head.net = doubled
         twice = p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
         assert torch.equal(twice[3], 2 * got[3])
+
+
+def _move_off_16_bytes(module, name):
+    p = getattr(module, name)
+    flat = torch.empty(p.numel() + 1, device=DEV)
+    view = flat[1:].view(p.shape).copy_(p.detach())
+    assert view.data_ptr() % 16 == 4
+    p.data = view
+
+
+def test_parameters_that_start_between_16_byte_boundaries():
+    """Copied where any start was taken before (biases, gains, seeds, a head's second weight, first weights of
+    odd widths), refused where it was refused."""
+    p = _policy(6, seed=4)
+    obs, hidden = _obs(21, 6, 2, 9, seed=9)
+    step = lambda: p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        ref = step()
+        _move_off_16_bytes(p.team_pma, "seeds")
+        _move_off_16_bytes(p.team_pma.norm, "weight")
+        for head in (p.action_head, p.value_head_local, p.value_head_win, p.next_state_head.net):
+            for module, name in ((head[0], "bias"), (head[1], "weight"), (head[3], "weight"), (head[3], "bias")):
+                _move_off_16_bytes(module, name)
+        for chain in (p.encoder.feature_extractor, p.bullet_encoder.net):   # 66 and 26 columns
+            for module, name in ((chain[0], "weight"), (chain[0], "bias"), (chain[1], "weight"), (chain[3], "bias"), (chain[4], "weight")):
+                _move_off_16_bytes(module, name)
+        for a, b in zip(step(), ref):
+            assert torch.equal(a, b)
+        for module, name in ((p.action_head[0], "weight"), (p.team_pma.attn, "in_proj_weight"), (p.team_pma.attn.out_proj, "weight"),
+                             (p.encoder.feature_extractor[3], "weight")):
+            held = getattr(module, name).data
+            _move_off_16_bytes(module, name)
+            with pytest.raises(RuntimeError, match="align"):
+                step()
+            getattr(module, name).data = held
+        for a, b in zip(step(), ref):
+            assert torch.equal(a, b)
