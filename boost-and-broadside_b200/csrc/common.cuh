@@ -36,6 +36,10 @@ __device__ __forceinline__ float gelu_erf(float v) {
 
 __device__ __forceinline__ float sigmoidf_(float v) { return 1.0f / (1.0f + expf(-v)); }
 
+// Stands for the logarithm of a sigmoid that underflowed to 0 (log_lambda below about -88): finite, so that no
+// difference or product with it is NaN, and so low that every power of the sigmoid but the zeroth still is 0.
+constexpr float kLogOfZero = -1e30f;
+
 // Geometry of a batch on the device: maps environments, ships and fields to rows.
 struct EnvMap {
   int n_envs;

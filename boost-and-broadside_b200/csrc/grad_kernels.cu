@@ -1257,10 +1257,12 @@ __global__ void __launch_bounds__(256) k_conv_fwd(const float* __restrict__ b1, 
 // powf has, at a quarter of its instructions.
 struct Decay {
   float hi, lo;
+  float slope;   // d pow(c) / d c over pow(c): the logarithm, and 0 for a base of 0, whose powers are constant
   __device__ __forceinline__ explicit Decay(float base) {
-    const double v = log((double)base);
+    const double v = base == 0.f ? (double)kLogOfZero : log((double)base);
     hi = (float)v;
     lo = (float)(v - (double)hi);
+    slope = base == 0.f ? 0.f : hi;
   }
   __device__ __forceinline__ float pow(float c) const {
     const float e = c * hi, rest = fmaf(c, lo, fmaf(c, hi, -e)), ea = expf(e);
@@ -1354,7 +1356,7 @@ __global__ void __launch_bounds__(256) k_scan_bwd(float* za, float* zx, const fl
       const float dgate = dh * ig * uv;
       const float di = dh * gate * uv;
       if (cc > kGateFloor) da -= dgate * a / gate;
-      const float dr = da * a * kRglruC * decay.hi;
+      const float dr = da * a * kRglruC * decay.slope;
       dl = fmaf(da * a * kRglruC * rg, 1.0f - base, dl);
       za[at] = dr * rg * (1.0f - rg);
       zx[at] = di * ig * (1.0f - ig);

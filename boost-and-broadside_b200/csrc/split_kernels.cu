@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackJobs j
   if (k == 0) {   // Lambda: the logarithm of its sigmoid as high and low part
     float* out = reinterpret_cast<float*>(dst);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
-      const double v = log((double)sigmoidf_(src[i]));
+      const float base = sigmoidf_(src[i]);
+      const double v = base == 0.f ? (double)kLogOfZero : log((double)base);
       out[i] = (float)v;
       out[rows + i] = (float)(v - (double)(float)v);
     }

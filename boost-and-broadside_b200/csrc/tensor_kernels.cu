@@ -114,7 +114,7 @@ __global__ void k_pack_spatial(BnbSpatialWeights w, uint8_t* out) {
 __global__ void k_pack_temporal(BnbTemporalWeights w, uint8_t* out) {
   if (blockIdx.x == 0 && threadIdx.x < D) {
     float sg = 1.0f / (1.0f + expf(-w.log_lambda[threadIdx.x]));
-    reinterpret_cast<float*>(out + (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES)[threadIdx.x] = kRglruC * log2f(sg);
+    reinterpret_cast<float*>(out + (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES)[threadIdx.x] = kRglruC * (sg == 0.f ? kLogOfZero : log2f(sg));
   }
   pack_image(w, N_TEMPORAL_CHUNKS, out, [](const BnbTemporalWeights& ww, int c, int r) { return temporal_chunk_row(ww, c, r); },
              [](const BnbTemporalWeights& ww, int c) { return temporal_chunk_gain(ww, c); });
@@ -141,7 +141,7 @@ __global__ void k_pack_trunk(const __grid_constant__ PackJobs jobs) {
     uint8_t* out = static_cast<uint8_t*>(const_cast<void*>(w.packed));
     if (blockIdx.x == 0 && threadIdx.x < D) {
       float sg = 1.0f / (1.0f + expf(-w.log_lambda[threadIdx.x]));
-      reinterpret_cast<float*>(out + (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES)[threadIdx.x] = kRglruC * log2f(sg);
+      reinterpret_cast<float*>(out + (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES)[threadIdx.x] = kRglruC * (sg == 0.f ? kLogOfZero : log2f(sg));
     }
     pack_image(w, N_TEMPORAL_CHUNKS, out, [](const BnbTemporalWeights& ww, int c, int r) { return temporal_chunk_row(ww, c, r); },
                [](const BnbTemporalWeights& ww, int c) { return temporal_chunk_gain(ww, c); });
