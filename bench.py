@@ -39,10 +39,10 @@ UNIT = "entity_tokens/s"
 FALLBACK_HBM_GBS = 6650.0
 FALLBACK_BF16_TFLOPS = 1590.0
 # DRAM bytes per entity token of the fused C2 step, from one ncu capture of k_trunk_pipelined on the
-# half-size case (dram__bytes_read.sum + dram__bytes_write.sum = 310 730 496 B for 49 152 tokens,
-# profiles/k_trunk_pipelined_c2_half.md); traffic grows in proportion to the tokens, so a full
+# half-size case (dram__bytes_read.sum + dram__bytes_write.sum = 309 414 400 B for 49 152 tokens,
+# profiles/trunk_step.md); traffic grows in proportion to the tokens, so a full
 # launch is this times its tokens.
-NCU_C2_DRAM_BYTES_PER_TOKEN = (173093120 + 137637376) / 49152
+NCU_C2_DRAM_BYTES_PER_TOKEN = (172023040 + 137391360) / 49152
 
 
 def measured_peaks() -> tuple[float, float, float, str]:

@@ -3,7 +3,9 @@
 //
 // Row tiles of 128 pass by persistent CTAs, one per SM, that keep the 64 KB of weights; the rows of the next tile are
 // on their way while this one is normed and multiplied, and the result of the tile before is written out while the
-// tensor cores work.  Bound by the rows' way through the SM: 256 or 512 bytes in (eight lines a request), 512 out.
+// tensor cores work.  Bound by the rows' way through the SM: 256 or 512 bytes in (eight lines a request), 512 out: 33 us for
+// the 147 000 active rows of 8192 environments of 80 bullets, with DRAM at 23 % of its peak, issue slots 27 % busy, the tensor
+// pipe 16 %, and the stalls shared out between loads, the shared-memory port and its queue.
 // As a program of a general tile kernel, with weights streamed per tile and a thread per row on the way in and out,
 // it took 73 us for the active rows of 8192 environments of 80 bullets.
 #include "bullet_kv.h"

@@ -89,7 +89,8 @@ __device__ __forceinline__ void rows_product(float (&acc)[2][4], uint32_t sA, in
 
 // Persistent CTAs of 16 warps, both weights resident as bfloat16.  A round is 16 environments: a warp
 // scores and pools one of them (a lane owns 4 channels, so a ship row is one 256-byte request), then the
-// 32 team rows go through Wv and out_proj as mma.sync products of 8 columns per warp.
+// 32 team rows go through Wv and out_proj as mma.sync products of 8 columns per warp.  Bound by latency: 55 us for
+// 8192 environments of 8 ships, issue slots 27 % busy, DRAM 4 % of its peak, a warp's rows read one after the other.
 __global__ void __launch_bounds__(THREADS, 1) k_team_rows(const Ships s, const float* __restrict__ qk, const float* __restrict__ in_proj,
                                                           const float* __restrict__ out_w, const float* __restrict__ norm_w,
                                                           __nv_bfloat16* __restrict__ rows) {
