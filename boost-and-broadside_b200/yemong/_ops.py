@@ -3,9 +3,9 @@
 ``torch.compile(policy)`` (the reference trains and evaluates through it,
 train/rl/ppo.py:396-400) must neither trace into ctypes nor break CUDA-graph capture, so the
 calls into the library are registered as custom operators: Dynamo sees one opaque node with a
-shape-only fake implementation; the real implementation below builds the ctypes argument
-structs, looks up (or rebuilds) the tensor-core weight images, takes scratch from torch's
-allocator and launches on the current stream.  Nothing here synchronises.
+shape-only fake implementation.  The real implementations are native code (csrc/host_path.cpp),
+which eager calls that nobody has to see (``direct``) enter without the operator dispatcher; the
+single-sublayer operator builds its ctypes structs here.  Nothing here synchronises.
 
 ``trunk_forward`` carries an autograd formula (``trunk_backward`` -> ``bnb_trunk_sequence_bwd``,
 environments of one size, recomputing activations); a call known to need gradients goes through
@@ -17,9 +17,8 @@ single-sublayer operators are forward-only and their module methods refuse input
 
 from __future__ import annotations
 
-from typing import List, Optional, Tuple
-
 import os
+from typing import List, Optional, Tuple
 
 import torch
 from torch import Tensor
