@@ -629,25 +629,33 @@ bool chain_supported(int64_t in_dim, int64_t hidden, int64_t out_dim) {
   return in_dim <= 128 && hidden <= 256 && out_dim <= 128 && bnb::mlp::supported(pad32(in_dim), (int)hidden, pad32(out_dim));
 }
 bool on16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+const float* held_parameter(const Tensor& copy, const c10::Device& dev, const char* what, std::vector<Tensor>& held) {
+  held.push_back(copy);
+  return parameter(copy, dev, what);
+}
 // A parameter that its kernel reads in pieces of 16 bytes and that may start anywhere: a view into a flat buffer that
 // does not is copied, and the copy lives in `held` until the call is queued.
 const float* aligned_parameter(const Tensor& t, const c10::Device& dev, const char* what, std::vector<Tensor>& held) {
   const float* p = parameter(t, dev, what);
-  if (on16(p)) return p;
-  held.push_back(t.detach().clone());
-  return static_cast<const float*>(held.back().data_ptr());
+  return on16(p) ? p : held_parameter(t.detach().clone(), dev, what, held);
 }
-// Kernels read first weights of whole 32-column pieces, and an encoder's second one, in 16-byte pieces and refuse them
-// elsewhere; first weights of other widths are read element by element, a head's second weight may start anywhere.
+// One that may be strided (a transposed view).
+const float* strided_parameter(const Tensor& t, const c10::Device& dev, const char* what, std::vector<Tensor>& held) {
+  return t.is_contiguous() ? parameter(t, dev, what) : held_parameter(t.detach().contiguous(), dev, what, held);
+}
+// An encoder's first layer and a head's second one may be strided, the latter may start anywhere too.  Kernels read first
+// weights of whole 32-column pieces, and an encoder's second one, in 16-byte pieces and refuse them elsewhere; first
+// weights of other widths are read element by element.
 bnb::mlp::MlpChain chain_of(const std::vector<Tensor>& ps, const c10::Device& dev, const char* what, void* y, int out, int y_ld,
                             std::vector<Tensor>& held) {
   bnb::mlp::MlpChain c{};
-  c.w1 = parameter(ps[0], dev, what);
+  const bool encoder = ps.size() > 5;
+  c.w1 = encoder ? strided_parameter(ps[0], dev, what, held) : parameter(ps[0], dev, what);
   c.b1 = parameter(ps[1], dev, what);
   c.g1 = parameter(ps[2], dev, what);
-  c.w2 = ps.size() > 5 ? parameter(ps[3], dev, what) : aligned_parameter(ps[3], dev, what, held);
-  c.b2 = parameter(ps[4], dev, what);
-  c.g2 = ps.size() > 5 ? parameter(ps[5], dev, what) : nullptr;
+  c.w2 = encoder ? parameter(ps[3], dev, what) : ps[3].is_contiguous() ? aligned_parameter(ps[3], dev, what, held) : strided_parameter(ps[3], dev, what, held);
+  c.b2 = encoder ? parameter(ps[4], dev, what) : strided_parameter(ps[4], dev, what, held);
+  c.g2 = encoder ? parameter(ps[5], dev, what) : nullptr;
   if ((ps[0].size(1) % 32 == 0 && !on16(c.w1)) || !on16(c.w2))
     throw std::runtime_error(std::string(what) + " parameter is not 16-byte aligned");
   c.y = static_cast<__nv_bfloat16*>(y);
@@ -691,7 +699,7 @@ Tensor mlp_chain(const Tensor& x, const std::vector<Tensor>& params, int precisi
   const float *b1 = parameter(params[1], dev, what), *g1 = parameter(params[2], dev, what);
   if (encoder) {
     const int in_pad = pad32(in_dim);
-    const Tensor w1 = in_pad == in_dim ? params[0] : at::constant_pad_nd(params[0].detach(), {0, in_pad - in_dim});
+    const Tensor w1 = in_pad == in_dim ? contiguous(params[0].detach()) : at::constant_pad_nd(params[0].detach(), {0, in_pad - in_dim});
     check("bnb_encoder_mlp_fwd",
           bnb_encoder_mlp_fwd(parameter(w1, dev, what), b1, g1, parameter(params[3], dev, what), parameter(params[4], dev, what),
                               parameter(params[5], dev, what), (int)in_dim, in_pad, (int)hidden, (int)out_dim,

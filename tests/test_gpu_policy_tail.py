@@ -196,3 +196,32 @@ def test_parameters_that_start_between_16_byte_boundaries():
             getattr(module, name).data = held
         for a, b in zip(step(), ref):
             assert torch.equal(a, b)
+
+
+def test_parameters_that_are_transposed_views():
+    """An encoder's first weight and a head's second one (and its bias) are copied when they are strided."""
+    p = _policy(6, seed=4)
+    obs, hidden = _obs(21, 6, 2, 9, seed=9)
+    step = lambda: p.get_action_and_value(obs, hidden, generator=torch.Generator(device=DEV).manual_seed(3))
+    heads = (p.action_head, p.value_head_local, p.value_head_win, p.next_state_head.net)
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        ref, x = step(), torch.randn(70, 128, device=DEV).to(torch.bfloat16)
+        rows = [h(x) for h in heads]
+        for linear in (p.encoder.feature_extractor[0], p.bullet_encoder.net[0], *(h[3] for h in heads)):
+            linear.weight.data = linear.weight.data.t().contiguous().t()
+            assert not linear.weight.is_contiguous()
+        for h in heads:
+            h[3].bias.data = torch.stack([h[3].bias.data, h[3].bias.data], dim=1)[:, 0]
+        for a, b in zip([*step(), *(h(x) for h in heads)], [*ref, *rows]):
+            assert torch.equal(a, b)
+        p.action_head[0].weight.data = p.action_head[0].weight.data.t().contiguous().t()
+        with pytest.raises(RuntimeError, match="contiguous"):
+            step()
+    with torch.no_grad():   # float32: a first weight of whole 32-column pieces goes in without a padded copy
+        from boost_and_broadside_b200 import _capi
+        ps = [torch.randn(256, 64, device=DEV), *(torch.randn(256, device=DEV) for _ in range(2)), torch.randn(128, 256, device=DEV),
+              *(torch.randn(128, device=DEV) for _ in range(2))]
+        raw = torch.randn(33, 64, device=DEV)
+        a = _capi.host.mlp_chain(raw, ps, _capi.BNB_FP32, None)
+        b = _capi.host.mlp_chain(raw, [ps[0].t().contiguous().t(), *ps[1:]], _capi.BNB_FP32, None)
+        assert torch.equal(a, b)
