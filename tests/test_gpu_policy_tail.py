@@ -225,3 +225,15 @@ def test_parameters_that_are_transposed_views():
         a = _capi.host.mlp_chain(raw, ps, _capi.BNB_FP32, None)
         b = _capi.host.mlp_chain(raw, [ps[0].t().contiguous().t(), *ps[1:]], _capi.BNB_FP32, None)
         assert torch.equal(a, b)
+
+
+def test_a_policy_without_a_team_value_compiles_to_one_graph():
+    p = _policy(8, seed=5, ks=())
+    obs, hidden = _obs(16, 8, 4, 24, seed=6)
+    compiled = torch.compile(p.get_action_and_value, mode="reduce-overhead", fullgraph=True)
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        _, _, v0, p0, h0 = p.get_action_and_value(obs, hidden)
+        for _ in range(3):
+            _, _, v, pn, h = compiled(obs, hidden)
+            v, pn, h = v.clone(), pn.clone(), h.clone()
+    assert torch.equal(v, v0) and torch.equal(pn, p0) and torch.equal(h, h0)
