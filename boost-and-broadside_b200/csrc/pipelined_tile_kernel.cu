@@ -5,7 +5,7 @@
 //   16 epilogue warps   four threads per tile row (thread (row, part): TMEM lane = row, a quarter
 //                       of whatever columns are being read).  RMSNorm, q|k|v staging, attention
 //                       (mma.sync), gelu(gate) * up, causal conv, RG-LRU gates and state update.
-//   1 issuing warp      issues every tcgen05.mma.  It waits for "operand ready" (the
+//   2 issuing warps     issue every tcgen05.mma, one the down projections, one the rest.  They wait for "operand ready" (the
 //                       epilogue warps arrive on an mbarrier after fence.proxy.async) and for
 //                       "chunk landed" (the bulk copy's complete_tx), and signals "accumulator
 //                       ready" / "slot free" with tcgen05.commit.
@@ -39,9 +39,10 @@ namespace pipe {
 
 constexpr int EPI_WARPS = 16;
 constexpr int EPI_THREADS = 32 * EPI_WARPS;
-constexpr int MMA_WARP = EPI_WARPS;
-constexpr int LOAD_WARP = EPI_WARPS + 1;
-constexpr int THREADS = EPI_THREADS + 64;
+constexpr int MMA_WARP = EPI_WARPS;        // every product but the down projections
+constexpr int DOWN_WARP = EPI_WARPS + 1;   // the down projections
+constexpr int LOAD_WARP = EPI_WARPS + 2;
+constexpr int THREADS = EPI_THREADS + 96;
 // Weight ring: three pair slots (32 KB: both K atoms of one 128-row weight block, consumed by
 // eight MMAs) and three single slots (16 KB: one down-projection chunk).  Slots 0, 1 (pairs) and
 // 3 (single) are dedicated; 2, 4 and 5 live in the key/value staging area and carry weights only
@@ -66,12 +67,12 @@ constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
 // issued after the wait, so a phase is never overtaken.  KVREL: the key/value area
 // may take weights again (epilogue warps -> fetching warp).  FULL[s]: the weights of slot s have landed.
 // DONE[s]: the MMAs that read slot s are complete (tcgen05.commit) -- the fetching warp takes it as
-// "slot free" and the epilogue warps as "accumulator ready" for gate|up of one chunk, whose slot is not
-// used again before they have seen it.  QKV[h]: q|k|v of head h is complete (a barrier per head: a slot
-// serves two heads, and a phase waited for too late would look like the one after next).  ACC: every MMA of a round is complete (one more commit per round).
+// "slot free", the epilogue warps as "accumulator ready" for gate|up of one chunk, whose slot is not
+// used again before they have seen it, and the issuing warp of gate|up as "accumulator free" for a down projection.
+// ACC: every MMA of a round is complete (one more commit per round).
 // EARLY: the first product of a temporal sublayer's two larger rounds is.  DRAIN: every MMA of the
-// CTA is complete (once, at the end).
-enum : int { B_OP0 = 0, B_FFN0, B_FFN1, B_FFN2, B_KVREL, B_ACC, B_EARLY, B_DRAIN, B_QKV0, B_FULL0 = B_QKV0 + HEADS, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
+// CTA is complete (once per issuing warp, at the end).
+enum : int { B_OP0 = 0, B_FFN0, B_FFN1, B_FFN2, B_KVREL, B_DRAIN, B_ACC, B_EARLY, B_FULL0, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
 static_assert(B_COUNT * 8 + 8 <= 256, "barrier area");
 
 constexpr uint32_t COL_RESID = 0;
@@ -122,81 +123,58 @@ __device__ __forceinline__ void trace(Trace& t, int id) {
 
 // One ring operation as the fetching warp needs it: source of the first chunk (64 bits), byte distance
 // from it to the second chunk (0: a single), and slot (bits 0-2) | wait for the key/value area first (8).
-// Resolved once at kernel start, so that a fetch is a dozen instructions.
-constexpr uint32_t NO_CHUNK = 63;
-__device__ __forceinline__ uint4 sched_entry(int slot, const uint8_t* image, int ch0, uint32_t ch1, bool kvwait) {
-  const unsigned long long src = reinterpret_cast<unsigned long long>(image + (size_t)ch0 * CHUNK_BYTES);
-  return make_uint4((uint32_t)src, (uint32_t)(src >> 32), ch1 == NO_CHUNK ? 0u : (ch1 - (uint32_t)ch0) * CHUNK_BYTES,
-                    (uint32_t)slot | (kvwait ? 8u : 0u));
-}
+// Resolved once at kernel start, a thread per operation, so that a fetch is a dozen instructions.
 constexpr int MAX_SCHED = MAX_SUBLAYERS * 22;
+static_assert(MAX_SCHED <= THREADS, "one thread writes one entry");
 
-// Ring operations of a sublayer in the order the issuing warp consumes them.  All three roles walk the
-// same order with the same slot rotation.  GatedMLP with image base b: gate|up of chunk c are chunks
-// b + 3c, b + 3c + 1 (a pair), its down projection is b + 3c + 2 (a single); the three-deep pipeline
-// consumes GU0 GU1 GU2 D0 GU3 D1 GU4 D2 ... GU7 D5 D6 D7.
-struct SlotRotation {
-  uint32_t pair, single;
-  __device__ __forceinline__ uint32_t next_pair() { const uint32_t r = pair; pair = pair == 2 ? 0 : pair + 1; return r; }
-  __device__ __forceinline__ uint32_t next_single() { const uint32_t r = single; single = single == 5 ? 3 : single + 1; return r; }
-};
-// q|k|v of the four heads: the one slot inside the key/value area first, because keys and values are
-// staged there as soon as a head is ready; then the dedicated slots.
-__device__ __forceinline__ uint32_t qkv_slot(uint32_t h) { return h == 0 ? 2u : h == 2 ? 0u : 1u; }
-// After them out_proj goes to pair slot 0, the first gate|up to pair slot 1 and the first down projection
-// to single slot 3 (all dedicated: fetched while the attention runs); the second gate|up is the first
-// operation that goes to the key/value area and waits for it.
-__device__ __forceinline__ void after_qkv(SlotRotation& rot) { rot.pair = 0; rot.single = 3; }
-
-__device__ __forceinline__ int ffn_ops(uint4* out, int n, const uint8_t* image, int base, SlotRotation& rot, int first_flagged) {
-  // first_flagged: index (in GU order) of the first gate|up pair that must wait for the key/value area, or -1
-  for (int c = 0; c < 3; ++c) out[n++] = sched_entry(rot.next_pair(), image, base + 3 * c, base + 3 * c + 1, c == first_flagged);
-  for (int c = 0; c < 8; ++c) {
-    out[n++] = sched_entry(rot.next_single(), image, base + 3 * c + 2, NO_CHUNK, false);
-    if (c + 3 < 8) out[n++] = sched_entry(rot.next_pair(), image, base + 3 * (c + 3), base + 3 * (c + 3) + 1, false);
-  }
-  return n;
+// Ring operations of a sublayer.  Every sublayer starts at pair slot 0 and single slot 3 and takes them in turn, so that
+// all roles know the slot of an operation from its place in the sublayer.
+//   spatial    q, k, v -> pairs 0 1 2; out_proj -> 0 (dedicated: fetched while the attention runs); GatedMLP from pair 1 on,
+//              whose second gate|up is the first operation that goes to the key/value area and waits for it
+//   PRE        q, k, v;  POST  out_proj and the GatedMLP
+//   temporal   linear2, linear1 -> 0 1; gates -> 2 0; field_sub -> 1 (left out without fields); linear_out -> 2; GatedMLP from 0 on
+// GatedMLP with image base b: gate|up of chunk c are chunks b + 3c, b + 3c + 1 (a pair), its down projection is
+// b + 3c + 2 (a single); fetched in the order GU0 GU1 GU2 D0 GU3 D1 GU4 D2 ... GU7 D5 D6 D7.
+constexpr uint32_t SPATIAL_FFN_PAIR = 1, TEMPORAL_FFN_PAIR = 0;   // pair slot of gate|up of chunk 0
+constexpr int FFN_OPS = 16;
+__device__ __forceinline__ int sublayer_ops(int type, bool has_fields) {
+  return type == SUB_SPATIAL ? 4 + FFN_OPS : type == SUB_SPATIAL_PRE ? 3 : type == SUB_SPATIAL_POST ? 1 + FFN_OPS : (has_fields ? 6 : 5) + FFN_OPS;
 }
-__device__ __forceinline__ int build_schedule(const SubLayer* subs, int n_sub, bool has_fields, uint4* out) {
-  int n = 0;
-  SlotRotation rot{0, 3};
-  for (int si = 0; si < n_sub; ++si) {
-    const uint8_t* image = subs[si].packed;
-    if (subs[si].type == SUB_SPATIAL || subs[si].type == SUB_SPATIAL_PRE) {
-      for (int h = 0; h < HEADS; ++h) {
-        const int ch = 5 * (h >> 1) + 2 * (h & 1);
-        out[n++] = sched_entry(qkv_slot(h), image, ch, ch + 1, false);
-      }
-      after_qkv(rot);
-      if (subs[si].type == SUB_SPATIAL_PRE) continue;   // the attention runs in a kernel of its own between this launch and the next
-      out[n++] = sched_entry(rot.next_pair(), image, 4, 9, false);
-      n = ffn_ops(out, n, image, 10, rot, 1);
-    } else if (subs[si].type == SUB_SPATIAL_POST) {
-      // out_proj on the attention output read back from global memory, then the GatedMLP; nothing
-      // of this sublayer uses the key/value area, so no operation waits for it
-      out[n++] = sched_entry(rot.next_pair(), image, 4, 9, false);
-      n = ffn_ops(out, n, image, 10, rot, -1);
-    } else {
-      for (int i = 0; i < 6; ++i) {
-        if (!has_fields && i == 4) continue;
-        out[n++] = sched_entry(rot.next_pair(), image, 2 * i, 2 * i + 1, false);
-      }
-      n = ffn_ops(out, n, image, 12, rot, -1);
-    }
+__device__ __forceinline__ uint4 sched_entry(const SubLayer& s, int op, bool has_fields) {
+  int slot, chunk, base;
+  bool pair = true, kvwait = false;
+  int f;   // place inside the GatedMLP, negative before it
+  uint32_t first;
+  if (s.type == SUB_TEMPORAL) {
+    f = op - (has_fields ? 6 : 5);
+    const int k = has_fields || op < 4 ? op : op + 1;   // 0 linear2, 1 linear1, 2 and 3 gates, 4 field_sub, 5 linear_out
+    slot = k % 3;
+    chunk = 2 * k;
+    base = 12;
+    first = TEMPORAL_FFN_PAIR;
+  } else {
+    const int k = s.type == SUB_SPATIAL_POST ? op + 3 : op;   // 0 q, 1 k, 2 v, 3 out_proj
+    f = k - 4;
+    slot = k % 3;
+    chunk = 2 * k;
+    base = 8;
+    first = SPATIAL_FFN_PAIR;
   }
-  return n;
+  if (f >= 0) {
+    const int k = f - 3;
+    const int c = f < 3 ? f : k < 10 ? ((k & 1) ? 3 + (k >> 1) : k >> 1) : k - 5;
+    pair = f < 3 || (k < 10 && (k & 1));
+    slot = pair ? (int)(first + c) % 3 : 3 + c % 3;
+    chunk = base + 3 * c + (pair ? 0 : 2);
+    kvwait = s.type == SUB_SPATIAL && f == 1;
+  }
+  const unsigned long long src = reinterpret_cast<unsigned long long>(s.packed + (size_t)chunk * CHUNK_BYTES);
+  return make_uint4((uint32_t)src, (uint32_t)(src >> 32), pair ? CHUNK_BYTES : 0u, (uint32_t)slot | (kvwait ? 8u : 0u));
 }
 
-__device__ __forceinline__ uint32_t slot_offset(uint32_t slot) {
-  switch (slot) {
-    case 0: return OFF_RING;
-    case 1: return OFF_RING + 2 * CHUNK_BYTES;
-    case 2: return OFF_KV;
-    case 3: return OFF_RING + 4 * CHUNK_BYTES;
-    case 4: return OFF_KV + 2 * CHUNK_BYTES;
-    default: return OFF_KV + 3 * CHUNK_BYTES;
-  }
-}
+__device__ __forceinline__ uint32_t pair_offset(uint32_t slot) { return slot == 2 ? OFF_KV : OFF_RING + slot * 2 * CHUNK_BYTES; }
+__device__ __forceinline__ uint32_t single_offset(uint32_t i) { return i == 0 ? OFF_RING + 4 * CHUNK_BYTES : OFF_KV + (1 + i) * CHUNK_BYTES; }
+__device__ __forceinline__ uint32_t slot_offset(uint32_t slot) { return slot < 3 ? pair_offset(slot) : single_offset(slot - 3); }
 
 // ------------------------------------------------------------------ epilogue side
 
@@ -212,8 +190,7 @@ struct Epi {
   uint32_t sbase;       // shared address of smem
   uint32_t bars;        // shared address of the barrier array
   uint32_t lane_addr;   // tensor-memory address of this thread's lane, column 0
-  uint32_t par;         // phase bits of the pair slots' DONE barriers (0..2), of ACC (8) and of QKV (9)
-  SlotRotation rot;     // pair slot of the next ring operation
+  uint32_t par;         // phase bits of the pair slots' DONE barriers (0..2), of ACC (8) and of EARLY (10)
   int row, part;
   bool wide;            // 32-byte accesses: every row pointer is aligned for them
   int* status;
@@ -231,7 +208,7 @@ __device__ __forceinline__ void post(Epi& e, int bar) {
   TRACE(e.tr, 210 + bar);
 }
 // The epilogue threads keep one phase bit per pair slot and flip it for every pair operation of the
-// schedule, in order, whether they wait for it or not.
+// schedule, whether they wait for it or not.
 //
 // wait_acc: every MMA issued so far is complete (a commit on ACC ends every round).
 __device__ __forceinline__ void wait_acc(Epi& e) {
@@ -251,10 +228,10 @@ __device__ __forceinline__ void wait_early(Epi& e) {
   tc_fence_after();
   T_END(e.tacc, e.wait_slot);
 }
-// wait_round: a round of n pair operations in rotation order, then a commit on ACC.
-__device__ __forceinline__ void wait_round(Epi& e, int n) {
+// wait_round: a round whose pair operations took an odd number of turns on the slots of `flips`, then a commit on ACC.
+__device__ __forceinline__ void wait_round(Epi& e, uint32_t flips) {
   wait_acc(e);
-  for (int i = 0; i < n; ++i) e.par ^= 1u << e.rot.next_pair();
+  e.par ^= flips;
 }
 // wait_op: gate|up of one chunk.  A thread that skips operations of a slot must not find the slot a phase
 // behind or two ahead: it waits only when an operation issued after the skipped one is known to be
@@ -337,12 +314,11 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* s) {
 // The gated product stays in tensor memory as the A operand of the down projection: 16 k at a time
 // (8 columns of packed bf16 pairs) over the first half of 16 gate columns the thread has just read;
 // K step s of the MMA reads exactly the columns at 16 s.
-__device__ __forceinline__ void ffn(Epi& e) {
+__device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slot of chunk 0
   const int group = e.part >> 1, half = e.part & 1;
   T_WAITSLOT(e, TE_FFN_ACC_WAIT);
 #pragma unroll 1
   for (int c = 0; c < 8; ++c) {
-    const uint32_t slot = e.rot.next_pair();
     if ((c & 1) == group) {
       wait_op(e, slot);   // gate|up of chunk c; the slot's previous operation, c - 3, came before c - 2
       T_BEGIN();
@@ -364,6 +340,7 @@ __device__ __forceinline__ void ffn(Epi& e) {
       post(e, B_FFN0 + c % 3);
     }
     e.par ^= 1u << slot;
+    slot = slot == 2 ? 0 : slot + 1;
   }
   T_WAITSLOT(e, TE_ACC_WAIT);
   wait_acc(e);   // residual complete: every down projection
@@ -486,29 +463,17 @@ __device__ __forceinline__ void attention(Epi& e, int n_items) {
   }
 }
 
-// q|k|v of head `part` in columns [128 + 96 part, +96): the threads of part h go on while the later heads
-// are multiplied.
-__device__ __forceinline__ void wait_qkv(Epi& e) {
-  T_BEGIN();
-  mbar_wait(e.bars + 8 * (B_QKV0 + e.part), (e.par >> 9) & 1u, e.status, e.aborted, ST_TIMEOUT_ACC);
-  tc_fence_after();
-  e.par ^= 1u << 9;
-#pragma unroll
-  for (uint32_t h = 0; h < HEADS; ++h) e.par ^= 1u << qkv_slot(h);
-  after_qkv(e.rot);
-  T_END(e.tacc, e.wait_slot);
-  TRACE(e.tr, 114);
-}
+// q | k | v of all heads in the three accumulators.
+constexpr uint32_t QKV_FLIPS = 7, OUT_FLIPS = 1;
 
 __device__ __forceinline__ void run_spatial(Epi& e, int n_items, bool row_valid) {
   norm_to_A(e);
   post(e, B_OP0);
-  wait_qkv(e);
+  wait_round(e, QKV_FLIPS);
   {
     T_BEGIN();
-    // this thread stages head `part` of its row: q into the P area (the normed operand is still being
-    // read for the later heads), k and v into the KV area (whose ring slot served head 0), all in the
-    // swizzled atom layout.  Rows outside every environment are zero rows from the input on.
+    // this thread stages head `part` of its row: q into the P area, k and v into the KV area (whose ring slot
+    // served v), all in the swizzled atom layout.  Rows outside every environment are zero rows from the input on.
     const int h = e.part;
     const uint32_t atom = (uint32_t)(h >> 1) * CHUNK_BYTES;
     const int c8h = (h & 1) * 4;
@@ -516,7 +481,7 @@ __device__ __forceinline__ void run_spatial(Epi& e, int n_items, bool row_valid)
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
       uint32_t v[32];
-      tmem_ld32(e.lane_addr + COL_ACC0 + h * 96 + p * 32, v);
+      tmem_ld32(e.lane_addr + COL_ACC0 + p * D + h * DH, v);
 #pragma unroll
       for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(e.smem + dst[p] + swz(e.row, c8h + q)) = row_valid ? pack8(&v[q * 8]) : make_uint4(0u, 0u, 0u, 0u);
     }
@@ -533,10 +498,10 @@ __device__ __forceinline__ void run_spatial(Epi& e, int n_items, bool row_valid)
   __syncwarp();
   if ((threadIdx.x & 31) == 0) mbar_arrive(e.bars + 8 * B_KVREL);
   post(e, B_OP0);   // attention output in P
-  wait_round(e, 1);   // out_proj accumulated into the residual
+  wait_round(e, OUT_FLIPS);   // out_proj accumulated into the residual
   norm_to_A(e);
   post(e, B_OP0);
-  ffn(e);
+  ffn(e, SPATIAL_FFN_PAIR);
 }
 
 // A spatial sublayer around a separate attention kernel (environments larger than a tile, or a
@@ -545,13 +510,13 @@ __device__ __forceinline__ void run_spatial(Epi& e, int n_items, bool row_valid)
 __device__ __forceinline__ void run_spatial_pre(Epi& e, const SubLayer& s, size_t grow, bool row_valid) {
   norm_to_A(e);
   post(e, B_OP0);
-  wait_qkv(e);
+  wait_round(e, QKV_FLIPS);
   const int h = e.part;
   __nv_bfloat16* dst = s.qkv_out + grow * (3 * D) + h * DH;
 #pragma unroll
   for (int p = 0; p < 3; ++p) {
     uint32_t v[32];
-    tmem_ld32(e.lane_addr + COL_ACC0 + h * 96 + p * 32, v);
+    tmem_ld32(e.lane_addr + COL_ACC0 + p * D + h * DH, v);
     if (row_valid) {
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
@@ -579,10 +544,10 @@ __device__ __forceinline__ void run_spatial_post(Epi& e, const SubLayer& s, size
     }
   }
   post(e, B_OP0);
-  wait_round(e, 1);   // out_proj accumulated into the residual
+  wait_round(e, OUT_FLIPS);   // out_proj accumulated into the residual
   norm_to_A(e);
   post(e, B_OP0);
-  ffn(e);
+  ffn(e, SPATIAL_FFN_PAIR);
 }
 
 struct RowState {
@@ -610,7 +575,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
 #pragma unroll
     for (int j = 0; j < 8; ++j) b2p[rnd][j] = pack_bf16(gelu_fast(__uint_as_float(v[2 * j])), gelu_fast(__uint_as_float(v[2 * j + 1])));
   }
-  wait_round(e, 2);   // acc1 = linear1 n
+  wait_round(e, 3);   // acc1 = linear1 n; slots 0 and 1
   // b1 = bf16(linear1 n) into the A operand; ships: causal conv with the stored taps -> u
   {
     uint32_t v[32];
@@ -707,7 +672,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
   // gates and state update
 #pragma unroll
   for (int rnd = 0; rnd < 2; ++rnd) {
-    if (rnd == 1) wait_round(e, has_fields ? 3 : 2);   // the rest; acc2 = field_sub b1
+    if (rnd == 1) wait_round(e, has_fields ? 7 : 5);   // the rest; acc2 = field_sub b1; slots 2, 0 (and 1)
     uint32_t rv[16], iv[16];
     const uint32_t acc = e.lane_addr + COL_ACC0 + rnd * 128 + e.part * 16;
     tmem_ld16_nowait(acc, rv);        // executed by every lane of the warp
@@ -804,20 +769,22 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
   }
   post(e, B_OP0);   // branch operand
   T_SINCE(e.tacc, TE_TEMPORAL, tu);
-  wait_round(e, 1);   // residual += linear_out(branch)
+  wait_round(e, 4);   // residual += linear_out(branch); slot 2
   norm_to_A(e);
   post(e, B_OP0);
-  ffn(e);
+  ffn(e, TEMPORAL_FFN_PAIR);
 }
 
-// ------------------------------------------------------------------ issuing side (one warp)
+// ------------------------------------------------------------------ issuing side (two warps)
 //
-// The whole warp runs this code with the same values in every lane, and one elected lane issues: the
-// operands of the MMAs then stay in uniform registers and an MMA costs three instructions.  Run by a
-// single lane, each MMA had to move its descriptors over first, and under the instruction-cache pressure
-// of the sixteen epilogue warps eight MMAs took 790 cycles of issue (1000 for the four of a down
-// projection) against the 520 (260) they need in the tensor pipe, which made the issue the slowest stage
-// of the GatedMLP.  For the same reason everything here is inlined.
+// A whole warp runs this code with the same values in every lane, and one elected lane issues: the
+// operands of the MMAs then stay in uniform registers and an MMA costs three instructions.
+//
+// What bounds the GatedMLP is issue, not the tensor pipe: with one warp issuing everything, a chunk's two waits for
+// weights, one for its operand and twelve MMAs were a serial chain of 1 400 cycles where the pipe needs 770 (64 cycles per
+// 128 x 128 x 16).  So the down projections have a warp of their own, on another scheduler.  What the order of one thread's
+// MMAs gave for free is then a wait: gate|up of chunk c + 3 overwrites the accumulator that the down projection of chunk c
+// reads its operand from, and waits for its commit.
 
 struct Issuer {
 #ifdef BNB_TRACE
@@ -830,7 +797,7 @@ struct Issuer {
   uint32_t elected;    // 1 in the lane that issues
   uint32_t full_par;   // per-slot phase bits of the FULL barriers
   uint32_t op_par;     // phase bits of OP0 and FFN0..2
-  SlotRotation rot;
+  uint32_t down_par;   // phase bits of the single slots' DONE barriers
   int* status;
   volatile int* aborted;
 };
@@ -844,23 +811,21 @@ __device__ __forceinline__ void wait_operand(Issuer& m, int bar) {
   TRACE(m.tr, 400 + bar);
 }
 __device__ __forceinline__ void commit_one(const Issuer& m, uint32_t bar) { tc_commit_if(m.elected, m.bars + 8 * bar); }
-// Waits for the weights of a slot; returns the low descriptor word of its first chunk.
-__device__ __forceinline__ uint32_t wait_weights(Issuer& m, uint32_t slot) {
+// Waits for the weights of a slot.
+__device__ __forceinline__ void wait_weights(Issuer& m, uint32_t slot) {
   T_MARK(tw);
   mbar_wait(m.bars + 8 * (B_FULL0 + slot), (m.full_par >> slot) & 1u, m.status, m.aborted, ST_TIMEOUT_FULL);
   m.full_par ^= 1u << slot;
   T_SINCE(m.tacc, TM_FULL_WAIT, tw);
   TRACE(m.tr, 410);
-  return uniform(desc_lo(m.sbase + slot_offset(slot)));
 }
-// A pair operation: D[128 x n] (+)= A[128 x 128] * W[n x 128]^T, K atom 0 of the operand at a_off0 and K
+// A pair operation: D[128 x 128] (+)= A[128 x 128] * W[128 x 128]^T, K atom 0 of the operand at a_off0 and K
 // atom 1 at a_off1; commits on the slot's DONE barrier.  (A step of 16 K columns = 32 bytes = 2 in
 // descriptor units; a K atom = 16 KB = 1024 units.)
-__device__ __forceinline__ void issue_pair(Issuer& m, uint32_t slot, uint32_t a_off0, uint32_t a_off1, uint32_t n, uint32_t d_col,
-                                           uint32_t accumulate) {
-  const uint32_t b_lo = wait_weights(m, slot);
+__device__ __forceinline__ void multiply_pair(Issuer& m, uint32_t slot, uint32_t a_off0, uint32_t a_off1, uint32_t d_col, uint32_t accumulate) {
   T_MARK(tw);
-  const uint32_t idesc = instr_desc(n);
+  constexpr uint32_t idesc = instr_desc(128);
+  const uint32_t b_lo = uniform(desc_lo(m.sbase + pair_offset(slot)));
   const uint32_t a0 = desc_lo(m.sbase + a_off0), a1 = desc_lo(m.sbase + a_off1);
 #pragma unroll
   for (uint32_t k = 0; k < 4; ++k) mma_one<false>(m.elected, m.tmem + d_col, a0 + 2 * k, b_lo + 2 * k, idesc, (accumulate | k) ? 1u : 0u);
@@ -870,33 +835,50 @@ __device__ __forceinline__ void issue_pair(Issuer& m, uint32_t slot, uint32_t a_
   T_SINCE(m.tacc, TM_ISSUE, tw);
   TRACE(m.tr, 420);
 }
-__device__ __forceinline__ void issue_from_A(Issuer& m, uint32_t slot, uint32_t n, uint32_t d_col) {
-  issue_pair(m, slot, OFF_A, OFF_A + CHUNK_BYTES, n, d_col, 0);
+__device__ __forceinline__ void issue_pair(Issuer& m, uint32_t slot, uint32_t a_off0, uint32_t a_off1, uint32_t d_col, uint32_t accumulate) {
+  wait_weights(m, slot);
+  multiply_pair(m, slot, a_off0, a_off1, d_col, accumulate);
 }
-// The down projection of a chunk: its A operand in tensor memory, K step k in the 8 columns at a_col + 16 k.
-__device__ __forceinline__ void issue_down(Issuer& m, uint32_t a_col) {
-  const uint32_t slot = m.rot.next_single();
-  const uint32_t b_lo = wait_weights(m, slot);
-  T_MARK(tw);
-  const uint32_t idesc = instr_desc(128);
-#pragma unroll
-  for (uint32_t k = 0; k < 4; ++k) mma_one<true>(m.elected, m.tmem + COL_RESID, m.tmem + a_col + 16 * k, b_lo + 2 * k, idesc, 1u);
-  commit_one(m, B_DONE0 + slot);
-  T_SINCE(m.tacc, TM_ISSUE, tw);
-  TRACE(m.tr, 430);
+__device__ __forceinline__ void issue_from_A(Issuer& m, uint32_t slot, uint32_t d_col) {
+  issue_pair(m, slot, OFF_A, OFF_A + CHUNK_BYTES, d_col, 0);
 }
 __device__ __forceinline__ void commit_round(const Issuer& m) { commit_one(m, B_ACC); }
 
-__device__ __forceinline__ void issue_ffn(Issuer& m) {
+// gate|up of the eight chunks; slot: pair slot of chunk 0.
+__device__ __forceinline__ void issue_gate_up(Issuer& m, uint32_t slot) {
   wait_operand(m, B_OP0);
-#pragma unroll 1
-  for (uint32_t c = 0; c < 3; ++c) issue_from_A(m, m.rot.next_pair(), 128, COL_ACC0 + 128 * c);
   uint32_t a = 0;
 #pragma unroll 1
   for (uint32_t c = 0; c < 8; ++c) {
+    wait_weights(m, slot);
+    if (c >= 3) {   // the down projection of chunk c - 3 has read this accumulator; its slot's next one comes after this product
+      mbar_wait(m.bars + 8 * (B_DONE0 + 3 + a), (m.down_par >> a) & 1u, m.status, m.aborted, ST_TIMEOUT_ACC);
+      m.down_par ^= 1u << a;
+      tc_fence_after();
+      TRACE(m.tr, 404);
+    }
+    multiply_pair(m, slot, OFF_A, OFF_A + CHUNK_BYTES, COL_ACC0 + 128 * a, 0);
+    slot = slot == 2 ? 0 : slot + 1;
+    a = a == 2 ? 0 : a + 1;
+  }
+  m.down_par ^= 7;   // those of chunks 5, 6, 7 are not waited for here
+}
+// The down projections of the eight chunks: A operand in tensor memory, K step k in the 8 columns at 16 k of the accumulator.
+__device__ __forceinline__ void issue_downs(Issuer& m) {
+  constexpr uint32_t idesc = instr_desc(128);
+  uint32_t a = 0;
+#pragma unroll 1
+  for (uint32_t c = 0; c < 8; ++c) {
+    wait_weights(m, 3 + a);
     wait_operand(m, B_FFN0 + a);   // product of chunk c written, accumulator a = c % 3 read
-    issue_down(m, COL_ACC0 + 128 * a);
-    if (c + 3 < 8) issue_from_A(m, m.rot.next_pair(), 128, COL_ACC0 + 128 * a);
+    T_MARK(tw);
+    const uint32_t b_lo = uniform(desc_lo(m.sbase + single_offset(a)));
+    const uint32_t a_col = m.tmem + COL_ACC0 + 128 * a;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) mma_one<true>(m.elected, m.tmem + COL_RESID, a_col + 16 * k, b_lo + 2 * k, idesc, 1u);
+    commit_one(m, B_DONE0 + 3 + a);
+    T_SINCE(m.tacc, TM_ISSUE, tw);
+    TRACE(m.tr, 430);
     a = a == 2 ? 0 : a + 1;
   }
   commit_round(m);
@@ -904,31 +886,28 @@ __device__ __forceinline__ void issue_ffn(Issuer& m) {
 __device__ __forceinline__ void issue_qkv(Issuer& m) {
   wait_operand(m, B_OP0);
 #pragma unroll 1
-  for (uint32_t h = 0; h < HEADS; ++h) {
-    issue_from_A(m, qkv_slot(h), 96, COL_ACC0 + 96 * h);
-    commit_one(m, B_QKV0 + h);
-  }
-  after_qkv(m.rot);
+  for (uint32_t i = 0; i < 3; ++i) issue_from_A(m, i, COL_ACC0 + 128 * i);
+  commit_round(m);
 }
 __device__ __forceinline__ void issue_out_proj(Issuer& m, uint32_t a_off) {
   wait_operand(m, B_OP0);   // attention output: K atom 0 = heads 0, 1; K atom 1 = heads 2, 3
-  issue_pair(m, m.rot.next_pair(), a_off, a_off + CHUNK_BYTES, 128, COL_RESID, 1);
+  issue_pair(m, 0, a_off, a_off + CHUNK_BYTES, COL_RESID, 1);
   commit_round(m);
 }
 __device__ __forceinline__ void issue_temporal(Issuer& m, bool has_fields) {
   wait_operand(m, B_OP0);
-  issue_from_A(m, m.rot.next_pair(), 128, COL_ACC0);   // linear2
+  issue_from_A(m, 0, COL_ACC0);   // linear2
   commit_one(m, B_EARLY);
-  issue_from_A(m, m.rot.next_pair(), 128, COL_ACC1);   // linear1
+  issue_from_A(m, 1, COL_ACC1);   // linear1
   commit_round(m);
   wait_operand(m, B_OP0);
-  issue_from_A(m, m.rot.next_pair(), 128, COL_ACC0);   // gates of hidden columns [0,64)
+  issue_from_A(m, 2, COL_ACC0);   // gates of hidden columns [0,64)
   commit_one(m, B_EARLY);
-  issue_from_A(m, m.rot.next_pair(), 128, COL_ACC1);   // gates of hidden columns [64,128)
-  if (has_fields) issue_from_A(m, m.rot.next_pair(), 128, COL_ACC2);   // field_sub
+  issue_from_A(m, 0, COL_ACC1);   // gates of hidden columns [64,128)
+  if (has_fields) issue_from_A(m, 1, COL_ACC2);   // field_sub
   commit_round(m);
   wait_operand(m, B_OP0);
-  issue_pair(m, m.rot.next_pair(), OFF_P, OFF_A + CHUNK_BYTES, 128, COL_RESID, 1);   // linear_out: K atom 0 from P0, K atom 1 in place in A
+  issue_pair(m, 2, OFF_P, OFF_A + CHUNK_BYTES, COL_RESID, 1);   // linear_out: K atom 0 from P0, K atom 1 in place in A
   commit_round(m);
 }
 
@@ -944,10 +923,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
   __shared__ int s_items;
   __shared__ SubLayer s_sub[MAX_SUBLAYERS];  // kernel parameters are slow to index dynamically
   __shared__ uint4 s_sched[MAX_SCHED];
-  __shared__ int s_sched_len;
   const int tid = threadIdx.x, warp = tid >> 5;
   if (tid < args.n_sub) s_sub[tid] = args.sub[tid];
-  if (tid == 32) s_sched_len = build_schedule(args.sub, args.n_sub, args.has_fields != 0, s_sched);
+  int sched_len = 0;
+  for (int si = 0; si < args.n_sub; ++si) {
+    const int ops = sublayer_ops(args.sub[si].type, args.has_fields != 0), op = tid - sched_len;
+    if (op >= 0 && op < ops) s_sched[tid] = sched_entry(args.sub[si], op, args.has_fields != 0);
+    sched_len += ops;
+  }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 8 * B_COUNT);
   if (tid == 0) {
@@ -957,6 +940,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     mbar_init(smem_u32(&bars[B_OP0]), EPI_WARPS);
     for (int i = B_FFN0; i <= B_FFN2; ++i) mbar_init(smem_u32(&bars[i]), EPI_WARPS / 2);
     mbar_init(smem_u32(&bars[B_KVREL]), EPI_WARPS);
+    mbar_init(smem_u32(&bars[B_DRAIN]), 2);   // both issuing warps
     for (int i = B_ACC; i < B_COUNT; ++i) mbar_init(smem_u32(&bars[i]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -979,7 +963,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       const bool elected = elect_one() != 0;
       uint32_t free_par = (1u << N_SLOTS) - 1u;   // a fresh barrier passes a wait on parity 1: every slot starts free
       uint32_t kv_par = 0;
-      const int len = s_sched_len;
+      const int len = sched_len;
       const int skip_op = blockIdx.x == 0 ? args.skip_op : -1;
 #ifdef BNB_TIMING
       long long tacc[T_COUNT];
@@ -1025,7 +1009,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       if ((tid & 31) == 0) T_STORE(args, tacc, TL_FREE_WAIT, T_COUNT);
 #endif
     }
-  } else if (warp == MMA_WARP) {
+  } else if (warp == MMA_WARP || warp == DOWN_WARP) {
     // ---------------------------------------------------------------- tensor-core issue
     {
       Issuer m;
@@ -1035,21 +1019,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       m.elected = elect_one();
       m.full_par = 0;
       m.op_par = 0;
-      m.rot = SlotRotation{0, 3};
+      m.down_par = 0;
       m.status = args.status;
       m.aborted = s_aborted;
 #ifdef BNB_TRACE
-      trace_init(m.tr, args.status, 1);
+      trace_init(m.tr, args.status, warp == MMA_WARP ? 1 : 3);
       if ((tid & 31) != 0) m.tr.n = 1500;
 #endif
 #ifdef BNB_TIMING
       for (int i = 0; i < T_COUNT; ++i) m.tacc[i] = 0;
 #endif
       T_MARK(t_start);
+      const bool down = warp == DOWN_WARP;
       for (int pass = 0; pass < passes; ++pass) {
-        m.rot = SlotRotation{0, 3};   // every pass walks the schedule from its start
         for (int si = 0; si < args.n_sub; ++si) {
           const int type = (int)uniform((uint32_t)s_sub[si].type);
+          if (down) {
+            if (WHOLE || type != SUB_SPATIAL_PRE) issue_downs(m);
+            continue;
+          }
           if (type == SUB_TEMPORAL) {
             issue_temporal(m, args.has_fields != 0);
           } else {
@@ -1057,7 +1045,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
             if (!WHOLE && type == SUB_SPATIAL_PRE) continue;
             issue_out_proj(m, !WHOLE && type == SUB_SPATIAL_POST ? OFF_A : OFF_P);
           }
-          issue_ffn(m);
+          issue_gate_up(m, type == SUB_TEMPORAL ? TEMPORAL_FFN_PAIR : SPATIAL_FFN_PAIR);
         }
       }
       // Nothing issued here may outlive the CTA: its tensor memory is freed and its barriers go
@@ -1068,7 +1056,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       }
 #ifdef BNB_TIMING
       m.tacc[TM_TOTAL] = clock64() - t_start;
-      if ((tid & 31) == 0) T_STORE(args, m.tacc, TM_FULL_WAIT, TL_FREE_WAIT);
+      if (!down && (tid & 31) == 0) T_STORE(args, m.tacc, TM_FULL_WAIT, TL_FREE_WAIT);
 #endif
     }
   } else {
@@ -1082,7 +1070,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     e.wide = args.wide != 0;
     e.lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
     e.par = 0;
-    e.rot = SlotRotation{0, 3};
     e.status = args.status;
     e.aborted = s_aborted;
     e.ss_part = reinterpret_cast<float*>(smem + OFF_SS);
@@ -1212,7 +1199,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
         epi_sync();
         T_SINCE(e.tacc, TE_IO, t_io);
         const int n_items = s_items;
-        e.rot = SlotRotation{0, 3};
         for (int si = 0; si < args.n_sub; ++si) {
           const SubLayer& s = s_sub[si];
           // Ask L2 for the recurrent state of the temporal sublayer that follows this one: the

@@ -17,7 +17,7 @@ constexpr int HEADS = 4;
 constexpr int DH = 32;
 constexpr int TILE = 128;
 constexpr int CHUNK_BYTES = 16384;       // one weight chunk: up to 128 rows x 64 bf16
-constexpr int N_SPATIAL_CHUNKS = 34;       // chunks of a spatial sublayer proper
+constexpr int N_SPATIAL_CHUNKS = 32;       // chunks of a spatial sublayer proper
 constexpr int N_BULLET_CHUNKS = 4;         // kv_bullet: keys (2 K atoms), values (2 K atoms); zero when absent
 constexpr int N_SPATIAL_IMAGE = N_SPATIAL_CHUNKS + N_BULLET_CHUNKS;
 constexpr int N_TEMPORAL_CHUNKS = 36;
@@ -128,7 +128,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 // Instruction descriptor: fp32 accumulator, bf16 A and B, both K-major, M = 128, N = n.
-__device__ __forceinline__ uint32_t instr_desc(uint32_t n) {
+__host__ __device__ constexpr uint32_t instr_desc(uint32_t n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 

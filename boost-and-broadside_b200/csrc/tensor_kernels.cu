@@ -40,22 +40,16 @@ __device__ __forceinline__ const float* ffn_chunk_row(int c, int r, const float*
   return down + (size_t)r * 4 * D + 64 * cc;
 }
 __device__ __forceinline__ const float* spatial_chunk_row(const BnbSpatialWeights& w, int c, int r) {
-  if (c < 10) {
-    int p = c / 5, i = c % 5;
-    if (i < 4) {
-      int h = 2 * p + i / 2, kh = i % 2;
-      if (r >= 96) return nullptr;
-      return w.qkv_w + (size_t)((r / 32) * D + h * DH + (r % 32)) * D + kh * 64;
-    }
-    return w.out_w + (size_t)r * D + 64 * p;
-  }
+  // two K halves each of q, k, v (all heads) and out_proj
+  if (c < 6) return w.qkv_w + (size_t)((c >> 1) * D + r) * D + (c & 1) * 64;
+  if (c < 8) return w.out_w + (size_t)r * D + (c & 1) * 64;
   if (c >= N_SPATIAL_CHUNKS) {
     // kv_bullet (2D, D): rows 0..127 are the keys of all heads, 128..255 the values
     if (!w.kv_bullet_w) return nullptr;
     const int i = c - N_SPATIAL_CHUNKS;
     return w.kv_bullet_w + (size_t)((i >> 1) * D + r) * D + (i & 1) * 64;
   }
-  return ffn_chunk_row(c - 10, r, w.gate_w, w.up_w, w.down_w);
+  return ffn_chunk_row(c - 8, r, w.gate_w, w.up_w, w.down_w);
 }
 __device__ __forceinline__ const float* temporal_chunk_row(const BnbTemporalWeights& w, int c, int r) {
   int kh = c & 1;
@@ -74,9 +68,9 @@ __device__ __forceinline__ const float* temporal_chunk_row(const BnbTemporalWeig
 // input is a normed activation, else nullptr.  The kernels then feed x * rsqrt(mean x^2 + eps)
 // without the gain, and the products see W[n][k] * g[k] rounded to bf16 once.
 __device__ __forceinline__ const float* spatial_chunk_gain(const BnbSpatialWeights& w, int c) {
-  if (c < 10) { const int i = c % 5; return i < 4 ? w.norm1_w + (i % 2) * 64 : nullptr; }
+  if (c < 8) return c < 6 ? w.norm1_w + (c & 1) * 64 : nullptr;
   if (c >= N_SPATIAL_CHUNKS) return w.norm_bullet_w ? w.norm_bullet_w + ((c - N_SPATIAL_CHUNKS) & 1) * 64 : nullptr;
-  const int i = (c - 10) % 3;
+  const int i = (c - 8) % 3;
   return i < 2 ? w.norm2_w + i * 64 : nullptr;
 }
 __device__ __forceinline__ const float* temporal_chunk_gain(const BnbTemporalWeights& w, int c) {
