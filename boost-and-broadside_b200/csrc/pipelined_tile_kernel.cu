@@ -176,6 +176,18 @@ __device__ __forceinline__ uint32_t pair_offset(uint32_t slot) { return slot == 
 __device__ __forceinline__ uint32_t single_offset(uint32_t i) { return i == 0 ? OFF_RING + 4 * CHUNK_BYTES : OFF_KV + (1 + i) * CHUNK_BYTES; }
 __device__ __forceinline__ uint32_t slot_offset(uint32_t slot) { return slot < 3 ? pair_offset(slot) : single_offset(slot - 3); }
 
+// Bounded wait of this kernel: as mbar_wait, but a wait that runs out only leaves its code in the CTA's abort word, which the
+// last thread out reports; two dozen waits are inlined here, and the kernel's code is what its warps stall on
+// in every phase they meet for the first time.  aborted[0]: 0, or the first code (-1: the call had failed before).
+__device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity, volatile int* aborted, int code) {
+  if (mbar_try_wait(bar, parity)) return;
+  const int limit = aborted[0] ? 4 : code == ST_TIMEOUT_FULL ? aborted[1] : 2 * aborted[1];
+#pragma unroll 1
+  for (int i = 0; i < limit; ++i)
+    if (mbar_try_wait(bar, parity)) return;
+  if (aborted[0] == 0) aborted[0] = code;
+}
+
 // ------------------------------------------------------------------ epilogue side
 
 struct Epi {
@@ -193,7 +205,6 @@ struct Epi {
   uint32_t par;         // phase bits of the pair slots' DONE barriers (0..2), of ACC (8) and of EARLY (10)
   int row, part;
   bool wide;            // 32-byte accesses: every row pointer is aligned for them
-  int* status;
   volatile int* aborted;
   float* ss_part;
 };
@@ -213,7 +224,7 @@ __device__ __forceinline__ void post(Epi& e, int bar) {
 // wait_acc: every MMA issued so far is complete (a commit on ACC ends every round).
 __device__ __forceinline__ void wait_acc(Epi& e) {
   T_BEGIN();
-  mbar_wait(e.bars + 8 * B_ACC, (e.par >> 8) & 1u, e.status, e.aborted, ST_TIMEOUT_ACC);
+  wait_bar(e.bars + 8 * B_ACC, (e.par >> 8) & 1u, e.aborted, ST_TIMEOUT_ACC);
   e.par ^= 1u << 8;
   tc_fence_after();
   T_END(e.tacc, e.wait_slot);
@@ -223,7 +234,7 @@ __device__ __forceinline__ void wait_acc(Epi& e) {
 // Every thread waits for each of its phases before it posts what the next one is issued after.
 __device__ __forceinline__ void wait_early(Epi& e) {
   T_BEGIN();
-  mbar_wait(e.bars + 8 * B_EARLY, (e.par >> 10) & 1u, e.status, e.aborted, ST_TIMEOUT_ACC);
+  wait_bar(e.bars + 8 * B_EARLY, (e.par >> 10) & 1u, e.aborted, ST_TIMEOUT_ACC);
   e.par ^= 1u << 10;
   tc_fence_after();
   T_END(e.tacc, e.wait_slot);
@@ -238,7 +249,7 @@ __device__ __forceinline__ void wait_round(Epi& e, uint32_t flips) {
 // complete (MMAs complete in order), and the slot's next one is issued only after its post.
 __device__ __forceinline__ void wait_op(Epi& e, uint32_t slot) {
   T_BEGIN();
-  mbar_wait(e.bars + 8 * (B_DONE0 + slot), (e.par >> slot) & 1u, e.status, e.aborted, ST_TIMEOUT_ACC);
+  wait_bar(e.bars + 8 * (B_DONE0 + slot), (e.par >> slot) & 1u, e.aborted, ST_TIMEOUT_ACC);
   tc_fence_after();
   T_END(e.tacc, e.wait_slot);
   TRACE(e.tr, 100);
@@ -266,6 +277,13 @@ __device__ __forceinline__ void store8(float* p, const float (&v)[8], bool wide)
     reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
     reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
   }
+}
+
+__device__ __forceinline__ void load4(float4& v, const float* p) {
+  asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+}
+__device__ __forceinline__ void store4(float* p, const float4& v) {
+  asm volatile("st.global.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
 }
 
 // residual (TMEM) -> x * rsqrt(mean x^2 + eps) -> bf16 A operand (the RMSNorm gain is in the weights)
@@ -306,42 +324,58 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* s) {
 }
 
 // GatedMLP on the A operand (already normed and posted on OP0): residual += down(gelu(gate) * up).
-// Chunk c: gate = acc[c % 3][0,64), up = acc[c % 3][64,128).  Two groups of eight warps take turns
-// (parts 0, 1 the even chunks, parts 2, 3 the odd ones), so that one group's waits and tensor-memory
+// Chunk c: gate / 2 = acc[c % 3][0,64) (the image holds half the gate weights), up = acc[c % 3][64,128).  Two groups of
+// eight warps take turns (parts 0, 1 the even chunks, parts 2, 3 the odd ones), so that one group's waits and tensor-memory
 // latencies hide behind the other's arithmetic; a thread owns 32 of the 64 hidden columns of its row,
-// columns [32 (part & 1), +32), in two passes of 16.
+// columns [32 (part & 1), +32), in two passes of 16; the second pass's columns are on their way during the first's arithmetic.
 //
 // The gated product stays in tensor memory as the A operand of the down projection: 16 k at a time
 // (8 columns of packed bf16 pairs) over the first half of 16 gate columns the thread has just read;
 // K step s of the MMA reads exactly the columns at 16 s.
+__device__ __forceinline__ void gated_product(const uint32_t (&gv)[16], const uint32_t (&uv)[16], uint32_t dst) {
+  uint32_t w8[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w8[j] = gelu_half_mul(gv[2 * j], gv[2 * j + 1], uv[2 * j], uv[2 * j + 1]);
+  tmem_st8_nowait(dst, w8);
+}
 __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slot of chunk 0
-  const int group = e.part >> 1, half = e.part & 1;
-  T_WAITSLOT(e, TE_FFN_ACC_WAIT);
-#pragma unroll 1
-  for (int c = 0; c < 8; ++c) {
-    if ((c & 1) == group) {
-      wait_op(e, slot);   // gate|up of chunk c; the slot's previous operation, c - 3, came before c - 2
-      T_BEGIN();
-      const uint32_t acc = e.lane_addr + COL_ACC0 + (c % 3) * 128 + half * 32;
-#pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        uint32_t gv[16], uv[16];
-        tmem_ld16_nowait(acc + 16 * p, gv);
-        tmem_ld16_nowait(acc + 64 + 16 * p, uv);
-        tmem_wait_ld();
-        uint32_t w8[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          w8[j] = gelu_mul_bf16x2(__uint_as_float(gv[2 * j]), __uint_as_float(gv[2 * j + 1]), __uint_as_float(uv[2 * j]), __uint_as_float(uv[2 * j + 1]));
-        tmem_st8_nowait(acc + 16 * p, w8);
-      }
-      tmem_wait_st();
-      T_END(e.tacc, TE_FFN_MATH);
-      post(e, B_FFN0 + c % 3);
-    }
+  const uint32_t group = e.part >> 1;
+  uint32_t a = group;   // accumulator of the chunk
+  if (group) {   // past chunk 0
     e.par ^= 1u << slot;
     slot = slot == 2 ? 0 : slot + 1;
   }
+  T_WAITSLOT(e, TE_FFN_ACC_WAIT);
+#pragma unroll 1
+  for (int i = 0; i < 4; ++i) {
+    // gate|up of chunk 2 i + group; the slot's previous operation came before those of the two chunks in between
+    wait_op(e, slot);
+    T_BEGIN();
+    const uint32_t acc = e.lane_addr + COL_ACC0 + a * 128 + (e.part & 1) * 32;
+    uint32_t gv[16], uv[16], gw[16], uw[16];
+    tmem_ld16_nowait(acc, gv);
+    tmem_ld16_nowait(acc + 64, uv);
+    tmem_wait_ld();
+    tmem_ld16_nowait(acc + 16, gw);
+    tmem_ld16_nowait(acc + 80, uw);
+    gated_product(gv, uv, acc);
+    tmem_wait_ld();
+    gated_product(gw, uw, acc + 16);
+    tmem_wait_st();
+    T_END(e.tacc, TE_FFN_MATH);
+    // nothing of this operand is in shared memory: no proxy fence
+    TRACE(e.tr, 201);
+    tc_fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(e.bars + 8 * (B_FFN0 + a));
+    // two operations further: chunks c + 1 and c + 2, whose slots are this one's successors
+    e.par ^= 1u << slot;
+    slot = slot == 2 ? 0 : slot + 1;
+    e.par ^= 1u << slot;
+    slot = slot == 2 ? 0 : slot + 1;
+    a = a == 0 ? 2 : a - 1;   // (a + 2) mod 3
+  }
+  if (group) e.par ^= 1u << (slot == 0 ? 2 : slot - 1);   // there is no chunk 8
   T_WAITSLOT(e, TE_ACC_WAIT);
   wait_acc(e);   // residual complete: every down projection
 }
@@ -349,8 +383,8 @@ __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slo
 // Attention of every head and environment of the tile from the staged q (P area), k and v (KV
 // area), all in the swizzled operand layout (128 rows x 64 bf16 atoms; head h sits in atom h / 2,
 // columns 32 (h % 2) ..).  The four warps of part h serve head h, which they have staged themselves,
-// and take turns at the blocks of 16 query rows; keys are walked in blocks of 16 with a running
-// maximum.  Output: bf16 into the P area as the A operand of out_proj, each block over its own q.
+// and take turns at the blocks of 16 query rows (each head from another warp on: warp & 3 is the scheduler); keys are
+// walked in blocks of 16 with a running maximum.  Output: bf16 into the P area as the A operand of out_proj, each block over its own q.
 __device__ __forceinline__ void attention(Epi& e, int n_items) {
   TRACE(e.tr, 310);
   const uint8_t* meta = e.smem + OFF_META;
@@ -362,7 +396,7 @@ __device__ __forceinline__ void attention(Epi& e, int n_items) {
   const uint32_t sQ = e.sbase + OFF_P + atom, sK = e.sbase + OFF_KV + atom, sV = sK + 2 * CHUNK_BYTES;
   const float* key_bias = reinterpret_cast<const float*>(e.smem + OFF_BIAS);
   const float c2 = 0.17677669529663687f * 1.4426950408889634f;  // log2(e) / sqrt(32): scores in the log2 domain
-  for (int it = warp & 3; it < n_items; it += EPI_WARPS / 4) {
+  for (int it = (warp + h) & 3; it < n_items; it += EPI_WARPS / 4) {
     const int r0 = meta[384 + it];
     const int e0 = meta[r0], n = meta[128 + r0] + 1;   // first tile row and size of the environment
     const int last = e0 + n - 1;
@@ -464,11 +498,11 @@ __device__ __forceinline__ void attention(Epi& e, int n_items) {
 }
 
 // q | k | v of all heads in the three accumulators.
-constexpr uint32_t QKV_FLIPS = 7, OUT_FLIPS = 1;
+constexpr uint32_t QKV_FLIPS = 7, OUT_FLIPS = 1, LINEAR_OUT_FLIPS = 4;
 
+// The sublayers from "normed operand posted" to "last operand of the round that ends in the residual posted"; the norms, the
+// wait for that round and the GatedMLP are the same code for all of them (the kernel's loop).
 __device__ __forceinline__ void run_spatial(Epi& e, int n_items, bool row_valid) {
-  norm_to_A(e);
-  post(e, B_OP0);
   wait_round(e, QKV_FLIPS);
   {
     T_BEGIN();
@@ -498,18 +532,12 @@ __device__ __forceinline__ void run_spatial(Epi& e, int n_items, bool row_valid)
   __syncwarp();
   if ((threadIdx.x & 31) == 0) mbar_arrive(e.bars + 8 * B_KVREL);
   post(e, B_OP0);   // attention output in P
-  wait_round(e, OUT_FLIPS);   // out_proj accumulated into the residual
-  norm_to_A(e);
-  post(e, B_OP0);
-  ffn(e, SPATIAL_FFN_PAIR);
 }
 
 // A spatial sublayer around a separate attention kernel (environments larger than a tile, or a
 // sublayer that reads bullets).  First part: norm1 and q|k|v of every head, written as bf16 to
 // global scratch, (rows, 384) = q | k | v with the heads side by side inside each third.
 __device__ __forceinline__ void run_spatial_pre(Epi& e, const SubLayer& s, size_t grow, bool row_valid) {
-  norm_to_A(e);
-  post(e, B_OP0);
   wait_round(e, QKV_FLIPS);
   const int h = e.part;
   __nv_bfloat16* dst = s.qkv_out + grow * (3 * D) + h * DH;
@@ -544,10 +572,6 @@ __device__ __forceinline__ void run_spatial_post(Epi& e, const SubLayer& s, size
     }
   }
   post(e, B_OP0);
-  wait_round(e, OUT_FLIPS);   // out_proj accumulated into the residual
-  norm_to_A(e);
-  post(e, B_OP0);
-  ffn(e, SPATIAL_FFN_PAIR);
 }
 
 struct RowState {
@@ -561,8 +585,6 @@ struct RowState {
 __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const RowState& rs, bool is_field, bool boundary,
                                              bool has_fields, const float* hid_in) {
   const bool is_ship = rs.hrow >= 0;
-  norm_to_A(e);
-  post(e, B_OP0);
   wait_early(e);      // acc0 = linear2 n
   T_MARK(tt);
   // b2 = bf16(gelu(linear2 n)) for this thread's columns, parked as packed bf16 pairs
@@ -607,53 +629,52 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
     }
     const int* row_hrow = reinterpret_cast<const int*>(e.smem + OFF_ROWINFO);
     const uint8_t* row_flags = e.smem + OFF_ROWINFO + 512;
-    // Four rows at a time: all loads of the group are issued before any store, because the
-    // state may be updated in place and the compiler must otherwise keep loads behind stores.
+    // A warp takes rows warp, warp + 16, ...: four rows' taps are on their way at any time, each row's registers asked
+    // for the row four further on as soon as it is done.  Rows are distinct, so no load needs to wait for another row's
+    // store; volatile accesses keep the compiler to that order (the state may be updated in place).
+    float4 t0[4], t1[4], t2[4];
+    int hr[4], fl[4];
+    const auto request = [&](int k, int r) {
+      hr[k] = row_hrow[r];
+      fl[k] = row_flags[r];
+      t0[k] = t1[k] = t2[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (hr[k] >= 0 && !(fl[k] & 4)) {
+        const float* hi = hid_in + (size_t)hr[k] * 4 * D + col;
+        load4(t0[k], hi + D);
+        load4(t1[k], hi + 2 * D);
+        load4(t2[k], hi + 3 * D);
+      }
+    };
+#pragma unroll
+    for (int k = 0; k < 4; ++k) request(k, warp + EPI_WARPS * k);
 #pragma unroll 1
     for (int r0 = warp; r0 < TILE; r0 += 4 * EPI_WARPS) {
-      float4 t0[4], t1[4], t2[4];
-      uint2 bw[4];
-      int hr[4], lag[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int r = r0 + EPI_WARPS * k;
-        hr[k] = row_hrow[r];
-        const int flags = row_flags[r];
-        lag[k] = flags & 3;
-        t0[k] = t1[k] = t2[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        bw[k] = make_uint2(0u, 0u);
         if (hr[k] >= 0) {
-          if (!(flags & 4)) {
-            const float* hi = hid_in + (size_t)hr[k] * 4 * D + col;
-            t0[k] = *reinterpret_cast<const float4*>(hi + D);
-            t1[k] = *reinterpret_cast<const float4*>(hi + 2 * D);
-            t2[k] = *reinterpret_cast<const float4*>(hi + 3 * D);
+          const int lag = fl[k] & 3;
+          uint2* at = reinterpret_cast<uint2*>(e.smem + OFF_A + (lane >> 4) * CHUNK_BYTES + swz(r, (lane & 15) >> 1) + (lane & 1) * 8);
+          const uint2 bw = *at;
+          float* ho = s.hid_out + (size_t)hr[k] * 4 * D + col;
+          const float b1[4] = {bf16_lo(bw.x), bf16_hi(bw.x), bf16_lo(bw.y), bf16_hi(bw.y)};
+          store4(ho + D, t1[k]);
+          store4(ho + 2 * D, t2[k]);
+          store4(ho + 3 * D, make_float4(b1[0], b1[1], b1[2], b1[3]));
+          const float a0[4] = {t0[k].x, t0[k].y, t0[k].z, t0[k].w}, a1[4] = {t1[k].x, t1[k].y, t1[k].z, t1[k].w},
+                      a2[4] = {t2[k].x, t2[k].y, t2[k].z, t2[k].w};
+          float u[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float p0 = lag >= 3 ? __fmul_rn(a0[i], cw[i][0]) : 0.f;
+            const float p1 = lag >= 2 ? __fmul_rn(a1[i], cw[i][1]) : 0.f;
+            const float p2 = lag >= 1 ? __fmul_rn(a2[i], cw[i][2]) : 0.f;
+            const float p3 = __fmul_rn(b1[i], cw[i][3]);
+            u[i] = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p0, p1), p2), p3), cb[i]);
           }
-          bw[k] = *reinterpret_cast<const uint2*>(e.smem + OFF_A + (lane >> 4) * CHUNK_BYTES + swz(r, (lane & 15) >> 1) + (lane & 1) * 8);
+          *at = make_uint2(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]));
         }
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (hr[k] < 0) continue;
-        const int r = r0 + EPI_WARPS * k;
-        float* ho = s.hid_out + (size_t)hr[k] * 4 * D + col;
-        const float b1[4] = {bf16_lo(bw[k].x), bf16_hi(bw[k].x), bf16_lo(bw[k].y), bf16_hi(bw[k].y)};
-        *reinterpret_cast<float4*>(ho + D) = t1[k];
-        *reinterpret_cast<float4*>(ho + 2 * D) = t2[k];
-        *reinterpret_cast<float4*>(ho + 3 * D) = make_float4(b1[0], b1[1], b1[2], b1[3]);
-        const float a0[4] = {t0[k].x, t0[k].y, t0[k].z, t0[k].w}, a1[4] = {t1[k].x, t1[k].y, t1[k].z, t1[k].w},
-                    a2[4] = {t2[k].x, t2[k].y, t2[k].z, t2[k].w};
-        float u[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float p0 = lag[k] >= 3 ? __fmul_rn(a0[i], cw[i][0]) : 0.f;
-          const float p1 = lag[k] >= 2 ? __fmul_rn(a1[i], cw[i][1]) : 0.f;
-          const float p2 = lag[k] >= 1 ? __fmul_rn(a2[i], cw[i][2]) : 0.f;
-          const float p3 = __fmul_rn(b1[i], cw[i][3]);
-          u[i] = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p0, p1), p2), p3), cb[i]);
-        }
-        *reinterpret_cast<uint2*>(e.smem + OFF_A + (lane >> 4) * CHUNK_BYTES + swz(r, (lane & 15) >> 1) + (lane & 1) * 8) =
-            make_uint2(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]));
+        if (r + 4 * EPI_WARPS < TILE) request(k, r + 4 * EPI_WARPS);
       }
     }
   }
@@ -769,10 +790,6 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
   }
   post(e, B_OP0);   // branch operand
   T_SINCE(e.tacc, TE_TEMPORAL, tu);
-  wait_round(e, 4);   // residual += linear_out(branch); slot 2
-  norm_to_A(e);
-  post(e, B_OP0);
-  ffn(e, TEMPORAL_FFN_PAIR);
 }
 
 // ------------------------------------------------------------------ issuing side (two warps)
@@ -798,13 +815,12 @@ struct Issuer {
   uint32_t full_par;   // per-slot phase bits of the FULL barriers
   uint32_t op_par;     // phase bits of OP0 and FFN0..2
   uint32_t down_par;   // phase bits of the single slots' DONE barriers
-  int* status;
   volatile int* aborted;
 };
 
 __device__ __forceinline__ void wait_operand(Issuer& m, int bar) {
   T_BEGIN();
-  mbar_wait(m.bars + 8 * bar, (m.op_par >> bar) & 1u, m.status, m.aborted, ST_TIMEOUT_OPERAND);
+  wait_bar(m.bars + 8 * bar, (m.op_par >> bar) & 1u, m.aborted, ST_TIMEOUT_OPERAND);
   m.op_par ^= 1u << bar;
   tc_fence_after();
   T_END(m.tacc, TM_OP_WAIT);
@@ -814,7 +830,7 @@ __device__ __forceinline__ void commit_one(const Issuer& m, uint32_t bar) { tc_c
 // Waits for the weights of a slot.
 __device__ __forceinline__ void wait_weights(Issuer& m, uint32_t slot) {
   T_MARK(tw);
-  mbar_wait(m.bars + 8 * (B_FULL0 + slot), (m.full_par >> slot) & 1u, m.status, m.aborted, ST_TIMEOUT_FULL);
+  wait_bar(m.bars + 8 * (B_FULL0 + slot), (m.full_par >> slot) & 1u, m.aborted, ST_TIMEOUT_FULL);
   m.full_par ^= 1u << slot;
   T_SINCE(m.tacc, TM_FULL_WAIT, tw);
   TRACE(m.tr, 410);
@@ -852,7 +868,7 @@ __device__ __forceinline__ void issue_gate_up(Issuer& m, uint32_t slot) {
   for (uint32_t c = 0; c < 8; ++c) {
     wait_weights(m, slot);
     if (c >= 3) {   // the down projection of chunk c - 3 has read this accumulator; its slot's next one comes after this product
-      mbar_wait(m.bars + 8 * (B_DONE0 + 3 + a), (m.down_par >> a) & 1u, m.status, m.aborted, ST_TIMEOUT_ACC);
+      wait_bar(m.bars + 8 * (B_DONE0 + 3 + a), (m.down_par >> a) & 1u, m.aborted, ST_TIMEOUT_ACC);
       m.down_par ^= 1u << a;
       tc_fence_after();
       TRACE(m.tr, 404);
@@ -863,8 +879,53 @@ __device__ __forceinline__ void issue_gate_up(Issuer& m, uint32_t slot) {
   }
   m.down_par ^= 7;   // those of chunks 5, 6, 7 are not waited for here
 }
+// Rows that the tile owners need next are asked into L2 by the warp of the down projections, whose own work is a quarter of its
+// time.  As prefetches of the epilogue threads the state alone held their load pipe for 1 400 cycles of every tile and
+// temporal sublayer; as bulk prefetches they stand in the way of the weight copies (7 000 cycles).
+__device__ __forceinline__ void prefetch_line(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// The recurrent state of 16 tile rows (2 KB each, two lanes a row).
+__device__ __forceinline__ void prefetch_state(const float* hid, const int* row_hrow, int row0) {
+  const int lane = threadIdx.x & 31, hrow = row_hrow[row0 + (lane >> 1)];
+  if (hrow < 0) return;
+  const float* p = hid + (size_t)hrow * 4 * D + (lane & 1) * 2 * D;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) prefetch_line(p + 32 * i);
+}
+// Tokens and masks of a tile at timestep t.
+__device__ __forceinline__ void prefetch_tokens(const TrunkArgs& args, int tile, int t) {
+  const EnvMap& map = args.map;
+  const int lane = threadIdx.x & 31;
+  const int grp = tile / args.env_tiles, eb = tile - grp * args.env_tiles;
+  const size_t group_row = (size_t)(grp + t) * map.total_tokens;
+  const size_t row_bytes = args.io_bf16 ? D * 2 : D * 4;
+  const uint8_t* x = reinterpret_cast<const uint8_t*>(args.x) + group_row * row_bytes;
+  const auto range = [&](int first, int n) {
+    const uint8_t* p = x + first * row_bytes;
+    for (int i = lane; i < n * (int)row_bytes / 128; i += 32) prefetch_line(p + 128 * i);
+    if (args.alive && lane < 2 && n > 0) prefetch_line(args.alive + group_row + first + (lane ? n - 1 : 0));
+  };
+  if (args.tile_env_begin) {
+    const int end = args.tile_env_begin[eb + 1];
+    for (int k0 = args.tile_env_begin[eb]; k0 < end; k0 += 32) {
+      int first = 0, n = 0;
+      if (k0 + lane < end) {
+        const int env = args.tile_env_ids[k0 + lane];
+        first = map.tok_off[env];
+        n = map.tok_off[env + 1] - first;
+      }
+      for (int j = 0; j < min(32, end - k0); ++j) range(__shfl_sync(0xffffffffu, first, j), __shfl_sync(0xffffffffu, n, j));
+    }
+  } else if (args.flat_rows) {
+    range(eb * TILE, min(TILE, map.total_tokens - eb * TILE));
+  } else {
+    const int env0 = eb * args.envs_per_tile;
+    range(env0 * map.tokens_per_env, min(args.envs_per_tile, map.n_envs - env0) * map.tokens_per_env);
+  }
+}
+
 // The down projections of the eight chunks: A operand in tensor memory, K step k in the 8 columns at 16 k of the accumulator.
-__device__ __forceinline__ void issue_downs(Issuer& m) {
+// next_hid: the state that the following sublayer reads (null: none, or it is at hand), asked for on the way.
+__device__ __forceinline__ void issue_downs(Issuer& m, const float* next_hid, const int* row_hrow) {
   constexpr uint32_t idesc = instr_desc(128);
   uint32_t a = 0;
 #pragma unroll 1
@@ -879,6 +940,8 @@ __device__ __forceinline__ void issue_downs(Issuer& m) {
     commit_one(m, B_DONE0 + 3 + a);
     T_SINCE(m.tacc, TM_ISSUE, tw);
     TRACE(m.tr, 430);
+    if (next_hid) prefetch_state(next_hid, row_hrow, 16 * (int)c);
+    __syncwarp();
     a = a == 2 ? 0 : a + 1;
   }
   commit_round(m);
@@ -919,7 +982,7 @@ template <bool WHOLE>
 __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_constant__ TrunkArgs args) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) int s_aborted[4];   // [2..3]: address of the host's status word
+  __shared__ int s_aborted[2];
   __shared__ int s_items;
   __shared__ SubLayer s_sub[MAX_SUBLAYERS];  // kernel parameters are slow to index dynamically
   __shared__ uint4 s_sched[MAX_SCHED];
@@ -934,8 +997,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 8 * B_COUNT);
   if (tid == 0) {
-    s_aborted[0] = (*args.status != 0) ? 1 : 0;
-    *reinterpret_cast<int**>(&s_aborted[2]) = args.host_status;
+    s_aborted[0] = (*args.status != 0) ? -1 : 0;
     s_aborted[1] = args.poll_limit > 0 ? args.poll_limit : DEFAULT_POLL_LIMIT;
     mbar_init(smem_u32(&bars[B_OP0]), EPI_WARPS);
     for (int i = B_FFN0; i <= B_FFN2; ++i) mbar_init(smem_u32(&bars[i]), EPI_WARPS / 2);
@@ -982,11 +1044,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
           const uint32_t slot = uniform(en.w & 7u);
           T_MARK(tw);
           if (en.w & 8u) {
-            mbar_wait(bar0 + 8 * B_KVREL, kv_par, args.status, s_aborted, ST_TIMEOUT_FREE);
+            wait_bar(bar0 + 8 * B_KVREL, kv_par, s_aborted, ST_TIMEOUT_FREE);
             kv_par ^= 1u;
           }
           T_SINCE(tacc, TL_KV_WAIT, tw);
-          mbar_wait(bar0 + 8 * (B_DONE0 + slot), (free_par >> slot) & 1u, args.status, s_aborted, ST_TIMEOUT_FREE);
+          wait_bar(bar0 + 8 * (B_DONE0 + slot), (free_par >> slot) & 1u, s_aborted, ST_TIMEOUT_FREE);
           free_par ^= 1u << slot;
           // Once a wait of this CTA has run out nothing is in step any more: stop fetching.  Arming a
           // FULL barrier again before its previous copy has landed would arrive on it twice in one
@@ -1020,7 +1082,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       m.full_par = 0;
       m.op_par = 0;
       m.down_par = 0;
-      m.status = args.status;
       m.aborted = s_aborted;
 #ifdef BNB_TRACE
       trace_init(m.tr, args.status, warp == MMA_WARP ? 1 : 3);
@@ -1031,11 +1092,21 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
 #endif
       T_MARK(t_start);
       const bool down = warp == DOWN_WARP;
+      int tile = blockIdx.x, t = 0;
       for (int pass = 0; pass < passes; ++pass) {
+        const int this_t = t;
+        if (++t == args.t_loop) {
+          t = 0;
+          tile += gridDim.x;
+        }
         for (int si = 0; si < args.n_sub; ++si) {
           const int type = (int)uniform((uint32_t)s_sub[si].type);
           if (down) {
-            if (WHOLE || type != SUB_SPATIAL_PRE) issue_downs(m);
+            if (si + 1 == args.n_sub && pass + 1 < passes) prefetch_tokens(args, tile, t);
+            __syncwarp();
+            const bool state_next = this_t == 0 && type != SUB_TEMPORAL && si + 1 < args.n_sub && s_sub[si + 1].type == SUB_TEMPORAL;
+            if (WHOLE || type != SUB_SPATIAL_PRE)
+              issue_downs(m, state_next ? s_sub[si + 1].hid_in : nullptr, reinterpret_cast<const int*>(smem + OFF_ROWINFO));
             continue;
           }
           if (type == SUB_TEMPORAL) {
@@ -1070,7 +1141,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     e.wide = args.wide != 0;
     e.lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
     e.par = 0;
-    e.status = args.status;
     e.aborted = s_aborted;
     e.ss_part = reinterpret_cast<float*>(smem + OFF_SS);
 #ifdef BNB_TRACE
@@ -1201,18 +1271,27 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
         const int n_items = s_items;
         for (int si = 0; si < args.n_sub; ++si) {
           const SubLayer& s = s_sub[si];
-          // Ask L2 for the recurrent state of the temporal sublayer that follows this one: the
-          // rows are needed one sublayer from now.
-          if (is_ship && t == 0 && si + 1 < args.n_sub && s_sub[si + 1].type == SUB_TEMPORAL && s.type != SUB_TEMPORAL) {
-            const char* base = reinterpret_cast<const char*>(s_sub[si + 1].hid_in + (size_t)rs.hrow * 4 * D) + e.part * 512;
-#pragma unroll
-            for (int l = 0; l < 4; ++l) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + l * 128));
+          const int type = s.type;
+          const bool temporal = type == SUB_TEMPORAL;
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
+            if (WHOLE || half || type != SUB_SPATIAL_POST) {
+              norm_to_A(e);
+              post(e, B_OP0);
+            }
+            if (half) {
+              ffn(e, temporal ? TEMPORAL_FFN_PAIR : SPATIAL_FFN_PAIR);
+              break;
+            }
+            if (temporal) run_temporal(e, s, rs, is_field, boundary, args.has_fields != 0, t == 0 ? s.hid_in : s.hid_out);
+            else if (WHOLE || type == SUB_SPATIAL) run_spatial(e, n_items, valid);
+            else if (type == SUB_SPATIAL_POST) run_spatial_post(e, s, trow, valid);
+            else {
+              run_spatial_pre(e, s, trow, valid);
+              break;
+            }
+            wait_round(e, temporal ? LINEAR_OUT_FLIPS : OUT_FLIPS);   // out_proj or linear_out accumulated into the residual
           }
-          if (s.type == SUB_SPATIAL) run_spatial(e, n_items, valid);
-          else if (WHOLE) run_temporal(e, s, rs, is_field, boundary, args.has_fields != 0, t == 0 ? s.hid_in : s.hid_out);
-          else if (s.type == SUB_SPATIAL_PRE) run_spatial_pre(e, s, trow, valid);
-          else if (s.type == SUB_SPATIAL_POST) run_spatial_post(e, s, trow, valid);
-          else run_temporal(e, s, rs, is_field, boundary, args.has_fields != 0, t == 0 ? s.hid_in : s.hid_out);
         }
         // y <- residual
         T_RESET(t_io);
@@ -1252,6 +1331,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     // a wait ran out: copies may still be in flight towards this CTA's shared memory; give them
     // time to land before the CTA gives it up
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    // the first code of the call is the one reported
+    if ((tid & 31) == 0 && s_aborted[0] > 0 && atomicCAS(args.status, 0, s_aborted[0]) == 0 && args.host_status)
+      *static_cast<volatile int*>(args.host_status) = s_aborted[0];
   }
   __syncthreads();
   if (warp == 0) {

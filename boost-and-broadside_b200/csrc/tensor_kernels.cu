@@ -80,8 +80,11 @@ __device__ __forceinline__ const float* temporal_chunk_gain(const BnbTemporalWei
   return i < 2 ? w.norm2_w + i * 64 : nullptr;
 }
 
-template <class W, class F, class G>
-__device__ __forceinline__ void pack_image(const W& w, int n_chunks, uint8_t* out, F row_of, G gain_of) {
+// Rows of gate weights are stored halved (the GatedMLP's elementwise part works on gate / 2: gelu_half_mul).
+__device__ __forceinline__ bool ffn_gate_row(int c, int r) { return c % 3 < 2 && r < 64; }
+
+template <class W, class F, class G, class H>
+__device__ __forceinline__ void pack_image(const W& w, int n_chunks, uint8_t* out, F row_of, G gain_of, H halved) {
   // one thread per 16-byte group: (chunk, row, group of 8 columns)
   const int total = n_chunks * TILE * 8;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -96,14 +99,20 @@ __device__ __forceinline__ void pack_image(const W& w, int n_chunks, uint8_t* ou
         a.x *= ga.x; a.y *= ga.y; a.z *= ga.z; a.w *= ga.w;
         b.x *= gb.x; b.y *= gb.y; b.z *= gb.z; b.w *= gb.w;
       }
+      if (halved(c, r)) {
+        a.x *= 0.5f; a.y *= 0.5f; a.z *= 0.5f; a.w *= 0.5f;
+        b.x *= 0.5f; b.y *= 0.5f; b.z *= 0.5f; b.w *= 0.5f;
+      }
       v = make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
     }
     *reinterpret_cast<uint4*>(out + (size_t)c * CHUNK_BYTES + swz(r, g)) = v;
   }
 }
+__device__ __forceinline__ bool spatial_chunk_halved(int c, int r) { return c >= 8 && c < N_SPATIAL_CHUNKS && ffn_gate_row(c - 8, r); }
+__device__ __forceinline__ bool temporal_chunk_halved(int c, int r) { return c >= 12 && ffn_gate_row(c - 12, r); }
 __global__ void k_pack_spatial(BnbSpatialWeights w, uint8_t* out) {
   pack_image(w, N_SPATIAL_IMAGE, out, [](const BnbSpatialWeights& ww, int c, int r) { return spatial_chunk_row(ww, c, r); },
-             [](const BnbSpatialWeights& ww, int c) { return spatial_chunk_gain(ww, c); });
+             [](const BnbSpatialWeights& ww, int c) { return spatial_chunk_gain(ww, c); }, [](int c, int r) { return spatial_chunk_halved(c, r); });
 }
 __global__ void k_pack_temporal(BnbTemporalWeights w, uint8_t* out) {
   if (blockIdx.x == 0 && threadIdx.x < D) {
@@ -111,7 +120,7 @@ __global__ void k_pack_temporal(BnbTemporalWeights w, uint8_t* out) {
     reinterpret_cast<float*>(out + (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES)[threadIdx.x] = kRglruC * (sg == 0.f ? kLogOfZero : log2f(sg));
   }
   pack_image(w, N_TEMPORAL_CHUNKS, out, [](const BnbTemporalWeights& ww, int c, int r) { return temporal_chunk_row(ww, c, r); },
-             [](const BnbTemporalWeights& ww, int c) { return temporal_chunk_gain(ww, c); });
+             [](const BnbTemporalWeights& ww, int c) { return temporal_chunk_gain(ww, c); }, [](int c, int r) { return temporal_chunk_halved(c, r); });
 }
 
 // Every image of a trunk in one launch: blockIdx.y selects the sublayer.
@@ -129,7 +138,7 @@ __global__ void k_pack_trunk(const __grid_constant__ PackJobs jobs) {
     const BnbSpatialWeights& w = jobs.sw[j];
     pack_image(w, N_SPATIAL_IMAGE, static_cast<uint8_t*>(const_cast<void*>(w.packed)),
                [](const BnbSpatialWeights& ww, int c, int r) { return spatial_chunk_row(ww, c, r); },
-               [](const BnbSpatialWeights& ww, int c) { return spatial_chunk_gain(ww, c); });
+               [](const BnbSpatialWeights& ww, int c) { return spatial_chunk_gain(ww, c); }, [](int c, int r) { return spatial_chunk_halved(c, r); });
   } else {
     const BnbTemporalWeights& w = jobs.tw[j - jobs.n_spatial];
     uint8_t* out = static_cast<uint8_t*>(const_cast<void*>(w.packed));
@@ -138,7 +147,7 @@ __global__ void k_pack_trunk(const __grid_constant__ PackJobs jobs) {
       reinterpret_cast<float*>(out + (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES)[threadIdx.x] = kRglruC * (sg == 0.f ? kLogOfZero : log2f(sg));
     }
     pack_image(w, N_TEMPORAL_CHUNKS, out, [](const BnbTemporalWeights& ww, int c, int r) { return temporal_chunk_row(ww, c, r); },
-               [](const BnbTemporalWeights& ww, int c) { return temporal_chunk_gain(ww, c); });
+               [](const BnbTemporalWeights& ww, int c) { return temporal_chunk_gain(ww, c); }, [](int c, int r) { return temporal_chunk_halved(c, r); });
   }
 }
 
