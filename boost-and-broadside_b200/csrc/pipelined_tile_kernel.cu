@@ -70,9 +70,10 @@ constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
 // "slot free", the epilogue warps as "accumulator ready" for gate|up of one chunk, whose slot is not
 // used again before they have seen it, and the issuing warp of gate|up as "accumulator free" for a down projection.
 // ACC: every MMA of a round is complete (one more commit per round).
-// EARLY: the first product of a temporal sublayer's two larger rounds is.  DRAIN: every MMA of the
+// EARLY: the first half of a temporal sublayer's gates is.  PARK: linear2's accumulator has been read (epilogue warps ->
+// issuing warp); FIELD: field_sub, multiplied into it then, is complete.  DRAIN: every MMA of the
 // CTA is complete (once per issuing warp, at the end).
-enum : int { B_OP0 = 0, B_FFN0, B_FFN1, B_FFN2, B_KVREL, B_DRAIN, B_ACC, B_EARLY, B_FULL0, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
+enum : int { B_OP0 = 0, B_FFN0, B_FFN1, B_FFN2, B_KVREL, B_PARK, B_DRAIN, B_ACC, B_EARLY, B_FIELD, B_FULL0, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
 static_assert(B_COUNT * 8 + 8 <= 256, "barrier area");
 
 constexpr uint32_t COL_RESID = 0;
@@ -202,7 +203,7 @@ struct Epi {
   uint32_t sbase;       // shared address of smem
   uint32_t bars;        // shared address of the barrier array
   uint32_t lane_addr;   // tensor-memory address of this thread's lane, column 0
-  uint32_t par;         // phase bits of the pair slots' DONE barriers (0..2), of ACC (8) and of EARLY (10)
+  uint32_t par;         // phase bits of the pair slots' DONE barriers (0..2), of ACC (8), EARLY (10) and FIELD (11)
   int row, part;
   bool wide;            // 32-byte accesses: every row pointer is aligned for them
   volatile int* aborted;
@@ -230,15 +231,17 @@ __device__ __forceinline__ void wait_acc(Epi& e) {
   T_END(e.tacc, e.wait_slot);
   TRACE(e.tr, 110);
 }
-// wait_early: the first product of a temporal round, read while the others are multiplied (1 % of a step).
+// The first half of a temporal sublayer's gates, read while the others are multiplied; field_sub.
 // Every thread waits for each of its phases before it posts what the next one is issued after.
-__device__ __forceinline__ void wait_early(Epi& e) {
+__device__ __forceinline__ void wait_other(Epi& e, int bar, uint32_t bit) {
   T_BEGIN();
-  wait_bar(e.bars + 8 * B_EARLY, (e.par >> 10) & 1u, e.aborted, ST_TIMEOUT_ACC);
-  e.par ^= 1u << 10;
+  wait_bar(e.bars + 8 * bar, (e.par >> bit) & 1u, e.aborted, ST_TIMEOUT_ACC);
+  e.par ^= 1u << bit;
   tc_fence_after();
   T_END(e.tacc, e.wait_slot);
 }
+__device__ __forceinline__ void wait_early(Epi& e) { wait_other(e, B_EARLY, 10); }
+__device__ __forceinline__ void wait_field(Epi& e) { wait_other(e, B_FIELD, 11); }
 // wait_round: a round whose pair operations took an odd number of turns on the slots of `flips`, then a commit on ACC.
 __device__ __forceinline__ void wait_round(Epi& e, uint32_t flips) {
   wait_acc(e);
@@ -318,6 +321,7 @@ __device__ __forceinline__ void norm_to_A(Epi& e) {
   T_END(e.tacc, TE_NORM);
 }
 
+__device__ __forceinline__ F2 acc_pair(const uint32_t* v) { return f2(__uint_as_float(v[0]), __uint_as_float(v[1])); }
 __device__ __forceinline__ uint4 pack8(const uint32_t* s) {
   return make_uint4(pack_bf16(__uint_as_float(s[0]), __uint_as_float(s[1])), pack_bf16(__uint_as_float(s[2]), __uint_as_float(s[3])),
                     pack_bf16(__uint_as_float(s[4]), __uint_as_float(s[5])), pack_bf16(__uint_as_float(s[6]), __uint_as_float(s[7])));
@@ -582,36 +586,9 @@ struct RowState {
 
 // One temporal sublayer on the tile at one timestep.  In the gate epilogue thread (row, part)
 // works on hidden columns [64 rnd + 16 part, +16), and parks b2 for exactly those.
-__device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const RowState& rs, bool is_field, bool boundary,
-                                             bool has_fields, const float* hid_in) {
+__device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const RowState& rs, bool boundary, bool has_fields,
+                                             const float* hid_in) {
   const bool is_ship = rs.hrow >= 0;
-  wait_early(e);      // acc0 = linear2 n
-  T_MARK(tt);
-  // b2 = bf16(gelu(linear2 n)) for this thread's columns, parked as packed bf16 pairs
-  uint32_t b2p[2][8];
-#pragma unroll
-  for (int rnd = 0; rnd < 2; ++rnd) {
-    uint32_t v[16];
-    tmem_ld16_nowait(e.lane_addr + COL_ACC0 + rnd * 64 + e.part * 16, v);
-    tmem_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 8; ++j) b2p[rnd][j] = pack_bf16(gelu_fast(__uint_as_float(v[2 * j])), gelu_fast(__uint_as_float(v[2 * j + 1])));
-  }
-  wait_round(e, 3);   // acc1 = linear1 n; slots 0 and 1
-  // b1 = bf16(linear1 n) into the A operand; ships: causal conv with the stored taps -> u
-  {
-    uint32_t v[32];
-    tmem_ld32(e.lane_addr + COL_ACC1 + e.part * 32, v);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int col = e.part * 32 + q * 8;
-      *reinterpret_cast<uint4*>(e.smem + OFF_A + (col >> 6) * CHUNK_BYTES + swz(e.row, (col & 63) >> 3)) = pack8(&v[q * 8]);
-    }
-  }
-  tc_fence_before();
-  T_SINCE(e.tacc, TE_TEMPORAL, tt);
-  epi_sync();
-  T_SINCE(e.tacc, TE_SYNC, tt);
   const float* hin = is_ship ? hid_in + (size_t)rs.hrow * 4 * D : nullptr;
   float* hout = is_ship ? s.hid_out + (size_t)rs.hrow * 4 * D : nullptr;
   // Causal conv, one warp per ship row and four columns per lane, so that the stored taps are
@@ -620,18 +597,12 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
   {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int col = lane * 4;
-    float cw[4][4], cb[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float4 w4 = __ldg(reinterpret_cast<const float4*>(s.conv_w + (col + i) * 4));
-      cw[i][0] = w4.x; cw[i][1] = w4.y; cw[i][2] = w4.z; cw[i][3] = w4.w;
-      cb[i] = __ldg(s.conv_b + col + i);
-    }
     const int* row_hrow = reinterpret_cast<const int*>(e.smem + OFF_ROWINFO);
     const uint8_t* row_flags = e.smem + OFF_ROWINFO + 512;
-    // A warp takes rows warp, warp + 16, ...: four rows' taps are on their way at any time, each row's registers asked
-    // for the row four further on as soon as it is done.  Rows are distinct, so no load needs to wait for another row's
-    // store; volatile accesses keep the compiler to that order (the state may be updated in place).
+    // A warp takes rows warp, warp + 16, ...: four rows' taps are on their way at any time, the first four before the
+    // products are waited for, and each row's registers ask for the row four further on as soon as it is done.  Rows are
+    // distinct, so no load needs to wait for another row's store; volatile accesses keep the compiler to that
+    // order (the state may be updated in place).
     float4 t0[4], t1[4], t2[4];
     int hr[4], fl[4];
     const auto request = [&](int k, int r) {
@@ -647,6 +618,28 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
     };
 #pragma unroll
     for (int k = 0; k < 4; ++k) request(k, warp + EPI_WARPS * k);
+    wait_round(e, 3);   // acc0 = linear1 n, acc1 = linear2 n / 2; slots 0 and 1
+    // b1 = bf16(linear1 n) into the A operand
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      uint32_t v[16];
+      tmem_ld16_nowait(e.lane_addr + COL_ACC0 + e.part * 32 + p * 16, v);
+      tmem_wait_ld();
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int c8 = e.part * 32 + p * 16 + q * 8;
+        *reinterpret_cast<uint4*>(e.smem + OFF_A + (c8 >> 6) * CHUNK_BYTES + swz(e.row, (c8 & 63) >> 3)) = pack8(&v[q * 8]);
+      }
+    }
+    float cw[4][4], cb[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 w4 = __ldg(reinterpret_cast<const float4*>(s.conv_w + (col + i) * 4));
+      cw[i][0] = w4.x; cw[i][1] = w4.y; cw[i][2] = w4.z; cw[i][3] = w4.w;
+      cb[i] = __ldg(s.conv_b + col + i);
+    }
+    tc_fence_before();
+    epi_sync();
 #pragma unroll 1
     for (int r0 = warp; r0 < TILE; r0 += 4 * EPI_WARPS) {
 #pragma unroll
@@ -679,35 +672,40 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
     }
   }
   post(e, B_OP0);   // A = u (ship rows) / b1 (field rows)
-  T_SINCE(e.tacc, TE_TEMPORAL, tt);
-  // previous state of this thread's columns of the first half, requested before the gates arrive
-  float hprev[2][8];
+  // While the gates are multiplied: the previous state of this thread's columns is asked for ...
+  float hprev[2][2][8];
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
+  for (int i = 0; i < 4; ++i) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) hprev[q][i] = 0.f;
-    if (is_ship && !rs.zero_in) load8(hprev[q], hin + e.part * 16 + q * 8, e.wide);
+    for (int j = 0; j < 8; ++j) hprev[i >> 1][i & 1][j] = 0.f;
+    if (is_ship && !rs.zero_in) load8(hprev[i >> 1][i & 1], hin + (i >> 1) * 64 + e.part * 16 + (i & 1) * 8, e.wide);
   }
-  wait_early(e);   // acc0 / acc1 = [W_a u | W_x u] of hidden columns [0,64) / [64,128)
-  T_MARK(tu);
-  // gates and state update
+  // ... and b2 = bf16(gelu(linear2 n)) parked as packed bf16 pairs
+  uint32_t b2p[2][8];
 #pragma unroll
   for (int rnd = 0; rnd < 2; ++rnd) {
-    if (rnd == 1) wait_round(e, has_fields ? 7 : 5);   // the rest; acc2 = field_sub b1; slots 2, 0 (and 1)
+    uint32_t v[16];
+    tmem_ld16_nowait(e.lane_addr + COL_ACC1 + rnd * 64 + e.part * 16, v);
+    tmem_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) b2p[rnd][j] = pack_bf16(gelu_half(acc_pair(&v[2 * j])));
+  }
+  if (has_fields) {   // acc1 may take field_sub
+    tc_fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(e.bars + 8 * B_PARK);
+  }
+  wait_early(e);   // acc0 / acc2 = halves of [W_a u | W_x u] of hidden columns [0,64) / [64,128)
+  // gates and state update
+  const F2 keep = f2(boundary ? 0.f : 1.f), one = f2(1.f);
+#pragma unroll
+  for (int rnd = 0; rnd < 2; ++rnd) {
+    if (rnd == 1) wait_round(e, has_fields ? 7 : 5);   // slots 2, 0 (and 1 for field_sub)
     uint32_t rv[16], iv[16];
-    const uint32_t acc = e.lane_addr + COL_ACC0 + rnd * 128 + e.part * 16;
+    const uint32_t acc = e.lane_addr + (rnd ? COL_ACC2 : COL_ACC0) + e.part * 16;
     tmem_ld16_nowait(acc, rv);        // executed by every lane of the warp
     tmem_ld16_nowait(acc + 64, iv);
     tmem_wait_ld();
-    float hnext[2][8];
-    if (rnd == 0) {
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) hnext[q][i] = 0.f;
-        if (is_ship && !rs.zero_in) load8(hnext[q], hin + 64 + e.part * 16 + q * 8, e.wide);
-      }
-    }
     if (is_ship) {
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
@@ -720,28 +718,25 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
         float hn[8];
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
-          const int cc = col + hf * 4;
-          const float4 ab = __ldg(reinterpret_cast<const float4*>(s.a_b + cc));
-          const float4 xb = __ldg(reinterpret_cast<const float4*>(s.x_b + cc));
-          const float4 dl = __ldg(reinterpret_cast<const float4*>(s.decay_log2 + cc));
-          const float abv[4] = {ab.x, ab.y, ab.z, ab.w}, xbv[4] = {xb.x, xb.y, xb.z, xb.w}, dlv[4] = {dl.x, dl.y, dl.z, dl.w};
+          const float* table = s.decay_log2 + col + hf * 4;
+          const float4 dl = __ldg(reinterpret_cast<const float4*>(table)), ab = __ldg(reinterpret_cast<const float4*>(table + D)),
+                       xb = __ldg(reinterpret_cast<const float4*>(table + 2 * D));
+          const F2 dlv[2] = {f2(dl.x, dl.y), f2(dl.z, dl.w)}, abv[2] = {f2(ab.x, ab.y), f2(ab.z, ab.w)}, xbv[2] = {f2(xb.x, xb.y), f2(xb.z, xb.w)};
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int k = q * 8 + hf * 4 + i, j = hf * 4 + i;
-            const float rg = round_bf16(sigmoid_fast(__uint_as_float(rv[k]) + abv[i]));
-            const float ig = round_bf16(sigmoid_fast(__uint_as_float(iv[k]) + xbv[i]));
+          for (int i = 0; i < 2; ++i) {
+            const int k = q * 8 + hf * 4 + 2 * i, j = hf * 4 + 2 * i, w = hf * 2 + i;
+            const F2 rg = sigmoid_twice_bf16(add(acc_pair(&rv[k]), abv[i])), ig = sigmoid_twice_bf16(add(acc_pair(&iv[k]), xbv[i]));
             // sigmoid(Lambda)^(8 r) = 2^(r * 8 log2 sigmoid(Lambda)); the table is part of the weight image
-            float a = ex2_fast(rg * dlv[i]);
-            const float gate = sqrt_fast(fmaxf((1.0f - a) * (1.0f + a), kGateFloor));
-            const uint32_t uword = uw[hf * 2 + (i >> 1)];
-            const float uu = (i & 1) ? bf16_hi(uword) : bf16_lo(uword);
-            const float bb = gate * (ig * uu);
-            if (boundary) a = 0.f;
-            hn[j] = fmaf(a, hprev[q][j], bb);
+            const float2 ad = halves(mul(rg, dlv[i]));
+            const F2 a = f2(ex2_fast(ad.x), ex2_fast(ad.y));
+            const float2 rest = halves(mul(fma(a, f2(-1.f), one), add(one, a)));
+            const F2 gate = f2(sqrt_fast(fmaxf(rest.x, kGateFloor)), sqrt_fast(fmaxf(rest.y, kGateFloor)));
+            const F2 next = fma(mul(a, keep), f2(hprev[rnd][q][j], hprev[rnd][q][j + 1]), mul(gate, mul(ig, unpack_bf16(uw[w]))));
+            const float2 n = halves(next);
+            hn[j] = n.x;
+            hn[j + 1] = n.y;
+            ob[w] = pack_bf16(mul(next, unpack_bf16(b2p[rnd][q * 4 + w])));
           }
-          const int bi = q * 4 + hf * 2;
-          ob[hf * 2] = pack_bf16(hn[hf * 4] * bf16_lo(b2p[rnd][bi]), hn[hf * 4 + 1] * bf16_hi(b2p[rnd][bi]));
-          ob[hf * 2 + 1] = pack_bf16(hn[hf * 4 + 2] * bf16_lo(b2p[rnd][bi + 1]), hn[hf * 4 + 3] * bf16_hi(b2p[rnd][bi + 1]));
         }
         store8(hout + col, hn, e.wide);
         // branch operand of linear_out: K atom 0 lives in P0, K atom 1 in place in A
@@ -749,34 +744,23 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
         *reinterpret_cast<uint4*>(dst) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
       }
     }
-    if (rnd == 0) {
-#pragma unroll
-      for (int q = 0; q < 2; ++q)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) hprev[q][i] = hnext[q][i];
-    }
   }
   if (has_fields) {
-    // field rows: branch = bf16(bf16(field_sub b1) * b2)
+    // field rows: branch = bf16(bf16(field_sub b1) * b2); rows outside every environment are zeros throughout
+    wait_field(e);
 #pragma unroll
     for (int rnd = 0; rnd < 2; ++rnd) {
       uint32_t v[16];
-      tmem_ld16_nowait(e.lane_addr + COL_ACC2 + rnd * 64 + e.part * 16, v);        // executed by every lane of the warp
+      tmem_ld16_nowait(e.lane_addr + COL_ACC1 + rnd * 64 + e.part * 16, v);        // executed by every lane of the warp
       tmem_wait_ld();
       if (!is_ship) {
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          uint32_t ob[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int bi = q * 4 + j;
-            const float f0 = is_field ? round_bf16(__uint_as_float(v[q * 8 + 2 * j])) * bf16_lo(b2p[rnd][bi]) : 0.f;
-            const float f1 = is_field ? round_bf16(__uint_as_float(v[q * 8 + 2 * j + 1])) * bf16_hi(b2p[rnd][bi]) : 0.f;
-            ob[j] = pack_bf16(f0, f1);
-          }
+          const uint4 f = pack8(&v[q * 8]);
+          const uint32_t* b2 = &b2p[rnd][q * 4];
           uint8_t* dst = rnd == 0 ? e.smem + OFF_P + swz(e.row, e.part * 2 + q)
                                   : e.smem + OFF_A + CHUNK_BYTES + swz(e.row, e.part * 2 + q);
-          *reinterpret_cast<uint4*>(dst) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
+          *reinterpret_cast<uint4*>(dst) = make_uint4(mul_bf16x2(f.x, b2[0]), mul_bf16x2(f.y, b2[1]), mul_bf16x2(f.z, b2[2]), mul_bf16x2(f.w, b2[3]));
         }
       }
     }
@@ -789,7 +773,6 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
     }
   }
   post(e, B_OP0);   // branch operand
-  T_SINCE(e.tacc, TE_TEMPORAL, tu);
 }
 
 // ------------------------------------------------------------------ issuing side (two warps)
@@ -959,16 +942,19 @@ __device__ __forceinline__ void issue_out_proj(Issuer& m, uint32_t a_off) {
 }
 __device__ __forceinline__ void issue_temporal(Issuer& m, bool has_fields) {
   wait_operand(m, B_OP0);
-  issue_from_A(m, 0, COL_ACC0);   // linear2
-  commit_one(m, B_EARLY);
-  issue_from_A(m, 1, COL_ACC1);   // linear1
+  issue_from_A(m, 0, COL_ACC1);   // linear2
+  issue_from_A(m, 1, COL_ACC0);   // linear1
   commit_round(m);
   wait_operand(m, B_OP0);
   issue_from_A(m, 2, COL_ACC0);   // gates of hidden columns [0,64)
   commit_one(m, B_EARLY);
-  issue_from_A(m, 0, COL_ACC1);   // gates of hidden columns [64,128)
-  if (has_fields) issue_from_A(m, 1, COL_ACC2);   // field_sub
+  issue_from_A(m, 0, COL_ACC2);   // gates of hidden columns [64,128)
   commit_round(m);
+  if (has_fields) {
+    wait_operand(m, B_PARK);
+    issue_from_A(m, 1, COL_ACC1);   // field_sub
+    commit_one(m, B_FIELD);
+  }
   wait_operand(m, B_OP0);
   issue_pair(m, 2, OFF_P, OFF_A + CHUNK_BYTES, COL_RESID, 1);   // linear_out: K atom 0 from P0, K atom 1 in place in A
   commit_round(m);
@@ -1002,6 +988,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     mbar_init(smem_u32(&bars[B_OP0]), EPI_WARPS);
     for (int i = B_FFN0; i <= B_FFN2; ++i) mbar_init(smem_u32(&bars[i]), EPI_WARPS / 2);
     mbar_init(smem_u32(&bars[B_KVREL]), EPI_WARPS);
+    mbar_init(smem_u32(&bars[B_PARK]), EPI_WARPS);
     mbar_init(smem_u32(&bars[B_DRAIN]), 2);   // both issuing warps
     for (int i = B_ACC; i < B_COUNT; ++i) mbar_init(smem_u32(&bars[i]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1211,7 +1198,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       }
       if (!valid) { grow = 0; env = 0; }
       const bool is_ship = valid && tok < env_ships;
-      const bool is_field = valid && !is_ship;
       RowState rs;
       rs.hrow = is_ship ? hrow_if_ship : -1;
       rs.lag_ok = BNB_CONV_KERNEL - 1;
@@ -1283,7 +1269,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
               ffn(e, temporal ? TEMPORAL_FFN_PAIR : SPATIAL_FFN_PAIR);
               break;
             }
-            if (temporal) run_temporal(e, s, rs, is_field, boundary, args.has_fields != 0, t == 0 ? s.hid_in : s.hid_out);
+            if (temporal) run_temporal(e, s, rs, boundary, args.has_fields != 0, t == 0 ? s.hid_in : s.hid_out);
             else if (WHOLE || type == SUB_SPATIAL) run_spatial(e, n_items, valid);
             else if (type == SUB_SPATIAL_POST) run_spatial_post(e, s, trow, valid);
             else {

@@ -34,9 +34,7 @@ struct SubLayer {
   const uint8_t* packed;
   const float* conv_w;
   const float* conv_b;
-  const float* a_b;
-  const float* x_b;
-  const float* decay_log2;   // 8 * log2(sigmoid(log_lambda)), written by the pack kernel
+  const float* decay_log2;   // 8 * log2(sigmoid(log_lambda)), then half of a_b, half of x_b (D floats each), written by the pack kernel
   const float* hid_in;
   float* hid_out;
   __nv_bfloat16* qkv_out;        // PRE: (rows, 384) q|k|v, head-major inside each third
@@ -214,6 +212,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
+// Two floats in one 64-bit register pair: one instruction for two multiply-adds.
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float lo, float hi) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ F2 f2(float both) { return f2(both, both); }
+__device__ __forceinline__ float2 halves(F2 a) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v)); return r; }
+__device__ __forceinline__ F2 mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 add(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
 // MUFU-based elementwise functions for the bf16 path.  Their results are rounded to bf16 (or
 // feed products that are), so approximations a few 1e-4 relative are below the rounding.
 __device__ __forceinline__ float tanh_fast(float v) {
@@ -260,8 +266,28 @@ __device__ __forceinline__ uint32_t gelu_half_mul(uint32_t h0, uint32_t h1, uint
       : "+f"(f.x), "+f"(f.y) : "f"(__uint_as_float(u0)), "f"(__uint_as_float(u1)));
   return pack_bf16(f.x, f.y);
 }
+// gelu_fast(2 h) of two elements.
+__device__ __forceinline__ F2 gelu_half(F2 h) {
+  const float2 y = halves(mul(h, h));
+  const F2 y2 = f2(fminf(y.x, 25.0f), fminf(y.y, 25.0f));
+  const float2 a = halves(mul(h, fma(y2, fma(y2, f2(-32 * 3.51516841e-4f), f2(8 * 3.70056464e-2f)), f2(2 * 7.97507884e-1f))));
+  return fma(h, f2(tanh_fast(a.x), tanh_fast(a.y)), h);
+}
+// sigmoid(2 v) of two elements, each rounded to bfloat16.
+__device__ __forceinline__ F2 sigmoid_twice_bf16(F2 v) {
+  const float2 h = halves(v);
+  const float2 g = halves(fma(f2(tanh_fast(h.x), tanh_fast(h.y)), f2(0.5f), f2(0.5f)));
+  return f2(round_bf16(g.x), round_bf16(g.y));
+}
 __device__ __forceinline__ float sigmoid_fast(float v) { return fmaf(0.5f, tanh_fast(0.5f * v), 0.5f); }
 
+__device__ __forceinline__ F2 unpack_bf16(uint32_t v) { return f2(__uint_as_float(v << 16), __uint_as_float(v & 0xFFFF0000u)); }
+__device__ __forceinline__ uint32_t pack_bf16(F2 a) { const float2 v = halves(a); return pack_bf16(v.x, v.y); }
+// Product of two pairs of bfloat16, rounded once.
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
 

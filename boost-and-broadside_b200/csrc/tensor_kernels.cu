@@ -80,7 +80,7 @@ __device__ __forceinline__ const float* temporal_chunk_gain(const BnbTemporalWei
   return i < 2 ? w.norm2_w + i * 64 : nullptr;
 }
 
-// Rows of gate weights are stored halved (the GatedMLP's elementwise part works on gate / 2: gelu_half_mul).
+// Some rows are stored halved (exactly): the elementwise part of the GatedMLP works on gate / 2 (gelu_half_mul).
 __device__ __forceinline__ bool ffn_gate_row(int c, int r) { return c % 3 < 2 && r < 64; }
 
 template <class W, class F, class G, class H>
@@ -109,16 +109,23 @@ __device__ __forceinline__ void pack_image(const W& w, int n_chunks, uint8_t* ou
   }
 }
 __device__ __forceinline__ bool spatial_chunk_halved(int c, int r) { return c >= 8 && c < N_SPATIAL_CHUNKS && ffn_gate_row(c - 8, r); }
-__device__ __forceinline__ bool temporal_chunk_halved(int c, int r) { return c >= 12 && ffn_gate_row(c - 12, r); }
+// linear2 (GELU) and the recurrence's gates (tanh form of the sigmoid) are wanted halved as well
+__device__ __forceinline__ bool temporal_chunk_halved(int c, int r) { return c < 12 ? c < 2 || (c >= 4 && c < 8) : ffn_gate_row(c - 12, r); }
+// What stands behind the chunks of a temporal image (SubLayer::decay_log2).
+__device__ __forceinline__ void pack_recurrence(const BnbTemporalWeights& w, uint8_t* out) {
+  float* t = reinterpret_cast<float*>(out + (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES);
+  const int i = threadIdx.x;
+  const float sg = 1.0f / (1.0f + expf(-w.log_lambda[i]));
+  t[i] = kRglruC * (sg == 0.f ? kLogOfZero : log2f(sg));
+  t[D + i] = 0.5f * w.a_b[i];
+  t[2 * D + i] = 0.5f * w.x_b[i];
+}
 __global__ void k_pack_spatial(BnbSpatialWeights w, uint8_t* out) {
   pack_image(w, N_SPATIAL_IMAGE, out, [](const BnbSpatialWeights& ww, int c, int r) { return spatial_chunk_row(ww, c, r); },
              [](const BnbSpatialWeights& ww, int c) { return spatial_chunk_gain(ww, c); }, [](int c, int r) { return spatial_chunk_halved(c, r); });
 }
 __global__ void k_pack_temporal(BnbTemporalWeights w, uint8_t* out) {
-  if (blockIdx.x == 0 && threadIdx.x < D) {
-    float sg = 1.0f / (1.0f + expf(-w.log_lambda[threadIdx.x]));
-    reinterpret_cast<float*>(out + (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES)[threadIdx.x] = kRglruC * (sg == 0.f ? kLogOfZero : log2f(sg));
-  }
+  if (blockIdx.x == 0 && threadIdx.x < D) pack_recurrence(w, out);
   pack_image(w, N_TEMPORAL_CHUNKS, out, [](const BnbTemporalWeights& ww, int c, int r) { return temporal_chunk_row(ww, c, r); },
              [](const BnbTemporalWeights& ww, int c) { return temporal_chunk_gain(ww, c); }, [](int c, int r) { return temporal_chunk_halved(c, r); });
 }
@@ -142,10 +149,7 @@ __global__ void k_pack_trunk(const __grid_constant__ PackJobs jobs) {
   } else {
     const BnbTemporalWeights& w = jobs.tw[j - jobs.n_spatial];
     uint8_t* out = static_cast<uint8_t*>(const_cast<void*>(w.packed));
-    if (blockIdx.x == 0 && threadIdx.x < D) {
-      float sg = 1.0f / (1.0f + expf(-w.log_lambda[threadIdx.x]));
-      reinterpret_cast<float*>(out + (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES)[threadIdx.x] = kRglruC * (sg == 0.f ? kLogOfZero : log2f(sg));
-    }
+    if (blockIdx.x == 0 && threadIdx.x < D) pack_recurrence(w, out);
     pack_image(w, N_TEMPORAL_CHUNKS, out, [](const BnbTemporalWeights& ww, int c, int r) { return temporal_chunk_row(ww, c, r); },
                [](const BnbTemporalWeights& ww, int c) { return temporal_chunk_gain(ww, c); }, [](int c, int r) { return temporal_chunk_halved(c, r); });
   }
@@ -578,7 +582,7 @@ size_t scratch_bytes(int, const BnbBatch& b, int T, int bullets_per_env) {
   return bytes;
 }
 size_t packed_spatial_bytes(int d_model) { return d_model == D ? (size_t)N_SPATIAL_IMAGE * CHUNK_BYTES : 0; }
-size_t packed_temporal_bytes(int d_model) { return d_model == D ? (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES + 1024 : 0; }
+size_t packed_temporal_bytes(int d_model) { return d_model == D ? (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES + 2048 : 0; }
 
 int pack_spatial(const BnbSpatialWeights& w, int d_model, int n_heads, void* packed, cudaStream_t st) {
   if (d_model != D || n_heads != HEADS) return BNB_ERR_UNSUPPORTED_DIMS;
@@ -729,8 +733,6 @@ static void fill_temporal(SubLayer& s, const BnbTemporalWeights& w, const float*
   s.packed = static_cast<const uint8_t*>(w.packed);
   s.conv_w = w.conv_w;
   s.conv_b = w.conv_b;
-  s.a_b = w.a_b;
-  s.x_b = w.x_b;
   s.decay_log2 = reinterpret_cast<const float*>(static_cast<const uint8_t*>(w.packed) + (size_t)N_TEMPORAL_CHUNKS * CHUNK_BYTES);
   s.hid_in = hin;
   s.hid_out = hout;

@@ -10,14 +10,6 @@ namespace tensor {
 constexpr int EPI_WARPS = 16, EPI_THREADS = 512, MMA_WARP = 16, LOAD_WARP = 17, THREADS = 576;
 enum : int { TIMEOUT_FULL = 101, TIMEOUT_FREE = 102, TIMEOUT_ACC = 103, TIMEOUT_OPERAND = 104 };
 
-// Two floats in one 64-bit register pair: one instruction for two multiply-adds.
-struct F2 { unsigned long long v; };
-__device__ __forceinline__ F2 f2(float lo, float hi) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi)); return r; }
-__device__ __forceinline__ F2 f2(float both) { return f2(both, both); }
-__device__ __forceinline__ float2 halves(F2 a) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v)); return r; }
-__device__ __forceinline__ F2 mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
-
 // What every role needs for its waits.
 struct Sync {
   uint32_t bars;           // shared address of the barrier array
