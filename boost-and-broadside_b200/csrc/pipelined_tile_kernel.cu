@@ -54,11 +54,14 @@ constexpr int OFF_A = 0;
 constexpr int OFF_P = 32768;
 constexpr int OFF_KV = 65536;
 constexpr int OFF_RING = 131072;
-constexpr int OFF_META = OFF_RING + RING_BYTES;  // env_first[128], env_n[128], alive[128], items[128]
-constexpr int OFF_ROWINFO = OFF_META + 512;                     // hidden row of each tile row (int), then flags[128]
-constexpr int OFF_SS = OFF_ROWINFO + 640;                       // partial sums of squares [4][128]
-constexpr int OFF_BIAS = OFF_SS + 2048;                         // attention bias of each tile row as a key (float), + 16 of slack
-constexpr int OFF_BAR = OFF_BIAS + 576;
+constexpr int OFF_SS = OFF_RING + RING_BYTES;                   // partial sums of squares [4][128]
+// What the rows of a pass are, twice (the pass at work and the next one): Place[128], then the blocks of 16 queries (first
+// row | first row of the environment << 8 | its tokens less one << 16), then the attention bias of each row as a key
+// (float, 16 of slack), then the number of blocks.
+constexpr int OFF_TAB = OFF_SS + 2048;
+constexpr int TAB_BLOCKS = 2048, TAB_BIAS = TAB_BLOCKS + 512, TAB_COUNT = TAB_BIAS + 576, TAB_BYTES = TAB_COUNT + 16;
+static_assert(TAB_BYTES % 16 == 0, "16-byte accesses");
+constexpr int OFF_BAR = OFF_TAB + 2 * TAB_BYTES;
 constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
 
 // mbarrier indices
@@ -71,9 +74,11 @@ constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
 // used again before they have seen it, and the issuing warp of gate|up as "accumulator free" for a down projection.
 // ACC: every MMA of a round is complete (one more commit per round).
 // EARLY: the first half of a temporal sublayer's gates is.  PARK: linear2's accumulator has been read (epilogue warps ->
-// issuing warp); FIELD: field_sub, multiplied into it then, is complete.  DRAIN: every MMA of the
+// issuing warp); FIELD: field_sub, multiplied into it then, is complete.  XFULL: the row table of the next pass is
+// written and its tokens have landed in the P area (down-projection warp -> epilogue warps); XFREE: the tokens have been read, and
+// nobody works on the pass before any more.  DRAIN: every MMA of the
 // CTA is complete (once per issuing warp, at the end).
-enum : int { B_OP0 = 0, B_FFN0, B_FFN1, B_FFN2, B_KVREL, B_PARK, B_DRAIN, B_ACC, B_EARLY, B_FIELD, B_FULL0, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
+enum : int { B_OP0 = 0, B_FFN0, B_FFN1, B_FFN2, B_KVREL, B_PARK, B_XFREE, B_XFULL, B_DRAIN, B_ACC, B_EARLY, B_FIELD, B_FULL0, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
 static_assert(B_COUNT * 8 + 8 <= 256, "barrier area");
 
 constexpr uint32_t COL_RESID = 0;
@@ -189,6 +194,15 @@ __device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity, volatile
   if (aborted[0] == 0) aborted[0] = code;
 }
 
+// What one tile row is in a pass (16 bytes of the row table).
+struct Place {
+  int hrow;        // row of the packed hidden state, -1 for field / invalid rows
+  uint32_t flags;  // P_*, and from bit 8 on the stored conv lags still inside the current episode (0..3)
+  int trow;        // token row of the call (0 for rows outside every environment)
+  int unused;
+};
+enum : uint32_t { P_VALID = 1, P_ZERO_IN = 2 /* incoming state taken as zero (reset_env) */, P_BOUNDARY = 4 };
+
 // ------------------------------------------------------------------ epilogue side
 
 struct Epi {
@@ -203,10 +217,12 @@ struct Epi {
   uint32_t sbase;       // shared address of smem
   uint32_t bars;        // shared address of the barrier array
   uint32_t lane_addr;   // tensor-memory address of this thread's lane, column 0
-  uint32_t par;         // phase bits of the pair slots' DONE barriers (0..2), of ACC (8), EARLY (10) and FIELD (11)
+  uint32_t par;         // phase bits of the pair slots' DONE barriers (0..2), of ACC (8), EARLY (10), FIELD (11)
+                        // and XFULL (12)
   int row, part;
   bool wide;            // 32-byte accesses: every row pointer is aligned for them
   volatile int* aborted;
+  const uint8_t* tab;   // the row table of this pass
   float* ss_part;
 };
 
@@ -391,18 +407,18 @@ __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slo
 // walked in blocks of 16 with a running maximum.  Output: bf16 into the P area as the A operand of out_proj, each block over its own q.
 __device__ __forceinline__ void attention(Epi& e, int n_items) {
   TRACE(e.tr, 310);
-  const uint8_t* meta = e.smem + OFF_META;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int h = e.part;
   const uint32_t atom = (uint32_t)(h >> 1) * CHUNK_BYTES;
   const int c8h = (h & 1) * 4;
   const uint32_t sQ = e.sbase + OFF_P + atom, sK = e.sbase + OFF_KV + atom, sV = sK + 2 * CHUNK_BYTES;
-  const float* key_bias = reinterpret_cast<const float*>(e.smem + OFF_BIAS);
+  const float* key_bias = reinterpret_cast<const float*>(e.tab + TAB_BIAS);
+  const uint32_t* blocks = reinterpret_cast<const uint32_t*>(e.tab + TAB_BLOCKS);
   const float c2 = 0.17677669529663687f * 1.4426950408889634f;  // log2(e) / sqrt(32): scores in the log2 domain
   for (int it = (warp + h) & 3; it < n_items; it += EPI_WARPS / 4) {
-    const int r0 = meta[384 + it];
-    const int e0 = meta[r0], n = meta[128 + r0] + 1;   // first tile row and size of the environment
+    const uint32_t block = blocks[it];
+    const int r0 = block & 255, e0 = block >> 8 & 255, n = (int)(block >> 16) + 1;   // first row; first tile row and size of the environment
     const int last = e0 + n - 1;
     uint32_t qa[2][4];
     {
@@ -578,16 +594,9 @@ __device__ __forceinline__ void run_spatial_post(Epi& e, const SubLayer& s, size
   post(e, B_OP0);
 }
 
-struct RowState {
-  int hrow;        // row of the packed hidden state, -1 for field / invalid rows
-  int lag_ok;      // stored conv lags still inside the current episode (0..3)
-  bool zero_in;    // incoming state taken as zero (reset_env)
-};
-
 // One temporal sublayer on the tile at one timestep.  In the gate epilogue thread (row, part)
 // works on hidden columns [64 rnd + 16 part, +16), and parks b2 for exactly those.
-__device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const RowState& rs, bool boundary, bool has_fields,
-                                             const float* hid_in) {
+__device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Place& rs, bool has_fields, const float* hid_in) {
   const bool is_ship = rs.hrow >= 0;
   const float* hin = is_ship ? hid_in + (size_t)rs.hrow * 4 * D : nullptr;
   float* hout = is_ship ? s.hid_out + (size_t)rs.hrow * 4 * D : nullptr;
@@ -597,8 +606,6 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
   {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int col = lane * 4;
-    const int* row_hrow = reinterpret_cast<const int*>(e.smem + OFF_ROWINFO);
-    const uint8_t* row_flags = e.smem + OFF_ROWINFO + 512;
     // A warp takes rows warp, warp + 16, ...: four rows' taps are on their way at any time, the first four before the
     // products are waited for, and each row's registers ask for the row four further on as soon as it is done.  Rows are
     // distinct, so no load needs to wait for another row's store; volatile accesses keep the compiler to that
@@ -606,10 +613,11 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
     float4 t0[4], t1[4], t2[4];
     int hr[4], fl[4];
     const auto request = [&](int k, int r) {
-      hr[k] = row_hrow[r];
-      fl[k] = row_flags[r];
+      const int2 at = *reinterpret_cast<const int2*>(e.tab + 16 * r);
+      hr[k] = at.x;
+      fl[k] = at.y;
       t0[k] = t1[k] = t2[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (hr[k] >= 0 && !(fl[k] & 4)) {
+      if (hr[k] >= 0 && !(fl[k] & P_ZERO_IN)) {
         const float* hi = hid_in + (size_t)hr[k] * 4 * D + col;
         load4(t0[k], hi + D);
         load4(t1[k], hi + 2 * D);
@@ -646,7 +654,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
       for (int k = 0; k < 4; ++k) {
         const int r = r0 + EPI_WARPS * k;
         if (hr[k] >= 0) {
-          const int lag = fl[k] & 3;
+          const int lag = fl[k] >> 8;
           uint2* at = reinterpret_cast<uint2*>(e.smem + OFF_A + (lane >> 4) * CHUNK_BYTES + swz(r, (lane & 15) >> 1) + (lane & 1) * 8);
           const uint2 bw = *at;
           float* ho = s.hid_out + (size_t)hr[k] * 4 * D + col;
@@ -678,7 +686,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
   for (int i = 0; i < 4; ++i) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) hprev[i >> 1][i & 1][j] = 0.f;
-    if (is_ship && !rs.zero_in) load8(hprev[i >> 1][i & 1], hin + (i >> 1) * 64 + e.part * 16 + (i & 1) * 8, e.wide);
+    if (is_ship && !(rs.flags & P_ZERO_IN)) load8(hprev[i >> 1][i & 1], hin + (i >> 1) * 64 + e.part * 16 + (i & 1) * 8, e.wide);
   }
   // ... and b2 = bf16(gelu(linear2 n)) parked as packed bf16 pairs
   uint32_t b2p[2][8];
@@ -697,7 +705,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Ro
   }
   wait_early(e);   // acc0 / acc2 = halves of [W_a u | W_x u] of hidden columns [0,64) / [64,128)
   // gates and state update
-  const F2 keep = f2(boundary ? 0.f : 1.f), one = f2(1.f);
+  const F2 keep = f2(rs.flags & P_BOUNDARY ? 0.f : 1.f), one = f2(1.f);
 #pragma unroll
   for (int rnd = 0; rnd < 2; ++rnd) {
     if (rnd == 1) wait_round(e, has_fields ? 7 : 5);   // slots 2, 0 (and 1 for field_sub)
@@ -867,28 +875,22 @@ __device__ __forceinline__ void issue_gate_up(Issuer& m, uint32_t slot) {
 // temporal sublayer; as bulk prefetches they stand in the way of the weight copies (7 000 cycles).
 __device__ __forceinline__ void prefetch_line(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // The recurrent state of 16 tile rows (2 KB each, two lanes a row).
-__device__ __forceinline__ void prefetch_state(const float* hid, const int* row_hrow, int row0) {
-  const int lane = threadIdx.x & 31, hrow = row_hrow[row0 + (lane >> 1)];
+__device__ __forceinline__ void prefetch_state(const float* hid, const uint8_t* tab, int row0) {
+  const int lane = threadIdx.x & 31, hrow = *reinterpret_cast<const int*>(tab + 16 * (row0 + (lane >> 1)));
   if (hrow < 0) return;
   const float* p = hid + (size_t)hrow * 4 * D + (lane & 1) * 2 * D;
 #pragma unroll
   for (int i = 0; i < 8; ++i) prefetch_line(p + 32 * i);
 }
-// Tokens and masks of a tile at timestep t.
-__device__ __forceinline__ void prefetch_tokens(const TrunkArgs& args, int tile, int t) {
+// Runs of consecutive token rows that make up the rows of a tile: f(first tile row, first token row of the step, rows), the
+// whole warp.
+template <class F>
+__device__ __forceinline__ void for_token_runs(const TrunkArgs& args, int eb, F f) {
   const EnvMap& map = args.map;
   const int lane = threadIdx.x & 31;
-  const int grp = tile / args.env_tiles, eb = tile - grp * args.env_tiles;
-  const size_t group_row = (size_t)(grp + t) * map.total_tokens;
-  const size_t row_bytes = args.io_bf16 ? D * 2 : D * 4;
-  const uint8_t* x = reinterpret_cast<const uint8_t*>(args.x) + group_row * row_bytes;
-  const auto range = [&](int first, int n) {
-    const uint8_t* p = x + first * row_bytes;
-    for (int i = lane; i < n * (int)row_bytes / 128; i += 32) prefetch_line(p + 128 * i);
-    if (args.alive && lane < 2 && n > 0) prefetch_line(args.alive + group_row + first + (lane ? n - 1 : 0));
-  };
   if (args.tile_env_begin) {
     const int end = args.tile_env_begin[eb + 1];
+    int row = 0;
     for (int k0 = args.tile_env_begin[eb]; k0 < end; k0 += 32) {
       int first = 0, n = 0;
       if (k0 + lane < end) {
@@ -896,19 +898,139 @@ __device__ __forceinline__ void prefetch_tokens(const TrunkArgs& args, int tile,
         first = map.tok_off[env];
         n = map.tok_off[env + 1] - first;
       }
-      for (int j = 0; j < min(32, end - k0); ++j) range(__shfl_sync(0xffffffffu, first, j), __shfl_sync(0xffffffffu, n, j));
+      for (int j = 0; j < min(32, end - k0); ++j) {
+        const int rows = __shfl_sync(0xffffffffu, n, j);
+        f(row, __shfl_sync(0xffffffffu, first, j), rows);
+        row += rows;
+      }
     }
   } else if (args.flat_rows) {
-    range(eb * TILE, min(TILE, map.total_tokens - eb * TILE));
+    f(0, eb * TILE, min(TILE, map.total_tokens - eb * TILE));
   } else {
     const int env0 = eb * args.envs_per_tile;
-    range(env0 * map.tokens_per_env, min(args.envs_per_tile, map.n_envs - env0) * map.tokens_per_env);
+    f(0, env0 * map.tokens_per_env, min(args.envs_per_tile, map.n_envs - env0) * map.tokens_per_env);
   }
+}
+// The row table of a pass: tile `tile` at timestep t.
+template <bool WHOLE>
+__device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int t, uint8_t* tab) {
+  const EnvMap& map = args.map;
+  const int lane = threadIdx.x & 31;
+  const int grp = tile / args.env_tiles, eb = tile - grp * args.env_tiles;
+  const int group_row = (grp + t) * map.total_tokens;
+  uint32_t* blocks = reinterpret_cast<uint32_t*>(tab + TAB_BLOCKS);
+  float* bias = reinterpret_cast<float*>(tab + TAB_BIAS);
+  const auto invalid = [&](int row) {
+    reinterpret_cast<int4*>(tab)[row] = make_int4(-1, 0, 0, 0);
+    bias[row] = kMaskedScore;
+  };
+  // token `tok` of environment env, which has `ships` ships
+  const auto put = [&](int row, int env, int tok, int ships, int step_row, int hrow) {
+    uint32_t flags = P_VALID;
+    const int trow = group_row + step_row;
+    bias[row] = !args.alive || args.alive[trow] ? 0.f : kMaskedScore;
+    if (tok < ships) {
+      // steps since the last episode boundary, as far as the conv looks back; before the call there was none
+      uint32_t lags = BNB_CONV_KERNEL - 1;
+      if (args.done)
+#pragma unroll
+        for (int k = BNB_CONV_KERNEL - 1; k >= 1; --k)
+          if (t >= k && args.done[(size_t)(t - k) * map.n_envs + env]) lags = k - 1;
+      if (t >= 1 && lags == 0) flags |= P_BOUNDARY;
+      flags |= lags << 8;
+      if (t == 0 && args.reset_env && args.reset_env[env]) flags |= P_ZERO_IN;
+    } else {
+      hrow = -1;
+    }
+    reinterpret_cast<int4*>(tab)[row] = make_int4(hrow, (int)flags, trow, 0);
+  };
+  int n_blocks = 0;
+  if (!WHOLE && args.flat_rows) {
+    // plain 128-row slices of the token rows (programs without attention inside: the
+    // environments are larger than a tile); the environment of a row is looked up
+#pragma unroll 1
+    for (int row = lane; row < TILE; row += 32) {
+      const int r = eb * TILE + row;
+      if (r < map.total_tokens) {
+        const int env = map.env_of_token(r), tok = r - map.env_tok_begin(env);
+        put(row, env, tok, map.env_ship_count(env), r, map.env_ship_begin(env) + tok);
+      } else {
+        invalid(row);
+      }
+    }
+  } else if (args.tile_env_begin) {
+    // ragged: the tile holds the environments tile_env_ids[k_lo .. k_hi), rows in that order
+    const int end = args.tile_env_begin[eb + 1];
+    int first = 0;
+    for (int k0 = args.tile_env_begin[eb]; k0 < end; k0 += 32) {
+      int my_env = 0, my_tok = 0, my_n = 0, my_ship = 0, my_ships = 0;
+      if (k0 + lane < end) {
+        my_env = args.tile_env_ids[k0 + lane];
+        my_tok = map.tok_off[my_env];
+        my_n = map.tok_off[my_env + 1] - my_tok;
+        my_ship = map.ship_off[my_env];
+        my_ships = map.ship_off[my_env + 1] - my_ship;
+      }
+      for (int j = 0; j < min(32, end - k0); ++j) {
+        const int env = __shfl_sync(0xffffffffu, my_env, j), tok0 = __shfl_sync(0xffffffffu, my_tok, j), n = __shfl_sync(0xffffffffu, my_n, j),
+                  ship0 = __shfl_sync(0xffffffffu, my_ship, j), ships = __shfl_sync(0xffffffffu, my_ships, j);
+        for (int i = lane; i < n; i += 32) {
+          put(first + i, env, i, ships, tok0 + i, ship0 + i);
+          if ((i & 15) == 0) blocks[n_blocks + (i >> 4)] = (uint32_t)(first + i) | (uint32_t)first << 8 | (uint32_t)(n - 1) << 16;
+        }
+        first += n;
+        n_blocks += (n + 15) >> 4;
+      }
+    }
+    for (int row = first + lane; row < TILE; row += 32) invalid(row);
+  } else {
+    const int NM = map.tokens_per_env, per_env = (NM + 15) >> 4;
+    const int env0 = eb * args.envs_per_tile, envs = min(args.envs_per_tile, map.n_envs - env0);
+#pragma unroll 1
+    for (int row = lane; row < TILE; row += 32) {
+      const int el = row / NM, tok = row - el * NM;
+      if (el < envs) {
+        put(row, env0 + el, tok, map.ships_per_env, (env0 + el) * NM + tok, (env0 + el) * map.ships_per_env + tok);
+        if ((tok & 15) == 0) blocks[el * per_env + (tok >> 4)] = (uint32_t)row | (uint32_t)(el * NM) << 8 | (uint32_t)(NM - 1) << 16;
+      } else {
+        invalid(row);
+      }
+    }
+    n_blocks = envs * per_env;
+  }
+  if (lane == 0) *reinterpret_cast<int*>(tab + TAB_COUNT) = n_blocks;
+  __syncwarp();
+}
+// Tokens of a pass into L2.
+__device__ __forceinline__ void prefetch_tokens(const TrunkArgs& args, int tile, int t) {
+  const int lane = threadIdx.x & 31, row_bytes = args.io_bf16 ? D * 2 : D * 4;
+  const int grp = tile / args.env_tiles, group_row = (grp + t) * args.map.total_tokens;
+  for_token_runs(args, tile - grp * args.env_tiles, [&](int, int first, int n) {
+    const uint8_t* p = reinterpret_cast<const uint8_t*>(args.x) + (size_t)(group_row + first) * row_bytes;
+    for (int i = lane; i < n * (row_bytes / 128); i += 32) prefetch_line(p + 128 * i);
+  });
+}
+// bfloat16 tokens of a pass into the P area (free from a sublayer's out_proj or linear_out on), as two swizzled atoms.
+__device__ __forceinline__ void copy_tokens(const TrunkArgs& args, int tile, int t, uint32_t p_area) {
+  const int lane = threadIdx.x & 31;
+  const int grp = tile / args.env_tiles, group_row = (grp + t) * args.map.total_tokens;
+  for_token_runs(args, tile - grp * args.env_tiles, [&](int row, int first, int n) {
+    const uint8_t* p = reinterpret_cast<const uint8_t*>(args.x) + (size_t)(group_row + first) * (2 * D);
+    for (int i = lane; i < n * 16; i += 32) {
+      const int c8 = i & 15;
+      cp_async16(p_area + (c8 >> 3) * CHUNK_BYTES + swz(row + (i >> 4), c8 & 7), p + 16 * i);
+    }
+  });
+}
+// What this lane has written and copied for the next pass: two arrivals on XFULL.
+__device__ __forceinline__ void hand_over(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+  mbar_arrive(bar);
 }
 
 // The down projections of the eight chunks: A operand in tensor memory, K step k in the 8 columns at 16 k of the accumulator.
 // next_hid: the state that the following sublayer reads (null: none, or it is at hand), asked for on the way.
-__device__ __forceinline__ void issue_downs(Issuer& m, const float* next_hid, const int* row_hrow) {
+__device__ __forceinline__ void issue_downs(Issuer& m, const float* next_hid, const uint8_t* tab) {
   constexpr uint32_t idesc = instr_desc(128);
   uint32_t a = 0;
 #pragma unroll 1
@@ -923,7 +1045,7 @@ __device__ __forceinline__ void issue_downs(Issuer& m, const float* next_hid, co
     commit_one(m, B_DONE0 + 3 + a);
     T_SINCE(m.tacc, TM_ISSUE, tw);
     TRACE(m.tr, 430);
-    if (next_hid) prefetch_state(next_hid, row_hrow, 16 * (int)c);
+    if (next_hid) prefetch_state(next_hid, tab, 16 * (int)c);
     __syncwarp();
     a = a == 2 ? 0 : a + 1;
   }
@@ -967,9 +1089,8 @@ __device__ __forceinline__ void issue_temporal(Issuer& m, bool has_fields) {
 template <bool WHOLE>
 __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_constant__ TrunkArgs args) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // an offset: the compiler still knows it as shared memory
   __shared__ int s_aborted[2];
-  __shared__ int s_items;
   __shared__ SubLayer s_sub[MAX_SUBLAYERS];  // kernel parameters are slow to index dynamically
   __shared__ uint4 s_sched[MAX_SCHED];
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -980,6 +1101,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     if (op >= 0 && op < ops) s_sched[tid] = sched_entry(args.sub[si], op, args.has_fields != 0);
     sched_len += ops;
   }
+  // Both row tables start without rows: after a wait has run out they may be read before they are written.
+  for (int i = tid; i < 2 * TAB_BYTES / 16; i += THREADS)
+    reinterpret_cast<int4*>(smem + OFF_TAB)[i] = make_int4(i % (TAB_BYTES / 16) < TILE ? -1 : 0, 0, 0, 0);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 8 * B_COUNT);
   if (tid == 0) {
@@ -989,6 +1113,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     for (int i = B_FFN0; i <= B_FFN2; ++i) mbar_init(smem_u32(&bars[i]), EPI_WARPS / 2);
     mbar_init(smem_u32(&bars[B_KVREL]), EPI_WARPS);
     mbar_init(smem_u32(&bars[B_PARK]), EPI_WARPS);
+    mbar_init(smem_u32(&bars[B_XFREE]), EPI_WARPS);
+    mbar_init(smem_u32(&bars[B_XFULL]), 64);   // every lane of the copying warp: its copies, its writes
     mbar_init(smem_u32(&bars[B_DRAIN]), 2);   // both issuing warps
     for (int i = B_ACC; i < B_COUNT; ++i) mbar_init(smem_u32(&bars[i]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1079,6 +1205,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
 #endif
       T_MARK(t_start);
       const bool down = warp == DOWN_WARP;
+      if (down && passes > 0) {
+        fill_table<WHOLE>(args, blockIdx.x, 0, smem + OFF_TAB);
+        if (args.io_bf16) copy_tokens(args, blockIdx.x, 0, m.sbase + OFF_P);
+        hand_over(m.bars + 8 * B_XFULL);
+        __syncwarp();
+      }
       int tile = blockIdx.x, t = 0;
       for (int pass = 0; pass < passes; ++pass) {
         const int this_t = t;
@@ -1089,11 +1221,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
         for (int si = 0; si < args.n_sub; ++si) {
           const int type = (int)uniform((uint32_t)s_sub[si].type);
           if (down) {
-            if (si + 1 == args.n_sub && pass + 1 < passes) prefetch_tokens(args, tile, t);
+            if (si + 1 == args.n_sub && pass + 1 < passes) {
+              prefetch_tokens(args, tile, t);
+              wait_bar(m.bars + 8 * B_XFREE, pass & 1u, m.aborted, ST_TIMEOUT_OPERAND);
+              fill_table<WHOLE>(args, tile, t, smem + OFF_TAB + (~pass & 1) * TAB_BYTES);
+            }
             __syncwarp();
             const bool state_next = this_t == 0 && type != SUB_TEMPORAL && si + 1 < args.n_sub && s_sub[si + 1].type == SUB_TEMPORAL;
             if (WHOLE || type != SUB_SPATIAL_PRE)
-              issue_downs(m, state_next ? s_sub[si + 1].hid_in : nullptr, reinterpret_cast<const int*>(smem + OFF_ROWINFO));
+              issue_downs(m, state_next ? s_sub[si + 1].hid_in : nullptr, smem + OFF_TAB + (pass & 1) * TAB_BYTES);
             continue;
           }
           if (type == SUB_TEMPORAL) {
@@ -1104,6 +1240,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
             issue_out_proj(m, !WHOLE && type == SUB_SPATIAL_POST ? OFF_A : OFF_P);
           }
           issue_gate_up(m, type == SUB_TEMPORAL ? TEMPORAL_FFN_PAIR : SPATIAL_FFN_PAIR);
+        }
+        if (down && pass + 1 < passes) {
+          if (args.io_bf16) copy_tokens(args, tile, t, m.sbase + OFF_P);
+          hand_over(m.bars + 8 * B_XFULL);
+          __syncwarp();
         }
       }
       // Nothing issued here may outlive the CTA: its tensor memory is freed and its barriers go
@@ -1139,172 +1280,104 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     e.wait_slot = TE_ACC_WAIT;
 #endif
     T_MARK(t_start);
-    uint8_t* meta = smem + OFF_META;
-    const EnvMap& map = args.map;
-    const int NM = map.tokens_per_env;
-    const int row = e.row;
+    const int row = e.row, lane = tid & 31;
+    // Rows of bfloat16 tokens move through shared memory, so that a warp's access to global memory is two whole rows: 4
+    // accesses of 512 bytes, where a thread per row took 2 that touch 32 lines each (a pass's last wait to its
+    // first operand: 10 000 cycles, of a time walk's 45 000).  Row of this lane's i-th access, and its 16 bytes of the row:
+    const auto io_row = [&](int i) { return 32 * (warp & 3) + 8 * e.part + 2 * i + (lane >> 4); };
+    const uint32_t io_atom = ((lane & 15) >> 3) * CHUNK_BYTES;
+    const auto own16 = [&](int area, int j) { return reinterpret_cast<uint4*>(smem + area + (e.part >> 1) * CHUNK_BYTES + swz(row, (e.part & 1) * 4 + j)); };
 
-    for (int tile = blockIdx.x; tile < args.n_tiles; tile += gridDim.x) {
-      // ---- rows of this tile: whole environments, ships first then fields in each
+    int t = 0;
+    for (int pass = 0; pass < passes; ++pass) {
+      // ---- the pass: a tile of whole environments, ships first then fields in each
       T_MARK(t_io);
-      const int grp = tile / args.env_tiles, eb = tile - grp * args.env_tiles;
-      bool valid;
-      int env, tok, env_first, env_n, env_ships;
-      size_t grow = 0;
-      int hrow_if_ship;
-      if (!WHOLE && args.flat_rows) {
-        // plain 128-row slices of the token rows (programs without attention inside: the
-        // environments are larger than a tile); the environment of a row is looked up
-        const int r = eb * TILE + row;
-        valid = r < map.total_tokens;
-        env = valid ? map.env_of_token(r) : 0;
-        env_first = 0;
-        env_n = 1;
-        tok = valid ? r - map.env_tok_begin(env) : 0;
-        env_ships = valid ? map.env_ship_count(env) : 0;
-        grow = (size_t)grp * map.total_tokens + (size_t)r;
-        hrow_if_ship = map.env_ship_begin(env) + tok;
-      } else if (args.tile_env_begin) {
-        // ragged: the tile holds the environments tile_env_ids[k_lo .. k_hi), rows in that order
-        const int k_lo = args.tile_env_begin[eb], k_hi = args.tile_env_begin[eb + 1];
-        int k = k_lo, first = 0;
-        env = args.tile_env_ids[k];
-        int cnt = map.tok_off[env + 1] - map.tok_off[env];
-        while (row >= first + cnt && k + 1 < k_hi) {
-          first += cnt;
-          ++k;
-          env = args.tile_env_ids[k];
-          cnt = map.tok_off[env + 1] - map.tok_off[env];
-        }
-        valid = row < first + cnt;
-        env_first = first;
-        env_n = cnt;
-        env_ships = map.ship_off[env + 1] - map.ship_off[env];
-        tok = row - first;
-        grow = (size_t)grp * map.total_tokens + (size_t)(map.tok_off[env] + tok);
-        hrow_if_ship = map.ship_off[env] + tok;
-      } else {
-        const int env0 = eb * args.envs_per_tile;
-        const int env_cnt = min(args.envs_per_tile, map.n_envs - env0);
-        const int el = row / NM;
-        tok = row - el * NM;
-        valid = el < env_cnt;
-        env = env0 + el;
-        env_first = el * NM;
-        env_n = NM;
-        env_ships = map.ships_per_env;
-        grow = (size_t)grp * map.total_tokens + (size_t)env * NM + tok;
-        hrow_if_ship = env * map.ships_per_env + tok;
-      }
-      if (!valid) { grow = 0; env = 0; }
-      const bool is_ship = valid && tok < env_ships;
-      RowState rs;
-      rs.hrow = is_ship ? hrow_if_ship : -1;
-      rs.lag_ok = BNB_CONV_KERNEL - 1;
-      rs.zero_in = is_ship && args.reset_env && args.reset_env[env];
-      epi_sync();  // previous tile's readers of the meta arrays are done
-      if (e.part == 0) {
-        meta[row] = (uint8_t)(valid ? env_first : row);
-        meta[128 + row] = (uint8_t)(valid ? env_n - 1 : 0);
-        reinterpret_cast<int*>(smem + OFF_ROWINFO)[row] = rs.hrow;
-      }
-      if (tid == 0) s_items = 0;
-      epi_sync();
-      if (e.part == 0 && valid && (tok & 15) == 0) meta[384 + atomicAdd(&s_items, 1)] = (uint8_t)row;
-
-      for (int t = 0; t < args.t_loop; ++t) {
-        const size_t trow = grow + (size_t)t * map.total_tokens;
-        if (e.part == 0) {
-          const bool live = valid && (!args.alive || args.alive[trow]);
-          meta[256 + row] = live ? (uint8_t)1 : (uint8_t)0;
-          reinterpret_cast<float*>(smem + OFF_BIAS)[row] = live ? 0.f : kMaskedScore;
-        }
-        // residual <- x (this thread: columns [32 part, 32 part + 32))
-        {
-          uint32_t v[32];
-          if (args.io_bf16) {
-            const float* src = reinterpret_cast<const float*>(reinterpret_cast<const __nv_bfloat16*>(args.x) + trow * D + e.part * 32);
+      const bool first_step = t == 0;
+      if (++t == args.t_loop) t = 0;
+      wait_other(e, B_XFULL, 12);
+      e.tab = smem + OFF_TAB + (pass & 1) * TAB_BYTES;
+      const int4 own = reinterpret_cast<const int4*>(e.tab)[row];
+      const Place rs{own.x, (uint32_t)own.y, own.z, 0};
+      const bool valid = rs.flags & P_VALID;
+      // residual <- x (this thread: columns [32 part, 32 part + 32))
+      {
+        uint32_t v[32];
+        if (args.io_bf16) {
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              float w[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-              if (valid) load8(w, src + 8 * q, e.wide);
+          for (int j = 0; j < 4; ++j) {
+            const uint4 w = valid ? *own16(OFF_P, j) : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                v[q * 16 + 2 * j] = __float_as_uint(w[j]) << 16;              // a bfloat16 is the upper half of its float
-                v[q * 16 + 2 * j + 1] = __float_as_uint(w[j]) & 0xFFFF0000u;
-              }
-            }
-          } else {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-              if (valid) load8(f, args.x + trow * D + e.part * 32 + q * 8, e.wide);
-#pragma unroll
-              for (int j = 0; j < 8; ++j) v[q * 8 + j] = __float_as_uint(f[j]);
+            for (int k = 0; k < 4; ++k) {
+              v[j * 8 + 2 * k] = ws[k] << 16;              // a bfloat16 is the upper half of its float
+              v[j * 8 + 2 * k + 1] = ws[k] & 0xFFFF0000u;
             }
           }
-          tmem_st32(e.lane_addr + COL_RESID + e.part * 32, v);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (valid) load8(f, args.x + (size_t)rs.trow * D + e.part * 32 + q * 8, e.wide);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[q * 8 + j] = __float_as_uint(f[j]);
+          }
         }
-        bool boundary = false;
-        if (t >= 1) {
-          boundary = is_ship && args.done && args.done[(size_t)(t - 1) * map.n_envs + env];
-          rs.lag_ok = boundary ? 0 : min(rs.lag_ok + 1, BNB_CONV_KERNEL - 1);
-          rs.zero_in = false;
-        }
-        if (e.part == 0) smem[OFF_ROWINFO + 512 + row] = (uint8_t)(rs.lag_ok | (rs.zero_in ? 4 : 0));
-        epi_sync();
-        T_SINCE(e.tacc, TE_IO, t_io);
-        const int n_items = s_items;
-        for (int si = 0; si < args.n_sub; ++si) {
-          const SubLayer& s = s_sub[si];
-          const int type = s.type;
-          const bool temporal = type == SUB_TEMPORAL;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(e.bars + 8 * B_XFREE);
+        tmem_st32(e.lane_addr + COL_RESID + e.part * 32, v);
+      }
+      T_SINCE(e.tacc, TE_IO, t_io);
+      const int n_items = *reinterpret_cast<const int*>(e.tab + TAB_COUNT);
+      for (int si = 0; si < args.n_sub; ++si) {
+        const SubLayer& s = s_sub[si];
+        const int type = s.type;
+        const bool temporal = type == SUB_TEMPORAL;
 #pragma unroll 1
-          for (int half = 0; half < 2; ++half) {
-            if (WHOLE || half || type != SUB_SPATIAL_POST) {
-              norm_to_A(e);
-              post(e, B_OP0);
-            }
-            if (half) {
-              ffn(e, temporal ? TEMPORAL_FFN_PAIR : SPATIAL_FFN_PAIR);
-              break;
-            }
-            if (temporal) run_temporal(e, s, rs, boundary, args.has_fields != 0, t == 0 ? s.hid_in : s.hid_out);
-            else if (WHOLE || type == SUB_SPATIAL) run_spatial(e, n_items, valid);
-            else if (type == SUB_SPATIAL_POST) run_spatial_post(e, s, trow, valid);
-            else {
-              run_spatial_pre(e, s, trow, valid);
-              break;
-            }
-            wait_round(e, temporal ? LINEAR_OUT_FLIPS : OUT_FLIPS);   // out_proj or linear_out accumulated into the residual
+        for (int half = 0; half < 2; ++half) {
+          if (WHOLE || half || type != SUB_SPATIAL_POST) {
+            norm_to_A(e);
+            post(e, B_OP0);
           }
-        }
-        // y <- residual
-        T_RESET(t_io);
-        {
-          uint32_t v[32];
-          tmem_ld32(e.lane_addr + COL_RESID + e.part * 32, v);
-          if (valid && args.io_bf16) {
-            float* dst = reinterpret_cast<float*>(reinterpret_cast<__nv_bfloat16*>(args.y) + trow * D + e.part * 32);
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              float w[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) w[j] = __uint_as_float(pack_bf16(__uint_as_float(v[q * 16 + 2 * j]), __uint_as_float(v[q * 16 + 2 * j + 1])));
-              store8(dst + 8 * q, w, e.wide);
-            }
-          } else if (valid) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              float f[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[q * 8 + j]);
-              store8(args.y + trow * D + e.part * 32 + q * 8, f, e.wide);
-            }
+          if (half) {
+            ffn(e, temporal ? TEMPORAL_FFN_PAIR : SPATIAL_FFN_PAIR);
+            break;
           }
+          if (temporal) run_temporal(e, s, rs, args.has_fields != 0, first_step ? s.hid_in : s.hid_out);
+          else if (WHOLE || type == SUB_SPATIAL) run_spatial(e, n_items, valid);
+          else if (type == SUB_SPATIAL_POST) run_spatial_post(e, s, rs.trow, valid);
+          else {
+            run_spatial_pre(e, s, rs.trow, valid);
+            break;
+          }
+          wait_round(e, temporal ? LINEAR_OUT_FLIPS : OUT_FLIPS);   // out_proj or linear_out accumulated into the residual
         }
-        T_SINCE(e.tacc, TE_IO, t_io);
       }
+      // y <- residual
+      T_RESET(t_io);
+      {
+        uint32_t v[32];
+        tmem_ld32(e.lane_addr + COL_RESID + e.part * 32, v);
+        if (args.io_bf16) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) *own16(OFF_A, j) = pack8(&v[8 * j]);
+          asm volatile("bar.sync %0, 128;" ::"r"(3 + (warp & 3)) : "memory");   // the four warps of these rows
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int at = __shfl_sync(0xffffffffu, valid ? rs.trow : -1, 8 * e.part + 2 * i + (lane >> 4));
+            const uint4 w = *reinterpret_cast<const uint4*>(smem + OFF_A + io_atom + swz(io_row(i), lane & 7));
+            if (at >= 0) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(args.y) + (size_t)at * (2 * D) + (lane & 15) * 16) = w;
+          }
+        } else if (valid) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float f[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[q * 8 + j]);
+            store8(args.y + (size_t)rs.trow * D + e.part * 32 + q * 8, f, e.wide);
+          }
+        }
+      }
+      T_SINCE(e.tacc, TE_IO, t_io);
     }
 #ifdef BNB_TIMING
     e.tacc[TE_TOTAL] = clock64() - t_start;
