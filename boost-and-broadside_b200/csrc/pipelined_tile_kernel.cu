@@ -198,10 +198,17 @@ __device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity, volatile
 struct Place {
   int hrow;        // row of the packed hidden state, -1 for field / invalid rows
   uint32_t flags;  // P_*, and from bit 8 on the stored conv lags still inside the current episode (0..3)
-  int trow;        // token row of the call (0 for rows outside every environment)
+  int trow;        // token row of the call, -1 for rows outside every environment
   int unused;
 };
-enum : uint32_t { P_VALID = 1, P_ZERO_IN = 2 /* incoming state taken as zero (reset_env) */, P_BOUNDARY = 4 };
+enum : uint32_t { P_VALID = 1, P_ZERO_IN = 2 /* incoming state taken as zero (reset_env) */, P_BOUNDARY = 4, P_LAST = 8 /* its step's state is stored */ };
+
+// What a launch's program may hold; the code it does not need costs registers and instruction fetches.
+//   ANY    every kind of sublayer
+//   WHOLE  whole sublayers on tiles of whole environments, most calls by far
+//   STEPS  one temporal sublayer of a sequence on tiles of 128 / C tokens x C consecutive timesteps (TrunkArgs::chunk); a CTA
+//          walks the chunks of its tokens in order
+enum : int { ANY = 0, WHOLE = 1, STEPS = 2 };
 
 // ------------------------------------------------------------------ epilogue side
 
@@ -594,24 +601,61 @@ __device__ __forceinline__ void run_spatial_post(Epi& e, const SubLayer& s, size
   post(e, B_OP0);
 }
 
-// One temporal sublayer on the tile at one timestep.  In the gate epilogue thread (row, part)
-// works on hidden columns [64 rnd + 16 part, +16), and parks b2 for exactly those.
-__device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Place& rs, bool has_fields, const float* hid_in) {
+// u = bias + w0 tap0 + w1 tap1 + w2 tap2 + w3 b1 of four columns, summed in the reference's order; lag: taps that belong to the
+// episode.  Returned as packed bf16.
+struct ConvWeights { float w[4][4], b[4]; };
+__device__ __forceinline__ ConvWeights conv_weights(const SubLayer& s, int col) {
+  ConvWeights c;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 w4 = __ldg(reinterpret_cast<const float4*>(s.conv_w + (col + i) * 4));
+    c.w[i][0] = w4.x; c.w[i][1] = w4.y; c.w[i][2] = w4.z; c.w[i][3] = w4.w;
+    c.b[i] = __ldg(s.conv_b + col + i);
+  }
+  return c;
+}
+__device__ __forceinline__ uint2 conv4(const ConvWeights& c, const float4& t0, const float4& t1, const float4& t2, const float4& b1, int lag) {
+  const float a0[4] = {t0.x, t0.y, t0.z, t0.w}, a1[4] = {t1.x, t1.y, t1.z, t1.w}, a2[4] = {t2.x, t2.y, t2.z, t2.w}, a3[4] = {b1.x, b1.y, b1.z, b1.w};
+  float u[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float p0 = lag >= 3 ? __fmul_rn(a0[i], c.w[i][0]) : 0.f;
+    const float p1 = lag >= 2 ? __fmul_rn(a1[i], c.w[i][1]) : 0.f;
+    const float p2 = lag >= 1 ? __fmul_rn(a2[i], c.w[i][2]) : 0.f;
+    const float p3 = __fmul_rn(a3[i], c.w[i][3]);
+    u[i] = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p0, p1), p2), p3), c.b[i]);
+  }
+  return make_uint2(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]));
+}
+__device__ __forceinline__ float4 unpack4(const uint2& v) { return make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y)); }
+
+// One temporal sublayer on the tile: at one timestep, or (STEPS) on chunks of `chunk` consecutive timesteps of its
+// tokens.  In the gate epilogue thread (row, part) works on hidden columns [64 rnd + 16 part, +16), and parks b2 for exactly
+// those.
+//
+// Chunks: a time walk of whole batches moves a state of 2 KB a row in and out of L2 at every step (512 KB a tile, all SMs at
+// once) and has as few tiles as the batch has rows.  With 128 / C tokens x C steps the state is read and written once a chunk,
+// taps come from the rows above, and the recurrence is a scan over the lanes of a warp (C rows of a
+// token are neighbouring lanes): 32 steps of 4096 x 8 tokens 6075 -> 5723, 5 of 67 x 11 306 -> 197 us.
+template <bool STEPS>
+__device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Place& rs, bool has_fields, const float* hid_in, int chunk) {
   const bool is_ship = rs.hrow >= 0;
   const float* hin = is_ship ? hid_in + (size_t)rs.hrow * 4 * D : nullptr;
   float* hout = is_ship ? s.hid_out + (size_t)rs.hrow * 4 * D : nullptr;
   // Causal conv, one warp per ship row and four columns per lane, so that the stored taps are
-  // read and written as whole 512-byte rows.  u = bias + w0 tap0 + w1 tap1 + w2 tap2 + w3 b1,
-  // summed in the reference's order; new taps = (tap1, tap2, b1); bf16(u) replaces b1 in A.
+  // read and written as whole 512-byte rows; new taps = (tap1, tap2, b1); bf16(u) replaces b1 in A.
   {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int col = lane * 4;
-    // A warp takes rows warp, warp + 16, ...: four rows' taps are on their way at any time, the first four before the
-    // products are waited for, and each row's registers ask for the row four further on as soon as it is done.  Rows are
-    // distinct, so no load needs to wait for another row's store; volatile accesses keep the compiler to that
+    const auto in_A = [&](int r) { return reinterpret_cast<uint2*>(e.smem + OFF_A + (lane >> 4) * CHUNK_BYTES + swz(r, (lane & 15) >> 1) + (lane & 1) * 8); };
+    // One timestep: a warp takes rows warp, warp + 16, ...: four rows' taps are on their way at any time, the first four
+    // before the products are waited for, and each row's registers ask for the row four further on as soon as it is done.
+    // Rows are distinct, so no load needs to wait for another row's store; volatile accesses keep the compiler to that
     // order (the state may be updated in place).
-    float4 t0[4], t1[4], t2[4];
-    int hr[4], fl[4];
+    // Chunks: a warp takes rows 8 warp .. + 8, the stored taps of the tokens that begin there (two of them at most).
+    constexpr int IN_FLIGHT = STEPS ? 2 : 4;
+    float4 t0[IN_FLIGHT], t1[IN_FLIGHT], t2[IN_FLIGHT];
+    int hr[IN_FLIGHT], fl[IN_FLIGHT];
     const auto request = [&](int k, int r) {
       const int2 at = *reinterpret_cast<const int2*>(e.tab + 16 * r);
       hr[k] = at.x;
@@ -624,8 +668,15 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
         load4(t2[k], hi + 3 * D);
       }
     };
+    ConvWeights cw;
+    if constexpr (STEPS) {
+      cw = conv_weights(s, col);
+      if ((8 * warp & (chunk - 1)) == 0) request(0, 8 * warp);
+      if (chunk == 4) request(1, 8 * warp + 4);
+    } else {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) request(k, warp + EPI_WARPS * k);
+      for (int k = 0; k < 4; ++k) request(k, warp + EPI_WARPS * k);
+    }
     wait_round(e, 3);   // acc0 = linear1 n, acc1 = linear2 n / 2; slots 0 and 1
     // b1 = bf16(linear1 n) into the A operand
 #pragma unroll
@@ -639,43 +690,60 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
         *reinterpret_cast<uint4*>(e.smem + OFF_A + (c8 >> 6) * CHUNK_BYTES + swz(e.row, (c8 & 63) >> 3)) = pack8(&v[q * 8]);
       }
     }
-    float cw[4][4], cb[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float4 w4 = __ldg(reinterpret_cast<const float4*>(s.conv_w + (col + i) * 4));
-      cw[i][0] = w4.x; cw[i][1] = w4.y; cw[i][2] = w4.z; cw[i][3] = w4.w;
-      cb[i] = __ldg(s.conv_b + col + i);
-    }
+    if constexpr (!STEPS) cw = conv_weights(s, col);
     tc_fence_before();
     epi_sync();
-#pragma unroll 1
-    for (int r0 = warp; r0 < TILE; r0 += 4 * EPI_WARPS) {
+    if constexpr (STEPS) {
+      uint2 bw[8];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int r = r0 + EPI_WARPS * k;
-        if (hr[k] >= 0) {
-          const int lag = fl[k] >> 8;
-          uint2* at = reinterpret_cast<uint2*>(e.smem + OFF_A + (lane >> 4) * CHUNK_BYTES + swz(r, (lane & 15) >> 1) + (lane & 1) * 8);
-          const uint2 bw = *at;
-          float* ho = s.hid_out + (size_t)hr[k] * 4 * D + col;
-          const float b1[4] = {bf16_lo(bw.x), bf16_hi(bw.x), bf16_lo(bw.y), bf16_hi(bw.y)};
-          store4(ho + D, t1[k]);
-          store4(ho + 2 * D, t2[k]);
-          store4(ho + 3 * D, make_float4(b1[0], b1[1], b1[2], b1[3]));
-          const float a0[4] = {t0[k].x, t0[k].y, t0[k].z, t0[k].w}, a1[4] = {t1[k].x, t1[k].y, t1[k].z, t1[k].w},
-                      a2[4] = {t2[k].x, t2[k].y, t2[k].z, t2[k].w};
-          float u[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float p0 = lag >= 3 ? __fmul_rn(a0[i], cw[i][0]) : 0.f;
-            const float p1 = lag >= 2 ? __fmul_rn(a1[i], cw[i][1]) : 0.f;
-            const float p2 = lag >= 1 ? __fmul_rn(a2[i], cw[i][2]) : 0.f;
-            const float p3 = __fmul_rn(b1[i], cw[i][3]);
-            u[i] = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p0, p1), p2), p3), cb[i]);
-          }
-          *at = make_uint2(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]));
+      for (int i = 0; i < 8; ++i) bw[i] = *in_A(8 * warp + i);
+      if (chunk > 8) {
+        if (8 * warp & (chunk - 1)) {   // the taps are the rows above, which their own warp is about to replace by u
+          t0[0] = unpack4(*in_A(8 * warp - 3));
+          t1[0] = unpack4(*in_A(8 * warp - 2));
+          t2[0] = unpack4(*in_A(8 * warp - 1));
         }
-        if (r + 4 * EPI_WARPS < TILE) request(k, r + 4 * EPI_WARPS);
+        asm volatile("bar.sync %0, 128;" ::"r"(11 + (warp >> 2)) : "memory");   // the four warps of 32 rows
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = 8 * warp + i;
+        if (i == 4 && chunk == 4) {
+          t0[0] = t0[1];
+          t1[0] = t1[1];
+          t2[0] = t2[1];
+        }
+        const int2 at = *reinterpret_cast<const int2*>(e.tab + 16 * r);
+        if (at.x >= 0) {
+          const float4 b1 = unpack4(bw[i]);
+          *in_A(r) = conv4(cw, t0[0], t1[0], t2[0], b1, at.y >> 8);
+          t0[0] = t1[0];
+          t1[0] = t2[0];
+          t2[0] = b1;
+          if (at.y & P_LAST) {
+            float* ho = s.hid_out + (size_t)at.x * 4 * D + col;
+            store4(ho + D, t0[0]);
+            store4(ho + 2 * D, t1[0]);
+            store4(ho + 3 * D, t2[0]);
+          }
+        }
+      }
+    } else {
+#pragma unroll 1
+      for (int r0 = warp; r0 < TILE; r0 += 4 * EPI_WARPS) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int r = r0 + EPI_WARPS * k;
+          if (hr[k] >= 0) {
+            const float4 b1 = unpack4(*in_A(r));
+            float* ho = s.hid_out + (size_t)hr[k] * 4 * D + col;
+            store4(ho + D, t1[k]);
+            store4(ho + 2 * D, t2[k]);
+            store4(ho + 3 * D, b1);
+            *in_A(r) = conv4(cw, t0[k], t1[k], t2[k], b1, fl[k] >> 8);
+          }
+          if (r + 4 * EPI_WARPS < TILE) request(k, r + 4 * EPI_WARPS);
+        }
       }
     }
   }
@@ -686,7 +754,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
   for (int i = 0; i < 4; ++i) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) hprev[i >> 1][i & 1][j] = 0.f;
-    if (is_ship && !(rs.flags & P_ZERO_IN)) load8(hprev[i >> 1][i & 1], hin + (i >> 1) * 64 + e.part * 16 + (i & 1) * 8, e.wide);
+    if (is_ship && !(rs.flags & P_ZERO_IN) && (!STEPS || (e.row & (chunk - 1)) == 0)) load8(hprev[i >> 1][i & 1], hin + (i >> 1) * 64 + e.part * 16 + (i & 1) * 8, e.wide);
   }
   // ... and b2 = bf16(gelu(linear2 n)) parked as packed bf16 pairs
   uint32_t b2p[2][8];
@@ -714,16 +782,31 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
     tmem_ld16_nowait(acc, rv);        // executed by every lane of the warp
     tmem_ld16_nowait(acc + 64, iv);
     tmem_wait_ld();
-    if (is_ship) {
+    // per column: h = a h_prev + b; with chunks h_prev stands in a token's first row (0 in the others) and the rest follows
+    // from the scan over its rows below, which lanes of field and empty rows run along with.
+    F2 av[STEPS ? 8 : 1], bv[STEPS ? 8 : 1];
+    // result of a pair of columns: new state, and the branch operand of linear_out
+    const auto finish = [&](F2 h, int k, float* hn, uint32_t& ob) {
+      const float2 n = halves(h);
+      hn[0] = n.x;
+      hn[1] = n.y;
+      ob = pack_bf16(mul(h, unpack_bf16(b2p[rnd][k])));
+    };
+    const auto put = [&](int q, const float (&hn)[8], const uint32_t (&ob)[4]) {
+      if (!STEPS || (rs.flags & P_LAST)) store8(hout + rnd * 64 + e.part * 16 + q * 8, hn, e.wide);
+      // K atom 0 of the operand lives in P0, K atom 1 in place in A
+      uint8_t* dst = rnd == 0 ? e.smem + OFF_P + swz(e.row, e.part * 2 + q) : e.smem + OFF_A + CHUNK_BYTES + swz(e.row, e.part * 2 + q);
+      *reinterpret_cast<uint4*>(dst) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
+    };
+    if (STEPS || is_ship) {
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         const int col = rnd * 64 + e.part * 16 + q * 8;
         // u (bf16) back from the A operand (K atom rnd)
-        uint8_t* ua = e.smem + OFF_A + rnd * CHUNK_BYTES + swz(e.row, e.part * 2 + q);
-        const uint4 ub = *reinterpret_cast<const uint4*>(ua);
+        const uint4 ub = *reinterpret_cast<const uint4*>(e.smem + OFF_A + rnd * CHUNK_BYTES + swz(e.row, e.part * 2 + q));
         const uint32_t uw[4] = {ub.x, ub.y, ub.z, ub.w};
-        uint32_t ob[4];
         float hn[8];
+        uint32_t ob[4];
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           const float* table = s.decay_log2 + col + hf * 4;
@@ -732,24 +815,56 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
           const F2 dlv[2] = {f2(dl.x, dl.y), f2(dl.z, dl.w)}, abv[2] = {f2(ab.x, ab.y), f2(ab.z, ab.w)}, xbv[2] = {f2(xb.x, xb.y), f2(xb.z, xb.w)};
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
-            const int k = q * 8 + hf * 4 + 2 * i, j = hf * 4 + 2 * i, w = hf * 2 + i;
+            const int k = q * 8 + hf * 4 + 2 * i, w = hf * 2 + i;
             const F2 rg = sigmoid_twice_bf16(add(acc_pair(&rv[k]), abv[i])), ig = sigmoid_twice_bf16(add(acc_pair(&iv[k]), xbv[i]));
             // sigmoid(Lambda)^(8 r) = 2^(r * 8 log2 sigmoid(Lambda)); the table is part of the weight image
             const float2 ad = halves(mul(rg, dlv[i]));
             const F2 a = f2(ex2_fast(ad.x), ex2_fast(ad.y));
             const float2 rest = halves(mul(fma(a, f2(-1.f), one), add(one, a)));
             const F2 gate = f2(sqrt_fast(fmaxf(rest.x, kGateFloor)), sqrt_fast(fmaxf(rest.y, kGateFloor)));
-            const F2 next = fma(mul(a, keep), f2(hprev[rnd][q][j], hprev[rnd][q][j + 1]), mul(gate, mul(ig, unpack_bf16(uw[w]))));
-            const float2 n = halves(next);
-            hn[j] = n.x;
-            hn[j + 1] = n.y;
-            ob[w] = pack_bf16(mul(next, unpack_bf16(b2p[rnd][q * 4 + w])));
+            const F2 ak = mul(a, keep);
+            const F2 b = fma(ak, f2(hprev[rnd][q][k & 7], hprev[rnd][q][(k & 7) + 1]), mul(gate, mul(ig, unpack_bf16(uw[w]))));
+            if constexpr (STEPS) {
+              av[k >> 1] = ak;
+              bv[k >> 1] = b;
+            } else {
+              finish(b, k >> 1, hn + 2 * w, ob[w]);
+            }
           }
         }
-        store8(hout + col, hn, e.wide);
-        // branch operand of linear_out: K atom 0 lives in P0, K atom 1 in place in A
-        uint8_t* dst = rnd == 0 ? e.smem + OFF_P + swz(e.row, e.part * 2 + q) : ua;
-        *reinterpret_cast<uint4*>(dst) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
+        if constexpr (!STEPS) put(q, hn, ob);
+      }
+    }
+    if constexpr (STEPS) {
+      const int step = e.row & (chunk - 1);
+      const auto level = [&](int d, bool last) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float2 b = halves(bv[k]);
+          const F2 b_up = f2(__shfl_up_sync(0xffffffffu, b.x, d), __shfl_up_sync(0xffffffffu, b.y, d));
+          F2 a_up = one;
+          if (!last) {
+            const float2 a = halves(av[k]);
+            a_up = f2(__shfl_up_sync(0xffffffffu, a.x, d), __shfl_up_sync(0xffffffffu, a.y, d));
+          }
+          if (step >= d) {
+            bv[k] = fma(av[k], b_up, bv[k]);
+            av[k] = mul(av[k], a_up);
+          }
+        }
+      };
+#pragma unroll 1
+      for (int d = 1; 2 * d < chunk; d <<= 1) level(d, false);
+      level(chunk >> 1, true);   // nobody needs this level's products of a
+      if (is_ship) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float hn[8];
+          uint32_t ob[4];
+#pragma unroll
+          for (int w = 0; w < 4; ++w) finish(bv[q * 4 + w], q * 4 + w, hn + 2 * w, ob[w]);
+          put(q, hn, ob);
+        }
       }
     }
   }
@@ -882,53 +997,22 @@ __device__ __forceinline__ void prefetch_state(const float* hid, const uint8_t* 
 #pragma unroll
   for (int i = 0; i < 8; ++i) prefetch_line(p + 32 * i);
 }
-// Runs of consecutive token rows that make up the rows of a tile: f(first tile row, first token row of the step, rows), the
-// whole warp.
-template <class F>
-__device__ __forceinline__ void for_token_runs(const TrunkArgs& args, int eb, F f) {
-  const EnvMap& map = args.map;
-  const int lane = threadIdx.x & 31;
-  if (args.tile_env_begin) {
-    const int end = args.tile_env_begin[eb + 1];
-    int row = 0;
-    for (int k0 = args.tile_env_begin[eb]; k0 < end; k0 += 32) {
-      int first = 0, n = 0;
-      if (k0 + lane < end) {
-        const int env = args.tile_env_ids[k0 + lane];
-        first = map.tok_off[env];
-        n = map.tok_off[env + 1] - first;
-      }
-      for (int j = 0; j < min(32, end - k0); ++j) {
-        const int rows = __shfl_sync(0xffffffffu, n, j);
-        f(row, __shfl_sync(0xffffffffu, first, j), rows);
-        row += rows;
-      }
-    }
-  } else if (args.flat_rows) {
-    f(0, eb * TILE, min(TILE, map.total_tokens - eb * TILE));
-  } else {
-    const int env0 = eb * args.envs_per_tile;
-    f(0, env0 * map.tokens_per_env, min(args.envs_per_tile, map.n_envs - env0) * map.tokens_per_env);
-  }
-}
 // The row table of a pass: tile `tile` at timestep t.
-template <bool WHOLE>
+template <int MODE>
 __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int t, uint8_t* tab) {
   const EnvMap& map = args.map;
   const int lane = threadIdx.x & 31;
   const int grp = tile / args.env_tiles, eb = tile - grp * args.env_tiles;
-  const int group_row = (grp + t) * map.total_tokens;
   uint32_t* blocks = reinterpret_cast<uint32_t*>(tab + TAB_BLOCKS);
   float* bias = reinterpret_cast<float*>(tab + TAB_BIAS);
   const auto invalid = [&](int row) {
-    reinterpret_cast<int4*>(tab)[row] = make_int4(-1, 0, 0, 0);
+    reinterpret_cast<int4*>(tab)[row] = make_int4(-1, 0, -1, 0);
     bias[row] = kMaskedScore;
   };
-  // token `tok` of environment env, which has `ships` ships
-  const auto put = [&](int row, int env, int tok, int ships, int step_row, int hrow) {
-    uint32_t flags = P_VALID;
-    const int trow = group_row + step_row;
-    bias[row] = !args.alive || args.alive[trow] ? 0.f : kMaskedScore;
+  // token `tok` of environment env, which has `ships` ships, at timestep t
+  const auto put = [&](int row, int env, int tok, int ships, int step_row, int hrow, int t, uint32_t flags) {
+    const int trow = (grp + t) * map.total_tokens + step_row;
+    if (MODE != STEPS) bias[row] = !args.alive || args.alive[trow] ? 0.f : kMaskedScore;
     if (tok < ships) {
       // steps since the last episode boundary, as far as the conv looks back; before the call there was none
       uint32_t lags = BNB_CONV_KERNEL - 1;
@@ -945,7 +1029,19 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
     reinterpret_cast<int4*>(tab)[row] = make_int4(hrow, (int)flags, trow, 0);
   };
   int n_blocks = 0;
-  if (!WHOLE && args.flat_rows) {
+  if constexpr (MODE == STEPS) {
+#pragma unroll 1
+    for (int row = lane; row < TILE; row += 32) {
+      const int step = row & (args.chunk - 1), r = (eb * TILE + row) / args.chunk, time = t * args.chunk + step;
+      if (r < map.total_tokens && time < args.steps) {
+        const int env = map.env_of_token(r), tok = r - map.env_tok_begin(env);
+        put(row, env, tok, map.env_ship_count(env), r, map.env_ship_begin(env) + tok, time,
+            P_VALID | (step == args.chunk - 1 || time == args.steps - 1 ? P_LAST : 0u));
+      } else {
+        invalid(row);
+      }
+    }
+  } else if (MODE == ANY && args.flat_rows) {
     // plain 128-row slices of the token rows (programs without attention inside: the
     // environments are larger than a tile); the environment of a row is looked up
 #pragma unroll 1
@@ -953,7 +1049,7 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
       const int r = eb * TILE + row;
       if (r < map.total_tokens) {
         const int env = map.env_of_token(r), tok = r - map.env_tok_begin(env);
-        put(row, env, tok, map.env_ship_count(env), r, map.env_ship_begin(env) + tok);
+        put(row, env, tok, map.env_ship_count(env), r, map.env_ship_begin(env) + tok, t, P_VALID);
       } else {
         invalid(row);
       }
@@ -975,7 +1071,7 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
         const int env = __shfl_sync(0xffffffffu, my_env, j), tok0 = __shfl_sync(0xffffffffu, my_tok, j), n = __shfl_sync(0xffffffffu, my_n, j),
                   ship0 = __shfl_sync(0xffffffffu, my_ship, j), ships = __shfl_sync(0xffffffffu, my_ships, j);
         for (int i = lane; i < n; i += 32) {
-          put(first + i, env, i, ships, tok0 + i, ship0 + i);
+          put(first + i, env, i, ships, tok0 + i, ship0 + i, t, P_VALID);
           if ((i & 15) == 0) blocks[n_blocks + (i >> 4)] = (uint32_t)(first + i) | (uint32_t)first << 8 | (uint32_t)(n - 1) << 16;
         }
         first += n;
@@ -990,7 +1086,7 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
     for (int row = lane; row < TILE; row += 32) {
       const int el = row / NM, tok = row - el * NM;
       if (el < envs) {
-        put(row, env0 + el, tok, map.ships_per_env, (env0 + el) * NM + tok, (env0 + el) * map.ships_per_env + tok);
+        put(row, env0 + el, tok, map.ships_per_env, (env0 + el) * NM + tok, (env0 + el) * map.ships_per_env + tok, t, P_VALID);
         if ((tok & 15) == 0) blocks[el * per_env + (tok >> 4)] = (uint32_t)row | (uint32_t)(el * NM) << 8 | (uint32_t)(NM - 1) << 16;
       } else {
         invalid(row);
@@ -1001,26 +1097,34 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
   if (lane == 0) *reinterpret_cast<int*>(tab + TAB_COUNT) = n_blocks;
   __syncwarp();
 }
-// Tokens of a pass into L2.
-__device__ __forceinline__ void prefetch_tokens(const TrunkArgs& args, int tile, int t) {
-  const int lane = threadIdx.x & 31, row_bytes = args.io_bf16 ? D * 2 : D * 4;
-  const int grp = tile / args.env_tiles, group_row = (grp + t) * args.map.total_tokens;
-  for_token_runs(args, tile - grp * args.env_tiles, [&](int, int first, int n) {
-    const uint8_t* p = reinterpret_cast<const uint8_t*>(args.x) + (size_t)(group_row + first) * row_bytes;
-    for (int i = lane; i < n * (row_bytes / 128); i += 32) prefetch_line(p + 128 * i);
-  });
-}
-// bfloat16 tokens of a pass into the P area (free from a sublayer's out_proj or linear_out on), as two swizzled atoms.
-__device__ __forceinline__ void copy_tokens(const TrunkArgs& args, int tile, int t, uint32_t p_area) {
+// The tokens of a pass into L2, and bfloat16 ones into the P area (free from a sublayer's out_proj or linear_out on) as two
+// swizzled atoms: rows as the pass's table has them.
+__device__ __forceinline__ int row_of(const uint8_t* tab, int row) { return *reinterpret_cast<const int*>(tab + 16 * row + 8); }
+__device__ __forceinline__ void prefetch_tokens(const TrunkArgs& args, const uint8_t* tab) {
   const int lane = threadIdx.x & 31;
-  const int grp = tile / args.env_tiles, group_row = (grp + t) * args.map.total_tokens;
-  for_token_runs(args, tile - grp * args.env_tiles, [&](int row, int first, int n) {
-    const uint8_t* p = reinterpret_cast<const uint8_t*>(args.x) + (size_t)(group_row + first) * (2 * D);
-    for (int i = lane; i < n * 16; i += 32) {
-      const int c8 = i & 15;
-      cp_async16(p_area + (c8 >> 3) * CHUNK_BYTES + swz(row + (i >> 4), c8 & 7), p + 16 * i);
-    }
-  });
+  const uint8_t* x = reinterpret_cast<const uint8_t*>(args.x);
+  const int lines = args.io_bf16 ? 2 : 4;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int at = row_of(tab, lane + 32 * k);
+    if (at >= 0)
+      for (int l = 0; l < lines; ++l) prefetch_line(x + ((size_t)at * lines + l) * 128);
+  }
+}
+// (Eight rows' places are read before the first copy: one by one, each copy waited for its own, 7 000 cycles a tile.)
+__device__ __forceinline__ void copy_tokens(const TrunkArgs& args, const uint8_t* tab, uint32_t p_area) {
+  const int lane = threadIdx.x & 31, c8 = lane & 15;
+  const uint8_t* x = reinterpret_cast<const uint8_t*>(args.x) + 16 * c8;
+  p_area += (c8 >> 3) * CHUNK_BYTES;
+#pragma unroll 1
+  for (int row0 = lane >> 4; row0 < TILE; row0 += 16) {
+    int at[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) at[k] = row_of(tab, row0 + 2 * k);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (at[k] >= 0) cp_async16(p_area + swz(row0 + 2 * k, c8 & 7), x + (size_t)at[k] * (2 * D));
+  }
 }
 // What this lane has written and copied for the next pass: two arrivals on XFULL.
 __device__ __forceinline__ void hand_over(uint32_t bar) {
@@ -1084,9 +1188,7 @@ __device__ __forceinline__ void issue_temporal(Issuer& m, bool has_fields) {
 
 // ------------------------------------------------------------------ the kernel
 
-// WHOLE: programs of whole sublayers on tiles of whole environments, most calls by far; the code they do not need cost
-// them registers and instruction fetches.
-template <bool WHOLE>
+template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_constant__ TrunkArgs args) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // an offset: the compiler still knows it as shared memory
@@ -1103,7 +1205,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
   }
   // Both row tables start without rows: after a wait has run out they may be read before they are written.
   for (int i = tid; i < 2 * TAB_BYTES / 16; i += THREADS)
-    reinterpret_cast<int4*>(smem + OFF_TAB)[i] = make_int4(i % (TAB_BYTES / 16) < TILE ? -1 : 0, 0, 0, 0);
+    reinterpret_cast<int4*>(smem + OFF_TAB)[i] = i % (TAB_BYTES / 16) < TILE ? make_int4(-1, 0, -1, 0) : make_int4(0, 0, 0, 0);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 8 * B_COUNT);
   if (tid == 0) {
@@ -1206,8 +1308,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       T_MARK(t_start);
       const bool down = warp == DOWN_WARP;
       if (down && passes > 0) {
-        fill_table<WHOLE>(args, blockIdx.x, 0, smem + OFF_TAB);
-        if (args.io_bf16) copy_tokens(args, blockIdx.x, 0, m.sbase + OFF_P);
+        fill_table<MODE>(args, blockIdx.x, 0, smem + OFF_TAB);
+        if (args.io_bf16) copy_tokens(args, smem + OFF_TAB, m.sbase + OFF_P);
         hand_over(m.bars + 8 * B_XFULL);
         __syncwarp();
       }
@@ -1222,27 +1324,27 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
           const int type = (int)uniform((uint32_t)s_sub[si].type);
           if (down) {
             if (si + 1 == args.n_sub && pass + 1 < passes) {
-              prefetch_tokens(args, tile, t);
               wait_bar(m.bars + 8 * B_XFREE, pass & 1u, m.aborted, ST_TIMEOUT_OPERAND);
-              fill_table<WHOLE>(args, tile, t, smem + OFF_TAB + (~pass & 1) * TAB_BYTES);
+              fill_table<MODE>(args, tile, t, smem + OFF_TAB + (~pass & 1) * TAB_BYTES);
+              prefetch_tokens(args, smem + OFF_TAB + (~pass & 1) * TAB_BYTES);
             }
             __syncwarp();
-            const bool state_next = this_t == 0 && type != SUB_TEMPORAL && si + 1 < args.n_sub && s_sub[si + 1].type == SUB_TEMPORAL;
-            if (WHOLE || type != SUB_SPATIAL_PRE)
+            const bool state_next = MODE != STEPS && this_t == 0 && type != SUB_TEMPORAL && si + 1 < args.n_sub && s_sub[si + 1].type == SUB_TEMPORAL;
+            if (MODE != ANY || type != SUB_SPATIAL_PRE)
               issue_downs(m, state_next ? s_sub[si + 1].hid_in : nullptr, smem + OFF_TAB + (pass & 1) * TAB_BYTES);
             continue;
           }
-          if (type == SUB_TEMPORAL) {
+          if (MODE == STEPS || type == SUB_TEMPORAL) {
             issue_temporal(m, args.has_fields != 0);
           } else {
-            if (WHOLE || type != SUB_SPATIAL_POST) issue_qkv(m);
-            if (!WHOLE && type == SUB_SPATIAL_PRE) continue;
-            issue_out_proj(m, !WHOLE && type == SUB_SPATIAL_POST ? OFF_A : OFF_P);
+            if (MODE != ANY || type != SUB_SPATIAL_POST) issue_qkv(m);
+            if (MODE == ANY && type == SUB_SPATIAL_PRE) continue;
+            issue_out_proj(m, MODE == ANY && type == SUB_SPATIAL_POST ? OFF_A : OFF_P);
           }
           issue_gate_up(m, type == SUB_TEMPORAL ? TEMPORAL_FFN_PAIR : SPATIAL_FFN_PAIR);
         }
         if (down && pass + 1 < passes) {
-          if (args.io_bf16) copy_tokens(args, tile, t, m.sbase + OFF_P);
+          if (args.io_bf16) copy_tokens(args, smem + OFF_TAB + (~pass & 1) * TAB_BYTES, m.sbase + OFF_P);
           hand_over(m.bars + 8 * B_XFULL);
           __syncwarp();
         }
@@ -1331,10 +1433,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       for (int si = 0; si < args.n_sub; ++si) {
         const SubLayer& s = s_sub[si];
         const int type = s.type;
-        const bool temporal = type == SUB_TEMPORAL;
+        const bool temporal = MODE == STEPS || type == SUB_TEMPORAL;
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
-          if (WHOLE || half || type != SUB_SPATIAL_POST) {
+          if (MODE != ANY || half || type != SUB_SPATIAL_POST) {
             norm_to_A(e);
             post(e, B_OP0);
           }
@@ -1342,8 +1444,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
             ffn(e, temporal ? TEMPORAL_FFN_PAIR : SPATIAL_FFN_PAIR);
             break;
           }
-          if (temporal) run_temporal(e, s, rs, args.has_fields != 0, first_step ? s.hid_in : s.hid_out);
-          else if (WHOLE || type == SUB_SPATIAL) run_spatial(e, n_items, valid);
+          if (temporal) run_temporal<MODE == STEPS>(e, s, rs, args.has_fields != 0, first_step ? s.hid_in : s.hid_out, args.chunk);
+          else if (MODE != ANY || type == SUB_SPATIAL) run_spatial(e, n_items, valid);
           else if (type == SUB_SPATIAL_POST) run_spatial_post(e, s, rs.trow, valid);
           else {
             run_spatial_pre(e, s, rs.trow, valid);
@@ -1363,7 +1465,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
           asm volatile("bar.sync %0, 128;" ::"r"(3 + (warp & 3)) : "memory");   // the four warps of these rows
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const int at = __shfl_sync(0xffffffffu, valid ? rs.trow : -1, 8 * e.part + 2 * i + (lane >> 4));
+            const int at = __shfl_sync(0xffffffffu, rs.trow, 8 * e.part + 2 * i + (lane >> 4));
             const uint4 w = *reinterpret_cast<const uint4*>(smem + OFF_A + io_atom + swz(io_row(i), lane & 7));
             if (at >= 0) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(args.y) + (size_t)at * (2 * D) + (lane & 15) * 16) = w;
           }
@@ -1408,17 +1510,16 @@ int launch_pipelined(const TrunkArgs& a, cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BNB_ERR_NO_DEVICE;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(pipe::k_trunk_pipelined<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pipe::SMEM_BYTES) != cudaSuccess ||
-        cudaFuncSetAttribute(pipe::k_trunk_pipelined<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, pipe::SMEM_BYTES) != cudaSuccess)
-      return BNB_ERR_LAUNCH;
+    for (auto* k : {pipe::k_trunk_pipelined<pipe::ANY>, pipe::k_trunk_pipelined<pipe::WHOLE>, pipe::k_trunk_pipelined<pipe::STEPS>})
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, pipe::SMEM_BYTES) != cudaSuccess) return BNB_ERR_LAUNCH;
     configured[dev] = true;
   }
   const int grid = a.n_tiles < 148 ? a.n_tiles : 148;
   count_launch();
   bool whole = !a.flat_rows;
   for (int i = 0; i < a.n_sub; ++i) whole = whole && (a.sub[i].type == SUB_SPATIAL || a.sub[i].type == SUB_TEMPORAL);
-  if (whole) pipe::k_trunk_pipelined<true><<<grid, pipe::THREADS, pipe::SMEM_BYTES, st>>>(a);
-  else pipe::k_trunk_pipelined<false><<<grid, pipe::THREADS, pipe::SMEM_BYTES, st>>>(a);
+  const auto kernel = a.chunk ? pipe::k_trunk_pipelined<pipe::STEPS> : whole ? pipe::k_trunk_pipelined<pipe::WHOLE> : pipe::k_trunk_pipelined<pipe::ANY>;
+  kernel<<<grid, pipe::THREADS, pipe::SMEM_BYTES, st>>>(a);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
 }
 

@@ -49,7 +49,9 @@ struct TrunkArgs {
   const uint8_t* reset_env;
   EnvMap map;
   int n_groups;       // replication of the batch for the spatial fold (T for a sequence)
-  int t_loop;         // timesteps walked inside the kernel (temporal programs of a sequence)
+  int t_loop;         // passes over a tile: timesteps walked inside the kernel (temporal programs of a sequence), or chunks of them
+  int chunk;          // timesteps of a token in one tile (4, 8, 16 or 32), 0: tiles of one timestep
+  int steps;          // timesteps of the sequence (with chunks)
   int n_sub;
   int n_tiles;
   int envs_per_tile;

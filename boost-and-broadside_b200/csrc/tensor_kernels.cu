@@ -677,9 +677,38 @@ void debug_wait_test(int skip_op, int poll_limit) {
   g_debug_poll_limit = poll_limit;
 }
 
+// Tiles that the environments of a batch fill at one timestep, as many environments to a tile as fit.
+static long long full_tiles(const BnbBatch& b, bool flat) {
+  if (flat) return (b.total_tokens + TILE - 1) / TILE;
+  if (b.tok_off) return b.n_tiles;
+  const int per = TILE / b.tokens_per_env;
+  return (b.n_envs + per - 1) / per;
+}
+// Timesteps per tile of a temporal sublayer over T timesteps, or 0 for a walk over tiles of one timestep: the fewest passes
+// over the busiest SM, small chunks first (their scan has fewer levels).  A pass of the walk costs 1.4 of a chunk's (it moves the
+// state of 128 rows).  What stays with the walk: two or three steps of a batch that fills the chip.
+static int steps_per_tile(const BnbBatch& b, bool flat, int T) {
+  const auto rounds = [](long long tiles) { return (tiles + 147) / 148; };
+  long long best = rounds(full_tiles(b, flat)) * T * 7;   // in fifths
+  int chunk = 0;
+  for (int c = 4; c <= 32; c *= 2) {
+    const long long cost = rounds(((long long)b.total_tokens * c + TILE - 1) / TILE) * ((T + c - 1) / c) * 5;
+    if (cost < best) {
+      best = cost;
+      chunk = c;
+    }
+  }
+  return chunk;
+}
+
 static int launch(TrunkArgs& a, const BnbBatch& b, cudaStream_t st) {
   a.map = make_env_map(b);
-  if (a.flat_rows) {
+  if (a.chunk) {
+    a.tile_env_begin = nullptr;
+    a.flat_rows = 0;
+    a.envs_per_tile = 0;
+    a.env_tiles = (int)(((long long)b.total_tokens * a.chunk + TILE - 1) / TILE);
+  } else if (a.flat_rows) {
     a.tile_env_begin = nullptr;
     a.envs_per_tile = 0;
     a.env_tiles = (b.total_tokens + TILE - 1) / TILE;
@@ -828,6 +857,12 @@ struct Plan {
     a.reset_env = reset_env;
     a.n_groups = n_groups;
     a.t_loop = t_loop;
+    a.chunk = 0;
+    a.steps = t_loop;
+    if (t_loop > 1) {
+      a.chunk = steps_per_tile(b, split, t_loop);
+      if (a.chunk) a.t_loop = (t_loop + a.chunk - 1) / a.chunk;
+    }
     a.n_sub = n;
     a.flat_rows = split ? 1 : 0;
     a.io_bf16 = io_bf16 ? 1 : 0;
