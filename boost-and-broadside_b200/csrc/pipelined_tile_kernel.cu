@@ -1,29 +1,29 @@
 // The fused trunk kernel for sm_100a: one CTA per SM walks a tile of 128 token rows (whole
-// environments) through a program of spatial and temporal sublayers, with the residual stream
-// resident in tensor memory and three warp roles that only meet at mbarriers:
+// environments, or several timesteps of a token) through a program of spatial and temporal sublayers, with the residual
+// stream resident in tensor memory and four warp roles that only meet at mbarriers:
 //
 //   16 epilogue warps   four threads per tile row (thread (row, part): TMEM lane = row, a quarter
 //                       of whatever columns are being read).  RMSNorm, q|k|v staging, attention
 //                       (mma.sync), gelu(gate) * up, causal conv, RG-LRU gates and state update.
-//   2 issuing warps     issue every tcgen05.mma, one the down projections, one the rest.  They wait for "operand ready" (the
+//   1 issuing warp      issues every tcgen05.mma but the down projections.  It waits for "operand ready" (the
 //                       epilogue warps arrive on an mbarrier after fence.proxy.async) and for
 //                       "chunk landed" (the bulk copy's complete_tx), and signals "accumulator
 //                       ready" / "slot free" with tcgen05.commit.
+//   1 down warp         issues the down projections, and prepares the next pass: its row table, its tokens and the
+//                       recurrent state on their way to the SM.
 //   1 fetching warp     streams the pre-tiled weight image through a ring of nine 16 KB
 //                       slots with cp.async.bulk, following a static schedule.
 //
 //   TMEM  [0,128)    residual stream, fp32, lane = tile row (out_proj, linear_out and down_proj
 //                    accumulate straight into it)
-//         [128,512)  three 128-column accumulators.  q|k|v of all four heads fill them in one
-//                    round; the GatedMLP runs them as a three-deep pipeline: gate|up of chunk
-//                    c + 3 is issued as soon as chunk c has been read, so the tensor pipe works
-//                    on chunks c + 1 .. c + 3 while the epilogue warps turn chunk c into the bf16
-//                    operand of its down projection.
+//         [128,512)  three 128-column accumulators.  q, k and v fill them in one round; the GatedMLP uses two, one for
+//                    each half of the epilogue warps (even and odd chunks of 64 hidden columns), and the third for four
+//                    buffers of gated products, the A operands of the down projections.
 //
-//   SMEM  A (32 KB)  normed activations (K-major, 128-byte swizzle); q of all heads during
-//                    attention.   P (2 x 16 KB)  gelu(gate) * up, double buffered; attention
-//                    output; RG-LRU branch.   KV (64 KB)  keys and values of all heads during
-//                    attention, four more ring slots otherwise.   Ring (5 x 16 KB).
+//   SMEM  A (32 KB)  normed activations (K-major, 128-byte swizzle); rows of the result on their way out.
+//         P (2 x 16 KB)  q of all heads, then the attention output; RG-LRU branch; the next pass's tokens.
+//         KV (64 KB)  keys and values of all heads during attention, four more ring slots otherwise.
+//         Ring (5 x 16 KB).  Row tables of two passes.
 //
 // Every mbarrier wait is bounded: a wait that runs out records a code in the status word, later
 // waits give up at once, and the kernel drains and returns.
@@ -56,7 +56,8 @@ constexpr int OFF_KV = 65536;
 constexpr int OFF_RING = 131072;
 constexpr int OFF_SS = OFF_RING + RING_BYTES;                   // partial sums of squares [4][128]
 // What the rows of a pass are, twice (the pass at work and the next one): Place[128], then the blocks of 16 queries (first
-// row | first row of the environment << 8 | its tokens less one << 16), then the attention bias of each row as a key
+// row | first row of the environment << 8 | its tokens less one << 16 | its tokens << 24; environments of up to 8 tokens
+// share a block, and the second number is the block's rows less one), then the attention bias of each row as a key
 // (float, 16 of slack), then the number of blocks.
 constexpr int OFF_TAB = OFF_SS + 2048;
 constexpr int TAB_BLOCKS = 2048, TAB_BIAS = TAB_BLOCKS + 512, TAB_COUNT = TAB_BIAS + 576, TAB_BYTES = TAB_COUNT + 16;
@@ -65,20 +66,20 @@ constexpr int OFF_BAR = OFF_TAB + 2 * TAB_BYTES;
 constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
 
 // mbarrier indices
-// OP0: operand ready (epilogue warps -> issuing warp).  FFN[a]: the GatedMLP product in accumulator a is
-// written (the eight warps that own the chunk -> issuing warp); the next chunk of that accumulator is
-// issued after the wait, so a phase is never overtaken.  KVREL: the key/value area
+// OP0: operand ready (epilogue warps -> issuing warp).  REL[g]: gate|up of a chunk have been read from the accumulator of group
+// g (its eight warps -> issuing warp).  FFN[b]: a chunk's product stands in product buffer b (the eight warps that own the
+// chunk -> down-projection warp); PFREE[b]: its down projection is complete, twice in a GatedMLP.  KVREL: the key/value area
 // may take weights again (epilogue warps -> fetching warp).  FULL[s]: the weights of slot s have landed.
 // DONE[s]: the MMAs that read slot s are complete (tcgen05.commit) -- the fetching warp takes it as
 // "slot free", the epilogue warps as "accumulator ready" for gate|up of one chunk, whose slot is not
-// used again before they have seen it, and the issuing warp of gate|up as "accumulator free" for a down projection.
+// used again before they have seen it.
 // ACC: every MMA of a round is complete (one more commit per round).
 // EARLY: the first half of a temporal sublayer's gates is.  PARK: linear2's accumulator has been read (epilogue warps ->
 // issuing warp); FIELD: field_sub, multiplied into it then, is complete.  XFULL: the row table of the next pass is
 // written and its tokens have landed in the P area (down-projection warp -> epilogue warps); XFREE: the tokens have been read, and
 // nobody works on the pass before any more.  DRAIN: every MMA of the
 // CTA is complete (once per issuing warp, at the end).
-enum : int { B_OP0 = 0, B_FFN0, B_FFN1, B_FFN2, B_KVREL, B_PARK, B_XFREE, B_XFULL, B_DRAIN, B_ACC, B_EARLY, B_FIELD, B_FULL0, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
+enum : int { B_OP0 = 0, B_FFN0, B_FFN3 = B_FFN0 + 3, B_REL0, B_REL1, B_KVREL, B_PARK, B_XFREE, B_XFULL, B_DRAIN, B_ACC, B_EARLY, B_FIELD, B_PFREE0, B_FULL0 = B_PFREE0 + 4, B_DONE0 = B_FULL0 + N_SLOTS, B_COUNT = B_DONE0 + N_SLOTS };
 static_assert(B_COUNT * 8 + 8 <= 256, "barrier area");
 
 constexpr uint32_t COL_RESID = 0;
@@ -127,9 +128,9 @@ __device__ __forceinline__ void trace(Trace& t, int id) {
 #define TRACE(t, id)
 #endif
 
-// One ring operation as the fetching warp needs it: source of the first chunk (64 bits), byte distance
-// from it to the second chunk (0: a single), and slot (bits 0-2) | wait for the key/value area first (8).
-// Resolved once at kernel start, a thread per operation, so that a fetch is a dozen instructions.
+// One ring operation as the fetching warp needs it: source (64 bits), place in shared memory (relative to its start, a multiple
+// of 1 KB) | slot (bits 0-2) | wait for the key/value area first (8), bytes.  Resolved once at kernel start, a thread per
+// operation: the warp's time per operation bounds the GatedMLP (see the fetching loop).
 constexpr int MAX_SCHED = MAX_SUBLAYERS * 22;
 static_assert(MAX_SCHED <= THREADS, "one thread writes one entry");
 
@@ -143,6 +144,9 @@ static_assert(MAX_SCHED <= THREADS, "one thread writes one entry");
 // b + 3c + 2 (a single); fetched in the order GU0 GU1 GU2 D0 GU3 D1 GU4 D2 ... GU7 D5 D6 D7.
 constexpr uint32_t SPATIAL_FFN_PAIR = 1, TEMPORAL_FFN_PAIR = 0;   // pair slot of gate|up of chunk 0
 constexpr int FFN_OPS = 16;
+__device__ __forceinline__ uint32_t pair_offset(uint32_t slot) { return slot == 2 ? OFF_KV : OFF_RING + slot * 2 * CHUNK_BYTES; }
+__device__ __forceinline__ uint32_t single_offset(uint32_t i) { return i == 0 ? OFF_RING + 4 * CHUNK_BYTES : OFF_KV + (1 + i) * CHUNK_BYTES; }
+__device__ __forceinline__ uint32_t slot_offset(uint32_t slot) { return slot < 3 ? pair_offset(slot) : single_offset(slot - 3); }
 __device__ __forceinline__ int sublayer_ops(int type, bool has_fields) {
   return type == SUB_SPATIAL ? 4 + FFN_OPS : type == SUB_SPATIAL_PRE ? 3 : type == SUB_SPATIAL_POST ? 1 + FFN_OPS : (has_fields ? 6 : 5) + FFN_OPS;
 }
@@ -175,12 +179,8 @@ __device__ __forceinline__ uint4 sched_entry(const SubLayer& s, int op, bool has
     kvwait = s.type == SUB_SPATIAL && f == 1;
   }
   const unsigned long long src = reinterpret_cast<unsigned long long>(s.packed + (size_t)chunk * CHUNK_BYTES);
-  return make_uint4((uint32_t)src, (uint32_t)(src >> 32), pair ? CHUNK_BYTES : 0u, (uint32_t)slot | (kvwait ? 8u : 0u));
+  return make_uint4((uint32_t)src, (uint32_t)(src >> 32), slot_offset((uint32_t)slot) | (uint32_t)slot | (kvwait ? 8u : 0u), pair ? 2u * CHUNK_BYTES : (uint32_t)CHUNK_BYTES);
 }
-
-__device__ __forceinline__ uint32_t pair_offset(uint32_t slot) { return slot == 2 ? OFF_KV : OFF_RING + slot * 2 * CHUNK_BYTES; }
-__device__ __forceinline__ uint32_t single_offset(uint32_t i) { return i == 0 ? OFF_RING + 4 * CHUNK_BYTES : OFF_KV + (1 + i) * CHUNK_BYTES; }
-__device__ __forceinline__ uint32_t slot_offset(uint32_t slot) { return slot < 3 ? pair_offset(slot) : single_offset(slot - 3); }
 
 // Bounded wait of this kernel: as mbar_wait, but a wait that runs out only leaves its code in the CTA's abort word, which the
 // last thread out reports; two dozen waits are inlined here, and the kernel's code is what its warps stall on
@@ -351,14 +351,15 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* s) {
 }
 
 // GatedMLP on the A operand (already normed and posted on OP0): residual += down(gelu(gate) * up).
-// Chunk c: gate / 2 = acc[c % 3][0,64) (the image holds half the gate weights), up = acc[c % 3][64,128).  Two groups of
-// eight warps take turns (parts 0, 1 the even chunks, parts 2, 3 the odd ones), so that one group's waits and tensor-memory
-// latencies hide behind the other's arithmetic; a thread owns 32 of the 64 hidden columns of its row,
-// columns [32 (part & 1), +32), in two passes of 16; the second pass's columns are on their way during the first's arithmetic.
+// Two groups of eight warps take turns (parts 0, 1 the even chunks, parts 2, 3 the odd ones), so that one group's waits and
+// tensor-memory latencies hide behind the other's arithmetic.  A group has an accumulator of its own: gate / 2 (the image
+// holds half the gate weights) in columns [0,64), up in [64,128); a thread owns 32 of the 64 hidden columns of its row,
+// columns [32 (part & 1), +32).  As soon as both are in registers the accumulator takes the group's next chunk.
 //
-// The gated product stays in tensor memory as the A operand of the down projection: 16 k at a time
-// (8 columns of packed bf16 pairs) over the first half of 16 gate columns the thread has just read;
-// K step s of the MMA reads exactly the columns at 16 s.
+// The gated product becomes the A operand of the down projection in tensor memory, in one of four buffers of 32 columns
+// (column = two k as bfloat16), so that gate|up of a later chunk needn't wait for it: with the product over the gate columns it
+// had been read from, three accumulators in turn, a chunk was the third of a chain of 2 700 cycles (product, commit, arithmetic,
+// post, down projection, commit).
 __device__ __forceinline__ void gated_product(const uint32_t (&gv)[16], const uint32_t (&uv)[16], uint32_t dst) {
   uint32_t w8[8];
 #pragma unroll
@@ -367,7 +368,7 @@ __device__ __forceinline__ void gated_product(const uint32_t (&gv)[16], const ui
 }
 __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slot of chunk 0
   const uint32_t group = e.part >> 1;
-  uint32_t a = group;   // accumulator of the chunk
+  const uint32_t acc = e.lane_addr + COL_ACC0 + group * 128 + (e.part & 1) * 32;
   if (group) {   // past chunk 0
     e.par ^= 1u << slot;
     slot = slot == 2 ? 0 : slot + 1;
@@ -378,29 +379,33 @@ __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slo
     // gate|up of chunk 2 i + group; the slot's previous operation came before those of the two chunks in between
     wait_op(e, slot);
     T_BEGIN();
-    const uint32_t acc = e.lane_addr + COL_ACC0 + a * 128 + (e.part & 1) * 32;
+    const uint32_t buffer = 2 * (i & 1) + group;
     uint32_t gv[16], uv[16], gw[16], uw[16];
     tmem_ld16_nowait(acc, gv);
     tmem_ld16_nowait(acc + 64, uv);
-    tmem_wait_ld();
     tmem_ld16_nowait(acc + 16, gw);
     tmem_ld16_nowait(acc + 80, uw);
-    gated_product(gv, uv, acc);
     tmem_wait_ld();
-    gated_product(gw, uw, acc + 16);
+    tc_fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(e.bars + 8 * (B_REL0 + group));
+    // the buffer's previous product has been multiplied (its next one is this, so no phase is missed)
+    if (i >= 2) wait_bar(e.bars + 8 * (B_PFREE0 + buffer), 0, e.aborted, ST_TIMEOUT_ACC);
+    const uint32_t dst = e.lane_addr + COL_ACC2 + 32 * buffer + 16 * (e.part & 1);
+    gated_product(gv, uv, dst);
+    gated_product(gw, uw, dst + 8);
     tmem_wait_st();
     T_END(e.tacc, TE_FFN_MATH);
     // nothing of this operand is in shared memory: no proxy fence
     TRACE(e.tr, 201);
     tc_fence_before();
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive(e.bars + 8 * (B_FFN0 + a));
+    if ((threadIdx.x & 31) == 0) mbar_arrive(e.bars + 8 * (B_FFN0 + buffer));
     // two operations further: chunks c + 1 and c + 2, whose slots are this one's successors
     e.par ^= 1u << slot;
     slot = slot == 2 ? 0 : slot + 1;
     e.par ^= 1u << slot;
     slot = slot == 2 ? 0 : slot + 1;
-    a = a == 0 ? 2 : a - 1;   // (a + 2) mod 3
   }
   if (group) e.par ^= 1u << (slot == 0 ? 2 : slot - 1);   // there is no chunk 8
   T_WAITSLOT(e, TE_ACC_WAIT);
@@ -410,8 +415,99 @@ __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slo
 // Attention of every head and environment of the tile from the staged q (P area), k and v (KV
 // area), all in the swizzled operand layout (128 rows x 64 bf16 atoms; head h sits in atom h / 2,
 // columns 32 (h % 2) ..).  The four warps of part h serve head h, which they have staged themselves,
-// and take turns at the blocks of 16 query rows (each head from another warp on: warp & 3 is the scheduler); keys are
-// walked in blocks of 16 with a running maximum.  Output: bf16 into the P area as the A operand of out_proj, each block over its own q.
+// and take turns at the blocks of up to 16 query rows (each head from another warp on: warp & 3 is the scheduler).
+// Output: bf16 into the P area as the A operand of out_proj, each block over its own q.
+//
+// Environments of up to 16 tokens need no running maximum, and those of up to 8 share a block (keys of another environment score
+// -inf): 32 steps of 4096 x 8
+// tokens 5 730 -> 5 400 us.  Weights are normalised by the reciprocal (1 ulp, before the rounding to bfloat16): the division's code took 1.5 %
+// of a step.
+
+// A block of queries whose environments' keys are the block's own rows: block = first row | .. | rows less one << 16 | tokens of
+// an environment << 24.
+__device__ __forceinline__ void attend_block(const Epi& e, uint32_t block) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t atom = (uint32_t)(e.part >> 1) * CHUNK_BYTES;
+  const int c8h = (e.part & 1) * 4;
+  const uint32_t sQ = e.sbase + OFF_P + atom, sK = e.sbase + OFF_KV + atom, sV = sK + 2 * CHUNK_BYTES;
+  const float* key_bias = reinterpret_cast<const float*>(e.tab + TAB_BIAS);
+  const float c2 = 0.17677669529663687f * 1.4426950408889634f;  // log2(e) / sqrt(32): scores in the log2 domain
+  const int r0 = block & 255, n = (int)(block >> 16 & 255) + 1, size = (int)(block >> 24), last = r0 + n - 1;
+  uint32_t qa[2][4], kf[2][4], vf[2][4];
+  {
+    const int row = min(r0 + (lane & 7) + ((lane >> 3) & 1) * 8, last), krow = min(r0 + (lane >> 4) * 8 + (lane & 7), last);
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+      ldsm_x4(sQ + swz(row, c8h + ks * 2 + (lane >> 4)), qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3]);
+      ldsm_x4(sK + swz(krow, c8h + ks * 2 + ((lane >> 3) & 1)), kf[ks][0], kf[ks][1], kf[ks][2], kf[ks][3]);
+    }
+#pragma unroll
+    for (int np = 0; np < 2; ++np) ldsm_x4_t(sV + swz(row, c8h + np * 2 + (lane >> 4)), vf[np][0], vf[np][1], vf[np][2], vf[np][3]);
+  }
+  float sc[2][4];
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sc[nt][i] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks) {
+    mma_bf16(sc[0], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], kf[ks][0], kf[ks][1]);
+    mma_bf16(sc[1], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], kf[ks][2], kf[ks][3]);
+  }
+  // first key of the environment of query g, g + 8
+  const float per = rcp_fast((float)size);
+  const int lo0 = (int)(((float)min(g, n - 1) + 0.5f) * per) * size, lo1 = (int)(((float)min(g + 8, n - 1) + 0.5f) * per) * size;
+  float m0 = -INFINITY, m1 = -INFINITY;
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int j = nt * 8 + 2 * t + i;
+      // a dead key's bias (kMaskedScore) swallows its score: weight exactly 0 unless every key is dead, then uniform
+      const float bj = key_bias[r0 + j];
+      sc[nt][i] = (unsigned)(j - lo0) < (unsigned)size ? fmaf(sc[nt][i], c2, bj) : -INFINITY;
+      sc[nt][2 + i] = (unsigned)(j - lo1) < (unsigned)size ? fmaf(sc[nt][2 + i], c2, bj) : -INFINITY;
+      m0 = fmaxf(m0, sc[nt][i]);
+      m1 = fmaxf(m1, sc[nt][2 + i]);
+    }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+    m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+  }
+  float l0 = 0.f, l1 = 0.f;
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      sc[nt][i] = ex2_fast(sc[nt][i] - m0);
+      sc[nt][2 + i] = ex2_fast(sc[nt][2 + i] - m1);
+      l0 += sc[nt][i];
+      l1 += sc[nt][2 + i];
+    }
+  const uint32_t a0 = pack_bf16(sc[0][0], sc[0][1]), a1 = pack_bf16(sc[0][2], sc[0][3]);
+  const uint32_t a2 = pack_bf16(sc[1][0], sc[1][1]), a3 = pack_bf16(sc[1][2], sc[1][3]);
+  float acc[4][4];
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
+    mma_bf16(acc[nt], a0, a1, a2, a3, vf[nt >> 1][2 * (nt & 1)], vf[nt >> 1][2 * (nt & 1) + 1]);
+  }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, o);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+  }
+  const float i0 = rcp_fast(l0), i1 = rcp_fast(l1);
+  uint8_t* po = e.smem + OFF_P + atom;
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    if (g < n) *reinterpret_cast<uint32_t*>(po + swz(r0 + g, c8h + nt) + t * 4) = pack_bf16(acc[nt][0] * i0, acc[nt][1] * i0);
+    if (g + 8 < n) *reinterpret_cast<uint32_t*>(po + swz(r0 + g + 8, c8h + nt) + t * 4) = pack_bf16(acc[nt][2] * i1, acc[nt][3] * i1);
+  }
+}
+
 __device__ __forceinline__ void attention(Epi& e, int n_items) {
   TRACE(e.tr, 310);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -425,101 +521,108 @@ __device__ __forceinline__ void attention(Epi& e, int n_items) {
   const float c2 = 0.17677669529663687f * 1.4426950408889634f;  // log2(e) / sqrt(32): scores in the log2 domain
   for (int it = (warp + h) & 3; it < n_items; it += EPI_WARPS / 4) {
     const uint32_t block = blocks[it];
-    const int r0 = block & 255, e0 = block >> 8 & 255, n = (int)(block >> 16) + 1;   // first row; first tile row and size of the environment
-    const int last = e0 + n - 1;
-    uint32_t qa[2][4];
+    if ((block >> 16 & 255) < 16) {
+      attend_block(e, block);
+      continue;
+    }
+    // larger environments: keys are walked in blocks of 16 with a running maximum
     {
-      const int row = min(r0 + (lane & 7) + ((lane >> 3) & 1) * 8, last);
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks)
-        ldsm_x4(sQ + swz(row, c8h + ks * 2 + (lane >> 4)), qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3]);
-    }
-    const int nkb = (n + 15) >> 4;
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-    float acc[4][4];
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
-#pragma unroll 1
-    for (int kb = 0; kb < nkb; ++kb) {
-      float sc[2][4];
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) sc[nt][i] = 0.f;
-      const int krow = min(e0 + kb * 16 + (lane >> 4) * 8 + (lane & 7), last);
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        uint32_t b0, b1, b2, b3;
-        ldsm_x4(sK + swz(krow, c8h + ks * 2 + ((lane >> 3) & 1)), b0, b1, b2, b3);
-        mma_bf16(sc[0], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
-        mma_bf16(sc[1], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b2, b3);
+      const int r0 = block & 255, e0 = block >> 8 & 255, n = (int)(block >> 16 & 255) + 1;   // first row; first tile row and size of the environment
+      const int last = e0 + n - 1;
+      uint32_t qa[2][4];
+      {
+        const int row = min(r0 + (lane & 7) + ((lane >> 3) & 1) * 8, last);
+  #pragma unroll
+        for (int ks = 0; ks < 2; ++ks)
+          ldsm_x4(sQ + swz(row, c8h + ks * 2 + (lane >> 4)), qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3]);
       }
-      float bm0 = -INFINITY, bm1 = -INFINITY;
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int j = kb * 16 + nt * 8 + 2 * t + i;
-          const bool valid = j < n;
-          // a dead key's bias (kMaskedScore) swallows its score: weight exactly 0 unless every key is
-          // dead, then uniform; rows past the environment's last are no keys at all
-          const float bj = key_bias[e0 + j];
-          const float a = valid ? fmaf(sc[nt][i], c2, bj) : -INFINITY;
-          const float b = valid ? fmaf(sc[nt][2 + i], c2, bj) : -INFINITY;
-          sc[nt][i] = a;
-          sc[nt][2 + i] = b;
-          bm0 = fmaxf(bm0, a);
-          bm1 = fmaxf(bm1, b);
+      const int nkb = (n + 15) >> 4;
+      float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+      float acc[4][4];
+  #pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+  #pragma unroll
+        for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
+  #pragma unroll 1
+      for (int kb = 0; kb < nkb; ++kb) {
+        float sc[2][4];
+  #pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+  #pragma unroll
+          for (int i = 0; i < 4; ++i) sc[nt][i] = 0.f;
+        const int krow = min(e0 + kb * 16 + (lane >> 4) * 8 + (lane & 7), last);
+  #pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+          uint32_t b0, b1, b2, b3;
+          ldsm_x4(sK + swz(krow, c8h + ks * 2 + ((lane >> 3) & 1)), b0, b1, b2, b3);
+          mma_bf16(sc[0], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
+          mma_bf16(sc[1], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b2, b3);
         }
-      bm0 = fmaxf(bm0, __shfl_xor_sync(0xffffffffu, bm0, 1));
-      bm0 = fmaxf(bm0, __shfl_xor_sync(0xffffffffu, bm0, 2));
-      bm1 = fmaxf(bm1, __shfl_xor_sync(0xffffffffu, bm1, 1));
-      bm1 = fmaxf(bm1, __shfl_xor_sync(0xffffffffu, bm1, 2));
-      const float n0 = fmaxf(m0, bm0), n1 = fmaxf(m1, bm1);   // finite: every block holds a valid key
-      const float c0 = ex2_fast(m0 - n0), c1 = ex2_fast(m1 - n1); // 2^(-inf) = 0 on the first block
-      m0 = n0;
-      m1 = n1;
-      l0 *= c0;
-      l1 *= c1;
-#pragma unroll
+        float bm0 = -INFINITY, bm1 = -INFINITY;
+  #pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+  #pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int j = kb * 16 + nt * 8 + 2 * t + i;
+            const bool valid = j < n;
+            // a dead key's bias (kMaskedScore) swallows its score: weight exactly 0 unless every key is
+            // dead, then uniform; rows past the environment's last are no keys at all
+            const float bj = key_bias[e0 + j];
+            const float a = valid ? fmaf(sc[nt][i], c2, bj) : -INFINITY;
+            const float b = valid ? fmaf(sc[nt][2 + i], c2, bj) : -INFINITY;
+            sc[nt][i] = a;
+            sc[nt][2 + i] = b;
+            bm0 = fmaxf(bm0, a);
+            bm1 = fmaxf(bm1, b);
+          }
+        bm0 = fmaxf(bm0, __shfl_xor_sync(0xffffffffu, bm0, 1));
+        bm0 = fmaxf(bm0, __shfl_xor_sync(0xffffffffu, bm0, 2));
+        bm1 = fmaxf(bm1, __shfl_xor_sync(0xffffffffu, bm1, 1));
+        bm1 = fmaxf(bm1, __shfl_xor_sync(0xffffffffu, bm1, 2));
+        const float n0 = fmaxf(m0, bm0), n1 = fmaxf(m1, bm1);   // finite: every block holds a valid key
+        const float c0 = ex2_fast(m0 - n0), c1 = ex2_fast(m1 - n1); // 2^(-inf) = 0 on the first block
+        m0 = n0;
+        m1 = n1;
+        l0 *= c0;
+        l1 *= c1;
+  #pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          acc[nt][0] *= c0; acc[nt][1] *= c0;
+          acc[nt][2] *= c1; acc[nt][3] *= c1;
+        }
+  #pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+  #pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const float a = ex2_fast(sc[nt][i] - m0), b = ex2_fast(sc[nt][2 + i] - m1);
+            sc[nt][i] = a;
+            sc[nt][2 + i] = b;
+            l0 += a;
+            l1 += b;
+          }
+        const uint32_t a0 = pack_bf16(sc[0][0], sc[0][1]), a1 = pack_bf16(sc[0][2], sc[0][3]);
+        const uint32_t a2 = pack_bf16(sc[1][0], sc[1][1]), a3 = pack_bf16(sc[1][2], sc[1][3]);
+        const int vrow = min(e0 + kb * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), last);
+  #pragma unroll
+        for (int np = 0; np < 2; ++np) {
+          uint32_t b0, b1, b2, b3;
+          ldsm_x4_t(sV + swz(vrow, c8h + np * 2 + (lane >> 4)), b0, b1, b2, b3);
+          mma_bf16(acc[np * 2], a0, a1, a2, a3, b0, b1);
+          mma_bf16(acc[np * 2 + 1], a0, a1, a2, a3, b2, b3);
+        }
+      }
+      l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+      l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+      l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+      l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+      const float i0 = rcp_fast(l0), i1 = rcp_fast(l1);
+      const int q0 = r0 + g, q1 = r0 + g + 8;
+      uint8_t* po = e.smem + OFF_P + atom;
+  #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
-        acc[nt][0] *= c0; acc[nt][1] *= c0;
-        acc[nt][2] *= c1; acc[nt][3] *= c1;
+        if (q0 <= last) *reinterpret_cast<uint32_t*>(po + swz(q0, c8h + nt) + t * 4) = pack_bf16(acc[nt][0] * i0, acc[nt][1] * i0);
+        if (q1 <= last) *reinterpret_cast<uint32_t*>(po + swz(q1, c8h + nt) + t * 4) = pack_bf16(acc[nt][2] * i1, acc[nt][3] * i1);
       }
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const float a = ex2_fast(sc[nt][i] - m0), b = ex2_fast(sc[nt][2 + i] - m1);
-          sc[nt][i] = a;
-          sc[nt][2 + i] = b;
-          l0 += a;
-          l1 += b;
-        }
-      const uint32_t a0 = pack_bf16(sc[0][0], sc[0][1]), a1 = pack_bf16(sc[0][2], sc[0][3]);
-      const uint32_t a2 = pack_bf16(sc[1][0], sc[1][1]), a3 = pack_bf16(sc[1][2], sc[1][3]);
-      const int vrow = min(e0 + kb * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), last);
-#pragma unroll
-      for (int np = 0; np < 2; ++np) {
-        uint32_t b0, b1, b2, b3;
-        ldsm_x4_t(sV + swz(vrow, c8h + np * 2 + (lane >> 4)), b0, b1, b2, b3);
-        mma_bf16(acc[np * 2], a0, a1, a2, a3, b0, b1);
-        mma_bf16(acc[np * 2 + 1], a0, a1, a2, a3, b2, b3);
-      }
-    }
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    const float i0 = 1.0f / l0, i1 = 1.0f / l1;
-    const int q0 = r0 + g, q1 = r0 + g + 8;
-    uint8_t* po = e.smem + OFF_P + atom;
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      if (q0 <= last) *reinterpret_cast<uint32_t*>(po + swz(q0, c8h + nt) + t * 4) = pack_bf16(acc[nt][0] * i0, acc[nt][1] * i0);
-      if (q1 <= last) *reinterpret_cast<uint32_t*>(po + swz(q1, c8h + nt) + t * 4) = pack_bf16(acc[nt][2] * i1, acc[nt][3] * i1);
     }
   }
 }
@@ -905,9 +1008,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
 //
 // What bounds the GatedMLP is issue, not the tensor pipe: with one warp issuing everything, a chunk's two waits for
 // weights, one for its operand and twelve MMAs were a serial chain of 1 400 cycles where the pipe needs 770 (64 cycles per
-// 128 x 128 x 16).  So the down projections have a warp of their own, on another scheduler.  What the order of one thread's
-// MMAs gave for free is then a wait: gate|up of chunk c + 3 overwrites the accumulator that the down projection of chunk c
-// reads its operand from, and waits for its commit.
+// 128 x 128 x 16).  So the down projections have a warp of their own, on another scheduler.
 
 struct Issuer {
 #ifdef BNB_TRACE
@@ -919,8 +1020,7 @@ struct Issuer {
   uint32_t sbase, bars, tmem;
   uint32_t elected;    // 1 in the lane that issues
   uint32_t full_par;   // per-slot phase bits of the FULL barriers
-  uint32_t op_par;     // phase bits of OP0 and FFN0..2
-  uint32_t down_par;   // phase bits of the single slots' DONE barriers
+  uint32_t op_par;     // phase bits of OP0, FFN and REL
   volatile int* aborted;
 };
 
@@ -969,21 +1069,14 @@ __device__ __forceinline__ void commit_round(const Issuer& m) { commit_one(m, B_
 // gate|up of the eight chunks; slot: pair slot of chunk 0.
 __device__ __forceinline__ void issue_gate_up(Issuer& m, uint32_t slot) {
   wait_operand(m, B_OP0);
-  uint32_t a = 0;
 #pragma unroll 1
   for (uint32_t c = 0; c < 8; ++c) {
     wait_weights(m, slot);
-    if (c >= 3) {   // the down projection of chunk c - 3 has read this accumulator; its slot's next one comes after this product
-      wait_bar(m.bars + 8 * (B_DONE0 + 3 + a), (m.down_par >> a) & 1u, m.aborted, ST_TIMEOUT_ACC);
-      m.down_par ^= 1u << a;
-      tc_fence_after();
-      TRACE(m.tr, 404);
-    }
-    multiply_pair(m, slot, OFF_A, OFF_A + CHUNK_BYTES, COL_ACC0 + 128 * a, 0);
+    if (c >= 2) wait_operand(m, B_REL0 + (c & 1));   // gate|up of chunk c - 2 have been read
+    multiply_pair(m, slot, OFF_A, OFF_A + CHUNK_BYTES, COL_ACC0 + 128 * (c & 1), 0);
     slot = slot == 2 ? 0 : slot + 1;
-    a = a == 2 ? 0 : a + 1;
   }
-  m.down_par ^= 7;   // those of chunks 5, 6, 7 are not waited for here
+  m.op_par ^= 3u << B_REL0;   // those of chunks 6 and 7 are not waited for here: every operand posted from now on comes after them
 }
 // Rows that the tile owners need next are asked into L2 by the warp of the down projections, whose own work is a quarter of its
 // time.  As prefetches of the epilogue threads the state alone held their load pipe for 1 400 cycles of every tile and
@@ -1072,7 +1165,7 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
                   ship0 = __shfl_sync(0xffffffffu, my_ship, j), ships = __shfl_sync(0xffffffffu, my_ships, j);
         for (int i = lane; i < n; i += 32) {
           put(first + i, env, i, ships, tok0 + i, ship0 + i, t, P_VALID);
-          if ((i & 15) == 0) blocks[n_blocks + (i >> 4)] = (uint32_t)(first + i) | (uint32_t)first << 8 | (uint32_t)(n - 1) << 16;
+          if ((i & 15) == 0) blocks[n_blocks + (i >> 4)] = (uint32_t)(first + i) | (uint32_t)first << 8 | (uint32_t)(n - 1) << 16 | (uint32_t)n << 24;
         }
         first += n;
         n_blocks += (n + 15) >> 4;
@@ -1081,18 +1174,20 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
     for (int row = first + lane; row < TILE; row += 32) invalid(row);
   } else {
     const int NM = map.tokens_per_env, per_env = (NM + 15) >> 4;
+    const int share = NM <= 8 ? 16 / NM : 1;   // environments whose queries share a block (attend_two)
     const int env0 = eb * args.envs_per_tile, envs = min(args.envs_per_tile, map.n_envs - env0);
 #pragma unroll 1
     for (int row = lane; row < TILE; row += 32) {
       const int el = row / NM, tok = row - el * NM;
       if (el < envs) {
         put(row, env0 + el, tok, map.ships_per_env, (env0 + el) * NM + tok, (env0 + el) * map.ships_per_env + tok, t, P_VALID);
-        if ((tok & 15) == 0) blocks[el * per_env + (tok >> 4)] = (uint32_t)row | (uint32_t)(el * NM) << 8 | (uint32_t)(NM - 1) << 16;
+        if ((tok & 15) == 0 && el % share == 0)
+          blocks[el / share * per_env + (tok >> 4)] = (uint32_t)row | (uint32_t)(el * NM) << 8 | (uint32_t)(min(share, envs - el) * NM - 1) << 16 | (uint32_t)NM << 24;
       } else {
         invalid(row);
       }
     }
-    n_blocks = envs * per_env;
+    n_blocks = (envs + share - 1) / share * per_env;
   }
   if (lane == 0) *reinterpret_cast<int*>(tab + TAB_COUNT) = n_blocks;
   __syncwarp();
@@ -1132,7 +1227,7 @@ __device__ __forceinline__ void hand_over(uint32_t bar) {
   mbar_arrive(bar);
 }
 
-// The down projections of the eight chunks: A operand in tensor memory, K step k in the 8 columns at 16 k of the accumulator.
+// The down projections of the eight chunks: A operand in tensor memory, K step k in the 8 columns at 8 k of the buffer.
 // next_hid: the state that the following sublayer reads (null: none, or it is at hand), asked for on the way.
 __device__ __forceinline__ void issue_downs(Issuer& m, const float* next_hid, const uint8_t* tab) {
   constexpr uint32_t idesc = instr_desc(128);
@@ -1140,13 +1235,14 @@ __device__ __forceinline__ void issue_downs(Issuer& m, const float* next_hid, co
 #pragma unroll 1
   for (uint32_t c = 0; c < 8; ++c) {
     wait_weights(m, 3 + a);
-    wait_operand(m, B_FFN0 + a);   // product of chunk c written, accumulator a = c % 3 read
+    wait_operand(m, B_FFN0 + (c & 3));   // product of chunk c written
     T_MARK(tw);
     const uint32_t b_lo = uniform(desc_lo(m.sbase + single_offset(a)));
-    const uint32_t a_col = m.tmem + COL_ACC0 + 128 * a;
+    const uint32_t a_col = m.tmem + COL_ACC2 + 32 * (c & 3);
 #pragma unroll
-    for (uint32_t k = 0; k < 4; ++k) mma_one<true>(m.elected, m.tmem + COL_RESID, a_col + 16 * k, b_lo + 2 * k, idesc, 1u);
+    for (uint32_t k = 0; k < 4; ++k) mma_one<true>(m.elected, m.tmem + COL_RESID, a_col + 8 * k, b_lo + 2 * k, idesc, 1u);
     commit_one(m, B_DONE0 + 3 + a);
+    commit_one(m, B_PFREE0 + (c & 3));
     T_SINCE(m.tacc, TM_ISSUE, tw);
     TRACE(m.tr, 430);
     if (next_hid) prefetch_state(next_hid, tab, 16 * (int)c);
@@ -1212,7 +1308,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     s_aborted[0] = (*args.status != 0) ? -1 : 0;
     s_aborted[1] = args.poll_limit > 0 ? args.poll_limit : DEFAULT_POLL_LIMIT;
     mbar_init(smem_u32(&bars[B_OP0]), EPI_WARPS);
-    for (int i = B_FFN0; i <= B_FFN2; ++i) mbar_init(smem_u32(&bars[i]), EPI_WARPS / 2);
+    for (int i = B_FFN0; i <= B_REL1; ++i) mbar_init(smem_u32(&bars[i]), EPI_WARPS / 2);
     mbar_init(smem_u32(&bars[B_KVREL]), EPI_WARPS);
     mbar_init(smem_u32(&bars[B_PARK]), EPI_WARPS);
     mbar_init(smem_u32(&bars[B_XFREE]), EPI_WARPS);
@@ -1252,13 +1348,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       trace_init(ltr, args.status, 2);
       if ((tid & 31) != 0) ltr.n = 1500;
 #endif
+      // A chunk of the GatedMLP takes two operations, so what one takes here, instruction after instruction of a lone warp, is
+      // half of the least a chunk can take (770 cycles would keep the tensor pipe full).  One copy for a pair (its K halves are neighbours in the image and in the slot), the
+      // next entry read ahead, addresses from the table: 8192 x 12 tokens 586 -> 566 us.
       int op = 0;
+      uint4 en = s_sched[0];
       for (int pass = 0; pass < passes; ++pass)
         for (int i = 0; i < len; ++i, ++op) {
-          const uint4 en = s_sched[i];
-          const uint32_t slot = uniform(en.w & 7u);
+          const uint4 now = en;
+          en = s_sched[i + 1 < len ? i + 1 : 0];
+          const uint32_t slot = now.z & 7u;
           T_MARK(tw);
-          if (en.w & 8u) {
+          if (now.z & 8u) {
             wait_bar(bar0 + 8 * B_KVREL, kv_par, s_aborted, ST_TIMEOUT_FREE);
             kv_par ^= 1u;
           }
@@ -1268,18 +1369,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
           // Once a wait of this CTA has run out nothing is in step any more: stop fetching.  Arming a
           // FULL barrier again before its previous copy has landed would arrive on it twice in one
           // phase, which is undefined; the other roles' waits give up at once and the kernel drains.
-          if (__any_sync(0xffffffffu, *static_cast<volatile int*>(s_aborted))) { pass = passes; break; }
+          if (*static_cast<volatile int*>(s_aborted)) { pass = passes; break; }
           T_SINCE(tacc, TL_FREE_WAIT, tw);
           TRACE(ltr, 500 + slot);
-          const uint32_t full = bar0 + 8 * (B_FULL0 + slot);
-          const uint32_t dst = sbase + slot_offset(slot);
           if (elected && op != skip_op) {   // skip_op: test hook, this operation's weights never arrive
-            const uint8_t* src = reinterpret_cast<const uint8_t*>(((unsigned long long)en.y << 32) | en.x);
-            mbar_expect_tx(full, en.z ? 2 * CHUNK_BYTES : CHUNK_BYTES);
-            bulk_g2s(dst, src, CHUNK_BYTES, full);
-            if (en.z) bulk_g2s(dst + CHUNK_BYTES, src + en.z, CHUNK_BYTES, full);
+            const uint32_t full = bar0 + 8 * (B_FULL0 + slot);
+            mbar_expect_tx(full, now.w);
+            bulk_g2s(sbase + (now.z & ~15u), reinterpret_cast<const void*>(((unsigned long long)now.y << 32) | now.x), now.w, full);
           }
-          __syncwarp();
         }
 #ifdef BNB_TIMING
       tacc[TL_TOTAL] = clock64() - t_start;
@@ -1296,7 +1393,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       m.elected = elect_one();
       m.full_par = 0;
       m.op_par = 0;
-      m.down_par = 0;
       m.aborted = s_aborted;
 #ifdef BNB_TRACE
       trace_init(m.tr, args.status, warp == MMA_WARP ? 1 : 3);

@@ -108,11 +108,6 @@ struct Args {
   int* host_status;
 };
 
-__device__ __forceinline__ float rcp_fast(float v) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-  return r;
-}
 // Phi(x) and exp(-x^2 / 2) for two x: erf by formula 7.1.26 of Abramowitz and Stegun (absolute error 1.5e-7),
 // whose exponential is the density's too.
 __device__ __forceinline__ F2 normal_cdf(F2 x, F2& e) {
