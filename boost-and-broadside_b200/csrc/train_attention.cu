@@ -3,8 +3,8 @@
 // One CTA per environment-step, one warp per head, every row staged once in shared memory with 16-byte
 // asynchronous copies and written back as whole rows.  Its floor is the memory traffic of q|k|v (1.5 KB per
 // token) and its gradient; what bounds it is shared-memory and load latency: 8192 environment-steps of 8
-// tokens take 38 us forward (DRAM 37 % of peak, issue slots 52 % busy, 57 % of the warps) and 95 us for the gradient
-// (26 %, 49 %, and 24 % of the warps at 128 registers).  The kernels it replaces read rows element by element (one
+// tokens take 38 us forward (DRAM 37 % of peak, issue slots 52 % busy, 57 % of the warps) and 60 us for the gradient
+// (64 registers without bullets, where 128 held 24 % of the warps and it took 95).  The kernels it replaces read rows element by element (one
 // thread per query, or eight lanes per head), ran at 2.2 - 2.6 TB/s on environments of 8 tokens and took 425 /
 // 575 us (forward / gradient) for 1536 environment-steps of 12 tokens with 80 bullet slots, most of it
 // on slots that are not in use (45 / 99 us here, averaged over the sublayers that read them and those that do not).  Here only the slots in use are read.
@@ -191,20 +191,21 @@ __global__ void __launch_bounds__(THREADS) k_env_attn_fwd(const Call c) {
   }
 }
 
-// Gradient.  Lane (qs, sub) holds key sub's share of d k and d v over the queries of its group qs.
-template <int LPP>
-__global__ void __launch_bounds__(THREADS, 4) k_env_attn_bwd(const Call c) {
+// Gradient.
+// (Without bullets the sums of 32 channels a lane that their keys need would only cost registers, and so CTAs.)
+template <int LPP, bool BULLETS>
+__global__ void __launch_bounds__(THREADS, BULLETS || LPP == 32 ? 4 : LPP == 16 ? 6 : 8) k_env_attn_bwd(const Call c) {
   extern __shared__ __align__(16) char raw[];
   constexpr int QPW = 32 / LPP, CPL = DH / LPP;
   Smem s;
-  carve(raw, c.n, c.kvb ? c.nb : 0, true, &s);
+  carve(raw, c.n, BULLETS ? c.nb : 0, true, &s);
   const int h = threadIdx.x >> 5, lane = threadIdx.x & 31, qs = lane / LPP, sub = lane % LPP;
   const int n = c.n;
   const size_t g = blockIdx.x, tok0 = g * n;
   rows_in<3 * D>(s.rows, LDQ, c.qkv + tok0 * 3 * D, n);
   rows_in<D>(s.d_o, LDO, c.d_o + tok0 * D, n);
   int keys = 0;
-  if (c.kvb) {
+  if constexpr (BULLETS) {
     keys = key_list(c.bactive ? c.bactive + g * c.nb : nullptr, c.nb, s.list, s.count);
     for (int i = threadIdx.x; i < n * LDO; i += THREADS) s.dq[i] = 0.f;
     for (int i = threadIdx.x; i < n * H; i += THREADS) { s.m[i] = -INFINITY; s.l[i] = s.s[i] = 0.f; }
@@ -218,9 +219,8 @@ __global__ void __launch_bounds__(THREADS, 4) k_env_attn_bwd(const Call c) {
   float* k = q + D;
   float* v = q + 2 * D;
   const float* go = s.d_o + h * DH;
-  float dk[DH], dv[DH];
-
-  if (keys) {
+  if (BULLETS && keys) {
+    float dk[DH], dv[DH];
     // one sweep for the softmax statistics of every query, one for the gradients
     for (int k0 = 0; k0 < keys; k0 += BLOCK) {
       const int kn = min(BLOCK, keys - k0);
@@ -290,11 +290,10 @@ __global__ void __launch_bounds__(THREADS, 4) k_env_attn_bwd(const Call c) {
 
   const bool key = sub < n;
   const bool dead = key && c.alive && !c.alive[tok0 + sub];
-#pragma unroll
-  for (int d = 0; d < DH; ++d) dk[d] = dv[d] = 0.f;
-  for (int q0 = 0; q0 < n; q0 += QPW) {
-    const int i = q0 + qs, ic = min(i, n - 1);
-    float* qi = q + ic * LDQ;
+  // probability and score gradient of (query, key sub)
+  const auto weights = [&](int i, float& p, float& ds) {
+    const int ic = min(i, n - 1);
+    const float* qi = q + ic * LDQ;
     const float* gi = go + ic * LDO;
     float sc = -INFINITY, dp = 0.f;
     if (key) {
@@ -306,44 +305,95 @@ __global__ void __launch_bounds__(THREADS, 4) k_env_attn_bwd(const Call c) {
     const float l = seg_sum<LPP>(e);
     const float lse = mx + logf(l);
     const float delta = seg_sum<LPP>(e / l * dp);   // <d out, out>
-    const float p = key && i < n ? expf(sc - lse) : 0.f;
-    const float ds = p * (dp - delta) * SCALE;
-#pragma unroll
-    for (int d4 = 0; d4 < DH / 4; ++d4) {
-      const float4 a = ld4(qi + 4 * d4), b = ld4(gi + 4 * d4);
-      dk[4 * d4] = fmaf(ds, a.x, dk[4 * d4]); dk[4 * d4 + 1] = fmaf(ds, a.y, dk[4 * d4 + 1]);
-      dk[4 * d4 + 2] = fmaf(ds, a.z, dk[4 * d4 + 2]); dk[4 * d4 + 3] = fmaf(ds, a.w, dk[4 * d4 + 3]);
-      dv[4 * d4] = fmaf(p, b.x, dv[4 * d4]); dv[4 * d4 + 1] = fmaf(p, b.y, dv[4 * d4 + 1]);
-      dv[4 * d4 + 2] = fmaf(p, b.z, dv[4 * d4 + 2]); dv[4 * d4 + 3] = fmaf(p, b.w, dv[4 * d4 + 3]);
-    }
+    p = key && i < n ? expf(sc - lse) : 0.f;
+    ds = p * (dp - delta) * SCALE;
+  };
+  // d q of query i from its score gradients, one per lane; it takes the place of q
+  const auto query_gradient = [&](int i, float ds) {
     float dq[CPL];
 #pragma unroll
-    for (int d = 0; d < CPL; ++d) dq[d] = keys && i < n ? s.dq[i * LDO + h * DH + sub * CPL + d] : 0.f;
+    for (int d = 0; d < CPL; ++d) dq[d] = BULLETS && keys && i < n ? s.dq[i * LDO + h * DH + sub * CPL + d] : 0.f;
     for (int j = 0; j < n; ++j) {
       const float dsj = __shfl_sync(0xffffffffu, ds, qs * LPP + j);
       const float* kj = k + j * LDQ + sub * CPL;
 #pragma unroll
       for (int d = 0; d < CPL; ++d) dq[d] = fmaf(dsj, kj[d], dq[d]);
     }
-    __syncwarp();            // this head's q of these queries is done with: its gradient takes its place
+    __syncwarp();            // this head's q of these queries is done with
     if (i < n)
 #pragma unroll
-      for (int d = 0; d < CPL; ++d) qi[sub * CPL + d] = dq[d];
+      for (int d = 0; d < CPL; ++d) q[i * LDQ + sub * CPL + d] = dq[d];
+  };
+  if constexpr (LPP < 32) {
+    // Every query's weights first (ROUNDS a lane), then lane (qs, sub) sums CH = LPP channels of d k and d v of key sub over all
+    // queries: 2 CH accumulators and a broadcast per query, where shares of 32 channels each over the group's queries took 64
+    // accumulators and as many sums over the groups at the end: 32 768 environment-steps of 8 tokens 343 -> 237 us.
+    constexpr int ROUNDS = LPP / QPW, CH = LPP;
+    float p[ROUNDS], ds[ROUNDS];
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+      p[r] = ds[r] = 0.f;
+      if (r * QPW < n) weights(r * QPW + qs, p[r], ds[r]);
+    }
+    float gk[CH], gv[CH];
+#pragma unroll
+    for (int d = 0; d < CH; ++d) gk[d] = gv[d] = 0.f;
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r)
+#pragma unroll
+      for (int g2 = 0; g2 < QPW; ++g2) {
+        const int i = r * QPW + g2;
+        if (i >= n) break;
+        const float pi = __shfl_sync(0xffffffffu, p[r], g2 * LPP + sub), di = __shfl_sync(0xffffffffu, ds[r], g2 * LPP + sub);
+        const float* qi = q + i * LDQ + qs * CH;
+        const float* gi = go + i * LDO + qs * CH;
+#pragma unroll
+        for (int d4 = 0; d4 < CH / 4; ++d4) {
+          const float4 a = ld4(qi + 4 * d4), b = ld4(gi + 4 * d4);
+          gk[4 * d4] = fmaf(di, a.x, gk[4 * d4]); gk[4 * d4 + 1] = fmaf(di, a.y, gk[4 * d4 + 1]);
+          gk[4 * d4 + 2] = fmaf(di, a.z, gk[4 * d4 + 2]); gk[4 * d4 + 3] = fmaf(di, a.w, gk[4 * d4 + 3]);
+          gv[4 * d4] = fmaf(pi, b.x, gv[4 * d4]); gv[4 * d4 + 1] = fmaf(pi, b.y, gv[4 * d4 + 1]);
+          gv[4 * d4 + 2] = fmaf(pi, b.z, gv[4 * d4 + 2]); gv[4 * d4 + 3] = fmaf(pi, b.w, gv[4 * d4 + 3]);
+        }
+      }
+    __syncwarp();            // this head's q has been read
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r)
+      if (r * QPW < n) query_gradient(r * QPW + qs, ds[r]);
+    __syncwarp();            // and so have its k and v
+    if (key)
+#pragma unroll
+      for (int d4 = 0; d4 < CH / 4; ++d4) {
+        *reinterpret_cast<float4*>(k + sub * LDQ + qs * CH + 4 * d4) = make_float4(gk[4 * d4], gk[4 * d4 + 1], gk[4 * d4 + 2], gk[4 * d4 + 3]);
+        *reinterpret_cast<float4*>(v + sub * LDQ + qs * CH + 4 * d4) = make_float4(gv[4 * d4], gv[4 * d4 + 1], gv[4 * d4 + 2], gv[4 * d4 + 3]);
+      }
+  } else {
+    float dk[DH], dv[DH];
+#pragma unroll
+    for (int d = 0; d < DH; ++d) dk[d] = dv[d] = 0.f;
+    for (int i = 0; i < n; ++i) {
+      float p, ds;
+      weights(i, p, ds);
+      const float* qi = q + i * LDQ;
+      const float* gi = go + i * LDO;
+#pragma unroll
+      for (int d4 = 0; d4 < DH / 4; ++d4) {
+        const float4 a = ld4(qi + 4 * d4), b = ld4(gi + 4 * d4);
+        dk[4 * d4] = fmaf(ds, a.x, dk[4 * d4]); dk[4 * d4 + 1] = fmaf(ds, a.y, dk[4 * d4 + 1]);
+        dk[4 * d4 + 2] = fmaf(ds, a.z, dk[4 * d4 + 2]); dk[4 * d4 + 3] = fmaf(ds, a.w, dk[4 * d4 + 3]);
+        dv[4 * d4] = fmaf(p, b.x, dv[4 * d4]); dv[4 * d4 + 1] = fmaf(p, b.y, dv[4 * d4 + 1]);
+        dv[4 * d4 + 2] = fmaf(p, b.z, dv[4 * d4 + 2]); dv[4 * d4 + 3] = fmaf(p, b.w, dv[4 * d4 + 3]);
+      }
+      query_gradient(i, ds);
+    }
+    __syncwarp();
+    if (key)
+#pragma unroll
+      for (int d4 = 0; d4 < DH / 4; ++d4) {
+        *reinterpret_cast<float4*>(k + sub * LDQ + 4 * d4) = make_float4(dk[4 * d4], dk[4 * d4 + 1], dk[4 * d4 + 2], dk[4 * d4 + 3]);
+        *reinterpret_cast<float4*>(v + sub * LDQ + 4 * d4) = make_float4(dv[4 * d4], dv[4 * d4 + 1], dv[4 * d4 + 2], dv[4 * d4 + 3]);
+      }
   }
-#pragma unroll
-  for (int o = LPP; o < 32; o <<= 1)
-#pragma unroll
-    for (int d = 0; d < DH; ++d) {
-      dk[d] += __shfl_xor_sync(0xffffffffu, dk[d], o);
-      dv[d] += __shfl_xor_sync(0xffffffffu, dv[d], o);
-    }
-  __syncwarp();
-  if (key && qs == 0)
-#pragma unroll
-    for (int d4 = 0; d4 < DH / 4; ++d4) {
-      *reinterpret_cast<float4*>(k + sub * LDQ + 4 * d4) = make_float4(dk[4 * d4], dk[4 * d4 + 1], dk[4 * d4 + 2], dk[4 * d4 + 3]);
-      *reinterpret_cast<float4*>(v + sub * LDQ + 4 * d4) = make_float4(dv[4 * d4], dv[4 * d4 + 1], dv[4 * d4 + 2], dv[4 * d4 + 3]);
-    }
   __syncthreads();
   rows_out<3 * D>(c.dqkv + tok0 * 3 * D, s.rows, LDQ, n);
 }
@@ -372,9 +422,8 @@ int forward(const Call& c, cudaStream_t st) {
 }
 int backward(const Call& c, cudaStream_t st) {
   if (c.G <= 0) return 0;
-  if (c.n <= 8) return launch(k_env_attn_bwd<8>, c, true, st);
-  if (c.n <= 16) return launch(k_env_attn_bwd<16>, c, true, st);
-  return launch(k_env_attn_bwd<32>, c, true, st);
+  if (c.kvb) return c.n <= 8 ? launch(k_env_attn_bwd<8, true>, c, true, st) : c.n <= 16 ? launch(k_env_attn_bwd<16, true>, c, true, st) : launch(k_env_attn_bwd<32, true>, c, true, st);
+  return c.n <= 8 ? launch(k_env_attn_bwd<8, false>, c, true, st) : c.n <= 16 ? launch(k_env_attn_bwd<16, false>, c, true, st) : launch(k_env_attn_bwd<32, false>, c, true, st);
 }
 
 }  // namespace train_attn
