@@ -10,7 +10,7 @@
 // it took 73 us for the active rows of 8192 environments of 80 bullets.
 #include "bullet_kv.h"
 
-#include "launch_count.h"
+#include "launch_after.h"
 #include "tensor_kernels.h"
 #include "tile_rows.cuh"
 
@@ -180,10 +180,7 @@ int bullet_kv(const void* rows, bool rows_bf16, int n_rows, const int* index, co
   }
   const KvArgs a{rows, index, n_rows_dev, n_rows, image, kvb, status, host_status_word(st)};
   const int tiles = (n_rows + TILE - 1) / TILE, grid = tiles < 148 ? tiles : 148;
-  count_launch();
-  if (rows_bf16) k_bullet_kv<true><<<grid, THREADS, KV_BYTES, st>>>(a);
-  else k_bullet_kv<false><<<grid, THREADS, KV_BYTES, st>>>(a);
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+  return launch_after(rows_bf16 ? k_bullet_kv<true> : k_bullet_kv<false>, dim3(grid), THREADS, KV_BYTES, st, a);
 }
 
 }  // namespace tensor

@@ -13,7 +13,7 @@
 // twice for the norm, three heads of 65 536 rows took 139 us and take 67, one of 16 384 rows 39 and 14, one of 128 rows no less.
 #include "head_tiles.h"
 
-#include "launch_count.h"
+#include "launch_after.h"
 #include "tensor_kernels.h"
 #include "tile_rows.cuh"
 
@@ -52,7 +52,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
   constexpr int OUT = M::OUT;
   const MlpChain& chain = a.call.chain[blockIdx.y];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // operands: eight k of a row per thread and turn; rows of w2 past out_store are zero
+  wait_for_previous();
+  // operands: eight k of a row per thread and turn, several turns' loads under way; rows of w2 past out_store are zero
+#pragma unroll 4
   for (int i = tid; i < HIDDEN * 16; i += THREADS) {
     const int r = i >> 4, g = i & 15;
     uint4 v;
@@ -66,6 +68,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
     }
     *reinterpret_cast<uint4*>(smem + (g >> 3) * M::W1_ATOM + swz(r, g & 7)) = v;
   }
+#pragma unroll 4
   for (int i = tid; i < OUT * 32; i += THREADS) {
     const int r = i >> 5, g = i & 31;
     *reinterpret_cast<uint4*>(smem + M::W2 + (g >> 3) * M::W2_ATOM + swz(r, g & 7)) =
@@ -319,11 +322,9 @@ int head_tiles(const MlpCall& call, int n_chains, int out_dim, cudaStream_t st) 
   }
   const Args a{call, host_status_word(st)};
   const int tiles = (call.n_rows + TILE - 1) / TILE, per_chain = 148 / n_chains;
-  count_launch();
   const dim3 grid(tiles < per_chain ? tiles : per_chain, n_chains);
-  if (out_dim == 32) k_head_tiles<false><<<grid, THREADS, Map<false>::BYTES, st>>>(a);
-  else k_head_tiles<true><<<grid, THREADS, Map<true>::BYTES, st>>>(a);
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+  return out_dim == 32 ? launch_after(k_head_tiles<false>, grid, THREADS, Map<false>::BYTES, st, a)
+                       : launch_after(k_head_tiles<true>, grid, THREADS, Map<true>::BYTES, st, a);
 }
 
 }  // namespace mlp

@@ -24,7 +24,7 @@
 
 #include "common.cuh"
 #include "head_tiles.h"
-#include "launch_count.h"
+#include "launch_after.h"
 #include "tensor_common.cuh"
 
 namespace bnb {
@@ -107,6 +107,8 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
   const float* __restrict__ w2 = chain.w2;
   const float* __restrict__ g2 = chain.g2;
   extern __shared__ __align__(16) uint8_t sm[];
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   const Layout L = layout(in_pad, hidden, out_dim);
   __nv_bfloat16* W1 = reinterpret_cast<__nv_bfloat16*>(sm + L.w1);
   __nv_bfloat16* W2 = reinterpret_cast<__nv_bfloat16*>(sm + L.w2);
@@ -463,9 +465,7 @@ int run(const MlpCall& call, int n_chains, int in_pad, int hidden, int out_dim, 
   const int want = (n_units + L.warps - 1) / L.warps;
   // a CTA fills an SM and stages its weights once: the chains of a call share the SMs out
   const int per_chain = (sms + n_chains - 1) / n_chains;
-  count_launch();
-  kernel<<<dim3(want < per_chain ? want : per_chain, n_chains), 32 * L.warps, L.total, st>>>(call);
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+  return launch_after(kernel, dim3(want < per_chain ? want : per_chain, n_chains), 32 * L.warps, L.total, st, call);
 }
 
 int encoder_mlp_bf16(const float* w1, const float* b1, const float* g1, const float* w2, const float* b2, const float* g2,

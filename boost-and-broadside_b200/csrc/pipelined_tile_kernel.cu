@@ -29,7 +29,7 @@
 // waits give up at once, and the kernel drains and returns.
 //
 // Reference arithmetic: models/yemong/attention.py:76-169, models/yemong/griffin.py:67-317.
-#include "launch_count.h"
+#include "launch_after.h"
 #include "tensor_common.cuh"
 #include "tensor_kernels.h"
 
@@ -1305,7 +1305,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 8 * B_COUNT);
   if (tid == 0) {
-    s_aborted[0] = (*args.status != 0) ? -1 : 0;
+    s_aborted[0] = 0;
     s_aborted[1] = args.poll_limit > 0 ? args.poll_limit : DEFAULT_POLL_LIMIT;
     mbar_init(smem_u32(&bars[B_OP0]), EPI_WARPS);
     for (int i = B_FFN0; i <= B_REL1; ++i) mbar_init(smem_u32(&bars[i]), EPI_WARPS / 2);
@@ -1325,6 +1325,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  let_next_start();
+  wait_for_previous();
+  if (tid == 0 && *args.status != 0) *static_cast<volatile int*>(s_aborted) = -1;
   const int my_tiles = blockIdx.x < args.n_tiles ? (args.n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
   const int passes = my_tiles * args.t_loop;
 
@@ -1611,12 +1614,10 @@ int launch_pipelined(const TrunkArgs& a, cudaStream_t st) {
     configured[dev] = true;
   }
   const int grid = a.n_tiles < 148 ? a.n_tiles : 148;
-  count_launch();
   bool whole = !a.flat_rows;
   for (int i = 0; i < a.n_sub; ++i) whole = whole && (a.sub[i].type == SUB_SPATIAL || a.sub[i].type == SUB_TEMPORAL);
   const auto kernel = a.chunk ? pipe::k_trunk_pipelined<pipe::STEPS> : whole ? pipe::k_trunk_pipelined<pipe::WHOLE> : pipe::k_trunk_pipelined<pipe::ANY>;
-  kernel<<<grid, pipe::THREADS, pipe::SMEM_BYTES, st>>>(a);
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+  return launch_after(kernel, dim3(grid), pipe::THREADS, pipe::SMEM_BYTES, st, a);
 }
 
 }  // namespace tensor

@@ -10,7 +10,7 @@
 #include "policy_tail.h"
 
 #include "common.cuh"
-#include "launch_count.h"
+#include "launch_after.h"
 #include "tensor_common.cuh"
 
 namespace bnb {
@@ -47,6 +47,8 @@ __device__ __forceinline__ int team_of(const Ships& s, size_t e, int n) {
 // One block per (team, head): q = bf16(Wq_h seed), folded query = Wk_h^T q / sqrt(32).
 __global__ void __launch_bounds__(128) k_fold_query(const float* __restrict__ seeds, const float* __restrict__ in_proj, float* __restrict__ qk) {
   __shared__ float q[DH];
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   const int t = blockIdx.x / H, h = blockIdx.x % H;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float4 sv = *reinterpret_cast<const float4*>(seeds + t * D + lane * 4);
@@ -95,6 +97,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_team_rows(const Ships s, const f
                                                           const float* __restrict__ out_w, const float* __restrict__ norm_w,
                                                           __nv_bfloat16* __restrict__ rows) {
   extern __shared__ __align__(16) uint8_t sm[];
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   __nv_bfloat16* P = reinterpret_cast<__nv_bfloat16*>(sm + OFF_P);
   __nv_bfloat16* O = reinterpret_cast<__nv_bfloat16*>(sm + OFF_O);
   float* R = reinterpret_cast<float*>(sm + OFF_R);
@@ -102,6 +106,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_team_rows(const Ships s, const f
   float* has = reinterpret_cast<float*>(sm + OFF_HAS);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* sc = reinterpret_cast<float*>(sm + OFF_SC) + (size_t)warp * s.ships * H;
+#pragma unroll 4
   for (int i = tid; i < 2 * D * (D / 4); i += THREADS) {
     const int w = i / (D * (D / 4)), j = i - w * D * (D / 4), r = j / (D / 4), q = j % (D / 4);
     const float4 v = *reinterpret_cast<const float4*>((w ? out_w : in_proj + (size_t)2 * D * D) + (size_t)r * D + q * 4);
@@ -253,6 +258,8 @@ __global__ void __launch_bounds__(128) k_finish(const Ships s, const __nv_bfloat
                                                 int64_t* __restrict__ action, __nv_bfloat16* __restrict__ logprob,
                                                 const __nv_bfloat16* __restrict__ win, int n_win, const WinCols cols,
                                                 __nv_bfloat16* __restrict__ value, int value_ld) {
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= s.n_envs * s.ships) return;
   float lg[12];
@@ -311,12 +318,9 @@ int team_rows(const Ships& s, const float* seeds, const float* in_proj_w, const 
   const size_t smem = OFF_SC + (size_t)WARPS * s.ships * H * sizeof(float);
   if (cudaFuncSetAttribute(k_team_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return BNB_ERR_LAUNCH;
   float* qk = static_cast<float*>(scratch);
-  count_launch();
-  k_fold_query<<<2 * H, 128, 0, st>>>(seeds, in_proj_w, qk);
+  if (const int rc = launch_after(k_fold_query, dim3(2 * H), 128, 0, st, seeds, in_proj_w, qk)) return rc;
   const int rounds = (s.n_envs + ENVS - 1) / ENVS;
-  count_launch();
-  k_team_rows<<<rounds < 148 ? rounds : 148, THREADS, smem, st>>>(s, qk, in_proj_w, out_w, norm_w, rows);
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+  return launch_after(k_team_rows, dim3(rounds < 148 ? rounds : 148), THREADS, smem, st, s, qk, in_proj_w, out_w, norm_w, rows);
 }
 
 int finish(const Ships& s, const __nv_bfloat16* logits, const float* uniforms, int64_t* action, __nv_bfloat16* logprob,
@@ -325,9 +329,7 @@ int finish(const Ships& s, const __nv_bfloat16* logits, const float* uniforms, i
   if (n <= 0) return BNB_OK;
   WinCols wc{};
   for (int i = 0; i < n_win && i < 32; ++i) wc.c[i] = cols[i];
-  count_launch();
-  k_finish<<<(n + 127) / 128, 128, 0, st>>>(s, logits, uniforms, action, logprob, win, n_win, wc, value, value_ld);
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+  return launch_after(k_finish, dim3((n + 127) / 128), 128, 0, st, s, logits, uniforms, action, logprob, win, n_win, wc, value, value_ld);
 }
 
 }  // namespace tail

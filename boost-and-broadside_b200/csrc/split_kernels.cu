@@ -126,8 +126,6 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackJobs j
 
 // Programmatic dependence: everything an earlier launch wrote is visible after the wait.  The trigger comes
 // after it, so a launch that has started knows that the one before the one before it is complete.
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 struct Waits { int* status; int* host_status; int weights_early; };   // weights_early: the images are older than the launch before
 

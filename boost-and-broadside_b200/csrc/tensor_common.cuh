@@ -302,6 +302,13 @@ __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v 
 // 128-row x 64-column bf16 atom with the 128-byte swizzle.
 __device__ __forceinline__ uint32_t swz(int r, int c8) { return (uint32_t)(r * 128 + ((c8 ^ (r & 7)) << 4)); }
 
+// ------------------------------------------------------------------ programmatic dependence (launch_after.h)
+//
+// let_next_start comes after the CTA's tensor memory is allocated (a successor on the same SM that allocated it first would
+// wait for this kernel, and this kernel for it); nothing in global memory is read or written before wait_for_previous.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ------------------------------------------------------------------ issuing from a whole warp
 //
 // A warp that issues tensor-core work runs with the same values in every lane and lets one elected lane

@@ -20,7 +20,7 @@
 #include <vector>
 
 #include "common.cuh"
-#include "launch_count.h"
+#include "launch_after.h"
 
 #include "tensor_common.cuh"
 
@@ -140,6 +140,8 @@ struct PackJobs {
 };
 __global__ void k_pack_trunk(const __grid_constant__ PackJobs jobs) {
   const int j = blockIdx.y;
+  let_next_start();
+  wait_for_previous();
   if (jobs.status && j == 0 && blockIdx.x == 0 && threadIdx.x == 0) *jobs.status = 0;
   if (j < jobs.n_spatial) {
     const BnbSpatialWeights& w = jobs.sw[j];
@@ -275,6 +277,8 @@ __global__ void __launch_bounds__(256) k_attention_flash(const __nv_bfloat16* __
                                                          const __nv_bfloat16* __restrict__ kvb,
                                                          const int* __restrict__ env_off, int nb) {
   extern __shared__ __align__(16) uint8_t fs[];
+  let_next_start();
+  wait_for_previous();
   const int env_g = env_base + blockIdx.x, hd0 = blockIdx.y * hpc;
   const int grp = env_g / map.n_envs, e = env_g - grp * map.n_envs;
   const size_t tok0 = (size_t)grp * map.total_tokens + map.env_tok_begin(e);
@@ -361,6 +365,8 @@ __global__ void __launch_bounds__(256) k_attention_flash(const __nv_bfloat16* __
 
 // one warp per environment: cnt[e] = number of active slots
 __global__ void __launch_bounds__(256) k_bullet_count(const uint8_t* __restrict__ active, int n_env, int nb, int* __restrict__ cnt) {
+  let_next_start();
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   for (int e = blockIdx.x * 8 + (threadIdx.x >> 5); e < n_env; e += gridDim.x * 8) {
     int c = 0;
@@ -374,6 +380,8 @@ __global__ void __launch_bounds__(256) k_bullet_count(const uint8_t* __restrict_
 }
 // one CTA: env_off = exclusive scan of cnt, in place (env_off[n_env] = total)
 __global__ void __launch_bounds__(1024) k_bullet_scan(int* __restrict__ env_off, int n_env) {
+  let_next_start();
+  wait_for_previous();
   __shared__ int warp_sum[32];
   __shared__ int carry;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -411,6 +419,8 @@ __global__ void __launch_bounds__(1024) k_bullet_scan(int* __restrict__ env_off,
 // one warp per environment: the active slots of environment e, in order, at idx[env_off[e]...]
 __global__ void __launch_bounds__(256) k_bullet_fill(const uint8_t* __restrict__ active, int n_env, int nb,
                                                      const int* __restrict__ env_off, int* __restrict__ idx) {
+  let_next_start();
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   for (int e = blockIdx.x * 8 + (threadIdx.x >> 5); e < n_env; e += gridDim.x * 8) {
     int off = env_off[e];
@@ -430,6 +440,8 @@ __global__ void __launch_bounds__(256) k_bullet_fill(const uint8_t* __restrict__
 constexpr int SMALL_ENVS = 256;
 __global__ void __launch_bounds__(1024) k_bullet_compact(const uint8_t* __restrict__ active, int n_env, int nb, int* __restrict__ env_off,
                                                          int* __restrict__ idx) {
+  let_next_start();
+  wait_for_previous();
   __shared__ int off[SMALL_ENVS], warp_sum[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int e = warp; e < n_env; e += 32) {
@@ -613,9 +625,7 @@ int pack_trunk(const BnbSpatialWeights* spatial, int n_spatial, const BnbTempora
       if (!temporal[t0].packed) return BNB_ERR_NULL_POINTER;
       jobs.tw[jobs.n_temporal++] = temporal[t0];
     }
-    count_launch();
-    k_pack_trunk<<<dim3(24, jobs.n_spatial + jobs.n_temporal), 256, 0, st>>>(jobs);
-    if (cudaGetLastError() != cudaSuccess) return BNB_ERR_LAUNCH;
+    if (const int rc = launch_after(k_pack_trunk, dim3(24, jobs.n_spatial + jobs.n_temporal), 256, 0, st, jobs)) return rc;
   }
   return BNB_OK;
 }
@@ -792,27 +802,17 @@ static int launch_attention(const __nv_bfloat16* qkv, const uint8_t* alive, __nv
     const int idle = (items + w - 1) / w * w - items;
     if (idle < best_idle) { best_idle = idle; n_warps = w; }
   }
-  count_launch();
-  k_attention_flash<<<grid, 32 * n_warps, smem, st>>>(qkv, alive, o, make_env_map(b), env_base, hpc, kvb, env_off, nb);
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+  return launch_after(k_attention_flash, grid, 32 * n_warps, smem, st, qkv, alive, o, make_env_map(b), env_base, hpc, kvb, env_off, nb);
 }
 
 // env_off / idx of the active bullets of n_env environments (see the compaction kernels).
 static int launch_compact(const uint8_t* active, int n_env, int nb, int* env_off, int* idx, cudaStream_t st) {
   if (n_env <= 0) return BNB_OK;
-  if (n_env <= SMALL_ENVS) {
-    count_launch();
-    k_bullet_compact<<<1, 1024, 0, st>>>(active, n_env, nb, env_off, idx);
-    return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
-  }
+  if (n_env <= SMALL_ENVS) return launch_after(k_bullet_compact, dim3(1), 1024, 0, st, active, n_env, nb, env_off, idx);
   const int blocks = (n_env + 7) / 8 < 148 * 8 ? (n_env + 7) / 8 : 148 * 8;
-  count_launch();
-  k_bullet_count<<<blocks, 256, 0, st>>>(active, n_env, nb, env_off);
-  count_launch();
-  k_bullet_scan<<<1, 1024, 0, st>>>(env_off, n_env);
-  count_launch();
-  k_bullet_fill<<<blocks, 256, 0, st>>>(active, n_env, nb, env_off, idx);
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_LAUNCH;
+  if (const int rc = launch_after(k_bullet_count, dim3(blocks), 256, 0, st, active, n_env, nb, env_off)) return rc;
+  if (const int rc = launch_after(k_bullet_scan, dim3(1), 1024, 0, st, env_off, n_env)) return rc;
+  return launch_after(k_bullet_fill, dim3(blocks), 256, 0, st, active, n_env, nb, env_off, idx);
 }
 
 // Accumulates sublayers into tile-kernel launches.  In split mode (environments larger than

@@ -120,7 +120,7 @@ __device__ __forceinline__ Frame open_frame(uint8_t* at, int* status, int* host_
   static_assert(N <= 28, "barrier area");
   Frame f{reinterpret_cast<uint64_t*>(at), reinterpret_cast<uint32_t*>(at + 8 * 28), reinterpret_cast<int*>(at + 8 * 29)};
   if (threadIdx.x == 0) {
-    f.aborted[0] = *status != 0 ? 1 : 0;
+    f.aborted[0] = 0;
     f.aborted[1] = DEFAULT_POLL_LIMIT;
     *reinterpret_cast<int**>(&f.aborted[2]) = host_status;
 #pragma unroll
@@ -134,6 +134,9 @@ __device__ __forceinline__ Frame open_frame(uint8_t* at, int* status, int* host_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  let_next_start();
+  wait_for_previous();
+  if (threadIdx.x == 0 && *status != 0) *static_cast<volatile int*>(f.aborted) = 1;
   return f;
 }
 constexpr int FRAME_BYTES = 256;
