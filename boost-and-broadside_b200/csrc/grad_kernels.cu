@@ -31,7 +31,8 @@
 
 #include "common.cuh"
 #include "host_calls.h"
-#include "launch_count.h"
+#include "launch_after.h"
+#include "tensor_common.cuh"
 #include "train_attention.h"
 #include "train_linear.h"
 #include "train_mlp.h"
@@ -728,6 +729,8 @@ __device__ __forceinline__ float gelu_grad(float v) {
 
 // h = gelu(g) * u, four elements per thread
 __global__ void k_gelu_mul_fwd(const float4* __restrict__ g, const float4* __restrict__ u, float4* __restrict__ h, size_t n4) {
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
     const float4 a = g[i], b = u[i];
     h[i] = make_float4(gelu_erf(a.x) * b.x, gelu_erf(a.y) * b.y, gelu_erf(a.z) * b.z, gelu_erf(a.w) * b.w);
@@ -736,6 +739,8 @@ __global__ void k_gelu_mul_fwd(const float4* __restrict__ g, const float4* __res
 
 // dg = dh * u * gelu'(g), du = dh * gelu(g).  dg may alias g, du may alias dh (or u).
 __global__ void k_gelu_mul_bwd(const float4* g, const float4* u, const float4* dh, float4* dg, float4* du, size_t n4) {
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
     const float4 a = g[i], b = u[i], d = dh[i];
     dg[i] = make_float4(d.x * b.x * gelu_grad(a.x), d.y * b.y * gelu_grad(a.y), d.z * b.z * gelu_grad(a.z),
@@ -812,6 +817,8 @@ __global__ void __launch_bounds__(256) k_colsum(const float* __restrict__ a, flo
 // token tensor (groups of NM rows) and a compact buffer.  D4 = D / 4.
 __global__ void k_gather_rows(const float4* __restrict__ full, float4* __restrict__ compact, size_t n_rows, int D4,
                               int per_grp, int NM, int n0) {
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_rows * D4; i += (size_t)gridDim.x * blockDim.x) {
     const size_t q = i / D4;
     const int c = (int)(i - q * D4);
@@ -822,6 +829,8 @@ __global__ void k_gather_rows(const float4* __restrict__ full, float4* __restric
 }
 __global__ void k_scatter_rows(const float4* __restrict__ compact, float4* __restrict__ full, size_t n_rows, int D4,
                                int per_grp, int NM, int n0) {
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_rows * D4; i += (size_t)gridDim.x * blockDim.x) {
     const size_t q = i / D4;
     const int c = (int)(i - q * D4);
@@ -1226,6 +1235,8 @@ struct ShipGeom {
 __global__ void __launch_bounds__(256) k_conv_fwd(const float* __restrict__ b1, const float* __restrict__ hid,
                                                   const float* __restrict__ cw, const float* __restrict__ cb,
                                                   float* __restrict__ u, ShipGeom gm) {
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)gm.Rr * gm.D) return;
   const int s = (int)(idx / gm.D), d = (int)(idx - (size_t)s * gm.D);
@@ -1279,6 +1290,8 @@ __global__ void __launch_bounds__(256) k_scan_fwd(const float* __restrict__ za, 
                                                   const float* __restrict__ u, const float* __restrict__ hid,
                                                   const float* __restrict__ log_lambda, const float* __restrict__ b2,
                                                   float* __restrict__ hs, float* __restrict__ m, ShipGeom gm) {
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)gm.Rr * gm.D) return;
   const int s = (int)(idx / gm.D), d = (int)(idx - (size_t)s * gm.D);
@@ -1304,6 +1317,8 @@ __global__ void __launch_bounds__(256) k_scan_fwd(const float* __restrict__ za, 
 // State after the last step: h_T and the last three padded conv inputs (griffin.py:271-275).
 __global__ void __launch_bounds__(256) k_final_state(const float* __restrict__ hs, const float* __restrict__ b1,
                                                      const float* __restrict__ hid, float* __restrict__ hid_out, ShipGeom gm) {
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)gm.Rr * gm.D) return;
   const int s = (int)(idx / gm.D), d = (int)(idx - (size_t)s * gm.D);
@@ -1325,6 +1340,8 @@ __global__ void __launch_bounds__(256) k_scan_bwd(float* za, float* zx, const fl
                                                   const float* __restrict__ d_hid_out, float* __restrict__ d_hid_in,
                                                   const float* __restrict__ log_lambda, float* __restrict__ d_log_lambda,
                                                   ShipGeom gm) {
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   __shared__ float s_dl[MAXW];
   if ((int)threadIdx.x < gm.D) s_dl[threadIdx.x] = 0.f;
   __syncthreads();
@@ -1377,6 +1394,8 @@ __global__ void __launch_bounds__(256) k_conv_bwd(const float* __restrict__ du, 
                                                   float* __restrict__ d_hid_in, const float* __restrict__ cw,
                                                   float* __restrict__ db1, float* __restrict__ d_cw, float* __restrict__ d_cb,
                                                   ShipGeom gm) {
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   __shared__ float s_w[MAXW * 4], s_b[MAXW];
   for (int i = threadIdx.x; i < gm.D * 4; i += blockDim.x) s_w[i] = 0.f;
   if ((int)threadIdx.x < gm.D) s_b[threadIdx.x] = 0.f;
@@ -1578,16 +1597,14 @@ void rmsnorm_bwd(const Ctx& c, const float* x, const float* g, const float* inv,
 }
 void gelu_mul_fwd(const Ctx& c, const float* g, const float* u, float* h, size_t n) {
   if (!n) return;
-  count_launch();
-  k_gelu_mul_fwd<<<blocks_for(n / 4, 256), 256, 0, c.st>>>(reinterpret_cast<const float4*>(g), reinterpret_cast<const float4*>(u),
-                                                           reinterpret_cast<float4*>(h), n / 4);
+  c.note(launch_after(k_gelu_mul_fwd, dim3(blocks_for(n / 4, 256)), 256, 0, c.st, reinterpret_cast<const float4*>(g),
+                      reinterpret_cast<const float4*>(u), reinterpret_cast<float4*>(h), n / 4));
 }
 void gelu_mul_bwd(const Ctx& c, const float* g, const float* u, const float* dh, float* dg, float* du, size_t n) {
   if (!n) return;
-  count_launch();
-  k_gelu_mul_bwd<<<blocks_for(n / 4, 256), 256, 0, c.st>>>(reinterpret_cast<const float4*>(g), reinterpret_cast<const float4*>(u),
-                                                           reinterpret_cast<const float4*>(dh), reinterpret_cast<float4*>(dg),
-                                                           reinterpret_cast<float4*>(du), n / 4);
+  c.note(launch_after(k_gelu_mul_bwd, dim3(blocks_for(n / 4, 256)), 256, 0, c.st, reinterpret_cast<const float4*>(g),
+                      reinterpret_cast<const float4*>(u), reinterpret_cast<const float4*>(dh), reinterpret_cast<float4*>(dg),
+                      reinterpret_cast<float4*>(du), n / 4));
 }
 void colsum(const Ctx& c, const float* a, float* out, size_t rows, int N) {
   if (!rows) return;
@@ -1852,17 +1869,13 @@ int spatial_bwd(const Ctx& c, const BnbSpatialWeights& w, const BnbSpatialGrads&
 
 void gather(const Ctx& c, const float* full, float* compact, size_t rows, int per_grp, int NM, int n0) {
   if (!rows) return;
-  count_launch();
-  k_gather_rows<<<blocks_for(rows * (c.D / 4), 256), 256, 0, c.st>>>(reinterpret_cast<const float4*>(full),
-                                                                    reinterpret_cast<float4*>(compact), rows, c.D / 4,
-                                                                    per_grp, NM, n0);
+  c.note(launch_after(k_gather_rows, dim3(blocks_for(rows * (c.D / 4), 256)), 256, 0, c.st, reinterpret_cast<const float4*>(full),
+                      reinterpret_cast<float4*>(compact), rows, c.D / 4, per_grp, NM, n0));
 }
 void scatter(const Ctx& c, const float* compact, float* full, size_t rows, int per_grp, int NM, int n0) {
   if (!rows) return;
-  count_launch();
-  k_scatter_rows<<<blocks_for(rows * (c.D / 4), 256), 256, 0, c.st>>>(reinterpret_cast<const float4*>(compact),
-                                                                     reinterpret_cast<float4*>(full), rows, c.D / 4,
-                                                                     per_grp, NM, n0);
+  c.note(launch_after(k_scatter_rows, dim3(blocks_for(rows * (c.D / 4), 256)), 256, 0, c.st, reinterpret_cast<const float4*>(compact),
+                      reinterpret_cast<float4*>(full), rows, c.D / 4, per_grp, NM, n0));
 }
 
 struct TemporalGeom {
@@ -1893,8 +1906,7 @@ void ships_fwd(const Ctx& c, const BnbTemporalWeights& w, const float* x, const 
     mmh(c, NT, H_A, n, D, w.linear1_w, D, b1, D, M, D, D);
     mmh(c, NT, H_A, n, D, w.linear2_w, D, b2p, D, M, D, D);
   }
-  count_launch();
-  k_conv_fwd<<<sblocks, 256, 0, c.st>>>(b1, hid, w.conv_w, w.conv_b, u, gm);
+  c.note(launch_after(k_conv_fwd, dim3(sblocks), 256, 0, c.st, b1, hid, w.conv_w, w.conv_b, u, gm));
   if (c.linears) {
     train_linear::Forward f;
     f.x = u; f.image = block_image(c, L_GATES); f.blocks = 2; f.rows = Rs;
@@ -1904,12 +1916,8 @@ void ships_fwd(const Ctx& c, const BnbTemporalWeights& w, const float* x, const 
     mm(c, NT, u, D, w.a_w, D, za, D, M, D, D, w.a_b);
     mm(c, NT, u, D, w.x_w, D, zx, D, M, D, D, w.x_b);
   }
-  count_launch();
-  k_scan_fwd<<<sblocks, 256, 0, c.st>>>(za, zx, u, hid, w.log_lambda, b2p, hs, m, gm);   // m = h * gelu(linear2 n)
-  if (hid_out) {
-    count_launch();
-    k_final_state<<<sblocks, 256, 0, c.st>>>(hs, b1, hid, hid_out, gm);
-  }
+  c.note(launch_after(k_scan_fwd, dim3(sblocks), 256, 0, c.st, za, zx, u, hid, w.log_lambda, b2p, hs, m, gm));   // m = h * gelu(linear2 n)
+  if (hid_out) c.note(launch_after(k_final_state, dim3(sblocks), 256, 0, c.st, hs, b1, hid, hid_out, gm));
   linear(c, m, L_OUT_T, w.out_w, x1, Rs, nullptr, xs);
   mlp_fwd(c, x1, y ? (all ? y : b.d[14]) : nullptr, Rs, w.norm2_w, w.gate_w, w.up_w, w.down_w);
   if (y && !all) scatter(c, b.d[14], y, Rs, tg.n_rec, tg.NM, 0);
@@ -1971,8 +1979,7 @@ int temporal_bwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
     mlp_bwd(c, x1, dys, dx1, Rs, w.norm2_w, w.gate_w, w.up_w, w.down_w, dw.norm2_w, dw.gate_w, dw.up_w, dw.down_w);
 
     linear_bwd(c, dx1, m, L_OUT_T, w.out_w, dw.out_w, dm, Rs);
-    count_launch();
-    k_scan_bwd<<<sblocks, 256, 0, c.st>>>(za, zx, u, b2p, hs, dm, hid, d_hid_out, d_hid_in, w.log_lambda, dw.log_lambda, gm);
+    c.note(launch_after(k_scan_bwd, dim3(sblocks), 256, 0, c.st, za, zx, u, b2p, hs, dm, hid, d_hid_out, d_hid_in, w.log_lambda, dw.log_lambda, gm));
     // za, zx, b2p hold d za, d zx, d linear2 out; dm the direct part of d u
     if (c.linears) {
       train_linear::Backward g;
@@ -1989,8 +1996,7 @@ int temporal_bwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
       mm(c, NN, zx, D, w.x_w, D, dm, D, M, D, D, nullptr, nullptr, 0, 1);
     }
     float* db1 = za;   // free now
-    count_launch();
-    k_conv_bwd<<<sblocks, 256, 0, c.st>>>(dm, b1, hid, d_hid_out, d_hid_in, w.conv_w, db1, dw.conv_w, dw.conv_b, gm);
+    c.note(launch_after(k_conv_bwd, dim3(sblocks), 256, 0, c.st, dm, b1, hid, d_hid_out, d_hid_in, w.conv_w, db1, dw.conv_w, dw.conv_b, gm));
     if (c.linears) {
       norm_linear_bwd(c, {db1, b2p}, D, n, L_LIN1, {dw.linear1_w, dw.linear2_w}, xs, w.norm1_w, b.inv[0], dx1, dxs, dw.norm1_w, Rs);
     } else {

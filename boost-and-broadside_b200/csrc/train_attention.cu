@@ -15,7 +15,8 @@
 #include "train_attention.h"
 
 #include "common.cuh"
-#include "launch_count.h"
+#include "launch_after.h"
+#include "tensor_common.cuh"
 
 namespace bnb {
 namespace train_attn {
@@ -120,6 +121,8 @@ __host__ __device__ inline size_t carve(char* base, int n, int nb, bool grad, Sm
 template <int LPP>
 __global__ void __launch_bounds__(THREADS) k_env_attn_fwd(const Call c) {
   extern __shared__ __align__(16) char raw[];
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   constexpr int QPW = 32 / LPP, CPL = DH / LPP;
   Smem s;
   carve(raw, c.n, c.kvb ? c.nb : 0, false, &s);
@@ -196,6 +199,8 @@ __global__ void __launch_bounds__(THREADS) k_env_attn_fwd(const Call c) {
 template <int LPP, bool BULLETS>
 __global__ void __launch_bounds__(THREADS, BULLETS || LPP == 32 ? 4 : LPP == 16 ? 6 : 8) k_env_attn_bwd(const Call c) {
   extern __shared__ __align__(16) char raw[];
+  tensor::let_next_start();
+  tensor::wait_for_previous();
   constexpr int QPW = 32 / LPP, CPL = DH / LPP;
   Smem s;
   carve(raw, c.n, BULLETS ? c.nb : 0, true, &s);
@@ -404,9 +409,7 @@ template <typename K>
 int launch(K kernel, const Call& c, bool grad, cudaStream_t st) {
   const size_t smem = carve(nullptr, c.n, c.kvb ? c.nb : 0, grad, nullptr);
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX) != cudaSuccess) return 7;
-  count_launch();
-  kernel<<<c.G, THREADS, smem, st>>>(c);
-  return cudaGetLastError() == cudaSuccess ? 0 : 7;   // BNB_ERR_LAUNCH
+  return launch_after(kernel, dim3(c.G), THREADS, smem, st, c);
 }
 
 }  // namespace

@@ -22,7 +22,7 @@
 // waits for global and tensor memory, because a tile's tensors are requested one after the other into registers.
 #include "train_linear.h"
 
-#include "launch_count.h"
+#include "launch_after.h"
 #include "tensor_kernels.h"
 #include "tile_rows.cuh"
 
@@ -413,11 +413,10 @@ int forward(const Forward& f, int* status, cudaStream_t st) {
   if (!configure()) return BNB_ERR_LAUNCH;
   const int tiles = (int)((f.rows + TILE - 1) / TILE);
   const FwdArgs a{f, (int)f.rows, tiles, status, tensor::host_status_word(st)};
-  count_launch();
-  if (f.blocks == 1) k_linear_fwd<1><<<grid_of(tiles), THREADS, FwdMap<1>::BYTES, st>>>(a);
-  else if (f.blocks == 2) k_linear_fwd<2><<<grid_of(tiles), THREADS, FwdMap<2>::BYTES, st>>>(a);
-  else k_linear_fwd<3><<<grid_of(tiles), THREADS, FwdMap<3>::BYTES, st>>>(a);
-  return launched();
+  const dim3 grid(grid_of(tiles));
+  return f.blocks == 1   ? launch_after(k_linear_fwd<1>, grid, THREADS, FwdMap<1>::BYTES, st, a)
+         : f.blocks == 2 ? launch_after(k_linear_fwd<2>, grid, THREADS, FwdMap<2>::BYTES, st, a)
+                         : launch_after(k_linear_fwd<3>, grid, THREADS, FwdMap<3>::BYTES, st, a);
 }
 
 int backward(const Backward& b, int* status, cudaStream_t st) {
@@ -425,13 +424,12 @@ int backward(const Backward& b, int* status, cudaStream_t st) {
   if (!configure()) return BNB_ERR_LAUNCH;
   const int tiles = (int)((b.rows + TILE - 1) / TILE);
   const BwdArgs a{b, (int)b.rows, tiles, status, tensor::host_status_word(st)};
-  count_launch();
-  if (b.gain && b.blocks == 3) k_linear_bwd<3, true><<<grid_of(tiles), THREADS, BwdMap<3>::BYTES, st>>>(a);
-  else if (b.gain && b.blocks == 2) k_linear_bwd<2, true><<<grid_of(tiles), THREADS, BwdMap<2>::BYTES, st>>>(a);
-  else if (!b.gain && b.blocks == 2) k_linear_bwd<2, false><<<grid_of(tiles), THREADS, BwdMap<2>::BYTES, st>>>(a);
-  else if (!b.gain && b.blocks == 1) k_linear_bwd<1, false><<<grid_of(tiles), THREADS, BwdMap<1>::BYTES, st>>>(a);
-  else return BNB_ERR_BAD_ARGUMENT;
-  return launched();
+  const dim3 grid(grid_of(tiles));
+  if (b.gain && b.blocks == 3) return launch_after(k_linear_bwd<3, true>, grid, THREADS, BwdMap<3>::BYTES, st, a);
+  if (b.gain && b.blocks == 2) return launch_after(k_linear_bwd<2, true>, grid, THREADS, BwdMap<2>::BYTES, st, a);
+  if (!b.gain && b.blocks == 2) return launch_after(k_linear_bwd<2, false>, grid, THREADS, BwdMap<2>::BYTES, st, a);
+  if (!b.gain && b.blocks == 1) return launch_after(k_linear_bwd<1, false>, grid, THREADS, BwdMap<1>::BYTES, st, a);
+  return BNB_ERR_BAD_ARGUMENT;
 }
 
 }  // namespace train_linear

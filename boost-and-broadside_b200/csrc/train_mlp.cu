@@ -27,7 +27,7 @@
 // element are what the tensor cores wait for.
 #include "train_mlp.h"
 
-#include "launch_count.h"
+#include "launch_after.h"
 #include "tensor_kernels.h"
 #include "tile_rows.cuh"
 
@@ -656,9 +656,7 @@ int forward(const float* x1, const float* gain, const uint8_t* image, float* y, 
   a.tiles = (int)((rows + TILE - 1) / TILE);
   a.status = status;
   a.host_status = tensor::host_status_word(st);
-  count_launch();
-  k_mlp_fwd<<<a.tiles < 148 ? a.tiles : 148, THREADS, FW_BYTES, st>>>(a);
-  return launched();
+  return launch_after(k_mlp_fwd, dim3(a.tiles < 148 ? a.tiles : 148), THREADS, FW_BYTES, st, a);
 }
 
 int backward(const float* x1, const float* gain, const uint8_t* image, const float* dy, float* dx1, float* d_gain, float* d_gate,
@@ -673,12 +671,9 @@ int backward(const float* x1, const float* gain, const uint8_t* image, const flo
   a.tiles = (int)((rows + TILE - 1) / TILE);
   a.status = status;
   a.host_status = tensor::host_status_word(st);
-  count_launch();
-  k_mlp_dx<<<a.tiles < 148 ? a.tiles : 148, THREADS, DX_BYTES, st>>>(a);
-  count_launch();
+  if (const int rc = launch_after(k_mlp_dx, dim3(a.tiles < 148 ? a.tiles : 148), THREADS, DX_BYTES, st, a)) return rc;
   const int groups = a.tiles < 18 ? a.tiles : 18;   // 18 CTAs per chunk: 144 of the 148 SMs
-  k_mlp_dw<<<8 * groups, THREADS, DW_BYTES, st>>>(a);
-  return launched();
+  return launch_after(k_mlp_dw, dim3(8 * groups), THREADS, DW_BYTES, st, a);
 }
 
 }  // namespace train_mlp
