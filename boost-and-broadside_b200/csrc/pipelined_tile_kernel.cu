@@ -1103,9 +1103,9 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
     bias[row] = kMaskedScore;
   };
   // token `tok` of environment env, which has `ships` ships, at timestep t
-  const auto put = [&](int row, int env, int tok, int ships, int step_row, int hrow, int t, uint32_t flags) {
+  const auto put = [&](int row, int env, int tok, int ships, int step_row, int hrow, int t, uint32_t flags, bool live) {
     const int trow = (grp + t) * map.total_tokens + step_row;
-    if (MODE != STEPS) bias[row] = !args.alive || args.alive[trow] ? 0.f : kMaskedScore;
+    if (MODE != STEPS) bias[row] = live ? 0.f : kMaskedScore;
     if (tok < ships) {
       // steps since the last episode boundary, as far as the conv looks back; before the call there was none
       uint32_t lags = BNB_CONV_KERNEL - 1;
@@ -1129,7 +1129,7 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
       if (r < map.total_tokens && time < args.steps) {
         const int env = map.env_of_token(r), tok = r - map.env_tok_begin(env);
         put(row, env, tok, map.env_ship_count(env), r, map.env_ship_begin(env) + tok, time,
-            P_VALID | (step == args.chunk - 1 || time == args.steps - 1 ? P_LAST : 0u));
+            P_VALID | (step == args.chunk - 1 || time == args.steps - 1 ? P_LAST : 0u), true);
       } else {
         invalid(row);
       }
@@ -1142,7 +1142,7 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
       const int r = eb * TILE + row;
       if (r < map.total_tokens) {
         const int env = map.env_of_token(r), tok = r - map.env_tok_begin(env);
-        put(row, env, tok, map.env_ship_count(env), r, map.env_ship_begin(env) + tok, t, P_VALID);
+        put(row, env, tok, map.env_ship_count(env), r, map.env_ship_begin(env) + tok, t, P_VALID, true);   // no attention on such tiles
       } else {
         invalid(row);
       }
@@ -1164,7 +1164,7 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
         const int env = __shfl_sync(0xffffffffu, my_env, j), tok0 = __shfl_sync(0xffffffffu, my_tok, j), n = __shfl_sync(0xffffffffu, my_n, j),
                   ship0 = __shfl_sync(0xffffffffu, my_ship, j), ships = __shfl_sync(0xffffffffu, my_ships, j);
         for (int i = lane; i < n; i += 32) {
-          put(first + i, env, i, ships, tok0 + i, ship0 + i, t, P_VALID);
+          put(first + i, env, i, ships, tok0 + i, ship0 + i, t, P_VALID, !args.alive || args.alive[(size_t)(grp + t) * map.total_tokens + tok0 + i]);
           if ((i & 15) == 0) blocks[n_blocks + (i >> 4)] = (uint32_t)(first + i) | (uint32_t)first << 8 | (uint32_t)(n - 1) << 16 | (uint32_t)n << 24;
         }
         first += n;
@@ -1174,15 +1174,25 @@ __device__ __forceinline__ void fill_table(const TrunkArgs& args, int tile, int 
     for (int row = first + lane; row < TILE; row += 32) invalid(row);
   } else {
     const int NM = map.tokens_per_env, per_env = (NM + 15) >> 4;
-    const int share = NM <= 8 ? 16 / NM : 1;   // environments whose queries share a block (attend_two)
+    const int share = NM <= 8 ? 16 / NM : 1;   // environments whose queries share a block (attend_block)
     const int env0 = eb * args.envs_per_tile, envs = min(args.envs_per_tile, map.n_envs - env0);
-#pragma unroll 1
-    for (int row = lane; row < TILE; row += 32) {
-      const int el = row / NM, tok = row - el * NM;
-      if (el < envs) {
-        put(row, env0 + el, tok, map.ships_per_env, (env0 + el) * NM + tok, (env0 + el) * map.ships_per_env + tok, t, P_VALID);
-        if ((tok & 15) == 0 && el % share == 0)
-          blocks[el / share * per_env + (tok >> 4)] = (uint32_t)row | (uint32_t)(el * NM) << 8 | (uint32_t)(min(share, envs - el) * NM - 1) << 16 | (uint32_t)NM << 24;
+    int el[4], tok[4];
+    uint8_t live[4];   // the masks of this lane's rows, all on their way at once
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int row = lane + 32 * k;
+      el[k] = row / NM;
+      tok[k] = row - el[k] * NM;
+      live[k] = 1;
+      if (el[k] < envs && args.alive) live[k] = args.alive[(size_t)(grp + t) * map.total_tokens + env0 * NM + row];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int row = lane + 32 * k;
+      if (el[k] < envs) {
+        put(row, env0 + el[k], tok[k], map.ships_per_env, env0 * NM + row, (env0 + el[k]) * map.ships_per_env + tok[k], t, P_VALID, live[k] != 0);
+        if ((tok[k] & 15) == 0 && el[k] % share == 0)
+          blocks[el[k] / share * per_env + (tok[k] >> 4)] = (uint32_t)row | (uint32_t)(el[k] * NM) << 8 | (uint32_t)(min(share, envs - el[k]) * NM - 1) << 16 | (uint32_t)NM << 24;
       } else {
         invalid(row);
       }

@@ -132,6 +132,8 @@ __global__ void k_pack_temporal(BnbTemporalWeights w, uint8_t* out) {
 
 // Every image of a trunk in one launch: blockIdx.y selects the sublayer.
 constexpr int MAX_PACK_JOBS = 8;
+// One 16-byte group per thread: with a sixth of the blocks, six of them one after the other, the launch took 4.4 us; step of 16 x 12 tokens 78.6 -> 77.1 us with the masks of a row table read at once.
+constexpr int PACK_BLOCKS = (N_TEMPORAL_CHUNKS > N_SPATIAL_IMAGE ? N_TEMPORAL_CHUNKS : N_SPATIAL_IMAGE) * TILE * 8 / 256;
 struct PackJobs {
   int n_spatial, n_temporal;
   int* status;   // zeroed by the launch (null: nobody asked)
@@ -625,7 +627,7 @@ int pack_trunk(const BnbSpatialWeights* spatial, int n_spatial, const BnbTempora
       if (!temporal[t0].packed) return BNB_ERR_NULL_POINTER;
       jobs.tw[jobs.n_temporal++] = temporal[t0];
     }
-    if (const int rc = launch_after(k_pack_trunk, dim3(24, jobs.n_spatial + jobs.n_temporal), 256, 0, st, jobs)) return rc;
+    if (const int rc = launch_after(k_pack_trunk, dim3(PACK_BLOCKS, jobs.n_spatial + jobs.n_temporal), 256, 0, st, jobs)) return rc;
   }
   return BNB_OK;
 }
