@@ -380,7 +380,9 @@ __global__ void __launch_bounds__(256) k_bullet_count(const uint8_t* __restrict_
     if (lane == 0) cnt[e] = c;
   }
 }
-// one CTA: env_off = exclusive scan of cnt, in place (env_off[n_env] = total)
+// one CTA: env_off = exclusive scan of cnt, in place (env_off[n_env] = total).  Eight counts a thread and turn: the barriers of
+// a turn are what it takes (8192 environments in one turn instead of eight: {SC}).
+constexpr int SCAN_ITEMS = 8;
 __global__ void __launch_bounds__(1024) k_bullet_scan(int* __restrict__ env_off, int n_env) {
   let_next_start();
   wait_for_previous();
@@ -389,10 +391,15 @@ __global__ void __launch_bounds__(1024) k_bullet_scan(int* __restrict__ env_off,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
-  for (int base = 0; base < n_env; base += 1024) {
-    const int i = base + threadIdx.x;
-    const int v = i < n_env ? env_off[i] : 0;
-    int inc = v;
+  for (int base = 0; base < n_env; base += 1024 * SCAN_ITEMS) {
+    const int first = base + (int)threadIdx.x * SCAN_ITEMS;
+    int v[SCAN_ITEMS], sum = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k) {
+      v[k] = first + k < n_env ? env_off[first + k] : 0;
+      sum += v[k];
+    }
+    int inc = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int u = __shfl_up_sync(0xffffffffu, inc, o);
@@ -410,10 +417,14 @@ __global__ void __launch_bounds__(1024) k_bullet_scan(int* __restrict__ env_off,
       warp_sum[lane] = w;
     }
     __syncthreads();
-    const int before = carry + (warp ? warp_sum[warp - 1] : 0) + inc - v;
-    if (i < n_env) env_off[i] = before;
+    int before = carry + (warp ? warp_sum[warp - 1] : 0) + inc - sum;
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k) {
+      if (first + k < n_env) env_off[first + k] = before;
+      before += v[k];
+    }
     __syncthreads();
-    if (threadIdx.x == 1023) carry = before + v;
+    if (threadIdx.x == 1023) carry = before;
     __syncthreads();
   }
   if (threadIdx.x == 0) env_off[n_env] = carry;
