@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(256) k_bullet_count(const uint8_t* __restrict_
   }
 }
 // one CTA: env_off = exclusive scan of cnt, in place (env_off[n_env] = total).  Eight counts a thread and turn: the barriers of
-// a turn are what it takes (8192 environments in one turn instead of eight: {SC}).
+// a turn are what it takes (8192 environments in one turn instead of eight: step of 8192 x 12 tokens with bullets 870 -> 868 us).
 constexpr int SCAN_ITEMS = 8;
 __global__ void __launch_bounds__(1024) k_bullet_scan(int* __restrict__ env_off, int n_env) {
   let_next_start();
