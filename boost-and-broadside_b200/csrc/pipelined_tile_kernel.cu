@@ -494,6 +494,28 @@ __device__ __forceinline__ void attend_block(const Epi& e, uint32_t block) {
     for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
     mma_bf16(acc[nt], a0, a1, a2, a3, vf[nt >> 1][2 * (nt & 1)], vf[nt >> 1][2 * (nt & 1) + 1]);
   }
+  if (size < n) {
+    // Keys of another environment have weight 0, but 0 times a value that is not finite is NaN: where the block holds one, each
+    // environment's rows are multiplied with its own values alone.  The look (here, where the values are at hand: before the scores
+    // it held them up, 2 % of a step) costs batches that fill the chip nothing; 16 x 12 tokens 77.1 -> 78.0 us, by the code alone.
+    uint32_t zero = 0u;   // 0 v + 0 v + ..: not 0 once a value is not finite
+#pragma unroll
+    for (int i = 0; i < 8; ++i) zero = fma_bf16x2(vf[i >> 2][i & 3], 0u, zero);
+    if (__builtin_expect(__any_sync(0xffffffffu, zero != 0u), 0)) {
+#pragma unroll 1
+      for (int lo = 0; lo < n; lo += size) {
+        const auto own = [&](int row) { return ((unsigned)(row - lo) < (unsigned)size ? 0xFFFFu : 0u) | ((unsigned)(row + 1 - lo) < (unsigned)size ? 0xFFFF0000u : 0u); };
+        const uint32_t own0 = own(2 * t), own1 = own(2 * t + 8);   // rows of this lane's value registers
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          float one[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_bf16(one, a0, a1, a2, a3, vf[nt >> 1][2 * (nt & 1)] & own0, vf[nt >> 1][2 * (nt & 1) + 1] & own1);
+          if (lo0 == lo) { acc[nt][0] = one[0]; acc[nt][1] = one[1]; }
+          if (lo1 == lo) { acc[nt][2] = one[2]; acc[nt][3] = one[3]; }
+        }
+      }
+    }
+  }
 #pragma unroll
   for (int o = 1; o < 4; o <<= 1) {
     l0 += __shfl_xor_sync(0xffffffffu, l0, o);
