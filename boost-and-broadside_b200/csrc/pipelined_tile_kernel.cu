@@ -420,8 +420,7 @@ __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slo
 //
 // Environments of up to 16 tokens need no running maximum, and those of up to 8 share a block (keys of another environment score
 // -inf): 32 steps of 4096 x 8
-// tokens 5 730 -> 5 400 us.  Weights are normalised by the reciprocal (1 ulp, before the rounding to bfloat16): the division's code took 1.5 %
-// of a step.
+// tokens 5 730 -> 5 400 us.  The division's code took 1.5 % of a step, `reciprocal` is as exact.
 
 // A block of queries whose environments' keys are the block's own rows: block = first row | .. | rows less one << 16 | tokens of
 // an environment << 24.
@@ -521,7 +520,7 @@ __device__ __forceinline__ void attend_block(const Epi& e, uint32_t block) {
     l0 += __shfl_xor_sync(0xffffffffu, l0, o);
     l1 += __shfl_xor_sync(0xffffffffu, l1, o);
   }
-  const float i0 = rcp_fast(l0), i1 = rcp_fast(l1);
+  const float i0 = reciprocal(l0), i1 = reciprocal(l1);
   uint8_t* po = e.smem + OFF_P + atom;
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt) {
@@ -637,7 +636,7 @@ __device__ __forceinline__ void attention(Epi& e, int n_items) {
       l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
       l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
       l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-      const float i0 = rcp_fast(l0), i1 = rcp_fast(l1);
+      const float i0 = reciprocal(l0), i1 = reciprocal(l1);
       const int q0 = r0 + g, q1 = r0 + g + 8;
       uint8_t* po = e.smem + OFF_P + atom;
   #pragma unroll

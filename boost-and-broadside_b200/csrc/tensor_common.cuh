@@ -239,6 +239,12 @@ __device__ __forceinline__ float rcp_fast(float v) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
   return r;
 }
+// 1 / v for the sum of softmax weights: the instruction and one Newton-Raphson step r + r (1 - v r), which squares its relative
+// error.  Largest error over every float of [1, 256): 1.65 x 2^-24 without the step, 1.00 with it and by division.  NaN stays NaN.
+__device__ __forceinline__ float reciprocal(float v) {
+  const float r = rcp_fast(v);
+  return fmaf(r, fmaf(-v, r, 1.0f), r);
+}
 __device__ __forceinline__ float sqrt_fast(float v) {
   float r;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
