@@ -707,17 +707,21 @@ static long long full_tiles(const BnbBatch& b, bool flat) {
   const int per = TILE / b.tokens_per_env;
   return (b.n_envs + per - 1) / per;
 }
-// Timesteps per tile of a temporal sublayer over T timesteps, or 0 for a walk over tiles of one timestep: the fewest passes
-// over the busiest SM, small chunks first (their scan has fewer levels).  A pass of the walk costs 1.4 of a chunk's (it moves the
-// state of 128 rows).  What stays with the walk: two or three steps of a batch that fills the chip.
+// Timesteps per tile of a temporal sublayer over T timesteps, or 0 for a walk over tiles of one timestep: the fewest passes over
+// the busiest SM.  A pass takes 21.9 us in the walk and 21.4 in chunks at 2368 environments of 8 tokens, 22.2 and 21.6 at 16384, so
+// passes are what is compared; at as many of them, chunks (the walk: 8 % faster to 4 % slower).  What stays with the walk: a batch
+// that fills the chip, for step counts that would leave much of the last chunk empty -- 2368 environments: 5 steps 542 against 684
+// us in chunks of 4, 9 steps 927 against 1 066; 8192 environments of 12 tokens: 3 steps 1 714 against 1 890.  Chunks with
+// the same number of passes lie within 2 % of each other; the smallest is taken.
 static int steps_per_tile(const BnbBatch& b, bool flat, int T) {
   const auto rounds = [](long long tiles) { return (tiles + 147) / 148; };
-  long long best = rounds(full_tiles(b, flat)) * T * 7;   // in fifths
+  const long long walk = rounds(full_tiles(b, flat)) * T;
+  long long best = walk + 1;
   int chunk = 0;
   for (int c = 4; c <= 32; c *= 2) {
-    const long long cost = rounds(((long long)b.total_tokens * c + TILE - 1) / TILE) * ((T + c - 1) / c) * 5;
-    if (cost < best) {
-      best = cost;
+    const long long passes = rounds(((long long)b.total_tokens * c + TILE - 1) / TILE) * ((T + c - 1) / c);
+    if (passes < best) {
+      best = passes;
       chunk = c;
     }
   }

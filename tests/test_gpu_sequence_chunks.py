@@ -21,9 +21,12 @@ CASES = [
     (17, 5, 8, 4),       # 32
     (33, 9, 8, 0),       # 32, two chunks, one step in the second
     (33, 70, 10, 0),     # 16, three chunks
-    (20, 600, 8, 0),     # 8 or 16: more tiles than SMs
+    (20, 600, 8, 0),     # 8: more tiles than SMs
     (7, 2, 100, 52),     # environments larger than a tile
     (2, 2368, 8, 0),     # the walk: two steps of a batch that fills the chip
+    (3, 2365, 8, 0),     # the walk, a last tile that is not full
+    (5, 1475, 8, 4),     # the walk with fields
+    (4, 2368, 8, 0),     # as many passes in chunks of 4
 ]
 
 
