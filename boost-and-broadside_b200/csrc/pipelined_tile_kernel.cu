@@ -91,24 +91,30 @@ enum : int { ST_TIMEOUT_FULL = 101, ST_TIMEOUT_FREE = 102, ST_TIMEOUT_ACC = 103,
 // Optional cycle accounting (compile with -DBNB_TIMING): thread 0 (an epilogue thread), the
 // issuing lane and the fetching lane of every CTA add up the cycles they spend in each phase and
 // store them behind the status word: 32 counters per CTA from byte 256 on.
-enum : int { TE_ACC_WAIT = 0, TE_FFN_ACC_WAIT, TE_FFN_PF_WAIT, TE_FFN_MATH, TE_NORM, TE_STAGE, TE_ATTN, TE_SYNC, TE_TEMPORAL,
-             TE_IO, TE_TOTAL, TM_FULL_WAIT, TM_OP_WAIT, TM_ISSUE, TM_TOTAL, TL_FREE_WAIT, TL_KV_WAIT, TL_TOTAL, T_COUNT };
+// Of a temporal sublayer: TE_TAPS the first taps asked for, TE_B1 linear1's result into the A operand, TE_SYNC the barrier
+// behind it, TE_CONV the conv with its waits for taps, TE_PARK the state asked for and linear2's GELU, TE_GATES
+// gates, state update and the state's rows, TE_FIELDS field rows.  TE_POST: everywhere an operand is posted.
+enum : int { TE_ACC_WAIT = 0, TE_FFN_ACC_WAIT, TE_FFN_MATH, TE_NORM, TE_STAGE, TE_ATTN, TE_TAPS, TE_B1, TE_SYNC, TE_CONV, TE_PARK,
+             TE_GATES, TE_FIELDS, TE_POST, TE_IO, TE_TOTAL, TM_FULL_WAIT, TM_OP_WAIT, TM_ISSUE, TM_TOTAL, TL_FREE_WAIT, TL_KV_WAIT, TL_TOTAL, T_COUNT };
 #ifdef BNB_TIMING
-#define T_BEGIN() const long long _t0 = clock64()
-#define T_END(acc, slot) (acc)[slot] += clock64() - _t0
-#define T_WAITSLOT(e, s) (e).wait_slot = (s)
-#define T_MARK(name) long long name = clock64()
-#define T_RESET(name) name = clock64()
-#define T_SINCE(acc, slot, name) do { const long long _n = clock64(); (acc)[slot] += _n - name; name = _n; } while (0)
-#define T_STORE(args, acc, lo, hi) for (int _i = lo; _i < hi; ++_i) reinterpret_cast<long long*>((args).status)[32 + blockIdx.x * 32 + _i] = (acc)[_i]
+static_assert(T_COUNT <= 32, "counters of a CTA");
+// In shared memory, 32 bits each: as arrays of every thread they lay in local memory, and the kernel took half as long again.
+__device__ __forceinline__ uint32_t* time_counters() { __shared__ uint32_t counters[32]; return counters; }
+__device__ __forceinline__ void count_time(int slot, uint32_t cycles) {
+  if (threadIdx.x == 0 || threadIdx.x == 32 * MMA_WARP || threadIdx.x == 32 * LOAD_WARP) time_counters()[slot] += cycles;
+}
+__device__ __forceinline__ uint32_t cycles_now() { return (uint32_t)clock64(); }
+#define T_BEGIN() const uint32_t _t0 = cycles_now()
+#define T_END(slot) count_time(slot, cycles_now() - _t0)
+#define T_MARK(name) uint32_t name = cycles_now()
+#define T_RESET(name) name = cycles_now()
+#define T_SINCE(slot, name) do { const uint32_t _n = cycles_now(); count_time(slot, _n - name); name = _n; } while (0)
 #else
 #define T_BEGIN()
-#define T_END(acc, slot)
-#define T_WAITSLOT(e, s)
+#define T_END(slot)
 #define T_MARK(name)
 #define T_RESET(name)
-#define T_SINCE(acc, slot, name)
-#define T_STORE(args, acc, lo, hi)
+#define T_SINCE(slot, name)
 #endif
 
 // Optional event trace (compile with -DBNB_TRACE): CTA 0 records (event id, clock) pairs of one
@@ -216,10 +222,6 @@ struct Epi {
 #ifdef BNB_TRACE
   Trace tr;
 #endif
-#ifdef BNB_TIMING
-  long long tacc[T_COUNT];
-  int wait_slot;
-#endif
   uint8_t* smem;
   uint32_t sbase;       // shared address of smem
   uint32_t bars;        // shared address of the barrier array
@@ -236,10 +238,12 @@ struct Epi {
 // "My share of the operand is written and my reads of the accumulator are done."
 __device__ __forceinline__ void post(Epi& e, int bar) {
   TRACE(e.tr, 200 + bar);
+  T_BEGIN();
   fence_proxy_async();
   tc_fence_before();
   __syncwarp();
   if ((threadIdx.x & 31) == 0) mbar_arrive(e.bars + 8 * bar);
+  T_END(TE_POST);
   TRACE(e.tr, 210 + bar);
 }
 // The epilogue threads keep one phase bit per pair slot and flip it for every pair operation of the
@@ -251,7 +255,7 @@ __device__ __forceinline__ void wait_acc(Epi& e) {
   wait_bar(e.bars + 8 * B_ACC, (e.par >> 8) & 1u, e.aborted, ST_TIMEOUT_ACC);
   e.par ^= 1u << 8;
   tc_fence_after();
-  T_END(e.tacc, e.wait_slot);
+  T_END(TE_ACC_WAIT);
   TRACE(e.tr, 110);
 }
 // The first half of a temporal sublayer's gates, read while the others are multiplied; field_sub.
@@ -261,7 +265,7 @@ __device__ __forceinline__ void wait_other(Epi& e, int bar, uint32_t bit) {
   wait_bar(e.bars + 8 * bar, (e.par >> bit) & 1u, e.aborted, ST_TIMEOUT_ACC);
   e.par ^= 1u << bit;
   tc_fence_after();
-  T_END(e.tacc, e.wait_slot);
+  T_END(TE_ACC_WAIT);
 }
 __device__ __forceinline__ void wait_early(Epi& e) { wait_other(e, B_EARLY, 10); }
 __device__ __forceinline__ void wait_field(Epi& e) { wait_other(e, B_FIELD, 11); }
@@ -277,7 +281,7 @@ __device__ __forceinline__ void wait_op(Epi& e, uint32_t slot) {
   T_BEGIN();
   wait_bar(e.bars + 8 * (B_DONE0 + slot), (e.par >> slot) & 1u, e.aborted, ST_TIMEOUT_ACC);
   tc_fence_after();
-  T_END(e.tacc, e.wait_slot);
+  T_END(TE_FFN_ACC_WAIT);
   TRACE(e.tr, 100);
 }
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
@@ -341,7 +345,7 @@ __device__ __forceinline__ void norm_to_A(Epi& e) {
     *reinterpret_cast<uint4*>(e.smem + OFF_A + (col >> 6) * CHUNK_BYTES + swz(e.row, (col & 63) >> 3)) = o;
   }
   // the partial sums are read again by the next norm only after at least one full barrier
-  T_END(e.tacc, TE_NORM);
+  T_END(TE_NORM);
 }
 
 __device__ __forceinline__ F2 acc_pair(const uint32_t* v) { return f2(__uint_as_float(v[0]), __uint_as_float(v[1])); }
@@ -373,7 +377,6 @@ __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slo
     e.par ^= 1u << slot;
     slot = slot == 2 ? 0 : slot + 1;
   }
-  T_WAITSLOT(e, TE_FFN_ACC_WAIT);
 #pragma unroll 1
   for (int i = 0; i < 4; ++i) {
     // gate|up of chunk 2 i + group; the slot's previous operation came before those of the two chunks in between
@@ -395,7 +398,7 @@ __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slo
     gated_product(gv, uv, dst);
     gated_product(gw, uw, dst + 8);
     tmem_wait_st();
-    T_END(e.tacc, TE_FFN_MATH);
+    T_END(TE_FFN_MATH);
     // nothing of this operand is in shared memory: no proxy fence
     TRACE(e.tr, 201);
     tc_fence_before();
@@ -408,7 +411,6 @@ __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slo
     slot = slot == 2 ? 0 : slot + 1;
   }
   if (group) e.par ^= 1u << (slot == 0 ? 2 : slot - 1);   // there is no chunk 8
-  T_WAITSLOT(e, TE_ACC_WAIT);
   wait_acc(e);   // residual complete: every down projection
 }
 
@@ -670,14 +672,14 @@ __device__ __forceinline__ void run_spatial(Epi& e, int n_items, bool row_valid)
 #pragma unroll
       for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(e.smem + dst[p] + swz(e.row, c8h + q)) = row_valid ? pack8(&v[q * 8]) : make_uint4(0u, 0u, 0u, 0u);
     }
-    T_END(e.tacc, TE_STAGE);
+    T_END(TE_STAGE);
   }
   tc_fence_before();
   asm volatile("bar.sync %0, 128;" ::"r"(7 + e.part) : "memory");   // the four warps of this head
   {
     T_BEGIN();
     attention(e, n_items);
-    T_END(e.tacc, TE_ATTN);
+    T_END(TE_ATTN);
   }
   // keys and values are dead: the area may take weight chunks again
   __syncwarp();
@@ -768,6 +770,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
   float* hout = is_ship ? s.hid_out + (size_t)rs.hrow * 4 * D : nullptr;
   // Causal conv, one warp per ship row and four columns per lane, so that the stored taps are
   // read and written as whole 512-byte rows; new taps = (tap1, tap2, b1); bf16(u) replaces b1 in A.
+  T_MARK(tt);
   {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int col = lane * 4;
@@ -801,7 +804,9 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
 #pragma unroll
       for (int k = 0; k < 4; ++k) request(k, warp + EPI_WARPS * k);
     }
+    T_SINCE(TE_TAPS, tt);
     wait_round(e, 3);   // acc0 = linear1 n, acc1 = linear2 n / 2; slots 0 and 1
+    T_RESET(tt);
     // b1 = bf16(linear1 n) into the A operand
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
@@ -816,7 +821,9 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
     }
     if constexpr (!STEPS) cw = conv_weights(s, col);
     tc_fence_before();
+    T_SINCE(TE_B1, tt);
     epi_sync();
+    T_SINCE(TE_SYNC, tt);
     if constexpr (STEPS) {
       uint2 bw[8];
 #pragma unroll
@@ -871,7 +878,9 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
       }
     }
   }
+  T_SINCE(TE_CONV, tt);
   post(e, B_OP0);   // A = u (ship rows) / b1 (field rows)
+  T_RESET(tt);
   // While the gates are multiplied: the previous state of this thread's columns is asked for ...
   float hprev[2][2][8];
 #pragma unroll
@@ -895,12 +904,14 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive(e.bars + 8 * B_PARK);
   }
+  T_SINCE(TE_PARK, tt);
   wait_early(e);   // acc0 / acc2 = halves of [W_a u | W_x u] of hidden columns [0,64) / [64,128)
   // gates and state update
   const F2 keep = f2(rs.flags & P_BOUNDARY ? 0.f : 1.f), one = f2(1.f);
 #pragma unroll
   for (int rnd = 0; rnd < 2; ++rnd) {
     if (rnd == 1) wait_round(e, has_fields ? 7 : 5);   // slots 2, 0 (and 1 for field_sub)
+    T_RESET(tt);
     uint32_t rv[16], iv[16];
     const uint32_t acc = e.lane_addr + (rnd ? COL_ACC2 : COL_ACC0) + e.part * 16;
     tmem_ld16_nowait(acc, rv);        // executed by every lane of the warp
@@ -991,10 +1002,12 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
         }
       }
     }
+    T_SINCE(TE_GATES, tt);
   }
   if (has_fields) {
     // field rows: branch = bf16(bf16(field_sub b1) * b2); rows outside every environment are zeros throughout
     wait_field(e);
+    T_RESET(tt);
 #pragma unroll
     for (int rnd = 0; rnd < 2; ++rnd) {
       uint32_t v[16];
@@ -1019,6 +1032,7 @@ __device__ __forceinline__ void run_temporal(Epi& e, const SubLayer& s, const Pl
       *reinterpret_cast<uint4*>(e.smem + OFF_A + CHUNK_BYTES + swz(e.row, e.part * 2 + q)) = make_uint4(0u, 0u, 0u, 0u);
     }
   }
+  T_SINCE(TE_FIELDS, tt);
   post(e, B_OP0);   // branch operand
 }
 
@@ -1035,9 +1049,6 @@ struct Issuer {
 #ifdef BNB_TRACE
   Trace tr;
 #endif
-#ifdef BNB_TIMING
-  long long tacc[T_COUNT];
-#endif
   uint32_t sbase, bars, tmem;
   uint32_t elected;    // 1 in the lane that issues
   uint32_t full_par;   // per-slot phase bits of the FULL barriers
@@ -1050,7 +1061,7 @@ __device__ __forceinline__ void wait_operand(Issuer& m, int bar) {
   wait_bar(m.bars + 8 * bar, (m.op_par >> bar) & 1u, m.aborted, ST_TIMEOUT_OPERAND);
   m.op_par ^= 1u << bar;
   tc_fence_after();
-  T_END(m.tacc, TM_OP_WAIT);
+  T_END(TM_OP_WAIT);
   TRACE(m.tr, 400 + bar);
 }
 __device__ __forceinline__ void commit_one(const Issuer& m, uint32_t bar) { tc_commit_if(m.elected, m.bars + 8 * bar); }
@@ -1059,7 +1070,7 @@ __device__ __forceinline__ void wait_weights(Issuer& m, uint32_t slot) {
   T_MARK(tw);
   wait_bar(m.bars + 8 * (B_FULL0 + slot), (m.full_par >> slot) & 1u, m.aborted, ST_TIMEOUT_FULL);
   m.full_par ^= 1u << slot;
-  T_SINCE(m.tacc, TM_FULL_WAIT, tw);
+  T_SINCE(TM_FULL_WAIT, tw);
   TRACE(m.tr, 410);
 }
 // A pair operation: D[128 x 128] (+)= A[128 x 128] * W[128 x 128]^T, K atom 0 of the operand at a_off0 and K
@@ -1075,7 +1086,7 @@ __device__ __forceinline__ void multiply_pair(Issuer& m, uint32_t slot, uint32_t
 #pragma unroll
   for (uint32_t k = 0; k < 4; ++k) mma_one<false>(m.elected, m.tmem + d_col, a1 + 2 * k, b_lo + 1024 + 2 * k, idesc, 1u);
   commit_one(m, B_DONE0 + slot);
-  T_SINCE(m.tacc, TM_ISSUE, tw);
+  T_SINCE(TM_ISSUE, tw);
   TRACE(m.tr, 420);
 }
 __device__ __forceinline__ void issue_pair(Issuer& m, uint32_t slot, uint32_t a_off0, uint32_t a_off1, uint32_t d_col, uint32_t accumulate) {
@@ -1274,7 +1285,7 @@ __device__ __forceinline__ void issue_downs(Issuer& m, const float* next_hid, co
     for (uint32_t k = 0; k < 4; ++k) mma_one<true>(m.elected, m.tmem + COL_RESID, a_col + 8 * k, b_lo + 2 * k, idesc, 1u);
     commit_one(m, B_DONE0 + 3 + a);
     commit_one(m, B_PFREE0 + (c & 3));
-    T_SINCE(m.tacc, TM_ISSUE, tw);
+    T_SINCE(TM_ISSUE, tw);
     TRACE(m.tr, 430);
     if (next_hid) prefetch_state(next_hid, tab, 16 * (int)c);
     __syncwarp();
@@ -1331,6 +1342,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     sched_len += ops;
   }
   // Both row tables start without rows: after a wait has run out they may be read before they are written.
+#ifdef BNB_TIMING
+  if (tid < 32) time_counters()[tid] = 0;
+#endif
   for (int i = tid; i < 2 * TAB_BYTES / 16; i += THREADS)
     reinterpret_cast<int4*>(smem + OFF_TAB)[i] = i % (TAB_BYTES / 16) < TILE ? make_int4(-1, 0, -1, 0) : make_int4(0, 0, 0, 0);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
@@ -1372,10 +1386,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       uint32_t kv_par = 0;
       const int len = sched_len;
       const int skip_op = blockIdx.x == 0 ? args.skip_op : -1;
-#ifdef BNB_TIMING
-      long long tacc[T_COUNT];
-      for (int i = 0; i < T_COUNT; ++i) tacc[i] = 0;
-#endif
       T_MARK(t_start);
 #ifdef BNB_TRACE
       Trace ltr;
@@ -1397,14 +1407,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
             wait_bar(bar0 + 8 * B_KVREL, kv_par, s_aborted, ST_TIMEOUT_FREE);
             kv_par ^= 1u;
           }
-          T_SINCE(tacc, TL_KV_WAIT, tw);
+          T_SINCE(TL_KV_WAIT, tw);
           wait_bar(bar0 + 8 * (B_DONE0 + slot), (free_par >> slot) & 1u, s_aborted, ST_TIMEOUT_FREE);
           free_par ^= 1u << slot;
           // Once a wait of this CTA has run out nothing is in step any more: stop fetching.  Arming a
           // FULL barrier again before its previous copy has landed would arrive on it twice in one
           // phase, which is undefined; the other roles' waits give up at once and the kernel drains.
           if (*static_cast<volatile int*>(s_aborted)) { pass = passes; break; }
-          T_SINCE(tacc, TL_FREE_WAIT, tw);
+          T_SINCE(TL_FREE_WAIT, tw);
           TRACE(ltr, 500 + slot);
           if (elected && op != skip_op) {   // skip_op: test hook, this operation's weights never arrive
             const uint32_t full = bar0 + 8 * (B_FULL0 + slot);
@@ -1412,10 +1422,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
             bulk_g2s(sbase + (now.z & ~15u), reinterpret_cast<const void*>(((unsigned long long)now.y << 32) | now.x), now.w, full);
           }
         }
-#ifdef BNB_TIMING
-      tacc[TL_TOTAL] = clock64() - t_start;
-      if ((tid & 31) == 0) T_STORE(args, tacc, TL_FREE_WAIT, T_COUNT);
-#endif
+      T_SINCE(TL_TOTAL, t_start);
     }
   } else if (warp == MMA_WARP || warp == DOWN_WARP) {
     // ---------------------------------------------------------------- tensor-core issue
@@ -1431,9 +1438,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
 #ifdef BNB_TRACE
       trace_init(m.tr, args.status, warp == MMA_WARP ? 1 : 3);
       if ((tid & 31) != 0) m.tr.n = 1500;
-#endif
-#ifdef BNB_TIMING
-      for (int i = 0; i < T_COUNT; ++i) m.tacc[i] = 0;
 #endif
       T_MARK(t_start);
       const bool down = warp == DOWN_WARP;
@@ -1485,10 +1489,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       commit_one(m, B_DRAIN);
       for (int i = 0; i < DEFAULT_POLL_LIMIT && !mbar_try_wait(m.bars + 8 * B_DRAIN, 0); ++i) {
       }
-#ifdef BNB_TIMING
-      m.tacc[TM_TOTAL] = clock64() - t_start;
-      if (!down && (tid & 31) == 0) T_STORE(args, m.tacc, TM_FULL_WAIT, TL_FREE_WAIT);
-#endif
+      T_SINCE(TM_TOTAL, t_start);
     }
   } else {
     // ---------------------------------------------------------------- tile owners
@@ -1507,10 +1508,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
     trace_init(e.tr, args.status, 0);
     if (tid != 0) e.tr.n = 1500;
 #endif
-#ifdef BNB_TIMING
-    for (int i = 0; i < T_COUNT; ++i) e.tacc[i] = 0;
-    e.wait_slot = TE_ACC_WAIT;
-#endif
     T_MARK(t_start);
     const int row = e.row, lane = tid & 31;
     // Rows of bfloat16 tokens move through shared memory, so that a warp's access to global memory is two whole rows: 4
@@ -1527,6 +1524,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
       const bool first_step = t == 0;
       if (++t == args.t_loop) t = 0;
       wait_other(e, B_XFULL, 12);
+      T_RESET(t_io);
       e.tab = smem + OFF_TAB + (pass & 1) * TAB_BYTES;
       const int4 own = reinterpret_cast<const int4*>(e.tab)[row];
       const Place rs{own.x, (uint32_t)own.y, own.z, 0};
@@ -1558,7 +1556,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
         if (lane == 0) mbar_arrive(e.bars + 8 * B_XFREE);
         tmem_st32(e.lane_addr + COL_RESID + e.part * 32, v);
       }
-      T_SINCE(e.tacc, TE_IO, t_io);
+      T_SINCE(TE_IO, t_io);
       const int n_items = *reinterpret_cast<const int*>(e.tab + TAB_COUNT);
       for (int si = 0; si < args.n_sub; ++si) {
         const SubLayer& s = s_sub[si];
@@ -1609,15 +1607,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_trunk_pipelined(const __grid_con
           }
         }
       }
-      T_SINCE(e.tacc, TE_IO, t_io);
+      T_SINCE(TE_IO, t_io);
     }
-#ifdef BNB_TIMING
-    e.tacc[TE_TOTAL] = clock64() - t_start;
-    if (tid == 0) T_STORE(args, e.tacc, 0, TM_FULL_WAIT);
-#endif
+    T_SINCE(TE_TOTAL, t_start);
   }
   tc_fence_before();
   __syncthreads();
+#ifdef BNB_TIMING
+  if (tid < 32) reinterpret_cast<long long*>(args.status)[32 + blockIdx.x * 32 + tid] = time_counters()[tid];
+#endif
   if (s_aborted[0] && warp == LOAD_WARP) {
     // a wait ran out: copies may still be in flight towards this CTA's shared memory; give them
     // time to land before the CTA gives it up
