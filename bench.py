@@ -844,7 +844,7 @@ def run_ours(args) -> None:
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "traffic": (NCU_C2_DRAM_BYTES_PER_TOKEN * tokens if args.workload == "C2" and launches == 2 * args.steps else None),
                          "of": src, "algorithmic_bytes_per_step": alg_bytes,
-                         "kernel": ("k_trunk_pipelined (one launch = one trunk step; the 8 us k_pack_trunk launch that rewrites the weight images before it is inside the timed step)"
+                         "kernel": ("k_trunk_pipelined (one launch = one trunk step; the 5 us k_pack_trunk launch that rewrites the weight images before it is inside the timed step)"
                                     if launches == 2 * args.steps else "whole trunk step (all launches of one step)"), "kernel_ms": kernel_ms},
             "tensor": {"achieved": alg_flops / (kernel_ms * 1e-3) / 1e12, "peak": tflops_burst, "unit": "TFLOP/s",
                        "frac": alg_flops / (kernel_ms * 1e-3) / 1e12 / tflops_burst, "of": src + " (burst: the timed region lasts milliseconds)",

@@ -2,6 +2,7 @@
 // tensor memory, tables) while the one before still runs, and wait in wait_for_previous (tensor_common.cuh) before they
 // touch global memory.  A call of small batches is a chain of such launches: step of 16 x 12 tokens 83.0 -> 78.6 us, policy
 // step of 16 environments 227 -> 199, of 8192 1170 -> 1130, a sequence of 5 x 67 x 11 188 -> 164.
+// Not for the float32 step (split_kernels.cu), whose kernels read before they wait; it launches its own chain.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -124,10 +124,12 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackJobs j
 
 // ------------------------------------------------------------------ shared pieces of the tile kernels
 
-// Programmatic dependence: everything an earlier launch wrote is visible after the wait.  The trigger comes
-// after it, so a launch that has started knows that the one before the one before it is complete.
-
-struct Waits { int* status; int* host_status; int weights_early; };   // weights_early: the images are older than the launch before
+// Programmatic dependence: in this chain a kernel waits for the launch before it and triggers the one behind it after that (the
+// kernels of launch_after.h the other way round), so a launch that has started knows that the one before the one before it is
+// complete.  What is older than that is read before the wait: weight images from the chain's second launch on (weights_early;
+// k_pack before the first is a plain launch), in k_front also the state.  A kernel that triggers first, put into this chain, would
+// let its successor read both too early.
+struct Waits { int* status; int* host_status; int weights_early; };
 
 enum : int { B_FULL = 0, B_FREE = 7, B_OP0 = 14, B_OP1, B_ACC0, B_ACC1, B_GU0, B_H0 = B_GU0 + 8, B_COUNT = B_H0 + 8 };
 static_assert(8 * B_COUNT <= 400, "frame area");

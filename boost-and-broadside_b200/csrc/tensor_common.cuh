@@ -292,7 +292,6 @@ __device__ __forceinline__ F2 sigmoid_twice_bf16(F2 v) {
   const float2 g = halves(fma(f2(tanh_fast(h.x), tanh_fast(h.y)), f2(0.5f), f2(0.5f)));
   return f2(round_bf16(g.x), round_bf16(g.y));
 }
-__device__ __forceinline__ float sigmoid_fast(float v) { return fmaf(0.5f, tanh_fast(0.5f * v), 0.5f); }
 
 __device__ __forceinline__ F2 unpack_bf16(uint32_t v) { return f2(__uint_as_float(v << 16), __uint_as_float(v & 0xFFFF0000u)); }
 __device__ __forceinline__ uint32_t pack_bf16(F2 a) { const float2 v = halves(a); return pack_bf16(v.x, v.y); }
@@ -315,7 +314,8 @@ __device__ __forceinline__ uint32_t swz(int r, int c8) { return (uint32_t)(r * 1
 // ------------------------------------------------------------------ programmatic dependence (launch_after.h)
 //
 // let_next_start comes after the CTA's tensor memory is allocated (a successor on the same SM that allocated it first would
-// wait for this kernel, and this kernel for it); nothing in global memory is read or written before wait_for_previous.
+// wait for this kernel, and this kernel for it).  In the kernels of launch_after.h it comes before wait_for_previous, and nothing
+// in global memory is read or written before that; the float32 step's chain (split_kernels.cu) has the other order, and reads early.
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -54,7 +54,8 @@ def test_chunked_sequence_against_the_oracle(T, B, ships, fields, token_dtype):
 
 
 def test_a_sequence_continues_where_the_one_before_ended():
-    """Taps and state across calls: 12 steps at once against 5 and 7, bit for bit within the state's rounding."""
+    """Taps and state across calls: 12 steps at once against 5 and 7, whose chunks sum the recurrence in another order: equal to a
+    quarter of the tolerance (a float32 sum's last bit, and the bfloat16 roundings it moves)."""
     gen = torch.Generator().manual_seed(5)
     x = torch.randn(12, 6, 8, 128, generator=gen).to(DEV)
     done = (torch.rand(12, 6, generator=gen) < 0.2).to(DEV)
