@@ -3,8 +3,8 @@
 // One CTA per environment-step, one warp per head, every row staged once in shared memory with 16-byte
 // asynchronous copies and written back as whole rows.  Its floor is the memory traffic of q|k|v (1.5 KB per
 // token) and its gradient; what bounds it is shared-memory and load latency: 8192 environment-steps of 8
-// tokens take 38 us forward (DRAM 37 % of peak, issue slots 52 % busy, 57 % of the warps) and 60 us for the gradient
-// (64 registers without bullets, where 128 held 24 % of the warps and it took 95).  The kernels it replaces read rows element by element (one
+// tokens take 38 us forward (DRAM 36 % of peak, issue slots 53 % busy, 57 % of the warps) and 67 us for the gradient
+// (64 registers without bullets hold 47 % of the warps, where 128 held 24 % and it took 95).  The kernels it replaces read rows element by element (one
 // thread per query, or eight lanes per head), ran at 2.2 - 2.6 TB/s on environments of 8 tokens and took 425 /
 // 575 us (forward / gradient) for 1536 environment-steps of 12 tokens with 80 bullet slots, most of it
 // on slots that are not in use (45 / 99 us here, averaged over the sublayers that read them and those that do not).  Here only the slots in use are read.
