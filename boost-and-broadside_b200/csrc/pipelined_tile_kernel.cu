@@ -425,8 +425,9 @@ __device__ __forceinline__ void ffn(Epi& e, uint32_t slot) {   // slot: pair slo
 // tokens 5 730 -> 5 400 us.  The division's code took 1.5 % of a step, `reciprocal` is as exact.
 
 // A block of queries whose environments' keys are the block's own rows: block = first row | .. | rows less one << 16 | tokens of
-// an environment << 24.
-__device__ __forceinline__ void attend_block(const Epi& e, uint32_t block) {
+// an environment << 24.  False, and nothing written: it holds several environments and a value that is not finite.  Keys of
+// another environment have weight 0, but 0 times such a value is NaN, so the caller takes its environments one by one.
+__device__ __forceinline__ bool attend_block(const Epi& e, uint32_t block) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const uint32_t atom = (uint32_t)(e.part >> 1) * CHUNK_BYTES;
   const int c8h = (e.part & 1) * 4;
@@ -500,27 +501,12 @@ __device__ __forceinline__ void attend_block(const Epi& e, uint32_t block) {
     l0 += __shfl_xor_sync(0xffffffffu, l0, o);
     l1 += __shfl_xor_sync(0xffffffffu, l1, o);
   }
+  // The look costs nothing here, behind the sums (8192 x 12 tokens 549 us; before the scores it held them up, 560).
   if (size < n) {
-    // Keys of another environment have weight 0, but 0 times a value that is not finite is NaN: where the block holds one, each
-    // environment's rows are multiplied with its own values alone.  The look costs nothing here, behind the sums (before the scores
-    // it held them up: 8192 x 12 tokens 549 -> 560 us; before the sums 16 x 12 tokens took 78.0 us instead of 77.1).
     uint32_t zero = 0u;   // 0 v + 0 v + ..: not 0 once a value is not finite
 #pragma unroll
     for (int i = 0; i < 8; ++i) zero = fma_bf16x2(vf[i >> 2][i & 3], 0u, zero);
-    if (__builtin_expect(__any_sync(0xffffffffu, zero != 0u), 0)) {
-#pragma unroll 1
-      for (int lo = 0; lo < n; lo += size) {
-        const auto own = [&](int row) { return ((unsigned)(row - lo) < (unsigned)size ? 0xFFFFu : 0u) | ((unsigned)(row + 1 - lo) < (unsigned)size ? 0xFFFF0000u : 0u); };
-        const uint32_t own0 = own(2 * t), own1 = own(2 * t + 8);   // rows of this lane's value registers
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          float one[4] = {0.f, 0.f, 0.f, 0.f};
-          mma_bf16(one, a0, a1, a2, a3, vf[nt >> 1][2 * (nt & 1)] & own0, vf[nt >> 1][2 * (nt & 1) + 1] & own1);
-          if (lo0 == lo) { acc[nt][0] = one[0]; acc[nt][1] = one[1]; }
-          if (lo1 == lo) { acc[nt][2] = one[2]; acc[nt][3] = one[3]; }
-        }
-      }
-    }
+    if (__builtin_expect(__any_sync(0xffffffffu, zero != 0u), 0)) return false;
   }
   const float i0 = reciprocal(l0), i1 = reciprocal(l1);
   uint8_t* po = e.smem + OFF_P + atom;
@@ -529,6 +515,7 @@ __device__ __forceinline__ void attend_block(const Epi& e, uint32_t block) {
     if (g < n) *reinterpret_cast<uint32_t*>(po + swz(r0 + g, c8h + nt) + t * 4) = pack_bf16(acc[nt][0] * i0, acc[nt][1] * i0);
     if (g + 8 < n) *reinterpret_cast<uint32_t*>(po + swz(r0 + g + 8, c8h + nt) + t * 4) = pack_bf16(acc[nt][2] * i1, acc[nt][3] * i1);
   }
+  return true;
 }
 
 __device__ __forceinline__ void attention(Epi& e, int n_items) {
@@ -544,13 +531,14 @@ __device__ __forceinline__ void attention(Epi& e, int n_items) {
   const float c2 = 0.17677669529663687f * 1.4426950408889634f;  // log2(e) / sqrt(32): scores in the log2 domain
   for (int it = (warp + h) & 3; it < n_items; it += EPI_WARPS / 4) {
     const uint32_t block = blocks[it];
-    if ((block >> 16 & 255) < 16) {
-      attend_block(e, block);
-      continue;
-    }
-    // larger environments: keys are walked in blocks of 16 with a running maximum
-    {
-      const int r0 = block & 255, e0 = block >> 8 & 255, n = (int)(block >> 16 & 255) + 1;   // first row; first tile row and size of the environment
+    if ((block >> 16 & 255) < 16 && attend_block(e, block)) continue;
+    // larger environments, and those of a block that is taken apart, one after the other: keys are walked in blocks of 16 with a
+    // running maximum
+    const int n = max((int)(block >> 24), 1);   // tokens of the environment (0 may stand there after a wait has run out)
+    const int end = (int)(block & 255) + (int)(block >> 16 & 255);
+    int r0 = block & 255, e0 = block >> 8 & 255;   // first row; first tile row of the environment
+#pragma unroll 1
+    do {
       const int last = e0 + n - 1;
       uint32_t qa[2][4];
       {
@@ -646,7 +634,9 @@ __device__ __forceinline__ void attention(Epi& e, int n_items) {
         if (q0 <= last) *reinterpret_cast<uint32_t*>(po + swz(q0, c8h + nt) + t * 4) = pack_bf16(acc[nt][0] * i0, acc[nt][1] * i0);
         if (q1 <= last) *reinterpret_cast<uint32_t*>(po + swz(q1, c8h + nt) + t * 4) = pack_bf16(acc[nt][2] * i1, acc[nt][3] * i1);
       }
-    }
+      r0 += n;
+      e0 += n;
+    } while (n < 16 && r0 <= end);
   }
 }
 

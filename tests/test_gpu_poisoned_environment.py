@@ -26,12 +26,13 @@ def poisoned(gen, lead, tokens, ships):
 
 
 def compare(got, clean, ref, good, ships, what):
-    """The good environments bit for bit as in the call without bad ones, and near the oracle."""
+    """The good environments near the oracle, and as in the call without bad ones: taken one by one their softmax sums are float32
+    sums in another order, whose last bits move a few bfloat16 roundings (a quarter of the tolerance)."""
     rows = (good[:, None] * ships + torch.arange(ships)).flatten()
     for i, (dim, at, name) in enumerate(((-3, good, "y"), (1, rows, "hidden"))):
         assert not torch.isfinite(got[i]).all()   # the bad ones are bad
         ours = got[i].cpu().index_select(dim, at)
-        assert torch.equal(ours, clean[i].cpu().index_select(dim, at)), f"{what}: {name}"
+        assert_close(ours, clean[i].cpu().index_select(dim, at), "bf16", f"{what}: {name}, bad ones or not", scale=0.25)
         assert_close(ours, ref[i].index_select(dim, at), "bf16", f"{what}: {name}")
 
 
