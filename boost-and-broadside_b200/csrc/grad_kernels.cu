@@ -913,7 +913,7 @@ struct AttnBwdArgs {
   const uint8_t* mask;                     // (groups, nk) or null
   const float* d_o; int ldo;               // gradient of the attention output, rows like q
   float* dq; int lddq; int dq_accumulate;
-  float* dkv; int lddkv; int dvoff;        // rows like kv
+  float* dkv; int lddkv; size_t dvoff;     // rows like kv
   int nq, nk, dh;
   float scale;
   int gate_by_mask;                        // the branch is multiplied by any(mask) (bullets)
@@ -1767,10 +1767,10 @@ void linear_bwd(const Ctx& c, const float* dy, const float* x, int first, const 
   c.note(train_linear::backward(b, c.b.status, c.st));
 }
 // The gradients behind norm_linear: weights, the norm's gain, and dx = dres + what comes through the norm.
-void norm_linear_bwd(const Ctx& c, std::initializer_list<const float*> dy, int ld, const float* n, int first, std::initializer_list<float*> dW,
+void norm_linear_bwd(const Ctx& c, std::initializer_list<const float*> dy, const float* n, int first, std::initializer_list<float*> dW,
                      const float* x, const float* gain, const float* inv, const float* dres, float* dx, float* d_gain, size_t rows) {
   train_linear::Backward b;
-  b.ld_dy = ld; b.n = n; b.image = block_image(c, first); b.blocks = (int)dy.size();
+  b.n = n; b.image = block_image(c, first); b.blocks = (int)dy.size();
   std::copy(dy.begin(), dy.end(), b.dy);
   std::copy(dW.begin(), dW.end(), b.d_weight);
   b.x = x; b.gain = gain; b.inv = inv; b.dres = dres; b.dx = dx; b.d_gain = d_gain; b.rows = rows;
@@ -1828,18 +1828,22 @@ int spatial_bwd(const Ctx& c, const BnbSpatialWeights& w, const BnbSpatialGrads&
 
   linear_bwd(c, dx1, o, L_OUT, w.out_w, dw.out_w, d_o, R);
   int rc;
+  // d q | d k | d v and d keys | d values: each its own tensor for the row tiles, which read whole rows of one
+  const int ld_qkv = c.linears ? D : 3 * D, ld_kvb = c.linears ? D : 2 * D;
+  const size_t off_qkv = c.linears ? R * D : D, off_kvb = c.linears ? RB * D : D;
   if (train_attn::supported(D, c.H, NM, nb)) {
     train_attn::Call a{};
     a.qkv = qkv; a.alive = alive; a.kvb = reads ? b.kvb : nullptr; a.bactive = reads ? bul->active : nullptr;
     a.G = G; a.n = NM; a.nb = nb; a.d_o = d_o; a.dqkv = dqkv; a.dkvb = b.dkvb;
+    a.ld_dqkv = ld_qkv; a.off_dqkv = off_qkv; a.ld_dkvb = ld_kvb; a.off_dkvb = off_kvb;
     if ((rc = train_attn::backward(a, c.st))) return rc;
   } else {
     const int dh = D / c.H;
     const float scale = 1.0f / sqrtf((float)dh);
-    AttnBwdArgs self{qkv, 3 * D, qkv + D, 3 * D, D, alive, d_o, D, dqkv, 3 * D, 0, dqkv + D, 3 * D, D, NM, NM, dh, scale, 0};
+    AttnBwdArgs self{qkv, 3 * D, qkv + D, 3 * D, D, alive, d_o, D, dqkv, ld_qkv, 0, dqkv + off_qkv, ld_qkv, off_qkv, NM, NM, dh, scale, 0};
     if ((rc = attn_bwd(c, self, G))) return rc;
     if (reads) {
-      AttnBwdArgs cross{qkv, 3 * D, b.kvb, 2 * D, D, bul->active, d_o, D, dqkv, 3 * D, 1, b.dkvb, 2 * D, D, NM, nb, dh, scale,
+      AttnBwdArgs cross{qkv, 3 * D, b.kvb, 2 * D, D, bul->active, d_o, D, dqkv, ld_qkv, 1, b.dkvb, ld_kvb, off_kvb, NM, nb, dh, scale,
                         bul->active ? 1 : 0};
       if ((rc = attn_bwd(c, cross, G))) return rc;
     }
@@ -1848,9 +1852,9 @@ int spatial_bwd(const Ctx& c, const BnbSpatialWeights& w, const BnbSpatialGrads&
   if (c.linears) {
     // the bullet tokens feed every sublayer that reads them: their gradient accumulates
     if (reads)
-      norm_linear_bwd(c, {b.dkvb, b.dkvb + D}, 2 * D, b.bul_n, L_KVB, {dw.kv_bullet_w, dw.kv_bullet_w + square}, bul->tokens, w.norm_bullet_w,
+      norm_linear_bwd(c, {b.dkvb, b.dkvb + off_kvb}, b.bul_n, L_KVB, {dw.kv_bullet_w, dw.kv_bullet_w + square}, bul->tokens, w.norm_bullet_w,
                       b.bul_inv, d_bullets, d_bullets ? d_bullets : b.bul_dn, dw.norm_bullet_w, RB);
-    norm_linear_bwd(c, {dqkv, dqkv + D, dqkv + 2 * D}, 3 * D, n1, L_QKV, {dw.qkv_w, dw.qkv_w + square, dw.qkv_w + 2 * square}, x, w.norm1_w,
+    norm_linear_bwd(c, {dqkv, dqkv + off_qkv, dqkv + 2 * off_qkv}, n1, L_QKV, {dw.qkv_w, dw.qkv_w + square, dw.qkv_w + 2 * square}, x, w.norm1_w,
                     b.inv[0], dx1, dx, dw.norm1_w, R);
     return status_of(c);
   }
@@ -1998,7 +2002,7 @@ int temporal_bwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
     float* db1 = za;   // free now
     c.note(launch_after(k_conv_bwd, dim3(sblocks), 256, 0, c.st, dm, b1, hid, d_hid_out, d_hid_in, w.conv_w, db1, dw.conv_w, dw.conv_b, gm));
     if (c.linears) {
-      norm_linear_bwd(c, {db1, b2p}, D, n, L_LIN1, {dw.linear1_w, dw.linear2_w}, xs, w.norm1_w, b.inv[0], dx1, dxs, dw.norm1_w, Rs);
+      norm_linear_bwd(c, {db1, b2p}, n, L_LIN1, {dw.linear1_w, dw.linear2_w}, xs, w.norm1_w, b.inv[0], dx1, dxs, dw.norm1_w, Rs);
     } else {
       mmh(c, TN, H_B, b2p, D, n, D, dw.linear2_w, D, D, D, M);
       mm(c, NN, b2p, D, w.linear2_w, D, dn, D, M, D, D);
@@ -2023,7 +2027,7 @@ int temporal_bwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
     gelu_mul_bwd(c, b2p, b1, dm, b2p, dm, Rf * D);                      // b2p <- d linear2 out, dm <- d b1
     linear_bwd(c, dm, c1, L_FIELD, w.field_sub_w, dw.field_sub_w, dc1, Rf);
     if (c.linears) {
-      norm_linear_bwd(c, {dc1, b2p}, D, n, L_LIN1, {dw.linear1_w, dw.linear2_w}, xf, w.norm1_w, b.inv[0], dx1, dxf, dw.norm1_w, Rf);
+      norm_linear_bwd(c, {dc1, b2p}, n, L_LIN1, {dw.linear1_w, dw.linear2_w}, xf, w.norm1_w, b.inv[0], dx1, dxf, dw.norm1_w, Rf);
     } else {
       mmh(c, TN, H_B, dc1, D, n, D, dw.linear1_w, D, D, D, M);
       mm(c, NN, dc1, D, w.linear1_w, D, dn, D, M, D, D);

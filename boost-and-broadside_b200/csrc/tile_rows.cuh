@@ -90,9 +90,16 @@ __device__ __forceinline__ void transpose_rows(float4 (&v)[8], uint32_t taddr, u
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = staged_row(stage, i, m.lane);
 }
-// four values as bfloat16 into an operand tile
-__device__ __forceinline__ void put4(uint8_t* tile, int row, int col, float a, float b, float c, float d) {
-  *reinterpret_cast<uint2*>(tile + (col >> 6) * CHUNK_BYTES + swz(row, (col & 63) >> 3) + ((col >> 2) & 1) * 8) = make_uint2(pack_bf16(a, b), pack_bf16(c, d));
+// swz(m.row(i), c8): a row is four further per request and its swizzle alternates, so that the addresses of a loop over i are
+// two registers and constants.  (From the row's number the compiler kept eight for each use, and spilled them.)
+__device__ __forceinline__ uint32_t row_swz(const RowMap& m, int i, int c8) {
+  const int l = m.lane >> 3;
+  return (uint32_t)((((m.row0 + l) * 128 + ((c8 ^ l) << 4)) ^ ((i & 1) << 6)) + 512 * i);
+}
+// this lane's four values of its i-th row as bfloat16 into an operand tile
+__device__ __forceinline__ void put_row4(uint8_t* tile, const RowMap& m, int i, const float4& v) {
+  *reinterpret_cast<uint2*>(tile + (m.col >> 6) * CHUNK_BYTES + row_swz(m, i, (m.col & 63) >> 3) + ((m.col >> 2) & 1) * 8) =
+      make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
 }
 // The descriptor of an MN-major operand (two 64-wide atoms CHUNK_BYTES apart): see mma_one for the rest.
 __device__ __forceinline__ uint32_t desc_mn(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | ((CHUNK_BYTES >> 4) << 16); }

@@ -41,10 +41,11 @@ template <int W>
 __device__ __forceinline__ void rows_in(float* dst, int ld, const float* src, int rows) {
   for (int i = threadIdx.x; i < rows * (W / 4); i += THREADS) copy16(dst + (i / (W / 4)) * ld + (i % (W / 4)) * 4, src + (size_t)i * 4);
 }
-template <int W>
-__device__ __forceinline__ void rows_out(float* dst, const float* src, int ld, int rows) {
-  for (int i = threadIdx.x; i < rows * (W / 4); i += THREADS)
-    reinterpret_cast<float4*>(dst)[i] = *reinterpret_cast<const float4*>(src + (i / (W / 4)) * ld + (i % (W / 4)) * 4);
+// The q-th (mod PARTS * 32) four columns of a row of PARTS parts of D columns.
+template <int PARTS>
+__device__ __forceinline__ float4* parts_at(float* base, int ld, size_t off, size_t row, int q) {
+  q %= PARTS * (D / 4);
+  return reinterpret_cast<float4*>(base + row * ld + (q / (D / 4)) * off) + q % (D / 4);
 }
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float dot4(const float4& a, const float4& b, float s) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, s)))); }
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(THREADS, BULLETS || LPP == 32 ? 4 : LPP == 16 
     // slots that are no keys have no gradient
     const uint8_t* on = c.bactive ? c.bactive + g * c.nb : nullptr;
     for (int i = threadIdx.x; on && i < c.nb * (2 * D / 4); i += THREADS)
-      if (!on[i / (2 * D / 4)]) reinterpret_cast<float4*>(c.dkvb + g * c.nb * 2 * D)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (const int r = i / (2 * D / 4); !on[r]) *parts_at<2>(c.dkvb, c.ld_dkvb, c.off_dkvb, g * c.nb + r, i) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   copies_done();
   float* q = s.rows + h * DH;
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(THREADS, BULLETS || LPP == 32 ? 4 : LPP == 16 
       __syncthreads();
       for (int i = threadIdx.x; i < kn * (2 * D / 4); i += THREADS) {
         const int r = i / (2 * D / 4), qq = i % (2 * D / 4);
-        reinterpret_cast<float4*>(c.dkvb + (g * c.nb + s.list[k0 + r]) * 2 * D)[qq] = ld4(s.kv + r * LDB + qq * 4);
+        *parts_at<2>(c.dkvb, c.ld_dkvb, c.off_dkvb, g * c.nb + s.list[k0 + r], qq) = ld4(s.kv + r * LDB + qq * 4);
       }
     }
   }
@@ -400,7 +401,10 @@ __global__ void __launch_bounds__(THREADS, BULLETS || LPP == 32 ? 4 : LPP == 16 
       }
   }
   __syncthreads();
-  rows_out<3 * D>(c.dqkv + tok0 * 3 * D, s.rows, LDQ, n);
+  for (int i = threadIdx.x; i < n * (3 * D / 4); i += THREADS) {
+    const int r = i / (3 * D / 4), qq = i % (3 * D / 4);
+    *parts_at<3>(c.dqkv, c.ld_dqkv, c.off_dqkv, tok0 + r, qq) = ld4(s.rows + r * LDQ + qq * 4);
+  }
 }
 
 constexpr size_t SMEM_MAX = 200 * 1024;

@@ -15,9 +15,11 @@ struct Call {
   const uint8_t* bactive;   // (G * nb) or null: every slot is a key
   int G, n, nb;
   float* o;                 // forward: (G * n, 128)
-  const float* d_o;         // gradient: (G * n, 128) in; (G * n, 384) and (G * nb, 256) out
+  const float* d_o;         // gradient: (G * n, 128) in; out q | k | v and keys | values, rows ld apart, the parts off apart
   float* dqkv;
   float* dkvb;
+  int ld_dqkv, ld_dkvb;
+  size_t off_dqkv, off_dkvb;
 };
 
 // d_model 128, 4 heads, up to 32 tokens per environment.

@@ -8,18 +8,16 @@
 //   k_linear_bwd   gradient with respect to the input and the weights of up to three layers from one reading of
 //                  their dy, bias gradients as column sums on the way, and the norm's gradient as the epilogue
 //
-// Persistent CTAs, one per SM: the weights stay in shared memory, row tiles of 128 pass by.  Rows are on their way in
-// registers (64 KB per SM) while the tile before is worked on.  The weight images are plain K-major tiles; backward
-// reads them as MN-major operands (dn = dy W needs W's other direction), and dy and n as MN-major operands for
-// d W = dy^T n, whose accumulator stays in tensor memory over all tiles of a CTA.
+// Persistent CTAs, one per SM: the weights stay in shared memory, row tiles of 128 pass by.  The weight images are plain
+// K-major tiles; backward reads them as MN-major operands (dn = dy W needs W's other direction), and dy and n as MN-major
+// operands for d W = dy^T n, whose accumulator stays in tensor memory over all tiles of a CTA.
 //
 // 262 144 rows: forward and backward of a temporal sublayer's Linears and norm took 13 launches of mma.sync
 // products, each reading and writing its operands for itself.
 //
-// What bounds them now is the latency of the row loads, not the copy rate: for 65 536 rows the forward of three layers
-// takes 38 us at 30 % of DRAM's peak and of one layer 24 us at 36 %, the backward of one layer 36 us at 24 %, of two gates
-// 59 us at 31 %, of two layers with their norm 83 us at 26 %; 14 to 20 of 25 to 30 cycles between two issues of a warp are
-// waits for global and tensor memory, because a tile's tensors are requested one after the other into registers.
+// What bounds them is memory: for 262 144 rows the forward of three layers takes 117 us (603 MB, 5.2 TB/s) and of one 71 (403 MB, 5.7),
+// the backward of one layer 80 us (403 MB, 5.0), of two gates 111 (671 MB, 6.0), of two layers with their norm 157 (738 MB, 4.7), of
+// three with theirs 191 (872 MB, 4.6).  Backward through registers, a tensor of a tile behind the other, took 91, 178, 263 and 326.
 #include "train_linear.h"
 
 #include "launch_after.h"
@@ -48,7 +46,6 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackJobs j
 
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void store4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void put_row4(uint8_t* tile, int row, int col, const float4& v) { put4(tile, row, col, v.x, v.y, v.z, v.w); }
 __device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
 // ------------------------------------------------------------------ forward
@@ -149,7 +146,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_fwd(const __grid_constant
         for (int k = 0; k < 8; ++k) {
           inv[k] = rsqrtf(inv[k] / (float)D + kRmsEps);
           const uint2 n = make_uint2(pack_bf16(x[k].x * inv[k] * gain.x, x[k].y * inv[k] * gain.y), pack_bf16(x[k].z * inv[k] * gain.z, x[k].w * inv[k] * gain.w));
-          *reinterpret_cast<uint2*>(tile + (m.col >> 6) * CHUNK_BYTES + swz(m.row(k), (m.col & 63) >> 3) + ((m.col >> 2) & 1) * 8) = n;
+          *reinterpret_cast<uint2*>(tile + (m.col >> 6) * CHUNK_BYTES + row_swz(m, k, (m.col & 63) >> 3) + ((m.col >> 2) & 1) * 8) = n;
           const int r = first + m.row(k);
           if (r >= a.rows) continue;
           *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.f.n_out) + (size_t)r * D + m.col) = n;
@@ -157,7 +154,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_fwd(const __grid_constant
         }
       } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) put_row4(tile, m.row(k), m.col, x[k]);
+        for (int k = 0; k < 8; ++k) put_row4(tile, m, k, x[k]);
       }
       post(s, F_OP0 + set_of(i));
       if (i + 1 < my_tiles) rows_in(x, a.f.x, m, (blockIdx.x + (i + 1) * gridDim.x) * TILE, a.rows);
@@ -177,16 +174,25 @@ struct BwdArgs {
   int* status;
   int* host_status;
 };
-// Shared memory: weights, two dy tiles, one n tile, transposing stages (2 KB per warp: 16 columns), row sums, frame.
+// Shared memory: weights, the operand tiles of dy and n, float32 rows on their way, row sums, frame.  The rows: pieces of
+// 16 rows (8 KB), SLOTS of them for each group of four warps, which reads 32 rows of a tile.
+constexpr int PIECE_ROWS = 16, PIECE_BYTES = PIECE_ROWS * D * 4;
 template <int NB> struct BwdMap {
-  static constexpr uint32_t DY = NB * TILE_BYTES, N = DY + 2 * TILE_BYTES, STAGE = N + TILE_BYTES, SUMS = STAGE + 32768, FRAME = SUMS + 2048,
+  static constexpr int SLOTS = NB == 3 ? 2 : 3;
+  static constexpr uint32_t DY = NB * TILE_BYTES, N = DY + TILE_BYTES, RAW = N + TILE_BYTES, SUMS = RAW + 4 * SLOTS * PIECE_BYTES, FRAME = SUMS + 2048,
                             BYTES = FRAME + FRAME_BYTES;
+  static constexpr int FREE = 3 + 4 * SLOTS, COUNT = FREE + 4 * SLOTS;   // barriers behind G_FULL
 };
-enum : int { G_W = 0, G_OP0, G_ACC = G_OP0 + 2, G_FREE0, G_COUNT = G_FREE0 + 2 };   // operand and slot barriers per dy tile
+enum : int { G_W = 0, G_OP, G_DONE, G_FULL };   // weights, dy tile written, its products complete, pieces
 
-// Sixteen accumulator columns of 32 rows into the row layout: lane l of the i-th request (i < 8) holds columns
-// 4 (l % 8) .. of row 4 i + l / 8, so each half fills the lanes of its four column groups.
-__device__ __forceinline__ void unstage(float4 (&v)[8], uint32_t taddr, uint8_t* stage, const RowMap& m) {
+// Sixteen accumulator columns of 32 rows at a time into the row layout: lane l of the i-th request (i < 8) holds columns
+// 4 (l % 8) .. of row 4 i + l / 8, so each half fills the lanes of its four column groups.  Through the memory that only
+// this warp writes of the dy tile (64 bytes of its 32 rows).  ADD: onto what v holds.
+template <bool ADD>
+__device__ __forceinline__ void unstage(float4 (&v)[8], uint32_t taddr, uint8_t* dy_tile, const RowMap& m) {
+  const int part = threadIdx.x >> 7;
+  uint8_t* stage = dy_tile + (part >> 1) * CHUNK_BYTES;
+  const int g0 = 4 * (part & 1);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     uint32_t t[16];
@@ -195,23 +201,33 @@ __device__ __forceinline__ void unstage(float4 (&v)[8], uint32_t taddr, uint8_t*
     __syncwarp();
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      *reinterpret_cast<uint4*>(stage + m.lane * 64 + ((q ^ ((m.lane >> 1) & 3)) << 4)) = make_uint4(t[4 * q], t[4 * q + 1], t[4 * q + 2], t[4 * q + 3]);
+      *reinterpret_cast<uint4*>(stage + swz(m.row0 + m.lane, g0 + q)) = make_uint4(t[4 * q], t[4 * q + 1], t[4 * q + 2], t[4 * q + 3]);
     __syncwarp();
     if (((m.lane >> 2) & 1) == h)
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const int r = 4 * i + (m.lane >> 3);
-        v[i] = *reinterpret_cast<const float4*>(stage + r * 64 + (((m.lane & 3) ^ ((r >> 1) & 3)) << 4));
+        const float4 t4 = *reinterpret_cast<const float4*>(stage + row_swz(m, i, g0 + (m.lane & 3)));
+        v[i] = ADD ? add4(v[i], t4) : t4;
       }
   }
+  __syncwarp();
 }
 
 // NB blocks; NORM: n is bfloat16 and dn goes through the norm's gradient; otherwise n is float32.
+//
+// The fetching warp keeps the float32 rows of everything a tile reads on their way through shared memory, piece by piece, in the
+// order of their use: of dy0 .. dy(NB - 1), x, d residual with norm, of n, dy0 .. , dx before without.  A tile of three layers
+// with norm took 41 000 cycles with its loads one behind the other (d residual row by row between the stores), 31 000 with
+// loads into registers two tensors ahead, and takes 27 000 of which 17 000 are waits for pieces (416 KB: 19 000 at the copy
+// rate).  Every tensor is rows of 128 floats one behind the other: d q | d k | d v side by side in rows of 384 came as 512-byte
+// copies, 45 cycles each (39 000 cycles a tile).
 template <int NB, bool NORM>
 __global__ void __launch_bounds__(THREADS, 1) k_linear_bwd(const __grid_constant__ BwdArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   using Map = BwdMap<NB>;
-  const int counts[G_COUNT] = {1, EPI_WARPS, EPI_WARPS, 1, 1, 1};
+  int counts[Map::COUNT];
+#pragma unroll
+  for (int i = 0; i < Map::COUNT; ++i) counts[i] = i == G_OP ? EPI_WARPS : i >= Map::FREE ? 4 : 1;
   const Frame f = open_frame(smem + Map::FRAME, a.status, a.host_status, counts);
   const Sync s{smem_u32(f.bars), a.status, f.aborted};
   const uint32_t tmem = *f.tmem_slot, base = smem_u32(smem);
@@ -224,122 +240,177 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_bwd(const __grid_constant
       for (int b = 0; b < NB; ++b) bulk_g2s(base + b * TILE_BYTES, a.b.image + (size_t)b * BLOCK_IMAGE, TILE_BYTES, s.bars + 8 * G_W);
     }
     __syncwarp();
+    // eight lanes for each group's pieces
+    const int group = (tid & 31) >> 3, sub = tid & 7;
+    int slot = 0;
+    uint32_t free_parity = 1;   // a fresh barrier passes a wait on parity 1
+    auto stream = [&](int tile, const float* src) {
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        const int bar = group * Map::SLOTS + slot, row = tile * TILE + 32 * group + PIECE_ROWS * h;
+        const int n = min(max(a.rows - row, 0), PIECE_ROWS);
+        const uint32_t full = s.bars + 8 * (G_FULL + bar);
+        s.wait(Map::FREE + bar, free_parity, TIMEOUT_FREE);
+        if (__any_sync(0xffffffffu, s.aborted[0])) return false;
+        if (sub == 0) {
+          mbar_expect_tx(full, n * D * 4);
+          if (n > 0) bulk_g2s(base + Map::RAW + bar * PIECE_BYTES, src + (size_t)row * D, n * D * 4, full);
+        }
+        __syncwarp();
+        if (++slot == Map::SLOTS) { slot = 0; free_parity ^= 1u; }
+      }
+      return true;
+    };
+    bool go = true;
+#pragma unroll 1
+    for (int i = 0; i < my_tiles && go; ++i) {
+      const int tile = blockIdx.x + i * gridDim.x;
+      if (!NORM) go = stream(tile, static_cast<const float*>(a.b.n));
+#pragma unroll 1
+      for (int b = 0; b < NB && go; ++b) go = stream(tile, a.b.dy[b]);
+      if (NORM && go) go = stream(tile, a.b.x);
+      const float* last = NORM ? a.b.dres : a.b.accumulate ? a.b.dx : nullptr;
+      if (last && go) go = stream(tile, last);
+    }
     s.wait(G_W, 0, TIMEOUT_FULL);
   } else if (warp == MMA_WARP) {
     const uint32_t el = elect_one(), tm = uniform(tmem), idesc = instr_desc(128);
-    const uint32_t n_mn = desc_mn(base + Map::N);
+    const uint32_t n_mn = desc_mn(base + Map::N), dy_lo = desc_lo(base + Map::DY), dy_mn = desc_mn(base + Map::DY);
     s.wait(G_W, 0, TIMEOUT_FULL);
-    int item = 0;
+    uint32_t item = 0;
 #pragma unroll 1
     for (int i = 0; i < my_tiles; ++i)
 #pragma unroll 1
       for (uint32_t b = 0; b < NB; ++b, ++item) {
-        const uint32_t dy = base + Map::DY + (item & 1) * TILE_BYTES;
-        s.wait(G_OP0 + (item & 1), item >> 1, TIMEOUT_OPERAND);
+        s.wait(G_OP, item, TIMEOUT_OPERAND);
         tc_fence_after();
-        const uint32_t dy_lo = uniform(desc_lo(dy)), dy_mn = uniform(desc_mn(dy)), w_mn = uniform(desc_mn(base + b * TILE_BYTES));
+        const uint32_t w_mn = uniform(desc_mn(base + b * TILE_BYTES));
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k)   // dn += dy W: K = the block's output features
           mma_one<false>(el, tm + 384, dy_lo + (k >> 2) * 1024 + 2 * (k & 3), w_mn + 128 * k, idesc | (1u << 16), (b | k) ? 1u : 0u);
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k)   // d W += dy^T n: K = rows
           mma_one<false>(el, tm + 128 * b, dy_mn + 128 * k, n_mn + 128 * k, idesc | BOTH_MN, (i | (int)k) ? 1u : 0u);
-        tc_commit_if(el, s.bars + 8 * (G_FREE0 + (item & 1)));
-        if (b == NB - 1) tc_commit_if(el, s.bars + 8 * G_ACC);
+        tc_commit_if(el, s.bars + 8 * G_DONE);
       }
-    if (my_tiles > 0) s.wait(G_ACC, my_tiles - 1, TIMEOUT_ACC);
+    if (item > 0) s.wait(G_DONE, item - 1, TIMEOUT_ACC);
   } else {
     const RowMap m = row_map();
-    const int part = warp >> 2;
-    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    uint8_t* stage = smem + Map::STAGE + warp * 2048;
+    const int part = warp >> 2, group = warp & 3;
+    const uint32_t lane_addr = tmem + ((uint32_t)(group * 32) << 16);
     float* sums = reinterpret_cast<float*>(smem + Map::SUMS);
     float4 gsum = make_float4(0.f, 0.f, 0.f, 0.f), bsum[NB];
 #pragma unroll
     for (int b = 0; b < NB; ++b) bsum[b] = gsum;
-    float4 dy[8];
-    auto request = [&](int tile, const float* src) {
+    int slot = 0;
+    uint32_t parity = 0, item = 0;
+    // The next piece of this group, used by four calls of `row` with its place in the tile and this lane's columns there.
+    auto piece = [&](int first, int h, auto row) {
+      const int bar = group * Map::SLOTS + slot;
+      s.wait(G_FULL + bar, parity, TIMEOUT_FULL);
+      const uint8_t* at = smem + Map::RAW + bar * PIECE_BYTES + (m.lane >> 3) * (D * 4) + m.col * 4;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float4 v = *reinterpret_cast<const float4*>(at + 4 * k * (D * 4));
+        row(4 * h + k, first + m.row(4 * h + k) < a.rows ? v : make_float4(0.f, 0.f, 0.f, 0.f));
+      }
+      __syncwarp();
+      if (m.lane == 0) mbar_arrive(s.bars + 8 * (Map::FREE + bar));
+      if (++slot == Map::SLOTS) { slot = 0; parity ^= 1u; }
+    };
+    auto take = [&](float4 (&to)[8], int first) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) piece(first, h, [&](int k, const float4& v) { to[k] = v; });
+    };
+    // dy of block b as an operand; the products that read the tile before are complete
+    auto place = [&](const float4 (&from)[8], int b) {
+      if (b > 0) s.wait(G_DONE, item - 1, TIMEOUT_FREE);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int r = tile * TILE + m.row(k);
-        dy[k] = r < a.rows ? load4(src + (size_t)r * a.b.ld_dy + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
+        put_row4(smem + Map::DY, m, k, from[k]);
+        if (!NORM) bsum[b] = add4(bsum[b], from[k]);
+      }
+      post(s, G_OP);
+      ++item;
+    };
+    // bfloat16 n of a tile: this warp's 32 rows of 64 bytes as they are, zeros past the last row
+    auto copy_n = [&](int tile) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int row = m.row0 + 8 * k + (m.lane >> 2), r = tile * TILE + row, g = 4 * part + (m.lane & 3);
+        const uint32_t dst = smem_u32(smem + Map::N + (part >> 1) * CHUNK_BYTES + swz(row, g & 7));
+        const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.b.n) + (size_t)(r < a.rows ? r : 0) * D + 8 * g;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(r < a.rows ? 16 : 0) : "memory");
       }
     };
-    if (my_tiles > 0) request(blockIdx.x, a.b.dy[0]);
-    int item = 0;
+    const float4 gain = NORM ? load4(a.b.gain + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (NORM && my_tiles > 0) copy_n(blockIdx.x);
 #pragma unroll 1
     for (int i = 0; i < my_tiles; ++i) {
       const int tile = blockIdx.x + i * gridDim.x, first = tile * TILE;
-      // One layer: the next tile's rows on their way to L2 (98 -> 90 us; the kernels with more registers in use lost 10 %).
-      if (NB == 1 && tid == 0) {
-        prefetch_rows(a.b.dy[0], tile + gridDim.x, a.rows, D * 4);
-        prefetch_rows(a.b.n, tile + gridDim.x, a.rows, D * 4);
-        if (a.b.accumulate) prefetch_rows(a.b.dx, tile + gridDim.x, a.rows, D * 4);
-      }
-#pragma unroll
-      for (int b = 0; b < NB; ++b, ++item) {
-        if (b == 0) {   // n of the tile; the products of the tile before are complete
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int r = first + m.row(k);
-            if constexpr (NORM) {
-              const uint2 v = r < a.rows ? *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(a.b.n) + (size_t)r * D + m.col) : make_uint2(0u, 0u);
-              *reinterpret_cast<uint2*>(smem + Map::N + (m.col >> 6) * CHUNK_BYTES + swz(m.row(k), (m.col & 63) >> 3) + ((m.col >> 2) & 1) * 8) = v;
-            } else {
-              put_row4(smem + Map::N, m.row(k), m.col,
-                       r < a.rows ? load4(static_cast<const float*>(a.b.n) + (size_t)r * D + m.col) : make_float4(0.f, 0.f, 0.f, 0.f));
-            }
-          }
-        }
-        if (item >= 2) s.wait(G_FREE0 + (item & 1), (item >> 1) - 1, TIMEOUT_FREE);
-        uint8_t* at = smem + Map::DY + (item & 1) * TILE_BYTES;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          put_row4(at, m.row(k), m.col, dy[k]);
-          if (!NORM) bsum[b] = add4(bsum[b], dy[k]);
-        }
-        post(s, G_OP0 + (item & 1));
-        if (b + 1 < NB) request(tile, a.b.dy[b + 1]);
-        else if (!NORM && i + 1 < my_tiles) request(tile + gridDim.x, a.b.dy[0]);
-      }
-      float4 x[8], dn[8];
-      float iv[8];
+      float4 u[8], v[8];
+      float inv = 0.f;   // of the row that is this lane's among the warp's
+      if (NORM && first + m.row0 + m.lane < a.rows) inv = a.b.inv[first + m.row0 + m.lane];
+      take(u, first);
       if constexpr (NORM) {
-        rows_in(x, a.b.x, m, first, a.rows);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) iv[k] = first + m.row(k) < a.rows ? a.b.inv[first + m.row(k)] : 0.f;
-      }
-      s.wait(G_ACC, i, TIMEOUT_ACC);
-      tc_fence_after();
-      unstage(dn, lane_addr + 384 + part * 32, stage, m);
-      tc_fence_before();
-      if constexpr (NORM) {
-        const float4 gain = load4(a.b.gain + m.col);
-        float coef[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          coef[k] = fmaf(x[k].x * gain.x, dn[k].x, fmaf(x[k].y * gain.y, dn[k].y, fmaf(x[k].z * gain.z, dn[k].z, x[k].w * gain.w * dn[k].w)));
-        row_sums(coef, sums, m);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int r = first + m.row(k);
-          if (r >= a.rows) continue;
-          const float v = iv[k], c = coef[k] * v * v * v * (1.0f / D);
-          float4 d = a.b.dres ? load4(a.b.dres + (size_t)r * D + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
-          d.x += v * gain.x * dn[k].x - x[k].x * c; d.y += v * gain.y * dn[k].y - x[k].y * c;
-          d.z += v * gain.z * dn[k].z - x[k].z * c; d.w += v * gain.w * dn[k].w - x[k].w * c;
-          store4(a.b.dx + (size_t)r * D + m.col, d);
-          gsum.x = fmaf(dn[k].x * x[k].x, v, gsum.x); gsum.y = fmaf(dn[k].y * x[k].y, v, gsum.y);
-          gsum.z = fmaf(dn[k].z * x[k].z, v, gsum.z); gsum.w = fmaf(dn[k].w * x[k].w, v, gsum.w);
-        }
-        if (i + 1 < my_tiles) request(tile + gridDim.x, a.b.dy[0]);
+        asm volatile("cp.async.wait_all;" ::: "memory");   // n
       } else {
 #pragma unroll
+        for (int k = 0; k < 8; ++k) put_row4(smem + Map::N, m, k, u[k]);   // the products of the tile before are complete
+        take(u, first);
+      }
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        place(u, b);
+        if (b + 1 < NB) take(u, first);
+      }
+      if constexpr (NORM) {
+        take(v, first);   // x
+        s.wait(G_DONE, item - 1, TIMEOUT_ACC);
+        tc_fence_after();
+        if (i + 1 < my_tiles) copy_n(tile + gridDim.x);
+        unstage<false>(u, lane_addr + 384 + part * 32, smem + Map::DY, m);
+        tc_fence_before();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {   // sums of x gain dn over a row: eight lanes here, the four warps of the row through shared memory
+          float c = fmaf(v[k].x * gain.x, u[k].x, fmaf(v[k].y * gain.y, u[k].y, fmaf(v[k].z * gain.z, u[k].z, v[k].w * gain.w * u[k].w)));
+#pragma unroll
+          for (int o = 1; o < 8; o <<= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+          if ((m.lane & 7) == 0) sums[part * TILE + m.row(k)] = c;
+        }
+        // its next use comes behind a wait for products that every warp of these rows has to post for
+        asm volatile("bar.sync %0, 128;" ::"r"(3 + group) : "memory");
+        auto out = [&](int k, float4 d) {   // d: residual
+          const int r = first + m.row(k);
+          const float* p = sums + m.row(k);
+          const float w = __shfl_sync(0xffffffffu, inv, 4 * k + (m.lane >> 3)), c = ((p[0] + p[TILE]) + (p[2 * TILE] + p[3 * TILE])) * w * w * w * (1.0f / D);
+          if (r >= a.rows) return;
+          d.x += w * gain.x * u[k].x - v[k].x * c; d.y += w * gain.y * u[k].y - v[k].y * c;
+          d.z += w * gain.z * u[k].z - v[k].z * c; d.w += w * gain.w * u[k].w - v[k].w * c;
+          store4(a.b.dx + (size_t)r * D + m.col, d);
+          gsum.x = fmaf(u[k].x * v[k].x, w, gsum.x); gsum.y = fmaf(u[k].y * v[k].y, w, gsum.y);
+          gsum.z = fmaf(u[k].z * v[k].z, w, gsum.z); gsum.w = fmaf(u[k].w * v[k].w, w, gsum.w);
+        };
+        if (a.b.dres) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) piece(first, h, out);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) out(k, make_float4(0.f, 0.f, 0.f, 0.f));
+        }
+      } else {
+        if (a.b.accumulate) take(v, first);
+        else
+#pragma unroll
+          for (int k = 0; k < 8; ++k) v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        s.wait(G_DONE, item - 1, TIMEOUT_ACC);
+        tc_fence_after();
+        unstage<true>(v, lane_addr + 384 + part * 32, smem + Map::DY, m);
+        tc_fence_before();
+#pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int r = first + m.row(k);
-          if (r >= a.rows) continue;
-          float* p = a.b.dx + (size_t)r * D + m.col;
-          store4(p, a.b.accumulate ? add4(load4(p), dn[k]) : dn[k]);
+          if (r < a.rows) store4(a.b.dx + (size_t)r * D + m.col, v[k]);
         }
       }
     }

@@ -37,7 +37,6 @@ struct Forward {
 // dx may be dres.
 struct Backward {
   const float* dy[MAX_BLOCKS] = {};
-  int ld_dy = 128;
   const void* n = nullptr;
   const uint8_t* image = nullptr;
   int blocks = 1;

@@ -133,7 +133,7 @@ __device__ __forceinline__ void norm_rows(uint8_t* tile, const float4 (&x)[8], f
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     inv[i] = rsqrtf(inv[i] * (1.0f / D) + kRmsEps);
-    put4(tile, m.row(i), m.col, x[i].x * inv[i] * gain.x, x[i].y * inv[i] * gain.y, x[i].z * inv[i] * gain.z, x[i].w * inv[i] * gain.w);
+    put_row4(tile, m, i, make_float4(x[i].x * inv[i] * gain.x, x[i].y * inv[i] * gain.y, x[i].z * inv[i] * gain.z, x[i].w * inv[i] * gain.w));
   }
 }
 // One fetch by the fetching warp: wait for the slot, copy, signal.  Stops after a wait has run out.
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
         norm_rows(smem, x, inv, gain, sums, m);
         rows_in(x, a.dy, m, tile * TILE, a.rows);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) put4(smem + DX_DY, m.row(i), m.col, x[i].x, x[i].y, x[i].z, x[i].w);
+        for (int i = 0; i < 8; ++i) put_row4(smem + DX_DY, m, i, x[i]);
       }
       post(s, XB_OP);
       epi_sync();
