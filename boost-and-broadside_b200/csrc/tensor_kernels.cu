@@ -163,7 +163,7 @@ __global__ void k_pack_trunk(const __grid_constant__ PackJobs jobs) {
 //
 // One CTA per (environment, head): q, k, v of that head are staged from the bf16 scratch the
 // PRE phase wrote, then each warp takes blocks of 16 query rows and walks the keys in blocks of
-// 32 with a running maximum (mma.sync, fp32 softmax).  Dead keys score kMaskedScore, so their
+// 32 (the last up to 16 by themselves) with a running maximum (mma.sync, fp32 softmax).  Dead keys score kMaskedScore, so their
 // weight is exactly 0 unless no key of the environment is alive, in which case every key gets
 // the same weight (models/yemong/attention.py:101-112 of the reference).  When the sublayer
 // reads bullets, the environment's bullet keys and values (written by bullet_kv.cu) are
@@ -173,97 +173,124 @@ __global__ void k_pack_trunk(const __grid_constant__ PackJobs jobs) {
 // a staged row holds HPC x 32 bf16 plus 16 bytes of padding, which keeps ldmatrix conflict-free.
 __host__ __device__ constexpr int flash_stride(int hpc) { return hpc * 64 + 16; }
 
-// One softmax pass of a block of 16 queries (fragments qa) over n keys staged at sK / sV; returns
-// the normalised output fragments in acc.  Keys are walked 32 at a time.  `bias` holds one float
-// per key, padded to a multiple of 32: 0 for a live key, kMaskedScore for a dead one, -inf beyond
-// n.  Scores are carried in the log2 domain: t = (q.k) * log2(e) / sqrt(32) + bias, p = 2^(t - max).
-__device__ __forceinline__ void flash_pass(const uint32_t (&qa)[2][4], uint32_t sK, uint32_t sV, int stride,
-                                           const float* __restrict__ bias, int n, int lane, float (&acc)[4][4]) {
-  const int t = lane & 3;
-  const float c2 = 0.17677669529663687f * 1.4426950408889634f;
-  const int last = n - 1;
-  const int nkb = (n + 31) >> 5;
-  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+// Running softmax of a block of 16 queries: a lane's two query rows, sums of its own columns in pairs.
+struct FlashState {
+  float m[2];
+  F2 l[2];
+  float acc[4][4];
+};
+// One block of 8 NT keys from key0 on (at least one of them a key).  k and v: staged rows at this head and this lane's ldmatrix
+// column.  bias: one float per key, 0 for a live one, kMaskedScore for a dead one, -inf past the last.  Scores are carried in the log2
+// domain: t = (q.k) * log2(e) / sqrt(32) + bias, p = 2^(t - max).  FIRST: nothing to rescale.
+template <int HPC, int NT, bool FIRST>
+__device__ __forceinline__ void flash_block(FlashState& f, const uint32_t (&qa)[2][4], uint32_t k, uint32_t v, const float* bias, int key0, int last, int lane) {
+  constexpr int STRIDE = flash_stride(HPC);
+  float sc[NT][4];
 #pragma unroll
-  for (int nt = 0; nt < 4; ++nt)
+  for (int h = 0; h < NT / 2; ++h) {
+    const uint32_t row = k + min(key0 + h * 16 + (lane >> 4) * 8 + (lane & 7), last) * STRIDE;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
-  for (int kb = 0; kb < nkb; ++kb) {
-    float sc[4][4];
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) sc[nt][i] = 0.f;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int krow = min(kb * 32 + h * 16 + (lane >> 4) * 8 + (lane & 7), last);
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        uint32_t b0, b1, b2, b3;
-        ldsm_x4(sK + krow * stride + (ks * 16 + ((lane >> 3) & 1) * 8) * 2, b0, b1, b2, b3);
+    for (int ks = 0; ks < 2; ++ks) {
+      uint32_t b0, b1, b2, b3;
+      ldsm_x4(row + ks * 32, b0, b1, b2, b3);
+      if (ks == 0) {
+        mma_bf16_fresh(sc[2 * h], qa[ks], b0, b1);
+        mma_bf16_fresh(sc[2 * h + 1], qa[ks], b2, b3);
+      } else {
         mma_bf16(sc[2 * h], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
         mma_bf16(sc[2 * h + 1], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b2, b3);
       }
     }
-    float bm0 = -INFINITY, bm1 = -INFINITY;
+  }
+  const F2 c2 = f2(0.17677669529663687f * 1.4426950408889634f);
+  F2 t[NT][2];
+  float m0 = -INFINITY, m1 = -INFINITY;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    // a dead key's bias swallows its score: kMaskedScore exactly (weight 0 unless every key is dead)
+    F2 bj;
+    bj.v = *reinterpret_cast<const unsigned long long*>(bias + key0 + nt * 8 + 2 * (lane & 3));
+    t[nt][0] = fma(f2(sc[nt][0], sc[nt][1]), c2, bj);
+    t[nt][1] = fma(f2(sc[nt][2], sc[nt][3]), c2, bj);
+    const float2 a = halves(t[nt][0]), b = halves(t[nt][1]);
+    m0 = fmaxf(m0, fmaxf(a.x, a.y));
+    m1 = fmaxf(m1, fmaxf(b.x, b.y));
+  }
+  m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, 1));
+  m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, 2));
+  m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, 1));
+  m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, 2));
+  if constexpr (!FIRST) {
+    m0 = fmaxf(m0, f.m[0]);
+    m1 = fmaxf(m1, f.m[1]);
+    const F2 c0 = f2(ex2_fast(f.m[0] - m0)), c1 = f2(ex2_fast(f.m[1] - m1));
+    f.l[0] = mul(f.l[0], c0);
+    f.l[1] = mul(f.l[1], c1);
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
-      // a dead key's bias swallows its score: kMaskedScore exactly (weight 0 unless every key is dead)
-      const float2 bj = *reinterpret_cast<const float2*>(bias + kb * 32 + nt * 8 + 2 * t);
-      sc[nt][0] = fmaf(sc[nt][0], c2, bj.x);
-      sc[nt][1] = fmaf(sc[nt][1], c2, bj.y);
-      sc[nt][2] = fmaf(sc[nt][2], c2, bj.x);
-      sc[nt][3] = fmaf(sc[nt][3], c2, bj.y);
-      bm0 = fmaxf(bm0, fmaxf(sc[nt][0], sc[nt][1]));
-      bm1 = fmaxf(bm1, fmaxf(sc[nt][2], sc[nt][3]));
+      const float2 a = halves(mul(f2(f.acc[nt][0], f.acc[nt][1]), c0)), b = halves(mul(f2(f.acc[nt][2], f.acc[nt][3]), c1));
+      f.acc[nt][0] = a.x; f.acc[nt][1] = a.y; f.acc[nt][2] = b.x; f.acc[nt][3] = b.y;
     }
-    bm0 = fmaxf(bm0, __shfl_xor_sync(0xffffffffu, bm0, 1));
-    bm0 = fmaxf(bm0, __shfl_xor_sync(0xffffffffu, bm0, 2));
-    bm1 = fmaxf(bm1, __shfl_xor_sync(0xffffffffu, bm1, 1));
-    bm1 = fmaxf(bm1, __shfl_xor_sync(0xffffffffu, bm1, 2));
-    const float n0 = fmaxf(m0, bm0), n1 = fmaxf(m1, bm1);       // finite: every block holds a valid key
-    const float c0 = ex2_fast(m0 - n0), c1 = ex2_fast(m1 - n1); // 2^(-inf) = 0 on the first block
-    m0 = n0;
-    m1 = n1;
-    l0 *= c0;
-    l1 *= c1;
+  }
+  f.m[0] = m0;
+  f.m[1] = m1;
+  uint32_t p[NT][2];
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      acc[nt][0] *= c0; acc[nt][1] *= c0;
-      acc[nt][2] *= c1; acc[nt][3] *= c1;
+  for (int r = 0; r < 2; ++r) {
+    const F2 shift = f2(-f.m[r]);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const float2 d = halves(add(t[nt][r], shift));
+      const F2 e = f2(ex2_fast(d.x), ex2_fast(d.y));
+      f.l[r] = FIRST && nt == 0 ? e : add(f.l[r], e);
+      p[nt][r] = pack_bf16(e);
     }
+  }
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      sc[nt][0] = ex2_fast(sc[nt][0] - m0);
-      sc[nt][1] = ex2_fast(sc[nt][1] - m0);
-      sc[nt][2] = ex2_fast(sc[nt][2] - m1);
-      sc[nt][3] = ex2_fast(sc[nt][3] - m1);
-      l0 += sc[nt][0] + sc[nt][1];
-      l1 += sc[nt][2] + sc[nt][3];
-    }
+  for (int h = 0; h < NT / 2; ++h) {
+    const uint32_t row = v + min(key0 + h * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), last) * STRIDE;
+    const uint32_t a[4] = {p[2 * h][0], p[2 * h][1], p[2 * h + 1][0], p[2 * h + 1][1]};
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t a0 = pack_bf16(sc[2 * h][0], sc[2 * h][1]), a1 = pack_bf16(sc[2 * h][2], sc[2 * h][3]);
-      const uint32_t a2 = pack_bf16(sc[2 * h + 1][0], sc[2 * h + 1][1]), a3 = pack_bf16(sc[2 * h + 1][2], sc[2 * h + 1][3]);
-      const int vrow = min(kb * 32 + h * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), last);
-#pragma unroll
-      for (int np = 0; np < 2; ++np) {
-        uint32_t b0, b1, b2, b3;
-        ldsm_x4_t(sV + vrow * stride + ((np * 2 + (lane >> 4)) * 8) * 2, b0, b1, b2, b3);
-        mma_bf16(acc[np * 2], a0, a1, a2, a3, b0, b1);
-        mma_bf16(acc[np * 2 + 1], a0, a1, a2, a3, b2, b3);
+    for (int np = 0; np < 2; ++np) {
+      uint32_t b0, b1, b2, b3;
+      ldsm_x4_t(row + np * 32, b0, b1, b2, b3);
+      if (FIRST && h == 0) {
+        mma_bf16_fresh(f.acc[np * 2], a, b0, b1);
+        mma_bf16_fresh(f.acc[np * 2 + 1], a, b2, b3);
+      } else {
+        mma_bf16(f.acc[np * 2], a[0], a[1], a[2], a[3], b0, b1);
+        mma_bf16(f.acc[np * 2 + 1], a[0], a[1], a[2], a[3], b2, b3);
       }
     }
   }
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-  const float i0 = 1.0f / l0, i1 = 1.0f / l1;
+}
+// n > 0 keys, 32 at a time and the last up to 16 by themselves; fresh: the first ones of their softmax.
+template <int HPC>
+__device__ __forceinline__ void flash_walk(FlashState& f, bool fresh, const uint32_t (&qa)[2][4], uint32_t k, uint32_t v, const float* bias, int n, int lane) {
+  int key = 0;
+  if (fresh) {
+    if (n > 16) flash_block<HPC, 4, true>(f, qa, k, v, bias, 0, n - 1, lane);
+    else flash_block<HPC, 2, true>(f, qa, k, v, bias, 0, n - 1, lane);
+    key = n > 16 ? 32 : 16;
+  }
+#pragma unroll 1
+  for (; key + 16 < n; key += 32) flash_block<HPC, 4, false>(f, qa, k, v, bias, key, n - 1, lane);
+  if (key < n) flash_block<HPC, 2, false>(f, qa, k, v, bias, key, n - 1, lane);
+}
+// The normalised output.
+__device__ __forceinline__ void flash_finish(FlashState& f) {
 #pragma unroll
-  for (int nt = 0; nt < 4; ++nt) {
-    acc[nt][0] *= i0; acc[nt][1] *= i0;
-    acc[nt][2] *= i1; acc[nt][3] *= i1;
+  for (int r = 0; r < 2; ++r) {
+    const float2 h = halves(f.l[r]);
+    float l = h.x + h.y;
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    const float inv = reciprocal(l);
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      f.acc[nt][2 * r] *= inv;
+      f.acc[nt][2 * r + 1] *= inv;
+    }
   }
 }
 
@@ -272,89 +299,130 @@ __device__ __forceinline__ void flash_pass(const uint32_t (&qa)[2][4], uint32_t 
 // environment i of the launch owning rows [env_off[i], env_off[i+1]) (an inactive bullet has
 // weight exactly 0 and an environment without active bullets is gated off, so neither needs a
 // row); without env_off, nb rows per environment, all of them keys (no mask was given).
-// blockIdx.y selects a group of hpc heads; the warps (4 to 8, chosen by the launcher so that the
+// blockIdx.y selects a group of HPC heads; the warps (4 to 8, chosen by the launcher so that the
 // (head, query block) pairs divide evenly) share the pairs out.
-__global__ void __launch_bounds__(256) k_attention_flash(const __nv_bfloat16* __restrict__ qkv, const uint8_t* __restrict__ alive,
-                                                         __nv_bfloat16* __restrict__ o, EnvMap map, int env_base, int hpc,
+// stage: bullet rows staged at a time.  Fewer than an environment may have only where every warp has one pair at most, whose
+// softmax then goes on over the next rows.
+//
+// Bound by latency and issue around small mma.sync tiles.  8192 environments of 12 tokens with 18 of 80 bullets 74 -> 51 us, 1024
+// of 152 tokens 93 -> 80: keys past a block of 32 in one of 16, nothing to rescale in the first block (every block of most
+// environments), pairs of scores in one instruction, the heads of a CTA a constant (divisions by it), 48 bullet rows of shared
+// memory instead of every slot's, results out as whole rows.  Eighty registers with a few spilled: with 126 the steps take
+// 844 us instead of 835 and 1432 instead of 1404, with 64 860 and 1404.
+template <int HPC, bool BULLETS>
+__global__ void __launch_bounds__(256, 3) k_attention_flash(const __nv_bfloat16* __restrict__ qkv, const uint8_t* __restrict__ alive,
+                                                         __nv_bfloat16* __restrict__ o, EnvMap map, int env_base, int stage,
                                                          const __nv_bfloat16* __restrict__ kvb,
                                                          const int* __restrict__ env_off, int nb) {
   extern __shared__ __align__(16) uint8_t fs[];
   let_next_start();
   wait_for_previous();
-  const int env_g = env_base + blockIdx.x, hd0 = blockIdx.y * hpc;
+  constexpr int STRIDE = flash_stride(HPC), GPR = HPC * 4;   // 16-byte groups per staged row
+  const int env_g = env_base + blockIdx.x, hd0 = blockIdx.y * HPC;
   const int grp = env_g / map.n_envs, e = env_g - grp * map.n_envs;
   const size_t tok0 = (size_t)grp * map.total_tokens + map.env_tok_begin(e);
   const int n = map.env_tok_count(e);
   size_t brow0 = 0;
-  if (!kvb) {
-    nb = 0;
+  if constexpr (!BULLETS) {
+    nb = stage = 0;
   } else if (env_off) {
     brow0 = (size_t)env_off[blockIdx.x];
     nb = env_off[blockIdx.x + 1] - (int)brow0;
   } else {
     brow0 = (size_t)blockIdx.x * nb;
   }
-  const int stride = flash_stride(hpc);
-  uint8_t* Qs = fs;
-  uint8_t* Ks = Qs + (size_t)n * stride;
-  uint8_t* Vs = Ks + (size_t)n * stride;
-  uint8_t* Kb = Vs + (size_t)n * stride;
-  uint8_t* Vb = Kb + (size_t)nb * stride;
-  float* bias_s = reinterpret_cast<float*>(Vb + (size_t)nb * stride);   // strides are multiples of 16 bytes
-  const int n32 = (n + 31) & ~31, nb32 = (nb + 31) & ~31;
+  const int n_stage = min(nb, stage), n32 = (n + 31) & ~31, nb32 = (n_stage + 31) & ~31;
+  // q, k, v rows, then bullet keys and values (stage rows each), then the biases; strides are multiples of 16 bytes
+  const uint32_t q_at = smem_u32(fs), k_at = q_at + n * STRIDE, v_at = k_at + n * STRIDE, kb_at = v_at + n * STRIDE, vb_at = kb_at + n_stage * STRIDE;
+  float* bias_s = reinterpret_cast<float*>(fs + (size_t)(3 * n + 2 * n_stage) * STRIDE);
   float* bias_b = bias_s + n32;
-  const int gpr = hpc * 4;   // 16-byte groups per staged row
+  const int threads = blockDim.x;
   // asynchronous 16-byte copies: all of them are in flight before the first one is waited for
-  for (int i = threadIdx.x; i < n * 3 * gpr; i += blockDim.x) {
-    const int r = i / (3 * gpr), rem = i - r * 3 * gpr, part = rem / gpr, q = rem - part * gpr;
-    cp_async16(smem_u32(fs + ((size_t)part * n + r) * stride + q * 16),
-               qkv + (tok0 + r) * (3 * D) + part * D + hd0 * DH + q * 8);
+  {
+    const __nv_bfloat16* src = qkv + tok0 * (3 * D) + hd0 * DH;
+    for (int i = threadIdx.x; i < n * 3 * GPR; i += threads) {
+      const uint32_t r = (uint32_t)i / (3 * GPR), rem = (uint32_t)i % (3 * GPR), part = rem / GPR, q = rem % GPR;
+      cp_async16(q_at + (part * n + r) * STRIDE + q * 16, src + r * (3 * D) + part * D + q * 8);
+    }
   }
-  for (int i = threadIdx.x; i < nb * 2 * gpr; i += blockDim.x) {
-    const int r = i / (2 * gpr), rem = i - r * 2 * gpr, part = rem / gpr, q = rem - part * gpr;
-    cp_async16(smem_u32(Kb + ((size_t)part * nb + r) * stride + q * 16),
-               kvb + (brow0 + r) * (2 * D) + part * D + hd0 * DH + q * 8);
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  for (int i = threadIdx.x; i < n32; i += blockDim.x)
+  auto stage_bullets = [&](int b0, int rows) {
+    const __nv_bfloat16* src = kvb + (brow0 + b0) * (2 * D) + hd0 * DH;
+    for (int i = threadIdx.x; i < rows * 2 * GPR; i += threads) {
+      const uint32_t r = (uint32_t)i / (2 * GPR), rem = (uint32_t)i % (2 * GPR), part = rem / GPR, q = rem % GPR;
+      cp_async16((part ? vb_at : kb_at) + r * STRIDE + q * 16, src + r * (2 * D) + part * D + q * 8);
+    }
+    for (int i = threadIdx.x; i < nb32; i += threads) bias_b[i] = i < rows ? 0.f : -INFINITY;
+  };
+  if (BULLETS && nb > 0) stage_bullets(0, n_stage);
+  for (int i = threadIdx.x; i < n32; i += threads)
     bias_s[i] = i < n ? ((!alive || alive[tok0 + i]) ? 0.f : kMaskedScore) : -INFINITY;
-  for (int i = threadIdx.x; i < nb32; i += blockDim.x) bias_b[i] = i < nb ? 0.f : -INFINITY;
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int last = n - 1;
-  const int nqb = (n + 15) >> 4;
-  const int n_warps = blockDim.x >> 5;
-  for (int item = warp; item < hpc * nqb; item += n_warps) {
-    const int hl = item % hpc, qb = item / hpc;
+  const int items = HPC * ((n + 15) >> 4), n_warps = threads >> 5;
+  const uint32_t k_lane = ((lane >> 3) & 1) * 16, v_lane = (lane >> 4) * 16;
+  // a turn may have barriers in it (bullets that are staged piecewise): every warp takes part then
+  const int turns = nb > stage ? 1 : (items - warp + n_warps - 1) / n_warps;
+#pragma unroll 1
+  for (int turn = 0; turn < turns; ++turn) {
+    const int item = warp + turn * n_warps;
+    const bool mine = item < items;
+    const int hl = item % HPC, qb = item / HPC;
     const uint32_t hoff = (uint32_t)hl * 64;
-    const uint32_t sQ = smem_u32(Qs) + hoff, sK = smem_u32(Ks) + hoff, sV = smem_u32(Vs) + hoff;
-    uint32_t qa[2][4];
-    {
+    uint32_t qa[2][4], out[4][2];
+    FlashState f;
+    if (mine) {
       const int row = min(qb * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, last);
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks)
-        ldsm_x4(sQ + row * stride + (ks * 16 + (lane >> 4) * 8) * 2, qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3]);
-    }
-    float acc[4][4];
-    flash_pass(qa, sK, sV, stride, bias_s, n, lane, acc);
-    if (nb > 0) {
-      float accb[4][4];
-      flash_pass(qa, smem_u32(Kb) + hoff, smem_u32(Vb) + hoff, stride, bias_b, nb, lane, accb);
-      // both outputs are bf16 tensors in the reference; so is their sum
+        ldsm_x4(q_at + hoff + row * STRIDE + (ks * 16 + (lane >> 4) * 8) * 2, qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3]);
+      flash_walk<HPC>(f, true, qa, k_at + hoff + k_lane, v_at + hoff + v_lane, bias_s, n, lane);
+      flash_finish(f);
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[nt][i] = round_bf16(acc[nt][i]) + round_bf16(accb[nt][i]);
+      for (int nt = 0; nt < 4; ++nt) {
+        out[nt][0] = pack_bf16(f.acc[nt][0], f.acc[nt][1]);
+        out[nt][1] = pack_bf16(f.acc[nt][2], f.acc[nt][3]);
+      }
     }
-    const int q0 = qb * 16 + g, q1 = q0 + 8;
+    if (BULLETS && nb > 0) {
+      if (mine) flash_walk<HPC>(f, true, qa, kb_at + hoff + k_lane, vb_at + hoff + v_lane, bias_b, n_stage, lane);
+#pragma unroll 1
+      for (int b0 = stage; b0 < nb; b0 += stage) {
+        const int rows = min(stage, nb - b0);
+        __syncthreads();   // the rows before have been read
+        stage_bullets(b0, rows);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        if (mine) flash_walk<HPC>(f, false, qa, kb_at + hoff + k_lane, vb_at + hoff + v_lane, bias_b, rows, lane);
+      }
+      if (mine) {
+        flash_finish(f);
+        // both outputs are bf16 tensors in the reference; so is their sum
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      const int col = (hd0 + hl) * DH + nt * 8 + 2 * t;
-      if (q0 <= last) *reinterpret_cast<uint32_t*>(o + (tok0 + q0) * D + col) = pack_bf16(acc[nt][0], acc[nt][1]);
-      if (q1 <= last) *reinterpret_cast<uint32_t*>(o + (tok0 + q1) * D + col) = pack_bf16(acc[nt][2], acc[nt][3]);
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r)
+            out[nt][r] = pack_bf16(bf16_lo(out[nt][r]) + round_bf16(f.acc[nt][2 * r]), bf16_hi(out[nt][r]) + round_bf16(f.acc[nt][2 * r + 1]));
+      }
     }
+    // into the place of these queries, which this warp alone reads
+    if (mine) {
+      const int q0 = qb * 16 + g;
+      uint8_t* at = fs + q0 * STRIDE + hoff + 4 * t;
+      __syncwarp();
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        if (q0 <= last) *reinterpret_cast<uint32_t*>(at + nt * 16) = out[nt][0];
+        if (q0 + 8 <= last) *reinterpret_cast<uint32_t*>(at + 8 * STRIDE + nt * 16) = out[nt][1];
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n * GPR; i += threads) {
+    const int r = i / GPR, q = i % GPR;
+    *reinterpret_cast<uint4*>(o + (tok0 + r) * D + hd0 * DH + q * 8) = *reinterpret_cast<const uint4*>(fs + r * STRIDE + q * 16);
   }
 }
 
@@ -585,8 +653,10 @@ static size_t flash_smem(int max_tokens, int nb, int hpc) {
 }
 constexpr size_t FLASH_SMEM_MAX = 227 * 1024;
 // All four heads in one CTA while that leaves room for three CTAs per SM, else one head per CTA.
+// Bullet rows staged at a time: 48 where every warp (there are four at least) has one (head, query block) pair, so that six CTAs share an SM.
+static int flash_stage(int max_tokens, int nb, int hpc) { return hpc * ((max_tokens + 15) / 16) <= 4 && nb > 48 ? 48 : nb; }
 static int flash_heads_per_cta(int max_tokens, int nb) {
-  return flash_smem(max_tokens, nb, HEADS) <= 72 * 1024 ? HEADS : 1;
+  return flash_smem(max_tokens, flash_stage(max_tokens, nb, HEADS), HEADS) <= 72 * 1024 ? HEADS : 1;
 }
 bool supported_bullets(const BnbBatch& b, int bullets_per_env) {
   return bullets_per_env >= 1 && flash_smem(b.max_tokens_per_env, bullets_per_env, 1) <= FLASH_SMEM_MAX;
@@ -803,13 +873,14 @@ static int launch_attention(const __nv_bfloat16* qkv, const uint8_t* alive, __nv
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BNB_ERR_NO_DEVICE;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(k_attention_flash, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FLASH_SMEM_MAX) != cudaSuccess)
-      return BNB_ERR_LAUNCH;
+    for (auto kernel : {k_attention_flash<HEADS, true>, k_attention_flash<1, true>, k_attention_flash<HEADS, false>, k_attention_flash<1, false>})
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FLASH_SMEM_MAX) != cudaSuccess) return BNB_ERR_LAUNCH;
     configured[dev] = true;
   }
   if (n_env <= 0) return BNB_OK;
   const int hpc = flash_heads_per_cta(b.max_tokens_per_env, kvb ? nb : 0);
-  const size_t smem = flash_smem(b.max_tokens_per_env, kvb ? nb : 0, hpc);
+  const int stage = flash_stage(b.max_tokens_per_env, kvb ? nb : 0, hpc);
+  const size_t smem = flash_smem(b.max_tokens_per_env, stage, hpc);
   if (smem > FLASH_SMEM_MAX) return BNB_ERR_TOO_MANY_TOKENS;
   dim3 grid(n_env, HEADS / hpc);
   // warps per CTA: the fewest idle warp-rounds over the (head, query block) pairs of a full environment
@@ -819,7 +890,10 @@ static int launch_attention(const __nv_bfloat16* qkv, const uint8_t* alive, __nv
     const int idle = (items + w - 1) / w * w - items;
     if (idle < best_idle) { best_idle = idle; n_warps = w; }
   }
-  return launch_after(k_attention_flash, grid, 32 * n_warps, smem, st, qkv, alive, o, make_env_map(b), env_base, hpc, kvb, env_off, nb);
+  const auto kernel = kvb ? (hpc == HEADS ? k_attention_flash<HEADS, true> : k_attention_flash<1, true>)
+                          : (hpc == HEADS ? k_attention_flash<HEADS, false> : k_attention_flash<1, false>);
+  return launch_after(kernel, grid, 32 * n_warps, smem, st, qkv, alive, o, make_env_map(b), env_base, stage,
+                      kvb, env_off, nb);
 }
 
 // env_off / idx of the active bullets of n_env environments (see the compaction kernels).
