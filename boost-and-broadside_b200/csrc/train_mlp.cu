@@ -20,11 +20,11 @@
 //
 // All three: sixteen epilogue warps, one issuing and one fetching warp that meet at mbarriers; weights
 // stream from pre-tiled images through a ring (L2 to shared memory), every wait is bounded.
-// What bounds them is the latency of that hand-off, at 18 warps per SM: for 65 536 rows k_mlp_fwd takes 61 us (issue
-// slots 40 % busy, tensor pipe 25 %, DRAM 7 % of peak), k_mlp_dx 91 (35, 27, 15), k_mlp_dw 77 (29, 36, 6), and about
-// half of the stalls in each are waits for tensor memory and rows.  A tile's start (rows, norm) and end overlap with
-// no other tile's chunks; within a chunk the erf, its exponential and about 35 instructions of gradient per hidden
-// element are what the tensor cores wait for.
+// What bounds them is the latency of that hand-off, at 18 warps per SM.  262 144 rows: k_mlp_fwd 186 us, 22 000 cycles a tile of which
+// 9 800 are gelu, 2 400 waits for gate|up, 9 500 its start (rows, norm) and end, which overlap with no other tile's chunks (196 with each
+// request right in front of its use); k_mlp_dx 287, 36 000 cycles a tile, 9 100 gelu and its gradient, 7 400 waits for products,
+// 20 000 start and end (301 with dy row by row between the stores); k_mlp_dw 241, 2 900 cycles a tile and chunk, 1 600 gelu, 430 waits for
+// products (273 and 1 100 with n and dy in one copy that waited for both products, from HBM).
 #include "train_mlp.h"
 
 #include "launch_after.h"
@@ -233,12 +233,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
     uint32_t pair = 0, par = 0, acc_par = 0;
     const RowMap m = row_map();
     const float4 gain = *reinterpret_cast<const float4*>(a.gain + m.col);
+    // Rows are on their way before the waits in front of their use: the next tile's as this tile's leave, the residual's
+    // as the last chunk does.
+    float4 x[8];
+    rows_in(x, a.x1, m, blockIdx.x * TILE, a.rows);
     for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
       epi_sync();   // every warp is done with the operand area of the previous tile
       {
-        float4 x[8];
         float inv[8];
-        rows_in(x, a.x1, m, tile * TILE, a.rows);
         norm_rows(smem, x, inv, gain, reinterpret_cast<float*>(smem + FW_SUMS), m);
       }
       post(s, FB_OP);
@@ -268,12 +270,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
         par ^= 1u << pair;
         pair = pair == 2 ? 0 : pair + 1;
       }
+      rows_in(x, a.x1, m, tile * TILE, a.rows);
       s.wait(FB_ACC, acc_par, TIMEOUT_ACC);
       acc_par ^= 1u;
       tc_fence_after();
       // y = x + down, row layout; the first eight warps stage in the operand area, then the others
-      float4 x[8], d[8];
-      rows_in(x, a.x1, m, tile * TILE, a.rows);
+      float4 d[8];
       if (group == 0) transpose_rows(d, lane_addr + part * 32, smem + (warp & 7) * 4096, m);
       epi_sync();
       if (group == 1) transpose_rows(d, lane_addr + part * 32, smem + (warp & 7) * 4096, m);
@@ -283,6 +285,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
         if (r < a.rows)
           *reinterpret_cast<float4*>(a.out + (size_t)r * D + m.col) = make_float4(x[i].x + d[i].x, x[i].y + d[i].y, x[i].z + d[i].z, x[i].w + d[i].w);
       }
+      rows_in(x, a.x1, m, (tile + gridDim.x) * TILE, a.rows);
       tc_fence_before();
     }
   }
@@ -293,7 +296,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_fwd(const __grid_constant__ 
 
 // Shared memory: n and dy (32 KB each), two slots of gate|up and transposed down (48 KB), two of transposed
 // gate and up (32 KB), row sums, frame.
-constexpr uint32_t DX_DY = 32768, DX_W1 = 65536, DX_W2 = DX_W1 + 2 * 49152, DX_SUMS = DX_W2 + 2 * 32768, DX_FRAME = DX_SUMS + 2048,
+constexpr uint32_t DX_DY = 32768, DX_W1 = 65536, DX_W2 = DX_W1 + 2 * 49152, DX_SUMS = DX_W2 + 2 * 32768, DX_INV = DX_SUMS + 2048, DX_FRAME = DX_INV + 512,
                    DX_BYTES = DX_FRAME + FRAME_BYTES;
 enum : int { XB_OP = 0, XB_FF0, XB_ACC = XB_FF0 + 2, XB_DRAIN, XB_FULL1, XB_DONE1 = XB_FULL1 + 2, XB_FULL2 = XB_DONE1 + 2, XB_DONE2 = XB_FULL2 + 2, XB_COUNT = XB_DONE2 + 2 };
 // Tensor memory: dn [0, 128), two accumulator sets of gate|up (128 columns) and d h (64).
@@ -377,24 +380,27 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
   } else {
     const int part = tid >> 7, group = part >> 1, half = part & 1;
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    float* sums = reinterpret_cast<float*>(smem + DX_SUMS);
+    float *sums = reinterpret_cast<float*>(smem + DX_SUMS), *row_inv = reinterpret_cast<float*>(smem + DX_INV);
     uint32_t par = 0, acc_par = 0;
     const RowMap m = row_map();
     const float4 gain = *reinterpret_cast<const float4*>(a.gain + m.col);
     float4 gsum = make_float4(0.f, 0.f, 0.f, 0.f);   // gain gradient of this lane's columns
+    float4 x[8], dn[8];
     for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
-      float inv[8];
       // the operand area: its tiles on their way to global memory are read, the transposes of the previous
       // round done
       if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      rows_in(x, a.x1, m, tile * TILE, a.rows);
+      rows_in(dn, a.dy, m, tile * TILE, a.rows);
       epi_sync();
       {
-        float4 x[8];
-        rows_in(x, a.x1, m, tile * TILE, a.rows);
+        float inv[8];
         norm_rows(smem, x, inv, gain, sums, m);
-        rows_in(x, a.dy, m, tile * TILE, a.rows);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) put_row4(smem + DX_DY, m, i, x[i]);
+        for (int i = 0; i < 8; ++i) {
+          put_row4(smem + DX_DY, m, i, dn[i]);
+          if (m.col == 0) row_inv[m.row(i)] = inv[i];
+        }
       }
       post(s, XB_OP);
       epi_sync();
@@ -432,6 +438,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
         tmem_wait_st();
         post(s, XB_FF0 + group);
       }
+      rows_in(x, a.x1, m, tile * TILE, a.rows);
       s.wait(XB_ACC, acc_par, TIMEOUT_ACC);
       acc_par ^= 1u;
       tc_fence_after();
@@ -439,26 +446,38 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
       // area (64 KB, 4 KB per warp) stages the transpose once its copies to global memory have read it.
       if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
       epi_sync();
-      float4 x[8], dn[8];
-      rows_in(x, a.x1, m, tile * TILE, a.rows);
       transpose_rows(dn, lane_addr + part * 32, smem + warp * 4096, m);
       tc_fence_before();
-      float coef[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        coef[i] = fmaf(x[i].x * gain.x, dn[i].x, fmaf(x[i].y * gain.y, dn[i].y, fmaf(x[i].z * gain.z, dn[i].z, x[i].w * gain.w * dn[i].w)));
-      row_sums(coef, sums, m);
+      for (int i = 0; i < 8; ++i) {   // sums of x gain dn over a row: eight lanes here, the four warps of the row through shared memory
+        float c = fmaf(x[i].x * gain.x, dn[i].x, fmaf(x[i].y * gain.y, dn[i].y, fmaf(x[i].z * gain.z, dn[i].z, x[i].w * gain.w * dn[i].w)));
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int r = tile * TILE + m.row(i);
-        if (r >= a.rows) continue;
-        const float iv = inv[i], k = coef[i] * iv * iv * iv * (1.0f / D);
-        const float4 d = *reinterpret_cast<const float4*>(a.dy + (size_t)r * D + m.col);
-        *reinterpret_cast<float4*>(a.out + (size_t)r * D + m.col) =
-            make_float4(d.x + iv * gain.x * dn[i].x - x[i].x * k, d.y + iv * gain.y * dn[i].y - x[i].y * k,
-                        d.z + iv * gain.z * dn[i].z - x[i].z * k, d.w + iv * gain.w * dn[i].w - x[i].w * k);
-        gsum.x = fmaf(dn[i].x * x[i].x, iv, gsum.x); gsum.y = fmaf(dn[i].y * x[i].y, iv, gsum.y);
-        gsum.z = fmaf(dn[i].z * x[i].z, iv, gsum.z); gsum.w = fmaf(dn[i].w * x[i].w, iv, gsum.w);
+        for (int o = 1; o < 8; o <<= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        if ((m.lane & 7) == 0) sums[part * TILE + m.row(i)] = c;
+      }
+      asm volatile("bar.sync %0, 128;" ::"r"(3 + (warp & 3)) : "memory");   // their next use is behind the next tile's first barrier
+      // four rows of dy at a time: behind a store the next load would wait for it
+#pragma unroll
+      for (int i0 = 0; i0 < 8; i0 += 4) {
+        float4 dy[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = tile * TILE + m.row(i0 + i);
+          dy[i] = r < a.rows ? *reinterpret_cast<const float4*>(a.dy + (size_t)r * D + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = i0; i < i0 + 4; ++i) {
+          const int r = tile * TILE + m.row(i);
+          if (r >= a.rows) continue;
+          const float* p = sums + m.row(i);
+          const float iv = row_inv[m.row(i)], k = ((p[0] + p[TILE]) + (p[2 * TILE] + p[3 * TILE])) * iv * iv * iv * (1.0f / D);
+          const float4 d = dy[i - i0];
+          *reinterpret_cast<float4*>(a.out + (size_t)r * D + m.col) =
+              make_float4(d.x + iv * gain.x * dn[i].x - x[i].x * k, d.y + iv * gain.y * dn[i].y - x[i].y * k,
+                          d.z + iv * gain.z * dn[i].z - x[i].z * k, d.w + iv * gain.w * dn[i].w - x[i].w * k);
+          gsum.x = fmaf(dn[i].x * x[i].x, iv, gsum.x); gsum.y = fmaf(dn[i].y * x[i].y, iv, gsum.y);
+          gsum.z = fmaf(dn[i].z * x[i].z, iv, gsum.z); gsum.w = fmaf(dn[i].w * x[i].w, iv, gsum.w);
+        }
       }
     }
 #pragma unroll
@@ -479,14 +498,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dx(const __grid_constant__ A
 // Shared memory: the chunk's gate|up and transposed down (48 KB), two stages of n and dy tiles (64 KB),
 // d gate | d up (32 KB) and h (16 KB) of a tile as operands, frame.
 constexpr uint32_t DW_TILE = 49152, DW_G = DW_TILE + 2 * 65536, DW_H = DW_G + 32768, DW_FRAME = DW_H + 16384, DW_BYTES = DW_FRAME + FRAME_BYTES;
-enum : int { WB_WEIGHTS = 0, WB_READY, WB_READ, WB_STAGED, WB_DRAIN, WB_FULL0, WB_DONE0 = WB_FULL0 + 2, WB_COUNT = WB_DONE0 + 2 };
+enum : int { WB_WEIGHTS = 0, WB_READY, WB_READ, WB_STAGED, WB_DRAIN, WB_FULL0, WB_DONE0 = WB_FULL0 + 4, WB_COUNT = WB_DONE0 + 4 };   // slots of n, then of dy
 // Tensor memory: gate|up [0, 128), d h [128, 192), d Wg | d Wu (lane = hidden column) [192, 320), d Wd (lane =
 // model dimension) [320, 384).
 constexpr uint32_t DW_ACC1 = 192, DW_ACC2 = 320;
 
 __global__ void __launch_bounds__(THREADS, 1) k_mlp_dw(const __grid_constant__ Args a) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  const int counts[WB_COUNT] = {1, 1, EPI_WARPS, EPI_WARPS, 1, 1, 1, 1, 1};
+  const int counts[WB_COUNT] = {1, 1, EPI_WARPS, EPI_WARPS, 1, 1, 1, 1, 1, 1, 1, 1, 1};
   const int tid = threadIdx.x, warp = tid >> 5;
   const Frame f = open_frame(smem + DW_FRAME, a.status, a.host_status, counts);
   const Sync s{smem_u32(f.bars), a.status, f.aborted};
@@ -504,20 +523,27 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dw(const __grid_constant__ A
     }
     __syncwarp();
     uint32_t par = 3;
+    // A tile's copies start when the products of the tile two before are complete and are waited for a period later: it is in
+    // L2 by then, an eighth asked for by each CTA that reads it.
+    auto ask = [&](int i) {
+      if (i < my_tiles && elected) {
+        const size_t at = (size_t)(first + i * stride) * 32768 + chunk * 4096;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.n_image + at), "r"(4096) : "memory");
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.dy_image + at), "r"(4096) : "memory");
+      }
+    };
+    ask(2);
 #pragma unroll 1
     for (int i = 0; i < my_tiles; ++i) {
       const uint32_t slot = i & 1;
       const size_t at = (size_t)(first + i * stride) * 32768;
-      s.wait(WB_DONE0 + slot, par >> slot, TIMEOUT_FREE);
+      ask(i + 3);
+      bool go = true;
+#pragma unroll
+      for (int p = 0; p < 2 && go; ++p)   // n, whose products are the first and the last that are waited for, then dy
+        go = fetch(s, WB_FULL0 + 2 * p + slot, WB_DONE0 + 2 * p + slot, par >> slot, base + DW_TILE + slot * 65536 + p * 32768, (p ? a.dy_image : a.n_image) + at, 32768, elected);
+      if (!go) break;
       par ^= 1u << slot;
-      if (__any_sync(0xffffffffu, s.aborted[0])) break;
-      if (elected) {
-        const uint32_t bar = s.bars + 8 * (WB_FULL0 + slot), dst = base + DW_TILE + slot * 65536;
-        mbar_expect_tx(bar, 65536);
-        bulk_g2s(dst, a.n_image + at, 32768, bar);
-        bulk_g2s(dst + 32768, a.dy_image + at, 32768, bar);
-      }
-      __syncwarp();
     }
   } else if (warp == MMA_WARP) {
     const uint32_t base = smem_u32(smem), el = elect_one(), tm = uniform(tmem), w_lo = desc_lo(base);
@@ -526,9 +552,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dw(const __grid_constant__ A
     s.wait(WB_WEIGHTS, 0, TIMEOUT_FULL);
     auto recompute = [&](uint32_t slot) {
       s.wait(WB_FULL0 + slot, full >> slot, TIMEOUT_FULL);
-      full ^= 1u << slot;
       const uint32_t n_lo = uniform(desc_lo(base + DW_TILE + slot * 65536));
       product128(el, tm, n_lo, w_lo, 1024, id128);
+      s.wait(WB_FULL0 + 2 + slot, full >> slot, TIMEOUT_FULL);
+      full ^= 1u << slot;
       product128(el, tm + 128, n_lo + 2048, w_lo + 2048, 512, id64);
       tc_commit_if(el, s.bars + 8 * WB_READY);
     };
@@ -545,10 +572,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dw(const __grid_constant__ A
 #pragma unroll
       for (uint32_t k = 0; k < 8; ++k)           // 16 rows = 2048 bytes per k step
         mma_one<false>(el, tm + DW_ACC1, g_mn + 128 * k, n_mn + 128 * k, id128 | BOTH_MN, (i | (int)k) ? 1u : 0u);
+      tc_commit_if(el, s.bars + 8 * (WB_DONE0 + slot));
 #pragma unroll
       for (uint32_t k = 0; k < 8; ++k)
         mma_one<false>(el, tm + DW_ACC2, n_mn + 2048 + 128 * k, h_mn + 128 * k, id64 | BOTH_MN, (i | (int)k) ? 1u : 0u);
-      tc_commit_if(el, s.bars + 8 * (WB_DONE0 + slot));
+      tc_commit_if(el, s.bars + 8 * (WB_DONE0 + 2 + slot));
     }
     tc_commit_if(el, s.bars + 8 * WB_DRAIN);
     for (int i = 0; i < DEFAULT_POLL_LIMIT && !mbar_try_wait(s.bars + 8 * WB_DRAIN, 0); ++i) {
@@ -580,7 +608,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dw(const __grid_constant__ A
         wh[j] = pack_f2(mul(y, up));
       }
       if (i > 0) {   // the previous tile's operands have been read
-        s.wait(WB_DONE0 + ((i - 1) & 1), done >> ((i - 1) & 1), TIMEOUT_ACC);
+        s.wait(WB_DONE0 + 2 + ((i - 1) & 1), done >> ((i - 1) & 1), TIMEOUT_ACC);
         done ^= 1u << ((i - 1) & 1);
       }
 #pragma unroll
@@ -593,7 +621,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp_dw(const __grid_constant__ A
       post(s, WB_STAGED);
     }
     if (my_tiles > 0) {
-      s.wait(WB_DONE0 + ((my_tiles - 1) & 1), done >> ((my_tiles - 1) & 1), TIMEOUT_ACC);
+      s.wait(WB_DONE0 + 2 + ((my_tiles - 1) & 1), done >> ((my_tiles - 1) & 1), TIMEOUT_ACC);
       tc_fence_after();
       // lanes 0 - 63: d Wg rows, 64 - 127: d Wu rows of the chunk; this thread: 32 of the 128 columns
       float* dst = (row < 64 ? a.d_gate + (size_t)(64 * chunk + row) * D : a.d_up + (size_t)(64 * chunk + row - 64) * D) + part * 32;
