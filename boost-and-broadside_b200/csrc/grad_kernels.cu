@@ -1230,37 +1230,89 @@ struct ShipGeom {
   const uint8_t* done;   // (T, B) or null
 };
 
+// The conv has no recurrence: a thread takes four channels of a row for `seg` steps, with the next ones on their way while one is
+// worked on.  (A channel per thread over all steps, one step ahead, had 8 KB of rows on their way per SM: within a training
+// step of 262 144 rows 98 us and 150 for the gradient, where this takes 72 and 107, 268 and 402 MB besides the state.)
+constexpr int CONV_AHEAD = 4;
+// Episode boundaries right before the steps t - 1 - k, k < N, as bits; all loads at once.
+template <int N>
+__device__ __forceinline__ uint32_t boundaries(const ShipGeom& gm, int t, int b) {
+  uint8_t f[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) f[k] = gm.done && t - 1 - k >= 0 ? gm.done[(size_t)(t - 1 - k) * gm.B + b] : 0;
+  uint32_t bits = 0;
+#pragma unroll
+  for (int k = 0; k < N; ++k) bits |= (f[k] ? 1u : 0u) << k;
+  return bits;
+}
+// How many lags of a step are valid, given its boundaries: 3 but for the steps behind one (griffin.py:67-140).
+__device__ __forceinline__ int valid_lags(uint32_t bits) { return bits & 1u ? 0 : bits & 2u ? 1 : bits & 4u ? 2 : BNB_CONV_KERNEL - 1; }
+__device__ __forceinline__ float part(const float4& v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
+__device__ __forceinline__ float& part(float4& v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
+// Padded conv inputs p .. p + 2 of a row (0 .. 2 the stored taps, 3 + t the linear1 output of step t); b1 at the row's columns.
+__device__ __forceinline__ void padded_before(float4 (&pad)[4], const float* __restrict__ b1, const float* __restrict__ hid, const ShipGeom& gm, int s, int d, int p) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (p + k >= 3) {
+      pad[k] = *reinterpret_cast<const float4*>(b1 + ((size_t)(p + k - 3) * gm.Rr + s) * gm.D + d);
+    } else {
+      const float* h = hid + (size_t)s * 4 * gm.D + (size_t)(p + k + 1) * gm.D + d;   // the caller's: any alignment
+      pad[k] = make_float4(h[0], h[1], h[2], h[3]);
+    }
+  }
+}
+
 // u_t = conv bias + sum over lags of tap * padded value, a lag being valid while no episode boundary
-// lies between (griffin.py:67-140).
-__global__ void __launch_bounds__(256) k_conv_fwd(const float* __restrict__ b1, const float* __restrict__ hid,
+// lies between (griffin.py:67-140).  blockIdx.y: segment of steps.
+__global__ void __launch_bounds__(256, 3) k_conv_fwd(const float* __restrict__ b1, const float* __restrict__ hid,
                                                   const float* __restrict__ cw, const float* __restrict__ cb,
-                                                  float* __restrict__ u, ShipGeom gm) {
+                                                  float* __restrict__ u, ShipGeom gm, int seg) {
   tensor::let_next_start();
   tensor::wait_for_previous();
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)gm.Rr * gm.D) return;
-  const int s = (int)(idx / gm.D), d = (int)(idx - (size_t)s * gm.D);
-  const int b = s / gm.n_rec;
-  const float* hp = hid + (size_t)s * 4 * gm.D + d;
-  float p3 = hp[gm.D], p2 = hp[2 * gm.D], p1 = hp[3 * gm.D];
-  const float w0 = cw[d * 4], w1 = cw[d * 4 + 1], w2 = cw[d * 4 + 2], w3 = cw[d * 4 + 3], bias = cb[d];
-  int cur = BNB_CONV_KERNEL - 1;
+  const size_t quad = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int per_row = gm.D / 4;
+  if (quad >= (size_t)gm.Rr * per_row) return;
+  const int s = (int)(quad / per_row), d = 4 * (int)(quad - (size_t)s * per_row), b = s / gm.n_rec;
+  const int t0 = blockIdx.y * seg, t1 = min(t0 + seg, gm.T);
   const size_t step = (size_t)gm.Rr * gm.D;
-  float next = b1[idx];
-  for (int t = 0; t < gm.T; ++t) {
-    if (t >= 1) {
-      const bool boundary = gm.done && gm.done[(size_t)(t - 1) * gm.B + b];
-      cur = boundary ? 0 : min(cur + 1, BNB_CONV_KERNEL - 1);
+  const float* in = b1 + (size_t)s * gm.D + d;
+  float* out = u + (size_t)s * gm.D + d;
+  float4 pad[4], next[CONV_AHEAD];
+#pragma unroll
+  for (int i = 0; i < CONV_AHEAD; ++i)
+    if (t0 + i < t1) next[i] = *reinterpret_cast<const float4*>(in + (size_t)(t0 + i) * step);
+  padded_before(pad, b1, hid, gm, s, d, t0);
+  float w[4][4], bias[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    bias[c] = cb[d + c];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[c][k] = cw[(d + c) * 4 + k];
+  }
+  int cur = valid_lags(boundaries<3>(gm, t0, b));
+#pragma unroll 1
+  for (int t = t0; t < t1; t += CONV_AHEAD) {
+    bool boundary[CONV_AHEAD];
+#pragma unroll
+    for (int i = 0; i < CONV_AHEAD; ++i) boundary[i] = gm.done && t + i < t1 && gm.done[(size_t)(t + i) * gm.B + b];
+#pragma unroll
+    for (int i = 0; i < CONV_AHEAD; ++i) {
+      if (t + i >= t1) break;
+      pad[3] = next[i];
+      if (t + CONV_AHEAD + i < t1) next[i] = *reinterpret_cast<const float4*>(in + (size_t)(t + CONV_AHEAD + i) * step);
+      float4 v;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float a0 = cur >= 3 ? __fmul_rn(part(pad[0], c), w[c][0]) : 0.f;
+        const float a1 = cur >= 2 ? __fmul_rn(part(pad[1], c), w[c][1]) : 0.f;
+        const float a2 = cur >= 1 ? __fmul_rn(part(pad[2], c), w[c][2]) : 0.f;
+        const float a3 = __fmul_rn(part(pad[3], c), w[c][3]);
+        part(v, c) = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3), bias[c]);
+      }
+      *reinterpret_cast<float4*>(out + (size_t)(t + i) * step) = v;
+      pad[0] = pad[1]; pad[1] = pad[2]; pad[2] = pad[3];
+      cur = boundary[i] ? 0 : min(cur + 1, BNB_CONV_KERNEL - 1);
     }
-    const size_t at = (size_t)t * step + idx;
-    const float xt = next;
-    if (t + 1 < gm.T) next = b1[at + step];
-    const float t0 = cur >= 3 ? __fmul_rn(p3, w0) : 0.f;
-    const float t1 = cur >= 2 ? __fmul_rn(p2, w1) : 0.f;
-    const float t2 = cur >= 1 ? __fmul_rn(p1, w2) : 0.f;
-    const float t3 = __fmul_rn(xt, w3);
-    u[at] = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(t0, t1), t2), t3), bias);
-    p3 = p2; p2 = p1; p1 = xt;
   }
 }
 
@@ -1388,72 +1440,117 @@ __global__ void __launch_bounds__(256) k_scan_bwd(float* za, float* zx, const fl
 }
 
 // Adjoint of k_conv_fwd: d u -> d linear1 output, d stored taps, d conv weight and bias.  The
-// new tap buffer is the last three padded values, so its gradient joins there.
-__global__ void __launch_bounds__(256) k_conv_bwd(const float* __restrict__ du, const float* __restrict__ b1,
+// new tap buffer is the last three padded values, so its gradient joins there.  A segment's first padded values take the
+// gradients of up to three steps before it as well.
+__global__ void __launch_bounds__(256, 2) k_conv_bwd(const float* __restrict__ du, const float* __restrict__ b1,
                                                   const float* __restrict__ hid, const float* __restrict__ d_hid_out,
                                                   float* __restrict__ d_hid_in, const float* __restrict__ cw,
                                                   float* __restrict__ db1, float* __restrict__ d_cw, float* __restrict__ d_cb,
-                                                  ShipGeom gm) {
+                                                  ShipGeom gm, int seg) {
   tensor::let_next_start();
   tensor::wait_for_previous();
-  __shared__ float s_w[MAXW * 4], s_b[MAXW];
-  for (int i = threadIdx.x; i < gm.D * 4; i += blockDim.x) s_w[i] = 0.f;
-  if ((int)threadIdx.x < gm.D) s_b[threadIdx.x] = 0.f;
+  constexpr int BWD_AHEAD = 2;   // of two tensors
+  __shared__ float sums[20 * (MAXW / 4)];   // [tap and channel of the quad, or bias][quad]: lanes side by side
+  const int per_row = gm.D / 4;
+  for (int i = threadIdx.x; i < 20 * per_row; i += blockDim.x) sums[i] = 0.f;
   __syncthreads();
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = idx < (size_t)gm.Rr * gm.D;
-  const int s = live ? (int)(idx / gm.D) : 0, d = live ? (int)(idx - (size_t)s * gm.D) : 0;
-  if (live) {
-    const int b = s / gm.n_rec, T = gm.T, D = gm.D;
-    const float* hp = hid + (size_t)s * 4 * D + d;
+  for (size_t quad = (size_t)blockIdx.x * blockDim.x + threadIdx.x; quad < (size_t)gm.Rr * per_row; quad += (size_t)gridDim.x * blockDim.x) {
+    const int s = (int)(quad / per_row), d = 4 * (int)(quad - (size_t)s * per_row), b = s / gm.n_rec;
+    const int T = gm.T, D = gm.D, t0 = blockIdx.y * seg, t1 = min(t0 + seg, T);
+    const size_t step = (size_t)gm.Rr * D;
+    const float *gu = du + (size_t)s * D + d, *in = b1 + (size_t)s * D + d;
+    float4 nu[BWD_AHEAD], nb[BWD_AHEAD];
+#pragma unroll
+    for (int i = 0; i < BWD_AHEAD; ++i)
+      if (t0 + i < t1) {
+        nu[i] = *reinterpret_cast<const float4*>(gu + (size_t)(t0 + i) * step);
+        nb[i] = *reinterpret_cast<const float4*>(in + (size_t)(t0 + i) * step);
+      }
     // padded index p: 0..2 the stored taps, 3 + t the linear1 output of step t
-    auto emit = [&](int p, float v) {
-      if (p >= T && d_hid_out) v += d_hid_out[(size_t)s * 4 * D + D + (size_t)(p - T) * D + d];
-      if (p < 3) {
-        if (d_hid_in) d_hid_in[(size_t)s * 4 * D + D + (size_t)p * D + d] = v;
-      } else {
-        db1[((size_t)(p - 3) * gm.Rr + s) * D + d] = v;
+    auto emit = [&](int p, float4 v) {
+      if (p >= T && d_hid_out) {
+        const float* h = d_hid_out + (size_t)s * 4 * D + D + (size_t)(p - T) * D + d;
+        v.x += h[0]; v.y += h[1]; v.z += h[2]; v.w += h[3];
+      }
+      if (p >= 3) {
+        *reinterpret_cast<float4*>(db1 + ((size_t)(p - 3) * gm.Rr + s) * D + d) = v;
+      } else if (d_hid_in) {
+        float* h = d_hid_in + (size_t)s * 4 * D + D + (size_t)p * D + d;
+        h[0] = v.x; h[1] = v.y; h[2] = v.z; h[3] = v.w;
       }
     };
-    const float w[4] = {cw[d * 4], cw[d * 4 + 1], cw[d * 4 + 2], cw[d * 4 + 3]};
-    float pad[4] = {hp[D], hp[2 * D], hp[3 * D], 0.f};   // padded[t .. t+3] at step t
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};                 // d padded[t .. t+3]
-    float dw[4] = {0.f, 0.f, 0.f, 0.f}, dbias = 0.f;
+    float w[4][4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) w[c][k] = cw[(d + c) * 4 + k];
+    float4 acc[4], pad[4];   // d padded[t .. t+3], padded[t .. t+3] at step t
+    float dw[4][4] = {}, dbias[4] = {};
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    acc[0] = acc[1] = acc[2] = acc[3] = zero;
     int cur = BNB_CONV_KERNEL - 1;
-    const size_t step = (size_t)gm.Rr * D;
-    float nb1 = b1[idx], ndu = du[idx];
-    for (int t = 0; t < T; ++t) {
-      if (t >= 1) {
-        const bool boundary = gm.done && gm.done[(size_t)(t - 1) * gm.B + b];
-        cur = boundary ? 0 : min(cur + 1, BNB_CONV_KERNEL - 1);
-      }
-      const size_t at = (size_t)t * step + idx;
-      pad[3] = nb1;
-      const float g = ndu;
-      if (t + 1 < T) { nb1 = b1[at + step]; ndu = du[at + step]; }
-      dbias += g;
+    auto spread = [&](const float4& g) {   // tap k reads lag 3 - k
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const bool valid = (3 - k) <= cur;   // tap k reads lag 3 - k
-        if (valid) {
-          acc[k] = fmaf(g, w[k], acc[k]);
-          dw[k] = fmaf(g, pad[k], dw[k]);
-        }
-      }
-      emit(t, acc[0]);
-      acc[0] = acc[1]; acc[1] = acc[2]; acc[2] = acc[3]; acc[3] = 0.f;
-      pad[0] = pad[1]; pad[1] = pad[2]; pad[2] = pad[3];
+      for (int k = 0; k < 4; ++k)
+        if (3 - k <= cur)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) part(acc[k], c) = fmaf(part(g, c), w[c][k], part(acc[k], c));
+    };
+    const uint32_t bits = boundaries<6>(gm, t0, b);
+    float4 before[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) before[i] = t0 - 3 + i >= 0 ? *reinterpret_cast<const float4*>(gu + (size_t)(t0 - 3 + i) * step) : zero;
+    padded_before(pad, b1, hid, gm, s, d, t0);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      cur = valid_lags(bits >> (3 - i));
+      spread(before[i]);
+      acc[0] = acc[1]; acc[1] = acc[2]; acc[2] = acc[3]; acc[3] = zero;
     }
-    emit(T, acc[0]);
-    emit(T + 1, acc[1]);
-    emit(T + 2, acc[2]);
+    cur = valid_lags(bits);
+#pragma unroll 1
+    for (int t = t0; t < t1; t += BWD_AHEAD) {
+      bool boundary[BWD_AHEAD];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) atomicAdd(&s_w[d * 4 + k], dw[k]);
-    atomicAdd(&s_b[d], dbias);
+      for (int i = 0; i < BWD_AHEAD; ++i) boundary[i] = gm.done && t + i < t1 && gm.done[(size_t)(t + i) * gm.B + b];
+#pragma unroll
+      for (int i = 0; i < BWD_AHEAD; ++i) {
+        if (t + i >= t1) break;
+        const float4 g = nu[i];
+        pad[3] = nb[i];
+        if (t + BWD_AHEAD + i < t1) {
+          nu[i] = *reinterpret_cast<const float4*>(gu + (size_t)(t + BWD_AHEAD + i) * step);
+          nb[i] = *reinterpret_cast<const float4*>(in + (size_t)(t + BWD_AHEAD + i) * step);
+        }
+        spread(g);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          dbias[c] += part(g, c);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (3 - k <= cur) dw[c][k] = fmaf(part(g, c), part(pad[k], c), dw[c][k]);
+        }
+        emit(t + i, acc[0]);
+        acc[0] = acc[1]; acc[1] = acc[2]; acc[2] = acc[3]; acc[3] = zero;
+        pad[0] = pad[1]; pad[1] = pad[2]; pad[2] = pad[3];
+        cur = boundary[i] ? 0 : min(cur + 1, BNB_CONV_KERNEL - 1);
+      }
+    }
+    if (t1 == T)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) emit(T + k, acc[k]);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) atomicAdd(&sums[(4 * k + c) * per_row + d / 4], dw[c][k]);
+      atomicAdd(&sums[(16 + c) * per_row + d / 4], dbias[c]);
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < gm.D * 4; i += blockDim.x) atomicAdd(d_cw + i, s_w[i]);
-  if ((int)threadIdx.x < gm.D) atomicAdd(d_cb + threadIdx.x, s_b[threadIdx.x]);
+  for (int i = threadIdx.x; i < gm.D * 5; i += blockDim.x) {   // whole lines of d conv weight, then of its bias
+    const int k = i < gm.D * 4 ? i & 3 : 4, d = k < 4 ? i >> 2 : i - gm.D * 4;
+    atomicAdd(k < 4 ? d_cw + i : d_cb + d, sums[(4 * k + (d & 3)) * per_row + (d >> 2)]);
+  }
 }
 
 // ------------------------------------------------------------------------------ host side
@@ -1888,6 +1985,15 @@ struct TemporalGeom {
   size_t Rf() const { return (size_t)T * B * (NM - n_rec); }
 };
 
+// Blocks of the conv kernels and the steps of a thread: segments of four steps at least (each reads three rows more) until the
+// chip has two blocks of 256 on every SM.  The gradient, whose blocks end with sums over all of them, walks with that many.
+dim3 conv_grid(const ShipGeom& gm, int* seg, bool walk) {
+  const size_t blocks = ((size_t)gm.Rr * (gm.D / 4) + 255) / 256, chip = 2 * 148;
+  const int wanted = (int)std::min<size_t>((chip + blocks - 1) / blocks, (size_t)(gm.T + 3) / 4);
+  *seg = (gm.T + wanted - 1) / wanted;
+  return dim3((unsigned)(walk ? std::min(blocks, chip) : blocks), (unsigned)((gm.T + *seg - 1) / *seg));
+}
+
 // Recurrent path over the ship rows, forward part (griffin.py:249-286).  Buffers: xs d[0], n d[1],
 // linear1 out d[2], conv out d[3], gate pre-activations d[4] d[5], states d[6], linear2 out d[7],
 // gated branch d[8], x1 d[9]; with y, the sublayer's output goes to d[14] and from there to y's ship rows.
@@ -1900,6 +2006,7 @@ void ships_fwd(const Ctx& c, const BnbTemporalWeights& w, const float* x, const 
   ShipGeom gm{tg.T, Rr, D, tg.n_rec, tg.B, done};
   float *n = b.d[1], *b1 = b.d[2], *u = b.d[3], *za = b.d[4], *zx = b.d[5], *hs = b.d[6], *b2p = b.d[7], *m = b.d[8], *x1 = b.d[9];
   const int sblocks = (int)(((size_t)Rr * D + 255) / 256);
+  int seg = 0;
   const bool all = tg.Rf() == 0;   // every row is a ship's: nothing to pick out
   if (!all) gather(c, x, b.d[0], Rs, tg.n_rec, tg.NM, 0);
   const float* xs = all ? x : b.d[0];
@@ -1910,7 +2017,7 @@ void ships_fwd(const Ctx& c, const BnbTemporalWeights& w, const float* x, const 
     mmh(c, NT, H_A, n, D, w.linear1_w, D, b1, D, M, D, D);
     mmh(c, NT, H_A, n, D, w.linear2_w, D, b2p, D, M, D, D);
   }
-  c.note(launch_after(k_conv_fwd, dim3(sblocks), 256, 0, c.st, b1, hid, w.conv_w, w.conv_b, u, gm));
+  c.note(launch_after(k_conv_fwd, conv_grid(gm, &seg, false), 256, 0, c.st, b1, hid, w.conv_w, w.conv_b, u, gm, seg));
   if (c.linears) {
     train_linear::Forward f;
     f.x = u; f.image = block_image(c, L_GATES); f.blocks = 2; f.rows = Rs;
@@ -1975,6 +2082,7 @@ int temporal_bwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
     float *n = b.d[1], *b1 = b.d[2], *u = b.d[3], *za = b.d[4], *zx = b.d[5], *hs = b.d[6], *b2p = b.d[7],
           *m = b.d[8], *x1 = b.d[9], *dx1 = b.d[11], *dm = b.d[12], *dn = b.d[13];
     const int sblocks = (int)(((size_t)Rr * D + 255) / 256);
+    int seg = 0;
     const bool all = Rf == 0;
     const float *xs = all ? x : b.d[0], *dys = all ? dy : b.d[10];
     float* dxs = all ? dx : b.d[14];
@@ -2000,7 +2108,7 @@ int temporal_bwd(const Ctx& cs, const Ctx& cf, const BnbTemporalWeights& w, cons
       mm(c, NN, zx, D, w.x_w, D, dm, D, M, D, D, nullptr, nullptr, 0, 1);
     }
     float* db1 = za;   // free now
-    c.note(launch_after(k_conv_bwd, dim3(sblocks), 256, 0, c.st, dm, b1, hid, d_hid_out, d_hid_in, w.conv_w, db1, dw.conv_w, dw.conv_b, gm));
+    c.note(launch_after(k_conv_bwd, conv_grid(gm, &seg, true), 256, 0, c.st, dm, b1, hid, d_hid_out, d_hid_in, w.conv_w, db1, dw.conv_w, dw.conv_b, gm, seg));
     if (c.linears) {
       norm_linear_bwd(c, {db1, b2p}, n, L_LIN1, {dw.linear1_w, dw.linear2_w}, xs, w.norm1_w, b.inv[0], dx1, dxs, dw.norm1_w, Rs);
     } else {
