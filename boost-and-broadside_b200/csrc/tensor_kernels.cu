@@ -897,7 +897,7 @@ static int launch_attention(const __nv_bfloat16* qkv, const uint8_t* alive, __nv
 }
 
 // env_off / idx of the active bullets of n_env environments (see the compaction kernels).
-static int launch_compact(const uint8_t* active, int n_env, int nb, int* env_off, int* idx, cudaStream_t st) {
+int compact_active(const uint8_t* active, int n_env, int nb, int* env_off, int* idx, cudaStream_t st) {
   if (n_env <= 0) return BNB_OK;
   if (n_env <= SMALL_ENVS) return launch_after(k_bullet_compact, dim3(1), 1024, 0, st, active, n_env, nb, env_off, idx);
   const int blocks = (n_env + 7) / 8 < 148 * 8 ? (n_env + 7) / 8 : 148 * 8;
@@ -993,7 +993,7 @@ struct Plan {
         const bool masked = bullets->active != nullptr;
         if (masked && compacted_e0 != e0) {
           // the mask is the same for every reading sublayer of the call: one slice -> compact once
-          if ((rc = launch_compact(bullets->active + (size_t)e0 * nb, ne, nb, env_off, idx, st))) return rc;
+          if ((rc = compact_active(bullets->active + (size_t)e0 * nb, ne, nb, env_off, idx, st))) return rc;
           compacted_e0 = e0;
         }
         const bool rows_bf16 = bullets->tokens_bf16 != 0;

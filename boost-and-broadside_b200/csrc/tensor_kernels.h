@@ -37,6 +37,10 @@ void clear_status();
 int* host_status_word(cudaStream_t st);   // device address of that word, or null (see tensor_kernels.cu)
 void debug_wait_test(int skip_op, int poll_limit);
 
+// env_off: per environment the rows of its active slots in idx, [env_off[e], env_off[e + 1]), n_env + 1 values; idx: those slots
+// (e * nb + slot) in order, n_env * nb values at most.
+int compact_active(const uint8_t* active, int n_env, int nb, int* env_off, int* idx, cudaStream_t st);
+
 int spatial_block(const BnbSpatialWeights& w, int D, int H, const float* x, const uint8_t* alive,
                   const BnbBullets* bullets, float* y, const BnbBatch& b, int n_groups, void* scratch,
                   size_t scratch_bytes, cudaStream_t st);

@@ -7,7 +7,7 @@
 // (64 registers without bullets hold 47 % of the warps, where 128 held 24 % and it took 95).  The kernels it replaces read rows element by element (one
 // thread per query, or eight lanes per head), ran at 2.2 - 2.6 TB/s on environments of 8 tokens and took 425 /
 // 575 us (forward / gradient) for 1536 environment-steps of 12 tokens with 80 bullet slots, most of it
-// on slots that are not in use (45 / 99 us here, averaged over the sublayers that read them and those that do not).  Here only the slots in use are read.
+// on slots that are not in use (36 / 72 us here, averaged over the sublayers that read them and those that do not).  Here only the slots in use are read.
 //
 // Gradient contract: probabilities recomputed as exp(s - lse) with lse = max + log(sum) in float32, row
 // term <d out, out>, as the fused attention kernels behind F.scaled_dot_product_attention
@@ -48,12 +48,15 @@ __device__ __forceinline__ float4* parts_at(float* base, int ld, size_t off, siz
   return reinterpret_cast<float4*>(base + row * ld + (q / (D / 4)) * off) + q % (D / 4);
 }
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float dot4(const float4& a, const float4& b, float s) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, s)))); }
+// Four sums side by side: one of 32 terms is a chain of 32 latencies.
 __device__ __forceinline__ float dot32(const float* a, const float* b) {
-  float s = 0.f;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < DH / 4; ++i) s = dot4(ld4(a + 4 * i), ld4(b + 4 * i), s);
-  return s;
+  for (int i = 0; i < DH / 4; ++i) {
+    const float4 u = ld4(a + 4 * i), v = ld4(b + 4 * i);
+    s.x = fmaf(u.x, v.x, s.x); s.y = fmaf(u.y, v.y, s.y); s.z = fmaf(u.z, v.z, s.z); s.w = fmaf(u.w, v.w, s.w);
+  }
+  return (s.x + s.y) + (s.z + s.w);
 }
 template <int W>
 __device__ __forceinline__ float seg_sum(float v) {
@@ -84,10 +87,25 @@ __device__ __forceinline__ int key_list(const uint8_t* active, int nb, uint16_t*
   __syncthreads();
   return *count;
 }
-__device__ __forceinline__ void stage_keys(float* kv, const float* src, const uint16_t* list, int k0, int n) {
+// Where the k-th key of group g has its row: the first of its rows, or those of its list.
+struct KeyRows {
+  size_t first;
+  const uint16_t* list;   // null: one behind the other
+  __device__ __forceinline__ size_t operator()(int k) const { return first + (list ? list[k] : k); }
+};
+__device__ __forceinline__ KeyRows key_rows(const Call& c, size_t g, uint16_t* list, int* count, int* keys) {
+  if (c.boff) {
+    const int first = c.boff[g];
+    *keys = c.boff[g + 1] - first;
+    return {(size_t)first, nullptr};
+  }
+  *keys = key_list(c.bactive ? c.bactive + g * c.nb : nullptr, c.nb, list, count);
+  return {g * c.nb, list};
+}
+__device__ __forceinline__ void stage_keys(float* kv, const float* kvb, const KeyRows& row, int k0, int n) {
   for (int i = threadIdx.x; i < n * (2 * D / 4); i += THREADS) {
     const int r = i / (2 * D / 4), q = i % (2 * D / 4);
-    copy16(kv + r * LDB + q * 4, src + (size_t)list[k0 + r] * 2 * D + q * 4);
+    copy16(kv + r * LDB + q * 4, kvb + row(k0 + r) * 2 * D + q * 4);
   }
   copies_done();
 }
@@ -119,21 +137,22 @@ __host__ __device__ inline size_t carve(char* base, int n, int nb, bool grad, Sm
 
 // LPP lanes per query (8, 16 or 32: the smallest that holds the keys), so a warp serves 32 / LPP queries
 // of its head at once; lane `sub` scores key `sub`, then owns CPL channels of the output.
-template <int LPP>
+template <int LPP, bool BULLETS>
 __global__ void __launch_bounds__(THREADS) k_env_attn_fwd(const Call c) {
   extern __shared__ __align__(16) char raw[];
   tensor::let_next_start();
   tensor::wait_for_previous();
   constexpr int QPW = 32 / LPP, CPL = DH / LPP;
   Smem s;
-  carve(raw, c.n, c.kvb ? c.nb : 0, false, &s);
+  carve(raw, c.n, BULLETS ? c.nb : 0, false, &s);
   const int h = threadIdx.x >> 5, lane = threadIdx.x & 31, qs = lane / LPP, sub = lane % LPP;
   const int n = c.n;
   const size_t g = blockIdx.x, tok0 = g * n;
   rows_in<3 * D>(s.rows, LDQ, c.qkv + tok0 * 3 * D, n);
   int keys = 0;
-  if (c.kvb) {
-    keys = key_list(c.bactive ? c.bactive + g * c.nb : nullptr, c.nb, s.list, s.count);
+  KeyRows row{};
+  if constexpr (BULLETS) {
+    row = key_rows(c, g, s.list, s.count, &keys);
     for (int i = threadIdx.x; i < n * H; i += THREADS) { s.m[i] = -INFINITY; s.l[i] = 0.f; }
     for (int i = threadIdx.x; i < n * D; i += THREADS) s.acc[n * D + i] = 0.f;
   }
@@ -165,28 +184,81 @@ __global__ void __launch_bounds__(THREADS) k_env_attn_fwd(const Call c) {
       for (int d = 0; d < CPL; ++d) out[d] = acc[d];
     }
   }
+  if constexpr (!BULLETS) return;
   if (keys == 0) return;   // no bullet in use: the branch is gated off
   for (int k0 = 0; k0 < keys; k0 += BLOCK) {
     const int kn = min(BLOCK, keys - k0);
     __syncthreads();       // the previous block has been read
-    stage_keys(s.kv, c.kvb + g * c.nb * 2 * D, s.list, k0, kn);
-    const float* kb = s.kv + h * DH;
-    for (int i = 0; i < n; ++i) {
-      const float sc = lane < kn ? dot32(q + i * LDQ, kb + lane * LDB) * SCALE : -INFINITY;
-      const float m0 = s.m[i * H + h];
-      const float mx = fmaxf(m0, seg_max<32>(sc));
-      const float e = lane < kn ? expf(sc - mx) : 0.f;
-      const float corr = expf(m0 - mx);     // exp(-inf) = 0 on the first block
-      float a = s.acc[(n + i) * D + h * DH + lane] * corr;
-      for (int j = 0; j < kn; ++j) a = fmaf(__shfl_sync(0xffffffffu, e, j), kb[j * LDB + D + lane], a);
-      s.acc[(n + i) * D + h * DH + lane] = a;
-      const float sum = seg_sum<32>(e);
+    stage_keys(s.kv, c.kvb, row, k0, kn);
+    float* kb = s.kv + h * DH;
+    if constexpr (LPP < 32) {
+      // Lane = key: its key in registers, the weights of every query, which then take the key's place; lane = channel: every value
+      // once for all queries, their weights by fours.  (A query at a time read all keys, values and a weight by shuffle for each
+      // query: 68 -> 55 us for the environment-steps above.)
+      float k32[DH];
+#pragma unroll
+      for (int d4 = 0; d4 < DH / 4; ++d4) *reinterpret_cast<float4*>(&k32[4 * d4]) = ld4(kb + min(lane, kn - 1) * LDB + 4 * d4);
       __syncwarp();
-      if (lane == 0) {
-        s.m[i * H + h] = mx;
-        s.l[i * H + h] = s.l[i * H + h] * corr + sum;
+#pragma unroll 1
+      for (int i0 = 0; i0 < n; i0 += 4) {   // four queries side by side, the last ones perhaps the last query again
+        float m0[4], mx[4], sum[4], p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = min(i0 + u, n - 1);
+          const float sc = lane < kn ? dot32(q + i * LDQ, k32) * SCALE : -INFINITY;
+          m0[u] = s.m[i * H + h];
+          mx[u] = fmaxf(m0[u], seg_max<32>(sc));
+          p[u] = lane < kn ? expf(sc - mx[u]) : 0.f;
+          sum[u] = seg_sum<32>(p[u]);
+        }
+        if (lane < kn) *reinterpret_cast<float4*>(kb + lane * LDB + i0) = make_float4(p[0], p[1], p[2], p[3]);
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u;
+          if (i >= n) break;
+          const float corr = expf(m0[u] - mx[u]);     // exp(-inf) = 0 on the first block
+          s.acc[(n + i) * D + h * DH + lane] *= corr;
+          if (lane == 0) {
+            s.m[i * H + h] = mx[u];
+            s.l[i * H + h] = s.l[i * H + h] * corr + sum[u];
+          }
+        }
       }
       __syncwarp();
+      float a[LPP];
+#pragma unroll
+      for (int i = 0; i < LPP; ++i) a[i] = i < n ? s.acc[(n + i) * D + h * DH + lane] : 0.f;
+#pragma unroll 4
+      for (int j = 0; j < kn; ++j) {
+        const float v1 = kb[j * LDB + D + lane];
+#pragma unroll
+        for (int i = 0; i < LPP; i += 4) {
+          const float4 w = ld4(kb + j * LDB + i);
+          a[i] = fmaf(w.x, v1, a[i]); a[i + 1] = fmaf(w.y, v1, a[i + 1]); a[i + 2] = fmaf(w.z, v1, a[i + 2]); a[i + 3] = fmaf(w.w, v1, a[i + 3]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < LPP; ++i)
+        if (i < n) s.acc[(n + i) * D + h * DH + lane] = a[i];
+    } else {
+      for (int i = 0; i < n; ++i) {
+        const float sc = lane < kn ? dot32(q + i * LDQ, kb + lane * LDB) * SCALE : -INFINITY;
+        const float m0 = s.m[i * H + h];
+        const float mx = fmaxf(m0, seg_max<32>(sc));
+        const float e = lane < kn ? expf(sc - mx) : 0.f;
+        const float corr = expf(m0 - mx);     // exp(-inf) = 0 on the first block
+        float a = s.acc[(n + i) * D + h * DH + lane] * corr;
+        for (int j = 0; j < kn; ++j) a = fmaf(__shfl_sync(0xffffffffu, e, j), kb[j * LDB + D + lane], a);
+        s.acc[(n + i) * D + h * DH + lane] = a;
+        const float sum = seg_sum<32>(e);
+        __syncwarp();
+        if (lane == 0) {
+          s.m[i * H + h] = mx;
+          s.l[i * H + h] = s.l[i * H + h] * corr + sum;
+        }
+        __syncwarp();
+      }
     }
   }
   for (int i = 0; i < n; ++i) {
@@ -198,7 +270,7 @@ __global__ void __launch_bounds__(THREADS) k_env_attn_fwd(const Call c) {
 // Gradient.
 // (Without bullets the sums of 32 channels a lane that their keys need would only cost registers, and so CTAs.)
 template <int LPP, bool BULLETS>
-__global__ void __launch_bounds__(THREADS, BULLETS || LPP == 32 ? 4 : LPP == 16 ? 6 : 8) k_env_attn_bwd(const Call c) {
+__global__ void __launch_bounds__(THREADS, LPP == 32 ? 4 : BULLETS ? 3 : LPP == 16 ? 6 : 8) k_env_attn_bwd(const Call c) {
   extern __shared__ __align__(16) char raw[];
   tensor::let_next_start();
   tensor::wait_for_previous();
@@ -211,12 +283,13 @@ __global__ void __launch_bounds__(THREADS, BULLETS || LPP == 32 ? 4 : LPP == 16 
   rows_in<3 * D>(s.rows, LDQ, c.qkv + tok0 * 3 * D, n);
   rows_in<D>(s.d_o, LDO, c.d_o + tok0 * D, n);
   int keys = 0;
+  KeyRows row{};
   if constexpr (BULLETS) {
-    keys = key_list(c.bactive ? c.bactive + g * c.nb : nullptr, c.nb, s.list, s.count);
+    row = key_rows(c, g, s.list, s.count, &keys);
     for (int i = threadIdx.x; i < n * LDO; i += THREADS) s.dq[i] = 0.f;
     for (int i = threadIdx.x; i < n * H; i += THREADS) { s.m[i] = -INFINITY; s.l[i] = s.s[i] = 0.f; }
     // slots that are no keys have no gradient
-    const uint8_t* on = c.bactive ? c.bactive + g * c.nb : nullptr;
+    const uint8_t* on = c.bactive && !c.boff ? c.bactive + g * c.nb : nullptr;
     for (int i = threadIdx.x; on && i < c.nb * (2 * D / 4); i += THREADS)
       if (const int r = i / (2 * D / 4); !on[r]) *parts_at<2>(c.dkvb, c.ld_dkvb, c.off_dkvb, g * c.nb + r, i) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -227,11 +300,16 @@ __global__ void __launch_bounds__(THREADS, BULLETS || LPP == 32 ? 4 : LPP == 16 
   const float* go = s.d_o + h * DH;
   if (BULLETS && keys) {
     float dk[DH], dv[DH];
-    // one sweep for the softmax statistics of every query, one for the gradients
-    for (int k0 = 0; k0 < keys; k0 += BLOCK) {
+    // one sweep for the softmax statistics of every query, one for the gradients (up to a block of keys both in one)
+    constexpr bool FEW = LPP < 32;
+    if (FEW && keys <= BLOCK) {
+      __syncthreads();
+      stage_keys(s.kv, c.kvb, row, 0, keys);
+    }
+    for (int k0 = 0; k0 < keys && !(FEW && keys <= BLOCK); k0 += BLOCK) {
       const int kn = min(BLOCK, keys - k0);
       __syncthreads();
-      stage_keys(s.kv, c.kvb + g * c.nb * 2 * D, s.list, k0, kn);
+      stage_keys(s.kv, c.kvb, row, k0, kn);
       const float* kb = s.kv + h * DH;
       for (int i = 0; i < n; ++i) {
         const float sc = lane < kn ? dot32(q + i * LDQ, kb + lane * LDB) * SCALE : -INFINITY;
@@ -253,31 +331,112 @@ __global__ void __launch_bounds__(THREADS, BULLETS || LPP == 32 ? 4 : LPP == 16 
       const int kn = min(BLOCK, keys - k0);
       if (keys > BLOCK) {    // a single block is still there
         __syncthreads();
-        stage_keys(s.kv, c.kvb + g * c.nb * 2 * D, s.list, k0, kn);
+        stage_keys(s.kv, c.kvb, row, k0, kn);
       }
       float* kb = s.kv + h * DH;
-#pragma unroll
-      for (int d = 0; d < DH; ++d) dk[d] = dv[d] = 0.f;
-      for (int i = 0; i < n; ++i) {
-        const float l = s.l[i * H + h], lse = s.m[i * H + h] + logf(l), delta = s.s[i * H + h] / l;
-        const float* qi = q + i * LDQ;
-        const float* gi = go + i * LDO;
-        float p = 0.f, ds = 0.f;
-        if (lane < kn) {
-          p = expf(dot32(qi, kb + lane * LDB) * SCALE - lse);
-          ds = p * (dot32(gi, kb + lane * LDB + D) - delta) * SCALE;
-        }
+      if constexpr (FEW) {
+        // Lane = key, its key and value in registers while every query's weight and score gradient are computed, which take the
+        // value's place; lane = channel sums d q of all queries over the keys, each read once; lane = key again its own
+        // gradients.  Loops over four queries stay loops: unrolled over all of them a quarter of the stalls were instruction
+        // fetches.  1536 environment-steps of 12 tokens with 18 of 80 bullets 155 -> 106 us; a query at a time read every key and value
+        // twice and each score gradient by shuffle, and the slots not in use got their zeros here.
+        const int mine = min(lane, kn - 1);
 #pragma unroll
         for (int d4 = 0; d4 < DH / 4; ++d4) {
-          const float4 a = ld4(qi + 4 * d4), b = ld4(gi + 4 * d4);
-          dk[4 * d4] = fmaf(ds, a.x, dk[4 * d4]); dk[4 * d4 + 1] = fmaf(ds, a.y, dk[4 * d4 + 1]);
-          dk[4 * d4 + 2] = fmaf(ds, a.z, dk[4 * d4 + 2]); dk[4 * d4 + 3] = fmaf(ds, a.w, dk[4 * d4 + 3]);
-          dv[4 * d4] = fmaf(p, b.x, dv[4 * d4]); dv[4 * d4 + 1] = fmaf(p, b.y, dv[4 * d4 + 1]);
-          dv[4 * d4 + 2] = fmaf(p, b.z, dv[4 * d4 + 2]); dv[4 * d4 + 3] = fmaf(p, b.w, dv[4 * d4 + 3]);
+          *reinterpret_cast<float4*>(&dk[4 * d4]) = ld4(kb + mine * LDB + 4 * d4);
+          *reinterpret_cast<float4*>(&dv[4 * d4]) = ld4(kb + mine * LDB + D + 4 * d4);
         }
-        float dq = s.dq[i * LDO + h * DH + lane];
-        for (int j = 0; j < kn; ++j) dq = fmaf(__shfl_sync(0xffffffffu, ds, j), kb[j * LDB + lane], dq);
-        s.dq[i * LDO + h * DH + lane] = dq;
+        __syncwarp();
+        float* own = kb + mine * LDB + D;   // in place of the value: score gradients of the queries, then their weights
+#pragma unroll 1
+        for (int i0 = 0; i0 < n; i0 += 4) {   // four queries side by side, the last ones perhaps the last query again
+          float sc[4], dp[4], m[4], l[4], sdp[4], p[4], ds[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int i = min(i0 + u, n - 1);
+            sc[u] = lane < kn ? dot32(q + i * LDQ, dk) * SCALE : -INFINITY;
+            dp[u] = lane < kn ? dot32(go + i * LDO, dv) : 0.f;
+            if (keys <= BLOCK) {
+              m[u] = seg_max<32>(sc[u]);
+              const float e = lane < kn ? expf(sc[u] - m[u]) : 0.f;
+              l[u] = seg_sum<32>(e);
+              sdp[u] = seg_sum<32>(e * dp[u]);
+            } else {
+              m[u] = s.m[i * H + h];
+              l[u] = s.l[i * H + h];
+              sdp[u] = s.s[i * H + h];
+            }
+            p[u] = i0 + u < n ? expf(sc[u] - (m[u] + logf(l[u]))) : 0.f;
+            ds[u] = p[u] * (dp[u] - sdp[u] / l[u]) * SCALE;
+          }
+          if (lane < kn) {
+            *reinterpret_cast<float4*>(own + i0) = make_float4(ds[0], ds[1], ds[2], ds[3]);
+            *reinterpret_cast<float4*>(own + 16 + i0) = make_float4(p[0], p[1], p[2], p[3]);
+          }
+        }
+        __syncwarp();
+        {
+          float a[LPP];
+#pragma unroll
+          for (int i = 0; i < LPP; ++i) a[i] = i < n ? s.dq[i * LDO + h * DH + lane] : 0.f;
+#pragma unroll 4
+          for (int j = 0; j < kn; ++j) {
+            const float k1 = kb[j * LDB + lane];
+#pragma unroll
+            for (int i = 0; i < LPP; i += 4) {
+              const float4 w = ld4(kb + j * LDB + D + i);
+              a[i] = fmaf(w.x, k1, a[i]); a[i + 1] = fmaf(w.y, k1, a[i + 1]); a[i + 2] = fmaf(w.z, k1, a[i + 2]); a[i + 3] = fmaf(w.w, k1, a[i + 3]);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < LPP; ++i)
+            if (i < n) s.dq[i * LDO + h * DH + lane] = a[i];
+        }
+#pragma unroll
+        for (int d = 0; d < DH; ++d) dk[d] = dv[d] = 0.f;
+#pragma unroll 1
+        for (int i0 = 0; i0 < n; i0 += 4) {
+          const float4 ds4 = ld4(own + i0), p4 = ld4(own + 16 + i0);
+          const float ds[4] = {ds4.x, ds4.y, ds4.z, ds4.w}, p[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {   // past the last query both are 0
+            const int i = min(i0 + u, n - 1);
+            const float* qi = q + i * LDQ;
+            const float* gi = go + i * LDO;
+#pragma unroll
+            for (int d4 = 0; d4 < DH / 4; ++d4) {
+              const float4 a = ld4(qi + 4 * d4), b = ld4(gi + 4 * d4);
+              dk[4 * d4] = fmaf(ds[u], a.x, dk[4 * d4]); dk[4 * d4 + 1] = fmaf(ds[u], a.y, dk[4 * d4 + 1]);
+              dk[4 * d4 + 2] = fmaf(ds[u], a.z, dk[4 * d4 + 2]); dk[4 * d4 + 3] = fmaf(ds[u], a.w, dk[4 * d4 + 3]);
+              dv[4 * d4] = fmaf(p[u], b.x, dv[4 * d4]); dv[4 * d4 + 1] = fmaf(p[u], b.y, dv[4 * d4 + 1]);
+              dv[4 * d4 + 2] = fmaf(p[u], b.z, dv[4 * d4 + 2]); dv[4 * d4 + 3] = fmaf(p[u], b.w, dv[4 * d4 + 3]);
+            }
+          }
+        }
+      } else {
+#pragma unroll
+        for (int d = 0; d < DH; ++d) dk[d] = dv[d] = 0.f;
+        for (int i = 0; i < n; ++i) {
+          const float l = s.l[i * H + h], lse = s.m[i * H + h] + logf(l), delta = s.s[i * H + h] / l;
+          const float* qi = q + i * LDQ;
+          const float* gi = go + i * LDO;
+          float p = 0.f, ds = 0.f;
+          if (lane < kn) {
+            p = expf(dot32(qi, kb + lane * LDB) * SCALE - lse);
+            ds = p * (dot32(gi, kb + lane * LDB + D) - delta) * SCALE;
+          }
+#pragma unroll
+          for (int d4 = 0; d4 < DH / 4; ++d4) {
+            const float4 a = ld4(qi + 4 * d4), b = ld4(gi + 4 * d4);
+            dk[4 * d4] = fmaf(ds, a.x, dk[4 * d4]); dk[4 * d4 + 1] = fmaf(ds, a.y, dk[4 * d4 + 1]);
+            dk[4 * d4 + 2] = fmaf(ds, a.z, dk[4 * d4 + 2]); dk[4 * d4 + 3] = fmaf(ds, a.w, dk[4 * d4 + 3]);
+            dv[4 * d4] = fmaf(p, b.x, dv[4 * d4]); dv[4 * d4 + 1] = fmaf(p, b.y, dv[4 * d4 + 1]);
+            dv[4 * d4 + 2] = fmaf(p, b.z, dv[4 * d4 + 2]); dv[4 * d4 + 3] = fmaf(p, b.w, dv[4 * d4 + 3]);
+          }
+          float dq = s.dq[i * LDO + h * DH + lane];
+          for (int j = 0; j < kn; ++j) dq = fmaf(__shfl_sync(0xffffffffu, ds, j), kb[j * LDB + lane], dq);
+          s.dq[i * LDO + h * DH + lane] = dq;
+        }
       }
       __syncwarp();          // the head's keys and values of this block are done: their gradients take their place
       if (lane < kn)
@@ -289,7 +448,7 @@ __global__ void __launch_bounds__(THREADS, BULLETS || LPP == 32 ? 4 : LPP == 16 
       __syncthreads();
       for (int i = threadIdx.x; i < kn * (2 * D / 4); i += THREADS) {
         const int r = i / (2 * D / 4), qq = i % (2 * D / 4);
-        *parts_at<2>(c.dkvb, c.ld_dkvb, c.off_dkvb, g * c.nb + s.list[k0 + r], qq) = ld4(s.kv + r * LDB + qq * 4);
+        *parts_at<2>(c.dkvb, c.ld_dkvb, c.off_dkvb, row(k0 + r), qq) = ld4(s.kv + r * LDB + qq * 4);
       }
     }
   }
@@ -423,9 +582,8 @@ bool supported(int d_model, int n_heads, int n, int nb) {
 }
 int forward(const Call& c, cudaStream_t st) {
   if (c.G <= 0) return 0;
-  if (c.n <= 8) return launch(k_env_attn_fwd<8>, c, false, st);
-  if (c.n <= 16) return launch(k_env_attn_fwd<16>, c, false, st);
-  return launch(k_env_attn_fwd<32>, c, false, st);
+  if (c.kvb) return c.n <= 8 ? launch(k_env_attn_fwd<8, true>, c, false, st) : c.n <= 16 ? launch(k_env_attn_fwd<16, true>, c, false, st) : launch(k_env_attn_fwd<32, true>, c, false, st);
+  return c.n <= 8 ? launch(k_env_attn_fwd<8, false>, c, false, st) : c.n <= 16 ? launch(k_env_attn_fwd<16, false>, c, false, st) : launch(k_env_attn_fwd<32, false>, c, false, st);
 }
 int backward(const Call& c, cudaStream_t st) {
   if (c.G <= 0) return 0;

@@ -13,6 +13,7 @@ struct Call {
   const uint8_t* alive;     // (G * n) or null
   const float* kvb;         // (G * nb, 2 * 128) bullet keys | values, or null
   const uint8_t* bactive;   // (G * nb) or null: every slot is a key
+  const int* boff;          // or rows of the slots that are keys only: those of group g are [boff[g], boff[g + 1]), in kvb and dkvb
   int G, n, nb;
   float* o;                 // forward: (G * n, 128)
   const float* d_o;         // gradient: (G * n, 128) in; out q | k | v and keys | values, rows ld apart, the parts off apart

@@ -52,7 +52,7 @@ __device__ __forceinline__ float4 add4(const float4& a, const float4& b) { retur
 
 struct FwdArgs {
   Forward f;
-  int rows, tiles;
+  int rows;
   int* status;
   int* host_status;
 };
@@ -79,7 +79,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_fwd(const __grid_constant
   const int warp = threadIdx.x >> 5;
   auto set_of = [](int i) { return LAG ? i & 1 : 0; };
   auto phase_of = [](int i) { return (uint32_t)(LAG ? i >> 1 : i); };
-  const int my_tiles = (int)blockIdx.x < a.tiles ? (a.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  const int rows = a.f.count ? min(*a.f.count, a.rows) : a.rows, tiles = (rows + TILE - 1) / TILE;
+  const int my_tiles = (int)blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
   if (warp == LOAD_WARP) {
     if (elect_one()) {
       mbar_expect_tx(s.bars + 8 * F_W, NB * TILE_BYTES);
@@ -116,14 +117,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_fwd(const __grid_constant
       for (int b = 0; b < NB; ++b) {
         float4 extra[8];
         const float4 bias = a.f.bias[b] ? load4(a.f.bias[b] + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (NB == 1 && a.f.residual) rows_in(extra, a.f.residual, m, first, a.rows);
+        if (NB == 1 && a.f.residual) rows_in(extra, a.f.residual, m, first, rows);
         __syncwarp();
         stage_rows(lane_addr + set_of(i) * (NB * 128) + 128 * b + part * 32, stage, m.lane);
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int r = first + m.row(k);
-          if (r >= a.rows) continue;
+          if (r >= rows) continue;
           float4 v = add4(staged_row(stage, k, m.lane), bias);
           if (NB == 1 && a.f.residual) v = add4(v, extra[k]);
           store4(a.f.out[b] + (size_t)r * a.f.ld_out + m.col, v);
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_fwd(const __grid_constant
       tc_fence_before();
     };
     float4 x[8];
-    if (my_tiles > 0) rows_in(x, a.f.x, m, blockIdx.x * TILE, a.rows);
+    if (my_tiles > 0) rows_in(x, a.f.x, m, blockIdx.x * TILE, rows);
 #pragma unroll 1
     for (int i = 0; i < my_tiles; ++i) {
       const int first = (blockIdx.x + i * gridDim.x) * TILE;
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_fwd(const __grid_constant
           const uint2 n = make_uint2(pack_bf16(x[k].x * inv[k] * gain.x, x[k].y * inv[k] * gain.y), pack_bf16(x[k].z * inv[k] * gain.z, x[k].w * inv[k] * gain.w));
           *reinterpret_cast<uint2*>(tile + (m.col >> 6) * CHUNK_BYTES + row_swz(m, k, (m.col & 63) >> 3) + ((m.col >> 2) & 1) * 8) = n;
           const int r = first + m.row(k);
-          if (r >= a.rows) continue;
+          if (r >= rows) continue;
           *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.f.n_out) + (size_t)r * D + m.col) = n;
           if (m.col == 0) a.f.inv[r] = inv[k];
         }
@@ -157,7 +158,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_fwd(const __grid_constant
         for (int k = 0; k < 8; ++k) put_row4(tile, m, k, x[k]);
       }
       post(s, F_OP0 + set_of(i));
-      if (i + 1 < my_tiles) rows_in(x, a.f.x, m, (blockIdx.x + (i + 1) * gridDim.x) * TILE, a.rows);
+      if (i + 1 < my_tiles) rows_in(x, a.f.x, m, (blockIdx.x + (i + 1) * gridDim.x) * TILE, rows);
       if (!LAG) finish(i);
       else if (i > 0) finish(i - 1);
     }
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_fwd(const __grid_constant
 
 struct BwdArgs {
   Backward b;
-  int rows, tiles;
+  int rows;
   int* status;
   int* host_status;
 };
@@ -232,7 +233,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_bwd(const __grid_constant
   const Sync s{smem_u32(f.bars), a.status, f.aborted};
   const uint32_t tmem = *f.tmem_slot, base = smem_u32(smem);
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int my_tiles = (int)blockIdx.x < a.tiles ? (a.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  const int rows = a.b.count ? min(*a.b.count, a.rows) : a.rows, tiles = (rows + TILE - 1) / TILE;
+  const int my_tiles = (int)blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
   // tensor memory: d W of block b at 128 b, dn at 384
   if (warp == LOAD_WARP) {
     if (elect_one()) {
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_bwd(const __grid_constant
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
         const int bar = group * Map::SLOTS + slot, row = tile * TILE + 32 * group + PIECE_ROWS * h;
-        const int n = min(max(a.rows - row, 0), PIECE_ROWS);
+        const int n = min(max(rows - row, 0), PIECE_ROWS);
         const uint32_t full = s.bars + 8 * (G_FULL + bar);
         s.wait(Map::FREE + bar, free_parity, TIMEOUT_FREE);
         if (__any_sync(0xffffffffu, s.aborted[0])) return false;
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_bwd(const __grid_constant
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float4 v = *reinterpret_cast<const float4*>(at + 4 * k * (D * 4));
-        row(4 * h + k, first + m.row(4 * h + k) < a.rows ? v : make_float4(0.f, 0.f, 0.f, 0.f));
+        row(4 * h + k, first + m.row(4 * h + k) < rows ? v : make_float4(0.f, 0.f, 0.f, 0.f));
       }
       __syncwarp();
       if (m.lane == 0) mbar_arrive(s.bars + 8 * (Map::FREE + bar));
@@ -339,8 +341,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_bwd(const __grid_constant
       for (int k = 0; k < 4; ++k) {
         const int row = m.row0 + 8 * k + (m.lane >> 2), r = tile * TILE + row, g = 4 * part + (m.lane & 3);
         const uint32_t dst = smem_u32(smem + Map::N + (part >> 1) * CHUNK_BYTES + swz(row, g & 7));
-        const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.b.n) + (size_t)(r < a.rows ? r : 0) * D + 8 * g;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(r < a.rows ? 16 : 0) : "memory");
+        const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.b.n) + (size_t)(r < rows ? r : 0) * D + 8 * g;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(r < rows ? 16 : 0) : "memory");
       }
     };
     const float4 gain = NORM ? load4(a.b.gain + m.col) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -350,7 +352,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_bwd(const __grid_constant
       const int tile = blockIdx.x + i * gridDim.x, first = tile * TILE;
       float4 u[8], v[8];
       float inv = 0.f;   // of the row that is this lane's among the warp's
-      if (NORM && first + m.row0 + m.lane < a.rows) inv = a.b.inv[first + m.row0 + m.lane];
+      if (NORM && first + m.row0 + m.lane < rows) inv = a.b.inv[first + m.row0 + m.lane];
       take(u, first);
       if constexpr (NORM) {
         asm volatile("cp.async.wait_all;" ::: "memory");   // n
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_bwd(const __grid_constant
           const int r = first + m.row(k);
           const float* p = sums + m.row(k);
           const float w = __shfl_sync(0xffffffffu, inv, 4 * k + (m.lane >> 3)), c = ((p[0] + p[TILE]) + (p[2 * TILE] + p[3 * TILE])) * w * w * w * (1.0f / D);
-          if (r >= a.rows) return;
+          if (r >= rows) return;
           d.x += w * gain.x * u[k].x - v[k].x * c; d.y += w * gain.y * u[k].y - v[k].y * c;
           d.z += w * gain.z * u[k].z - v[k].z * c; d.w += w * gain.w * u[k].w - v[k].w * c;
           store4(a.b.dx + (size_t)r * D + m.col, d);
@@ -410,7 +412,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_linear_bwd(const __grid_constant
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int r = first + m.row(k);
-          if (r < a.rows) store4(a.b.dx + (size_t)r * D + m.col, v[k]);
+          if (r < rows) store4(a.b.dx + (size_t)r * D + m.col, v[k]);
         }
       }
     }
@@ -483,7 +485,7 @@ int forward(const Forward& f, int* status, cudaStream_t st) {
   if (f.rows == 0) return BNB_OK;
   if (!configure()) return BNB_ERR_LAUNCH;
   const int tiles = (int)((f.rows + TILE - 1) / TILE);
-  const FwdArgs a{f, (int)f.rows, tiles, status, tensor::host_status_word(st)};
+  const FwdArgs a{f, (int)f.rows, status, tensor::host_status_word(st)};
   const dim3 grid(grid_of(tiles));
   return f.blocks == 1   ? launch_after(k_linear_fwd<1>, grid, THREADS, FwdMap<1>::BYTES, st, a)
          : f.blocks == 2 ? launch_after(k_linear_fwd<2>, grid, THREADS, FwdMap<2>::BYTES, st, a)
@@ -494,7 +496,7 @@ int backward(const Backward& b, int* status, cudaStream_t st) {
   if (b.rows == 0) return BNB_OK;
   if (!configure()) return BNB_ERR_LAUNCH;
   const int tiles = (int)((b.rows + TILE - 1) / TILE);
-  const BwdArgs a{b, (int)b.rows, tiles, status, tensor::host_status_word(st)};
+  const BwdArgs a{b, (int)b.rows, status, tensor::host_status_word(st)};
   const dim3 grid(grid_of(tiles));
   if (b.gain && b.blocks == 3) return launch_after(k_linear_bwd<3, true>, grid, THREADS, BwdMap<3>::BYTES, st, a);
   if (b.gain && b.blocks == 2) return launch_after(k_linear_bwd<2, true>, grid, THREADS, BwdMap<2>::BYTES, st, a);

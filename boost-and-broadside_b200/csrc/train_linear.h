@@ -28,6 +28,7 @@ struct Forward {
   int ld_out = 128;
   const float* residual = nullptr;
   size_t rows = 0;
+  const int* count = nullptr;   // on the device: how many of the rows there are, or null: all
 };
 [[nodiscard]] int forward(const Forward& f, int* status, cudaStream_t st);
 
@@ -50,6 +51,7 @@ struct Backward {
   const float* dres = nullptr;
   float* d_gain = nullptr;
   size_t rows = 0;
+  const int* count = nullptr;   // as in Forward
 };
 [[nodiscard]] int backward(const Backward& b, int* status, cudaStream_t st);
 
