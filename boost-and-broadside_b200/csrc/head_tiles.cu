@@ -8,9 +8,10 @@
 // The hidden layer never leaves tensor memory and registers: a thread takes 64 hidden columns of its row, four threads
 // add up the row's squares, and the activations go back as the A operand of the second product over the columns they
 // came from.  Tensor memory holds two tiles, so the first product of the next tile runs under this one's epilogue, which
-// is the bound: about 24 instructions per hidden element (issue slots 57 % busy for three heads of 65 536 rows, the tensor
-// pipe 12 %, DRAM 3 % of peak; 40 % for an encoder, whose rows come in element by element).  On mma.sync tiles of 16 rows, with the first product computed
-// twice for the norm, three heads of 65 536 rows took 139 us and take 67, one of 16 384 rows 39 and 14, one of 128 rows no less.
+// is the bound: about 12 instructions per hidden element, two elements at a time (24 one by one: three heads of 65 536 rows and the win
+// head's teams 73 -> 67 us, an encoder of 98 304 rows 64 -> 59; issue slots were 57 % busy, the tensor pipe 12 %, DRAM 3 % of
+// peak, and the chain of a tile's phases is what is left; an encoder's rows come in element by element).  On mma.sync tiles of 16 rows, with
+// the first product computed twice for the norm, three heads of 65 536 rows took 139 us, one of 16 384 rows 39 (14 here), one of 128 rows no less.
 #include "head_tiles.h"
 
 #include "launch_after.h"
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
   float *g1 = b1 + HIDDEN, *b2 = g1 + HIDDEN, *g2 = b2 + OUT;
   for (int i = tid; i < HIDDEN; i += THREADS) {
     b1[i] = round_bf16(chain.b1[i]);
-    g1[i] = chain.g1[i];
+    g1[i] = 0.5f * chain.g1[i];   // see activation
   }
   if (tid < OUT) {
     b2[tid] = tid < chain.out_store ? round_bf16(chain.b2[tid]) : 0.f;
@@ -186,13 +187,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
         uint32_t v[32];
         tmem_ld32(lane_addr + 256 * (i & 1) + 128 + 32 * part, v);
         tc_fence_before();
-        float ss = 0.f;
+        F2 sq = f2(0.f);
+        const F2* bias = reinterpret_cast<const F2*>(b2 + 32 * part);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float h = round_bf16(__uint_as_float(v[j]) + b2[32 * part + j]);
-          ss = fmaf(h, h, ss);
-          v[j] = __float_as_uint(h);
+        for (int j = 0; j < 16; ++j) {
+          v[j] = pack_bf16(add(f2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), bias[j]));
+          const F2 h = unpack_bf16(v[j]);
+          sq = fma(h, h, sq);
         }
+        const float2 sq2 = halves(sq);
+        const float ss = sq2.x + sq2.y;
         float* sums = reinterpret_cast<float*>(smem + M::SUMS) + 1024 + (i & 1) * 512 + (tid & (TILE - 1));
         sums[part * TILE] = ss;
         asm volatile("bar.sync %0, 128;" ::"r"(3 + quarter) : "memory");
@@ -203,10 +207,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
         for (int q = 0; q < 4; ++q) {
           uint32_t w[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int c = 8 * q + 2 * j;
-            w[j] = pack_bf16(__uint_as_float(v[c]) * inv * g2[32 * part + c], __uint_as_float(v[c + 1]) * inv * g2[32 * part + c + 1]);
-          }
+          for (int j = 0; j < 4; ++j)
+            w[j] = pack_bf16(mul(mul(unpack_bf16(v[4 * q + j]), f2(inv)), reinterpret_cast<const F2*>(g2 + 32 * part)[4 * q + j]));
           if (r < rows) y[q] = make_uint4(w[0], w[1], w[2], w[3]);
         }
       } else {     // eight output columns of this thread's row
@@ -248,22 +250,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
       s.wait(HB_ACC0 + (i & 1), i >> 1, TIMEOUT_ACC);
       tc_fence_after();
       const uint32_t acc = lane_addr + 256 * (i & 1);
-      uint32_t v[64];
-      tmem_ld_cols<64>(acc + 64 * part, v);
-      tmem_wait_ld();
-      float ss = 0.f;
+      uint32_t v[32];   // the Linear's output, two bfloat16 a word
+      F2 sq = f2(0.f);
       const float4* bias = reinterpret_cast<const float4*>(b1 + 64 * part);
 #pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const float4 b = bias[q];
-        const float bb[4] = {b.x, b.y, b.z, b.w};
+      for (int c = 0; c < 2; ++c) {
+        uint32_t t[32];
+        tmem_ld32(acc + 64 * part + 32 * c, t);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float h = round_bf16(__uint_as_float(v[4 * q + j]) + bb[j]);
-          ss = fmaf(h, h, ss);
-          v[4 * q + j] = __float_as_uint(h);
+        for (int q = 0; q < 8; ++q) {
+          const float4 b = bias[8 * c + q];
+          uint32_t* w = v + 16 * c + 2 * q;
+          w[0] = pack_bf16(add(f2(__uint_as_float(t[4 * q]), __uint_as_float(t[4 * q + 1])), f2(b.x, b.y)));
+          w[1] = pack_bf16(add(f2(__uint_as_float(t[4 * q + 2]), __uint_as_float(t[4 * q + 3])), f2(b.z, b.w)));
+          const F2 h0 = unpack_bf16(w[0]), h1 = unpack_bf16(w[1]);
+          sq = fma(h1, h1, fma(h0, h0, sq));
         }
       }
+      const float2 sq2 = halves(sq);
+      const float ss = sq2.x + sq2.y;
       float* sums = reinterpret_cast<float*>(smem + M::SUMS) + (i & 1) * 512 + (tid & (TILE - 1));   // two buffers: one barrier a tile
       sums[part * TILE] = ss;
       tc_fence_before();
@@ -271,18 +276,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
       tc_fence_after();
       const float inv = rsqrtf(((sums[0] + sums[TILE]) + (sums[2 * TILE] + sums[3 * TILE])) / (float)HIDDEN + kRmsEps);
       const float4* gain = reinterpret_cast<const float4*>(g1 + 64 * part);
+      const F2 inv2 = f2(inv);
 #pragma unroll
       for (int o = 0; o < 4; ++o) {
         uint32_t w[8];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const float4 g = gain[4 * o + q];
-          const float gg[4] = {g.x, g.y, g.z, g.w};
-          float z[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) z[j] = gelu_fast(round_bf16(__uint_as_float(v[16 * o + 4 * q + j]) * inv * gg[j]));
-          w[2 * q] = pack_bf16(z[0], z[1]);
-          w[2 * q + 1] = pack_bf16(z[2], z[3]);
+          w[2 * q] = activation(v[8 * o + 2 * q], inv2, f2(g.x, g.y));
+          w[2 * q + 1] = activation(v[8 * o + 2 * q + 1], inv2, f2(g.z, g.w));
         }
         tmem_st8_nowait(acc + 32 * part + 8 * o, w);
       }

@@ -18,7 +18,7 @@
 // passed through the GELU and multiplied into the output accumulators straight away.  The RMSNorm
 // needs the whole row's sum of squares first: for a hidden layer wider than one chunk Linear 1 is
 // computed twice, once for the sum alone (cheaper than a trip through shared memory: the kernel is
-// bound by instruction issue and latency at 16 warps, not by the tensor pipe: 64 us for the 147 000 rows wanted of
+// bound by instruction issue and latency at 16 warps, not by the tensor pipe: 59 us (62 with its activations one by one) for the 147 000 rows wanted of
 // 655 360, issue slots 44 % busy, tensor pipe 16 %, DRAM 6 % of its peak).  No CTA-wide barrier after the weights.
 #include "mlp_kernels.h"
 
@@ -30,13 +30,22 @@
 namespace bnb {
 namespace mlp {
 
-using tensor::gelu_fast;   // the fused trunk kernel's fit of the erf GELU (max relative error 1.2e-3, below bfloat16 rounding)
+using tensor::activation;
+using tensor::add;
+using tensor::f2;
+using tensor::F2;
+using tensor::fma;
+using tensor::halves;
 using tensor::ldsm_x4;
 using tensor::mma_bf16;
 using tensor::pack_bf16;
 using tensor::smem_u32;
+using tensor::unpack_bf16;
 
 namespace {
+
+// A Linear's output of two columns, bias added.
+__device__ __forceinline__ uint32_t biased(float a, float b, const float2& bias) { return pack_bf16(add(f2(a, b), f2(bias.x, bias.y))); }
 
 constexpr int SLICE = 16;      // rows per warp slice (one mma.sync row block)
 // Warps per CTA: 16 where the output accumulators take 64 registers (out_dim 128), 28 where they
@@ -180,7 +189,7 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
   }
   for (int i = tid; i < hidden; i += n_threads) {
     b1s[i] = round_bf16(chain.b1[i]);
-    g1s[i] = chain.g1[i];
+    g1s[i] = 0.5f * chain.g1[i];   // see activation
   }
   for (int i = tid; i < out_dim; i += n_threads) {
     b2s[i] = i < out_store ? round_bf16(chain.b2[i]) : 0.f;
@@ -306,7 +315,7 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
     __syncwarp();
 
     float acc[8][4];
-    float ss0 = 0.f, ss1 = 0.f;
+    F2 sq0 = f2(0.f), sq1 = f2(0.f);
     if (two_pass) {   // the sum of squares of the rounded Linear 1 output, every chunk
 #pragma unroll 1
       for (int ch = 0; ch < NCH; ++ch) {
@@ -315,10 +324,9 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
           const float2 bb = *reinterpret_cast<const float2*>(b1s + c0 + nt * 8 + 2 * t);
-          const float h00 = round_bf16(acc[nt][0] + bb.x), h01 = round_bf16(acc[nt][1] + bb.y);
-          const float h10 = round_bf16(acc[nt][2] + bb.x), h11 = round_bf16(acc[nt][3] + bb.y);
-          ss0 = fmaf(h00, h00, fmaf(h01, h01, ss0));
-          ss1 = fmaf(h10, h10, fmaf(h11, h11, ss1));
+          const F2 h0 = unpack_bf16(biased(acc[nt][0], acc[nt][1], bb)), h1 = unpack_bf16(biased(acc[nt][2], acc[nt][3], bb));
+          sq0 = fma(h0, h0, sq0);
+          sq1 = fma(h1, h1, sq1);
         }
       }
     }
@@ -332,19 +340,21 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
     for (int ch = 0; ch < NCH; ++ch) {
       const int c0 = ch * 64;
       linear1_chunk<IN16>(acc, sX, sW1, ldx, c0, a_off, b_row, b_k);
+      uint32_t hid[8][2];   // the Linear's output
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt) {
         const float2 bb = *reinterpret_cast<const float2*>(b1s + c0 + nt * 8 + 2 * t);
-        acc[nt][0] = round_bf16(acc[nt][0] + bb.x);
-        acc[nt][1] = round_bf16(acc[nt][1] + bb.y);
-        acc[nt][2] = round_bf16(acc[nt][2] + bb.x);
-        acc[nt][3] = round_bf16(acc[nt][3] + bb.y);
+        hid[nt][0] = biased(acc[nt][0], acc[nt][1], bb);
+        hid[nt][1] = biased(acc[nt][2], acc[nt][3], bb);
         if (!two_pass) {
-          ss0 = fmaf(acc[nt][0], acc[nt][0], fmaf(acc[nt][1], acc[nt][1], ss0));
-          ss1 = fmaf(acc[nt][2], acc[nt][2], fmaf(acc[nt][3], acc[nt][3], ss1));
+          const F2 h0 = unpack_bf16(hid[nt][0]), h1 = unpack_bf16(hid[nt][1]);
+          sq0 = fma(h0, h0, sq0);
+          sq1 = fma(h1, h1, sq1);
         }
       }
       if (c0 == 0) {   // the row sums are complete: after the first pass, or with this only chunk
+        const float2 a = halves(sq0), b = halves(sq1);
+        float ss0 = a.x + a.y, ss1 = b.x + b.y;
         ss0 += __shfl_xor_sync(0xffffffffu, ss0, 1);
         ss0 += __shfl_xor_sync(0xffffffffu, ss0, 2);
         ss1 += __shfl_xor_sync(0xffffffffu, ss1, 1);
@@ -361,8 +371,8 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
           for (int hf = 0; hf < 2; ++hf) {
             const int nt = 2 * kk + hf;
             const float2 gg = *reinterpret_cast<const float2*>(g1s + c0 + nt * 8 + 2 * t);
-            a[2 * hf] = pack_bf16(gelu_fast(round_bf16(acc[nt][0] * inv0 * gg.x)), gelu_fast(round_bf16(acc[nt][1] * inv0 * gg.y)));
-            a[2 * hf + 1] = pack_bf16(gelu_fast(round_bf16(acc[nt][2] * inv1 * gg.x)), gelu_fast(round_bf16(acc[nt][3] * inv1 * gg.y)));
+            a[2 * hf] = activation(hid[nt][0], f2(inv0), f2(gg.x, gg.y));
+            a[2 * hf + 1] = activation(hid[nt][1], f2(inv1), f2(gg.x, gg.y));
           }
 #pragma unroll
           for (int np = 0; np < NP2; ++np) {
@@ -378,8 +388,7 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
     }
 
     // ---- bias [+ RMSNorm] of Linear 2, then the first out_store columns of the 16 rows
-    ss0 = 0.f;
-    ss1 = 0.f;
+    float ss0 = 0.f, ss1 = 0.f;
 #pragma unroll
     for (int nt = 0; nt < 2 * NP2; ++nt) {
       {

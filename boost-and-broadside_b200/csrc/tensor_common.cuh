@@ -257,17 +257,9 @@ __device__ __forceinline__ float sqrt_fast(float v) {
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
   return r;
 }
-// erf GeLU as 0.5 x (1 + tanh(x (c1 + c3 x^2 + c5 x^4))): the inner polynomial is a minimax
-// fit to x * Phi(x) (max abs error 2.5e-5, max relative error 1.2e-3 where |gelu| > 1e-2).
-__device__ __forceinline__ float gelu_fast(float v) {
-  const float x2 = fminf(v * v, 100.0f);  // beyond |x| = 10 the polynomial stays positive and tanh saturates
-  float p = fmaf(x2, -3.51516841e-4f, 3.70056464e-2f);
-  p = fmaf(x2, p, 7.97507884e-1f);
-  const float t = tanh_fast(v * p);
-  const float h = 0.5f * v;
-  return fmaf(h, t, h);
-}
-// gelu(2 h) * u for two elements, packed as two bf16: the polynomial of gelu_fast in h = gate / 2 (an exact halving), GELU in
+// erf GELU as 0.5 x (1 + tanh(x (c1 + c3 x^2 + c5 x^4))): the inner polynomial is a minimax fit to x * Phi(x) (max abs error 2.5e-5, max
+// relative error 1.2e-3 where |gelu| > 1e-2); beyond |x| = 10 its x^2 is held at 100, where it is positive and tanh saturates.
+// gelu(2 h) * u for two elements, packed as two bf16: that polynomial in h = gate / 2 (an exact halving), GELU in
 // half precision (11 mantissa bits against the 8 of the bf16 result; h * h saturates at 25 as there, an overflow to inf lands
 // there too), one tanh.approx.f16x2; the product with u in float32.  Halving in the weights saves the
 // multiplication by 0.5 and leaving u in float32 two conversions: 12 instructions instead of 14 for what the GatedMLP spends most of its issue slots on.
@@ -286,7 +278,7 @@ __device__ __forceinline__ uint32_t gelu_half_mul(uint32_t h0, uint32_t h1, uint
       : "+f"(f.x), "+f"(f.y) : "f"(__uint_as_float(u0)), "f"(__uint_as_float(u1)));
   return pack_bf16(f.x, f.y);
 }
-// gelu_fast(2 h) of two elements.
+// gelu(2 h) of two elements in float32.
 __device__ __forceinline__ F2 gelu_half(F2 h) {
   const float2 y = halves(mul(h, h));
   const F2 y2 = f2(fminf(y.x, 25.0f), fminf(y.y, 25.0f));
@@ -302,6 +294,11 @@ __device__ __forceinline__ F2 sigmoid_twice_bf16(F2 v) {
 
 __device__ __forceinline__ F2 unpack_bf16(uint32_t v) { return f2(__uint_as_float(v << 16), __uint_as_float(v & 0xFFFF0000u)); }
 __device__ __forceinline__ uint32_t pack_bf16(F2 a) { const float2 v = halves(a); return pack_bf16(v.x, v.y); }
+// GELU(norm) of two values: rounded to bfloat16 behind the norm (h inv gain) and behind the GELU, the fit above.  half_gain: half
+// the gain, since gelu_half takes half its argument and a halving commutes with the rounding.
+__device__ __forceinline__ uint32_t activation(uint32_t h, F2 inv, F2 half_gain) {
+  return pack_bf16(gelu_half(unpack_bf16(pack_bf16(mul(mul(unpack_bf16(h), inv), half_gain)))));
+}
 // Product of two pairs of bfloat16, rounded once.
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
