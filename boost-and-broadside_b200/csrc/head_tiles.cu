@@ -37,7 +37,9 @@ template <bool ENC> struct Map {
 enum : int { HB_OP0 = 0, HB_ACC0 = 2, HB_ACT0 = 4, HB_OUT0 = 6, HB_COUNT = 8 };
 
 struct Args {
-  MlpCall call;
+  MlpCall calls[2];
+  int n_first;                       // chains of the first call
+  int first[2 * MAX_CHAINS + 1];     // first CTA of each chain, then the grid
   int* host_status;
 };
 
@@ -51,7 +53,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
   extern __shared__ __align__(1024) uint8_t smem[];
   using M = Map<ENC>;
   constexpr int OUT = M::OUT;
-  const MlpChain& chain = a.call.chain[blockIdx.y];
+  int c = 0;
+  while ((int)blockIdx.x >= a.first[c + 1]) ++c;
+  const int block = blockIdx.x - a.first[c], blocks = a.first[c + 1] - a.first[c], in_call = c < a.n_first ? 0 : 1;
+  const MlpCall& call = a.calls[in_call];
+  const MlpChain& chain = call.chain[in_call ? c - a.n_first : c];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   wait_for_previous();
   // operands: eight k of a row per thread and turn, several turns' loads under way; rows of w2 past out_store are zero
@@ -62,7 +68,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
     if constexpr (ENC) {   // rows of any width, zero past it
       float w[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) w[j] = 8 * g + j < a.call.in_dim ? chain.w1[(size_t)r * a.call.w1_ld + 8 * g + j] : 0.f;
+      for (int j = 0; j < 8; ++j) w[j] = 8 * g + j < call.in_dim ? chain.w1[(size_t)r * call.w1_ld + 8 * g + j] : 0.f;
       v = make_uint4(pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]), pack_bf16(w[4], w[5]), pack_bf16(w[6], w[7]));
     } else {
       v = pack_row8(chain.w1 + r * D + 8 * g);
@@ -95,8 +101,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
   const Frame f = open_frame(smem + M::FRAME, status, a.host_status, counts);
   const Sync s{smem_u32(f.bars), status, f.aborted};
   const uint32_t tmem = *f.tmem_slot, base = smem_u32(smem);
-  const int rows = a.call.n_rows, tiles = (rows + TILE - 1) / TILE;
-  const int my_tiles = (int)blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  const int rows = call.n_rows, tiles = (rows + TILE - 1) / TILE;
+  const int my_tiles = block < tiles ? (tiles - block + blocks - 1) / blocks : 0;
 
   if (warp == MMA_WARP) {
     const uint32_t el = elect_one(), tm = uniform(tmem), w1 = desc_lo(base), w2 = desc_lo(base + M::W2);
@@ -106,7 +112,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
       tc_fence_after();
       const uint32_t x = uniform(desc_lo(base + M::A + set * 32768));
       if constexpr (ENC) {
-        const int steps = (a.call.in_dim + 15) / 16;
+        const int steps = (call.in_dim + 15) / 16;
 #pragma unroll 1
         for (int k = 0; k < steps; ++k)
           mma_one<false>(el, tm + 256 * set, uniform(x + (k >> 2) * 1024 + 2 * (k & 3)), uniform(w1 + (k >> 2) * (M::W1_ATOM >> 4) + 2 * (k & 3)), instr_desc(256), k ? 1u : 0u);
@@ -136,12 +142,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
     const bool pairs = ((chain.out_store | chain.y_ld) & 1) == 0;                  // two columns share an aligned word
     // heads: sixteen bytes of four rows; encoder: pairs of the tile's values, which lie in one piece
     uint4 in[ENC ? 8 : 4];
-    const int half = a.call.in_dim >> 1, n_pairs = ENC ? TILE * half : 0;
+    const int half = call.in_dim >> 1, n_pairs = ENC ? TILE * half : 0;
     const float inv_half = ENC ? 1.0f / (float)half : 0.f;
     auto request = [&](int i) {
       if constexpr (ENC) {
-        const float2* src = static_cast<const float2*>(a.call.x) + (size_t)(blockIdx.x + (size_t)i * gridDim.x) * TILE * half;
-        const int left = i < my_tiles ? min(TILE, rows - (int)(blockIdx.x + i * gridDim.x) * TILE) * half : 0;
+        const float2* src = static_cast<const float2*>(call.x) + (size_t)(block + (size_t)i * blocks) * TILE * half;
+        const int left = i < my_tiles ? min(TILE, rows - (block + i * blocks) * TILE) * half : 0;
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
           const int at = tid + EPI_THREADS * k;
@@ -152,12 +158,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
       } else {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const int r = (blockIdx.x + i * gridDim.x) * TILE + row0 + 8 * k;
+          const int r = (block + i * blocks) * TILE + row0 + 8 * k;
           in[k] = make_uint4(0u, 0u, 0u, 0u);
           if (i < my_tiles && r < rows) {
-            const int from = a.call.group_rows ? r / a.call.group_rows * a.call.group_stride + r % a.call.group_rows : r;
-            in[k] = a.call.x_bf16 ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.call.x) + (size_t)from * D + col)
-                                  : pack_row8(static_cast<const float*>(a.call.x) + (size_t)from * D + col);
+            const int from = call.group_rows ? r / call.group_rows * call.group_stride + r % call.group_rows : r;
+            in[k] = call.x_bf16 ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(call.x) + (size_t)from * D + col)
+                                  : pack_row8(static_cast<const float*>(call.x) + (size_t)from * D + col);
           }
         }
       }
@@ -201,7 +207,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
         sums[part * TILE] = ss;
         asm volatile("bar.sync %0, 128;" ::"r"(3 + quarter) : "memory");
         const float inv = rsqrtf(((sums[0] + sums[TILE]) + (sums[2 * TILE] + sums[3 * TILE])) / (float)OUT + kRmsEps);
-        const int r = (blockIdx.x + i * gridDim.x) * TILE + (tid & (TILE - 1));
+        const int r = (block + i * blocks) * TILE + (tid & (TILE - 1));
         uint4* y = reinterpret_cast<uint4*>(chain.y + (size_t)r * OUT + 32 * part);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -218,7 +224,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
         tmem_ld8_nowait(lane_addr + 256 * (i & 1) + 128 + 8 * part, v);
         tmem_wait_ld();
         tc_fence_before();
-        const int r = (blockIdx.x + i * gridDim.x) * TILE + (tid & (TILE - 1));
+        const int r = (block + i * blocks) * TILE + (tid & (TILE - 1));
         if (r >= rows) return;
         __nv_bfloat16* y = chain.y + (size_t)r * chain.y_ld;
 #pragma unroll
@@ -312,7 +318,7 @@ bool head_tiles_serve(const MlpCall& call, int n_chains, int in_pad, int hidden,
          at(call.x) % 8 == 0 && (at(c.w2) | at(c.y)) % 16 == 0;
 }
 
-int head_tiles(const MlpCall& call, int n_chains, int out_dim, cudaStream_t st) {
+int head_tiles(const MlpCall& call, int n_chains, int out_dim, cudaStream_t st, const MlpCall* more, int n_more) {
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BNB_ERR_NO_DEVICE;
@@ -322,9 +328,30 @@ int head_tiles(const MlpCall& call, int n_chains, int out_dim, cudaStream_t st) 
       return BNB_ERR_LAUNCH;
     configured[dev] = true;
   }
-  const Args a{call, host_status_word(st)};
-  const int tiles = (call.n_rows + TILE - 1) / TILE, per_chain = 148 / n_chains;
-  const dim3 grid(tiles < per_chain ? tiles : per_chain, n_chains);
+  Args a{};
+  a.calls[0] = call;
+  if (more) a.calls[1] = *more;
+  a.n_first = n_chains;
+  a.host_status = host_status_word(st);
+  // a CTA fills an SM and stages its weights once: the chains share the SMs out so that none takes more rounds of tiles than it must
+  const int n = n_chains + (more ? n_more : 0);
+  int tiles[2 * MAX_CHAINS], longest = 0;
+  for (int i = 0; i < n; ++i) {
+    tiles[i] = ((i < n_chains ? call : *more).n_rows + TILE - 1) / TILE;
+    longest = tiles[i] > longest ? tiles[i] : longest;
+  }
+  const auto ctas = [&](int rounds) {
+    a.first[0] = 0;
+    for (int i = 0; i < n; ++i) a.first[i + 1] = a.first[i] + (tiles[i] + rounds - 1) / rounds;
+    return a.first[n];
+  };
+  int enough = longest;   // rounds: a CTA a chain
+  for (int few = 0; few + 1 < enough;) {
+    const int mid = few + (enough - few) / 2;
+    if (ctas(mid) <= 148) enough = mid;
+    else few = mid;
+  }
+  const dim3 grid((unsigned)ctas(enough));
   return out_dim == 32 ? launch_after(k_head_tiles<false>, grid, THREADS, Map<false>::BYTES, st, a)
                        : launch_after(k_head_tiles<true>, grid, THREADS, Map<true>::BYTES, st, a);
 }

@@ -17,7 +17,7 @@ namespace mlp {
 //   rows between 16-byte  heads of float32 rows 19 us for 128 rows, 43 for 65 536 (12, 29 on a boundary)
 //   boundaries
 bool head_tiles_serve(const MlpCall& call, int n_chains, int in_pad, int hidden, int out_dim);
-int head_tiles(const MlpCall& call, int n_chains, int out_dim, cudaStream_t st);
+int head_tiles(const MlpCall& call, int n_chains, int out_dim, cudaStream_t st, const MlpCall* more = nullptr, int n_more = 0);
 
 }  // namespace mlp
 }  // namespace bnb

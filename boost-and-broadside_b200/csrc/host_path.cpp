@@ -847,9 +847,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const
   call.chain[0] = chain_of(five(0), dev, "head", logits.data_ptr(), 12, 12, held);
   call.chain[1] = chain_of(five(1), dev, "head", pred.data_ptr(), (int)P, (int)P, held);
   call.chain[2] = chain_of(five(2), dev, "head", value.data_ptr(), (int)K, (int)K, held);
-  check("bnb_head_mlp_fwd", bnb::mlp::run(call, 3, (int)D, (int)(2 * D), 32, stream));
-
   Tensor win, rows, fold;
+  bnb::mlp::MlpCall wc{};   // the win head over the teams' rows, in the heads' launch
   if (W > 0) {
     rows = at::empty({B * 2, D}, bf);
     win = at::empty({B * 2, W}, bf);
@@ -859,14 +858,13 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> policy_tail(const Tensor& x_in, const
     check("bnb_team_pma_fwd", bnb::tail::team_rows(s, aligned_parameter(pma[0], dev, "TeamPMA", held), in_proj, out_proj,
                                                    aligned_parameter(pma[3], dev, "TeamPMA", held), fold.data_ptr(),
                                                    static_cast<__nv_bfloat16*>(rows.data_ptr()), stream));
-    bnb::mlp::MlpCall wc{};
     wc.x = rows.data_ptr();
     wc.x_bf16 = 1;
     wc.n_rows = (int)(B * 2);
     wc.in_dim = wc.w1_ld = (int)D;
     wc.chain[0] = chain_of(five(3), dev, "head", win.data_ptr(), (int)W, (int)W, held);
-    check("bnb_head_mlp_fwd", bnb::mlp::run(wc, 1, (int)D, (int)(2 * D), 32, stream));
   }
+  check("bnb_head_mlp_fwd", bnb::mlp::run(call, 3, (int)D, (int)(2 * D), 32, stream, W > 0 ? &wc : nullptr, 1));
   check("bnb_action_dist_fwd", bnb::tail::finish(s, static_cast<const __nv_bfloat16*>(logits.data_ptr()), static_cast<const float*>(uniforms.data_ptr()),
                                                  static_cast<int64_t*>(action.data_ptr()), static_cast<__nv_bfloat16*>(logprob.data_ptr()),
                                                  W > 0 ? static_cast<const __nv_bfloat16*>(win.data_ptr()) : nullptr, (int)W, cols.data(),

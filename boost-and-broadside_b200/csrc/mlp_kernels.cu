@@ -451,7 +451,18 @@ bool supported(int in_pad, int hidden, int out_dim) {
   return layout(in_pad, hidden, out_dim).warps >= 4;
 }
 
-int run(const MlpCall& call, int n_chains, int in_pad, int hidden, int out_dim, cudaStream_t st) {
+int run(const MlpCall& call, int n_chains, int in_pad, int hidden, int out_dim, cudaStream_t st, const MlpCall* more, int n_more) {
+  if (more && more->n_rows > 0 && n_more > 0) {
+    const auto tiled = [&](const MlpCall& c, int n) {
+      if (!supported(in_pad, hidden, out_dim) || n < 1 || n > MAX_CHAINS || c.n_rows <= 0 || (c.x_bf16 && (c.in_dim != in_pad || (reinterpret_cast<uintptr_t>(c.x) & 15)))) return false;
+      for (int i = 0; i < n; ++i)
+        if (reinterpret_cast<uintptr_t>(c.chain[i].y) & 3) return false;
+      return head_tiles_serve(c, n, in_pad, hidden, out_dim);
+    };
+    if (out_dim == 32 && tiled(call, n_chains) && tiled(*more, n_more)) return head_tiles(call, n_chains, out_dim, st, more, n_more);
+    const int rc = run(call, n_chains, in_pad, hidden, out_dim, st);
+    return rc ? rc : run(*more, n_more, in_pad, hidden, out_dim, st);
+  }
   if (!supported(in_pad, hidden, out_dim) || n_chains < 1 || n_chains > MAX_CHAINS) return BNB_ERR_UNSUPPORTED_DIMS;
   if (call.x_bf16 && (call.in_dim != in_pad || (reinterpret_cast<uintptr_t>(call.x) & 15))) return BNB_ERR_UNSUPPORTED_DIMS;
   if (call.n_rows <= 0) return BNB_OK;

@@ -32,7 +32,8 @@ struct MlpCall {
   const uint8_t* active;    // only rows with a non-zero byte are computed and written; null: all
   MlpChain chain[MAX_CHAINS];
 };
-int run(const MlpCall& call, int n_chains, int in_pad, int hidden, int out_dim, cudaStream_t st);
+// more: chains of the same widths over other rows, in the same launch where the row tiles take both.
+int run(const MlpCall& call, int n_chains, int in_pad, int hidden, int out_dim, cudaStream_t st, const MlpCall* more = nullptr, int n_more = 0);
 
 // bfloat16 contract (see bnb_encoder_mlp_fwd / bnb_head_mlp_fwd).  g2 null: no final norm.
 // x holds float32 rows, or (x_bf16) bfloat16 rows on a 16-byte boundary with in_dim == in_pad.
