@@ -307,7 +307,8 @@ __device__ __forceinline__ void flash_finish(FlashState& f) {
 // Bound by latency and issue around small mma.sync tiles.  8192 environments of 12 tokens with 18 of 80 bullets 74 -> 51 us, 1024
 // of 152 tokens 93 -> 80: keys past a block of 32 in one of 16, nothing to rescale in the first block (every block of most
 // environments), pairs of scores in one instruction, the heads of a CTA a constant (divisions by it), 48 bullet rows of shared
-// memory instead of every slot's, results out as whole rows.  Eighty registers with a few spilled: with 126 the steps take
+// memory instead of every slot's, results out as whole rows.  One copy of the walk and loops that stay loops: a small launch waits for its
+// instructions (28 environments of 6 tokens with bullets 117.3 us a step with a copy each, unrolled, 115.7 so; 1024 of 152 1404 and 1396).  Eighty registers with a few spilled: with 126 the steps take
 // 844 us instead of 835 and 1432 instead of 1404, with 64 860 and 1404.
 template <int HPC, bool BULLETS>
 __global__ void __launch_bounds__(256, 3) k_attention_flash(const __nv_bfloat16* __restrict__ qkv, const uint8_t* __restrict__ alive,
@@ -340,6 +341,7 @@ __global__ void __launch_bounds__(256, 3) k_attention_flash(const __nv_bfloat16*
   // asynchronous 16-byte copies: all of them are in flight before the first one is waited for
   {
     const __nv_bfloat16* src = qkv + tok0 * (3 * D) + hd0 * DH;
+#pragma unroll 1
     for (int i = threadIdx.x; i < n * 3 * GPR; i += threads) {
       const uint32_t r = (uint32_t)i / (3 * GPR), rem = (uint32_t)i % (3 * GPR), part = rem / GPR, q = rem % GPR;
       cp_async16(q_at + (part * n + r) * STRIDE + q * 16, src + r * (3 * D) + part * D + q * 8);
@@ -347,13 +349,16 @@ __global__ void __launch_bounds__(256, 3) k_attention_flash(const __nv_bfloat16*
   }
   auto stage_bullets = [&](int b0, int rows) {
     const __nv_bfloat16* src = kvb + (brow0 + b0) * (2 * D) + hd0 * DH;
+#pragma unroll 1
     for (int i = threadIdx.x; i < rows * 2 * GPR; i += threads) {
       const uint32_t r = (uint32_t)i / (2 * GPR), rem = (uint32_t)i % (2 * GPR), part = rem / GPR, q = rem % GPR;
       cp_async16((part ? vb_at : kb_at) + r * STRIDE + q * 16, src + r * (2 * D) + part * D + q * 8);
     }
+#pragma unroll 1
     for (int i = threadIdx.x; i < nb32; i += threads) bias_b[i] = i < rows ? 0.f : -INFINITY;
   };
   if (BULLETS && nb > 0) stage_bullets(0, n_stage);
+#pragma unroll 1
   for (int i = threadIdx.x; i < n32; i += threads)
     bias_s[i] = i < n ? ((!alive || alive[tok0 + i]) ? 0.f : kMaskedScore) : -INFINITY;
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -378,34 +383,33 @@ __global__ void __launch_bounds__(256, 3) k_attention_flash(const __nv_bfloat16*
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks)
         ldsm_x4(q_at + hoff + row * STRIDE + (ks * 16 + (lane >> 4) * 8) * 2, qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3]);
-      flash_walk<HPC>(f, true, qa, k_at + hoff + k_lane, v_at + hoff + v_lane, bias_s, n, lane);
+    }
+    // The environment's own keys, then its bullets: one copy of the walk.
+#pragma unroll 1
+    for (int pass = 0; pass < (BULLETS && nb > 0 ? 2 : 1); ++pass) {
+      const int keys = pass ? nb : n, step = pass ? stage : n;
+      const uint32_t k = (pass ? kb_at : k_at) + hoff + k_lane, v = (pass ? vb_at : v_at) + hoff + v_lane;
+#pragma unroll 1
+      for (int b0 = 0; b0 < keys; b0 += step) {
+        const int rows = min(step, keys - b0);
+        if (b0 > 0) {   // bullets past the first stage
+          __syncthreads();   // the rows before have been read
+          if constexpr (BULLETS) stage_bullets(b0, rows);
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          __syncthreads();
+        }
+        if (mine) flash_walk<HPC>(f, b0 == 0, qa, k, v, pass ? bias_b : bias_s, rows, lane);
+      }
+      if (!mine) continue;
       flash_finish(f);
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        out[nt][0] = pack_bf16(f.acc[nt][0], f.acc[nt][1]);
-        out[nt][1] = pack_bf16(f.acc[nt][2], f.acc[nt][3]);
-      }
-    }
-    if (BULLETS && nb > 0) {
-      if (mine) flash_walk<HPC>(f, true, qa, kb_at + hoff + k_lane, vb_at + hoff + v_lane, bias_b, n_stage, lane);
-#pragma unroll 1
-      for (int b0 = stage; b0 < nb; b0 += stage) {
-        const int rows = min(stage, nb - b0);
-        __syncthreads();   // the rows before have been read
-        stage_bullets(b0, rows);
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-        if (mine) flash_walk<HPC>(f, false, qa, kb_at + hoff + k_lane, vb_at + hoff + v_lane, bias_b, rows, lane);
-      }
-      if (mine) {
-        flash_finish(f);
-        // both outputs are bf16 tensors in the reference; so is their sum
+      for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-          for (int r = 0; r < 2; ++r)
-            out[nt][r] = pack_bf16(bf16_lo(out[nt][r]) + round_bf16(f.acc[nt][2 * r]), bf16_hi(out[nt][r]) + round_bf16(f.acc[nt][2 * r + 1]));
-      }
+        for (int r = 0; r < 2; ++r) {
+          const uint32_t o16 = pack_bf16(f.acc[nt][2 * r], f.acc[nt][2 * r + 1]);
+          // both outputs are bf16 tensors in the reference; so is their sum
+          out[nt][r] = pass ? pack_bf16(bf16_lo(out[nt][r]) + bf16_lo(o16), bf16_hi(out[nt][r]) + bf16_hi(o16)) : o16;
+        }
     }
     // into the place of these queries, which this warp alone reads
     if (mine) {
@@ -420,6 +424,7 @@ __global__ void __launch_bounds__(256, 3) k_attention_flash(const __nv_bfloat16*
     }
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = threadIdx.x; i < n * GPR; i += threads) {
     const int r = i / GPR, q = i % GPR;
     *reinterpret_cast<uint4*>(o + (tok0 + r) * D + hd0 * DH + q * 8) = *reinterpret_cast<const uint4*>(fs + r * STRIDE + q * 16);
