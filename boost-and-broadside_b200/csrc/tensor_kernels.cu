@@ -173,10 +173,12 @@ __global__ void k_pack_trunk(const __grid_constant__ PackJobs jobs) {
 // a staged row holds HPC x 32 bf16 plus 16 bytes of padding, which keeps ldmatrix conflict-free.
 __host__ __device__ constexpr int flash_stride(int hpc) { return hpc * 64 + 16; }
 
-// Running softmax of a block of 16 queries: a lane's two query rows, sums of its own columns in pairs.
+// Running softmax of a block of 16 queries: a lane's two query rows, the sums of its own columns side by side.  A row's sum takes
+// its two columns of 8 keys together and those of the blocks one after the other, whatever the stage: an order of its own for
+// each size moves the last bits of the result, and bfloat16 roundings of the sublayers behind it carry that on (1e-4 of the state).
 struct FlashState {
   float m[2];
-  F2 l[2];
+  F2 l;
   float acc[4][4];
 };
 // One block of 8 NT keys from key0 on (at least one of them a key).  k and v: staged rows at this head and this lane's ldmatrix
@@ -223,12 +225,11 @@ __device__ __forceinline__ void flash_block(FlashState& f, const uint32_t (&qa)[
   if constexpr (!FIRST) {
     m0 = fmaxf(m0, f.m[0]);
     m1 = fmaxf(m1, f.m[1]);
-    const F2 c0 = f2(ex2_fast(f.m[0] - m0)), c1 = f2(ex2_fast(f.m[1] - m1));
-    f.l[0] = mul(f.l[0], c0);
-    f.l[1] = mul(f.l[1], c1);
+    const float c0 = ex2_fast(f.m[0] - m0), c1 = ex2_fast(f.m[1] - m1);
+    f.l = mul(f.l, f2(c0, c1));
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
-      const float2 a = halves(mul(f2(f.acc[nt][0], f.acc[nt][1]), c0)), b = halves(mul(f2(f.acc[nt][2], f.acc[nt][3]), c1));
+      const float2 a = halves(mul(f2(f.acc[nt][0], f.acc[nt][1]), f2(c0))), b = halves(mul(f2(f.acc[nt][2], f.acc[nt][3]), f2(c1)));
       f.acc[nt][0] = a.x; f.acc[nt][1] = a.y; f.acc[nt][2] = b.x; f.acc[nt][3] = b.y;
     }
   }
@@ -236,15 +237,13 @@ __device__ __forceinline__ void flash_block(FlashState& f, const uint32_t (&qa)[
   f.m[1] = m1;
   uint32_t p[NT][2];
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const F2 shift = f2(-f.m[r]);
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const float2 d = halves(add(t[nt][r], shift));
-      const F2 e = f2(ex2_fast(d.x), ex2_fast(d.y));
-      f.l[r] = FIRST && nt == 0 ? e : add(f.l[r], e);
-      p[nt][r] = pack_bf16(e);
-    }
+  for (int nt = 0; nt < NT; ++nt) {
+    const float2 d0 = halves(add(t[nt][0], f2(-m0))), d1 = halves(add(t[nt][1], f2(-m1)));
+    const float2 e0 = make_float2(ex2_fast(d0.x), ex2_fast(d0.y)), e1 = make_float2(ex2_fast(d1.x), ex2_fast(d1.y));
+    const F2 both = add(f2(e0.x, e1.x), f2(e0.y, e1.y));
+    f.l = FIRST && nt == 0 ? both : add(f.l, both);
+    p[nt][0] = pack_bf16(e0.x, e0.y);
+    p[nt][1] = pack_bf16(e1.x, e1.y);
   }
 #pragma unroll
   for (int h = 0; h < NT / 2; ++h) {
@@ -279,13 +278,13 @@ __device__ __forceinline__ void flash_walk(FlashState& f, bool fresh, const uint
 }
 // The normalised output.
 __device__ __forceinline__ void flash_finish(FlashState& f) {
+  const float2 sums = halves(f.l);
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    const float2 h = halves(f.l[r]);
-    float l = h.x + h.y;
+    float l = r ? sums.y : sums.x;
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
-    const float inv = reciprocal(l);
+    const float inv = 1.0f / l;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
       f.acc[nt][2 * r] *= inv;
@@ -304,11 +303,13 @@ __device__ __forceinline__ void flash_finish(FlashState& f) {
 // stage: bullet rows staged at a time.  Fewer than an environment may have only where every warp has one pair at most, whose
 // softmax then goes on over the next rows.
 //
-// Bound by latency and issue around small mma.sync tiles.  8192 environments of 12 tokens with 18 of 80 bullets 74 -> 51 us, 1024
-// of 152 tokens 93 -> 80: keys past a block of 32 in one of 16, nothing to rescale in the first block (every block of most
-// environments), pairs of scores in one instruction, the heads of a CTA a constant (divisions by it), 48 bullet rows of shared
-// memory instead of every slot's, results out as whole rows.  One copy of the walk and loops that stay loops: a small launch waits for its
-// instructions (28 environments of 6 tokens with bullets 117.3 us a step with a copy each, unrolled, 115.7 so; 1024 of 152 1404 and 1396).  Eighty registers with a few spilled: with 126 the steps take
+// Bound by latency and issue around small mma.sync tiles.  8192 environments of 12 tokens with 18 of 80 bullets 73.3 -> 48.5 us, 1024
+// of 152 tokens 93.0 -> 80.2: keys past a block of 32 in one of 16, nothing to rescale in the first block (every block of most
+// environments), pairs of scores in one instruction, the heads of a CTA a constant (divisions by it), 32 bullet rows of shared
+// memory instead of every slot's (with 64 the step takes 837 us instead of 828), results out as whole rows.  A row's sum over pairs of
+// its columns instead of over even and odd ones, and a division instead of a reciprocal, take 1.0 and 1.6 us of that.  One copy of the walk and
+// loops that stay loops: a small launch waits for its instructions (28 environments of 6 tokens with bullets 117.3 us a step with a copy
+// each, unrolled, 115.7 so; 1024 of 152 1404 and 1396).  Eighty registers with a few spilled: with 126 the steps take
 // 844 us instead of 835 and 1432 instead of 1404, with 64 860 and 1404.
 template <int HPC, bool BULLETS>
 __global__ void __launch_bounds__(256, 3) k_attention_flash(const __nv_bfloat16* __restrict__ qkv, const uint8_t* __restrict__ alive,
@@ -658,8 +659,9 @@ static size_t flash_smem(int max_tokens, int nb, int hpc) {
 }
 constexpr size_t FLASH_SMEM_MAX = 227 * 1024;
 // All four heads in one CTA while that leaves room for three CTAs per SM, else one head per CTA.
-// Bullet rows staged at a time: 48 where every warp (there are four at least) has one (head, query block) pair, so that six CTAs share an SM.
-static int flash_stage(int max_tokens, int nb, int hpc) { return hpc * ((max_tokens + 15) / 16) <= 4 && nb > 48 ? 48 : nb; }
+// Bullet rows staged at a time: 32 where every warp (there are four at least) has one (head, query block) pair, so that registers and not
+// shared memory bound the CTAs of an SM (six).  Whole blocks of 32 keys, or the stage would decide which keys share a block.
+static int flash_stage(int max_tokens, int nb, int hpc) { return hpc * ((max_tokens + 15) / 16) <= 4 && nb > 32 ? 32 : nb; }
 static int flash_heads_per_cta(int max_tokens, int nb) {
   return flash_smem(max_tokens, flash_stage(max_tokens, nb, HEADS), HEADS) <= 72 * 1024 ? HEADS : 1;
 }

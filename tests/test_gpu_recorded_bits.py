@@ -1,0 +1,48 @@
+"""Inference outputs that have no sums in an order of chance, bit for bit as recorded (golden/recorded_bits.json, digests).  The order
+of a float32 sum is part of these results: another one moves bfloat16 roundings in every sublayer behind it, the float32 recurrent
+state by 1e-4 and a few of the actions drawn from the same random numbers."""
+
+import hashlib
+import json
+import os
+
+import pytest
+import torch
+
+from tests.helpers import GOLDEN, build_trunk
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+# tokens, bullet slots, share of them in use (None: no mask): one and several blocks of queries, of keys, of bullet rows
+STEPS = [(12, 80, 0.3), (12, 80, None), (16, 33, 0.5), (5, 16, 0.6), (3, 160, 0.9), (33, 100, 0.5), (129, 0, 0.0), (152, 0, 0.0)]
+
+
+def digest(*tensors) -> str:
+    h = hashlib.sha256()
+    for t in tensors:
+        h.update(t.detach().cpu().contiguous().view(torch.uint8).numpy().tobytes())
+    return h.hexdigest()[:24]
+
+
+def step_digest(tokens, slots, share) -> str:
+    gen = torch.Generator().manual_seed(1000 * tokens + slots)
+    envs = 9
+    trunk = build_trunk([128, 4, 2, 2, 1, 1]).to(DEV)
+    x = torch.randn(envs, tokens, 128, generator=gen).to(DEV, torch.bfloat16)
+    alive = (torch.rand(envs, tokens, generator=gen) < 0.8).to(DEV)
+    hidden = (torch.randn(2, envs * tokens, 512, generator=gen) * 0.5).to(DEV)
+    bullets = torch.randn(envs, slots, 128, generator=gen).to(DEV, torch.bfloat16) if slots else None
+    mask = (torch.rand(envs, slots, generator=gen) < share).to(DEV) if slots and share is not None else None
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        return digest(*trunk.step(x, alive, hidden, bullets=bullets, bullet_mask=mask))
+
+
+def recorded() -> dict:
+    with open(os.path.join(GOLDEN, "recorded_bits.json")) as f:
+        return json.load(f)
+
+
+@pytest.mark.parametrize("tokens,slots,share", STEPS)
+def test_step(tokens, slots, share):
+    assert step_digest(tokens, slots, share) == recorded()[f"step {tokens} {slots} {share}"]
