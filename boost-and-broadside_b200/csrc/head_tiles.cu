@@ -8,8 +8,8 @@
 // The hidden layer never leaves tensor memory and registers: a thread takes 64 hidden columns of its row, four threads
 // add up the row's squares, and the activations go back as the A operand of the second product over the columns they
 // came from.  Tensor memory holds two tiles, so the first product of the next tile runs under this one's epilogue, which
-// is the bound: about 12 instructions per hidden element, two elements at a time (24 one by one: three heads of 65 536 rows and the win
-// head's teams 73 -> 67 us, an encoder of 98 304 rows 64 -> 59; issue slots were 57 % busy, the tensor pipe 12 %, DRAM 3 % of
+// is the bound: about 12 instructions per hidden element, two elements at a time but for the row's squares (24 one by one: three heads of 65 536 rows
+// and the win head's teams 78.2 -> 67.3 us, an encoder of 98 304 rows 66.3 -> 62.4; issue slots were 57 % busy, the tensor pipe 12 %, DRAM 3 % of
 // peak, and the chain of a tile's phases is what is left; an encoder's rows come in element by element).  On mma.sync tiles of 16 rows, with
 // the first product computed twice for the norm, three heads of 65 536 rows took 139 us, one of 16 384 rows 39 (14 here), one of 128 rows no less.
 #include "head_tiles.h"
@@ -47,6 +47,10 @@ __device__ __forceinline__ uint4 pack_row8(const float* src) {
   const float4 a = reinterpret_cast<const float4*>(src)[0], b = reinterpret_cast<const float4*>(src)[1];
   return make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
 }
+
+// A row's squares one after the other: in two chains the norm's root differs in its last bit, and roundings behind it with it, down to
+// the action that is drawn.
+__device__ __forceinline__ float add_squares(float sum, uint32_t two) { return fmaf(bf16_hi(two), bf16_hi(two), fmaf(bf16_lo(two), bf16_lo(two), sum)); }
 
 template <bool ENC>
 __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant__ Args a) {
@@ -193,16 +197,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
         uint32_t v[32];
         tmem_ld32(lane_addr + 256 * (i & 1) + 128 + 32 * part, v);
         tc_fence_before();
-        F2 sq = f2(0.f);
+        float ss = 0.f;
         const F2* bias = reinterpret_cast<const F2*>(b2 + 32 * part);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           v[j] = pack_bf16(add(f2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), bias[j]));
-          const F2 h = unpack_bf16(v[j]);
-          sq = fma(h, h, sq);
+          ss = add_squares(ss, v[j]);
         }
-        const float2 sq2 = halves(sq);
-        const float ss = sq2.x + sq2.y;
         float* sums = reinterpret_cast<float*>(smem + M::SUMS) + 1024 + (i & 1) * 512 + (tid & (TILE - 1));
         sums[part * TILE] = ss;
         asm volatile("bar.sync %0, 128;" ::"r"(3 + quarter) : "memory");
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
       tc_fence_after();
       const uint32_t acc = lane_addr + 256 * (i & 1);
       uint32_t v[32];   // the Linear's output, two bfloat16 a word
-      F2 sq = f2(0.f);
+      float ss = 0.f;
       const float4* bias = reinterpret_cast<const float4*>(b1 + 64 * part);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -269,12 +270,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_head_tiles(const __grid_constant
           uint32_t* w = v + 16 * c + 2 * q;
           w[0] = pack_bf16(add(f2(__uint_as_float(t[4 * q]), __uint_as_float(t[4 * q + 1])), f2(b.x, b.y)));
           w[1] = pack_bf16(add(f2(__uint_as_float(t[4 * q + 2]), __uint_as_float(t[4 * q + 3])), f2(b.z, b.w)));
-          const F2 h0 = unpack_bf16(w[0]), h1 = unpack_bf16(w[1]);
-          sq = fma(h1, h1, fma(h0, h0, sq));
+          ss = add_squares(add_squares(ss, w[0]), w[1]);
         }
       }
-      const float2 sq2 = halves(sq);
-      const float ss = sq2.x + sq2.y;
       float* sums = reinterpret_cast<float*>(smem + M::SUMS) + (i & 1) * 512 + (tid & (TILE - 1));   // two buffers: one barrier a tile
       sums[part * TILE] = ss;
       tc_fence_before();

@@ -33,17 +33,15 @@ namespace mlp {
 using tensor::activation;
 using tensor::add;
 using tensor::f2;
-using tensor::F2;
-using tensor::fma;
-using tensor::halves;
 using tensor::ldsm_x4;
 using tensor::mma_bf16;
 using tensor::pack_bf16;
 using tensor::smem_u32;
-using tensor::unpack_bf16;
 
 namespace {
 
+// Squares of two columns onto a row's sum, one after the other: in two chains the norm's root differs in its last bit.
+__device__ __forceinline__ float add_squares(float sum, uint32_t two) { return fmaf(tensor::bf16_lo(two), tensor::bf16_lo(two), fmaf(tensor::bf16_hi(two), tensor::bf16_hi(two), sum)); }
 // A Linear's output of two columns, bias added.
 __device__ __forceinline__ uint32_t biased(float a, float b, const float2& bias) { return pack_bf16(add(f2(a, b), f2(bias.x, bias.y))); }
 
@@ -315,7 +313,7 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
     __syncwarp();
 
     float acc[8][4];
-    F2 sq0 = f2(0.f), sq1 = f2(0.f);
+    float ss0 = 0.f, ss1 = 0.f;
     if (two_pass) {   // the sum of squares of the rounded Linear 1 output, every chunk
 #pragma unroll 1
       for (int ch = 0; ch < NCH; ++ch) {
@@ -324,9 +322,8 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
           const float2 bb = *reinterpret_cast<const float2*>(b1s + c0 + nt * 8 + 2 * t);
-          const F2 h0 = unpack_bf16(biased(acc[nt][0], acc[nt][1], bb)), h1 = unpack_bf16(biased(acc[nt][2], acc[nt][3], bb));
-          sq0 = fma(h0, h0, sq0);
-          sq1 = fma(h1, h1, sq1);
+          ss0 = add_squares(ss0, biased(acc[nt][0], acc[nt][1], bb));
+          ss1 = add_squares(ss1, biased(acc[nt][2], acc[nt][3], bb));
         }
       }
     }
@@ -347,14 +344,11 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
         hid[nt][0] = biased(acc[nt][0], acc[nt][1], bb);
         hid[nt][1] = biased(acc[nt][2], acc[nt][3], bb);
         if (!two_pass) {
-          const F2 h0 = unpack_bf16(hid[nt][0]), h1 = unpack_bf16(hid[nt][1]);
-          sq0 = fma(h0, h0, sq0);
-          sq1 = fma(h1, h1, sq1);
+          ss0 = add_squares(ss0, hid[nt][0]);
+          ss1 = add_squares(ss1, hid[nt][1]);
         }
       }
       if (c0 == 0) {   // the row sums are complete: after the first pass, or with this only chunk
-        const float2 a = halves(sq0), b = halves(sq1);
-        float ss0 = a.x + a.y, ss1 = b.x + b.y;
         ss0 += __shfl_xor_sync(0xffffffffu, ss0, 1);
         ss0 += __shfl_xor_sync(0xffffffffu, ss0, 2);
         ss1 += __shfl_xor_sync(0xffffffffu, ss1, 1);
@@ -388,7 +382,8 @@ __global__ void __launch_bounds__(32 * max_warps(16 * NP2), 1) k_mlp_bf16(const 
     }
 
     // ---- bias [+ RMSNorm] of Linear 2, then the first out_store columns of the 16 rows
-    float ss0 = 0.f, ss1 = 0.f;
+    ss0 = 0.f;
+    ss1 = 0.f;
 #pragma unroll
     for (int nt = 0; nt < 2 * NP2; ++nt) {
       {

@@ -10,12 +10,15 @@ import pytest
 import torch
 
 from tests.helpers import GOLDEN, build_trunk
+from tests.test_gpu_policy_tail import _Obs, _policy
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 # tokens, bullet slots, share of them in use (None: no mask): one and several blocks of queries, of keys, of bullet rows
 STEPS = [(12, 80, 0.3), (12, 80, None), (16, 33, 0.5), (5, 16, 0.6), (3, 160, 0.9), (33, 100, 0.5), (129, 0, 0.0), (152, 0, 0.0)]
+# environments, ships, fields, bullet slots: one row tile and several, the encoder of wanted rows and of all
+POLICIES = [(16, 8, 0, 0), (300, 8, 4, 80), (41, 5, 1, 33), (700, 2, 0, 0)]
 
 
 def digest(*tensors) -> str:
@@ -38,6 +41,18 @@ def step_digest(tokens, slots, share) -> str:
         return digest(*trunk.step(x, alive, hidden, bullets=bullets, bullet_mask=mask))
 
 
+def policy_digest(envs, ships, fields, slots) -> str:
+    p = _policy(ships, seed=envs)
+    gen = torch.Generator().manual_seed(envs + slots)
+    obs = _Obs(alive=(torch.rand(envs, ships + fields, generator=gen) < 0.8).to(DEV), raw=torch.randn(envs, ships + fields, 66, generator=gen).to(DEV),
+               team_id=torch.randint(0, 2, (envs, ships + fields), generator=gen).to(DEV))
+    obs.bullets = {"raw": torch.randn(envs, slots, 26, generator=gen).to(DEV), "ACTIVE": (torch.rand(envs, slots, generator=gen) < 0.3).to(DEV)} if slots else None
+    hidden = (torch.randn(2, envs * ships, 512, generator=gen) * 0.5).to(DEV)
+    with torch.no_grad(), torch.autocast(DEV, dtype=torch.bfloat16):
+        every = p.bullet_encoder.encode_raw(obs.bullets["raw"]) if slots else hidden   # in steps alone the slots in use are encoded
+        return digest(every, *p.get_action_and_value(obs, hidden, torch.Generator(device=DEV).manual_seed(3)))
+
+
 def recorded() -> dict:
     with open(os.path.join(GOLDEN, "recorded_bits.json")) as f:
         return json.load(f)
@@ -46,3 +61,8 @@ def recorded() -> dict:
 @pytest.mark.parametrize("tokens,slots,share", STEPS)
 def test_step(tokens, slots, share):
     assert step_digest(tokens, slots, share) == recorded()[f"step {tokens} {slots} {share}"]
+
+
+@pytest.mark.parametrize("envs,ships,fields,slots", POLICIES)
+def test_policy(envs, ships, fields, slots):
+    assert policy_digest(envs, ships, fields, slots) == recorded()[f"policy {envs} {ships} {fields} {slots}"]
