@@ -7,7 +7,7 @@
 // (64 registers without bullets hold 47 % of the warps, where 128 held 24 % and it took 95).  The kernels it replaces read rows element by element (one
 // thread per query, or eight lanes per head), ran at 2.2 - 2.6 TB/s on environments of 8 tokens and took 425 /
 // 575 us (forward / gradient) for 1536 environment-steps of 12 tokens with 80 bullet slots, most of it
-// on slots that are not in use (36 / 72 us here, averaged over the sublayers that read them and those that do not).  Here only the slots in use are read.
+// on slots that are not in use (39 / 73 us here, averaged over the sublayers that read them and those that do not).  Here only the slots in use are read.
 //
 // Gradient contract: probabilities recomputed as exp(s - lse) with lse = max + log(sum) in float32, row
 // term <d out, out>, as the fused attention kernels behind F.scaled_dot_product_attention
@@ -48,15 +48,14 @@ __device__ __forceinline__ float4* parts_at(float* base, int ld, size_t off, siz
   return reinterpret_cast<float4*>(base + row * ld + (q / (D / 4)) * off) + q % (D / 4);
 }
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-// Four sums side by side: one of 32 terms is a chain of 32 latencies.
+__device__ __forceinline__ float dot4(const float4& a, const float4& b, float s) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, s)))); }
+// One chain: its order is part of the results (in four chains they differ by 1e-7, and by 1e-3 behind the bfloat16 products that
+// follow), and four took no less time, with 40 and 176 bytes spilled in the gradient for 16 tokens and for 32 with bullets (0 and 124).
 __device__ __forceinline__ float dot32(const float* a, const float* b) {
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  float s = 0.f;
 #pragma unroll
-  for (int i = 0; i < DH / 4; ++i) {
-    const float4 u = ld4(a + 4 * i), v = ld4(b + 4 * i);
-    s.x = fmaf(u.x, v.x, s.x); s.y = fmaf(u.y, v.y, s.y); s.z = fmaf(u.z, v.z, s.z); s.w = fmaf(u.w, v.w, s.w);
-  }
-  return (s.x + s.y) + (s.z + s.w);
+  for (int i = 0; i < DH / 4; ++i) s = dot4(ld4(a + 4 * i), ld4(b + 4 * i), s);
+  return s;
 }
 template <int W>
 __device__ __forceinline__ float seg_sum(float v) {
@@ -194,7 +193,7 @@ __global__ void __launch_bounds__(THREADS) k_env_attn_fwd(const Call c) {
     if constexpr (LPP < 32) {
       // Lane = key: its key in registers, the weights of every query, which then take the key's place; lane = channel: every value
       // once for all queries, their weights by fours.  (A query at a time read all keys, values and a weight by shuffle for each
-      // query: 68 -> 55 us for the environment-steps above.)
+      // query: 66 -> 58 us for the environment-steps above.)
       float k32[DH];
 #pragma unroll
       for (int d4 = 0; d4 < DH / 4; ++d4) *reinterpret_cast<float4*>(&k32[4 * d4]) = ld4(kb + min(lane, kn - 1) * LDB + 4 * d4);
@@ -338,7 +337,7 @@ __global__ void __launch_bounds__(THREADS, LPP == 32 ? 4 : BULLETS ? 3 : LPP == 
         // Lane = key, its key and value in registers while every query's weight and score gradient are computed, which take the
         // value's place; lane = channel sums d q of all queries over the keys, each read once; lane = key again its own
         // gradients.  Loops over four queries stay loops: unrolled over all of them a quarter of the stalls were instruction
-        // fetches.  1536 environment-steps of 12 tokens with 18 of 80 bullets 155 -> 106 us; a query at a time read every key and value
+        // fetches.  1536 environment-steps of 12 tokens with 18 of 80 bullets 153 -> 108 us; a query at a time read every key and value
         // twice and each score gradient by shuffle, and the slots not in use got their zeros here.
         const int mine = min(lane, kn - 1);
 #pragma unroll
@@ -354,7 +353,8 @@ __global__ void __launch_bounds__(THREADS, LPP == 32 ? 4 : BULLETS ? 3 : LPP == 
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int i = min(i0 + u, n - 1);
-            sc[u] = lane < kn ? dot32(q + i * LDQ, dk) * SCALE : -INFINITY;
+            const float qk = dot32(q + i * LDQ, dk);
+            sc[u] = lane < kn ? qk * SCALE : -INFINITY;
             dp[u] = lane < kn ? dot32(go + i * LDO, dv) : 0.f;
             if (keys <= BLOCK) {
               m[u] = seg_max<32>(sc[u]);
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(THREADS, LPP == 32 ? 4 : BULLETS ? 3 : LPP == 
               l[u] = s.l[i * H + h];
               sdp[u] = s.s[i * H + h];
             }
-            p[u] = i0 + u < n ? expf(sc[u] - (m[u] + logf(l[u]))) : 0.f;
+            p[u] = lane < kn && i0 + u < n ? expf(fmaf(qk, SCALE, -(m[u] + logf(l[u])))) : 0.f;   // rounded once, as where a query comes at a time
             ds[u] = p[u] * (dp[u] - sdp[u] / l[u]) * SCALE;
           }
           if (lane < kn) {
