@@ -1589,7 +1589,10 @@ struct Bufs {
   float* w4[3];        // rows x 4D
   float* inv[2];       // rows
   float *bul_n, *bul_inv, *kvb, *dkvb, *bul_dn;
-  float* bul_rows;     // tokens of the bullets in use, one behind the other, with their places per group and their slots
+  // Rows of the bullets in use, where nothing else stands, so that a call plans no byte for them: their places per group and their slots
+  // in the half of bul_n that bfloat16 rows leave; their tokens one behind the other in kvb, where the activations are kept
+  // elsewhere, or else in the caller's gradient of the bullets until that is written (use_bullets).
+  float* bul_rows;
   int *bul_off, *bul_slot;
   // bf16 mode at d_model 128, where the gated MLPs run fused (train_mlp.cu)
   int* status;
@@ -1626,10 +1629,9 @@ void plan(Arena& ar, Bufs& b, int S, int n_images, size_t R, int D, size_t G, si
   b.kvb = ar.take(RB * 2 * D);
   b.dkvb = ar.take(RB * 2 * D);
   b.bul_dn = ar.take(RB * D);
-  if (fused_mlp(D, bf16)) {
-    b.bul_rows = ar.take(RB * D);
-    b.bul_off = reinterpret_cast<int*>(ar.take(G + 1));
-    b.bul_slot = reinterpret_cast<int*>(ar.take(RB));
+  if (fused_mlp(D, bf16) && ar.base) {   // RB * 64 words hold G + 1 + RB where there is a slot at all
+    b.bul_off = reinterpret_cast<int*>(b.bul_n + RB * D / 2);
+    b.bul_slot = b.bul_off + G + 1;
   }
 }
 
@@ -2275,6 +2277,7 @@ int open_buffers(Ctx& c, Kept* kept, const Walk& wk, int n_blocks, int n_spatial
   plan(ar, c.b, kept_ptr ? 0 : wk.S, wk.S, wk.R, wk.D, wk.G, wk.RB, c.bf16);
   if (ar.off + (base - reinterpret_cast<uintptr_t>(scratch)) > scratch_bytes) return BNB_ERR_SCRATCH_TOO_SMALL;
   if (kept_ptr) {
+    c.b.bul_rows = c.b.kvb;
     uintptr_t kb = (reinterpret_cast<uintptr_t>(kept_ptr) + 255) & ~(uintptr_t)255;
     Arena ka{reinterpret_cast<char*>(kb)};
     layout_kept(ka, *kept, wk, n_blocks, n_spatial, n_temporal, c.b, c.bf16);
@@ -2322,11 +2325,13 @@ int prepare_mlps(Ctx& c, const Walk& wk, const BnbSpatialWeights* spatial, const
 // Row tiles and attention take the bullets in use only, 22 % of the slots of a usual batch (the others' weights are exactly
 // 0, and so are their gradients): their rows one behind the other, where the attention kernels read such rows and a mask is given.
 // 1536 environment-steps with 80 slots, two sublayers that read them: training step 2 070 -> 1 920 us (and 1 874 with the attention gradient as it is now).
-int use_bullets(Ctx& c, const Walk& wk, const BnbBullets* bul) {
-  c.compact = bul && bul->active && wk.RB > 0 && wk.RB <= (size_t)INT32_MAX && fused_mlp(c.D, c.bf16) && train_attn::supported(c.D, c.H, wk.NM, wk.nb);
+// rows: where the tokens of those in use may stand for the whole call, or null (then nothing is gathered either).
+int use_bullets(Ctx& c, const Walk& wk, const BnbBullets* bul, float* rows) {
+  c.compact = rows && bul && bul->active && wk.RB > 0 && wk.RB <= (size_t)INT32_MAX && fused_mlp(c.D, c.bf16) && train_attn::supported(c.D, c.H, wk.NM, wk.nb);
   if (!c.compact) return BNB_OK;
+  c.b.bul_rows = rows;
   if (const int rc = tensor::compact_active(bul->active, wk.G, wk.nb, c.b.bul_off, c.b.bul_slot, c.st)) return rc;
-  return launch_after(k_rows_in_use, dim3(blocks_for(wk.RB, 8)), 256, 0, c.st, reinterpret_cast<const float4*>(bul->tokens), reinterpret_cast<float4*>(c.b.bul_rows),
+  return launch_after(k_rows_in_use, dim3(blocks_for(wk.RB, 8)), 256, 0, c.st, reinterpret_cast<const float4*>(bul->tokens), reinterpret_cast<float4*>(rows),
                       c.b.bul_slot, c.b.bul_off + wk.G, 0);
 }
 // The images of sublayer s, for the calls that follow.
@@ -2353,7 +2358,7 @@ int run_fwd_train(const TrunkFwdTrainArgs& a) {
     return status_of(c);
   }
   if ((rc = prepare_mlps(c, wk, a.spatial, a.temporal, a.n_blocks, a.n_spatial, a.n_temporal))) return rc;
-  if ((rc = use_bullets(c, wk, a.bullets))) return rc;
+  if ((rc = use_bullets(c, wk, a.bullets, c.b.bul_rows))) return rc;
   const float* cur = a.x;
   int s = 0;
   for (int blk = 0; blk < a.n_blocks; ++blk) {
@@ -2404,7 +2409,7 @@ int run_bwd(const TrunkBwdArgs& a) {
   }
 
   if ((rc = prepare_mlps(c, wk, a.spatial, a.temporal, a.n_blocks, a.n_spatial, a.n_temporal))) return rc;
-  if ((rc = use_bullets(c, wk, a.bullets))) return rc;
+  if ((rc = use_bullets(c, wk, a.bullets, have_fwd ? c.b.bul_rows : a.d_bullets))) return rc;
   bool bullets_read = false;   // by a sublayer that is behind us
   // the input of every sublayer: kept by the training forward, or from a first pass here
   const float* inputs[256];
@@ -2435,7 +2440,9 @@ int run_bwd(const TrunkBwdArgs& a) {
     }
   }
 
-  if (a.d_bullets && wk.RB) cudaMemsetAsync(a.d_bullets, 0, wk.RB * D * sizeof(float), st);
+  // with the activations recomputed it holds the tokens of the bullets in use until the last sublayer that reads them
+  const bool rows_in_gradient = c.compact && !have_fwd;
+  if (a.d_bullets && wk.RB && !rows_in_gradient) cudaMemsetAsync(a.d_bullets, 0, wk.RB * D * sizeof(float), st);
 
   // sublayers in reverse
   const float* dcur = a.dy;
@@ -2471,9 +2478,12 @@ int run_bwd(const TrunkBwdArgs& a) {
       dcur = dout;
     }
   }
-  if (c.compact && bullets_read && a.d_bullets)
-    c.note(launch_after(k_rows_in_use, dim3(blocks_for(wk.RB, 8)), 256, 0, st, reinterpret_cast<const float4*>(c.b.bul_dn), reinterpret_cast<float4*>(a.d_bullets),
-                        c.b.bul_slot, c.b.bul_off + wk.G, 1));
+  if (rows_in_gradient) cudaMemsetAsync(a.d_bullets, 0, wk.RB * D * sizeof(float), st);
+  if (c.compact && bullets_read && a.d_bullets) {   // behind what may be a memset: launched without programmatic dependence
+    count_launch();
+    k_rows_in_use<<<blocks_for(wk.RB, 8), 256, 0, st>>>(reinterpret_cast<const float4*>(c.b.bul_dn), reinterpret_cast<float4*>(a.d_bullets), c.b.bul_slot,
+                                                        c.b.bul_off + wk.G, 1);
+  }
   return status_of(c);
 }
 
