@@ -2019,8 +2019,9 @@ struct TemporalGeom {
   size_t Rf() const { return (size_t)T * B * (NM - n_rec); }
 };
 
-// Blocks of the conv kernels and the steps of a thread: segments of four steps at least (each reads three rows more) until the
-// chip has two blocks of 256 on every SM.  The gradient, whose blocks end with sums over all of them, walks with that many.
+// Blocks of the conv kernels and the steps of a thread: as many segments (each reads three rows more) as give the chip two blocks of 256
+// on every SM, of about four steps or more: three where there are 5, 6 or 9, and the last segment takes what is left, one step or more.
+// The gradient, whose blocks end with sums over all of them, walks with that many blocks.
 dim3 conv_grid(const ShipGeom& gm, int* seg, bool walk) {
   const size_t blocks = ((size_t)gm.Rr * (gm.D / 4) + 255) / 256, chip = 2 * 148;
   const int wanted = (int)std::min<size_t>((chip + blocks - 1) / blocks, (size_t)(gm.T + 3) / 4);
