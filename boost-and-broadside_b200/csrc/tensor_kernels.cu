@@ -658,10 +658,10 @@ static size_t flash_smem(int max_tokens, int nb, int hpc) {
   return (size_t)(3 * max_tokens + 2 * nb) * flash_stride(hpc) + 4 * (size_t)(((max_tokens + 31) & ~31) + ((nb + 31) & ~31)) + 16;
 }
 constexpr size_t FLASH_SMEM_MAX = 227 * 1024;
-// All four heads in one CTA while that leaves room for three CTAs per SM, else one head per CTA.
 // Bullet rows staged at a time: 32 where every warp (there are four at least) has one (head, query block) pair, so that registers and not
 // shared memory bound the CTAs of an SM (six).  Whole blocks of 32 keys, or the stage would decide which keys share a block.
 static int flash_stage(int max_tokens, int nb, int hpc) { return hpc * ((max_tokens + 15) / 16) <= 4 && nb > 32 ? 32 : nb; }
+// All four heads in one CTA while that leaves room for three CTAs per SM, else one head per CTA.
 static int flash_heads_per_cta(int max_tokens, int nb) {
   return flash_smem(max_tokens, flash_stage(max_tokens, nb, HEADS), HEADS) <= 72 * 1024 ? HEADS : 1;
 }
@@ -933,7 +933,7 @@ struct Plan {
   __nv_bfloat16* o;
   __nv_bfloat16* kvb;    // bullet keys and values of one slice
   int kvb_envs;          // environments per slice
-  int* env_off;          // compaction of the slice's active bullets (see launch_compact)
+  int* env_off;          // compaction of the slice's active bullets (see compact_active)
   int* idx;
   int compacted_e0;      // first environment of the slice env_off / idx currently describe, -1 = none
   bool io_bf16 = false;  // x and y (and so the stream between launches) hold bfloat16
