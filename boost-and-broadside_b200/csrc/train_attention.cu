@@ -57,6 +57,10 @@ __device__ __forceinline__ float dot32(const float* a, const float* b) {
   for (int i = 0; i < DH / 4; ++i) s = dot4(ld4(a + 4 * i), ld4(b + 4 * i), s);
   return s;
 }
+__device__ __forceinline__ void load32(float* to, const float* from) {
+#pragma unroll
+  for (int i = 0; i < DH / 4; ++i) *reinterpret_cast<float4*>(to + 4 * i) = ld4(from + 4 * i);
+}
 template <int W>
 __device__ __forceinline__ float seg_sum(float v) {
 #pragma unroll
@@ -161,10 +165,16 @@ __global__ void __launch_bounds__(THREADS) k_env_attn_fwd(const Call c) {
   const float* v = q + 2 * D;
   const bool key = sub < n;
   const bool dead = key && c.alive && !c.alive[tok0 + sub];
+  // More than 16 tokens: a warp takes one query at a time and a lane one key for all of them, in registers.  1184 environment-steps of 20 tokens
+  // 54 -> 45 us, 1280 of 32 106 -> 89; with bullets the same below, 80 for 20 tokens 282 -> 239, 40 for 32 604 -> 511.  (Read from shared memory for
+  // each query the instances with and without bullets were slower than the one kernel for both had been: 51, 100, 260 and 531.)
+  constexpr bool ONE = LPP == 32;
+  float own[ONE ? DH : 1];
+  if constexpr (ONE) load32(own, k + min(sub, n - 1) * LDQ);
   for (int q0 = 0; q0 < n; q0 += QPW) {
     const int i = q0 + qs, ic = min(i, n - 1);
     float sc = -INFINITY;
-    if (key) sc = dead ? kMaskedScore : dot32(q + ic * LDQ, k + sub * LDQ) * SCALE;
+    if (key) sc = dead ? kMaskedScore : dot32(q + ic * LDQ, ONE ? own : k + sub * LDQ) * SCALE;
     const float mx = seg_max<LPP>(sc);
     const float e = key ? expf(sc - mx) : 0.f;
     const float p = e / seg_sum<LPP>(e);
@@ -195,8 +205,7 @@ __global__ void __launch_bounds__(THREADS) k_env_attn_fwd(const Call c) {
       // once for all queries, their weights by fours.  (A query at a time read all keys, values and a weight by shuffle for each
       // query: 66 -> 58 us for the environment-steps above.)
       float k32[DH];
-#pragma unroll
-      for (int d4 = 0; d4 < DH / 4; ++d4) *reinterpret_cast<float4*>(&k32[4 * d4]) = ld4(kb + min(lane, kn - 1) * LDB + 4 * d4);
+      load32(k32, kb + min(lane, kn - 1) * LDB);
       __syncwarp();
 #pragma unroll 1
       for (int i0 = 0; i0 < n; i0 += 4) {   // four queries side by side, the last ones perhaps the last query again
@@ -241,8 +250,9 @@ __global__ void __launch_bounds__(THREADS) k_env_attn_fwd(const Call c) {
       for (int i = 0; i < LPP; ++i)
         if (i < n) s.acc[(n + i) * D + h * DH + lane] = a[i];
     } else {
+      load32(own, kb + min(lane, kn - 1) * LDB);
       for (int i = 0; i < n; ++i) {
-        const float sc = lane < kn ? dot32(q + i * LDQ, kb + lane * LDB) * SCALE : -INFINITY;
+        const float sc = lane < kn ? dot32(q + i * LDQ, own) * SCALE : -INFINITY;
         const float m0 = s.m[i * H + h];
         const float mx = fmaxf(m0, seg_max<32>(sc));
         const float e = lane < kn ? expf(sc - mx) : 0.f;
