@@ -1246,7 +1246,10 @@ struct ShipGeom {
 
 // The conv has no recurrence: a thread takes four channels of a row for `seg` steps, with the next ones on their way while one is
 // worked on.  (A channel per thread over all steps, one step ahead, had 8 KB of rows on their way per SM: within a training
-// step of 262 144 rows 98 us and 150 for the gradient, where this takes 72 and 107, 268 and 402 MB besides the state.)
+// step of 262 144 rows 97 us and 153 for the gradient, where this takes 54 and 101, 268 and 402 MB besides the state.)  Taps, weights and
+// state come as 16 bytes: every pointer of a call is on such a boundary (BNB_ERR_MISALIGNED otherwise).  One by one, 28 loads a
+// thread, they were most of a call of few steps: 16 384 rows of one step 28 -> 14 us (a channel per thread: 16), gradient 36 -> 26 (76),
+// 603 rows of five 6.4 -> 4.4 (4.4), 8.1 -> 7.2 (6.8).
 constexpr int CONV_AHEAD = 4;
 // Episode boundaries right before the steps t - 1 - k, k < N, as bits; all loads at once.
 template <int N>
@@ -1267,13 +1270,15 @@ __device__ __forceinline__ float& part(float4& v, int c) { return c == 0 ? v.x :
 __device__ __forceinline__ void padded_before(float4 (&pad)[4], const float* __restrict__ b1, const float* __restrict__ hid, const ShipGeom& gm, int s, int d, int p) {
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    if (p + k >= 3) {
-      pad[k] = *reinterpret_cast<const float4*>(b1 + ((size_t)(p + k - 3) * gm.Rr + s) * gm.D + d);
-    } else {
-      const float* h = hid + (size_t)s * 4 * gm.D + (size_t)(p + k + 1) * gm.D + d;   // the caller's: any alignment
-      pad[k] = make_float4(h[0], h[1], h[2], h[3]);
-    }
+    pad[k] = *reinterpret_cast<const float4*>(p + k >= 3 ? b1 + ((size_t)(p + k - 3) * gm.Rr + s) * gm.D + d
+                                                         : hid + (size_t)s * 4 * gm.D + (size_t)(p + k + 1) * gm.D + d);
   }
+}
+
+// The four taps of channels d .. d + 3.
+__device__ __forceinline__ void conv_taps(float (&w)[4][4], const float* __restrict__ cw, int d) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) *reinterpret_cast<float4*>(w[c]) = *reinterpret_cast<const float4*>(cw + (d + c) * 4);
 }
 
 // u_t = conv bias + sum over lags of tap * padded value, a lag being valid while no episode boundary
@@ -1296,13 +1301,9 @@ __global__ void __launch_bounds__(256, 3) k_conv_fwd(const float* __restrict__ b
   for (int i = 0; i < CONV_AHEAD; ++i)
     if (t0 + i < t1) next[i] = *reinterpret_cast<const float4*>(in + (size_t)(t0 + i) * step);
   padded_before(pad, b1, hid, gm, s, d, t0);
-  float w[4][4], bias[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    bias[c] = cb[d + c];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) w[c][k] = cw[(d + c) * 4 + k];
-  }
+  alignas(16) float w[4][4], bias[4];
+  conv_taps(w, cw, d);
+  *reinterpret_cast<float4*>(bias) = *reinterpret_cast<const float4*>(cb + d);
   int cur = valid_lags(boundaries<3>(gm, t0, b));
 #pragma unroll 1
   for (int t = t0; t < t1; t += CONV_AHEAD) {
@@ -1462,12 +1463,15 @@ __global__ void __launch_bounds__(256, 2) k_conv_bwd(const float* __restrict__ d
                                                   float* __restrict__ db1, float* __restrict__ d_cw, float* __restrict__ d_cb,
                                                   ShipGeom gm, int seg) {
   tensor::let_next_start();
-  tensor::wait_for_previous();
   constexpr int BWD_AHEAD = 2;   // of two tensors
-  __shared__ float sums[20 * (MAXW / 4)];   // [tap and channel of the quad, or bias][quad]: lanes side by side
+  // [tap and channel of the quad, or bias][copy, quad]: lanes side by side, about eight threads to a sum whatever the width (one copy of
+  // 32 channels has 32 threads to each: gradient of 768 rows of 16 steps 14.7 -> 6.7 us)
+  constexpr int COLUMNS = MAXW / 4;
+  __shared__ float sums[20 * COLUMNS];
   const int per_row = gm.D / 4;
-  for (int i = threadIdx.x; i < 20 * per_row; i += blockDim.x) sums[i] = 0.f;
+  for (int i = threadIdx.x; i < 20 * COLUMNS; i += blockDim.x) sums[i] = 0.f;
   __syncthreads();
+  tensor::wait_for_previous();
   for (size_t quad = (size_t)blockIdx.x * blockDim.x + threadIdx.x; quad < (size_t)gm.Rr * per_row; quad += (size_t)gridDim.x * blockDim.x) {
     const int s = (int)(quad / per_row), d = 4 * (int)(quad - (size_t)s * per_row), b = s / gm.n_rec;
     const int T = gm.T, D = gm.D, t0 = blockIdx.y * seg, t1 = min(t0 + seg, T);
@@ -1483,21 +1487,17 @@ __global__ void __launch_bounds__(256, 2) k_conv_bwd(const float* __restrict__ d
     // padded index p: 0..2 the stored taps, 3 + t the linear1 output of step t
     auto emit = [&](int p, float4 v) {
       if (p >= T && d_hid_out) {
-        const float* h = d_hid_out + (size_t)s * 4 * D + D + (size_t)(p - T) * D + d;
-        v.x += h[0]; v.y += h[1]; v.z += h[2]; v.w += h[3];
+        const float4 h = *reinterpret_cast<const float4*>(d_hid_out + (size_t)s * 4 * D + D + (size_t)(p - T) * D + d);
+        v.x += h.x; v.y += h.y; v.z += h.z; v.w += h.w;
       }
       if (p >= 3) {
         *reinterpret_cast<float4*>(db1 + ((size_t)(p - 3) * gm.Rr + s) * D + d) = v;
       } else if (d_hid_in) {
-        float* h = d_hid_in + (size_t)s * 4 * D + D + (size_t)p * D + d;
-        h[0] = v.x; h[1] = v.y; h[2] = v.z; h[3] = v.w;
+        *reinterpret_cast<float4*>(d_hid_in + (size_t)s * 4 * D + D + (size_t)p * D + d) = v;
       }
     };
-    float w[4][4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) w[c][k] = cw[(d + c) * 4 + k];
+    alignas(16) float w[4][4];
+    conv_taps(w, cw, d);
     float4 acc[4], pad[4];   // d padded[t .. t+3], padded[t .. t+3] at step t
     float dw[4][4] = {}, dbias[4] = {};
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1553,17 +1553,22 @@ __global__ void __launch_bounds__(256, 2) k_conv_bwd(const float* __restrict__ d
     if (t1 == T)
 #pragma unroll
       for (int k = 0; k < 3; ++k) emit(T + k, acc[k]);
+    const int copies = COLUMNS / per_row;
+    float* to = sums + d / 4 + (copies > 1 ? (int)threadIdx.x / per_row % copies * per_row : 0);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) atomicAdd(&sums[(4 * k + c) * per_row + d / 4], dw[c][k]);
-      atomicAdd(&sums[(16 + c) * per_row + d / 4], dbias[c]);
+      for (int k = 0; k < 4; ++k) atomicAdd(to + (4 * k + c) * COLUMNS, dw[c][k]);
+      atomicAdd(to + (16 + c) * COLUMNS, dbias[c]);
     }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < gm.D * 5; i += blockDim.x) {   // whole lines of d conv weight, then of its bias
     const int k = i < gm.D * 4 ? i & 3 : 4, d = k < 4 ? i >> 2 : i - gm.D * 4;
-    atomicAdd(k < 4 ? d_cw + i : d_cb + d, sums[(4 * k + (d & 3)) * per_row + (d >> 2)]);
+    const float* from = sums + (4 * k + (d & 3)) * COLUMNS + (d >> 2);
+    float v = 0.f;
+    for (int j = 0; j + per_row <= COLUMNS; j += per_row) v += from[j];
+    atomicAdd(k < 4 ? d_cw + i : d_cb + d, v);
   }
 }
 
